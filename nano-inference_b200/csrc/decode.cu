@@ -22,7 +22,6 @@ const void* decode_kernel_tp_lean(int HD, int G);
 const void* decode_kernel_tp_prof_lean(int HD, int G);
 const void* decode_kernel_lean_mid(int HD, int G);
 const void* decode_kernel_lean_long(int HD, int G);
-int reset_after_error(mi_ctx* ctx, mi_model* m);
 }
 
 namespace {
@@ -169,7 +168,7 @@ extern "C" int mi_model_free(mi_ctx* ctx, mi_model* m) {
     cudaDeviceSynchronize();
     for (void* p : m->ipc_opened) cudaIpcCloseMemHandle(p);
     for (void* p : m->allocs) cudaFree(p);
-    for (void* g : m->vb.graph) if (g) cudaGraphExecDestroy((cudaGraphExec_t)g);
+    mi::free_verify_bufs(m);
     for (void* g : m->step_graph) if (g) cudaGraphExecDestroy((cudaGraphExec_t)g);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
@@ -937,12 +936,9 @@ static int launch_phases(mi_ctx* ctx, mi_model* m, int pos, int phase_begin, int
 int mi::reset_after_error(mi_ctx* ctx, mi_model* m) {
     if (m->errors_seen == ctx->errors_reported) return MI_OK;
     m->errors_seen = ctx->errors_reported;
-    reset_counters_kernel<<<1, 256, 0, ctx->stream>>>(m->P.attn_cnt, m->NH, m->vb.attn_cnt, m->vb.attn_cnt ? 16 * m->NH : 0);
+    reset_counters_kernel<<<1, 256, 0, ctx->stream>>>(m->P.attn_cnt, m->NH, m->vb.attn_cnt, m->vb.cap * m->NH);
     MI_CUDA(ctx, cudaGetLastError());
-    if (m->vb.amax_cnt) {
-        MI_CUDA(ctx, cudaMemsetAsync(m->vb.amax_cnt, 0, 16 * sizeof(unsigned), ctx->stream));
-        MI_CUDA(ctx, cudaMemsetAsync(m->vb.amax_key, 0, 16 * sizeof(unsigned long long), ctx->stream));
-    }
+    if (m->vb.pick_cnt) MI_CUDA(ctx, cudaMemsetAsync(m->vb.pick_cnt, 0, m->vb.cap_logits * sizeof(unsigned), ctx->stream));
     return MI_OK;
 }
 

@@ -61,7 +61,7 @@
 // exact and the fp32 value cannot depend on their order; beyond that it has been
 // observed, not proved.  Each token is processed exactly as if it were alone.
 #pragma once
-#include "gemv_core.cuh"
+#include "gemm_tok.cuh"
 #ifndef MI_ATT_FN
 #define MI_ATT_FN static __device__ __noinline__
 #endif
@@ -203,7 +203,7 @@ struct DecodeParams {
     // plain (untagged) vectors: inputs / outputs of the attention code when it runs as a kernel of its own (M-token step)
     float* qkv_out;
     float* att;                      // merged attention output, fp32 (also written by the decode loop, for inspection)
-    int8_t* att_q; __half* att_d;
+    TokX att_x; int att_token;       // the same as q8_0 in operand order, as this token (M-token step; null elsewhere)
     __half* kc; __half* vc; int max_seq;       // [L][max_seq][KVD]
     double* attn_part; unsigned* attn_cnt; int max_chunks;  // [NH][max_chunks][HD+2], [NKV]
     float* out_margins;              // optional [n_steps]: top-1 minus top-2 logit of every step
@@ -577,31 +577,11 @@ __device__ MI_PIECE bool run_warp_job(WarpStream& ws, int j, int lane, const int
 
 // ---- activation staging (whole CTA; returns a CTA-uniform ok) -----------------------
 
-// Warp-wide maximum of non-negative floats and warp-wide integer sum as single redux
-// instructions (the bit pattern of a non-negative float orders like an unsigned integer);
-// a shuffle tree costs five issue slots of a pipe that retires one warp instruction per clock.
-__device__ __forceinline__ float warp_max_nonneg(float a) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(a))); }
-__device__ __forceinline__ int warp_sum_int(int v) { return __reduce_add_sync(0xffffffffu, v); }
 // warp-wide maximum of arbitrary finite floats (or -inf): order-preserving key
 __device__ __forceinline__ float warp_max_float(float a) {
     const unsigned b = __float_as_uint(a), key = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
     const unsigned m = __reduce_max_sync(0xffffffffu, key);
     return __uint_as_float((m & 0x80000000u) ? (m & 0x7fffffffu) : ~m);
-}
-
-// q8_0 of one 32-element block held one element per lane; returns the int8 value,
-// writes the fp16 scale through lane 0 (plain stores: the attention kernel of the M-token step).
-__device__ __forceinline__ int quant_block_warp(float v, int lane, float2* xs_out, __half* xd_out) {
-    const float a = warp_max_nonneg(fabsf(v));
-    const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
-    const int q = __float2int_rn(__fmul_rn(v, inv));
-    const int s = warp_sum_int(q);
-    if (lane == 0) {
-        const __half d = __float2half_rn(__fdiv_rn(a, 127.f));
-        if (xs_out) *xs_out = make_float2(__half2float(d), __int2float_rn(8 * s));
-        if (xd_out) *xd_out = d;
-    }
-    return q;
 }
 
 // Residual add + RMSNorm + q8_0 staging:
@@ -1083,7 +1063,7 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
                     const int qv8 = quant_block_warp2(v, dq, sq);
                     publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
                 } else {
-                    P.att_q[e] = (int8_t)quant_block_warp(v, lane, nullptr, P.att_d + (e >> 5));
+                    if (P.att_x.q) store_tok_block(P.att_x, e >> 5, P.att_token, lane, v);
                 }
             }
         } else {
@@ -1154,7 +1134,7 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
                 const int qv8 = quant_block_warp2(v, dq, sq);
                 publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
             } else {
-                P.att_q[e] = (int8_t)quant_block_warp(v, lane, nullptr, P.att_d + (e >> 5));
+                if (P.att_x.q) store_tok_block(P.att_x, e >> 5, P.att_token, lane, v);
             }
         }
     }
@@ -1347,7 +1327,7 @@ MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* s
             const int qv8 = quant_block_warp2(v, dq, sq);
             publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
         } else {
-            P.att_q[e] = (int8_t)quant_block_warp(v, lane, nullptr, P.att_d + (e >> 5));
+            if (P.att_x.q) store_tok_block(P.att_x, e >> 5, P.att_token, lane, v);
         }
     }
     prof_mark(P, 17);

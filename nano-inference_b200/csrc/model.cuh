@@ -2,26 +2,33 @@
 #pragma once
 #include "decode_kernel.cuh"
 
+#include <map>
+#include <set>
+#include <tuple>
 #include <vector>
 
 namespace mi {
+// what a captured pass depends on besides the buffers: tokens, attention grid, kind of meta block, the cache
+struct PassKey {
+    int M, regime, ragged; const void* kc; const void* vc; int max_seq;
+    bool operator<(const PassKey& o) const { return std::tie(M, regime, ragged, kc, vc, max_seq) < std::tie(o.M, o.regime, o.ragged, o.kc, o.vc, o.max_seq); }
+};
 // device buffers of the M-token step (all [tokens][...], token-major)
 struct VerifyBufs {
-    int cap = 0;                       // tokens the buffers hold
+    int cap = 0, cap_logits = 0;       // tokens the buffers hold
+    std::vector<void*> mem;            // the allocations behind the pointers below
     float* X = nullptr;                // residual stream [M][E]
-    float* Y = nullptr;                // projection output [M][max(qkv_rows, 2FF, E)]
-    float* qkv = nullptr;              // [M][qkv_rows (padded)] after bias and RoPE, packed row order
-    int8_t* xq = nullptr; __half* xd = nullptr;         // q8_0 of the normed input [M][E]
-    float* att = nullptr; int8_t* att_q = nullptr; __half* att_d = nullptr;   // [M][NQ]
-    int8_t* act_q = nullptr; __half* act_d = nullptr;   // [M][FF]
+    double* part = nullptr; int ldp = 0;    // sums of a projection per K range [range][M][ldp]
+    float* q = nullptr;                // [M][NQ] after bias and RoPE, natural order
+    TokX xf{}, attf{}, actf{};         // q8_0 of the normed input, the attention output and SwiGLU, in operand order
+    float* att = nullptr;              // [M][NQ]
     float* logits = nullptr;           // [M][V]
-    int* tokens = nullptr; int* out = nullptr;          // [M]
-    int* pos0 = nullptr;               // first position of the pass (device resident so that the launch sequence is position-free)
-    void* graph[51] = {};              // cudaGraphExec_t of the pass per M, and the scratch addresses each was built with
-    const void* graph_part[51] = {}; const void* graph_cnt[51] = {};
-    bool warm[51] = {};                // index: M + 17 * attention regime (see verify.cu)
+    int* meta = nullptr; int* h_meta = nullptr;         // tokens | positions | slots, or tokens | first position; its pinned image
+    int* out = nullptr;                // [M]
+    std::map<PassKey, void*> graphs;   // cudaGraphExec_t
+    std::set<PassKey> warm;            // kinds of pass that have run plainly once
     double* attn_part = nullptr; unsigned* attn_cnt = nullptr;   // [M][NH][max_chunks][HD+2], [M][NH]
-    unsigned long long* amax_key = nullptr; unsigned* amax_cnt = nullptr;   // [M] argmax scratch, self-clearing
+    float* pick = nullptr; unsigned* pick_cnt = nullptr;         // greedy pick: candidates per slice, arrival counters (self-clearing)
     float* margins = nullptr;          // [M] greedy logit minus the runner-up
 };
 }
@@ -65,6 +72,9 @@ struct mi_model {
 
 
 namespace mi {
+
+void free_verify_bufs(mi_model* m);
+int reset_after_error(mi_ctx* ctx, mi_model* m);
 
 template <typename T>
 int dev_alloc(mi_ctx* ctx, mi_model* m, T** p, size_t n, bool zero = true) {
