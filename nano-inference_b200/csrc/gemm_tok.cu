@@ -37,16 +37,13 @@ namespace mi {
 constexpr int kRing = 2;                                     // ring slots per warp
 constexpr int kStaticSmem = 64;                              // room for static shared memory
 constexpr int kFoldLd = 34;                                  // doubles per token in the fold buffer: conflict-free for the MMA's layout
-constexpr int kRowLd = 36;                                   // floats per token in a warp's own buffer
 __host__ __device__ constexpr int tok_warps(int NT) { return NT <= 2 ? 12 : 8; }
 
-template <int KB, int NT, int MODE, bool FOLD>
+template <int KB, int NT, bool FOLD>
 struct TokSmem {
     static constexpr int W = tok_warps(NT), TB = tile_bytes(KB), N = NT * 8;
     static constexpr int ring = W * kRing * TB;
-    // partial sums of all warps; or per warp the unit's rows as fp32 (gate and up), where the epilogue wants a row on every lane
-    static constexpr int rows = MODE == GEMM_GU ? 2 : MODE == GEMM_QKV ? 1 : 0;
-    static constexpr int scratch = FOLD ? W * N * kFoldLd * 8 : W * N * rows * kRowLd * 4;
+    static constexpr int scratch = FOLD ? W * N * kFoldLd * 8 : 0;                          // partial sums of all warps
     static constexpr int bars = ((W * kRing + 1) * 8 + 15) / 16 * 16;
     static constexpr int fixed = ring + scratch + bars;
     static constexpr int x_block = NT * 256 + N * 8, x_tile = KB * x_block;
@@ -109,41 +106,11 @@ __device__ __forceinline__ void tile_mma(const uint8_t* tile, const uint2* bs, c
     }
 }
 
-// ---- epilogues: one warp, lane = row of a group, one token -------------------------------------------------------------
-// v: the row's sum with the bias added (all lanes call)
-__device__ __forceinline__ void store_qkv(const GemmParams& p, int row, int n, float v) {
-    const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
-    if (row >= p.nq + 2 * p.KVD) return;
-    const int pos = p.pos_arr ? __ldg(p.pos_arr + n) : __ldg(p.pos0) + n;
-    const size_t slab = p.slot_arr ? (size_t)__ldg(p.slot_arr + n) * (size_t)p.slab_stride : 0;
-    const size_t crow = slab + ((size_t)p.layer * p.max_seq + pos) * p.KVD;
-    if (row >= p.nq + p.KVD) { p.vc[crow + (row - p.nq - p.KVD)] = __float2half_rn(v); return; }
-    // q and k rows come pair-adjacent: slots 2i and 2i + 1 of a head are its dims i and i + HD / 2
-    const int within0 = row < p.nq ? row : row - p.nq, head = within0 / p.HD, within = within0 - head * p.HD, i = within >> 1;
-    double c, s;
-    if (pos < p.rope_rows) {
-        c = (double)__ldg(p.rope_cs + (size_t)pos * p.HD + i); s = (double)__ldg(p.rope_cs + (size_t)pos * p.HD + p.HD / 2 + i);
-    } else {
-        const double th = (double)__fmul_rn((float)pos, __ldg(p.rope_freq + i));            // fp32 angle, as src/cpu_infer.cpp:54
-        c = (double)__double2float_rn(cos(th)); s = (double)__double2float_rn(sin(th));
-    }
-    const bool odd = within & 1;
-    const float out = odd ? __double2float_rn(__dadd_rn(__dmul_rn((double)partner, s), __dmul_rn((double)v, c)))
-                          : __double2float_rn(__dsub_rn(__dmul_rn((double)v, c), __dmul_rn((double)partner, s)));
-    const int nat = head * p.HD + i + (odd ? p.HD / 2 : 0);
-    if (row < p.nq) p.q[(size_t)n * p.nq + nat] = out;
-    else p.kc[crow + nat] = __float2half_rn(out);
-}
-
-__device__ __forceinline__ float swiglu(float gate, float up) {
-    const double gd = (double)gate;
-    return __double2float_rn(__dmul_rn(__ddiv_rn(gd, __dadd_rn(1.0, exp(-gd))), (double)up));
-}
-
 template <int KB, int NT, int MODE, bool ROWMAJOR, bool FOLD>
 __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(const __grid_constant__ GemmParams p) {
-    using SM = TokSmem<KB, NT, MODE, FOLD>;
-    constexpr int W = SM::W, TB = SM::TB, N = SM::N, U = MODE == GEMM_GU ? 2 : 1, PASS = FOLD ? 1 : U;
+    using SM = TokSmem<KB, NT, FOLD>;
+    constexpr int W = SM::W, TB = SM::TB, N = SM::N, U = MODE == GEMM_GU ? 2 : 1;
+    static_assert(FOLD || MODE == GEMM_PLAIN || MODE == GEMM_PART, "epilogues across rows work on folded sums");
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* scratch = smem + SM::ring;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::ring + SM::scratch);
@@ -153,10 +120,10 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int sp = (int)(blockIdx.x % p.ksg), rest = (int)(blockIdx.x / p.ksg), c = rest % p.C, tt = rest / p.C;
     const int k0 = sp * p.nt / p.ksg, k1 = (sp + 1) * p.nt / p.ksg, nchunk = (k1 - k0 + p.kct - 1) / p.kct;      // this CTA's K range, in tiles
-    // the warp's row group of round r and pass q: group0 + r * gstride + q, while below glimit
+    // the warp's row group of round r: group0 + r * gstride, while below glimit
     const int kw = FOLD ? p.kw : 1, rg = FOLD ? W / kw : W, gi = FOLD ? warp / kw : warp, part = FOLD ? warp - gi * kw : 0;
-    const int group0 = FOLD ? c * rg + gi : (warp * p.C + c) * U, gstride = p.C * rg * (FOLD ? 1 : U), glimit = gi < rg ? p.groups : 0;
-    const int rounds = FOLD ? ((p.groups + rg - 1) / rg - c + p.C - 1) / p.C : (p.groups / U + p.C * W - 1) / (p.C * W);
+    const int group0 = FOLD ? c * rg + gi : warp * p.C + c, gstride = p.C * rg, glimit = gi < rg ? p.groups : 0;
+    const int rounds = FOLD ? ((p.groups + rg - 1) / rg - c + p.C - 1) / p.C : (p.groups + p.C * W - 1) / (p.C * W);
     const int ntok = min(N, p.M - tt * N);
 
     uint8_t* ring = smem + (size_t)warp * kRing * TB;
@@ -168,18 +135,18 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
         mbar_fence_init();
     }
     __syncwarp();
-    // producer (lane 0), kRing tiles ahead of the consumer below: every kw-th tile of the K range, pass after pass, round after round
+    // producer (lane 0), kRing tiles ahead of the consumer below: every kw-th tile of the K range, round after round
     const uint64_t policy = l2_policy_evict_first();
-    int issued = 0, consumed = 0, pr = 0, pq = 0, pt = k0 + part;
+    int issued = 0, consumed = 0, pr = 0, pt = k0 + part;
     auto issue_one = [&]() {
         if (pr >= rounds || pt >= k1) return;                                            // done, or more warps than tiles
-        const int grp = group0 + pr * gstride + pq;
+        const int grp = group0 + pr * gstride;
         if (grp >= glimit) { pr = rounds; return; }                                      // groups only grow: nothing follows
         const int s = issued % kRing;
         mbar_expect_tx(&rbar[s], TB);
         bulk_g2s_hint(ring + (size_t)s * TB, p.base + ((size_t)grp * p.nt + pt) * TB, TB, &rbar[s], policy);
         issued++; pt += kw;
-        if (pt >= k1) { pt = k0 + part; if (++pq == PASS) { pq = 0; pr++; } }
+        if (pt >= k1) { pt = k0 + part; pr++; }
     };
     if (lane == 0) {
         #pragma unroll
@@ -235,87 +202,61 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
     for (int r = 0; r < rounds; r++) {
         const int grp0 = group0 + r * gstride;
         const bool mine = grp0 < glimit;
-        float* mrows = reinterpret_cast<float*>(scratch) + (size_t)warp * (N * SM::rows * kRowLd);      // [pass][token][row]
         double acc[NT][8];
-        #pragma unroll 1
-        for (int q = 0; q < PASS; q++) {
+        #pragma unroll
+        for (int j = 0; j < NT; j++)
             #pragma unroll
-            for (int j = 0; j < NT; j++)
-                #pragma unroll
-                for (int i = 0; i < 8; i++) acc[j][i] = 0.0;
-            __half2 poison[4];
-            #pragma unroll
-            for (int i = 0; i < 4; i++) poison[i] = __half2half2(__ushort_as_half(0));
-            int t = k0 + part;
-            for (int ch = 0; ch < nchunk; ch++) {
-                const int c0 = k0 + ch * p.kct, c1 = min(c0 + p.kct, k1);
-                if (nchunk > 1 && !first) {                                              // everyone has left the previous chunk: the next one over it
-                    __syncthreads();
-                    if constexpr (!ROWMAJOR) { if (warp == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-                    stage(c0 * KB, (c1 - c0) * KB);
-                    if constexpr (ROWMAJOR) __syncthreads(); else xready = false;
-                }
-                first = false;
-                if (!xready) {
-                    if (ok && !mbar_wait_bounded(xbar, xphase)) ok = false;
-                    xphase ^= 1u; xready = true;
-                }
-                if (mine) {
-                    for (; t < c1 && ok; t += kw) {
-                        const int s = consumed % kRing;
-                        if (!mbar_wait_bounded(&rbar[s], (consumed / kRing) & 1)) { ok = false; break; }
-                        tile_mma<KB, NT>(ring + (size_t)s * TB, bs + (size_t)(t - c0) * (KB * NT * 32), dxs + (size_t)(t - c0) * (KB * N), lane, acc, poison, pair);
-                        consumed++;
-                        __syncwarp();
-                        if (lane == 0) issue_one();
-                    }
-                }
+            for (int i = 0; i < 8; i++) acc[j][i] = 0.0;
+        __half2 poison[4];
+        #pragma unroll
+        for (int i = 0; i < 4; i++) poison[i] = __half2half2(__ushort_as_half(0));
+        int t = k0 + part;
+        for (int ch = 0; ch < nchunk; ch++) {
+            const int c0 = k0 + ch * p.kct, c1 = min(c0 + p.kct, k1);
+            if (nchunk > 1 && !first) {                                              // everyone has left the previous chunk: the next one over it
+                __syncthreads();
+                if constexpr (!ROWMAJOR) { if (warp == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+                stage(c0 * KB, (c1 - c0) * KB);
+                if constexpr (ROWMAJOR) __syncthreads(); else xready = false;
             }
-            #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const double po = (double)__half2float(__hadd(__low2half(poison[i]), __high2half(poison[i])));
-                #pragma unroll
-                for (int j = 0; j < NT; j++) { acc[j][2 * i] = __dadd_rn(acc[j][2 * i], po); acc[j][2 * i + 1] = __dadd_rn(acc[j][2 * i + 1], po); }
+            first = false;
+            if (!xready) {
+                if (ok && !mbar_wait_bounded(xbar, xphase)) ok = false;
+                xphase ^= 1u; xready = true;
             }
-            if constexpr (!FOLD && SM::rows > 0) {
-                if (mine) {
-                    #pragma unroll
-                    for (int j = 0; j < NT; j++)
-                        #pragma unroll
-                        for (int i = 0; i < 8; i++) mrows[(q * N + 8 * j + 2 * t4 + (i & 1)) * kRowLd + g + 8 * (i >> 1)] = __double2float_rn(acc[j][i]);
+            if (mine) {
+                for (; t < c1 && ok; t += kw) {
+                    const int s = consumed % kRing;
+                    if (!mbar_wait_bounded(&rbar[s], (consumed / kRing) & 1)) { ok = false; break; }
+                    tile_mma<KB, NT>(ring + (size_t)s * TB, bs + (size_t)(t - c0) * (KB * NT * 32), dxs + (size_t)(t - c0) * (KB * N), lane, acc, poison, pair);
+                    consumed++;
+                    __syncwarp();
+                    if (lane == 0) issue_one();
                 }
             }
         }
+        #pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const double po = (double)__half2float(__hadd(__low2half(poison[i]), __high2half(poison[i])));
+            #pragma unroll
+            for (int j = 0; j < NT; j++) { acc[j][2 * i] = __dadd_rn(acc[j][2 * i], po); acc[j][2 * i + 1] = __dadd_rn(acc[j][2 * i + 1], po); }
+        }
         if constexpr (!FOLD) {
             if (!mine) continue;
-            if constexpr (MODE == GEMM_GU || MODE == GEMM_QKV) {
-                // a loop over the tokens, not unrolled: the exponential, the division and the angles are a few hundred
-                // instructions, and one copy of them stays in the instruction cache (32 copies took longer than the products)
-                __syncwarp();
-                const float bv = MODE == GEMM_QKV ? __ldg(p.bias + grp0 * 32 + lane) : 0.f;
-                #pragma unroll 1
-                for (int n = 0; n < ntok; n++) {
-                    const float v = mrows[n * kRowLd + lane];
-                    if constexpr (MODE == GEMM_GU) store_tok_block(p.act, grp0 >> 1, tt * N + n, lane, swiglu(v, mrows[(N + n) * kRowLd + lane]));
-                    else store_qkv(p, grp0 * 32 + lane, tt * N + n, __fadd_rn(v, bv));
-                }
-                __syncwarp();
-            } else {
-                // straight from the MMA's layout: lane (g, t4) has rows g + 8 i and tokens 8 j + 2 t4 + cc
+            // straight from the MMA's layout: lane (g, t4) has rows g + 8 i and tokens 8 j + 2 t4 + cc
+            #pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int row = grp0 * 32 + g + 8 * i;
+                const float bv = MODE == GEMM_PLAIN && p.bias && row < p.rows ? __ldg(p.bias + row) : 0.f;
                 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int row = grp0 * 32 + g + 8 * i;
-                    const float bv = MODE == GEMM_PLAIN && p.bias && row < p.rows ? __ldg(p.bias + row) : 0.f;
+                for (int j = 0; j < NT; j++)
                     #pragma unroll
-                    for (int j = 0; j < NT; j++)
-                        #pragma unroll
-                        for (int cc = 0; cc < 2; cc++) {
-                            const int n = 8 * j + 2 * t4 + cc;
-                            if (n >= ntok || row >= p.rows) continue;
-                            if constexpr (MODE == GEMM_PART) __stcg(p.part + ((size_t)sp * p.M + tt * N + n) * p.ldp + row, acc[j][2 * i + cc]);
-                            else p.y[(size_t)(tt * N + n) * p.rows + row] = __double2float_rn(acc[j][2 * i + cc]) + bv;
-                        }
-                }
+                    for (int cc = 0; cc < 2; cc++) {
+                        const int n = 8 * j + 2 * t4 + cc;
+                        if (n >= ntok || row >= p.rows) continue;
+                        if constexpr (MODE == GEMM_PART) __stcg(p.part + ((size_t)sp * p.M + tt * N + n) * p.ldp + row, acc[j][2 * i + cc]);
+                        else p.y[(size_t)(tt * N + n) * p.rows + row] = __double2float_rn(acc[j][2 * i + cc]) + bv;
+                    }
             }
         } else {
             double* fold = reinterpret_cast<double*>(scratch);                           // [warp][token][kFoldLd]
@@ -344,7 +285,7 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
                     for (int q = 1; q < kw; q++) v1 = __dadd_rn(v1, f1[(size_t)q * N * kFoldLd]);
                     store_tok_block(p.act, grp >> 1, m, lane, swiglu(__double2float_rn(v0), __double2float_rn(v1)));
                 } else if constexpr (MODE == GEMM_QKV) {
-                    store_qkv(p, row, m, __fadd_rn(__double2float_rn(v0), __ldg(p.bias + row)));
+                    rope_store(p.rope, row, m, __fadd_rn(__double2float_rn(v0), __ldg(p.bias + row)));
                 } else if constexpr (MODE == GEMM_PART) {
                     if (row < p.rows) __stcg(p.part + ((size_t)sp * p.M + m) * p.ldp + row, v0);
                 } else {
@@ -367,7 +308,7 @@ namespace {
 struct SmemNeed { int ring_bars, fold, x_tile; };
 SmemNeed smem_need(int kb, int NT) {
     switch (kb * 8 + NT) {
-        #define MI_F(kb, nt) case kb * 8 + nt: { using S = TokSmem<kb, nt, GEMM_PLAIN, false>; using F = TokSmem<kb, nt, GEMM_PLAIN, true>; return SmemNeed{S::fixed, F::fixed, S::x_tile}; }
+        #define MI_F(kb, nt) case kb * 8 + nt: { using S = TokSmem<kb, nt, false>; using F = TokSmem<kb, nt, true>; return SmemNeed{S::fixed, F::fixed, S::x_tile}; }
         MI_F(1, 1) MI_F(1, 2) MI_F(1, 3) MI_F(1, 4) MI_F(2, 1) MI_F(2, 2) MI_F(2, 3) MI_F(2, 4)
         MI_F(4, 1) MI_F(4, 2) MI_F(4, 3) MI_F(4, 4) MI_F(8, 1) MI_F(8, 2) MI_F(8, 3) MI_F(8, 4)
         #undef MI_F
@@ -385,36 +326,34 @@ int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* ou
     const int NT = tl.NT, TT = tl.TT, W = tok_warps(NT), N = NT * 8, U = mode == GEMM_GU ? 2 : 1, ntok = std::min(M, N);
     const SmemNeed need = smem_need(w->kb, NT);
     const double c_tile = w->kb * (45.0 + 76.0 * NT) + 100;
-    const double c_tok = mode == GEMM_GU ? 300 : mode == GEMM_QKV ? 160 : 60;             // end of a unit, per token and warp
+    const double c_tok = mode == GEMM_GU ? 640 : mode == GEMM_QKV ? 300 : 60;             // end of a round, per token and warp
     double best = 1e300;
     const int max_ksg = mode == GEMM_PART ? std::min(w->nt, 8) : 1;
     for (int ksg = 1; ksg <= max_ksg; ksg++) {
         const int ntr = (w->nt + ksg - 1) / ksg, cmax = std::max(1, ctx->sm_count / (ksg * TT));
-        for (int kw = 1; kw <= W; kw++) {
-            const int rg = W / kw;
-            if (kw > 1 && (rg % U || W / rg != kw)) continue;                         // pairs stay together; no warps idle by rounding
-            const int fixed = kw > 1 ? need.fold : need.ring_bars + W * N * (mode == GEMM_GU ? 2 : mode == GEMM_QKV ? 1 : 0) * kRowLd * 4;
+        for (int v = 0; v <= W; v++) {                                                // 0: warps alone; else v warps per row group, sums through shared memory
+            const bool fold = v > 0;
+            const int kw = std::max(1, v), rg = W / kw;
+            if (fold ? (v == 1 && U == 1) || rg % U || W / rg != kw : U == 2 || mode == GEMM_QKV) continue;   // pairs stay together; no warps idle by rounding
+            const int fixed = fold ? need.fold : need.ring_bars;
             const int fit = (ctx->smem_optin - kStaticSmem - fixed) / need.x_tile;
             if (fit < 1) continue;
             const int kct = std::min(ntr, fit), nchunk = (ntr + kct - 1) / kct;
+            const int nsets = fold ? (w->groups + rg - 1) / rg : w->groups, C = std::min(nsets, cmax);
+            const int rounds = fold ? (nsets + C - 1) / C : (nsets + C * W - 1) / (C * W), waves = (ksg * TT * C + ctx->sm_count - 1) / ctx->sm_count;
             double cost;
-            int C, rounds;
-            if (kw > 1) {
-                const int nsets = (w->groups + rg - 1) / rg;
-                C = std::min(nsets, cmax); rounds = (nsets + C - 1) / C;
-                const int tiles = (ntr + kw - 1) / kw, sub = (std::min(kw, ntr) * std::min(rg, w->groups) + 3) / 4;
-                cost = rounds * (tiles * std::max(sub * c_tile, c_tile + 200.0) + 900 + 60.0 * NT + ((rg / U) * ntok + W - 1) / W * (c_tok + 20.0 * U * kw) * 1.5);
+            if (fold) {
+                const int tiles = (ntr + kw - 1) / kw, sub = (std::min(kw, ntr) * std::min(rg, w->groups) + 3) / 4;       // warps with tiles per sub-partition
+                const int items = (rg / U * ntok + W - 1) / W;
+                cost = rounds * (tiles * std::max(sub * c_tile, c_tile * 1.2) + 900 + 60.0 * NT + items * (c_tok + 20.0 * U * kw));
             } else {
-                const int units = w->groups / U;
-                C = std::min(units, cmax); rounds = (units + C * W - 1) / (C * W);
-                const int sub = (int)((units + (long long)C * 4 - 1) / ((long long)C * 4));              // units of the busiest sub-partition
-                cost = sub * (ntr * U * c_tile + (mode == GEMM_PLAIN || mode == GEMM_PART ? 250.0 * NT : ntok * c_tok)) + 500;
+                const int sub = (int)((nsets + (long long)C * 4 - 1) / ((long long)C * 4));                                // units of the busiest sub-partition
+                cost = sub * (ntr * c_tile * (sub > 1 ? 1.0 : 1.2) + 250.0 * NT) + 300;
             }
-            const int waves = (ksg * TT * C + ctx->sm_count - 1) / ctx->sm_count;
-            cost = waves * (cost + 600 + (nchunk > 1 ? rounds * nchunk * U * 1500.0 : 0.0)) + (mode == GEMM_PART ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 24.0) : 0.0);
+            cost = waves * (cost + 600 + (nchunk > 1 ? rounds * nchunk * 1500.0 : 0.0)) + (mode == GEMM_PART ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
             if (cost < best) {
                 best = cost;
-                *out = GemmPlan{NT, TT, ksg, kct, C, kw, (size_t)fixed + (size_t)kct * need.x_tile};
+                *out = GemmPlan{NT, TT, ksg, kct, C, kw, fold, (size_t)fixed + (size_t)kct * need.x_tile};
             }
         }
     }
@@ -443,16 +382,17 @@ int launch_mode(mi_ctx* ctx, const GemmPlan& pl, int mode, bool rowmajor, const 
         if constexpr (NT <= 2) return launch_one<KB, NT, GEMM_PLAIN, true, FOLD>(ctx, pl, p, pdl);
         return set_error(ctx, MI_ERR_LIMIT, "gemm: row-major activations of more than 16 tokens");
     }
-    switch (mode) {
-        case GEMM_PLAIN: return launch_one<KB, NT, GEMM_PLAIN, false, FOLD>(ctx, pl, p, pdl);
-        case GEMM_PART: return launch_one<KB, NT, GEMM_PART, false, FOLD>(ctx, pl, p, pdl);
-        case GEMM_QKV: return launch_one<KB, NT, GEMM_QKV, false, FOLD>(ctx, pl, p, pdl);
-        default: return launch_one<KB, NT, GEMM_GU, false, FOLD>(ctx, pl, p, pdl);
+    if (mode == GEMM_PLAIN) return launch_one<KB, NT, GEMM_PLAIN, false, FOLD>(ctx, pl, p, pdl);
+    if (mode == GEMM_PART) return launch_one<KB, NT, GEMM_PART, false, FOLD>(ctx, pl, p, pdl);
+    if constexpr (NT * 8 <= kMaxFusedTok && FOLD) {
+        if (mode == GEMM_QKV) return launch_one<KB, NT, GEMM_QKV, false, FOLD>(ctx, pl, p, pdl);
+        if (mode == GEMM_GU) return launch_one<KB, NT, GEMM_GU, false, FOLD>(ctx, pl, p, pdl);
     }
+    return set_error(ctx, MI_ERR_LIMIT, "gemm: mode %d for %d token groups", mode, NT);
 }
 template <int KB, int NT>
 int launch_fold(mi_ctx* ctx, const GemmPlan& pl, int mode, bool rowmajor, const GemmParams& p, bool pdl) {
-    return pl.kw > 1 ? launch_mode<KB, NT, true>(ctx, pl, mode, rowmajor, p, pdl) : launch_mode<KB, NT, false>(ctx, pl, mode, rowmajor, p, pdl);
+    return pl.fold ? launch_mode<KB, NT, true>(ctx, pl, mode, rowmajor, p, pdl) : launch_mode<KB, NT, false>(ctx, pl, mode, rowmajor, p, pdl);
 }
 template <int KB>
 int launch_nt(mi_ctx* ctx, const GemmPlan& pl, int mode, bool rowmajor, const GemmParams& p, bool pdl) {

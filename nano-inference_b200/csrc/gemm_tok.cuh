@@ -42,9 +42,52 @@ __device__ __forceinline__ void store_tok_block(const TokX& x, int b, int n, int
 enum GemmMode {
     GEMM_PLAIN = 0,    // y[m][row] = fp32(sum) + bias
     GEMM_PART = 1,     // double sums of every K range, part[range][m][row]: the kernel that consumes them adds the ranges
-    GEMM_QKV = 2,      // + bias, rotary embedding; q in natural order, k and v as fp16 into the cache
-    GEMM_GU = 3        // rows come as (gate, up) groups of 32: SwiGLU, q8_0, operand order
+    GEMM_QKV = 2,      // + bias, rotary embedding; q in natural order, k and v as fp16 into the cache          (up to kMaxFusedTok tokens)
+    GEMM_GU = 3        // rows come as (gate, up) groups of 32: SwiGLU, q8_0, operand order                         (up to kMaxFusedTok tokens)
 };
+// Up to this many tokens the rotary embedding and SwiGLU run in the product's epilogue, which saves a launch.  Each of their
+// items (a warp's 32 elements of a token) is a dependent chain of 500 - 900 clocks (a double-precision exponential and
+// division; the position's angles from memory), of which the product's eight warps overlap two per sub-partition: 640
+// clocks per item measured.  With more tokens that is longer than a kernel of their own at full occupancy (gate/up of the 1.5B shape,
+// 64 tokens: 37 us fused, 27 + 4 apart).
+constexpr int kMaxFusedTok = 16;
+
+// Rotary embedding, and where q, k and v of a token go: token n sits at position pos_arr[n] (or *pos0 + n) of cache slab slot_arr[n]
+struct RopeParams {
+    float* q; int nq, HD; __half* kc; __half* vc; int KVD; long long slab_stride; int layer, max_seq;
+    const float* cs; const float* freq; int rows;       // angles of positions below `rows`: cos then sin [HD/2] each; frequencies for the others
+    const int* pos0; const int* pos_arr; const int* slot_arr;
+};
+#ifdef __CUDACC__
+// v: row `row` of the packed QKV vector of token n with the bias added, one row per lane (all lanes of a warp call, rows 32-aligned)
+__device__ __forceinline__ void rope_store(const RopeParams& p, int row, int n, float v) {
+    const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
+    if (row >= p.nq + 2 * p.KVD) return;
+    const int pos = p.pos_arr ? __ldg(p.pos_arr + n) : __ldg(p.pos0) + n;
+    const size_t slab = p.slot_arr ? (size_t)__ldg(p.slot_arr + n) * (size_t)p.slab_stride : 0;
+    const size_t crow = slab + ((size_t)p.layer * p.max_seq + pos) * p.KVD;
+    if (row >= p.nq + p.KVD) { p.vc[crow + (row - p.nq - p.KVD)] = __float2half_rn(v); return; }
+    // q and k rows come pair-adjacent: slots 2i and 2i + 1 of a head are its dims i and i + HD / 2
+    const int within0 = row < p.nq ? row : row - p.nq, head = within0 / p.HD, within = within0 - head * p.HD, i = within >> 1;
+    double c, s;
+    if (pos < p.rows) {
+        c = (double)__ldg(p.cs + (size_t)pos * p.HD + i); s = (double)__ldg(p.cs + (size_t)pos * p.HD + p.HD / 2 + i);
+    } else {
+        const double th = (double)__fmul_rn((float)pos, __ldg(p.freq + i));                // fp32 angle, as src/cpu_infer.cpp:54
+        c = (double)__double2float_rn(cos(th)); s = (double)__double2float_rn(sin(th));
+    }
+    const bool odd = within & 1;
+    const float out = odd ? __double2float_rn(__dadd_rn(__dmul_rn((double)partner, s), __dmul_rn((double)v, c)))
+                          : __double2float_rn(__dsub_rn(__dmul_rn((double)v, c), __dmul_rn((double)partner, s)));
+    const int nat = head * p.HD + i + (odd ? p.HD / 2 : 0);
+    if (row < p.nq) p.q[(size_t)n * p.nq + nat] = out;
+    else p.kc[crow + nat] = __float2half_rn(out);
+}
+__device__ __forceinline__ float swiglu(float gate, float up) {
+    const double gd = (double)gate;
+    return __double2float_rn(__dmul_rn(__ddiv_rn(gd, __dadd_rn(1.0, exp(-gd))), (double)up));
+}
+#endif
 
 struct GemmParams {
     const uint8_t* base; int groups, nt, nb, rows;      // tiled weights
@@ -54,10 +97,7 @@ struct GemmParams {
     const int8_t* xq; const __half* xd;                 // row-major: [M][nb*32], [M][nb]
     const float* bias; float* y;
     double* part; int ldp;                              // part[(range * M + m) * ldp + row]
-    // GEMM_QKV
-    float* q; int nq, HD; __half* kc; __half* vc; int KVD; long long slab_stride; int layer, max_seq;
-    const float* rope_cs; const float* rope_freq; int rope_rows;
-    const int* pos0; const int* pos_arr; const int* slot_arr;
+    RopeParams rope;                                    // GEMM_QKV
     TokX act;                                           // GEMM_GU
     int* err;
 };
@@ -69,7 +109,7 @@ inline TokTiling tok_tiling(int M) {
     return TokTiling{(J + TT - 1) / TT, TT};
 }
 // How a launch over one matrix and M tokens is cut (see plan_gemm_tok).
-struct GemmPlan { int NT, TT, ksg, kct, C, kw; size_t smem; };
+struct GemmPlan { int NT, TT, ksg, kct, C, kw; bool fold; size_t smem; };
 int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* out);
 int launch_gemm_tok(mi_ctx* ctx, const mi_weight* w, const GemmPlan& plan, int mode, bool rowmajor, GemmParams p, bool pdl);
 

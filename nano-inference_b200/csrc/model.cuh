@@ -19,6 +19,7 @@ struct VerifyBufs {
     std::vector<void*> mem;            // the allocations behind the pointers below
     float* X = nullptr;                // residual stream [M][E]
     double* part = nullptr; int ldp = 0;    // sums of a projection per K range [range][M][ldp]
+    float* Y = nullptr;                // fp32 rows of the QKV and gate/up products (more than kMaxFusedTok tokens)
     float* q = nullptr;                // [M][NQ] after bias and RoPE, natural order
     TokX xf{}, attf{}, actf{};         // q8_0 of the normed input, the attention output and SwiGLU, in operand order
     float* att = nullptr;              // [M][NQ]

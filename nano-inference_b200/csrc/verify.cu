@@ -137,6 +137,23 @@ __global__ void __launch_bounds__(DNT, 1) vf_attention(const __grid_constant__ D
     else attention_phase<HD, G, G, false, QNAT>(Q, l, pos, smem);
 }
 
+// The QKV product's epilogue as a kernel of its own (more than kMaxFusedTok tokens): one warp per 32 rows and token of y (bias added)
+__global__ void __launch_bounds__(256) vf_rope(const RopeParams r, const float* y, int rows) {
+    const int n = blockIdx.y, row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32, lane = threadIdx.x & 31;
+    pdl_launch_dependents(); pdl_wait_prior();
+    if (row0 >= rows) return;
+    rope_store(r, row0 + lane, n, __ldcg(y + (size_t)n * rows + row0 + lane));
+}
+
+// The gate/up product's epilogue likewise: one warp per q8_0 block and token; the rows of y come as (gate, up) groups of 32
+__global__ void __launch_bounds__(256) vf_swiglu(const float* y, int FF, TokX act) {
+    const int n = blockIdx.y, b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_launch_dependents(); pdl_wait_prior();
+    if (b >= FF / 32) return;
+    const float* v = y + (size_t)n * 2 * FF + (size_t)b * 64 + lane;
+    store_tok_block(act, b, n, lane, swiglu(__ldcg(v), __ldcg(v + 32)));
+}
+
 // greedy pick of every token, lowest index on ties (src/cpu_infer.cpp:153-154), and its logit margin (greedy logit minus the
 // largest other one) in one reading of the logits.  grid = (slices, tokens): every CTA reduces its slice to {best, row, second};
 // the last CTA of a token to arrive merges the slices and clears the counter for the next pass.  A NaN in row 0 wins like +inf
@@ -236,7 +253,7 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
     int st;
     if ((st = take(&b.X, (size_t)cap * E)) || (st = take(&b.part, (size_t)kMaxRanges * cap * b.ldp)) || (st = take(&b.q, (size_t)cap * NQ)) ||
         (st = take_tok(&b.xf, E, cap)) || (st = take_tok(&b.attf, NQ, cap)) || (st = take_tok(&b.actf, FF, cap)) ||
-        (st = take(&b.att, (size_t)cap * NQ)) || (st = take(&b.logits, (size_t)capl * m->V)) ||
+        (st = take(&b.att, (size_t)cap * NQ)) || (st = take(&b.Y, cap > kMaxFusedTok ? (size_t)cap * std::max(2 * FF, m->qkv_rows) : 0)) || (st = take(&b.logits, (size_t)capl * m->V)) ||
         (st = take(&b.meta, (size_t)3 * cap + 4)) || (st = take(&b.out, (size_t)cap)) || (st = take(&b.margins, (size_t)cap)) ||
         (st = take(&b.attn_part, (size_t)cap * m->NH * m->max_chunks * (m->HD + 2))) || (st = take(&b.attn_cnt, (size_t)cap * m->NH)) ||
         (st = take(&b.pick, (size_t)capl * kPickSlices * 3)) || (st = take(&b.pick_cnt, (size_t)capl)))
@@ -285,10 +302,11 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     const std::vector<LayerPtrs>& lp = m->layer_ptrs;
     const int attn_grid = a.lp_max <= kShortAttnMax ? std::min(m->grid, m->NH) : a.lp_max <= kPerHeadAttnMax ? std::min(m->grid, m->NH * (kPerHeadAttnMax / 256)) : m->grid;
     static const bool pdl = [] { const char* e = getenv("MINFER_VERIFY_PDL"); return !(e && atoi(e) == 0); }();
+    const bool fused = M <= kMaxFusedTok;
     GemmPlan pq, po, pg, pd, pl;
     int st;
-    if ((st = plan_gemm_tok(ctx, &m->views[0], GEMM_QKV, M, &pq)) || (st = plan_gemm_tok(ctx, &m->views[1], GEMM_PART, M, &po)) ||
-        (st = plan_gemm_tok(ctx, &m->views[2], GEMM_GU, M, &pg)) || (st = plan_gemm_tok(ctx, &m->views[3], GEMM_PART, M, &pd)) ||
+    if ((st = plan_gemm_tok(ctx, &m->views[0], fused ? GEMM_QKV : GEMM_PLAIN, M, &pq)) || (st = plan_gemm_tok(ctx, &m->views[1], GEMM_PART, M, &po)) ||
+        (st = plan_gemm_tok(ctx, &m->views[2], fused ? GEMM_GU : GEMM_PLAIN, M, &pg)) || (st = plan_gemm_tok(ctx, &m->views[3], GEMM_PART, M, &pd)) ||
         (st = plan_gemm_tok(ctx, &m->views[4 * L], GEMM_PLAIN, a.last_only ? 1 : M, &pl))) return st;
     const int nt_norm = std::min(1024, (E / 4 + 31) / 32 * 32);
     GemmParams g{};
@@ -302,16 +320,17 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         const mi_weight *wqkv = &m->views[4 * l], *wo = &m->views[4 * l + 1], *wgu = &m->views[4 * l + 2], *wdn = &m->views[4 * l + 3];
         if ((st = norm(l == 0, 0, M, l == 0 ? 0 : pd.ksg, lp[l].attn_norm, xf))) return st;
         GemmParams gq = g;
-        gq.x = xf; gq.bias = lp[l].bqkv; gq.q = b.q; gq.nq = NQ; gq.HD = m->HD; gq.kc = P.kc; gq.vc = P.vc; gq.KVD = m->KVD; gq.slab_stride = a.slab_stride;
-        gq.layer = l; gq.max_seq = a.max_seq; gq.rope_cs = P.rope_cs; gq.rope_freq = P.rope_freq; gq.rope_rows = P.rope_rows;
-        gq.pos0 = pos0; gq.pos_arr = pos_arr; gq.slot_arr = slot_arr;
-        if ((st = launch_gemm_tok(ctx, wqkv, pq, GEMM_QKV, false, gq, pdl))) return st;
+        gq.x = xf; gq.bias = lp[l].bqkv; gq.y = b.Y;
+        gq.rope = RopeParams{b.q, NQ, m->HD, P.kc, P.vc, m->KVD, a.slab_stride, l, a.max_seq, P.rope_cs, P.rope_freq, P.rope_rows, pos0, pos_arr, slot_arr};
+        if ((st = launch_gemm_tok(ctx, wqkv, pq, fused ? GEMM_QKV : GEMM_PLAIN, false, gq, pdl))) return st;
+        if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_rope, dim3(((int)wqkv->rows / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, gq.rope, (const float*)b.Y, (int)wqkv->rows));
         if ((st = launch_attention<true>(ctx, P, m->HD, m->G, attn_grid, M, l, pos0, 0, NQ, pos_arr, slot_arr, a.slab_stride, pdl))) return st;
         GemmParams go = g; go.x = attf; go.part = b.part; go.ldp = b.ldp;
         if ((st = launch_gemm_tok(ctx, wo, po, GEMM_PART, false, go, pdl))) return st;
         if ((st = norm(false, 0, M, po.ksg, lp[l].ffn_norm, xf))) return st;
-        GemmParams gg = g; gg.x = xf; gg.act = actf;
-        if ((st = launch_gemm_tok(ctx, wgu, pg, GEMM_GU, false, gg, pdl))) return st;
+        GemmParams gg = g; gg.x = xf; gg.act = actf; gg.y = b.Y;
+        if ((st = launch_gemm_tok(ctx, wgu, pg, fused ? GEMM_GU : GEMM_PLAIN, false, gg, pdl))) return st;
+        if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_swiglu, dim3((m->FF / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, (const float*)b.Y, m->FF, actf));
         GemmParams gd = g; gd.x = actf; gd.part = b.part; gd.ldp = b.ldp;
         if ((st = launch_gemm_tok(ctx, wdn, pd, GEMM_PART, false, gd, pdl))) return st;
     }
