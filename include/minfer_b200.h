@@ -328,6 +328,14 @@ MI_API int mi_decode_phases(mi_ctx* ctx, mi_model* model, int32_t token, int pos
 MI_API int mi_verify(mi_ctx* ctx, mi_model* model, const int32_t* tokens_host, int M, int pos0,
                      int32_t* out_tokens_host, float* logits_dev, float* elapsed_ms);
 
+/* Prompt processing: n tokens (any number that fits the cache) at positions pos0 .. pos0+n-1, many per pass over the weights;
+ * the same keys, values and prediction, bit for bit, as n single-token steps.  next_token_host (optional) = greedy token after the
+ * last one, which also becomes the model's current token; its margin is the first one mi_verify_margins returns.
+ * Logits of the other tokens are not computed.  Synchronous.  Unsharded models only.  Replaces the chunked prompt
+ * processing of src/cuda_infer.cu:1130-1144. */
+MI_API int mi_prefill(mi_ctx* ctx, mi_model* model, const int32_t* tokens_host, int n, int pos0, int32_t* next_token_host,
+                      float* elapsed_ms);
+
 /* Greedy generation with lossless n-gram speculation: process the prompt (16 tokens per weight
  * pass), then generate n_gen tokens.  Each step drafts up to draftk (0..15; 0 = no speculation)
  * tokens by prompt lookup - the tokens that followed the latest earlier occurrence of the last

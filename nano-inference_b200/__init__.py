@@ -78,6 +78,7 @@ SIGNATURES = {
     "mi_ring_peek": (_i32, [_vp, C.POINTER(_i32), C.POINTER(_vp), C.POINTER(_vp), C.POINTER(_vp)]),
     "mi_decode_run": (_i32, [_vp, _vp, _vp, _i32, _i32, _i32, _vp]),
     "mi_verify": (_i32, [_vp, _vp, _vp, _i32, _i32, _vp, _vp, C.POINTER(C.c_float)]),
+    "mi_prefill": (_i32, [_vp, _vp, _vp, _i32, _i32, _vp, C.POINTER(C.c_float)]),
     "mi_generate_spec": (_i32, [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp]),
     "mi_verify_margins": (_i32, [_vp, _vp, _i32, _vp]),
     "mi_batch_create": (_i32, [_vp, _vp, _i32, _i32, C.POINTER(_vp)]),
@@ -407,7 +408,14 @@ class Model:
                                       "margins": mg[:n_gen]}
 
     def prefill(self, tokens, pos0=0, chunk=16):
-        """Prompt processing through the M-token step, `chunk` tokens per weight pass; returns (token after the last one, ms)."""
+        """Prompt processing; returns (token after the last one, ms).  `chunk`: tokens per weight pass, at least - from 16 on the
+        library takes as many per pass as it can hold, below that exactly `chunk` (the results are the same bits)."""
+        if chunk >= 16 and len(tokens):
+            import numpy as np
+            toks = np.ascontiguousarray(tokens, dtype=np.int32)
+            last, ms = C.c_int32(), C.c_float(0)
+            self.ctx.check(self.ctx.lib.mi_prefill(self.ctx.h, self.h, _ptr(toks), toks.size, pos0, C.addressof(last), C.byref(ms)), "mi_prefill")
+            return last.value, ms.value
         total, last = 0.0, None
         for i in range(0, len(tokens), chunk):
             out, ms = self.verify(tokens[i:i + chunk], pos0 + i)

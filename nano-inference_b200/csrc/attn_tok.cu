@@ -1,0 +1,334 @@
+// Split-KV causal attention with grouped queries for M queries over the fp16 cache: the M-token pass (prompt chunks, drafted
+// tokens, batches) and mi_attn_splitkv.
+//
+// Replaces attn_partial + attn_combine (reference src/cuda_infer.cu:650-702) and mega's attention + combine
+// (src/mega.cu:414-521, 705-741).  Scores are double dot products rounded to fp32 once and scaled by 1/sqrt(HD) in fp32; weights,
+// denominator and weighted sum are double, as everywhere in this library.
+//
+// What bounds it: the FP64 pipe (64 FMAs per clock and SM), 2 HD FMAs per (query, head, position); the cache itself is a few
+// microseconds of HBM time.  So both products run as FP64 MMAs (mma.m8n8k4.f64: the pipe's full rate from one issue slot per
+// 256 FMAs, where the scalar code this replaces spent more slots on fp16 -> double conversions and broadcast loads than on FMAs),
+// and the rows of an MMA are (query, head) pairs that share a kv head: a K or V element is converted once for up to
+// 4 queries x all heads of the group.
+//
+// A CTA has qb queries of one kv head and one chunk of their positions, and walks it 128 positions at a time:
+//   scores   warp = every 8th group of 8 positions; a lane holds HD/4 consecutive dims of one K row (64 bytes straight from
+//            global memory); q waits in shared memory as doubles in the order the MMA reads it;
+//   weights  one warp per row: running maximum, exp, sum; stored in MMA order;
+//   values   warp = HD/8 dims, all positions; a lane's V elements of two 8-dim tiles are one 4-byte load.
+// Two CTAs share an SM, so that one's exponentials run beside the other's MMAs.  With several chunks per range the CTAs leave
+// {sum, maximum, denominator} per row and attn_tok_merge folds them against their common maximum; with one chunk the CTA
+// finishes.  The number of chunks comes from the host and only sets how a range is cut, so a captured launch stays valid for
+// any position.
+#include "attn_tok.cuh"
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+
+namespace mi {
+
+constexpr int kAT = 256, kAW = kAT / 32;          // threads, warps
+constexpr int kSub = 128;                         // positions per step
+constexpr int kScLd = kSub + 4;                   // floats per row of scores
+constexpr int kMaxQB = 4;                         // queries per CTA
+
+__host__ __device__ constexpr int attn_row_tiles(int G, int QB) { return (G * QB + 7) / 8; }
+template <int HD, int RT> constexpr size_t attn_tok_smem() {
+    return (size_t)RT * 8 * HD * 8 + (size_t)RT * 8 * kSub * 8 + (size_t)RT * 8 * kScLd * 4 + (size_t)RT * 8 * 3 * 8;
+}
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+__device__ __forceinline__ double half_lo(unsigned w) { return (double)__half2float(__ushort_as_half((unsigned short)(w & 0xffffu))); }
+__device__ __forceinline__ double half_hi(unsigned w) { return (double)__half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+
+// Four consecutive dims e .. e+3 of one (token, head): fp32 out, and q8_0 over the eight threads that share a 32-dim block
+__device__ __forceinline__ void attn_emit(const AttnParams& p, int token, int e, float4 v) {
+    *reinterpret_cast<float4*>(p.out + (size_t)token * p.NH * p.HD + e) = v;
+    if (!p.x.q) return;                            // uniform
+    float a = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+    const unsigned mask = 0xffu << (threadIdx.x & 24);               // a block's eight threads, all here or none
+    a = fmaxf(a, __shfl_xor_sync(mask, a, 1));
+    a = fmaxf(a, __shfl_xor_sync(mask, a, 2));
+    a = fmaxf(a, __shfl_xor_sync(mask, a, 4));
+    const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
+    const unsigned q = ((unsigned)__float2int_rn(__fmul_rn(v.x, inv)) & 0xffu) | (((unsigned)__float2int_rn(__fmul_rn(v.y, inv)) & 0xffu) << 8) |
+                       (((unsigned)__float2int_rn(__fmul_rn(v.z, inv)) & 0xffu) << 16) | ((unsigned)__float2int_rn(__fmul_rn(v.w, inv)) << 24);
+    p.x.q[tok_word(p.x.J, e >> 5, token, e & 31)] = q;
+    if ((e & 31) == 0) p.x.d[tok_scale(p.x.J, e >> 5, token)] = tok_scale_value(__float2half_rn(__fdiv_rn(a, 127.f)));
+}
+
+template <int HD, int G, int QB>
+__global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant__ AttnParams p) {
+    constexpr int RT = attn_row_tiles(G, QB), R = RT * 8, ROWS = G * QB;
+    constexpr int DPL = HD / 4;                     // dims per lane in the score product
+    constexpr int NTW = HD >= 64 ? HD / 64 : 1;     // 8-dim tiles per warp in the value product
+    constexpr int VW = HD / 8 / NTW;                // warps that have some
+    extern __shared__ __align__(128) uint8_t smem[];
+    double* qs = reinterpret_cast<double*>(smem);                    // [step < DPL][row tile][lane]
+    double* wt = qs + R * HD;                                        // [kSub / 4][row tile][lane]
+    float* sc = reinterpret_cast<float*>(wt + R * kSub);             // [R][kScLd]
+    double* rm = reinterpret_cast<double*>(sc + R * kScLd);          // [R] running maximum
+    double* rl = rm + R;                                             // [R] denominator
+    double* rf = rl + R;                                             // [R] rescale factor of this step
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int nqb = (p.M + QB - 1) / QB;
+    // later queries have longer ranges: they go first
+    const int ch = (int)(blockIdx.x % p.nch), rest = (int)(blockIdx.x / p.nch), kvh = rest % p.NKV, q0 = (nqb - 1 - rest / p.NKV) * QB;
+    const int nq = min(QB, p.M - q0);
+    pdl_launch_dependents();
+    pdl_wait_prior();
+    const int posq0 = p.pos_arr ? __ldg(p.pos_arr + q0) : (p.pos0 ? __ldg(p.pos0) : p.pos0_val) + q0;      // position of query q0; the CTA's others follow (QB > 1: one sequence)
+    const size_t base = (p.slot_arr ? (size_t)__ldg(p.slot_arr + q0) * (size_t)p.slab_stride : 0) + (size_t)p.layer * p.max_seq * p.KVD + (size_t)kvh * HD;
+    const __half* kb = p.kc + base; const __half* vb = p.vc + base;
+    const int Lp = posq0 + nq;                      // positions the last query sees
+    const int p0 = (int)((long long)Lp * ch / p.nch), p1 = (int)((long long)Lp * (ch + 1) / p.nch);
+    // q into the order the MMA reads it: step s, row tile r, lane (row, t) holds dim DPL t + s of row 8 r + row
+    for (int i = tid; i < R * HD; i += kAT) {
+        const int d = i % HD, row = i / HD, qi = row / G, h = row - qi * G, tt = d / DPL, s = d - tt * DPL;
+        const float v = row < ROWS && qi < nq ? __ldcg(p.q + (size_t)(q0 + qi) * p.NH * HD + (size_t)(kvh * G + h) * HD + d) : 0.f;
+        qs[(s * RT + (row >> 3)) * 32 + (row & 7) * 4 + tt] = (double)v;
+    }
+    for (int i = tid; i < R; i += kAT) { rm[i] = -INFINITY; rl[i] = 0.0; }
+    const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
+    double o[RT][NTW][2];
+    #pragma unroll
+    for (int r = 0; r < RT; r++)
+        #pragma unroll
+        for (int n = 0; n < NTW; n++) o[r][n][0] = o[r][n][1] = 0.0;
+    __syncthreads();
+
+    for (int b0 = p0; b0 < p1; b0 += kSub) {
+        const int np = min(kSub, p1 - b0);
+        // ---- scores
+        #pragma unroll 1
+        for (int t = warp; t * 8 < np; t += kAW) {
+            const __half* kr = kb + (size_t)(b0 + min(t * 8 + g, np - 1)) * p.KVD + t4 * DPL;
+            uint4 kw[DPL / 8];
+            #pragma unroll
+            for (int i = 0; i < DPL / 8; i++) kw[i] = __ldcg(reinterpret_cast<const uint4*>(kr) + i);
+            double c[RT][2][2];                     // two chains per row tile
+            #pragma unroll
+            for (int r = 0; r < RT; r++) c[r][0][0] = c[r][0][1] = c[r][1][0] = c[r][1][1] = 0.0;
+            #pragma unroll
+            for (int i = 0; i < DPL / 8; i++) {
+                const unsigned w[4] = {kw[i].x, kw[i].y, kw[i].z, kw[i].w};
+                #pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const double k0 = half_lo(w[e]), k1 = half_hi(w[e]);
+                    const double* a = qs + (size_t)((i * 8 + e * 2) * RT) * 32 + lane;
+                    #pragma unroll
+                    for (int r = 0; r < RT; r++) { dmma(c[r][0], a[r * 32], k0); dmma(c[r][1], a[(RT + r) * 32], k1); }
+                }
+            }
+            #pragma unroll
+            for (int r = 0; r < RT; r++)
+                #pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int row = 8 * r + g, pp = t * 8 + 2 * t4 + e, qi = row / G;
+                    const float s = __fmul_rn(__double2float_rn(__dadd_rn(c[r][0][e], c[r][1][e])), inv);
+                    sc[row * kScLd + pp] = b0 + pp < p1 && b0 + pp <= posq0 + qi ? s : -INFINITY;
+                }
+        }
+        __syncthreads();
+        // ---- weights: one warp per row
+        #pragma unroll 1
+        for (int row = warp; row < R; row += kAW) {
+            float s[kSub / 32], m = -INFINITY;
+            #pragma unroll
+            for (int i = 0; i < kSub / 32; i++) { s[i] = lane + 32 * i < np ? sc[row * kScLd + lane + 32 * i] : -INFINITY; m = fmaxf(m, s[i]); }
+            #pragma unroll
+            for (int q = 16; q; q >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, q));
+            const double mo = rm[row], mn = fmax(mo, (double)m);
+            double l = 0.0;
+            #pragma unroll
+            for (int i = 0; i < kSub / 32; i++) {
+                const double w = s[i] == -INFINITY ? 0.0 : exp((double)s[i] - mn);
+                const int pp = lane + 32 * i;
+                wt[((pp >> 2) * RT + (row >> 3)) * 32 + (row & 7) * 4 + (pp & 3)] = w;
+                l = __dadd_rn(l, w);
+            }
+            #pragma unroll
+            for (int q = 16; q; q >>= 1) l = __dadd_rn(l, __shfl_xor_sync(0xffffffffu, l, q));
+            if (lane == 0) {
+                const double f = mo == mn ? 1.0 : mo == -INFINITY ? 0.0 : exp(mo - mn);        // 1 while the maximum stands (and while there is none)
+                rf[row] = f; rm[row] = mn; rl[row] = __fma_rn(rl[row], f, l);
+            }
+        }
+        __syncthreads();
+        // ---- values
+        if (warp < VW) {
+            if (b0 > p0) {
+                #pragma unroll
+                for (int r = 0; r < RT; r++) {
+                    const double f = rf[8 * r + g];
+                    #pragma unroll
+                    for (int n = 0; n < NTW; n++) { o[r][n][0] = __dmul_rn(o[r][n][0], f); o[r][n][1] = __dmul_rn(o[r][n][1], f); }
+                }
+            }
+            constexpr int PF = 8;                   // steps of four positions whose V elements are requested together
+            const __half* vr = vb + warp * (8 * NTW) + g * NTW;
+            #pragma unroll 1
+            for (int s0 = 0; s0 * 4 < np; s0 += PF) {
+                unsigned vw[PF];
+                #pragma unroll
+                for (int u = 0; u < PF; u++) {
+                    const __half* v = vr + (size_t)(b0 + min((s0 + u) * 4 + t4, np - 1)) * p.KVD;
+                    if constexpr (NTW == 2) vw[u] = __ldcg(reinterpret_cast<const unsigned*>(v));
+                    else vw[u] = __ldcg(reinterpret_cast<const unsigned short*>(v));
+                }
+                #pragma unroll
+                for (int u = 0; u < PF; u++) {
+                    if ((s0 + u) * 4 >= np) break;  // warp-uniform
+                    const double* a = wt + (size_t)((s0 + u) * RT) * 32 + lane;
+                    const double v0 = half_lo(vw[u]), v1 = NTW == 2 ? half_hi(vw[u]) : 0.0;
+                    #pragma unroll
+                    for (int r = 0; r < RT; r++) {
+                        const double w = a[r * 32];
+                        dmma(o[r][0], w, v0);
+                        if constexpr (NTW == 2) dmma(o[r][NTW - 1], w, v1);
+                    }
+                }
+            }
+        }
+        __syncthreads();                            // scores and weights may be written again
+    }
+    // ---- the chunk's rows
+    if (p.nch > 1) {
+        if (warp < VW) {
+            #pragma unroll
+            for (int r = 0; r < RT; r++) {
+                const int row = 8 * r + g, qi = row / G, h = row - qi * G;
+                if (row >= ROWS || qi >= nq) continue;
+                double* gp = p.part + (((size_t)(q0 + qi) * p.NH + kvh * G + h) * p.nch + ch) * (HD + 2);
+                #pragma unroll
+                for (int n = 0; n < NTW; n++)
+                    #pragma unroll
+                    for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + n, o[r][n][e]);
+            }
+        }
+        for (int row = tid; row < ROWS; row += kAT) {
+            const int qi = row / G, h = row - qi * G;
+            if (qi >= nq) continue;
+            double* gp = p.part + (((size_t)(q0 + qi) * p.NH + kvh * G + h) * p.nch + ch) * (HD + 2) + HD;
+            __stcg(gp, rm[row]); __stcg(gp + 1, rl[row]);
+        }
+        return;
+    }
+    float* of = reinterpret_cast<float*>(qs);       // [row][HD] fp32 (q is not needed any more)
+    if (warp < VW) {
+        #pragma unroll
+        for (int r = 0; r < RT; r++) {
+            const double l = rl[8 * r + g];
+            #pragma unroll
+            for (int n = 0; n < NTW; n++)
+                #pragma unroll
+                for (int e = 0; e < 2; e++) of[(8 * r + g) * HD + warp * (8 * NTW) + (2 * t4 + e) * NTW + n] = __double2float_rn(__ddiv_rn(o[r][n][e], l));
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < nq * G * (HD / 4); i += kAT) {              // a multiple of 8 items: the threads of a 32-dim block stay together
+        const int row = i / (HD / 4), d = (i - row * (HD / 4)) * 4, qi = row / G, h = row - qi * G;
+        attn_emit(p, q0 + qi, (kvh * G + h) * HD + d, *reinterpret_cast<const float4*>(of + row * HD + d));
+    }
+}
+
+// Fold the chunks of one (query, kv head) against their common maximum.  Thread = four dims of one head.
+template <int HD>
+__global__ void __launch_bounds__(kAT) attn_tok_merge(const __grid_constant__ AttnParams p, int G) {
+    extern __shared__ __align__(16) double fs[];                     // [G][nch] rescale factors, then [G] denominators
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, token = blockIdx.y, kvh = blockIdx.x, nch = p.nch;
+    pdl_launch_dependents();
+    pdl_wait_prior();
+    const double* gp = p.part + ((size_t)token * p.NH + (size_t)kvh * G) * nch * (HD + 2);
+    double* den = fs + G * nch;
+    for (int h = warp; h < G; h += kAW) {
+        double m = -INFINITY, l = 0.0;
+        for (int c = lane; c < nch; c += 32) m = fmax(m, __ldcg(gp + ((size_t)h * nch + c) * (HD + 2) + HD));
+        #pragma unroll
+        for (int q = 16; q; q >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, q));
+        for (int c = lane; c < nch; c += 32) {
+            const double* s = gp + ((size_t)h * nch + c) * (HD + 2) + HD;
+            const double mc = __ldcg(s), f = mc == -INFINITY ? 0.0 : exp(mc - m);
+            fs[h * nch + c] = f;
+            l = __fma_rn(__ldcg(s + 1), f, l);
+        }
+        #pragma unroll
+        for (int q = 16; q; q >>= 1) l = __dadd_rn(l, __shfl_xor_sync(0xffffffffu, l, q));
+        if (lane == 0) den[h] = l;
+    }
+    __syncthreads();
+    for (int i = tid; i < G * (HD / 4); i += kAT) {
+        const int h = i / (HD / 4), d = (i - h * (HD / 4)) * 4;
+        const double* s = gp + (size_t)h * nch * (HD + 2) + d;
+        double o[4] = {0.0, 0.0, 0.0, 0.0};
+        constexpr int U = 8;
+        for (int c0 = 0; c0 < nch; c0 += U) {
+            double2 a[U], b[U];
+            #pragma unroll
+            for (int u = 0; u < U; u++) {
+                const double2* sp = reinterpret_cast<const double2*>(s + (size_t)min(c0 + u, nch - 1) * (HD + 2));
+                a[u] = __ldcg(sp); b[u] = __ldcg(sp + 1);
+            }
+            #pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (c0 + u < nch) {
+                    const double f = fs[h * nch + c0 + u];
+                    o[0] = __fma_rn(a[u].x, f, o[0]); o[1] = __fma_rn(a[u].y, f, o[1]); o[2] = __fma_rn(b[u].x, f, o[2]); o[3] = __fma_rn(b[u].y, f, o[3]);
+                }
+            }
+        }
+        const double l = den[h];
+        attn_emit(p, token, (kvh * G + h) * HD + d, make_float4(__double2float_rn(__ddiv_rn(o[0], l)), __double2float_rn(__ddiv_rn(o[1], l)),
+                                                                __double2float_rn(__ddiv_rn(o[2], l)), __double2float_rn(__ddiv_rn(o[3], l))));
+    }
+}
+
+// ---- host side -----------------------------------------------------------------------------------------------------
+
+// Queries per CTA: four where the ranges are long (their work is FP64 time, and an MMA's rows should be full: 4 x 6 heads are three
+// whole row tiles, one query's 6 heads fill three quarters of one), one where they are short or belong to different sequences
+// (the work is latency, and more CTAs share it).  Chunks: one up to 320 positions (a CTA walks them in the time a second
+// launch takes); beyond, enough that two CTAs per SM have work, and none shorter than 64 positions.
+AttnPlan plan_attn_tok(const mi_ctx* ctx, int NH, int NKV, int HD, int M, int lp_max, bool ragged) {
+    AttnPlan a;
+    a.qb = !ragged && M > 1 && (long long)M * lp_max >= 16384 ? kMaxQB : 1;
+    const int units = NKV * ((M + a.qb - 1) / a.qb);
+    a.nch = lp_max <= 320 ? 1 : std::max(1, std::min((lp_max + 63) / 64, 2 * ctx->sm_count / units));
+    a.part_doubles = a.nch > 1 ? (size_t)M * NH * a.nch * (HD + 2) : 0;
+    return a;
+}
+
+// units x chunks is at most two CTAs per SM, a unit at most kMaxQB queries of one group
+size_t attn_part_max(const mi_ctx* ctx, int NH, int NKV, int HD) { return (size_t)kMaxQB * (NH / NKV) * 2 * ctx->sm_count * (HD + 2); }
+
+namespace {
+template <int HD, int G, int QB>
+int launch_qb(mi_ctx* ctx, const AttnParams& p, bool pdl) {
+    constexpr size_t smem = attn_tok_smem<HD, attn_row_tiles(G, QB)>();
+    auto kern = attn_tok_kernel<HD, G, QB>;
+    static std::mutex mu;
+    static std::atomic<unsigned> raised{0};                   // bit per device: opt-in shared memory set
+    if (!(raised.load(std::memory_order_acquire) >> (ctx->device & 31) & 1u)) {
+        std::lock_guard<std::mutex> hold(mu);
+        MI_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        raised.fetch_or(1u << (ctx->device & 31), std::memory_order_release);
+    }
+    const int units = p.NKV * ((p.M + QB - 1) / QB);
+    MI_CUDA(ctx, launch_k(pdl, kern, dim3(units * p.nch), dim3(kAT), smem, ctx->stream, p));
+    if (p.nch > 1) MI_CUDA(ctx, launch_k(pdl, attn_tok_merge<HD>, dim3(p.NKV, p.M), dim3(kAT), (size_t)(G * p.nch + G) * 8, ctx->stream, p, G));
+    return MI_OK;
+}
+}  // namespace
+
+int launch_attn_tok(mi_ctx* ctx, AttnParams p, const AttnPlan& plan, bool pdl) {
+    p.qb = plan.qb; p.nch = plan.nch;
+    const int G = p.NH / p.NKV;
+    #define MI_A(hd, g) if (p.HD == hd && G == g) return plan.qb == 1 ? launch_qb<hd, g, 1>(ctx, p, pdl) : launch_qb<hd, g, kMaxQB>(ctx, p, pdl);
+    MI_A(32, 2) MI_A(64, 2) MI_A(64, 7) MI_A(128, 6) MI_A(128, 8)
+    #undef MI_A
+    return set_error(ctx, MI_ERR_UNSUPPORTED, "attention: head_dim %d with %d query heads per kv head is not instantiated", p.HD, G);
+}
+
+}  // namespace mi

@@ -806,10 +806,6 @@ extern "C" int mi_decode_phases(mi_ctx* ctx, mi_model* m, int32_t token, int pos
 namespace {
 __global__ void set_token_kernel(int* dst, int tok) { *dst = tok; }
 __global__ void add_int_kernel(int* dst, int delta) { *dst += delta; }
-__global__ void reset_counters_kernel(unsigned* a, int na, unsigned* b, int nb) {
-    for (int i = threadIdx.x; i < na; i += blockDim.x) a[i] = 0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) b[i] = 0;
-}
 // gathered: [world] x {float best value, int token}; the largest value wins, the lowest token id on ties
 // (the rule of src/cpu_infer.cpp:153-154 applied across the GPUs' row ranges)
 __global__ void tp_pick_kernel(const float* gathered, int world, float* best_val, int* cur_token) {
@@ -936,8 +932,7 @@ static int launch_phases(mi_ctx* ctx, mi_model* m, int pos, int phase_begin, int
 int mi::reset_after_error(mi_ctx* ctx, mi_model* m) {
     if (m->errors_seen == ctx->errors_reported) return MI_OK;
     m->errors_seen = ctx->errors_reported;
-    reset_counters_kernel<<<1, 256, 0, ctx->stream>>>(m->P.attn_cnt, m->NH, m->vb.attn_cnt, m->vb.cap * m->NH);
-    MI_CUDA(ctx, cudaGetLastError());
+    MI_CUDA(ctx, cudaMemsetAsync(m->P.attn_cnt, 0, m->NH * sizeof(unsigned), ctx->stream));
     if (m->vb.pick_cnt) MI_CUDA(ctx, cudaMemsetAsync(m->vb.pick_cnt, 0, m->vb.cap_logits * sizeof(unsigned), ctx->stream));
     return MI_OK;
 }

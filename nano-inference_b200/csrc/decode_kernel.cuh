@@ -61,7 +61,7 @@
 // exact and the fp32 value cannot depend on their order; beyond that it has been
 // observed, not proved.  Each token is processed exactly as if it were alone.
 #pragma once
-#include "gemm_tok.cuh"
+#include "gemv_core.cuh"
 #ifndef MI_ATT_FN
 #define MI_ATT_FN static __device__ __noinline__
 #endif
@@ -200,10 +200,7 @@ struct DecodeParams {
     unsigned* epoch_dev;
     unsigned long long wait_ns;      // time budget of every device-side wait
     int drop_phase;                  // test hook: the producers of this phase publish nothing (-1: none), so that its consumers' waits run out
-    // plain (untagged) vectors: inputs / outputs of the attention code when it runs as a kernel of its own (M-token step)
-    float* qkv_out;
-    float* att;                      // merged attention output, fp32 (also written by the decode loop, for inspection)
-    TokX att_x; int att_token;       // the same as q8_0 in operand order, as this token (M-token step; null elsewhere)
+    float* att;                      // merged attention output, fp32, for inspection
     __half* kc; __half* vc; int max_seq;       // [L][max_seq][KVD]
     double* attn_part; unsigned* attn_cnt; int max_chunks;  // [NH][max_chunks][HD+2], [NKV]
     float* out_margins;              // optional [n_steps]: top-1 minus top-2 logit of every step
@@ -823,14 +820,11 @@ inline bool lean_shape_ok(int E, int FF, int NQ) {
 // G = query heads handled by one CTA: all heads of a kv head (one K/V read serves the group: long
 // contexts, bandwidth matters) or a single head (short contexts: K/V come from L2 anyway, and six
 // times as many CTAs each carry a sixth of the serial work).  GQ = query heads per kv head.
-// STORE_KV: the CTA whose range ends at the new position writes that position's K and V from the packed QKV
-// vector (the decode loop); callers that stored them beforehand pass false.  QNAT: q is in natural dimension
-// order (the stand-alone entry point) instead of the packed pair-adjacent order of the fused QKV projection.
-// TG: inputs (q, and k / v of the new position) and the q8_0 output travel as tagged words (the decode loop); otherwise they
-// are plain arrays (the attention kernel of the M-token step).  Returns false if a wait gave up (CTA-uniform).
-template <int HD, int G, int GQ, bool STORE_KV = true, bool QNAT = false, bool TG = false>
+// Inputs (q, and k / v of the new position) and the q8_0 output travel as tagged words; the CTA whose range ends at the new
+// position also writes that position's K and V into the cache.  Returns false if a wait gave up (CTA-uniform).
+template <int HD, int G, int GQ>
 __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, int pos, uint8_t* stage,
-                                                unsigned tag_in = 0, const Pub pub = Pub()) {
+                                                unsigned tag_in, const Pub pub) {
     constexpr int DPW = HD / 32;           // dims per lane in pass 2 and while folding (dim = lane + 32*i)
     constexpr int SW = HD + 2;             // doubles per (head) state: o[HD], m, l
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -844,50 +838,34 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
     double* wts = scr + DNW * G * SW;                                       // [warp][32][G]
     constexpr int LPP = 8, DPL = HD / LPP, QSTR = DPL + 2;                   // lanes per position in pass 1, dims per lane, padded stride
     double* qs = wts + DNW * 32 * G;                                        // [G][LPP][QSTR]: 16-byte skew per lane, conflict-free
-    const bool store_kv = STORE_KV && ch == nch - 1;     // this CTA's range ends at the new position: it stores that position's K and V (fp16); CTAs that share a kv head store the same bits
-    if constexpr (TG) {
-        // q of this CTA's G query heads, and k / v of the new position, from the tagged QKV vector (packed order: dim d of a
-        // head sits at 2d (d < HD/2) or 2(d-HD/2)+1); one poll for all of a thread's words
-        constexpr int QN = (G * HD + DNT - 1) / DNT;
-        const int nq = P.NH * HD;
-        unsigned qw[QN + 2], valid = 0;
-        #pragma unroll
-        for (int k = 0; k < QN; k++) if (tid + k * DNT < G * HD) valid |= 1u << k;
-        if (store_kv && tid < HD) valid |= 3u << QN;
-        const unsigned long long* qv = P.xw + P.xo.qkv;
-        const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;           // packed slot of dim `tid` (threads below HD)
-        bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
-            if (k < QN) {
-                const int i = tid + k * DNT, j = i / HD, d = i % HD, pk = d < HD / 2 ? 2 * d : 2 * (d - HD / 2) + 1;
-                return qv + (size_t)(h0 + j) * HD + pk;
-            }
-            return k == QN ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
-        }, qw);
-        #pragma unroll
-        for (int k = 0; k < QN; k++) {
-            const int i = tid + k * DNT;
-            if (i < G * HD) { const int j = i / HD, d = i % HD; qs[(j * LPP + d / DPL) * QSTR + d % DPL] = (double)__uint_as_float(qw[k]); }
+    const bool store_kv = ch == nch - 1;     // this CTA's range ends at the new position: it stores that position's K and V (fp16); CTAs that share a kv head store the same bits
+    // q of this CTA's G query heads, and k / v of the new position, from the tagged QKV vector (packed order: dim d of a
+    // head sits at 2d (d < HD/2) or 2(d-HD/2)+1); one poll for all of a thread's words
+    constexpr int QN = (G * HD + DNT - 1) / DNT;
+    const int nq = P.NH * HD;
+    unsigned qw[QN + 2], valid = 0;
+    #pragma unroll
+    for (int k = 0; k < QN; k++) if (tid + k * DNT < G * HD) valid |= 1u << k;
+    if (store_kv && tid < HD) valid |= 3u << QN;
+    const unsigned long long* qv = P.xw + P.xo.qkv;
+    const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;           // packed slot of dim `tid` (threads below HD)
+    bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
+        if (k < QN) {
+            const int i = tid + k * DNT, j = i / HD, d = i % HD, pk = d < HD / 2 ? 2 * d : 2 * (d - HD / 2) + 1;
+            return qv + (size_t)(h0 + j) * HD + pk;
         }
-        if (store_kv && tid < HD) {
-            P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[QN]));
-            P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[QN + 1]));
-        }
-        if (!__syncthreads_and(okq ? 1 : 0)) return false;
-    } else {
-        for (int i = tid; i < G * HD; i += DNT) {
-            const int j = i / HD, d = i % HD, pk = QNAT ? d : (d < HD / 2 ? 2 * d : 2 * (d - HD / 2) + 1);
-            qs[(j * LPP + d / DPL) * QSTR + d % DPL] = (double)__ldcg(P.qkv_out + (size_t)(h0 + j) * HD + pk);
-        }
-        if (store_kv) {
-            const int nq = P.NH * HD;
-            for (int d = tid; d < HD; d += DNT) {
-                const int pk = d < HD / 2 ? 2 * d : 2 * (d - HD / 2) + 1;
-                P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + d] = __float2half_rn(__ldcg(P.qkv_out + nq + (size_t)kvh * HD + pk));
-                P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + d] = __float2half_rn(__ldcg(P.qkv_out + nq + P.KVD + (size_t)kvh * HD + d));
-            }
-        }
-        __syncthreads();
+        return k == QN ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
+    }, qw);
+    #pragma unroll
+    for (int k = 0; k < QN; k++) {
+        const int i = tid + k * DNT;
+        if (i < G * HD) { const int j = i / HD, d = i % HD; qs[(j * LPP + d / DPL) * QSTR + d % DPL] = (double)__uint_as_float(qw[k]); }
     }
+    if (store_kv && tid < HD) {
+        P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[QN]));
+        P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[QN + 1]));
+    }
+    if (!__syncthreads_and(okq ? 1 : 0)) return false;
     prof_mark(P, 14);
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
     const int n = p1 - p0, a0 = p0 + (int)((long long)n * warp / DNW), a1 = p0 + (int)((long long)n * (warp + 1) / DNW);
@@ -1030,7 +1008,7 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
     }
     // the new position's K / V rows (plain stores above) are performed before anything this CTA publishes from here on:
     // a CTA that reads them in a later step has consumed words that descend from this CTA's output
-    if (TG && store_kv && tid < HD) __threadfence();
+    if (store_kv && tid < HD) __threadfence();
     __syncthreads();
     // warp j folds head j's DNW warp states against their common maximum and publishes the chunk partial
     if (warp < G) {
@@ -1058,13 +1036,9 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
                 const float v = __double2float_rn(__ddiv_rn(ob[i], ll));
                 const int e = head * HD + 32 * i + lane;
                 __stcg(P.att + e, v);
-                if constexpr (TG) {
-                    __half dq; int sq;
-                    const int qv8 = quant_block_warp2(v, dq, sq);
-                    publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
-                } else {
-                    if (P.att_x.q) store_tok_block(P.att_x, e >> 5, P.att_token, lane, v);
-                }
+                __half dq; int sq;
+                const int qv8 = quant_block_warp2(v, dq, sq);
+                publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
             }
         } else {
             double* gp = P.attn_part + ((size_t)head * P.max_chunks + ch) * SW;
@@ -1129,13 +1103,9 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
             const float v = __double2float_rn(__ddiv_rn(ob[i], ll));
             const int e = head * HD + 32 * i + lane;
             __stcg(P.att + e, v);
-            if constexpr (TG) {
-                __half dq; int sq;
-                const int qv8 = quant_block_warp2(v, dq, sq);
-                publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
-            } else {
-                if (P.att_x.q) store_tok_block(P.att_x, e >> 5, P.att_token, lane, v);
-            }
+            __half dq; int sq;
+            const int qv8 = quant_block_warp2(v, dq, sq);
+            publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
         }
     }
     return true;
@@ -1151,10 +1121,10 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
 //   pass 2  warp w, same positions: lane = dims {lane + 32 i}; o += w[p] * V[p], l += w[p] in position order;
 //   finish  warp i (i < HD/32) adds the eight warps' partial sums in warp order, divides, rounds to fp32, quantizes its
 //           32-dim block to q8_0 and publishes it.
-// Same interface and template flags as attention_phase.
-template <int HD, int GQ, bool STORE_KV = true, bool QNAT = false, bool TG = false>
+// Same interface as attention_phase.
+template <int HD, int GQ>
 MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* stage,
-                                                unsigned tag_in = 0, const Pub pub = Pub()) {
+                                                unsigned tag_in, const Pub pub) {
     constexpr int DPW = HD / 32;
     constexpr int LPP = 8, DPL = HD / LPP, QSTR = DPL + 2;                 // lanes per position in pass 1, dims per lane, padded stride
     constexpr int KV4 = DPL * 2 / 16 > 0 ? DPL * 2 / 16 : 1;              // 16-byte loads per lane and position
@@ -1166,35 +1136,21 @@ MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* s
     double* ow = wt + 256;                                                 // [DNW][HD] partial outputs
     double* lw = ow + DNW * HD;                                            // [DNW] partial denominators
     float* sc = reinterpret_cast<float*>(lw + DNW);                        // [256] scores
-    if constexpr (TG) {
-        const int nq = P.NH * HD;
-        unsigned qw[3], valid = 0;
-        if (tid < HD) valid = STORE_KV ? 7u : 1u;
-        const unsigned long long* qv = P.xw + P.xo.qkv;
-        const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;    // packed slot of dim `tid`
-        const bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
-            return k == 0 ? qv + (size_t)head * HD + dk : k == 1 ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
-        }, qw);
-        if (tid < HD) {
-            qs[(tid / DPL) * QSTR + tid % DPL] = (double)__uint_as_float(qw[0]);
-            if (STORE_KV) {                                               // CTAs that share a kv head store the same bits
-                P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[1]));
-                P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[2]));
-            }
-        }
-        if (!__syncthreads_and(okq ? 1 : 0)) return false;
-    } else {
-        if (tid < HD) {
-            const int pk = QNAT ? tid : (tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1);
-            qs[(tid / DPL) * QSTR + tid % DPL] = (double)__ldcg(P.qkv_out + (size_t)head * HD + pk);
-            if (STORE_KV) {
-                const int nq = P.NH * HD, pkk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;
-                P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__ldcg(P.qkv_out + nq + (size_t)kvh * HD + pkk));
-                P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__ldcg(P.qkv_out + nq + P.KVD + (size_t)kvh * HD + tid));
-            }
-        }
-        __syncthreads();
+    const int nq = P.NH * HD;
+    unsigned qw[3], valid = 0;
+    if (tid < HD) valid = 7u;
+    const unsigned long long* qv = P.xw + P.xo.qkv;
+    const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;    // packed slot of dim `tid`
+    const bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
+        return k == 0 ? qv + (size_t)head * HD + dk : k == 1 ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
+    }, qw);
+    if (tid < HD) {
+        qs[(tid / DPL) * QSTR + tid % DPL] = (double)__uint_as_float(qw[0]);
+        // CTAs that share a kv head store the same bits
+        P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[1]));
+        P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[2]));
     }
+    if (!__syncthreads_and(okq ? 1 : 0)) return false;
     prof_mark(P, 14);
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
     const int a0 = (int)((long long)Lp * warp / DNW), a1 = (int)((long long)Lp * (warp + 1) / DNW);      // at most 32 positions
@@ -1311,7 +1267,7 @@ MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* s
     if (lane == 0) lw[warp] = ls;
     prof_mark(P, 31);
     // the new position's K / V rows (plain stores above) are performed before anything this CTA publishes
-    if (TG && STORE_KV && tid < HD) __threadfence();
+    if (tid < HD) __threadfence();
     __syncthreads();
     prof_mark(P, 16);
     if (warp < DPW) {
@@ -1322,13 +1278,9 @@ MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* s
         const float v = __double2float_rn(__ddiv_rn(ob, ll));
         const int e = head * HD + d;
         __stcg(P.att + e, v);
-        if constexpr (TG) {
-            __half dq; int sq;
-            const int qv8 = quant_block_warp2(v, dq, sq);
-            publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
-        } else {
-            if (P.att_x.q) store_tok_block(P.att_x, e >> 5, P.att_token, lane, v);
-        }
+        __half dq; int sq;
+        const int qv8 = quant_block_warp2(v, dq, sq);
+        publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
     }
     prof_mark(P, 17);
     return true;
@@ -1615,13 +1567,13 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
 #if MI_LEAN == 0
             else {
                 if (apf.pending) { (void)mbar_wait_bounded(apf.bar, apf.parity); apf.parity ^= 1u; apf.pending = false; apf.layer = -1; }
-                if (pos + 1 <= kPerHeadAttnMax) ok = attention_phase<HD, 1, G, true, false, true>(P, l, pos, stage, pub.tag - 1u, pub);
-                else ok = attention_phase<HD, G, G, true, false, true>(P, l, pos, stage, pub.tag - 1u, pub);
+                if (pos + 1 <= kPerHeadAttnMax) ok = attention_phase<HD, 1, G>(P, l, pos, stage, pub.tag - 1u, pub);
+                else ok = attention_phase<HD, G, G>(P, l, pos, stage, pub.tag - 1u, pub);
             }
 #elif MI_LEAN == 2
-            ok = attention_phase<HD, 1, G, true, false, true>(P, l, pos, stage, pub.tag - 1u, pub);
+            ok = attention_phase<HD, 1, G>(P, l, pos, stage, pub.tag - 1u, pub);
 #elif MI_LEAN == 3
-            ok = attention_phase<HD, G, G, true, false, true>(P, l, pos, stage, pub.tag - 1u, pub);
+            ok = attention_phase<HD, G, G>(P, l, pos, stage, pub.tag - 1u, pub);
 #endif
             ok = __syncthreads_and(ok ? 1 : 0) != 0;
             prof_mark(P, 3);
@@ -1776,13 +1728,13 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                     // the attention CTAs' business
                 }
 #if MI_LEAN == 0
-                else if (pos + 1 <= kShortAttnMax) ok = attention_short<HD, G, true, false, true>(P, l, pos, sm.stage, pub.tag - 1u, pub);
-                else if (pos + 1 <= kPerHeadAttnMax) ok = attention_phase<HD, 1, G, true, false, true>(P, l, pos, sm.stage, pub.tag - 1u, pub);
-                else ok = attention_phase<HD, G, G, true, false, true>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else if (pos + 1 <= kShortAttnMax) ok = attention_short<HD, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else if (pos + 1 <= kPerHeadAttnMax) ok = attention_phase<HD, 1, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else ok = attention_phase<HD, G, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
 #elif MI_LEAN == 2
-                else ok = attention_phase<HD, 1, G, true, false, true>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else ok = attention_phase<HD, 1, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
 #elif MI_LEAN == 3
-                else ok = attention_phase<HD, G, G, true, false, true>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else ok = attention_phase<HD, G, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
 #endif
             } else if (k != 5) {
                 const int jn = 4 * l + (k == 0 ? 0 : k == 2 ? 1 : k == 3 ? 2 : 3);

@@ -1,6 +1,7 @@
 // The loaded model as the decode and the M-token step see it.
 #pragma once
 #include "decode_kernel.cuh"
+#include "gemm_tok.cuh"
 
 #include <map>
 #include <set>
@@ -28,7 +29,7 @@ struct VerifyBufs {
     int* out = nullptr;                // [M]
     std::map<PassKey, void*> graphs;   // cudaGraphExec_t
     std::set<PassKey> warm;            // kinds of pass that have run plainly once
-    double* attn_part = nullptr; unsigned* attn_cnt = nullptr;   // [M][NH][max_chunks][HD+2], [M][NH]
+    double* attn_part = nullptr;       // chunk sums of the attention (attn_tok.cu)
     float* pick = nullptr; unsigned* pick_cnt = nullptr;         // greedy pick: candidates per slice, arrival counters (self-clearing)
     float* margins = nullptr;          // [M] greedy logit minus the runner-up
 };

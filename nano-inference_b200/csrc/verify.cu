@@ -14,6 +14,7 @@
 // sums, the same attention code with the token's own causal range and chunking), so its
 // logits do not depend on how many tokens share the pass.
 #include "model.cuh"
+#include "attn_tok.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -25,7 +26,7 @@ namespace {
 
 constexpr int VMAX = 16;                    // tokens of one mi_verify call
 constexpr int BMAX = 64;                    // sequences of one batched pass
-constexpr int PMAX = 64;                    // prompt tokens of one pass
+constexpr int PMAX = 512;                   // prompt tokens of one pass
 constexpr int kMaxRanges = 8;               // K ranges of a split product (plan_gemm_tok)
 constexpr size_t kMaxPassGraphs = 64;
 
@@ -117,26 +118,6 @@ __global__ void __launch_bounds__(1024) vf_norm_quant(const DecodeParams P, cons
     }
 }
 
-// attention of M queries: blockIdx.y = query; every query runs the decode kernel's attention over its own causal range
-template <int HD, int G, bool QNAT>
-__global__ void __launch_bounds__(DNT, 1) vf_attention(const __grid_constant__ DecodeParams P, int l, const int* pos0_dev, int pos0_val, long long q_stride,
-                                                       const int* pos_arr, const int* slot_arr, long long slab_stride) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    pdl_launch_dependents(); pdl_wait_prior();
-    const int m = blockIdx.y, nq = P.NH * HD;
-    DecodeParams Q = P;
-    Q.qkv_out = P.qkv_out + (size_t)m * q_stride;
-    Q.att = P.att + (size_t)m * nq; Q.att_token = m;
-    Q.attn_part = P.attn_part + (size_t)m * P.NH * P.max_chunks * (HD + 2);
-    Q.attn_cnt = P.attn_cnt + (size_t)m * P.NH;
-    Q.prof = nullptr;
-    const int pos = pos_arr ? __ldg(pos_arr + m) : (pos0_dev ? __ldg(pos0_dev) : pos0_val) + m;
-    if (slot_arr) { const size_t slab = (size_t)__ldg(slot_arr + m) * (size_t)slab_stride; Q.kc = P.kc + slab; Q.vc = P.vc + slab; }
-    if (pos + 1 <= kShortAttnMax) attention_short<HD, G, false, QNAT>(Q, l, pos, smem);
-    else if (pos + 1 <= kPerHeadAttnMax) attention_phase<HD, 1, G, false, QNAT>(Q, l, pos, smem);
-    else attention_phase<HD, G, G, false, QNAT>(Q, l, pos, smem);
-}
-
 // The QKV product's epilogue as a kernel of its own (more than kMaxFusedTok tokens): one warp per 32 rows and token of y (bias added)
 __global__ void __launch_bounds__(256) vf_rope(const RopeParams r, const float* y, int rows) {
     const int n = blockIdx.y, row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32, lane = threadIdx.x & 31;
@@ -203,24 +184,6 @@ __global__ void __launch_bounds__(512) vf_pick(const float* logits, long long st
     }
 }
 
-size_t attn_smem_bytes(int HD, int G) {
-    return ((size_t)DNW * G * (HD + 2) * 8 + (size_t)DNW * 32 * G * 8 + (size_t)G * (HD + 16) * 8 + 127) / 128 * 128;
-}
-
-template <bool QNAT>
-int launch_attention(mi_ctx* ctx, const DecodeParams& P, int HD, int G, int grid, int M, int l, const int* pos0_dev, int pos0, long long q_stride,
-                     const int* pos_arr, const int* slot_arr, long long slab_stride, bool pdl) {
-    void (*kern)(DecodeParams, int, const int*, int, long long, const int*, const int*, long long) = nullptr;
-    #define MI_PICK(hd, g) if (HD == hd && G == g) kern = vf_attention<hd, g, QNAT>;
-    MI_PICK(32, 2) MI_PICK(64, 2) MI_PICK(64, 7) MI_PICK(128, 6) MI_PICK(128, 8)
-    #undef MI_PICK
-    if (!kern) return set_error(ctx, MI_ERR_UNSUPPORTED, "attention: head_dim %d with %d query heads per kv head is not instantiated", HD, G);
-    const size_t smem = attn_smem_bytes(HD, G);
-    MI_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MI_CUDA(ctx, launch_k(pdl, kern, dim3(grid, M), dim3(DNT), smem, ctx->stream, P, l, pos0_dev, pos0, q_stride, pos_arr, slot_arr, slab_stride));
-    return MI_OK;
-}
-
 void drop_graphs(VerifyBufs& b) {
     for (auto& g : b.graphs) cudaGraphExecDestroy((cudaGraphExec_t)g.second);
     b.graphs.clear();
@@ -255,7 +218,7 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
         (st = take_tok(&b.xf, E, cap)) || (st = take_tok(&b.attf, NQ, cap)) || (st = take_tok(&b.actf, FF, cap)) ||
         (st = take(&b.att, (size_t)cap * NQ)) || (st = take(&b.Y, cap > kMaxFusedTok ? (size_t)cap * std::max(2 * FF, m->qkv_rows) : 0)) || (st = take(&b.logits, (size_t)capl * m->V)) ||
         (st = take(&b.meta, (size_t)3 * cap + 4)) || (st = take(&b.out, (size_t)cap)) || (st = take(&b.margins, (size_t)cap)) ||
-        (st = take(&b.attn_part, (size_t)cap * m->NH * m->max_chunks * (m->HD + 2))) || (st = take(&b.attn_cnt, (size_t)cap * m->NH)) ||
+        (st = take(&b.attn_part, attn_part_max(ctx, m->NH, m->NKV, m->HD))) ||
         (st = take(&b.pick, (size_t)capl * kPickSlices * 3)) || (st = take(&b.pick_cnt, (size_t)capl)))
         return st;
     if (!b.h_meta) {
@@ -283,8 +246,17 @@ struct Pass {
     bool ragged;                                   // every token has a position and a cache slab of its own
     __half* kc; __half* vc; int max_seq; long long slab_stride;
     int lp_max;                                    // longest causal range among the tokens
-    bool last_only;                                // logits of the last token only (prompt processing)
+    int head;                                      // whose logits are wanted
 };
+enum { HEAD_ALL, HEAD_LAST, HEAD_NONE };
+
+// Positions that a launch sequence is planned for: captured passes of up to 320 cached positions share one plan, beyond that those
+// of a power of two (the plan only cuts the ranges, it is right for any position).
+int attn_bucket(int lp_max) {
+    int b = 320;
+    if (lp_max > b) for (b = 512; b < lp_max;) b *= 2;
+    return b;
+}
 
 // Every launch may overlap its predecessor's tail (each kernel waits before it touches what the predecessor wrote);
 // MINFER_VERIFY_PDL=0 restores plain stream order.
@@ -294,20 +266,18 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     DecodeParams P = m->P;
     P.kc = a.kc; P.vc = a.vc; P.max_seq = a.max_seq;
     const int* tokens = b.meta; const int* pos0 = b.meta + M; const int* pos_arr = a.ragged ? b.meta + M : nullptr; const int* slot_arr = a.ragged ? b.meta + 2 * M : nullptr;
-    P.qkv_out = b.q; P.att = b.att; P.attn_part = b.attn_part; P.attn_cnt = b.attn_cnt;
     P.prof = nullptr;
     TokX xf = b.xf, attf = b.attf, actf = b.actf;
     xf.J = attf.J = actf.J = tok_tiling(M).J();
-    P.att_x = attf;
     const std::vector<LayerPtrs>& lp = m->layer_ptrs;
-    const int attn_grid = a.lp_max <= kShortAttnMax ? std::min(m->grid, m->NH) : a.lp_max <= kPerHeadAttnMax ? std::min(m->grid, m->NH * (kPerHeadAttnMax / 256)) : m->grid;
+    const AttnPlan pa = plan_attn_tok(ctx, m->NH, m->NKV, m->HD, M, attn_bucket(a.lp_max), a.ragged);
     static const bool pdl = [] { const char* e = getenv("MINFER_VERIFY_PDL"); return !(e && atoi(e) == 0); }();
     const bool fused = M <= kMaxFusedTok;
     GemmPlan pq, po, pg, pd, pl;
     int st;
     if ((st = plan_gemm_tok(ctx, &m->views[0], fused ? GEMM_QKV : GEMM_PLAIN, M, &pq)) || (st = plan_gemm_tok(ctx, &m->views[1], GEMM_PART, M, &po)) ||
         (st = plan_gemm_tok(ctx, &m->views[2], fused ? GEMM_GU : GEMM_PLAIN, M, &pg)) || (st = plan_gemm_tok(ctx, &m->views[3], GEMM_PART, M, &pd)) ||
-        (st = plan_gemm_tok(ctx, &m->views[4 * L], GEMM_PLAIN, a.last_only ? 1 : M, &pl))) return st;
+        (st = plan_gemm_tok(ctx, &m->views[4 * L], GEMM_PLAIN, a.head == HEAD_LAST ? 1 : M, &pl))) return st;
     const int nt_norm = std::min(1024, (E / 4 + 31) / 32 * 32);
     GemmParams g{};
     g.M = M;
@@ -324,7 +294,8 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         gq.rope = RopeParams{b.q, NQ, m->HD, P.kc, P.vc, m->KVD, a.slab_stride, l, a.max_seq, P.rope_cs, P.rope_freq, P.rope_rows, pos0, pos_arr, slot_arr};
         if ((st = launch_gemm_tok(ctx, wqkv, pq, fused ? GEMM_QKV : GEMM_PLAIN, false, gq, pdl))) return st;
         if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_rope, dim3(((int)wqkv->rows / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, gq.rope, (const float*)b.Y, (int)wqkv->rows));
-        if ((st = launch_attention<true>(ctx, P, m->HD, m->G, attn_grid, M, l, pos0, 0, NQ, pos_arr, slot_arr, a.slab_stride, pdl))) return st;
+        const AttnParams at{b.q, P.kc, P.vc, M, m->NH, m->NKV, m->HD, m->KVD, l, a.max_seq, pos0, 0, pos_arr, slot_arr, a.slab_stride, b.att, attf, b.attn_part, 1, 1};
+        if ((st = launch_attn_tok(ctx, at, pa, pdl))) return st;
         GemmParams go = g; go.x = attf; go.part = b.part; go.ldp = b.ldp;
         if ((st = launch_gemm_tok(ctx, wo, po, GEMM_PART, false, go, pdl))) return st;
         if ((st = norm(false, 0, M, po.ksg, lp[l].ffn_norm, xf))) return st;
@@ -334,7 +305,8 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         GemmParams gd = g; gd.x = actf; gd.part = b.part; gd.ldp = b.ldp;
         if ((st = launch_gemm_tok(ctx, wdn, pd, GEMM_PART, false, gd, pdl))) return st;
     }
-    const int ML = a.last_only ? 1 : M;
+    if (a.head == HEAD_NONE) return MI_OK;
+    const int ML = a.head == HEAD_LAST ? 1 : M;
     TokX lf = b.xf; lf.J = tok_tiling(ML).J();
     if ((st = norm(false, M - ML, ML, pd.ksg, m->P.out_norm, lf))) return st;
     GemmParams gl = g; gl.M = ML; gl.x = lf; gl.y = b.logits;
@@ -351,9 +323,9 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
 int run_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     VerifyBufs& b = m->vb;
     static const bool use_graph = [] { const char* e = getenv("MINFER_VERIFY_GRAPH"); return !(e && atoi(e) == 0); }();
-    const int regime = a.lp_max <= kShortAttnMax ? 0 : a.lp_max <= kPerHeadAttnMax ? 1 : 2;
+    const int regime = attn_bucket(a.lp_max);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!use_graph || a.last_only || cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return enqueue_pass(ctx, m, a);
+    if (!use_graph || a.head != HEAD_ALL || cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return enqueue_pass(ctx, m, a);
     const PassKey key{a.M, regime, a.ragged ? 1 : 0, (const void*)a.kc, (const void*)a.vc, a.max_seq};
     auto it = b.graphs.find(key);
     if (it == b.graphs.end()) {
@@ -404,13 +376,46 @@ extern "C" int mi_verify(mi_ctx* ctx, mi_model* m, const int32_t* tokens_host, i
     b.h_meta[M] = pos0;
     MI_CUDA(ctx, cudaMemcpyAsync(b.meta, b.h_meta, (size_t)(M + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
     MI_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
-    if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + M, false}))) return st;
+    if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + M, HEAD_ALL}))) return st;
     MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
     if (logits_dev) MI_CUDA(ctx, cudaMemcpyAsync(logits_dev, b.logits, (size_t)M * m->V * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     if (out_tokens_host) MI_CUDA(ctx, cudaMemcpyAsync(b.h_meta, b.out, (size_t)M * 4, cudaMemcpyDeviceToHost, ctx->stream));
     st = mi_ctx_sync(ctx);
     if (st != MI_OK) return st;
     if (out_tokens_host) memcpy(out_tokens_host, b.h_meta, (size_t)M * 4);
+    if (elapsed_ms) MI_CUDA(ctx, cudaEventElapsedTime(elapsed_ms, m->ev0, m->ev1));
+    return MI_OK;
+}
+
+extern "C" int mi_prefill(mi_ctx* ctx, mi_model* m, const int32_t* tokens_host, int n, int pos0, int32_t* next_token_host, float* elapsed_ms) {
+    if (!ctx) return MI_ERR_INVALID;
+    if (!m || !tokens_host || n < 1) return set_error(ctx, MI_ERR_INVALID, "prefill: null argument, or no tokens");
+    if (pos0 < 0 || (long long)pos0 + n > m->max_seq)
+        return set_error(ctx, MI_ERR_LIMIT, "prefill: positions %d..%lld exceed the KV cache of %d", pos0, (long long)pos0 + n - 1, m->max_seq);
+    if (m->tp_world != 1) return set_error(ctx, MI_ERR_UNSUPPORTED, "prefill: the M-token step runs on an unsharded model");
+    for (int i = 0; i < n; i++)
+        if (tokens_host[i] < 0 || tokens_host[i] >= m->V) return set_error(ctx, MI_ERR_INVALID, "prefill: token id %d out of range", tokens_host[i]);
+    MI_CUDA(ctx, cudaSetDevice(ctx->device));
+    int st;
+    if ((st = ensure_bufs(ctx, m, std::min(n, PMAX), 1))) return st;
+    VerifyBufs& b = m->vb;
+    if ((st = mi::reset_after_error(ctx, m))) return st;
+    MI_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
+    // passes of equal size (to one token), so that the last one is not a small one at a large one's latency
+    const int passes = (n + PMAX - 1) / PMAX;
+    for (int k = 0; k < passes; k++) {
+        const int i0 = (int)((long long)n * k / passes), M = (int)((long long)n * (k + 1) / passes) - i0;
+        if (k > 0) MI_CUDA(ctx, cudaEventSynchronize(m->ev1));         // the pinned block has been copied
+        memcpy(b.h_meta, tokens_host + i0, (size_t)M * 4);
+        b.h_meta[M] = pos0 + i0;
+        MI_CUDA(ctx, cudaMemcpyAsync(b.meta, b.h_meta, (size_t)(M + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
+        MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
+        if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + i0 + M, k == passes - 1 ? HEAD_LAST : HEAD_NONE}))) return st;
+    }
+    MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
+    if (next_token_host) MI_CUDA(ctx, cudaMemcpyAsync(b.h_meta, b.out, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    if ((st = mi_ctx_sync(ctx))) return st;
+    if (next_token_host) *next_token_host = b.h_meta[0];
     if (elapsed_ms) MI_CUDA(ctx, cudaEventElapsedTime(elapsed_ms, m->ev0, m->ev1));
     return MI_OK;
 }
@@ -431,25 +436,13 @@ extern "C" int mi_attn_splitkv(mi_ctx* ctx, const float* q_dev, const uint16_t* 
     if (M < 1 || M > VMAX) return set_error(ctx, MI_ERR_LIMIT, "attention: M=%d queries per call; this entry point takes 1..%d", M, VMAX);
     if (n_head <= 0 || n_head_kv <= 0 || n_head % n_head_kv || pos0 < 0) return set_error(ctx, MI_ERR_INVALID, "attention: bad head counts or position");
     MI_CUDA(ctx, cudaSetDevice(ctx->device));
-    const int G = n_head / n_head_kv, grid = ctx->sm_count, max_chunks = std::max(1, grid / n_head_kv), NQ = n_head * head_dim;
-    // scratch: chunk partials as doubles, arrival counters
-    int st = ensure_scratch(ctx, (size_t)M * n_head * max_chunks * (head_dim + 2), (size_t)M * n_head);
+    const AttnPlan plan = plan_attn_tok(ctx, n_head, n_head_kv, head_dim, M, pos0 + M, false);
+    int st = ensure_scratch(ctx, plan.part_doubles, 0);
     if (st != MI_OK) return st;
-    DecodeParams P{};
-    P.NH = n_head; P.NKV = n_head_kv; P.HD = head_dim; P.KVD = n_head_kv * head_dim;
-    P.qkv_out = const_cast<float*>(q_dev);
-    P.kc = reinterpret_cast<__half*>(const_cast<uint16_t*>(kcache_dev)); P.vc = reinterpret_cast<__half*>(const_cast<uint16_t*>(vcache_dev));
-    P.max_seq = 0;                        // one layer: the layer index never moves the base
-    P.max_chunks = max_chunks;
-    P.att = out_dev;
-    P.attn_part = ctx->part; P.attn_cnt = ctx->counters;
-    P.err = ctx->d_err;
-    // CTAs per query that the longest causal range of the call can use (the chunking of a query does not depend on it)
-    const int lp_max = pos0 + M;
-    const int agrid = lp_max <= 256 ? std::min(grid, n_head) : lp_max <= kPerHeadAttnMax ? std::min(grid, n_head * (kPerHeadAttnMax / 256)) : grid;
-    return launch_attention<true>(ctx, P, head_dim, G, agrid, M, 0, nullptr, pos0, NQ, nullptr, nullptr, 0, ctx->pdl);
+    const AttnParams p{q_dev, reinterpret_cast<const __half*>(kcache_dev), reinterpret_cast<const __half*>(vcache_dev), M, n_head, n_head_kv, head_dim, n_head_kv * head_dim,
+                       0, 0, nullptr, pos0, nullptr, nullptr, 0, out_dev, TokX{nullptr, nullptr, 0}, ctx->part, 1, 1};
+    return launch_attn_tok(ctx, p, plan, ctx->pdl);
 }
-
 
 // ---- batched decode of independent sequences -------------------------------------------------------------
 // One step of up to B sequences per call: the current token of each goes through ONE pass over the weights as a column
@@ -517,7 +510,7 @@ extern "C" int mi_batch_step(mi_ctx* ctx, mi_batch* b, int n, const int32_t* tok
         memcpy(vb.h_meta + 2 * M, slots_host + i0, (size_t)M * 4);
         const int lp_max = *std::max_element(positions_host + i0, positions_host + i0 + M) + 1;
         MI_CUDA(ctx, cudaMemcpyAsync(vb.meta, vb.h_meta, (size_t)3 * M * 4, cudaMemcpyHostToDevice, ctx->stream));
-        if ((st = run_pass(ctx, m, Pass{M, true, b->kc, b->vc, b->max_seq, b->slab_stride, lp_max, false}))) return st;
+        if ((st = run_pass(ctx, m, Pass{M, true, b->kc, b->vc, b->max_seq, b->slab_stride, lp_max, HEAD_ALL}))) return st;
         if (logits_dev) MI_CUDA(ctx, cudaMemcpyAsync(logits_dev + (size_t)i0 * m->V, vb.logits, (size_t)M * m->V * 4, cudaMemcpyDeviceToDevice, ctx->stream));
         if (out_tokens_host) MI_CUDA(ctx, cudaMemcpyAsync(out_tokens_host + i0, vb.out, (size_t)M * 4, cudaMemcpyDeviceToHost, ctx->stream));
         if (i0 + BMAX < n) MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));       // the pinned block is filled again by the next pass
