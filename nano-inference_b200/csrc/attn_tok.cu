@@ -11,15 +11,16 @@
 // and the rows of an MMA are (query, head) pairs that share a kv head: a K or V element is converted once for up to
 // 4 queries x all heads of the group.
 //
-// A CTA has qb queries of one kv head and one chunk of their positions, and walks it 128 positions at a time:
-//   scores   warp = every 8th group of 8 positions; a lane holds HD/4 consecutive dims of one K row (64 bytes straight from
-//            global memory); q waits in shared memory as doubles in the order the MMA reads it;
+// A CTA has qb queries of one kv head and one chunk of their positions, and walks it in steps of 64 (one query: 128) positions:
+//   scores   warp = every 8th group of 8 positions, all dims; q waits in shared memory as doubles in the order the MMA reads it;
 //   weights  one warp per row: running maximum, exp, sum; stored in MMA order;
-//   values   warp = HD/8 dims, all positions; a lane's V elements of two 8-dim tiles are one 4-byte load.
-// Two CTAs share an SM, so that one's exponentials run beside the other's MMAs.  With several chunks per range the CTAs leave
-// {sum, maximum, denominator} per row and attn_tok_merge folds them against their common maximum; with one chunk the CTA
-// finishes.  The number of chunks comes from the host and only sets how a range is cut, so a captured launch stays valid for
-// any position.
+//   values   warp = HD/8 dims, all positions.
+// K and V rows come through shared memory by asynchronous copies, the K rows of the next step while this step's weights and
+// values are worked on, its V rows during the next scores (fetched by the lanes that use them, they left each warp waiting
+// 7 of 12 cycles per instruction).  Two CTAs share an SM, so that one's exponentials run beside the other's MMAs.  With
+// several chunks per range the CTAs leave {sum, maximum, denominator} per row and attn_tok_merge folds them against their
+// common maximum; with one chunk the CTA finishes.  The number of chunks comes from the host and only sets how a range is
+// cut, so a captured launch stays valid for any position.
 #include "attn_tok.cuh"
 #include <algorithm>
 #include <atomic>
@@ -28,15 +29,22 @@
 namespace mi {
 
 constexpr int kAT = 256, kAW = kAT / 32;          // threads, warps
-constexpr int kSub = 128;                         // positions per step
-constexpr int kScLd = kSub + 4;                   // floats per row of scores
 constexpr int kMaxQB = 4;                         // queries per CTA
-
 __host__ __device__ constexpr int attn_row_tiles(int G, int QB) { return (G * QB + 7) / 8; }
-template <int HD, int RT> constexpr size_t attn_tok_smem() {
-    return (size_t)RT * 8 * HD * 8 + (size_t)RT * 8 * kSub * 8 + (size_t)RT * 8 * kScLd * 4 + (size_t)RT * 8 * 3 * 8;
-}
 
+template <int HD, int RT> struct AttnSmem {
+    static constexpr int R = RT * 8, SUB = RT == 1 ? 128 : 64;       // rows; positions per step
+    static constexpr int SCL = SUB + 4;                              // floats per row of scores
+    // bytes per K and V row: a lane's 16 bytes of K (eight lanes: two rows x 64 bytes) and its 4 bytes of V (four rows x 32
+    // bytes) meet no bank twice
+    static constexpr int KLD = 2 * HD + 64, VLD = 2 * HD + 32;
+    static constexpr int q = 0, wt = q + R * HD * 8, k = wt + R * SUB * 8, v = k + SUB * KLD, sc = v + SUB * VLD, st = sc + R * SCL * 4;
+    static constexpr int bytes = st + R * 3 * 8;
+};
+
+__device__ __forceinline__ void cp16(void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
@@ -61,15 +69,18 @@ __device__ __forceinline__ void attn_emit(const AttnParams& p, int token, int e,
 
 template <int HD, int G, int QB>
 __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant__ AttnParams p) {
-    constexpr int RT = attn_row_tiles(G, QB), R = RT * 8, ROWS = G * QB;
-    constexpr int DPL = HD / 4;                     // dims per lane in the score product
+    constexpr int RT = attn_row_tiles(G, QB), ROWS = G * QB;
+    using SM = AttnSmem<HD, RT>;
+    constexpr int R = SM::R, SUB = SM::SUB, SCL = SM::SCL;
     constexpr int NTW = HD >= 64 ? HD / 64 : 1;     // 8-dim tiles per warp in the value product
     constexpr int VW = HD / 8 / NTW;                // warps that have some
+    constexpr int CH = RT == 1 ? 2 : 1;             // accumulator chains per row tile in the value product
     extern __shared__ __align__(128) uint8_t smem[];
-    double* qs = reinterpret_cast<double*>(smem);                    // [step < DPL][row tile][lane]
-    double* wt = qs + R * HD;                                        // [kSub / 4][row tile][lane]
-    float* sc = reinterpret_cast<float*>(wt + R * kSub);             // [R][kScLd]
-    double* rm = reinterpret_cast<double*>(sc + R * kScLd);          // [R] running maximum
+    double* qs = reinterpret_cast<double*>(smem + SM::q);             // [dim of a lane][row tile][lane]
+    double* wt = reinterpret_cast<double*>(smem + SM::wt);            // [SUB / 4][row tile][lane]
+    uint8_t* ks = smem + SM::k; uint8_t* vs = smem + SM::v;          // [SUB] rows
+    float* sc = reinterpret_cast<float*>(smem + SM::sc);             // [R][SCL]
+    double* rm = reinterpret_cast<double*>(smem + SM::st);           // [R] running maximum
     double* rl = rm + R;                                             // [R] denominator
     double* rf = rl + R;                                             // [R] rescale factor of this step
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -81,39 +92,48 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
     pdl_wait_prior();
     const int posq0 = p.pos_arr ? __ldg(p.pos_arr + q0) : (p.pos0 ? __ldg(p.pos0) : p.pos0_val) + q0;      // position of query q0; the CTA's others follow (QB > 1: one sequence)
     const size_t base = (p.slot_arr ? (size_t)__ldg(p.slot_arr + q0) * (size_t)p.slab_stride : 0) + (size_t)p.layer * p.max_seq * p.KVD + (size_t)kvh * HD;
-    const __half* kb = p.kc + base; const __half* vb = p.vc + base;
     const int Lp = posq0 + nq;                      // positions the last query sees
     const int p0 = (int)((long long)Lp * ch / p.nch), p1 = (int)((long long)Lp * (ch + 1) / p.nch);
-    // q into the order the MMA reads it: step s, row tile r, lane (row, t) holds dim DPL t + s of row 8 r + row
+    auto copy_rows = [&](uint8_t* dst, int ld, const __half* src, int b0) {                  // rows b0 .. of the step, 16 bytes per thread and copy
+        const int np = min(SUB, p1 - b0);
+        for (int i = tid; i < np * (HD / 8); i += kAT) {
+            const int r = i / (HD / 8), c = i - r * (HD / 8);
+            cp16(dst + r * ld + c * 16, src + base + (size_t)(b0 + r) * p.KVD + c * 8);
+        }
+        cp_commit();
+    };
+    if (p0 < p1) { copy_rows(ks, SM::KLD, p.kc, p0); copy_rows(vs, SM::VLD, p.vc, p0); }
+    // q into the order the MMA reads it: lane (row, t) takes the 16-byte pieces t, t + 4, .. of a row: its dim s is 8 (4 (s / 8) + t) + s % 8
     for (int i = tid; i < R * HD; i += kAT) {
-        const int d = i % HD, row = i / HD, qi = row / G, h = row - qi * G, tt = d / DPL, s = d - tt * DPL;
+        const int d = i % HD, row = i / HD, qi = row / G, h = row - qi * G, tt = (d >> 3) & 3, s = (d >> 5) * 8 + (d & 7);
         const float v = row < ROWS && qi < nq ? __ldcg(p.q + (size_t)(q0 + qi) * p.NH * HD + (size_t)(kvh * G + h) * HD + d) : 0.f;
         qs[(s * RT + (row >> 3)) * 32 + (row & 7) * 4 + tt] = (double)v;
     }
     for (int i = tid; i < R; i += kAT) { rm[i] = -INFINITY; rl[i] = 0.0; }
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
-    double o[RT][NTW][2];
+    double o[CH][RT][NTW][2];
     #pragma unroll
-    for (int r = 0; r < RT; r++)
+    for (int c = 0; c < CH; c++)
         #pragma unroll
-        for (int n = 0; n < NTW; n++) o[r][n][0] = o[r][n][1] = 0.0;
-    __syncthreads();
+        for (int r = 0; r < RT; r++)
+            #pragma unroll
+            for (int n = 0; n < NTW; n++) o[c][r][n][0] = o[c][r][n][1] = 0.0;
 
-    for (int b0 = p0; b0 < p1; b0 += kSub) {
-        const int np = min(kSub, p1 - b0);
+    for (int b0 = p0; b0 < p1; b0 += SUB) {
+        const int np = min(SUB, p1 - b0);
+        cp_wait<1>();                               // the K rows (the V rows were requested after them)
+        __syncthreads();
         // ---- scores
         #pragma unroll 1
         for (int t = warp; t * 8 < np; t += kAW) {
-            const __half* kr = kb + (size_t)(b0 + min(t * 8 + g, np - 1)) * p.KVD + t4 * DPL;
-            uint4 kw[DPL / 8];
-            #pragma unroll
-            for (int i = 0; i < DPL / 8; i++) kw[i] = __ldcg(reinterpret_cast<const uint4*>(kr) + i);
+            const uint8_t* kr = ks + min(t * 8 + g, np - 1) * SM::KLD + t4 * 16;
             double c[RT][2][2];                     // two chains per row tile
             #pragma unroll
             for (int r = 0; r < RT; r++) c[r][0][0] = c[r][0][1] = c[r][1][0] = c[r][1][1] = 0.0;
             #pragma unroll
-            for (int i = 0; i < DPL / 8; i++) {
-                const unsigned w[4] = {kw[i].x, kw[i].y, kw[i].z, kw[i].w};
+            for (int i = 0; i < HD / 32; i++) {
+                const uint4 kw = *reinterpret_cast<const uint4*>(kr + i * 64);
+                const unsigned w[4] = {kw.x, kw.y, kw.z, kw.w};
                 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const double k0 = half_lo(w[e]), k1 = half_hi(w[e]);
@@ -128,22 +148,23 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
                 for (int e = 0; e < 2; e++) {
                     const int row = 8 * r + g, pp = t * 8 + 2 * t4 + e, qi = row / G;
                     const float s = __fmul_rn(__double2float_rn(__dadd_rn(c[r][0][e], c[r][1][e])), inv);
-                    sc[row * kScLd + pp] = b0 + pp < p1 && b0 + pp <= posq0 + qi ? s : -INFINITY;
+                    sc[row * SCL + pp] = b0 + pp < p1 && b0 + pp <= posq0 + qi ? s : -INFINITY;
                 }
         }
         __syncthreads();
+        if (b0 + SUB < p1) copy_rows(ks, SM::KLD, p.kc, b0 + SUB); else cp_commit();
         // ---- weights: one warp per row
         #pragma unroll 1
-        for (int row = warp; row < R; row += kAW) {
-            float s[kSub / 32], m = -INFINITY;
+        for (int row = warp; row < ROWS; row += kAW) {
+            float s[SUB / 32], m = -INFINITY;
             #pragma unroll
-            for (int i = 0; i < kSub / 32; i++) { s[i] = lane + 32 * i < np ? sc[row * kScLd + lane + 32 * i] : -INFINITY; m = fmaxf(m, s[i]); }
+            for (int i = 0; i < SUB / 32; i++) { s[i] = lane + 32 * i < np ? sc[row * SCL + lane + 32 * i] : -INFINITY; m = fmaxf(m, s[i]); }
             #pragma unroll
             for (int q = 16; q; q >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, q));
             const double mo = rm[row], mn = fmax(mo, (double)m);
             double l = 0.0;
             #pragma unroll
-            for (int i = 0; i < kSub / 32; i++) {
+            for (int i = 0; i < SUB / 32; i++) {
                 const double w = s[i] == -INFINITY ? 0.0 : exp((double)s[i] - mn);
                 const int pp = lane + 32 * i;
                 wt[((pp >> 2) * RT + (row >> 3)) * 32 + (row & 7) * 4 + (pp & 3)] = w;
@@ -156,43 +177,49 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
                 rf[row] = f; rm[row] = mn; rl[row] = __fma_rn(rl[row], f, l);
             }
         }
+        cp_wait<1>();                               // the V rows
         __syncthreads();
         // ---- values
         if (warp < VW) {
             if (b0 > p0) {
                 #pragma unroll
                 for (int r = 0; r < RT; r++) {
-                    const double f = rf[8 * r + g];
+                    const double f = 8 * r + g < ROWS ? rf[8 * r + g] : 1.0;
                     #pragma unroll
-                    for (int n = 0; n < NTW; n++) { o[r][n][0] = __dmul_rn(o[r][n][0], f); o[r][n][1] = __dmul_rn(o[r][n][1], f); }
+                    for (int c = 0; c < CH; c++)
+                        #pragma unroll
+                        for (int n = 0; n < NTW; n++) { o[c][r][n][0] = __dmul_rn(o[c][r][n][0], f); o[c][r][n][1] = __dmul_rn(o[c][r][n][1], f); }
                 }
             }
-            constexpr int PF = 8;                   // steps of four positions whose V elements are requested together
-            const __half* vr = vb + warp * (8 * NTW) + g * NTW;
-            #pragma unroll 1
-            for (int s0 = 0; s0 * 4 < np; s0 += PF) {
-                unsigned vw[PF];
+            const uint8_t* vr = vs + (warp * (8 * NTW) + g * NTW) * 2;
+            #pragma unroll 4
+            for (int s = 0; s * 4 < np; s++) {
+                const uint8_t* v = vr + min(s * 4 + t4, np - 1) * SM::VLD;
+                unsigned vw;
+                if constexpr (NTW == 2) vw = *reinterpret_cast<const unsigned*>(v); else vw = *reinterpret_cast<const unsigned short*>(v);
+                const double v0 = half_lo(vw), v1 = NTW == 2 ? half_hi(vw) : 0.0;
+                const double* a = wt + (size_t)(s * RT) * 32 + lane;
                 #pragma unroll
-                for (int u = 0; u < PF; u++) {
-                    const __half* v = vr + (size_t)(b0 + min((s0 + u) * 4 + t4, np - 1)) * p.KVD;
-                    if constexpr (NTW == 2) vw[u] = __ldcg(reinterpret_cast<const unsigned*>(v));
-                    else vw[u] = __ldcg(reinterpret_cast<const unsigned short*>(v));
-                }
-                #pragma unroll
-                for (int u = 0; u < PF; u++) {
-                    if ((s0 + u) * 4 >= np) break;  // warp-uniform
-                    const double* a = wt + (size_t)((s0 + u) * RT) * 32 + lane;
-                    const double v0 = half_lo(vw[u]), v1 = NTW == 2 ? half_hi(vw[u]) : 0.0;
-                    #pragma unroll
-                    for (int r = 0; r < RT; r++) {
-                        const double w = a[r * 32];
-                        dmma(o[r][0], w, v0);
-                        if constexpr (NTW == 2) dmma(o[r][NTW - 1], w, v1);
+                for (int r = 0; r < RT; r++) {
+                    const double w = a[r * 32];
+                    if constexpr (CH == 2) {
+                        if (s & 1) { dmma(o[1][r][0], w, v0); if constexpr (NTW == 2) dmma(o[1][r][NTW - 1], w, v1); }
+                        else { dmma(o[0][r][0], w, v0); if constexpr (NTW == 2) dmma(o[0][r][NTW - 1], w, v1); }
+                    } else {
+                        dmma(o[0][r][0], w, v0);
+                        if constexpr (NTW == 2) dmma(o[0][r][NTW - 1], w, v1);
                     }
                 }
             }
         }
-        __syncthreads();                            // scores and weights may be written again
+        __syncthreads();                            // scores, weights and V rows may be written again
+        if (b0 + SUB < p1) copy_rows(vs, SM::VLD, p.vc, b0 + SUB);
+    }
+    if constexpr (CH == 2) {
+        #pragma unroll
+        for (int r = 0; r < RT; r++)
+            #pragma unroll
+            for (int n = 0; n < NTW; n++) { o[0][r][n][0] = __dadd_rn(o[0][r][n][0], o[1][r][n][0]); o[0][r][n][1] = __dadd_rn(o[0][r][n][1], o[1][r][n][1]); }
     }
     // ---- the chunk's rows
     if (p.nch > 1) {
@@ -205,7 +232,7 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
                 #pragma unroll
                 for (int n = 0; n < NTW; n++)
                     #pragma unroll
-                    for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + n, o[r][n][e]);
+                    for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + n, o[0][r][n][e]);
             }
         }
         for (int row = tid; row < ROWS; row += kAT) {
@@ -220,11 +247,12 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
     if (warp < VW) {
         #pragma unroll
         for (int r = 0; r < RT; r++) {
+            if (8 * r + g >= ROWS) continue;
             const double l = rl[8 * r + g];
             #pragma unroll
             for (int n = 0; n < NTW; n++)
                 #pragma unroll
-                for (int e = 0; e < 2; e++) of[(8 * r + g) * HD + warp * (8 * NTW) + (2 * t4 + e) * NTW + n] = __double2float_rn(__ddiv_rn(o[r][n][e], l));
+                for (int e = 0; e < 2; e++) of[(8 * r + g) * HD + warp * (8 * NTW) + (2 * t4 + e) * NTW + n] = __double2float_rn(__ddiv_rn(o[0][r][n][e], l));
         }
     }
     __syncthreads();
@@ -306,13 +334,13 @@ size_t attn_part_max(const mi_ctx* ctx, int NH, int NKV, int HD) { return (size_
 namespace {
 template <int HD, int G, int QB>
 int launch_qb(mi_ctx* ctx, const AttnParams& p, bool pdl) {
-    constexpr size_t smem = attn_tok_smem<HD, attn_row_tiles(G, QB)>();
+    constexpr int smem = AttnSmem<HD, attn_row_tiles(G, QB)>::bytes;
     auto kern = attn_tok_kernel<HD, G, QB>;
     static std::mutex mu;
     static std::atomic<unsigned> raised{0};                   // bit per device: opt-in shared memory set
     if (!(raised.load(std::memory_order_acquire) >> (ctx->device & 31) & 1u)) {
         std::lock_guard<std::mutex> hold(mu);
-        MI_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MI_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         raised.fetch_or(1u << (ctx->device & 31), std::memory_order_release);
     }
     const int units = p.NKV * ((p.M + QB - 1) / QB);
