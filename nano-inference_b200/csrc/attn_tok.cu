@@ -317,19 +317,21 @@ __global__ void __launch_bounds__(kAT) attn_tok_merge(const __grid_constant__ At
 
 // Queries per CTA: four where the ranges are long (their work is FP64 time, and an MMA's rows should be full: 4 x 6 heads are three
 // whole row tiles, one query's 6 heads fill three quarters of one), one where they are short or belong to different sequences
-// (the work is latency, and more CTAs share it).  Chunks: one up to 320 positions (a CTA walks them in the time a second
-// launch takes); beyond, enough that two CTAs per SM have work, and none shorter than 64 positions.
+// (the work is latency, and more CTAs share it).  Chunks: one up to 320 positions where CTAs have one query (a CTA walks them in the
+// time a second launch takes), up to 128 where they have four; beyond, enough that two CTAs per SM have work, and none
+// shorter than 64 positions.
 AttnPlan plan_attn_tok(const mi_ctx* ctx, int NH, int NKV, int HD, int M, int lp_max, bool ragged) {
     AttnPlan a;
     a.qb = !ragged && M > 1 && (long long)M * lp_max >= 16384 ? kMaxQB : 1;
     const int units = NKV * ((M + a.qb - 1) / a.qb);
-    a.nch = lp_max <= 320 ? 1 : std::max(1, std::min((lp_max + 63) / 64, 2 * ctx->sm_count / units));
+    const int share = a.qb > 1 ? (2 * ctx->sm_count + units - 1) / units : 2 * ctx->sm_count / units;
+    a.nch = lp_max <= (a.qb > 1 ? 128 : 320) ? 1 : std::max(1, std::min((lp_max + 63) / 64, share));
     a.part_doubles = a.nch > 1 ? (size_t)M * NH * a.nch * (HD + 2) : 0;
     return a;
 }
 
-// units x chunks is at most two CTAs per SM, a unit at most kMaxQB queries of one group
-size_t attn_part_max(const mi_ctx* ctx, int NH, int NKV, int HD) { return (size_t)kMaxQB * (NH / NKV) * 2 * ctx->sm_count * (HD + 2); }
+// with more than one chunk, units x chunks is below two CTAs per SM and another unit each; a unit is at most kMaxQB queries of one group
+size_t attn_part_max(const mi_ctx* ctx, int NH, int NKV, int HD) { return (size_t)kMaxQB * (NH / NKV) * 4 * ctx->sm_count * (HD + 2); }
 
 namespace {
 template <int HD, int G, int QB>
