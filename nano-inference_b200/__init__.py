@@ -142,12 +142,12 @@ def detok_piece(piece):
 
 def _ptr(t):
     """Device (or host) address of a torch tensor / numpy array / int / None."""
-    if t is None:
-        return None
-    if isinstance(t, int):
+    try:
+        return t.data_ptr()              # torch tensors: what the hot calls pass
+    except AttributeError:
+        pass
+    if t is None or isinstance(t, int):
         return t
-    if hasattr(t, "data_ptr"):
-        return t.data_ptr()
     if hasattr(t, "ctypes"):
         return t.ctypes.data
     raise TypeError(f"cannot take the address of {type(t)}")
@@ -158,6 +158,7 @@ class Context:
 
     def __init__(self, device=0):
         self.lib = load_library()
+        self._quant_q8, self._gemv_q4_q8, self._gemm_q4_q8 = self.lib.mi_quant_q8, self.lib.mi_gemv_q4_q8_ex, self.lib.mi_gemm_q4_q8
         h = _vp()
         st = self.lib.mi_ctx_create(device, C.byref(h))
         if st != MI_OK:
@@ -228,12 +229,16 @@ class Context:
         self.check(self.lib.mi_requant_q4_0(self.h, ggml_type, _ptr(src_dev), rows, cols, _ptr(dst_dev)), "mi_requant_q4_0")
 
     # ---- kernels (device pointers: torch CUDA tensors)
+    # (these are called per matrix by programs that own the layer loop: a microsecond here is a microsecond per product)
     def quant_q8(self, x, xq, xd, n=None, M=1):
-        n = x.shape[-1] if n is None else n
-        self.check(self.lib.mi_quant_q8(self.h, _ptr(x), n, M, _ptr(xq), _ptr(xd)), "mi_quant_q8")
+        st = self._quant_q8(self.h, _ptr(x), x.shape[-1] if n is None else n, M, _ptr(xq), _ptr(xd))
+        if st:
+            self.check(st, "mi_quant_q8")
 
     def gemv_q4_q8(self, w, xq, xd, y, bias=None, ksplit=0, variant=0):
-        self.check(self.lib.mi_gemv_q4_q8_ex(self.h, w.h, _ptr(xq), _ptr(xd), _ptr(bias), _ptr(y), ksplit, variant), "mi_gemv_q4_q8")
+        st = self._gemv_q4_q8(self.h, w.h, _ptr(xq), _ptr(xd), None if bias is None else _ptr(bias), _ptr(y), ksplit, variant)
+        if st:
+            self.check(st, "mi_gemv_q4_q8")
 
     def gemv_q4_q8_noalloc(self, w, xq, xd, y, bias=None):
         """The GEMV through the entry point that never allocates (fixed built-in scratch)."""
@@ -241,7 +246,9 @@ class Context:
 
     def gemm_q4_q8(self, w, xq, xd, M, y, bias=None):
         """M token vectors per weight pass on the tensor cores; y is [M][rows]."""
-        self.check(self.lib.mi_gemm_q4_q8(self.h, w.h, _ptr(xq), _ptr(xd), M, _ptr(bias), _ptr(y)), "mi_gemm_q4_q8")
+        st = self._gemm_q4_q8(self.h, w.h, _ptr(xq), _ptr(xd), M, None if bias is None else _ptr(bias), _ptr(y))
+        if st:
+            self.check(st, "mi_gemm_q4_q8")
 
     def attn_splitkv(self, q, kcache, vcache, n_head, n_head_kv, head_dim, pos0, M, out):
         """Causal GQA attention of M consecutive queries over an fp16 cache [positions][n_head_kv*head_dim]."""

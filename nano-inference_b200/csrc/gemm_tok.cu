@@ -434,5 +434,5 @@ extern "C" int mi_gemm_q4_q8(mi_ctx* ctx, const mi_weight* w, const int8_t* xq_d
     if (st != MI_OK) return st;
     GemmParams p{};
     p.M = M; p.xq = xq_dev; p.xd = reinterpret_cast<const __half*>(xd_dev); p.bias = bias_dev; p.y = y_dev;
-    return launch_gemm_tok(ctx, w, pl, GEMM_PLAIN, true, p, ctx->pdl);
+    return launch_gemm_tok(ctx, w, pl, GEMM_PLAIN, true, p, true);
 }

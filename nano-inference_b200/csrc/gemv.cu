@@ -37,6 +37,78 @@ gemv_q4_q8_kernel(const __grid_constant__ GemvShape sh, const __grid_constant__ 
     if (!ok && lane == 0) atomicMax(io.err, MI_ERR_TIMEOUT);
 }
 
+// The GEMV where the streaming kernel above would have too few row groups for its warps: one CTA per row group, its warps take
+// the K tiles (lane = row, as there) and meet in shared memory.  What bounds these sizes is latency - a matrix is 0.1 - 4 us of
+// HBM time - so a warp's first tile is requested straight into registers (nine 16-byte loads per lane, each a contiguous 512
+// bytes per warp) before the kernel waits for its predecessor, each warp stages only the activations of its own tile, and several
+// CTAs share an SM instead of a loop.  The streaming kernel reached these sizes by splitting K over the grid: partial sums, fence,
+// atomic and a second read in global memory, 14 us of the 17 that quantizing and multiplying an 11008 x 2048 matrix took.
+template <int KB, int W>
+__global__ void __launch_bounds__(W * 32) gemv_q4_q8_fold_kernel(const __grid_constant__ GemvShape sh, const __grid_constant__ GemvIO io) {
+    __shared__ double fold[W][32];
+    __shared__ __align__(16) int8_t xs_all[W][KB * 32];
+    __shared__ float2 sc_all[W][KB];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = (int)blockIdx.x / sh.groups, g = (int)blockIdx.x - c * sh.groups;
+    const uint8_t* base = sh.base + (size_t)c * sh.mat_stride + (size_t)g * sh.nt * tile_bytes(KB);
+    int8_t* xs = xs_all[warp]; float2* sc = sc_all[warp];
+    uint4 wq[KB];
+    uint4 ws = make_uint4(0u, 0u, 0u, 0u);
+    auto load_tile = [&](int t) {
+        const uint8_t* tile = base + (size_t)t * tile_bytes(KB);
+        #pragma unroll
+        for (int k = 0; k < KB; k++) wq[k] = __ldcs(reinterpret_cast<const uint4*>(tile) + k * 32 + lane);
+        const uint8_t* sp = tile + KB * 512 + lane * (KB * 2);
+        if constexpr (KB == 8) ws = __ldcs(reinterpret_cast<const uint4*>(sp));
+        else if constexpr (KB == 4) { const uint2 v = __ldcs(reinterpret_cast<const uint2*>(sp)); ws.x = v.x; ws.y = v.y; }
+        else if constexpr (KB == 2) ws.x = __ldcs(reinterpret_cast<const unsigned*>(sp));
+        else ws.x = __ldcs(reinterpret_cast<const unsigned short*>(sp));
+    };
+    if (warp < sh.nt) load_tile(warp);                    // weights do not depend on any earlier kernel
+    pdl_launch_dependents();
+    pdl_wait_prior();                                     // activations do
+    double acc = 0.0;
+    for (int t = warp; t < sh.nt; t += W) {
+        // the tile's activations: 16 bytes per lane, and per block {fp32 of the fp16 scale, float(8 * sum of the values)}
+        int s = 0;
+        if (lane < 2 * KB) {
+            const int4 x = __ldg(reinterpret_cast<const int4*>(io.xq + (size_t)t * KB * 32) + lane);
+            *reinterpret_cast<int4*>(xs + lane * 16) = x;
+            s = __dp4a(0x01010101, x.x, 0); s = __dp4a(0x01010101, x.y, s); s = __dp4a(0x01010101, x.z, s); s = __dp4a(0x01010101, x.w, s);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if (lane < 2 * KB && !(lane & 1)) sc[lane >> 1] = make_float2(__half2float(__ldg(io.xd + t * KB + (lane >> 1))), __int2float_rn(8 * s));
+        __syncwarp();
+        const unsigned wsv[4] = {ws.x, ws.y, ws.z, ws.w};
+        #pragma unroll
+        for (int k = 0; k < KB; k++) {
+            const int4 xa = *reinterpret_cast<const int4*>(xs + k * 32), xc = *reinterpret_cast<const int4*>(xs + k * 32 + 16);
+            const float2 x2 = sc[k];
+            const float dw = __half2float(__ushort_as_half((unsigned short)(wsv[k / 2] >> (16 * (k & 1)))));
+            acc = blk_acc(acc, dw, x2.x, dot_q4_block(wq[k], xa, xc), x2.y);
+        }
+        if (t + W < sh.nt) load_tile(t + W);
+        __syncwarp();
+    }
+    fold[warp][lane] = acc;
+    __syncthreads();
+    if (warp != 0) return;
+    #pragma unroll
+    for (int w = 1; w < W; w++) acc = __dadd_rn(acc, fold[w][lane]);
+    const int r = g * 32 + lane;
+    if (r < io.rows) io.y[(long long)c * io.y_stride + r] = __double2float_rn(acc) + (io.bias ? io.bias[r] : 0.f);
+}
+
+template <int KB>
+static int launch_fold(mi_ctx* ctx, const mi_weight* w, const GemvIO& io) {
+    const GemvShape sh{w->dev, (long long)w->mat_stride, (int)w->count, w->groups, w->nt, 1, w->nb, (int)w->rows};
+    const dim3 grid((unsigned)(w->count * w->groups));
+    if (w->nt <= 8) MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 8>, grid, dim3(256), 0, ctx->stream, sh, io));
+    else if (w->nt <= 16) MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 16>, grid, dim3(512), 0, ctx->stream, sh, io));
+    else MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 24>, grid, dim3(768), 0, ctx->stream, sh, io));
+    return MI_OK;
+}
+
 // variant -> {warps per CTA, ring stages per warp}; see launch_kb
 constexpr int kNumVariants = 8;
 
@@ -85,14 +157,15 @@ static int launch_one(mi_ctx* ctx, const mi_weight* w, const GemvIO& io, int ksp
         if (st != MI_OK) return st;
         sc.part = ctx->part; sc.counters = ctx->counters;
     }
-    kern<<<(unsigned)ctas, NW * 32, smem, ctx->stream>>>(sh, sc, io);
-    MI_CUDA(ctx, cudaGetLastError());
+    MI_CUDA(ctx, launch_k(true, kern, dim3((unsigned)ctas), dim3(NW * 32), smem, ctx->stream, sh, sc, io));
     return MI_OK;
 }
 
 template <int KB, bool DUMP>
 static int launch_kb(mi_ctx* ctx, const mi_weight* w, const GemvIO& io, int ksplit, int variant) {
     if (DUMP) return launch_one<KB, 8, 2, true>(ctx, w, io, 1);
+    // fewer than two row groups per warp of the streaming kernel's grid: there it would have to split K over the grid
+    if (variant == 0 && ksplit <= 0 && w->count * w->groups < 2LL * ctx->sm_count * 8) return launch_fold<KB>(ctx, w, io);
     switch (variant) {
         case 0: return launch_one<KB, 8, 3, false>(ctx, w, io, ksplit);
         case 1: return launch_one<KB, 8, 4, false>(ctx, w, io, ksplit);

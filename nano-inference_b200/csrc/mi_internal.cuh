@@ -22,7 +22,6 @@ struct mi_ctx {
     double* part = nullptr; size_t part_count = 0;
     unsigned* counters = nullptr; size_t n_counters = 0;
     // staging for the host-buffer convenience calls
-    bool pdl = false;                // launches may start before their predecessor in the stream has finished (see launch_k)
     void* h_pinned = nullptr; size_t h_pinned_bytes = 0;
     void* d_stage = nullptr; size_t d_stage_bytes = 0;
     std::string last_error;
@@ -58,7 +57,8 @@ int launch_requant_q4_0(mi_ctx* ctx, int type, const void* src_dev, long long ro
 
 // Kernel launch, optionally with programmatic stream serialization: the kernel may become resident while its
 // predecessor in the stream still runs; it must execute griddepcontrol.wait (pdl_wait_prior) before it reads what the
-// predecessor wrote or writes anything the predecessor may read.  Used for the launch sequence of the M-token pass.
+// predecessor wrote or writes anything the predecessor may read (weights, complete when their handle is returned, may be read
+// before).  The predecessor may be anyone's kernel: one that does not announce its dependents is simply waited for.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg{};

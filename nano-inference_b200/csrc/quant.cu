@@ -10,6 +10,8 @@ namespace mi {
 __global__ void __launch_bounds__(256) quant_q8_kernel(const float* __restrict__ x, long long n_blocks, int8_t* __restrict__ xq,
                                                        __half* __restrict__ xd) {
     const int lane = threadIdx.x & 31, sub = lane >> 3, li = lane & 7;
+    pdl_launch_dependents();                              // the product that follows may fetch its weights meanwhile
+    pdl_wait_prior();
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5), w0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     for (long long b4 = w0 * 4; b4 < n_blocks; b4 += warps * 4) {
         const long long blk = b4 + sub;
@@ -33,8 +35,7 @@ int launch_quant_q8(mi_ctx* ctx, const float* x, long long n_blocks, int8_t* xq,
     if (n_blocks == 0) return MI_OK;
     const long long want = (n_blocks + 31) / 32;                       // CTAs if every warp made one trip
     const long long cap = (long long)ctx->sm_count * 8;                 // full occupancy; larger inputs loop
-    quant_q8_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, ctx->stream>>>(x, n_blocks, xq, xd);
-    MI_CUDA(ctx, cudaGetLastError());
+    MI_CUDA(ctx, launch_k(true, quant_q8_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, ctx->stream, x, n_blocks, xq, xd));
     return MI_OK;
 }
 

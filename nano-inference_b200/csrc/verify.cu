@@ -441,7 +441,7 @@ extern "C" int mi_attn_splitkv(mi_ctx* ctx, const float* q_dev, const uint16_t* 
     if (st != MI_OK) return st;
     const AttnParams p{q_dev, reinterpret_cast<const __half*>(kcache_dev), reinterpret_cast<const __half*>(vcache_dev), M, n_head, n_head_kv, head_dim, n_head_kv * head_dim,
                        0, 0, nullptr, pos0, nullptr, nullptr, 0, out_dev, TokX{nullptr, nullptr, 0}, ctx->part, 1, 1};
-    return launch_attn_tok(ctx, p, plan, ctx->pdl);
+    return launch_attn_tok(ctx, p, plan, true);
 }
 
 // ---- batched decode of independent sequences -------------------------------------------------------------
