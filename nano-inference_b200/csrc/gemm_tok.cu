@@ -39,14 +39,17 @@ constexpr int kStaticSmem = 64;                              // room for static 
 constexpr int kFoldLd = 34;                                  // doubles per token in the fold buffer: conflict-free for the MMA's layout
 __host__ __device__ constexpr int tok_warps(int NT) { return NT <= 2 ? 12 : 8; }
 
-template <int KB, int NT, bool FOLD>
+constexpr int kStepBlk = 8;                                  // blocks per ring slot: one tile of eight blocks, or as many smaller ones (they are contiguous)
+constexpr int kStepBytes = kStepBlk * kTileRowBytes;
+
+template <int NT, bool FOLD>
 struct TokSmem {
-    static constexpr int W = tok_warps(NT), TB = tile_bytes(KB), N = NT * 8;
+    static constexpr int W = tok_warps(NT), TB = kStepBytes, N = NT * 8;
     static constexpr int ring = W * kRing * TB;
     static constexpr int scratch = FOLD ? W * N * kFoldLd * 8 : 0;                          // partial sums of all warps
     static constexpr int bars = ((W * kRing + 1) * 8 + 15) / 16 * 16;
     static constexpr int fixed = ring + scratch + bars;
-    static constexpr int x_block = NT * 256 + N * 8, x_tile = KB * x_block;
+    static constexpr int x_block = NT * 256 + N * 8, x_step = kStepBlk * x_block;
 };
 
 __device__ __forceinline__ void mma_s8(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, const uint2& b) {
@@ -108,7 +111,7 @@ __device__ __forceinline__ void tile_mma(const uint8_t* tile, const uint2* bs, c
 
 template <int KB, int NT, int MODE, bool ROWMAJOR, bool FOLD>
 __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(const __grid_constant__ GemmParams p) {
-    using SM = TokSmem<KB, NT, FOLD>;
+    using SM = TokSmem<NT, FOLD>;
     constexpr int W = SM::W, TB = SM::TB, N = SM::N, U = MODE == GEMM_GU ? 2 : 1;
     static_assert(FOLD || MODE == GEMM_PLAIN || MODE == GEMM_PART, "epilogues across rows work on folded sums");
     extern __shared__ __align__(128) uint8_t smem[];
@@ -116,10 +119,10 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::ring + SM::scratch);
     uint64_t* xbar = bars + W * kRing;
     uint2* bs = reinterpret_cast<uint2*>(smem + SM::fixed);                              // staged activations: operands of a chunk, then its scales
-    double* dxs = reinterpret_cast<double*>(smem + SM::fixed + (size_t)p.kct * KB * NT * 256);
+    double* dxs = reinterpret_cast<double*>(smem + SM::fixed + (size_t)p.kct * kStepBlk * NT * 256);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int sp = (int)(blockIdx.x % p.ksg), rest = (int)(blockIdx.x / p.ksg), c = rest % p.C, tt = rest / p.C;
-    const int k0 = sp * p.nt / p.ksg, k1 = (sp + 1) * p.nt / p.ksg, nchunk = (k1 - k0 + p.kct - 1) / p.kct;      // this CTA's K range, in tiles
+    const int k0 = sp * p.nt / p.ksg, k1 = (sp + 1) * p.nt / p.ksg, nchunk = (k1 - k0 + p.kct - 1) / p.kct;      // this CTA's K range, in steps
     // the warp's row group of round r: group0 + r * gstride, while below glimit
     const int kw = FOLD ? p.kw : 1, rg = FOLD ? W / kw : W, gi = FOLD ? warp / kw : warp, part = FOLD ? warp - gi * kw : 0;
     const int group0 = FOLD ? c * rg + gi : warp * p.C + c, gstride = p.C * rg, glimit = gi < rg ? p.groups : 0;
@@ -143,8 +146,9 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
         const int grp = group0 + pr * gstride;
         if (grp >= glimit) { pr = rounds; return; }                                      // groups only grow: nothing follows
         const int s = issued % kRing;
-        mbar_expect_tx(&rbar[s], TB);
-        bulk_g2s_hint(ring + (size_t)s * TB, p.base + ((size_t)grp * p.nt + pt) * TB, TB, &rbar[s], policy);
+        const int bytes = min(kStepBlk, p.nb - pt * kStepBlk) * kTileRowBytes;
+        mbar_expect_tx(&rbar[s], bytes);
+        bulk_g2s_hint(ring + (size_t)s * TB, p.base + ((size_t)grp * p.nb + pt * kStepBlk) * kTileRowBytes, bytes, &rbar[s], policy);
         issued++; pt += kw;
         if (pt >= k1) { pt = k0 + part; pr++; }
     };
@@ -159,15 +163,26 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
     unsigned xphase = 0;
     auto stage = [&](int b0, int nblk) {                                                 // activations of blocks b0 .. b0 + nblk
         if constexpr (ROWMAJOR) {
-            for (int i = tid; i < nblk * NT * 32; i += W * 32) {
-                const int ln = i & 31, bj = i >> 5, j = bj % NT, b = bj / NT, n = tt * N + j * 8 + (ln >> 2);
-                uint2 v = make_uint2(0u, 0u);
-                if (n < p.M) {
-                    const unsigned* src = reinterpret_cast<const unsigned*>(p.xq + ((size_t)n * p.nb + b0 + b) * 32) + (ln & 3);
-                    v = make_uint2(__ldcg(src), __ldcg(src + 4));
+            // 16 bytes per thread and load (half h of block b of token n), four loads in flight; they land as four lanes' words
+            const int items = nblk * NT * 16;
+            for (int i0 = tid; i0 < items; i0 += 4 * W * 32) {
+                int4 v[4];
+                #pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int i = i0 + u * W * 32, n = tt * N + (i >> 1) % N, b = (i >> 1) / N;
+                    v[u] = make_int4(0, 0, 0, 0);
+                    if (i < items && n < p.M) v[u] = __ldcg(reinterpret_cast<const int4*>(p.xq + ((size_t)n * p.nb + b0 + b) * 32) + (i & 1));
                 }
-                bs[i] = v;
+                #pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int i = i0 + u * W * 32, n = (i >> 1) % N, b = (i >> 1) / N;
+                    if (i < items) {
+                        int* dst = reinterpret_cast<int*>(bs + ((size_t)b * NT + (n >> 3)) * 32 + (n & 7) * 4) + (i & 1);
+                        dst[0] = v[u].x; dst[2] = v[u].y; dst[4] = v[u].z; dst[6] = v[u].w;
+                    }
+                }
             }
+            #pragma unroll 4
             for (int i = tid; i < nblk * N; i += W * 32) {
                 const int n = tt * N + i % N, b = i / N;
                 dxs[i] = n < p.M ? tok_scale_value(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(p.xd) + (size_t)n * p.nb + b0 + b))) : 0.0;
@@ -188,7 +203,7 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
             }
         }
     };
-    stage(k0 * KB, (min(k0 + p.kct, k1) - k0) * KB);
+    stage(k0 * kStepBlk, min(min(k0 + p.kct, k1) * kStepBlk, p.nb) - k0 * kStepBlk);
     if constexpr (ROWMAJOR) __syncthreads();
     bool ok = true, xready = ROWMAJOR;
 
@@ -216,7 +231,7 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
             if (nchunk > 1 && !first) {                                              // everyone has left the previous chunk: the next one over it
                 __syncthreads();
                 if constexpr (!ROWMAJOR) { if (warp == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-                stage(c0 * KB, (c1 - c0) * KB);
+                stage(c0 * kStepBlk, min(c1 * kStepBlk, p.nb) - c0 * kStepBlk);
                 if constexpr (ROWMAJOR) __syncthreads(); else xready = false;
             }
             first = false;
@@ -228,7 +243,13 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
                 for (; t < c1 && ok; t += kw) {
                     const int s = consumed % kRing;
                     if (!mbar_wait_bounded(&rbar[s], (consumed / kRing) & 1)) { ok = false; break; }
-                    tile_mma<KB, NT>(ring + (size_t)s * TB, bs + (size_t)(t - c0) * (KB * NT * 32), dxs + (size_t)(t - c0) * (KB * N), lane, acc, poison, pair);
+                    if constexpr (KB == kStepBlk) tile_mma<KB, NT>(ring + (size_t)s * TB, bs + (size_t)(t - c0) * (KB * NT * 32), dxs + (size_t)(t - c0) * (KB * N), lane, acc, poison, pair);
+                    else {
+                        const int nb = min(kStepBlk, p.nb - t * kStepBlk);
+                        #pragma unroll 1
+                        for (int k = 0; k < nb; k += KB)
+                            tile_mma<KB, NT>(ring + (size_t)s * TB + k * kTileRowBytes, bs + (size_t)((t - c0) * kStepBlk + k) * (NT * 32), dxs + (size_t)((t - c0) * kStepBlk + k) * N, lane, acc, poison, pair);
+                    }
                     consumed++;
                     __syncwarp();
                     if (lane == 0) issue_one();
@@ -305,15 +326,14 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
 // ---- host side -----------------------------------------------------------------------------------------------------
 
 namespace {
-struct SmemNeed { int ring_bars, fold, x_tile; };
-SmemNeed smem_need(int kb, int NT) {
-    switch (kb * 8 + NT) {
-        #define MI_F(kb, nt) case kb * 8 + nt: { using S = TokSmem<kb, nt, false>; using F = TokSmem<kb, nt, true>; return SmemNeed{S::fixed, F::fixed, S::x_tile}; }
-        MI_F(1, 1) MI_F(1, 2) MI_F(1, 3) MI_F(1, 4) MI_F(2, 1) MI_F(2, 2) MI_F(2, 3) MI_F(2, 4)
-        MI_F(4, 1) MI_F(4, 2) MI_F(4, 3) MI_F(4, 4) MI_F(8, 1) MI_F(8, 2) MI_F(8, 3) MI_F(8, 4)
+struct SmemNeed { int ring_bars, fold, x_step; };
+SmemNeed smem_need(int NT) {
+    switch (NT) {
+        #define MI_F(nt) case nt: return SmemNeed{TokSmem<nt, false>::fixed, TokSmem<nt, true>::fixed, TokSmem<nt, true>::x_step};
+        MI_F(1) MI_F(2) MI_F(3)
         #undef MI_F
     }
-    return SmemNeed{1 << 30, 1 << 30, 1};
+    return SmemNeed{TokSmem<4, false>::fixed, TokSmem<4, true>::fixed, TokSmem<4, true>::x_step};
 }
 }  // namespace
 
@@ -324,19 +344,20 @@ SmemNeed smem_need(int kb, int NT) {
 int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* out) {
     const TokTiling tl = tok_tiling(M);
     const int NT = tl.NT, TT = tl.TT, W = tok_warps(NT), N = NT * 8, U = mode == GEMM_GU ? 2 : 1, ntok = std::min(M, N);
-    const SmemNeed need = smem_need(w->kb, NT);
-    const double c_tile = w->kb * (45.0 + 76.0 * NT) + 100;
+    const SmemNeed need = smem_need(NT);
+    const int nt = (w->nb + kStepBlk - 1) / kStepBlk;                                     // steps of eight blocks
+    const double c_tile = kStepBlk * (45.0 + 76.0 * NT + (w->kb < 8 ? 30 : 0)) + 100;
     const double c_tok = mode == GEMM_GU ? 640 : mode == GEMM_QKV ? 300 : 60;             // end of a round, per token and warp
     double best = 1e300;
-    const int max_ksg = mode == GEMM_PART ? std::min(w->nt, 8) : 1;
+    const int max_ksg = mode == GEMM_PART ? std::min(nt, 8) : 1;
     for (int ksg = 1; ksg <= max_ksg; ksg++) {
-        const int ntr = (w->nt + ksg - 1) / ksg, cmax = std::max(1, ctx->sm_count / (ksg * TT));
+        const int ntr = (nt + ksg - 1) / ksg, cmax = std::max(1, ctx->sm_count / (ksg * TT));
         for (int v = 0; v <= W; v++) {                                                // 0: warps alone; else v warps per row group, sums through shared memory
             const bool fold = v > 0;
             const int kw = std::max(1, v), rg = W / kw;
             if (fold ? (v == 1 && U == 1) || rg % U || W / rg != kw : U == 2 || mode == GEMM_QKV) continue;   // pairs stay together; no warps idle by rounding
             const int fixed = fold ? need.fold : need.ring_bars;
-            const int fit = (ctx->smem_optin - kStaticSmem - fixed) / need.x_tile;
+            const int fit = (ctx->smem_optin - kStaticSmem - fixed) / need.x_step;
             if (fit < 1) continue;
             const int kct = std::min(ntr, fit), nchunk = (ntr + kct - 1) / kct;
             const int nsets = fold ? (w->groups + rg - 1) / rg : w->groups, C = std::min(nsets, cmax);
@@ -353,7 +374,7 @@ int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* ou
             cost = waves * (cost + 600 + (nchunk > 1 ? rounds * nchunk * 1500.0 : 0.0)) + (mode == GEMM_PART ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
             if (cost < best) {
                 best = cost;
-                *out = GemmPlan{NT, TT, ksg, kct, C, kw, fold, (size_t)fixed + (size_t)kct * need.x_tile};
+                *out = GemmPlan{NT, TT, ksg, kct, C, kw, fold, (size_t)fixed + (size_t)kct * need.x_step};
             }
         }
     }
@@ -406,7 +427,7 @@ int launch_nt(mi_ctx* ctx, const GemmPlan& pl, int mode, bool rowmajor, const Ge
 }  // namespace
 
 int launch_gemm_tok(mi_ctx* ctx, const mi_weight* w, const GemmPlan& pl, int mode, bool rowmajor, GemmParams p, bool pdl) {
-    p.base = w->dev; p.groups = w->groups; p.nt = w->nt; p.nb = w->nb; p.rows = (int)w->rows;
+    p.base = w->dev; p.groups = w->groups; p.nt = (w->nb + kStepBlk - 1) / kStepBlk; p.nb = w->nb; p.rows = (int)w->rows;
     p.ksg = pl.ksg; p.kct = pl.kct; p.C = pl.C; p.kw = pl.kw; p.err = ctx->d_err;
     switch (w->kb) {
         case 8: return launch_nt<8>(ctx, pl, mode, rowmajor, p, pdl);

@@ -90,8 +90,8 @@ __device__ __forceinline__ float swiglu(float gate, float up) {
 #endif
 
 struct GemmParams {
-    const uint8_t* base; int groups, nt, nb, rows;      // tiled weights
-    int ksg, kct, C, kw;                                // K ranges of the grid; tiles per staged chunk; CTAs per (range, token tile); warps that share a unit's K tiles
+    const uint8_t* base; int groups, nt, nb, rows;      // tiled weights; nt: steps of eight blocks
+    int ksg, kct, C, kw;                                // K ranges of the grid; steps per staged chunk; CTAs per (range, token tile); warps that share a unit's steps
     int M;                                              // tokens
     TokX x;                                             // activations in operand order, or
     const int8_t* xq; const __half* xd;                 // row-major: [M][nb*32], [M][nb]

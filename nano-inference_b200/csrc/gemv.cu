@@ -39,55 +39,63 @@ gemv_q4_q8_kernel(const __grid_constant__ GemvShape sh, const __grid_constant__ 
 
 // The GEMV where the streaming kernel above would have too few row groups for its warps: one CTA per row group, its warps take
 // the K tiles (lane = row, as there) and meet in shared memory.  What bounds these sizes is latency - a matrix is 0.1 - 4 us of
-// HBM time - so a warp's first tile is requested straight into registers (nine 16-byte loads per lane, each a contiguous 512
-// bytes per warp) before the kernel waits for its predecessor, each warp stages only the activations of its own tile, and several
+// HBM time - so a warp's first eight blocks are requested straight into registers (nine 16-byte loads per lane, each a contiguous
+// 512 bytes per warp) before the kernel waits for its predecessor, each warp stages only the activations of its own tile, and several
 // CTAs share an SM instead of a loop.  The streaming kernel reached these sizes by splitting K over the grid: partial sums, fence,
 // atomic and a second read in global memory, 14 us of the 17 that quantizing and multiplying an 11008 x 2048 matrix took.
 template <int KB, int W>
 __global__ void __launch_bounds__(W * 32) gemv_q4_q8_fold_kernel(const __grid_constant__ GemvShape sh, const __grid_constant__ GemvIO io) {
     __shared__ double fold[W][32];
-    __shared__ __align__(16) int8_t xs_all[W][KB * 32];
-    __shared__ float2 sc_all[W][KB];
+    __shared__ __align__(16) int8_t xs_all[W][8 * 32];
+    __shared__ float2 sc_all[W][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = (int)blockIdx.x / sh.groups, g = (int)blockIdx.x - c * sh.groups;
     const uint8_t* base = sh.base + (size_t)c * sh.mat_stride + (size_t)g * sh.nt * tile_bytes(KB);
     int8_t* xs = xs_all[warp]; float2* sc = sc_all[warp];
-    uint4 wq[KB];
-    uint4 ws = make_uint4(0u, 0u, 0u, 0u);
-    auto load_tile = [&](int t) {
-        const uint8_t* tile = base + (size_t)t * tile_bytes(KB);
+    // a warp takes eight blocks at a time: a tile of eight, or consecutive smaller ones
+    constexpr int SB = 8;
+    const int nstep = (sh.nb + SB - 1) / SB;
+    uint4 wq[SB];
+    unsigned ws[SB / 2];                                  // fp16 scales, two per word
+    auto load_step = [&](int t) {
         #pragma unroll
-        for (int k = 0; k < KB; k++) wq[k] = __ldcs(reinterpret_cast<const uint4*>(tile) + k * 32 + lane);
-        const uint8_t* sp = tile + KB * 512 + lane * (KB * 2);
-        if constexpr (KB == 8) ws = __ldcs(reinterpret_cast<const uint4*>(sp));
-        else if constexpr (KB == 4) { const uint2 v = __ldcs(reinterpret_cast<const uint2*>(sp)); ws.x = v.x; ws.y = v.y; }
-        else if constexpr (KB == 2) ws.x = __ldcs(reinterpret_cast<const unsigned*>(sp));
-        else ws.x = __ldcs(reinterpret_cast<const unsigned short*>(sp));
+        for (int s = 0; s < SB / KB; s++) {
+            const uint8_t* tile = base + (size_t)min(t * SB + s * KB, sh.nb - KB) * kTileRowBytes;       // past the end: the last tile, not used
+            #pragma unroll
+            for (int k = 0; k < KB; k++) wq[s * KB + k] = __ldcs(reinterpret_cast<const uint4*>(tile) + k * 32 + lane);
+            const uint8_t* sp = tile + KB * 512 + lane * (KB * 2);
+            if constexpr (KB == 8) { const uint4 v = __ldcs(reinterpret_cast<const uint4*>(sp)); ws[0] = v.x; ws[1] = v.y; ws[2] = v.z; ws[3] = v.w; }
+            else if constexpr (KB == 4) { const uint2 v = __ldcs(reinterpret_cast<const uint2*>(sp)); ws[2 * s] = v.x; ws[2 * s + 1] = v.y; }
+            else if constexpr (KB == 2) ws[s] = __ldcs(reinterpret_cast<const unsigned*>(sp));
+            else if (s & 1) ws[s / 2] |= (unsigned)__ldcs(reinterpret_cast<const unsigned short*>(sp)) << 16;
+            else ws[s / 2] = __ldcs(reinterpret_cast<const unsigned short*>(sp));
+        }
     };
-    if (warp < sh.nt) load_tile(warp);                    // weights do not depend on any earlier kernel
+    if (warp < nstep) load_step(warp);                    // weights do not depend on any earlier kernel
     pdl_launch_dependents();
     pdl_wait_prior();                                     // activations do
     double acc = 0.0;
-    for (int t = warp; t < sh.nt; t += W) {
-        // the tile's activations: 16 bytes per lane, and per block {fp32 of the fp16 scale, float(8 * sum of the values)}
+    for (int t = warp; t < nstep; t += W) {
+        // the step's activations: 16 bytes per lane, and per block {fp32 of the fp16 scale, float(8 * sum of the values)}
+        const int nb = min(SB, sh.nb - t * SB);
         int s = 0;
-        if (lane < 2 * KB) {
-            const int4 x = __ldg(reinterpret_cast<const int4*>(io.xq + (size_t)t * KB * 32) + lane);
+        if (lane < 2 * nb) {
+            const int4 x = __ldg(reinterpret_cast<const int4*>(io.xq + (size_t)t * SB * 32) + lane);
             *reinterpret_cast<int4*>(xs + lane * 16) = x;
             s = __dp4a(0x01010101, x.x, 0); s = __dp4a(0x01010101, x.y, s); s = __dp4a(0x01010101, x.z, s); s = __dp4a(0x01010101, x.w, s);
         }
         s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if (lane < 2 * KB && !(lane & 1)) sc[lane >> 1] = make_float2(__half2float(__ldg(io.xd + t * KB + (lane >> 1))), __int2float_rn(8 * s));
+        if (lane < 2 * nb && !(lane & 1)) sc[lane >> 1] = make_float2(__half2float(__ldg(io.xd + t * SB + (lane >> 1))), __int2float_rn(8 * s));
         __syncwarp();
-        const unsigned wsv[4] = {ws.x, ws.y, ws.z, ws.w};
         #pragma unroll
-        for (int k = 0; k < KB; k++) {
+        for (int k = 0; k < SB; k++) {
+            if (k >= nb) break;                           // warp-uniform
             const int4 xa = *reinterpret_cast<const int4*>(xs + k * 32), xc = *reinterpret_cast<const int4*>(xs + k * 32 + 16);
             const float2 x2 = sc[k];
-            const float dw = __half2float(__ushort_as_half((unsigned short)(wsv[k / 2] >> (16 * (k & 1)))));
+            const float dw = __half2float(__ushort_as_half((unsigned short)(ws[k / 2] >> (16 * (k & 1)))));
             acc = blk_acc(acc, dw, x2.x, dot_q4_block(wq[k], xa, xc), x2.y);
         }
-        if (t + W < sh.nt) load_tile(t + W);
+        if (t + W < nstep) load_step(t + W);
         __syncwarp();
     }
     fold[warp][lane] = acc;
@@ -103,8 +111,9 @@ template <int KB>
 static int launch_fold(mi_ctx* ctx, const mi_weight* w, const GemvIO& io) {
     const GemvShape sh{w->dev, (long long)w->mat_stride, (int)w->count, w->groups, w->nt, 1, w->nb, (int)w->rows};
     const dim3 grid((unsigned)(w->count * w->groups));
-    if (w->nt <= 8) MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 8>, grid, dim3(256), 0, ctx->stream, sh, io));
-    else if (w->nt <= 16) MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 16>, grid, dim3(512), 0, ctx->stream, sh, io));
+    const int steps = (w->nb + 7) / 8;
+    if (steps <= 8) MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 8>, grid, dim3(256), 0, ctx->stream, sh, io));
+    else if (steps <= 16) MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 16>, grid, dim3(512), 0, ctx->stream, sh, io));
     else MI_CUDA(ctx, launch_k(true, gemv_q4_q8_fold_kernel<KB, 24>, grid, dim3(768), 0, ctx->stream, sh, io));
     return MI_OK;
 }
@@ -135,7 +144,8 @@ static int launch_one(mi_ctx* ctx, const mi_weight* w, const GemvIO& io, int ksp
         if (base_units < 2 * total_warps) ks = (int)((2 * total_warps + base_units - 1) / base_units);
         if (ks > 32) ks = 32;
     }
-    if (ks > w->nt) ks = w->nt;
+    const int slots = (w->nt + kSlotTiles<KB> - 1) / kSlotTiles<KB>;
+    if (ks > slots) ks = slots;
     if (DUMP) ks = 1;
     const long long n_units = base_units * ks;
     long long ctas = (n_units + NW - 1) / NW;

@@ -2,7 +2,7 @@
 // fused decode-step kernels.
 //
 // Work decomposition.  A "unit" is (matrix c, 32-row group g, K-split sp): the
-// tiles [sp*nt/ks, (sp+1)*nt/ks) of group g.  Units are dealt round-robin to
+// slots [sp*ns/ks, (sp+1)*ns/ks) of group g (a slot is one tile of eight blocks, or as many smaller ones).  Units are dealt round-robin to
 // the warps of a persistent grid.  Each warp owns a private ring of S tile
 // slots in shared memory; lane 0 keeps the ring full with plain single-CTA
 // cp.async.bulk copies (one contiguous tile per copy, completion counted on a
@@ -34,10 +34,15 @@ struct GemvScratch {
     unsigned* counters;       // [n_mats*groups] arrivals, zero between launches
 };
 
+// Tiles per ring slot: the tiles of a row group are contiguous, so shallow ones (cols / 32 not a multiple of 8) travel several
+// per bulk copy - at one 576-byte tile per copy and three copies in flight per warp the stream ran at a third of the HBM rate.
+template <int KB> constexpr int kSlotTiles = 8 / KB;
+__device__ __forceinline__ int slot_count(int nt, int per) { return (nt + per - 1) / per; }
+
 // Shared-memory carve-up of a GEMV CTA.
 template <int KB, int NW, int S>
 struct GemvSmem {
-    static constexpr int TB = tile_bytes(KB);
+    static constexpr int TB = tile_bytes(8);
     static constexpr int ring_bytes = NW * S * TB;
     static constexpr int bar_bytes = ((NW * S * 8) + 15) / 16 * 16;
     __host__ __device__ static constexpr size_t bytes(int nb) { return (size_t)ring_bytes + bar_bytes + (size_t)nb * 32 + (size_t)nb * 8; }
@@ -50,7 +55,7 @@ struct GemvSmem {
 // Position of a warp in its own tile sequence.
 struct TileCursor {
     long long u;          // current unit (>= n_units: exhausted)
-    int t, t1;            // next tile and end tile within the unit's group
+    int t, t1;            // next slot (kSlotTiles tiles) and end slot within the unit's group
     int c, g, sp;         // matrix, group, split of the unit
     const uint8_t* gbase; // first tile of (c, g)
 };
@@ -63,8 +68,9 @@ __device__ __forceinline__ void cursor_set(TileCursor& cu, long long u, long lon
     const long long gg = u / sh.ks;
     cu.g = (int)(gg % sh.groups);
     cu.c = (int)(gg / sh.groups);
-    cu.t = (int)((long long)cu.sp * sh.nt / sh.ks);
-    cu.t1 = (int)((long long)(cu.sp + 1) * sh.nt / sh.ks);
+    const int ns = slot_count(sh.nt, kSlotTiles<KB>);
+    cu.t = (int)((long long)cu.sp * ns / sh.ks);
+    cu.t1 = (int)((long long)(cu.sp + 1) * ns / sh.ks);
     cu.gbase = sh.base + (size_t)cu.c * sh.mat_stride + (size_t)cu.g * sh.nt * tile_bytes(KB);
 }
 
@@ -163,8 +169,9 @@ struct GemvWarp {
     __device__ __forceinline__ void issue_one(const GemvShape& sh) {
         if (pc.u >= n_units) return;
         const int slot = issued % S;
-        mbar_expect_tx(&bars[slot], TB);
-        bulk_g2s_hint(ring + (size_t)slot * TB, pc.gbase + (size_t)pc.t * TB, TB, &bars[slot], policy);
+        const int bytes = min(kSlotTiles<KB>, sh.nt - pc.t * kSlotTiles<KB>) * tile_bytes(KB);
+        mbar_expect_tx(&bars[slot], bytes);
+        bulk_g2s_hint(ring + (size_t)slot * TB, pc.gbase + (size_t)pc.t * TB, bytes, &bars[slot], policy);
         issued++;
         if (++pc.t == pc.t1) cursor_set<KB>(pc, pc.u + stride, n_units, sh);
     }
@@ -184,7 +191,10 @@ struct GemvWarp {
             for (int t = cc.t; t < cc.t1; t++) {
                 const int slot = consumed % S;
                 if (!mbar_wait_bounded(&bars[slot], (consumed / S) & 1)) { ok = false; break; }
-                acc = tile_dot_row<KB, DUMP>(ring + (size_t)slot * TB, lane, t * KB, xq_s, xs_s, acc, isum_row);
+                const int n = min(kSlotTiles<KB>, sh.nt - t * kSlotTiles<KB>);
+                #pragma unroll 1
+                for (int s = 0; s < n; s++)
+                    acc = tile_dot_row<KB, DUMP>(ring + (size_t)slot * TB + s * tile_bytes(KB), lane, (t * kSlotTiles<KB> + s) * KB, xq_s, xs_s, acc, isum_row);
                 consumed++;
                 __syncwarp();                       // every lane is done with the slot before it is refilled
                 if (lane == 0) issue_one(sh);
