@@ -15,6 +15,7 @@ from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 LIB_PATH = PKG_DIR / "lib" / "libminfer_b200.so"
+FAST_PATH = PKG_DIR / "lib" / "minfer_fastcall.so"
 BIN_DIR = PKG_DIR / "bin"
 
 MI_OK = 0
@@ -29,6 +30,7 @@ class MinferError(RuntimeError):
 
 
 _lib = None
+_fast = None             # lib/minfer_fastcall.so: the per-matrix calls without ctypes' argument conversion
 
 _vp, _i32, _i64 = C.c_void_p, C.c_int, C.c_int64
 # name -> (restype, argtypes); every symbol include/minfer_b200.h declares
@@ -130,6 +132,18 @@ def load_library(path=None):
     return lib
 
 
+def _load_fastcall():
+    global _fast
+    if _fast is None:
+        import importlib.util
+        if not FAST_PATH.exists():
+            raise FileNotFoundError(f"{FAST_PATH} not built: run `python nano-inference_b200/build.py`")
+        spec = importlib.util.spec_from_file_location("minfer_fastcall", FAST_PATH)
+        _fast = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_fast)
+    return _fast
+
+
 def detok_piece(piece):
     """Text bytes of one vocabulary piece of a byte-level BPE tokenizer (bytes or str in, bytes out).  Host only."""
     raw = piece.encode("utf-8") if isinstance(piece, str) else bytes(piece)
@@ -158,12 +172,14 @@ class Context:
 
     def __init__(self, device=0):
         self.lib = load_library()
-        self._quant_q8, self._gemv_q4_q8, self._gemm_q4_q8 = self.lib.mi_quant_q8, self.lib.mi_gemv_q4_q8_ex, self.lib.mi_gemm_q4_q8
+        fast = _load_fastcall()
+        self._quant_q8, self._gemv_q4_q8, self._gemm_q4_q8 = fast.quant_q8, fast.gemv_q4_q8, fast.gemm_q4_q8
         h = _vp()
         st = self.lib.mi_ctx_create(device, C.byref(h))
         if st != MI_OK:
             raise MinferError(st, "mi_ctx_create", "(no usable sm_100 CUDA device?)")
         self.h = h
+        self._addr = h.value
         self.device = device
 
     def check(self, st, where):
@@ -173,7 +189,7 @@ class Context:
     def close(self):
         if getattr(self, "h", None):
             self.lib.mi_ctx_destroy(self.h)
-            self.h = None
+            self.h = self._addr = None
 
     def __del__(self):
         try:
@@ -231,12 +247,12 @@ class Context:
     # ---- kernels (device pointers: torch CUDA tensors)
     # (these are called per matrix by programs that own the layer loop: a microsecond here is a microsecond per product)
     def quant_q8(self, x, xq, xd, n=None, M=1):
-        st = self._quant_q8(self.h, _ptr(x), x.shape[-1] if n is None else n, M, _ptr(xq), _ptr(xd))
+        st = self._quant_q8(self._addr, x, xq, xd, n, M)
         if st:
             self.check(st, "mi_quant_q8")
 
     def gemv_q4_q8(self, w, xq, xd, y, bias=None, ksplit=0, variant=0):
-        st = self._gemv_q4_q8(self.h, w.h, _ptr(xq), _ptr(xd), None if bias is None else _ptr(bias), _ptr(y), ksplit, variant)
+        st = self._gemv_q4_q8(self._addr, w.addr, xq, xd, bias, y, ksplit, variant)
         if st:
             self.check(st, "mi_gemv_q4_q8")
 
@@ -246,7 +262,7 @@ class Context:
 
     def gemm_q4_q8(self, w, xq, xd, M, y, bias=None):
         """M token vectors per weight pass on the tensor cores; y is [M][rows]."""
-        st = self._gemm_q4_q8(self.h, w.h, _ptr(xq), _ptr(xd), M, None if bias is None else _ptr(bias), _ptr(y))
+        st = self._gemm_q4_q8(self._addr, w.addr, xq, xd, M, bias, y)
         if st:
             self.check(st, "mi_gemm_q4_q8")
 
@@ -266,7 +282,7 @@ class Weight:
     """A q4_0 matrix stack in the tiled device layout: wraps mi_weight."""
 
     def __init__(self, ctx, h):
-        self.ctx, self.h = ctx, h
+        self.ctx, self.h, self.addr = ctx, h, h.value
         r, c, n, b = _i64(), _i64(), _i64(), _i64()
         ctx.lib.mi_weight_info(h, C.byref(r), C.byref(c), C.byref(n), C.byref(b))
         self.rows, self.cols, self.count, self.device_bytes = r.value, c.value, n.value, b.value
@@ -277,7 +293,7 @@ class Weight:
     def free(self):
         if self.h and self.ctx.h:
             self.ctx.lib.mi_weight_free(self.ctx.h, self.h)
-        self.h = None
+        self.h = self.addr = None
 
     def __del__(self):
         try:

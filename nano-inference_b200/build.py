@@ -4,6 +4,7 @@
 
 Outputs (all git-ignored, next to the sources so that they travel with the tree):
     nano-inference_b200/lib/libminfer_b200.so     CUDA kernels + C ABI
+    nano-inference_b200/lib/minfer_fastcall.so    argument passing of the per-matrix calls for the Python binding
     nano-inference_b200/bin/gguf_synth            synthetic model writer
     nano-inference_b200/bin/cuda_infer, mega      driver programs (same command line as the reference's)
 """
@@ -13,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -87,6 +89,11 @@ def build_host(force=False, verbose=False):
     if force or _newer(synth, [HOST / "gguf_synth.cpp"]):
         _run([GXX, "-O2", "-std=c++17", "-pthread", "-o", synth, HOST / "gguf_synth.cpp"], verbose)
     out.append(synth)
+    fast = LIB.parent / "minfer_fastcall.so"
+    if force or _newer(fast, [HOST / "fastcall.cpp", LIB, ROOT / "include" / "minfer_b200.h"]):
+        _run([GXX, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-I", ROOT / "include", "-o", fast,
+              HOST / "fastcall.cpp", "-L", LIB.parent, "-lminfer_b200", "-Wl,-rpath,$ORIGIN"], verbose)
+    out.append(fast)
     for name in ("cuda_infer", "mega"):
         src = HOST / f"{name}.cpp"
         if not src.exists():

@@ -101,6 +101,9 @@ extern "C" int mi_ctx_create(int device, mi_ctx** out) {
     if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess || cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) {
         cudaStreamDestroy(ctx->own_stream); delete ctx; return MI_ERR_NOMEM;
     }
+    if (cudaMallocHost(&ctx->h_io, kHostIoWords * sizeof(int)) != cudaSuccess) {
+        cudaFree(ctx->d_err); cudaStreamDestroy(ctx->own_stream); delete ctx; return MI_ERR_NOMEM;
+    }
     *out = ctx;
     return MI_OK;
 }
@@ -114,6 +117,7 @@ extern "C" int mi_ctx_destroy(mi_ctx* ctx) {
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->h_io) cudaFreeHost(ctx->h_io);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return MI_OK;
@@ -127,9 +131,10 @@ extern "C" int mi_ctx_set_stream(mi_ctx* ctx, void* cuda_stream) {
 
 extern "C" int mi_ctx_sync(mi_ctx* ctx) {
     if (!ctx) return MI_ERR_INVALID;
+    // the error word travels in stream order into pinned memory: one wait for the stream, not a wait and a synchronous copy behind it
+    MI_CUDA(ctx, cudaMemcpyAsync(ctx->h_io, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    int err = 0;
-    MI_CUDA(ctx, cudaMemcpy(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    const int err = ctx->h_io[0];
     if (err != 0) {
         // a kernel that gave up may have left the self-resetting arrival counters of the split-K GEMV partly counted
         ctx->errors_reported++;

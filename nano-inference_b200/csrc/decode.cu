@@ -752,10 +752,13 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
     if (async) return MI_OK;                          // the caller follows the ring and synchronizes itself
     std::vector<int32_t> scan;
     if (stop >= 0 && !out_tokens_host) { scan.resize((size_t)n_steps); out_tokens_host = scan.data(); }
+    // (a copy to pageable memory waits for the stream by itself: short runs go through the context's pinned words, with one wait)
+    const bool staged = n_steps <= kHostIoWords - kHostIoResult;
     if (out_tokens_host)
-        MI_CUDA(ctx, cudaMemcpyAsync(out_tokens_host, m->d_out_tokens, (size_t)n_steps * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        MI_CUDA(ctx, cudaMemcpyAsync(staged ? ctx->h_io + kHostIoResult : out_tokens_host, m->d_out_tokens, (size_t)n_steps * 4, cudaMemcpyDeviceToHost, ctx->stream));
     st = mi_ctx_sync(ctx);
     if (st != MI_OK) return st;
+    if (out_tokens_host && staged) memcpy(out_tokens_host, ctx->h_io + kHostIoResult, (size_t)n_steps * 4);
     if (stop >= 0 && mode == MI_DECODE_PERSISTENT)    // the kernel ended the run after the first consumed prediction equal to the stop token
         for (int s = std::max(n_forced - 1, 0); s < n_steps; s++)
             if (out_tokens_host[s] == stop) { m->last_count = s + 1; break; }

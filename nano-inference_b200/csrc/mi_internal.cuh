@@ -9,6 +9,8 @@
 
 // ---- host-side objects behind the opaque C handles ---------------------------
 
+constexpr int kHostIoResult = 16, kHostIoWords = 1024;     // words of mi_ctx::h_io: where results start, all
+
 struct mi_ctx {
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -16,6 +18,7 @@ struct mi_ctx {
     int sm_count = 0;
     int smem_optin = 0;
     int* d_err = nullptr;            // device error word (0 = none)
+    int* h_io = nullptr;             // pinned: [0] the error word as read back by mi_ctx_sync, [kHostIoResult..] results on their way to a caller's pageable memory
     unsigned long long wait_ns = 2000000000ull;   // time budget of the decode kernel's device-side waits (mi_ctx_set_wait_budget_ns)
     unsigned long long errors_reported = 0;       // device errors that mi_ctx_sync has reported so far
     // scratch of the split-K GEMV: partial sums and self-resetting arrival counters

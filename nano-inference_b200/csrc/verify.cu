@@ -512,12 +512,11 @@ extern "C" int mi_batch_step(mi_ctx* ctx, mi_batch* b, int n, const int32_t* tok
         MI_CUDA(ctx, cudaMemcpyAsync(vb.meta, vb.h_meta, (size_t)3 * M * 4, cudaMemcpyHostToDevice, ctx->stream));
         if ((st = run_pass(ctx, m, Pass{M, true, b->kc, b->vc, b->max_seq, b->slab_stride, lp_max, HEAD_ALL}))) return st;
         if (logits_dev) MI_CUDA(ctx, cudaMemcpyAsync(logits_dev + (size_t)i0 * m->V, vb.logits, (size_t)M * m->V * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-        if (out_tokens_host) MI_CUDA(ctx, cudaMemcpyAsync(out_tokens_host + i0, vb.out, (size_t)M * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        if (i0 + BMAX < n) MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));       // the pinned block is filled again by the next pass
+        if (i0 + BMAX >= n) MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
+        if (out_tokens_host) MI_CUDA(ctx, cudaMemcpyAsync(vb.h_meta, vb.out, (size_t)M * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        if ((st = mi_ctx_sync(ctx))) return st;                                    // (the pinned block is filled again by the next pass)
+        if (out_tokens_host) memcpy(out_tokens_host + i0, vb.h_meta, (size_t)M * 4);
     }
-    MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
-    st = mi_ctx_sync(ctx);
-    if (st != MI_OK) return st;
     if (elapsed_ms) MI_CUDA(ctx, cudaEventElapsedTime(elapsed_ms, m->ev0, m->ev1));
     return MI_OK;
 }
