@@ -20,7 +20,6 @@ const void* decode_kernel_prof(int HD, int G); const void* decode_kernel_tp(int 
 const void* decode_kernel_prof_lean(int HD, int G);
 const void* decode_kernel_tp_lean(int HD, int G);
 const void* decode_kernel_tp_prof_lean(int HD, int G);
-const void* decode_kernel_lean_mid(int HD, int G);
 const void* decode_kernel_lean_long(int HD, int G);
 }
 
@@ -102,8 +101,8 @@ __global__ void rope_cs_kernel(const float* __restrict__ freq, float* __restrict
     cs[(size_t)pos * HD + HD / 2 + i] = __double2float_rn(sin(th));
 }
 
-// range_hint 1 / 2 / 3: the caller vouches that every position of the launch lies in that context range (up to kShortAttnMax,
-// up to kPerHeadAttnMax, beyond) although the position is device-resident; 0: decided from pos0 and the steps.  (A build
+// range_hint 1 / 2: the caller vouches that every position of the launch lies in that context range (up to kShortAttnMax,
+// beyond) although the position is device-resident; 0: decided from pos0 and the steps.  (A build
 // launched outside its range ends with MI_ERR_LIMIT on every CTA, it computes nothing wrong.)  only_prepare: pick the
 // kernel and raise its shared-memory limit, launch nothing (what must not happen inside a stream capture).
 int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, int step1, int ph0, int ph1, bool coop, int range_hint = 0,
@@ -117,8 +116,7 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
     auto as_kernel = [](const void* p) { return reinterpret_cast<void (*)(DecodeParams, int, int, int, int)>(const_cast<void*>(p)); };
     // the context-range builds are instantiated for the head shapes that occur with the embedding widths they take; a
     // null pointer from their pickers means "not built for this head shape": the general build of the same family runs
-    const bool mid = shape_ok && (range_hint == 2 || (by_pos && (long long)P.pos0 + step0 + 1 > kShortAttnMax && (long long)P.pos0 + step1 <= kPerHeadAttnMax));
-    const bool far = shape_ok && (range_hint == 3 || (by_pos && (long long)P.pos0 + step0 + 1 > kPerHeadAttnMax));
+    const bool far = shape_ok && (range_hint == 2 || (by_pos && (long long)P.pos0 + step0 + 1 > kShortAttnMax));
     const void* pick = nullptr;
     if (P.tp.on) {                                  // the builds with the exchange between GPUs inside (decode_tp.cu, decode_tp_lean.cu)
         if (lean && P.prof) pick = decode_kernel_tp_prof_lean(m->HD, m->G);
@@ -129,7 +127,6 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
         if (!pick) pick = decode_kernel_prof(m->HD, m->G);
     } else {
         if (lean) pick = decode_kernel_lean(m->HD, m->G);
-        else if (mid) pick = decode_kernel_lean_mid(m->HD, m->G);
         else if (far) pick = decode_kernel_lean_long(m->HD, m->G);
     }
     if (pick) kern = as_kernel(pick);
@@ -460,13 +457,14 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         x.down = take((E + 31) / 32 * 32);
         x.dpart = take((E + 31) / 32 * (kMaxKSplit - 1) * 64);
         x.cand = take(kMaxWorldTP * m->grid * 4);
+        x.attm = take(m->NH * m->max_chunks);
         x.tokw = take(2);
         x.total = off;
     }
     if ((st = dev_alloc(ctx, m, &P.h_in, E)) || (st = dev_alloc(ctx, m, &P.h_mid, E)) || (st = dev_alloc(ctx, m, &P.att, NQ)) ||
         (st = dev_alloc(ctx, m, &P.xw, (size_t)P.xo.total)) ||
         (st = dev_alloc(ctx, m, &P.kc, (size_t)L * max_seq * KVD)) || (st = dev_alloc(ctx, m, &P.vc, (size_t)L * max_seq * KVD)) ||
-        (st = dev_alloc(ctx, m, &P.attn_part, (size_t)m->NH * m->max_chunks * (HD + 2))) || (st = dev_alloc(ctx, m, &P.attn_cnt, m->NH)) ||
+        (st = dev_alloc(ctx, m, &P.attn_part, (size_t)m->NH * m->max_chunks * (HD + 2))) ||
         (st = dev_alloc(ctx, m, &P.prof, kProfSlots)) || (st = dev_alloc(ctx, m, &m->best_buf, 2)) ||
         (st = dev_alloc(ctx, m, &m->d_pos, 2)))
         return st;
@@ -484,9 +482,9 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     P.max_seq = max_seq; P.max_chunks = m->max_chunks; P.err = ctx->d_err;
     m->prof_buf = P.prof;
     if (!getenv("MINFER_PROFILE")) P.prof = nullptr;         // the buffer exists either way; kernels only write it when asked
-    m->smem = decode_smem_bytes((int)m->jobs.size(), E, FF, HD, m->G);
+    m->smem = decode_smem_bytes((int)m->jobs.size(), E, FF, HD);
     if (m->attn_ctas > 0) {
-        const int hpc = (m->G % 2 == 0 && m->G > 2) ? m->G / 2 : (m->G <= 2 ? 1 : m->G);
+        const int hpc = attn_heads_per_cta(m->G);
         m->smem = std::max(m->smem, attn_dedicated_smem(HD, hpc));       // the attention CTAs lay the same allocation out their own way
     }
     if (m->smem > (size_t)ctx->smem_optin)
@@ -695,16 +693,14 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
     const int nph = 5 * m->L + 1;
     MI_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
     if (mode == MI_DECODE_PERSISTENT) {
-        // One launch, or one per context range the steps pass through (up to kShortAttnMax positions, up to kPerHeadAttnMax,
+        // One launch, or one per context range the steps pass through (up to kShortAttnMax positions,
         // beyond): each range has a build of the kernel with only its attention variant (dispatch_launch picks by the
         // launch's positions), a launch that straddles a boundary would fall back to the general build.  Under the stop
         // rule the host cannot know whether an earlier launch ended the run, so the run stays one launch.
-        int cuts[4] = {0, 0, 0, n_steps}, nc = 1;
+        int cuts[3] = {0, 0, n_steps}, nc = 1;
         if (stop < 0 && !P.tp.on && lean_shape_ok(m->E, m->FF, m->NH * m->HD)) {
-            for (int edge : {kShortAttnMax, kPerHeadAttnMax}) {
-                const long long s = (long long)edge - pos0;            // first step whose position count exceeds the edge
-                if (s > cuts[nc - 1] && s < n_steps) cuts[nc++] = (int)s;
-            }
+            const long long s = (long long)kShortAttnMax - pos0;       // first step whose position count exceeds the edge
+            if (s > 0 && s < n_steps) cuts[nc++] = (int)s;
         }
         cuts[nc] = n_steps;
         for (int i = 0; i < nc; i++) {
@@ -716,9 +712,9 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
     } else if (mode == MI_DECODE_PER_PHASE && !logits_dev && stop < 0 && !ring && ph0 == 0 && ph1 == nph && m->tp_world == 1 && P.drop_phase < 0 && !P.prof &&
                !getenv("MINFER_SEQ_NO_GRAPH")) {
         // whole steps, nothing to look at between them: the captured step, replayed per token
-        cudaGraphExec_t gx[4] = {nullptr, nullptr, nullptr, nullptr};
+        cudaGraphExec_t gx[3] = {nullptr, nullptr, nullptr};
         for (int s = 0; s < n_steps; s++) {             // every graph this run needs exists before the first replay
-            const int range = pos0 + s + 1 <= kShortAttnMax ? 1 : pos0 + s + 1 <= kPerHeadAttnMax ? 2 : 3;
+            const int range = pos0 + s + 1 <= kShortAttnMax ? 1 : 2;
             if (!gx[range] && (st = step_graph(ctx, m, range, &gx[range]))) return st;
         }
         const SeqCtl ctl{m->d_in_tokens, m->d_out_tokens, m->d_margins, n_forced, 0};
@@ -727,7 +723,7 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
         MI_CUDA(ctx, cudaGetLastError());
         MI_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));         // (the timed region starts after the set-up above)
         for (int s = 0; s < n_steps; s++) {
-            const int range = pos0 + s + 1 <= kShortAttnMax ? 1 : pos0 + s + 1 <= kPerHeadAttnMax ? 2 : 3;
+            const int range = pos0 + s + 1 <= kShortAttnMax ? 1 : 2;
             MI_CUDA(ctx, cudaGraphLaunch(gx[range], ctx->stream));
         }
     } else if (mode == MI_DECODE_PER_PHASE) {
@@ -935,7 +931,6 @@ static int launch_phases(mi_ctx* ctx, mi_model* m, int pos, int phase_begin, int
 int mi::reset_after_error(mi_ctx* ctx, mi_model* m) {
     if (m->errors_seen == ctx->errors_reported) return MI_OK;
     m->errors_seen = ctx->errors_reported;
-    MI_CUDA(ctx, cudaMemsetAsync(m->P.attn_cnt, 0, m->NH * sizeof(unsigned), ctx->stream));
     if (m->vb.pick_cnt) MI_CUDA(ctx, cudaMemsetAsync(m->vb.pick_cnt, 0, m->vb.cap_logits * sizeof(unsigned), ctx->stream));
     return MI_OK;
 }

@@ -79,13 +79,12 @@
 #define MI_ATTN_HPC_EVEN(G) 2
 #endif
 
-// The kernel exists in four builds.  The default one carries no profiling code and no peer stores.  A translation unit
+// The kernel exists in several builds.  The default one carries no profiling code and no peer stores.  A translation unit
 // that defines MI_PROF 1 before including this file gets the instrumented build (timer marks between the hot instructions
 // cost a few percent when merely compiled in); MI_TP 1 gives the tensor-parallel build, whose publishing stores also go to
-// the other GPUs; MI_LEAN 2 and 3 are the same idea for 257..kPerHeadAttnMax positions (one query head per CTA and chunk) and
-// beyond (a whole GQA group per CTA and chunk): one attention variant each; MI_LEAN 1 gives the short-context build, which holds no attention code but that of the dedicated
-// attention CTAs (launched only for step ranges that end within kShortAttnMax positions on a model with such CTAs: without
-// the other attention variants in the same function the GEMV CTAs' loop keeps its values in registers).  They live in
+// the other GPUs; MI_LEAN 1 gives the short-context build, which holds no attention code but that of the dedicated attention CTAs (launched only for step ranges that end within kShortAttnMax positions on a model with such CTAs: without
+// the other attention variants in the same function the GEMV CTAs' loop keeps its values in registers); MI_LEAN 2 is the same idea for more than kShortAttnMax
+// positions (attention_split).  They live in
 // different inline namespaces, so all can be linked into one library and picked at launch time.
 #ifndef MI_PROF
 #define MI_PROF 0
@@ -107,8 +106,6 @@
 #elif MI_TP
 #define MI_KVARIANT tpx
 #elif MI_LEAN == 2
-#define MI_KVARIANT leanmid
-#elif MI_LEAN == 3
 #define MI_KVARIANT leanlong
 #elif MI_LEAN
 #define MI_KVARIANT lean
@@ -122,9 +119,8 @@ constexpr int DNW = 8;            // warps per CTA
 constexpr int DNT = DNW * 32;
 constexpr int DS = 3;             // ring slots per warp
 constexpr int DSLOT = 4608;       // bytes per slot: the largest tile (8 blocks)
-constexpr int kAttnChunk = 64;    // smallest KV range worth its own CTA
+constexpr int kAttnChunk = 32;    // smallest KV range worth its own CTA
 constexpr int kShortAttnMax = 256;      // up to this many cached positions one CTA handles the whole range of a query head (attention_short)
-constexpr int kPerHeadAttnMax = 1024;   // up to this many cached positions a CTA handles one query head, beyond it a whole GQA group
 constexpr int kMaxKSplit = 4;     // cross-CTA K-splits of the down projection
 constexpr int kMaxWorldTP = 8;
 
@@ -165,6 +161,7 @@ struct XwLayout {
     int down;       // [E] fp32 bits: down projection                                    (pushed)
     int dpart;      // [E/32][kMaxKSplit-1][32][2]: double partial sums (lo, hi) of the down K-splits 1..
     int cand;       // [kMaxWorldTP][grid][4]: argmax candidates {best value}, {its row}, {second-best value}, -   (pushed)
+    int attm;       // [NH][max_chunks] fp32 bits: maximum of every chunk of the long-range attention
     int tokw;       // [2]: the token picked by the step that just ended, for the attention CTAs (written only under a stop rule)
     int total;
 };
@@ -202,7 +199,7 @@ struct DecodeParams {
     int drop_phase;                  // test hook: the producers of this phase publish nothing (-1: none), so that its consumers' waits run out
     float* att;                      // merged attention output, fp32, for inspection
     __half* kc; __half* vc; int max_seq;       // [L][max_seq][KVD]
-    double* attn_part; unsigned* attn_cnt; int max_chunks;  // [NH][max_chunks][HD+2], [NKV]
+    double* attn_part; int max_chunks;       // [NH][max_chunks][HD+2]: weighted sums and denominator of every chunk (attention_split)
     float* out_margins;              // optional [n_steps]: top-1 minus top-2 logit of every step
     TokenRing ring;                  // optional: host-mapped ring the first GEMV CTA publishes every step's token into
     float* best_val;                 // value of the best logit (tensor parallelism with host-side exchange: this GPU's rows only)
@@ -239,15 +236,25 @@ struct DecodeSmem {
 
 constexpr int kFoldBytes = 2 * DNW * 2 * 32 * 8;      // two buffers of [warp][acc][lane] doubles
 
-__host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD, int G) {
+// attention_split: positions per step, words of chunk maxima a lane polls (up to 160 chunks per kv head), layout of its staging area
+constexpr int kSplitSub = 64, kMaxChunkWords = 5;
+template <int HD> struct SplitSmem {
+    static constexpr int KLD = 2 * HD + 64, VLD = 2 * HD + 32, SCL = kSplitSub + 4;       // row strides: fragment loads without bank conflicts
+    static constexpr int q = 0, wt = 8 * HD * 8, k = wt + 8 * kSplitSub * 8, v = k + kSplitSub * KLD, sc = v + kSplitSub * VLD, st = sc + 8 * SCL * 4,
+                         red = st + 8 * 3 * 8, bytes = red + DNW * 33 * 8;
+};
+
+__host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD) {
     const int maxin = E > FF ? E : FF;
     size_t a = (size_t)maxin + (size_t)(maxin / 32) * 8;               // xq, xs
-    size_t b = (size_t)DNW * G * (HD + 2) * 8 + (size_t)DNW * 32 * G * 8 + (size_t)G * (HD + 16) * 8;   // attention: states, weights, q (double, padded)
+    const size_t split = HD == 128 ? SplitSmem<128>::bytes : HD == 64 ? SplitSmem<64>::bytes : SplitSmem<32>::bytes;
+    const size_t shrt = (size_t)(8 * (HD / 8 + 2) + 256 + DNW * HD + DNW) * 8 + 1024;                // attention_short
+    const size_t b = split > shrt ? split : shrt;
     return ((a > b ? a : b) + 127) / 128 * 128;
 }
-__host__ __device__ inline size_t decode_smem_bytes(int njobs, int E, int FF, int HD, int G) {
+__host__ __device__ inline size_t decode_smem_bytes(int njobs, int E, int FF, int HD) {
     return (size_t)DNW * DS * DSLOT + 256 + ((size_t)njobs * sizeof(Job) + 127) / 128 * 128 + 64 * sizeof(LayerPtrs) + 1024 + 256 + kFoldBytes +
-           ((size_t)E * 4 + 127) / 128 * 128 + decode_stage_bytes(E, FF, HD, G);
+           ((size_t)E * 4 + 127) / 128 * 128 + decode_stage_bytes(E, FF, HD);
 }
 
 // close the current profile interval: charge the time since t to slot k (CTA 0, thread 0 only).
@@ -805,310 +812,248 @@ inline bool lean_shape_ok(int E, int FF, int NQ) {
     return E > 1024 && E <= 2048 && kb8(E) && kb8(FF) && kb8(NQ) && np(FF) <= 8 && np(NQ) <= 8;
 }
 
-// ---- attention --------------------------------------------------------------------
-// CTA = (kv head, chunk of the causal range); its warps split the chunk.  A warp
-// walks its positions 32 at a time in two passes.  Pass 1, lane = position: the
-// full q.k dot of the lane's K row against all G query heads of the kv head (q
-// waits in shared memory as doubles, read as broadcasts: no cross-lane reduction,
-// and one K read serves the whole GQA group).  Pass 2, lane = dims {lane + 32 i}:
-// the 32 positions' softmax weights (parked in shared memory) times their V rows.
-// Running state per head: max m (an fp32 score), denominator l and output o[] in
-// double.  States fold warps -> chunk (shared memory) -> head (global scratch, by
-// the last CTA of the kv head to arrive), each fold against the common maximum so
-// that the rescale factors are independent of one another; then o/l is rounded to
-// fp32, stored, and quantized to q8_0 for the O projection.
-// G = query heads handled by one CTA: all heads of a kv head (one K/V read serves the group: long
-// contexts, bandwidth matters) or a single head (short contexts: K/V come from L2 anyway, and six
-// times as many CTAs each carry a sixth of the serial work).  GQ = query heads per kv head.
-// Inputs (q, and k / v of the new position) and the q8_0 output travel as tagged words; the CTA whose range ends at the new
-// position also writes that position's K and V into the cache.  Returns false if a wait gave up (CTA-uniform).
-template <int HD, int G, int GQ>
-__device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, int pos, uint8_t* stage,
-                                                unsigned tag_in, const Pub pub) {
-    constexpr int DPW = HD / 32;           // dims per lane in pass 2 and while folding (dim = lane + 32*i)
-    constexpr int SW = HD + 2;             // doubles per (head) state: o[HD], m, l
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ngrp = P.NH / G;
-    // one head per CTA: 256 positions are one 32-position batch per warp, and a single chunk needs no cross-CTA merge
-    const int Lp = pos + 1, nch = attn_chunks(Lp, min(P.max_chunks, (int)gridDim.x / ngrp), G == 1 ? 256 : kAttnChunk);
-    if ((int)blockIdx.x >= ngrp * nch) return true;
-    const int grp = blockIdx.x / nch, ch = blockIdx.x % nch, h0 = grp * G, kvh = h0 / GQ;
-    const int p0 = (int)((long long)ch * Lp / nch), p1 = (int)((long long)(ch + 1) * Lp / nch);
-    double* scr = reinterpret_cast<double*>(stage);                        // [warp][G][SW]
-    double* wts = scr + DNW * G * SW;                                       // [warp][32][G]
-    constexpr int LPP = 8, DPL = HD / LPP, QSTR = DPL + 2;                   // lanes per position in pass 1, dims per lane, padded stride
-    double* qs = wts + DNW * 32 * G;                                        // [G][LPP][QSTR]: 16-byte skew per lane, conflict-free
-    const bool store_kv = ch == nch - 1;     // this CTA's range ends at the new position: it stores that position's K and V (fp16); CTAs that share a kv head store the same bits
-    // q of this CTA's G query heads, and k / v of the new position, from the tagged QKV vector (packed order: dim d of a
-    // head sits at 2d (d < HD/2) or 2(d-HD/2)+1); one poll for all of a thread's words
-    constexpr int QN = (G * HD + DNT - 1) / DNT;
-    const int nq = P.NH * HD;
-    unsigned qw[QN + 2], valid = 0;
-    #pragma unroll
-    for (int k = 0; k < QN; k++) if (tid + k * DNT < G * HD) valid |= 1u << k;
-    if (store_kv && tid < HD) valid |= 3u << QN;
-    const unsigned long long* qv = P.xw + P.xo.qkv;
-    const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;           // packed slot of dim `tid` (threads below HD)
-    bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
-        if (k < QN) {
-            const int i = tid + k * DNT, j = i / HD, d = i % HD, pk = d < HD / 2 ? 2 * d : 2 * (d - HD / 2) + 1;
-            return qv + (size_t)(h0 + j) * HD + pk;
-        }
-        return k == QN ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
-    }, qw);
-    #pragma unroll
-    for (int k = 0; k < QN; k++) {
-        const int i = tid + k * DNT;
-        if (i < G * HD) { const int j = i / HD, d = i % HD; qs[(j * LPP + d / DPL) * QSTR + d % DPL] = (double)__uint_as_float(qw[k]); }
-    }
-    if (store_kv && tid < HD) {
-        P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[QN]));
-        P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[QN + 1]));
-    }
-    if (!__syncthreads_and(okq ? 1 : 0)) return false;
-    prof_mark(P, 14);
-    const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
-    const int n = p1 - p0, a0 = p0 + (int)((long long)n * warp / DNW), a1 = p0 + (int)((long long)n * (warp + 1) / DNW);
-    const __half* kbase = P.kc + ((size_t)l * P.max_seq) * P.KVD + (size_t)kvh * HD;
-    const __half* vbase = P.vc + ((size_t)l * P.max_seq) * P.KVD + (size_t)kvh * HD;
-    double* wl = wts + (size_t)warp * 32 * G;
-    float m[G]; double ls[G], o[G][DPW];
-    #pragma unroll
-    for (int j = 0; j < G; j++) {
-        m[j] = -INFINITY; ls[j] = 0.0;
+// ---- attention over a long causal range --------------------------------------------------
+// CTA = (kv head, chunk of the causal range), all query heads of the group at once, then one CTA per 32-dim block of the
+// output merges the chunks.  What bounds it is the FP64 pipe (2 HD FMAs per head and position) and a chain of latencies, so
+//   * both products are FP64 MMAs (m8n8k4: a group's heads are the rows): one issue slot per 256 FMAs, and a K or V element is
+//     converted to double once for the whole group.  (The scalar form of this phase took 26 us per layer at 8192 positions,
+//     most of it conversions and broadcast loads beside the FMAs.)
+//   * the chunk's K and V rows are requested (asynchronous copies into shared memory) before the CTA waits for q: they do not
+//     depend on this layer's projection, so their latency passes while the projection finishes;
+//   * a chunk leaves its weighted sums and denominator in global memory and, behind a fence, its maximum as a tagged word.  Whoever
+//     merges polls those words: no counter to reset, and 48 CTAs (1.5B shape) read 38 KB each where the last CTA of a kv head to
+//     arrive read 460 KB alone.
+// Scores: double dot products rounded to fp32 once, scaled in fp32; weights, denominator and sums in double, running maximum across
+// steps, common maximum across chunks.  Returns false if a wait gave up (CTA-uniform).
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ double half_to_double(unsigned w) { return (double)__half2float(__ushort_as_half((unsigned short)w)); }
+
+template <int HD, int G>
+__device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, int pos, uint8_t* stage, unsigned tag_in, const Pub pub) {
+    using SM = SplitSmem<HD>;
+    constexpr int NTW = HD >= 64 ? HD / 64 : 1, VW = HD / 8 / NTW, SW = HD + 2;      // 8-dim tiles per warp of the value product, warps that have some; doubles per partial
+    double* qs = reinterpret_cast<double*>(stage + SM::q); double* wt = reinterpret_cast<double*>(stage + SM::wt);      // q [dim of a lane][lane], weights [step of 4][lane]
+    uint8_t* ks = stage + SM::k; uint8_t* vs = stage + SM::v;
+    float* sc = reinterpret_cast<float*>(stage + SM::sc);
+    double* rm = reinterpret_cast<double*>(stage + SM::st); double* rl = rm + 8; double* rf = rl + 8;                    // per head: running maximum, denominator, rescale factor
+    double* red = reinterpret_cast<double*>(stage + SM::red);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int Lp = pos + 1, nch = attn_chunks(Lp, min(P.max_chunks, (int)gridDim.x / P.NKV)), nq = P.NH * HD;
+    bool ok = true;
+    if ((int)blockIdx.x < P.NKV * nch) {
+        const int kvh = blockIdx.x / nch, ch = blockIdx.x - kvh * nch, h0 = kvh * G;
+        const int p0 = (int)((long long)ch * Lp / nch), p1 = (int)((long long)(ch + 1) * Lp / nch), n = p1 - p0, nsub = (n + kSplitSub - 1) / kSplitSub;
+        const bool has_new = ch == nch - 1;
+        const size_t lbase = (size_t)l * P.max_seq * P.KVD + (size_t)kvh * HD;
+        auto sub_begin = [&](int s) { return p0 + n * s / nsub; };
+        auto copy_rows = [&](uint8_t* dst, int ld, const __half* src, int s) {
+            const int b0 = sub_begin(s), np = min(sub_begin(s + 1), pos) - b0;             // the new position is not in the cache yet
+            for (int i = tid; i < np * (HD / 8); i += DNT) {
+                const int r = i / (HD / 8), c = i - r * (HD / 8);
+                cp_async16(dst + r * ld + c * 16, src + lbase + (size_t)(b0 + r) * P.KVD + c * 8);
+            }
+            cp_async_commit();
+        };
+        // (A model of one layer waits for q first: between two steps nothing else orders the last position's rows before this read.)
+        const bool early = P.L > 1;
+        if (early) { copy_rows(ks, SM::KLD, P.kc, 0); copy_rows(vs, SM::VLD, P.vc, 0); }
+        // q of the group, and k / v of the new position (packed order: dim d of a head sits at 2d (d < HD/2) or 2(d-HD/2)+1)
+        constexpr int QN = (G * HD + DNT - 1) / DNT;
+        unsigned qw[QN + 2], valid = 0;
         #pragma unroll
-        for (int i = 0; i < DPW; i++) o[j][i] = 0.0;
-    }
-    for (int b0 = a0; b0 < a1; b0 += 32) {                                  // warp-uniform trip count
-        const int np = min(32, a1 - b0);
-        // pass 1: eight lanes share a position (DPL dims each), four positions per sweep; the
-        // scores of the batch are parked in the weights buffer, one row per position.  All K rows
-        // of the batch are requested before the first one is used.
-        {
-            const int sub = lane >> 3, li = lane & 7;
-            constexpr int KV4 = DPL * 2 / 16 > 0 ? DPL * 2 / 16 : 1;        // 16-byte loads per lane and position
-            // two rounds of four sweeps (16 positions): half the unrolled code of one round of eight; a round's K rows
-            // are all requested before the first one is used
+        for (int k = 0; k < QN; k++) if (tid + k * DNT < G * HD) valid |= 1u << k;
+        if (has_new && tid < HD) valid |= 3u << QN;
+        const unsigned long long* qv = P.xw + P.xo.qkv;
+        const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;
+        const bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
+            if (k < QN) {
+                const int i = tid + k * DNT, j = i / HD, d = i % HD, pk = d < HD / 2 ? 2 * d : 2 * (d - HD / 2) + 1;
+                return qv + (size_t)(h0 + j) * HD + pk;
+            }
+            return k == QN ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
+        }, qw);
+        if (!early) { copy_rows(ks, SM::KLD, P.kc, 0); copy_rows(vs, SM::VLD, P.vc, 0); }
+        // the order the MMA reads q in: lane (row, t) takes the 16-byte pieces t, t + 4, .. of a row
+        auto qslot = [](int row, int d) { return ((d >> 5) * 8 + (d & 7)) * 32 + row * 4 + ((d >> 3) & 3); };
+        #pragma unroll
+        for (int k = 0; k < QN; k++) {
+            const int i = tid + k * DNT;
+            if (i < G * HD) { const int j = i / HD, d = i % HD; qs[qslot(j, d)] = (double)__uint_as_float(qw[k]); }
+        }
+        for (int i = tid + G * HD; i < 8 * HD; i += DNT) qs[qslot(i / HD, i % HD)] = 0.0;
+        const __half knew = __float2half_rn(__uint_as_float(qw[QN])), vnew = __float2half_rn(__uint_as_float(qw[QN + 1]));
+        if (has_new && tid < HD) { P.kc[lbase + (size_t)pos * P.KVD + tid] = knew; P.vc[lbase + (size_t)pos * P.KVD + tid] = vnew; }
+        if (tid < 8) { rm[tid] = -INFINITY; rl[tid] = 0.0; }
+        prof_mark(P, 14);
+        const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
+        double o[2][NTW][2];                        // two chains
+        #pragma unroll
+        for (int c = 0; c < 2; c++)
+            #pragma unroll
+            for (int i = 0; i < NTW; i++) o[c][i][0] = o[c][i][1] = 0.0;
+        #pragma unroll 1
+        for (int s = 0; s < nsub; s++) {
+            const int b0 = sub_begin(s), np = sub_begin(s + 1) - b0;
+            cp_async_wait<1>();                     // the K rows (the V rows were requested after them)
+            if (has_new && s == nsub - 1 && tid < HD) {
+                reinterpret_cast<__half*>(ks + (pos - b0) * SM::KLD)[tid] = knew;
+                reinterpret_cast<__half*>(vs + (pos - b0) * SM::VLD)[tid] = vnew;
+            }
+            if (s == 0) { if (!__syncthreads_and(okq ? 1 : 0)) { ok = false; break; } } else __syncthreads();
+            // scores: warp = every 8th group of 8 positions
             #pragma unroll 1
-            for (int s0 = 0; s0 < 8 && s0 * 4 < np; s0 += 4) {
-                uint4 kraw[4][KV4];
+            for (int t = warp; t * 8 < np; t += DNW) {
+                const uint8_t* kr = ks + min(t * 8 + g, np - 1) * SM::KLD + t4 * 16;
+                double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
                 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int sw = s0 + u;
-                    if (sw * 4 >= np) continue;                              // warp-uniform
-                    const int pi = min(sw * 4 + sub, np - 1);
-                    const __half* kr = kbase + (size_t)(b0 + pi) * P.KVD + li * DPL;
-                    if constexpr (DPL >= 8) {
-                        #pragma unroll
-                        for (int c = 0; c < KV4; c++) kraw[u][c] = __ldcg(reinterpret_cast<const uint4*>(kr) + c);
-                    } else {
-                        const uint2 k2 = __ldcg(reinterpret_cast<const uint2*>(kr));
-                        kraw[u][0] = make_uint4(k2.x, k2.y, 0u, 0u);
-                    }
-                }
-                #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int sw = s0 + u;
-                    if (sw * 4 < np) {                                       // warp-uniform
-                        const int pi = sw * 4 + sub;
-                        double kd[DPL];
-                        #pragma unroll
-                        for (int c = 0; c < KV4; c++) {
-                            const __half2* hh = reinterpret_cast<const __half2*>(&kraw[u][c]);
-                            #pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                if (c * 8 + 2 * e < DPL) {
-                                    const float2 f = __half22float2(hh[e]);
-                                    kd[c * 8 + 2 * e] = (double)f.x; kd[c * 8 + 2 * e + 1] = (double)f.y;
-                                }
-                            }
-                        }
-                        double d[G];
-                        #pragma unroll
-                        for (int j = 0; j < G; j++) {
-                            const double* qj = qs + (j * LPP + li) * QSTR;
-                            double acc = 0.0;
-                            #pragma unroll
-                            for (int e = 0; e < DPL; e += 2) {
-                                const double2 qq = *reinterpret_cast<const double2*>(qj + e);
-                                acc = __fma_rn(qq.x, kd[e], acc);
-                                acc = __fma_rn(qq.y, kd[e + 1], acc);
-                            }
-                            d[j] = acc;
-                        }
-                        #pragma unroll
-                        for (int sft = 1; sft <= 4; sft <<= 1)
-                            #pragma unroll
-                            for (int j = 0; j < G; j++) d[j] = __dadd_rn(d[j], __shfl_xor_sync(0xffffffffu, d[j], sft));
-                        if (li == 0 && pi < np) {
-                            #pragma unroll
-                            for (int j = 0; j < G; j++) wl[pi * G + j] = (double)__fmul_rn(__double2float_rn(d[j]), inv);
-                        }
-                    }
-                }
-            }
-        }
-        __syncwarp();
-        const bool valid = lane < np;
-        float sc[G];
-        #pragma unroll
-        for (int j = 0; j < G; j++) sc[j] = valid ? (float)wl[lane * G + j] : -INFINITY;
-        __syncwarp();
-        // new running max, rescale, this batch's weights
-        #pragma unroll
-        for (int j = 0; j < G; j++) {
-            const float bm = warp_max_float(sc[j]);
-            const float mn = fmaxf(m[j], bm);                                // finite: the batch holds a valid position
-            // the running maximum is warp-uniform; while it stands the rescale factor is exp(0) = 1 exactly
-            const double cr = mn == m[j] ? 1.0 : (m[j] == -INFINITY ? 0.0 : exp_shared((double)m[j] - (double)mn));
-            const double w = valid ? exp_shared((double)sc[j] - (double)mn) : 0.0;
-            wl[lane * G + j] = w;                                            // the denominator picks the weights up in pass 2
-            ls[j] = __dmul_rn(ls[j], cr);
-            #pragma unroll
-            for (int i = 0; i < DPW; i++) o[j][i] = __dmul_rn(o[j][i], cr);
-            m[j] = mn;
-        }
-        __syncwarp();
-        // pass 2: o += w[p] * V[p]
-        constexpr int VB = G == 1 ? 16 : 8;                                  // V rows requested together (one head per CTA: registers to spare)
-        for (int pp0 = 0; pp0 < np; pp0 += VB) {
-            unsigned short vh[VB][DPW];
-            #pragma unroll
-            for (int u = 0; u < VB; u++) {
-                if (u >= 8 && pp0 + u >= np) continue;                       // warp-uniform: the second half of a round may be empty
-                const unsigned short* vp = reinterpret_cast<const unsigned short*>(vbase + (size_t)(b0 + min(pp0 + u, np - 1)) * P.KVD);
-                #pragma unroll
-                for (int i = 0; i < DPW; i++) vh[u][i] = __ldcg(vp + lane + 32 * i);
-            }
-            #pragma unroll
-            for (int u = 0; u < VB; u++) {
-                if (pp0 + u < np) {
-                    double vd[DPW];
+                for (int i = 0; i < HD / 32; i++) {
+                    const uint4 kw = *reinterpret_cast<const uint4*>(kr + i * 64);
+                    const unsigned w[4] = {kw.x, kw.y, kw.z, kw.w};
                     #pragma unroll
-                    for (int i = 0; i < DPW; i++) vd[i] = (double)__half2float(__ushort_as_half(vh[u][i]));
+                    for (int e = 0; e < 4; e++) {
+                        const double* a = qs + (i * 8 + e * 2) * 32 + lane;
+                        dmma884(c[0], a[0], half_to_double(w[e] & 0xffffu)); dmma884(c[1], a[32], half_to_double(w[e] >> 16));
+                    }
+                }
+                #pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int pp = t * 8 + 2 * t4 + e;
+                    if (pp < kSplitSub) sc[g * SM::SCL + pp] = pp < np ? __fmul_rn(__double2float_rn(__dadd_rn(c[0][e], c[1][e])), inv) : -INFINITY;
+                }
+            }
+            __syncthreads();
+            prof_mark(P, 27);
+            if (s + 1 < nsub) copy_rows(ks, SM::KLD, P.kc, s + 1); else cp_async_commit();
+            // weights: one warp per head
+            if (warp < G) {
+                float x[kSplitSub / 32], m = -INFINITY;
+                #pragma unroll
+                for (int i = 0; i < kSplitSub / 32; i++) { x[i] = lane + 32 * i < np ? sc[warp * SM::SCL + lane + 32 * i] : -INFINITY; m = fmaxf(m, x[i]); }
+                m = warp_max_float(m);
+                const double mo = rm[warp], mn = fmax(mo, (double)m);
+                double ls = 0.0;
+                #pragma unroll
+                for (int i = 0; i < kSplitSub / 32; i++) {
+                    const double w = lane + 32 * i < np ? exp_shared((double)x[i] - mn) : 0.0;
+                    const int pp = lane + 32 * i;
+                    wt[(pp >> 2) * 32 + warp * 4 + (pp & 3)] = w;
+                    ls = __dadd_rn(ls, w);
+                }
+                #pragma unroll
+                for (int q = 16; q; q >>= 1) ls = __dadd_rn(ls, __shfl_xor_sync(0xffffffffu, ls, q));
+                if (lane == 0) {
+                    const double f = mo == mn ? 1.0 : mo == -INFINITY ? 0.0 : exp_shared(mo - mn);
+                    rf[warp] = f; rm[warp] = mn; rl[warp] = __fma_rn(rl[warp], f, ls);
+                }
+            }
+            cp_async_wait<1>();                     // the V rows
+            __syncthreads();
+            prof_mark(P, 29);
+            // values: warp = HD/8 dims, all positions
+            if (warp < VW) {
+                if (s > 0) {
+                    const double f = g < G ? rf[g] : 1.0;
                     #pragma unroll
-                    for (int j = 0; j < G; j++) {
-                        const double w = wl[(pp0 + u) * G + j];
-                        ls[j] = __dadd_rn(ls[j], w);
+                    for (int c = 0; c < 2; c++)
                         #pragma unroll
-                        for (int i = 0; i < DPW; i++) o[j][i] = __fma_rn(w, vd[i], o[j][i]);
+                        for (int i = 0; i < NTW; i++) { o[c][i][0] = __dmul_rn(o[c][i][0], f); o[c][i][1] = __dmul_rn(o[c][i][1], f); }
+                }
+                const uint8_t* vr = vs + (warp * (8 * NTW) + g * NTW) * 2;
+                #pragma unroll 2
+                for (int u = 0; u * 4 < np; u += 2) {
+                    #pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        if ((u + c) * 4 >= np) break;                                      // warp-uniform
+                        const uint8_t* v = vr + min((u + c) * 4 + t4, np - 1) * SM::VLD;
+                        const double w = wt[(u + c) * 32 + lane];
+                        if constexpr (NTW == 2) {
+                            const unsigned vw = *reinterpret_cast<const unsigned*>(v);
+                            dmma884(o[c][0], w, half_to_double(vw & 0xffffu)); dmma884(o[c][NTW - 1], w, half_to_double(vw >> 16));
+                        } else {
+                            dmma884(o[c][0], w, half_to_double(*reinterpret_cast<const unsigned short*>(v)));
+                        }
                     }
                 }
             }
+            __syncthreads();                        // scores, weights and V rows may be written again
+            if (s + 1 < nsub) copy_rows(vs, SM::VLD, P.vc, s + 1);
         }
-        __syncwarp();
-    }
-    prof_mark(P, 15);
-    #pragma unroll
-    for (int j = 0; j < G; j++) {
-        double* sw = scr + (size_t)(warp * G + j) * SW;
-        #pragma unroll
-        for (int i = 0; i < DPW; i++) sw[lane + 32 * i] = o[j][i];
-        if (lane == 0) { sw[HD] = (double)m[j]; sw[HD + 1] = ls[j]; }
-    }
-    // the new position's K / V rows (plain stores above) are performed before anything this CTA publishes from here on:
-    // a CTA that reads them in a later step has consumed words that descend from this CTA's output
-    if (store_kv && tid < HD) __threadfence();
-    __syncthreads();
-    // warp j folds head j's DNW warp states against their common maximum and publishes the chunk partial
-    if (warp < G) {
-        const int j = warp, head = h0 + j;
-        // lane w takes warp w's maximum: one exponential for all eight rescale factors, then broadcast
-        const float mw_l = lane < DNW ? (float)scr[(size_t)(lane * G + j) * SW + HD] : -INFINITY;
-        const float mm = warp_max_float(mw_l);
-        const double f_l = mw_l == -INFINITY ? 0.0 : exp_shared((double)mw_l - (double)mm);
-        double f[DNW];
-        #pragma unroll
-        for (int w = 0; w < DNW; w++) f[w] = __shfl_sync(0xffffffffu, f_l, w);
-        double ob[DPW], ll = 0.0;
-        #pragma unroll
-        for (int i = 0; i < DPW; i++) ob[i] = 0.0;
-        #pragma unroll
-        for (int w = 0; w < DNW; w++) {
-            const double* s2 = scr + (size_t)(w * G + j) * SW;
-            ll = __fma_rn(s2[HD + 1], f[w], ll);
-            #pragma unroll
-            for (int i = 0; i < DPW; i++) ob[i] = __fma_rn(s2[lane + 32 * i], f[w], ob[i]);
-        }
-        if (nch == 1) {                                                     // the chunk is the whole range: finish here
-            #pragma unroll
-            for (int i = 0; i < DPW; i++) {
-                const float v = __double2float_rn(__ddiv_rn(ob[i], ll));
-                const int e = head * HD + 32 * i + lane;
-                __stcg(P.att + e, v);
-                __half dq; int sq;
-                const int qv8 = quant_block_warp2(v, dq, sq);
-                publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
+        if (!ok) cp_async_wait<0>();                // copies in flight target the staging area
+        prof_mark(P, 15);
+        if (ok) {
+            if (warp < VW && g < G) {
+                double* gp = P.attn_part + ((size_t)(h0 + g) * P.max_chunks + ch) * SW;
+                #pragma unroll
+                for (int i = 0; i < NTW; i++)
+                    #pragma unroll
+                    for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + i, __dadd_rn(o[0][i][e], o[1][i][e]));
             }
-        } else {
-            double* gp = P.attn_part + ((size_t)head * P.max_chunks + ch) * SW;
-            #pragma unroll
-            for (int i = 0; i < DPW; i++) __stcg(gp + lane + 32 * i, ob[i]);
-            if (lane == 0) { __stcg(gp + HD, (double)mm); __stcg(gp + HD + 1, ll); }
+            if (tid < G) __stcg(P.attn_part + ((size_t)(h0 + tid) * P.max_chunks + ch) * SW + HD, rl[tid]);
+            __threadfence();                        // the partial, and the new position's rows, before the word that announces them
+            __syncthreads();
+            if (tid < G) pub.local(P.xo.attm + (h0 + tid) * P.max_chunks + ch, __float_as_uint((float)rm[tid]));
         }
+        prof_mark(P, 16);
     }
-    prof_mark(P, 16);
-    if (nch == 1) return true;
-    __threadfence();
-    __syncthreads();
-    __shared__ unsigned s_prev;
-    if (tid == 0) s_prev = atomicAdd(P.attn_cnt + grp, 1u);
-    __syncthreads();
-    if (s_prev != (unsigned)nch - 1) return true;
-    // last chunk of this kv head: fold the chunk partials against their common maximum, normalise, emit fp32 + q8_0
-    __threadfence();
-    if (tid == 0) P.attn_cnt[grp] = 0;
-    if (warp < G) {
-        const int j = warp, head = h0 + j;
-        const double* gp = P.attn_part + (size_t)head * P.max_chunks * SW;
-        // rescale factors of all chunks first (lane = chunk, so the exponentials run side by side), parked in the
-        // warp-state buffer, which nobody reads any more; then the fold in chunk order, eight chunks' loads in flight
-        double* fs = scr + (size_t)j * DNW * SW;                            // nch <= grid size / kv heads <= DNW * SW
-        float mm = -INFINITY;
-        for (int c = lane; c < nch; c += 32) {
-            const float mc = (float)__ldcg(gp + (size_t)c * SW + HD);
-            fs[c] = (double)mc; mm = fmaxf(mm, mc);
-        }
+    // merge: one CTA per 32-dim block of a head, its warps share the chunks; lane = dim
+    const int nblk = P.NH * (HD / 32);
+    for (int b = blockIdx.x; b < nblk && ok; b += gridDim.x) {
+        const int head = b / (HD / 32), d0 = (b - head * (HD / 32)) * 32;
+        unsigned mw[kMaxChunkWords], valid = 0;
         #pragma unroll
-        for (int sft = 16; sft; sft >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, sft));
-        for (int c = lane; c < nch; c += 32) {
-            const float mc = (float)fs[c];
-            fs[c] = mc == -INFINITY ? 0.0 : exp_shared((double)mc - (double)mm);
-        }
-        __syncwarp();
-        double ob[DPW], ll = 0.0;
+        for (int k = 0; k < kMaxChunkWords; k++) if (lane + 32 * k < nch) valid |= 1u << k;
+        const unsigned long long* mv = P.xw + P.xo.attm + (size_t)head * P.max_chunks;
+        const bool okm = tw_poll(P, pub.tag, valid, [&](int k) { return mv + lane + 32 * k; }, mw);
+        __threadfence();
+        float m = -INFINITY;
         #pragma unroll
-        for (int i = 0; i < DPW; i++) ob[i] = 0.0;
-        for (int c0 = 0; c0 < nch; c0 += 8) {
-            double lv[8], ov[8][DPW];
+        for (int k = 0; k < kMaxChunkWords; k++) if (valid >> k & 1u) m = fmaxf(m, __uint_as_float(mw[k]));
+        m = warp_max_float(m);
+        // this warp's chunks: warp, warp + 8, ..; lane i prepares the factor of the i-th
+        const int mine = (nch - warp + DNW - 1) / DNW;
+        const double* gp = P.attn_part + ((size_t)head * P.max_chunks + warp) * SW;
+        double f_l = 0.0;
+        if (lane < mine) {
+            const float mc = __uint_as_float((unsigned)tw_ld(mv + warp + DNW * lane));
+            f_l = mc == -INFINITY ? 0.0 : exp_shared((double)mc - (double)m);
+        }
+        double ob = 0.0, lb = lane < mine ? __dmul_rn(__ldcg(gp + (size_t)lane * DNW * SW + HD), f_l) : 0.0;
+        for (int i0 = 0; i0 < mine; i0 += 8) {
+            double v[8];
+            #pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = __ldcg(gp + (size_t)min(i0 + u, mine - 1) * DNW * SW + d0 + lane);
             #pragma unroll
             for (int u = 0; u < 8; u++) {
-                const double* g2 = gp + (size_t)min(c0 + u, nch - 1) * SW;
-                lv[u] = __ldcg(g2 + HD + 1);
-                #pragma unroll
-                for (int i = 0; i < DPW; i++) ov[u][i] = __ldcg(g2 + lane + 32 * i);
-            }
-            #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                if (c0 + u < nch) {
-                    const double f = fs[c0 + u];
-                    ll = __fma_rn(lv[u], f, ll);
-                    #pragma unroll
-                    for (int i = 0; i < DPW; i++) ob[i] = __fma_rn(ov[u][i], f, ob[i]);
-                }
+                const double f = __shfl_sync(0xffffffffu, f_l, (i0 + u) & 31);
+                if (i0 + u < mine) ob = __fma_rn(v[u], f, ob);
             }
         }
         #pragma unroll
-        for (int i = 0; i < DPW; i++) {
-            const float v = __double2float_rn(__ddiv_rn(ob[i], ll));
-            const int e = head * HD + 32 * i + lane;
+        for (int q = 16; q; q >>= 1) lb = __dadd_rn(lb, __shfl_xor_sync(0xffffffffu, lb, q));
+        __syncthreads();                            // the buffer below is free (a second block of this CTA)
+        red[warp * 33 + lane] = ob;
+        if (lane == 0) red[warp * 33 + 32] = lb;
+        ok = __syncthreads_and(okm ? 1 : 0) != 0;
+        if (warp == 0 && ok) {
+            double den = red[32];
+            ob = red[lane];
+            #pragma unroll
+            for (int w = 1; w < DNW; w++) { ob = __dadd_rn(ob, red[w * 33 + lane]); den = __dadd_rn(den, red[w * 33 + 32]); }
+            const float v = __double2float_rn(__ddiv_rn(ob, den));
+            const int e = head * HD + d0 + lane;
             __stcg(P.att + e, v);
             __half dq; int sq;
             const int qv8 = quant_block_warp2(v, dq, sq);
             publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
         }
     }
-    return true;
+    prof_mark(P, 17);
+    return ok;
 }
 
 // ---- attention over a short causal range (at most 256 positions): one CTA per query head ---------------
@@ -1121,7 +1066,7 @@ __device__ __forceinline__ bool attention_phase(const DecodeParams& P, int l, in
 //   pass 2  warp w, same positions: lane = dims {lane + 32 i}; o += w[p] * V[p], l += w[p] in position order;
 //   finish  warp i (i < HD/32) adds the eight warps' partial sums in warp order, divides, rounds to fp32, quantizes its
 //           32-dim block to q8_0 and publishes it.
-// Same interface as attention_phase.
+// Same interface as attention_split.
 template <int HD, int GQ>
 MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* stage,
                                                 unsigned tag_in, const Pub pub) {
@@ -1302,8 +1247,7 @@ __host__ __device__ inline size_t attn_dedicated_smem(int HD, int HPC) {
            (size_t)DNW * HPC * 8 + (size_t)HPC * kAttnRows * 4 + 64;
 }
 // query heads per attention CTA: two where the group size is even (1.5B: six CTAs of two heads; three heads per CTA
-// measured 4.5 us per layer on the critical path, see the profile table in the repository's design notes), the whole
-// group where it is odd, one head for groups of one or two
+// measured 4.5 us per layer on the critical path), the whole group where it is odd, one head for groups of one or two
 __host__ __device__ constexpr int attn_heads_per_cta(int G) { return (G % 2 == 0 && G > 2) ? MI_ATTN_HPC_EVEN(G) : (G <= 2 ? 1 : G); }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
@@ -1514,9 +1458,7 @@ __device__ __forceinline__ bool lean_regime_ok(int pos, int attn_ctas) {
 #if MI_LEAN == 1
     return pos + 1 <= kShortAttnMax && attn_ctas > 0;
 #elif MI_LEAN == 2
-    return pos + 1 > kShortAttnMax && pos + 1 <= kPerHeadAttnMax;
-#elif MI_LEAN == 3
-    return pos + 1 > kPerHeadAttnMax;
+    return pos + 1 > kShortAttnMax;
 #else
     return true;
 #endif
@@ -1567,13 +1509,10 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
 #if MI_LEAN == 0
             else {
                 if (apf.pending) { (void)mbar_wait_bounded(apf.bar, apf.parity); apf.parity ^= 1u; apf.pending = false; apf.layer = -1; }
-                if (pos + 1 <= kPerHeadAttnMax) ok = attention_phase<HD, 1, G>(P, l, pos, stage, pub.tag - 1u, pub);
-                else ok = attention_phase<HD, G, G>(P, l, pos, stage, pub.tag - 1u, pub);
+                ok = attention_split<HD, G>(P, l, pos, stage, pub.tag - 1u, pub);
             }
 #elif MI_LEAN == 2
-            ok = attention_phase<HD, 1, G>(P, l, pos, stage, pub.tag - 1u, pub);
-#elif MI_LEAN == 3
-            ok = attention_phase<HD, G, G>(P, l, pos, stage, pub.tag - 1u, pub);
+            ok = attention_split<HD, G>(P, l, pos, stage, pub.tag - 1u, pub);
 #endif
             ok = __syncthreads_and(ok ? 1 : 0) != 0;
             prof_mark(P, 3);
@@ -1729,12 +1668,9 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                 }
 #if MI_LEAN == 0
                 else if (pos + 1 <= kShortAttnMax) ok = attention_short<HD, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
-                else if (pos + 1 <= kPerHeadAttnMax) ok = attention_phase<HD, 1, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
-                else ok = attention_phase<HD, G, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else ok = attention_split<HD, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
 #elif MI_LEAN == 2
-                else ok = attention_phase<HD, 1, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
-#elif MI_LEAN == 3
-                else ok = attention_phase<HD, G, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
+                else ok = attention_split<HD, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
 #endif
             } else if (k != 5) {
                 const int jn = 4 * l + (k == 0 ? 0 : k == 2 ? 1 : k == 3 ? 2 : 3);

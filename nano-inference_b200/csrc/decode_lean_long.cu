@@ -1,6 +1,6 @@
-// The build of the decode kernel for launches whose steps all have more than kPerHeadAttnMax cached positions: a whole GQA group per CTA and chunk.
+// The build of the decode kernel for launches whose steps all have more than kShortAttnMax cached positions (attention_split).
 // Like the short-context build (decode_lean.cu) it holds one attention variant and no call site in the step loop.
-#define MI_LEAN 3
+#define MI_LEAN 2
 #include "decode_kernel.cuh"
 
 namespace mi {
