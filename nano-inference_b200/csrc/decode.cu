@@ -21,6 +21,8 @@ const void* decode_kernel_prof_lean(int HD, int G);
 const void* decode_kernel_tp_lean(int HD, int G);
 const void* decode_kernel_tp_prof_lean(int HD, int G);
 const void* decode_kernel_lean_long(int HD, int G);
+const void* decode_kernel_lean_small(int HD, int G);
+const void* decode_kernel_lean_small_long(int HD, int G);
 }
 
 namespace {
@@ -110,7 +112,8 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
     void (*kern)(DecodeParams, int, int, int, int) = nullptr;
     // every step of this launch ends within the range the dedicated attention CTAs handle, on a shape the short-context
     // build takes: that build has no other attention variant in it (decode_lean.cu)
-    const bool shape_ok = lean_shape_ok(m->E, m->FF, m->NH * m->HD) && !getenv("MINFER_NO_LEAN");
+    const int shape = getenv("MINFER_NO_LEAN") ? 0 : lean_shape(m->E, m->FF, m->NH * m->HD);
+    const bool shape_ok = shape != 0;
     const bool by_pos = !P.pos_dev && range_hint == 0;
     const bool lean = m->attn_ctas > 0 && shape_ok && (range_hint == 1 || (by_pos && (long long)P.pos0 + step1 <= kShortAttnMax));
     auto as_kernel = [](const void* p) { return reinterpret_cast<void (*)(DecodeParams, int, int, int, int)>(const_cast<void*>(p)); };
@@ -119,15 +122,15 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
     const bool far = shape_ok && (range_hint == 2 || (by_pos && (long long)P.pos0 + step0 + 1 > kShortAttnMax));
     const void* pick = nullptr;
     if (P.tp.on) {                                  // the builds with the exchange between GPUs inside (decode_tp.cu, decode_tp_lean.cu)
-        if (lean && P.prof) pick = decode_kernel_tp_prof_lean(m->HD, m->G);
-        if (lean && !pick) pick = decode_kernel_tp_lean(m->HD, m->G);
+        if (lean && shape == 1 && P.prof) pick = decode_kernel_tp_prof_lean(m->HD, m->G);
+        if (lean && shape == 1 && !pick) pick = decode_kernel_tp_lean(m->HD, m->G);
         if (!pick) pick = decode_kernel_tp(m->HD, m->G);
     } else if (P.prof) {                            // the instrumented builds (decode_prof.cu, decode_prof_lean.cu)
-        if (lean) pick = decode_kernel_prof_lean(m->HD, m->G);
+        if (lean && shape == 1) pick = decode_kernel_prof_lean(m->HD, m->G);
         if (!pick) pick = decode_kernel_prof(m->HD, m->G);
     } else {
-        if (lean) pick = decode_kernel_lean(m->HD, m->G);
-        else if (far) pick = decode_kernel_lean_long(m->HD, m->G);
+        if (lean) pick = shape == 1 ? decode_kernel_lean(m->HD, m->G) : decode_kernel_lean_small(m->HD, m->G);
+        else if (far) pick = shape == 1 ? decode_kernel_lean_long(m->HD, m->G) : decode_kernel_lean_small_long(m->HD, m->G);
     }
     if (pick) kern = as_kernel(pick);
     else {
@@ -698,7 +701,7 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
         // launch's positions), a launch that straddles a boundary would fall back to the general build.  Under the stop
         // rule the host cannot know whether an earlier launch ended the run, so the run stays one launch.
         int cuts[3] = {0, 0, n_steps}, nc = 1;
-        if (stop < 0 && !P.tp.on && lean_shape_ok(m->E, m->FF, m->NH * m->HD)) {
+        if (stop < 0 && !P.tp.on && lean_shape(m->E, m->FF, m->NH * m->HD) != 0) {
             const long long s = (long long)kShortAttnMax - pos0;       // first step whose position count exceeds the edge
             if (s > 0 && s < n_steps) cuts[nc++] = (int)s;
         }

@@ -82,9 +82,10 @@
 // The kernel exists in several builds.  The default one carries no profiling code and no peer stores.  A translation unit
 // that defines MI_PROF 1 before including this file gets the instrumented build (timer marks between the hot instructions
 // cost a few percent when merely compiled in); MI_TP 1 gives the tensor-parallel build, whose publishing stores also go to
-// the other GPUs; MI_LEAN 1 gives the short-context build, which holds no attention code but that of the dedicated attention CTAs (launched only for step ranges that end within kShortAttnMax positions on a model with such CTAs: without
-// the other attention variants in the same function the GEMV CTAs' loop keeps its values in registers); MI_LEAN 2 is the same idea for more than kShortAttnMax
-// positions (attention_split).  They live in
+// the other GPUs; MI_LEAN 1 gives the short-context build, which holds no attention code but that of the dedicated attention
+// CTAs (launched only for step ranges that end within kShortAttnMax positions on a model with such CTAs: without the other
+// attention variants in the same function the GEMV CTAs' loop keeps its values in registers); MI_LEAN 2 is the same idea for
+// more than kShortAttnMax positions (attention_split); MI_SMALL 1 makes either one for narrow models (lean_shape).  They live in
 // different inline namespaces, so all can be linked into one library and picked at launch time.
 #ifndef MI_PROF
 #define MI_PROF 0
@@ -95,7 +96,14 @@
 #ifndef MI_LEAN
 #define MI_LEAN 0
 #endif
-#if MI_PROF && MI_TP && MI_LEAN
+#ifndef MI_SMALL
+#define MI_SMALL 0
+#endif
+#if MI_SMALL && MI_LEAN == 2
+#define MI_KVARIANT leansmalllong
+#elif MI_SMALL && MI_LEAN
+#define MI_KVARIANT leansmall
+#elif MI_PROF && MI_TP && MI_LEAN
 #define MI_KVARIANT tpxproflean
 #elif MI_PROF && MI_LEAN
 #define MI_KVARIANT proflean
@@ -473,7 +481,9 @@ __device__ __forceinline__ double tile_consume(WarpStream& ws, int lane, int kb,
     if (PP) prof_mark(*PP, 20);
     const uint8_t* tile = ws.ring + (size_t)slot * DSLOT;
 #if MI_LEAN
-    acc = tile_dot_row<8, false>(tile, lane, t * 8, xq_s, xs_s, acc, nullptr);          // lean_shape_ok(): every tile is 8 blocks deep
+    // lean_shape(): tiles are 8 blocks deep, or (small build) 8 or 4
+    if (MI_SMALL && kb == 4) acc = tile_dot_row<4, false>(tile, lane, t * 4, xq_s, xs_s, acc, nullptr);
+    else acc = tile_dot_row<8, false>(tile, lane, t * 8, xq_s, xs_s, acc, nullptr);
 #else
     if (kb == 8) acc = tile_dot_row<8, false>(tile, lane, t * 8, xq_s, xs_s, acc, nullptr);
     else acc = tile_dot_row_rare(kb, tile, lane, t, xq_s, xs_s, acc);
@@ -730,7 +740,7 @@ static __device__ __noinline__ bool stage_norm_q8_rare(MI_NORM_ARGS) {
 }
 __device__ __forceinline__ bool stage_norm_q8u(MI_NORM_ARGS) {
 #if MI_LEAN
-    return stage_norm_q8_t<8, 8>(MI_NORM_PASS);                                         // lean_shape_ok(): 1024 < E <= 2048
+    return stage_norm_q8_t<MI_SMALL ? 4 : 8, MI_SMALL ? 4 : 8>(MI_NORM_PASS);           // lean_shape(): 1024 < E <= 2048, or (small build) 512 < E <= 1024
 #else
     if (E > 1024 && E <= 2048) return stage_norm_q8_t<8, 8>(MI_NORM_PASS);
     return stage_norm_q8_rare(MI_NORM_PASS);
@@ -799,17 +809,20 @@ __device__ __forceinline__ bool stage_poll_q8(const DecodeParams& P, const unsig
     if (np <= 1) return stage_poll_q8_t<1>(P, vw, n, tag, xq_s, xs_s);
     if (np <= 5) return stage_poll_q8_t<5>(P, vw, n, tag, xq_s, xs_s);
 #if MI_LEAN
-    return stage_poll_q8_t<8>(P, vw, n, tag, xq_s, xs_s);                               // lean_shape_ok(): at most 8 word pairs per thread
+    return stage_poll_q8_t<8>(P, vw, n, tag, xq_s, xs_s);                               // lean_shape(): at most 8 word pairs per thread
 #else
     return stage_poll_q8_rare(P, vw, n, tag, xq_s, xs_s);
 #endif
 }
 
-// Shapes the short-context build takes: it holds one variant of each prologue and of the tile loop and no call to the others.
-inline bool lean_shape_ok(int E, int FF, int NQ) {
-    auto kb8 = [](int n) { return (n / 32) % 8 == 0; };
+// Shapes the context-range builds take: they hold one variant of each prologue and of the tile loop and no call to the others.
+// 1: embedding widths of 1025 to 2048 with tiles of 8 blocks; 2: of 513 to 1024 with tiles of 8 or 4 blocks (the small builds,
+// MI_SMALL: 443 us per token at the 0.5B shape where the general build, whose loop spills, took 539); 0: neither.
+inline int lean_shape(int E, int FF, int NQ) {
+    auto kb = [&](int k) { return (E / 32) % k == 0 && (FF / 32) % k == 0 && (NQ / 32) % k == 0; };
     auto np = [](int n) { return (q8_words(n) / 2 + DNT - 1) / DNT; };
-    return E > 1024 && E <= 2048 && kb8(E) && kb8(FF) && kb8(NQ) && np(FF) <= 8 && np(NQ) <= 8;
+    if (np(FF) > 8 || np(NQ) > 8) return 0;
+    return E > 1024 && E <= 2048 && kb(8) ? 1 : E > 512 && E <= 1024 && kb(4) ? 2 : 0;
 }
 
 // ---- attention over a long causal range --------------------------------------------------
@@ -1247,8 +1260,8 @@ __host__ __device__ inline size_t attn_dedicated_smem(int HD, int HPC) {
            (size_t)DNW * HPC * 8 + (size_t)HPC * kAttnRows * 4 + 64;
 }
 // query heads per attention CTA: two where the group size is even (1.5B: six CTAs of two heads; three heads per CTA
-// measured 4.5 us per layer on the critical path), the whole group where it is odd, one head for groups of one or two
-__host__ __device__ constexpr int attn_heads_per_cta(int G) { return (G % 2 == 0 && G > 2) ? MI_ATTN_HPC_EVEN(G) : (G <= 2 ? 1 : G); }
+// measured 4.5 us per layer on the critical path), one where it is odd or at most two
+__host__ __device__ constexpr int attn_heads_per_cta(int G) { return (G % 2 == 0 && G > 2) ? MI_ATTN_HPC_EVEN(G) : 1; }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
