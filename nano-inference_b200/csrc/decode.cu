@@ -485,7 +485,11 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     P.max_seq = max_seq; P.max_chunks = m->max_chunks; P.err = ctx->d_err;
     m->prof_buf = P.prof;
     if (!getenv("MINFER_PROFILE")) P.prof = nullptr;         // the buffer exists either way; kernels only write it when asked
-    m->smem = decode_smem_bytes((int)m->jobs.size(), E, FF, HD);
+    P.inv_e = 1.0 / (double)E;
+    // positions per step of the long-range attention: as many as fit, a multiple of 16 so that score rows stay apart in the banks
+    P.split_sub = kSplitSubMax;
+    while (P.split_sub > kSplitSubMin && decode_smem_bytes((int)m->jobs.size(), E, FF, HD, P.split_sub) + 1024 > (size_t)ctx->smem_optin) P.split_sub -= 16;
+    m->smem = decode_smem_bytes((int)m->jobs.size(), E, FF, HD, P.split_sub);
     if (m->attn_ctas > 0) {
         const int hpc = attn_heads_per_cta(m->G);
         m->smem = std::max(m->smem, attn_dedicated_smem(HD, hpc));       // the attention CTAs lay the same allocation out their own way

@@ -181,6 +181,7 @@ struct TokenRing { int* count; int* tokens; float* margins; unsigned long long* 
 struct DecodeParams {
     int L, E, FF, NH, NKV, HD, KVD, V;
     float eps;
+    double inv_e;                    // 1 / E
     const Job* jobs;                 // [4L+1] in phase order
     const unsigned long long* tile_tab;   // per warp slot: source address | kb code of every tile of one step, in consumption order
     const unsigned* tile_start;      // [grid*DNW][4L+2]: index of each job's first tile in the warp's list (last = count)
@@ -207,7 +208,7 @@ struct DecodeParams {
     int drop_phase;                  // test hook: the producers of this phase publish nothing (-1: none), so that its consumers' waits run out
     float* att;                      // merged attention output, fp32, for inspection
     __half* kc; __half* vc; int max_seq;       // [L][max_seq][KVD]
-    double* attn_part; int max_chunks;       // [NH][max_chunks][HD+2]: weighted sums and denominator of every chunk (attention_split)
+    double* attn_part; int max_chunks, split_sub;       // [NH][max_chunks][HD+2]: weighted sums and denominator of every chunk (attention_split)
     float* out_margins;              // optional [n_steps]: top-1 minus top-2 logit of every step
     TokenRing ring;                  // optional: host-mapped ring the first GEMV CTA publishes every step's token into
     float* best_val;                 // value of the best logit (tensor parallelism with host-side exchange: this GPU's rows only)
@@ -244,25 +245,35 @@ struct DecodeSmem {
 
 constexpr int kFoldBytes = 2 * DNW * 2 * 32 * 8;      // two buffers of [warp][acc][lane] doubles
 
-// attention_split: positions per step, words of chunk maxima a lane polls (up to 160 chunks per kv head), layout of its staging area
-constexpr int kSplitSub = 64, kMaxChunkWords = 5;
-template <int HD> struct SplitSmem {
-    static constexpr int KLD = 2 * HD + 64, VLD = 2 * HD + 32, SCL = kSplitSub + 4;       // row strides: fragment loads without bank conflicts
-    static constexpr int q = 0, wt = 8 * HD * 8, k = wt + 8 * kSplitSub * 8, v = k + kSplitSub * KLD, sc = v + kSplitSub * VLD, st = sc + 8 * SCL * 4,
-                         red = st + 8 * 3 * 8, bytes = red + DNW * 33 * 8;
+// attention_split: positions per step (as many as the shared memory allows: a chunk that fits one step has all its rows requested
+// before q is waited for; 8192 positions in two steps of 64 instead of one of 112: 3.9 instead of 2 us for the scores), words of
+// chunk maxima a lane polls (up to 160 chunks per kv head), layout of its staging area
+constexpr int kSplitSubMin = 64, kSplitSubMax = 128, kMaxChunkWords = 5;
+struct SplitSmem {
+    int HD, sub;
+    __host__ __device__ int kld() const { return 2 * HD + 64; }                          // row strides: fragment loads without bank conflicts
+    __host__ __device__ int vld() const { return 2 * HD + 32; }
+    __host__ __device__ int scl() const { return sub + 4; }
+    __host__ __device__ int wt() const { return 8 * HD * 8; }                            // q comes first
+    __host__ __device__ int k() const { return wt() + 8 * sub * 8; }
+    __host__ __device__ int v() const { return k() + sub * kld(); }
+    __host__ __device__ int sc() const { return v() + sub * vld(); }
+    __host__ __device__ int st() const { return sc() + 8 * scl() * 4; }
+    __host__ __device__ int red() const { return st() + 8 * 3 * 8; }
+    __host__ __device__ int bytes() const { return red() + DNW * 33 * 8; }
 };
 
-__host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD) {
+__host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD, int sub) {
     const int maxin = E > FF ? E : FF;
     size_t a = (size_t)maxin + (size_t)(maxin / 32) * 8;               // xq, xs
-    const size_t split = HD == 128 ? SplitSmem<128>::bytes : HD == 64 ? SplitSmem<64>::bytes : SplitSmem<32>::bytes;
+    const size_t split = SplitSmem{HD, sub}.bytes();
     const size_t shrt = (size_t)(8 * (HD / 8 + 2) + 256 + DNW * HD + DNW) * 8 + 1024;                // attention_short
     const size_t b = split > shrt ? split : shrt;
     return ((a > b ? a : b) + 127) / 128 * 128;
 }
-__host__ __device__ inline size_t decode_smem_bytes(int njobs, int E, int FF, int HD) {
+__host__ __device__ inline size_t decode_smem_bytes(int njobs, int E, int FF, int HD, int sub) {
     return (size_t)DNW * DS * DSLOT + 256 + ((size_t)njobs * sizeof(Job) + 127) / 128 * 128 + 64 * sizeof(LayerPtrs) + 1024 + 256 + kFoldBytes +
-           ((size_t)E * 4 + 127) / 128 * 128 + decode_stage_bytes(E, FF, HD);
+           ((size_t)E * 4 + 127) / 128 * 128 + decode_stage_bytes(E, FF, HD, sub);
 }
 
 // close the current profile interval: charge the time since t to slot k (CTA 0, thread 0 only).
@@ -519,20 +530,25 @@ __device__ __forceinline__ void publish_q8_block(const Pub& pub, int qoff, int s
     if (lane == 0) { if (SHARED) pub.shared(soff + b, sw); else pub.local(soff + b, sw); }
 }
 
+__device__ __forceinline__ double tree_sum8(double a, double b, double c, double d, double e, double f, double g, double h) {
+    return __dadd_rn(__dadd_rn(__dadd_rn(a, b), __dadd_rn(c, d)), __dadd_rn(__dadd_rn(e, f), __dadd_rn(g, h)));
+}
 // Per-layer job: this CTA's units, tiles split over its warps, partial sums folded in
 // shared memory in warp order by warp 0, which then calls epi(g, lane, v0, v1) with the
 // complete sums rounded to fp32.  A job that is K-split across CTAs (ks > 1; down projection)
 // adds one hop: the CTAs of splits 1.. publish their double partial sums as tagged word pairs,
 // the CTA of split 0 waits for them, adds them to its own in split order and calls epi.
 // Every warp passes the same number of __syncthreads, also after a wait gave up.
+// bias: added to complete sums by epi; requested before the tiles are worked on (it comes from the L2).
 template <class Epi>
 __device__ MI_PIECE bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, int j, int lane,
-                                            const int8_t* xq_s, const float2* xs_s, const Pub& pub, Epi epi) {
+                                            const int8_t* xq_s, const float2* xs_s, const Pub& pub, const float* __restrict__ bias, Epi epi) {
     const Job jb = ws.jobs[j];                          // registers: the fields are used many times
     bool ok = true;
     int uidx = 0;
     for (int u = ws.first_cta_unit(jb); u < jb.n_units; u += ws.ggrid, uidx++) {
         const UnitShape s = unit_shape(jb, u, uidx);
+        const float bv = bias && ws.warp == 0 ? __ldg(bias + (s.g + jb.g_off) * 32 + lane) : 0.f;
         double a0 = 0.0, a1 = 0.0;
         for (int i = (ws.warp - s.wrot) & (DNW - 1); i < s.n; i += DNW) {
             const bool first = i < s.ntu;                       // which of the unit's two accumulators (gate / up) the tile feeds
@@ -545,9 +561,9 @@ __device__ MI_PIECE bool run_cta_job(WarpStream& ws, const DecodeParams& P, cons
         fb[(ws.warp * 2 + 1) * 32 + lane] = a1;
         __syncthreads();
         if (ws.warp == 0) {
-            double v0 = fb[lane], v1 = fb[32 + lane];
-            #pragma unroll
-            for (int w = 1; w < DNW; w++) { v0 = __dadd_rn(v0, fb[(w * 2) * 32 + lane]); v1 = __dadd_rn(v1, fb[(w * 2 + 1) * 32 + lane]); }
+            // (a tree: the seven additions one after the other were 130 cycles of every phase)
+            double v0 = tree_sum8(fb[lane], fb[64 + lane], fb[128 + lane], fb[192 + lane], fb[256 + lane], fb[320 + lane], fb[384 + lane], fb[448 + lane]);
+            const double v1 = jb.nacc > 1 ? tree_sum8(fb[32 + lane], fb[96 + lane], fb[160 + lane], fb[224 + lane], fb[288 + lane], fb[352 + lane], fb[416 + lane], fb[480 + lane]) : 0.0;
             const int gg = s.g + jb.g_off;
             if (jb.ks > 1) {
                 const int slot = P.xo.dpart + ((gg * (kMaxKSplit - 1)) * 32 + lane) * 2;
@@ -564,11 +580,11 @@ __device__ MI_PIECE bool run_cta_job(WarpStream& ws, const DecodeParams& P, cons
                         #pragma unroll
                         for (int q = 0; q < kMaxKSplit - 1; q++)
                             if (q < jb.ks - 1) v0 = __dadd_rn(v0, __longlong_as_double((long long)(((unsigned long long)pw[2 * q + 1] << 32) | pw[2 * q])));
-                        epi(gg, lane, __double2float_rn(v0), 0.f);
+                        epi(gg, lane, __double2float_rn(v0), 0.f, bv);
                     }
                 }
             } else {
-                epi(gg, lane, __double2float_rn(v0), __double2float_rn(v1));
+                epi(gg, lane, __double2float_rn(v0), __double2float_rn(v1), bv);
             }
         }
         prof_mark(P, 19);
@@ -643,26 +659,24 @@ __device__ __forceinline__ bool stage_norm_q8_t(const DecodeParams& P, float* h_
         for (int k = 0; k < NB; k++) if (valid >> k & 1u) x[k] = __fadd_rn(x[k], __uint_as_float(aw[k]));
         prof_mark(P, 28);
     }
-    double ss = 0.0;
+    double s2[2] = {0.0, 0.0};                           // two chains
     #pragma unroll
     for (int k = 0; k < NB; k++) {
         if (valid >> k & 1u) {
             const int e = (warp + k * DNW) * 32 + lane;
             h_s[e] = x[k];
             if (commit && (int)blockIdx.x == P.attn_ctas) __stcg(commit + e, x[k]);
-            const double xd = x[k]; ss = __fma_rn(xd, xd, ss);
+            const double xd = x[k]; s2[k & 1] = __fma_rn(xd, xd, s2[k & 1]);
         }
     }
+    double ss = __dadd_rn(s2[0], s2[1]);
     #pragma unroll
     for (int o = 16; o; o >>= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
     if (lane == 0) red[warp] = ss;
     prof_mark(P, 23);
     if (!__syncthreads_and(ok ? 1 : 0)) return false;
     prof_mark(P, 24);
-    double tot = 0.0;
-    #pragma unroll
-    for (int v = 0; v < DNW; v++) tot = __dadd_rn(tot, red[v]);
-    const float mean = __double2float_rn(__ddiv_rn(tot, (double)E));
+    const float mean = __double2float_rn(div_known(tree_sum8(red[0], red[1], red[2], red[3], red[4], red[5], red[6], red[7]), (double)E, P.inv_e));
     const float scale = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(mean, eps)));
     // quantize: this thread's EPL elements of block qt_b (vectors beyond 256 * EPL elements: further rounds)
     for (int t = tid; (t & ~31) / LPB < nb; t += DNT) {              // warp-uniform trip count: the folds below are warp-wide
@@ -844,23 +858,26 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ double half_to_double(unsigned w) { return (double)__half2float(__ushort_as_half((unsigned short)w)); }
 
 template <int HD, int G>
 __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, int pos, uint8_t* stage, unsigned tag_in, const Pub pub) {
-    using SM = SplitSmem<HD>;
+    const SplitSmem lay{HD, P.split_sub};
+    constexpr int KLD = 2 * HD + 64, VLD = 2 * HD + 32;
+    const int SUB = P.split_sub, SCL = lay.scl();
     constexpr int NTW = HD >= 64 ? HD / 64 : 1, VW = HD / 8 / NTW, SW = HD + 2;      // 8-dim tiles per warp of the value product, warps that have some; doubles per partial
-    double* qs = reinterpret_cast<double*>(stage + SM::q); double* wt = reinterpret_cast<double*>(stage + SM::wt);      // q [dim of a lane][lane], weights [step of 4][lane]
-    uint8_t* ks = stage + SM::k; uint8_t* vs = stage + SM::v;
-    float* sc = reinterpret_cast<float*>(stage + SM::sc);
-    double* rm = reinterpret_cast<double*>(stage + SM::st); double* rl = rm + 8; double* rf = rl + 8;                    // per head: running maximum, denominator, rescale factor
-    double* red = reinterpret_cast<double*>(stage + SM::red);
+    double* qs = reinterpret_cast<double*>(stage); double* wt = reinterpret_cast<double*>(stage + lay.wt());      // q [dim of a lane][lane], weights [step of 4][lane]
+    uint8_t* ks = stage + lay.k(); uint8_t* vs = stage + lay.v();
+    float* sc = reinterpret_cast<float*>(stage + lay.sc());
+    double* rm = reinterpret_cast<double*>(stage + lay.st()); double* rl = rm + 8; double* rf = rl + 8;                    // per head: running maximum, denominator, rescale factor
+    double* red = reinterpret_cast<double*>(stage + lay.red());
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int Lp = pos + 1, nch = attn_chunks(Lp, min(P.max_chunks, (int)gridDim.x / P.NKV)), nq = P.NH * HD;
     bool ok = true;
     if ((int)blockIdx.x < P.NKV * nch) {
         const int kvh = blockIdx.x / nch, ch = blockIdx.x - kvh * nch, h0 = kvh * G;
-        const int p0 = (int)((long long)ch * Lp / nch), p1 = (int)((long long)(ch + 1) * Lp / nch), n = p1 - p0, nsub = (n + kSplitSub - 1) / kSplitSub;
+        const int p0 = (int)((long long)ch * Lp / nch), p1 = (int)((long long)(ch + 1) * Lp / nch), n = p1 - p0, nsub = (n + SUB - 1) / SUB;
         const bool has_new = ch == nch - 1;
         const size_t lbase = (size_t)l * P.max_seq * P.KVD + (size_t)kvh * HD;
         auto sub_begin = [&](int s) { return p0 + n * s / nsub; };
@@ -874,7 +891,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
         };
         // (A model of one layer waits for q first: between two steps nothing else orders the last position's rows before this read.)
         const bool early = P.L > 1;
-        if (early) { copy_rows(ks, SM::KLD, P.kc, 0); copy_rows(vs, SM::VLD, P.vc, 0); }
+        if (early) { copy_rows(ks, KLD, P.kc, 0); copy_rows(vs, VLD, P.vc, 0); }
         // q of the group, and k / v of the new position (packed order: dim d of a head sits at 2d (d < HD/2) or 2(d-HD/2)+1)
         constexpr int QN = (G * HD + DNT - 1) / DNT;
         unsigned qw[QN + 2], valid = 0;
@@ -890,7 +907,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
             }
             return k == QN ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
         }, qw);
-        if (!early) { copy_rows(ks, SM::KLD, P.kc, 0); copy_rows(vs, SM::VLD, P.vc, 0); }
+        if (!early) { copy_rows(ks, KLD, P.kc, 0); copy_rows(vs, VLD, P.vc, 0); }
         // the order the MMA reads q in: lane (row, t) takes the 16-byte pieces t, t + 4, .. of a row
         auto qslot = [](int row, int d) { return ((d >> 5) * 8 + (d & 7)) * 32 + row * 4 + ((d >> 3) & 3); };
         #pragma unroll
@@ -914,14 +931,14 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
             const int b0 = sub_begin(s), np = sub_begin(s + 1) - b0;
             cp_async_wait<1>();                     // the K rows (the V rows were requested after them)
             if (has_new && s == nsub - 1 && tid < HD) {
-                reinterpret_cast<__half*>(ks + (pos - b0) * SM::KLD)[tid] = knew;
-                reinterpret_cast<__half*>(vs + (pos - b0) * SM::VLD)[tid] = vnew;
+                reinterpret_cast<__half*>(ks + (pos - b0) * KLD)[tid] = knew;
+                reinterpret_cast<__half*>(vs + (pos - b0) * VLD)[tid] = vnew;
             }
             if (s == 0) { if (!__syncthreads_and(okq ? 1 : 0)) { ok = false; break; } } else __syncthreads();
             // scores: warp = every 8th group of 8 positions
             #pragma unroll 1
             for (int t = warp; t * 8 < np; t += DNW) {
-                const uint8_t* kr = ks + min(t * 8 + g, np - 1) * SM::KLD + t4 * 16;
+                const uint8_t* kr = ks + min(t * 8 + g, np - 1) * KLD + t4 * 16;
                 double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
                 #pragma unroll
                 for (int i = 0; i < HD / 32; i++) {
@@ -936,25 +953,26 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const int pp = t * 8 + 2 * t4 + e;
-                    if (pp < kSplitSub) sc[g * SM::SCL + pp] = pp < np ? __fmul_rn(__double2float_rn(__dadd_rn(c[0][e], c[1][e])), inv) : -INFINITY;
+                    if (pp < SUB) sc[g * SCL + pp] = pp < np ? __fmul_rn(__double2float_rn(__dadd_rn(c[0][e], c[1][e])), inv) : -INFINITY;
                 }
             }
             __syncthreads();
             prof_mark(P, 27);
-            if (s + 1 < nsub) copy_rows(ks, SM::KLD, P.kc, s + 1); else cp_async_commit();
+            if (s + 1 < nsub) copy_rows(ks, KLD, P.kc, s + 1); else cp_async_commit();
             // weights: one warp per head
             if (warp < G) {
-                float x[kSplitSub / 32], m = -INFINITY;
+                float x[kSplitSubMax / 32], m = -INFINITY;
                 #pragma unroll
-                for (int i = 0; i < kSplitSub / 32; i++) { x[i] = lane + 32 * i < np ? sc[warp * SM::SCL + lane + 32 * i] : -INFINITY; m = fmaxf(m, x[i]); }
+                for (int i = 0; i < kSplitSubMax / 32; i++) { x[i] = lane + 32 * i < np ? sc[warp * SCL + lane + 32 * i] : -INFINITY; m = fmaxf(m, x[i]); }
                 m = warp_max_float(m);
                 const double mo = rm[warp], mn = fmax(mo, (double)m);
                 double ls = 0.0;
                 #pragma unroll
-                for (int i = 0; i < kSplitSub / 32; i++) {
+                for (int i = 0; i < kSplitSubMax / 32; i++) {
+                    if (32 * i >= np) break;                                               // warp-uniform
                     const double w = lane + 32 * i < np ? exp_shared((double)x[i] - mn) : 0.0;
                     const int pp = lane + 32 * i;
-                    wt[(pp >> 2) * 32 + warp * 4 + (pp & 3)] = w;
+                    if (pp < SUB) wt[(pp >> 2) * 32 + warp * 4 + (pp & 3)] = w;
                     ls = __dadd_rn(ls, w);
                 }
                 #pragma unroll
@@ -982,7 +1000,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                     #pragma unroll
                     for (int c = 0; c < 2; c++) {
                         if ((u + c) * 4 >= np) break;                                      // warp-uniform
-                        const uint8_t* v = vr + min((u + c) * 4 + t4, np - 1) * SM::VLD;
+                        const uint8_t* v = vr + min((u + c) * 4 + t4, np - 1) * VLD;
                         const double w = wt[(u + c) * 32 + lane];
                         if constexpr (NTW == 2) {
                             const unsigned vw = *reinterpret_cast<const unsigned*>(v);
@@ -994,7 +1012,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                 }
             }
             __syncthreads();                        // scores, weights and V rows may be written again
-            if (s + 1 < nsub) copy_rows(vs, SM::VLD, P.vc, s + 1);
+            if (s + 1 < nsub) copy_rows(vs, VLD, P.vc, s + 1);
         }
         if (!ok) cp_async_wait<0>();                // copies in flight target the staging area
         prof_mark(P, 15);
@@ -1007,7 +1025,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                     for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + i, __dadd_rn(o[0][i][e], o[1][i][e]));
             }
             if (tid < G) __stcg(P.attn_part + ((size_t)(h0 + tid) * P.max_chunks + ch) * SW + HD, rl[tid]);
-            __threadfence();                        // the partial, and the new position's rows, before the word that announces them
+            fence_acq_rel_gpu();                    // the partial, and the new position's rows, before the word that announces them
             __syncthreads();
             if (tid < G) pub.local(P.xo.attm + (h0 + tid) * P.max_chunks + ch, __float_as_uint((float)rm[tid]));
         }
@@ -1022,7 +1040,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
         for (int k = 0; k < kMaxChunkWords; k++) if (lane + 32 * k < nch) valid |= 1u << k;
         const unsigned long long* mv = P.xw + P.xo.attm + (size_t)head * P.max_chunks;
         const bool okm = tw_poll(P, pub.tag, valid, [&](int k) { return mv + lane + 32 * k; }, mw);
-        __threadfence();
+        fence_acq_rel_gpu();
         float m = -INFINITY;
         #pragma unroll
         for (int k = 0; k < kMaxChunkWords; k++) if (valid >> k & 1u) m = fmaxf(m, __uint_as_float(mw[k]));
@@ -1031,9 +1049,13 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
         const int mine = (nch - warp + DNW - 1) / DNW;
         const double* gp = P.attn_part + ((size_t)head * P.max_chunks + warp) * SW;
         double f_l = 0.0;
-        if (lane < mine) {
-            const float mc = __uint_as_float((unsigned)tw_ld(mv + warp + DNW * lane));
-            f_l = mc == -INFINITY ? 0.0 : exp_shared((double)mc - (double)m);
+        {
+            const int c = warp + DNW * lane;                                               // its maximum is word c / 32 of lane c % 32
+            unsigned w = 0;
+            #pragma unroll
+            for (int k = 0; k < kMaxChunkWords; k++) { const unsigned x = __shfl_sync(0xffffffffu, mw[k], c & 31); if ((c >> 5) == k) w = x; }
+            const float mc = __uint_as_float(w);
+            if (lane < mine) f_l = mc == -INFINITY ? 0.0 : exp_shared((double)mc - (double)m);
         }
         double ob = 0.0, lb = lane < mine ? __dmul_rn(__ldcg(gp + (size_t)lane * DNW * SW + HD), f_l) : 0.0;
         for (int i0 = 0; i0 < mine; i0 += 8) {
@@ -1257,7 +1279,7 @@ constexpr int kAttnRows = kShortAttnMax;
 template <int HD> __host__ __device__ constexpr int attn_row_bytes() { return 2 * HD + 16; }
 __host__ __device__ inline size_t attn_dedicated_smem(int HD, int HPC) {
     return (size_t)2 * kAttnRows * (2 * HD + 16) + (size_t)HPC * (HD + 16) * 8 + (size_t)HPC * kAttnRows * 8 + (size_t)DNW * HPC * HD * 8 +
-           (size_t)DNW * HPC * 8 + (size_t)HPC * kAttnRows * 4 + 64;
+           (size_t)DNW * HPC * 8 + (size_t)HPC * kAttnRows * 4 + (size_t)DNW * HPC * kAttnRows * 8 + 64;
 }
 // query heads per attention CTA: two where the group size is even (1.5B: six CTAs of two heads; three heads per CTA
 // measured 4.5 us per layer on the critical path), one where it is odd or at most two
@@ -1297,7 +1319,8 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
     double* wt = qs + HPC * LPP * QSTR;                                         // [HPC][rows]
     double* ow = wt + HPC * kAttnRows;                                          // [DNW][HPC][HD]
     double* lw = ow + DNW * HPC * HD;                                           // [DNW][HPC]
-    float* sc = reinterpret_cast<float*>(lw + DNW * HPC);                       // [HPC][rows]
+    double* pd = lw + DNW * HPC;                                                // [DNW][HPC][rows] partial scores
+    float* sc = reinterpret_cast<float*>(pd + DNW * HPC * kAttnRows);           // [HPC][rows]
     // the rows of this (layer, position) should be on their way already; a launch's first layer requests them here
     if (!(pf.layer == l && pf.pos == pos)) {
         if (pf.pending) { (void)mbar_wait_bounded(pf.bar, pf.parity); pf.parity ^= 1u; }
@@ -1333,39 +1356,48 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
     prof_mark(P, 27);
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
     const int a0 = (int)((long long)Lp * warp / DNW), a1 = (int)((long long)Lp * (warp + 1) / DNW), np = a1 - a0;
-    // pass 1: thread = position (the range is at most 256 rows).  A thread walks its K row front to back, one fp16 ->
-    // double conversion of an element serving all heads, and adds the products in dimension order with one accumulator
-    // per head: the order in which the reference's CPU program adds this sum (src/cpu_infer.cpp:127-130).  q comes as
-    // 16-byte broadcast loads (every lane reads the same address); rows are 16 bytes longer than their data, so the
-    // eight lanes of a quarter warp cover all banks.  (Eight lanes per
-    // position with a shuffle tree per sweep measured 1.8 us per layer at a hundred positions: the conversions and the
-    // tree of every sweep were serial.)
-    if (warp * 32 < Lp) {
-        const uint4* kr = reinterpret_cast<const uint4*>(Kb + (size_t)min(tid, Lp - 1) * RSB);
-        double acc[HPC];
+    // pass 1: a warp takes an eighth of the dimensions, q of which stays in its registers, lane = position: one fp16 -> double
+    // conversion of a K element serves all heads, and the eight partial dot products meet in shared memory.  (A thread per position
+    // over all dimensions reads q as broadcasts, 128 of them per warp at four cycles each: 1.25 us per layer at a hundred positions.)
+    // Rows are 16 bytes longer than their data, so the eight lanes of a quarter warp cover all banks.
+    {
+        constexpr int DW = HD / DNW;                                            // dims of a warp
+        double qr[HPC][DW];
         #pragma unroll
-        for (int j = 0; j < HPC; j++) acc[j] = 0.0;
+        for (int j = 0; j < HPC; j++)
+            #pragma unroll
+            for (int e = 0; e < DW; e++) qr[j][e] = qs[(j * LPP + (warp * DW + e) / DPL) * QSTR + (warp * DW + e) % DPL];
         #pragma unroll 2
-        for (int c = 0; c < HD / 8; c++) {
-            const uint4 kk = kr[c];
-            const __half2* hh = reinterpret_cast<const __half2*>(&kk);
-            double kd[8];
-            #pragma unroll
-            for (int e = 0; e < 4; e++) { const float2 f = __half22float2(hh[e]); kd[2 * e] = (double)f.x; kd[2 * e + 1] = (double)f.y; }
-            #pragma unroll
-            for (int j = 0; j < HPC; j++) {
+        for (int p0 = 0; p0 < Lp; p0 += 32) {
+            const uint8_t* kr = Kb + (size_t)min(p0 + lane, Lp - 1) * RSB + warp * (DW * 2);
+            unsigned kw[DW / 2];
+            if constexpr (DW >= 8) {
                 #pragma unroll
-                for (int e = 0; e < 8; e += 2) {
-                    const int d = c * 8 + e;
-                    const double2 qq = *reinterpret_cast<const double2*>(qs + (j * LPP + d / DPL) * QSTR + d % DPL);
-                    acc[j] = __fma_rn(qq.x, kd[e], acc[j]);
-                    acc[j] = __fma_rn(qq.y, kd[e + 1], acc[j]);
-                }
+                for (int c = 0; c < DW / 8; c++) { const uint4 v = reinterpret_cast<const uint4*>(kr)[c]; kw[4 * c] = v.x; kw[4 * c + 1] = v.y; kw[4 * c + 2] = v.z; kw[4 * c + 3] = v.w; }
+            } else {
+                const uint2 v = *reinterpret_cast<const uint2*>(kr); kw[0] = v.x; kw[1] = v.y;
             }
-        }
-        if (tid < Lp) {
+            double acc[HPC][2];                                                 // two chains per head
             #pragma unroll
-            for (int j = 0; j < HPC; j++) sc[j * kAttnRows + tid] = __fmul_rn(__double2float_rn(acc[j]), inv);
+            for (int j = 0; j < HPC; j++) acc[j][0] = acc[j][1] = 0.0;
+            #pragma unroll
+            for (int e = 0; e < DW / 2; e++) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&kw[e]));
+                const double k0 = f.x, k1 = f.y;
+                #pragma unroll
+                for (int j = 0; j < HPC; j++) { acc[j][0] = __fma_rn(qr[j][2 * e], k0, acc[j][0]); acc[j][1] = __fma_rn(qr[j][2 * e + 1], k1, acc[j][1]); }
+            }
+            #pragma unroll
+            for (int j = 0; j < HPC; j++) pd[(warp * HPC + j) * kAttnRows + p0 + lane] = __dadd_rn(acc[j][0], acc[j][1]);
+        }
+    }
+    __syncthreads();
+    if (tid < Lp) {
+        #pragma unroll
+        for (int j = 0; j < HPC; j++) {
+            const double* p = pd + j * kAttnRows + tid;
+            constexpr int S = HPC * kAttnRows;
+            sc[j * kAttnRows + tid] = __fmul_rn(__double2float_rn(tree_sum8(p[0], p[S], p[2 * S], p[3 * S], p[4 * S], p[5 * S], p[6 * S], p[7 * S])), inv);
         }
     }
     __syncthreads();
@@ -1689,10 +1721,10 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                 const int jn = 4 * l + (k == 0 ? 0 : k == 2 ? 1 : k == 3 ? 2 : 3);
                 const float* bias = sm.lp[l].bqkv;
                 const int nq = P.NH * HD;
-                ok = run_cta_job(ws, P, sm, jn, lane, xq_s, xs_s, pub, [&](int g, int ln, float v0, float v1) {
+                ok = run_cta_job(ws, P, sm, jn, lane, xq_s, xs_s, pub, k == 0 ? bias : nullptr, [&](int g, int ln, float v0, float v1, float bv) {
                     if (k == 0) {                                            // + bias, RoPE, packed q / k / v
                         const int p = g * 32 + ln;
-                        const float v = __fadd_rn(v0, __ldg(bias + p));
+                        const float v = __fadd_rn(v0, bv);
                         const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
                         float out = v;
                         if (p < nq + P.KVD) {                                  // q or k: rotate the (even, odd) lane pair

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(1024) vf_norm_quant(const DecodeParams P, cons
     double tot = lane < nw ? red[lane] : 0.0;
     #pragma unroll
     for (int o = 16; o; o >>= 1) tot = __dadd_rn(tot, __shfl_xor_sync(0xffffffffu, tot, o));
-    const float mean = __double2float_rn(__ddiv_rn(tot, (double)E));
+    const float mean = __double2float_rn(div_known(tot, (double)E, P.inv_e));
     const float scale = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(mean, P.eps)));
     #pragma unroll
     for (int r = 0; r < R; r++) {
