@@ -89,20 +89,29 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
     const int ch = (int)(blockIdx.x % p.nch), rest = (int)(blockIdx.x / p.nch), kvh = rest % p.NKV, q0 = (nqb - 1 - rest / p.NKV) * QB;
     const int nq = min(QB, p.M - q0);
     pdl_launch_dependents();
-    pdl_wait_prior();
+    if (!p.early) pdl_wait_prior();
     const int posq0 = p.pos_arr ? __ldg(p.pos_arr + q0) : (p.pos0 ? __ldg(p.pos0) : p.pos0_val) + q0;      // position of query q0; the CTA's others follow (QB > 1: one sequence)
     const size_t base = (p.slot_arr ? (size_t)__ldg(p.slot_arr + q0) * (size_t)p.slab_stride : 0) + (size_t)p.layer * p.max_seq * p.KVD + (size_t)kvh * HD;
     const int Lp = posq0 + nq;                      // positions the last query sees
     const int p0 = (int)((long long)Lp * ch / p.nch), p1 = (int)((long long)Lp * (ch + 1) / p.nch);
-    auto copy_rows = [&](uint8_t* dst, int ld, const __half* src, int b0) {                  // rows b0 .. of the step, 16 bytes per thread and copy
-        const int np = min(SUB, p1 - b0);
-        for (int i = tid; i < np * (HD / 8); i += kAT) {
-            const int r = i / (HD / 8), c = i - r * (HD / 8);
+    auto copy_range = [&](uint8_t* dst, int ld, const __half* src, int b0, int lo, int hi) {  // rows lo .. hi of the step at b0, 16 bytes per thread and copy
+        for (int i = tid; i < (hi - lo) * (HD / 8); i += kAT) {
+            const int r = i / (HD / 8) + lo - b0, c = i % (HD / 8);
             cp16(dst + r * ld + c * 16, src + base + (size_t)(b0 + r) * p.KVD + c * 8);
         }
-        cp_commit();
     };
-    if (p0 < p1) { copy_rows(ks, SM::KLD, p.kc, p0); copy_rows(vs, SM::VLD, p.vc, p0); }
+    auto copy_rows = [&](uint8_t* dst, int ld, const __half* src, int b0) { copy_range(dst, ld, src, b0, b0, min(b0 + SUB, p1)); cp_commit(); };
+    // In a pass the rows of earlier positions have been there since before it began: they are requested before the kernel waits
+    // for the projection, and the rows that it writes after that.
+    const int step1 = min(p0 + SUB, p1), fresh = p.early ? min(max(p.pos_arr ? posq0 : posq0 - q0, p0), step1) : p0;
+    if (p.early) {
+        if (p0 < fresh) { copy_range(ks, SM::KLD, p.kc, p0, p0, fresh); copy_range(vs, SM::VLD, p.vc, p0, p0, fresh); }
+        pdl_wait_prior();
+    }
+    if (p0 < p1) {
+        copy_range(ks, SM::KLD, p.kc, p0, fresh, step1); cp_commit();
+        copy_range(vs, SM::VLD, p.vc, p0, fresh, step1); cp_commit();
+    }
     // q into the order the MMA reads it: lane (row, t) takes the 16-byte pieces t, t + 4, .. of a row: its dim s is 8 (4 (s / 8) + t) + s % 8
     for (int i = tid; i < R * HD; i += kAT) {
         const int d = i % HD, row = i / HD, qi = row / G, h = row - qi * G, tt = (d >> 3) & 3, s = (d >> 5) * 8 + (d & 7);
@@ -262,54 +271,82 @@ __global__ void __launch_bounds__(kAT, 2) attn_tok_kernel(const __grid_constant_
     }
 }
 
-// Fold the chunks of one (query, kv head) against their common maximum.  Thread = four dims of one head.
-template <int HD>
-__global__ void __launch_bounds__(kAT) attn_tok_merge(const __grid_constant__ AttnParams p, int G) {
-    extern __shared__ __align__(16) double fs[];                     // [G][nch] rescale factors, then [G] denominators
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, token = blockIdx.y, kvh = blockIdx.x, nch = p.nch;
+// Fold the chunks of one (query, head) against their common maximum.  What bounds it is latency (a launch, one trip to the L2, an
+// exponential, a division), so nothing waits for anything it need not: the first eight chunks of a warp are requested before the
+// maxima are known.  WPH warps share a head: all eight of a CTA where there are many chunks, one where there are few (and
+// mostly many queries: a CTA per head would be idle but for a warp or two, 333 queries of 12 heads took 22 us).  Lane = the dims lane,
+// lane + 32, ...  (A CTA per kv head that read maxima, factors and then all chunks in turn took 6.8 us for 5 queries and 29
+// chunks, as long as the chunks themselves.)
+template <int HD, int WPH>
+__global__ void __launch_bounds__(kAT) attn_tok_merge(const __grid_constant__ AttnParams p) {
+    constexpr int D = HD / 32, U = 8;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % WPH, nch = p.nch;
+    const int item = blockIdx.x * (kAW / WPH) + warp / WPH, token = item / p.NH, head = item - token * p.NH;
     pdl_launch_dependents();
     pdl_wait_prior();
-    const double* gp = p.part + ((size_t)token * p.NH + (size_t)kvh * G) * nch * (HD + 2);
-    double* den = fs + G * nch;
-    for (int h = warp; h < G; h += kAW) {
-        double m = -INFINITY, l = 0.0;
-        for (int c = lane; c < nch; c += 32) m = fmax(m, __ldcg(gp + ((size_t)h * nch + c) * (HD + 2) + HD));
+    if (WPH == 1 && token >= p.M) return;
+    const double* gp = p.part + (size_t)item * nch * (HD + 2);
+    const int mine = (nch - sub + WPH - 1) / WPH;                    // chunks sub, sub + WPH, ..
+    const double* own = gp + (size_t)sub * (HD + 2);
+    constexpr size_t stride = (size_t)WPH * (HD + 2);
+    auto fetch = [&](double (&v)[U][D], int i0) {
         #pragma unroll
-        for (int q = 16; q; q >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, q));
-        for (int c = lane; c < nch; c += 32) {
-            const double* s = gp + ((size_t)h * nch + c) * (HD + 2) + HD;
-            const double mc = __ldcg(s), f = mc == -INFINITY ? 0.0 : exp(mc - m);
-            fs[h * nch + c] = f;
-            l = __fma_rn(__ldcg(s + 1), f, l);
+        for (int u = 0; u < U; u++)
+            #pragma unroll
+            for (int d = 0; d < D; d++) v[u][d] = i0 + u < mine ? __ldcg(own + (size_t)(i0 + u) * stride + 32 * d + lane) : 0.0;
+    };
+    double v[U][D], o[D], l = 0.0, m = -INFINITY;
+    #pragma unroll
+    for (int d = 0; d < D; d++) o[d] = 0.0;
+    fetch(v, 0);
+    for (int c = lane; c < nch; c += 32) m = fmax(m, __ldcg(gp + (size_t)c * (HD + 2) + HD));
+    #pragma unroll
+    for (int q = 16; q; q >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, q));
+    for (int b = 0; b < mine; b += 32) {                             // lane i prepares the factor of the i-th
+        double f_l = 0.0;
+        if (b + lane < mine) {
+            const double* s = own + (size_t)(b + lane) * stride + HD;
+            const double mc = __ldcg(s);
+            f_l = mc == -INFINITY ? 0.0 : exp(mc - m);
+            l = __fma_rn(__ldcg(s + 1), f_l, l);
         }
-        #pragma unroll
-        for (int q = 16; q; q >>= 1) l = __dadd_rn(l, __shfl_xor_sync(0xffffffffu, l, q));
-        if (lane == 0) den[h] = l;
-    }
-    __syncthreads();
-    for (int i = tid; i < G * (HD / 4); i += kAT) {
-        const int h = i / (HD / 4), d = (i - h * (HD / 4)) * 4;
-        const double* s = gp + (size_t)h * nch * (HD + 2) + d;
-        double o[4] = {0.0, 0.0, 0.0, 0.0};
-        constexpr int U = 8;
-        for (int c0 = 0; c0 < nch; c0 += U) {
-            double2 a[U], b[U];
+        for (int i0 = b; i0 < min(mine, b + 32); i0 += U) {
+            if (i0 > 0) fetch(v, i0);
             #pragma unroll
             for (int u = 0; u < U; u++) {
-                const double2* sp = reinterpret_cast<const double2*>(s + (size_t)min(c0 + u, nch - 1) * (HD + 2));
-                a[u] = __ldcg(sp); b[u] = __ldcg(sp + 1);
-            }
-            #pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (c0 + u < nch) {
-                    const double f = fs[h * nch + c0 + u];
-                    o[0] = __fma_rn(a[u].x, f, o[0]); o[1] = __fma_rn(a[u].y, f, o[1]); o[2] = __fma_rn(b[u].x, f, o[2]); o[3] = __fma_rn(b[u].y, f, o[3]);
+                const double f = __shfl_sync(0xffffffffu, f_l, (i0 + u) & 31);
+                if (i0 + u < mine) {
+                    #pragma unroll
+                    for (int d = 0; d < D; d++) o[d] = __fma_rn(v[u][d], f, o[d]);
                 }
             }
         }
-        const double l = den[h];
-        attn_emit(p, token, (kvh * G + h) * HD + d, make_float4(__double2float_rn(__ddiv_rn(o[0], l)), __double2float_rn(__ddiv_rn(o[1], l)),
-                                                                __double2float_rn(__ddiv_rn(o[2], l)), __double2float_rn(__ddiv_rn(o[3], l))));
+    }
+    #pragma unroll
+    for (int q = 16; q; q >>= 1) l = __dadd_rn(l, __shfl_xor_sync(0xffffffffu, l, q));
+    auto emit = [&](int block, float y) {                            // 32 dims, one per lane
+        const int e = head * HD + block * 32;
+        p.out[(size_t)token * p.NH * HD + e + lane] = y;
+        if (p.x.q) store_tok_block(p.x, e >> 5, token, lane, y);
+    };
+    if constexpr (WPH == 1) {
+        float y[D];
+        #pragma unroll
+        for (int d = 0; d < D; d++) y[d] = __double2float_rn(__ddiv_rn(o[d], l));
+        #pragma unroll
+        for (int d = 0; d < D; d++) emit(d, y[d]);
+    } else {
+        static_assert(WPH == kAW, "a CTA per head");
+        __shared__ double red[kAW][HD], den[kAW];
+        #pragma unroll
+        for (int d = 0; d < D; d++) red[warp][32 * d + lane] = o[d];
+        if (lane == 0) den[warp] = l;
+        __syncthreads();
+        if (warp >= D) return;
+        double s = red[0][warp * 32 + lane], dn = den[0];
+        #pragma unroll
+        for (int w = 1; w < kAW; w++) { s = __dadd_rn(s, red[w][warp * 32 + lane]); dn = __dadd_rn(dn, den[w]); }
+        emit(warp, __double2float_rn(__ddiv_rn(s, dn)));
     }
 }
 
@@ -347,7 +384,8 @@ int launch_qb(mi_ctx* ctx, const AttnParams& p, bool pdl) {
     }
     const int units = p.NKV * ((p.M + QB - 1) / QB);
     MI_CUDA(ctx, launch_k(pdl, kern, dim3(units * p.nch), dim3(kAT), smem, ctx->stream, p));
-    if (p.nch > 1) MI_CUDA(ctx, launch_k(pdl, attn_tok_merge<HD>, dim3(p.NKV, p.M), dim3(kAT), (size_t)(G * p.nch + G) * 8, ctx->stream, p, G));
+    if (p.nch > 2 * kAW) MI_CUDA(ctx, launch_k(pdl, attn_tok_merge<HD, kAW>, dim3(p.NH * p.M), dim3(kAT), 0, ctx->stream, p));
+    else if (p.nch > 1) MI_CUDA(ctx, launch_k(pdl, attn_tok_merge<HD, 1>, dim3((p.NH * p.M + kAW - 1) / kAW), dim3(kAT), 0, ctx->stream, p));
     return MI_OK;
 }
 }  // namespace

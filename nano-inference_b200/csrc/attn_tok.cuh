@@ -15,6 +15,7 @@ struct AttnParams {
     double* part;                           // [M][NH][nch][HD + 2] when nch > 1: chunk sums, maximum, denominator
     int nch;                                // chunks per causal range
     int qb;                                 // queries per CTA
+    int early;                              // the cache rows below the first query's position may be read before the kernels ahead have finished
 };
 // the cut for M queries whose longest causal range has about lp_max positions (ragged: every query has a sequence of its own)
 struct AttnPlan { int qb, nch; size_t part_doubles; };

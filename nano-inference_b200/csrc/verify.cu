@@ -294,7 +294,7 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         gq.rope = RopeParams{b.q, NQ, m->HD, P.kc, P.vc, m->KVD, a.slab_stride, l, a.max_seq, P.rope_cs, P.rope_freq, P.rope_rows, pos0, pos_arr, slot_arr};
         if ((st = launch_gemm_tok(ctx, wqkv, pq, fused ? GEMM_QKV : GEMM_PLAIN, false, gq, pdl))) return st;
         if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_rope, dim3(((int)wqkv->rows / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, gq.rope, (const float*)b.Y, (int)wqkv->rows));
-        const AttnParams at{b.q, P.kc, P.vc, M, m->NH, m->NKV, m->HD, m->KVD, l, a.max_seq, pos0, 0, pos_arr, slot_arr, a.slab_stride, b.att, attf, b.attn_part, 1, 1};
+        const AttnParams at{b.q, P.kc, P.vc, M, m->NH, m->NKV, m->HD, m->KVD, l, a.max_seq, pos0, 0, pos_arr, slot_arr, a.slab_stride, b.att, attf, b.attn_part, 1, 1, 1};
         if ((st = launch_attn_tok(ctx, at, pa, pdl))) return st;
         GemmParams go = g; go.x = attf; go.part = b.part; go.ldp = b.ldp;
         if ((st = launch_gemm_tok(ctx, wo, po, GEMM_PART, false, go, pdl))) return st;
@@ -440,7 +440,7 @@ extern "C" int mi_attn_splitkv(mi_ctx* ctx, const float* q_dev, const uint16_t* 
     int st = ensure_scratch(ctx, plan.part_doubles, 0);
     if (st != MI_OK) return st;
     const AttnParams p{q_dev, reinterpret_cast<const __half*>(kcache_dev), reinterpret_cast<const __half*>(vcache_dev), M, n_head, n_head_kv, head_dim, n_head_kv * head_dim,
-                       0, 0, nullptr, pos0, nullptr, nullptr, 0, out_dev, TokX{nullptr, nullptr, 0}, ctx->part, 1, 1};
+                       0, 0, nullptr, pos0, nullptr, nullptr, 0, out_dev, TokX{nullptr, nullptr, 0}, ctx->part, 1, 1, 0};
     return launch_attn_tok(ctx, p, plan, true);
 }
 
