@@ -405,7 +405,7 @@ def run_ours(args, rank, world, local_rank):
         return
 
     if args.workload == "gemm":
-        # multi-token GEMM (tcgen05 int8 MMA) on the lm_head shape (131 MB, larger than the L2): one weight pass for M tokens
+        # multi-token GEMM (int8 MMA) on the lm_head shape (131 MB, larger than the L2): one weight pass for M tokens
         rows, cols = (151936, 1536) if not args.shapes else SWEEP[0]
         g = torch.Generator(device="cuda"); g.manual_seed(7)
         n = rows * (cols // 32)
@@ -433,12 +433,12 @@ def run_ours(args, rank, world, local_rank):
             return
         ach = byt / (res[8] * 1e-3) / 1e9
         print(json.dumps({
-            "metric": "q4_0 x q8_0 multi-token GEMM (tcgen05 int8 MMA): HBM GB/s of one weight pass at M=8", "value": round(ach, 1), "unit": "GB/s",
+            "metric": "q4_0 x q8_0 multi-token GEMM (int8 MMA): HBM GB/s of one weight pass at M=8", "value": round(ach, 1), "unit": "GB/s",
             "n_gpus": world, "steps": args.steps, "warmup": warmup, "ms_per_step": round(res[8], 5), "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "uint4 x int8 -> int32 on tcgen05 (kind::i8), fp64 scaling on CUDA cores", "data": "synthetic",
+            "vs_baseline": None, "dtype": "uint4 x int8 -> int32 on tensor cores, fp64 scaling on CUDA cores", "data": "synthetic",
             "config": {"workload": f"gemm(config 3, GEMM part): {rows}x{cols}, M in 1,2,4,8,16", "l2": "matrix larger than L2"},
             "roofline": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4),
-                         "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})", "traffic": None, "kernel": "gemm_q4_q8_tc_kernel",
+                         "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})", "traffic": None, "kernel": "gemm_q4_q8_tok_kernel",
                          "algorithmic_bytes_per_launch": byt},
             "pass_us_by_M": {str(M): round(v * 1e3, 1) for M, v in res.items()}, "cost_of_8_tokens_vs_1": round(res[8] / res[1], 3),
             "gpu_launches": args.steps * 5,
@@ -479,7 +479,7 @@ def run_ours(args, rank, world, local_rank):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "fp16 K/V, fp64-carried scores, weights and sums, fp32 out",
             "data": "synthetic", "config": {"workload": "attn(config 3, attention part): contexts 512 / 8192 / 32768, M in 1, 8", "l2": "L2 flushed between timed calls"},
             "roofline": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4),
-                         "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})", "traffic": None, "kernel": "vf_attention",
+                         "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})", "traffic": None, "kernel": "attn_tok_kernel",
                          "algorithmic_bytes_per_launch": kv_bytes[32768]},
             "call_us": {f"ctx{c}_M{M}": round(v * 1e3, 1) for (c, M), v in res.items()},
             "kv_gbs": {f"ctx{c}_M{M}": round(kv_bytes[c] / (v * 1e-3) / 1e9, 1) for (c, M), v in res.items()},
@@ -530,7 +530,7 @@ def run_ours(args, rank, world, local_rank):
 
     if args.workload == "batch":
         # batched decode of independent sequences (the batched configuration: 3B shape, batch 1 / 16 / 64, 128-token seeded
-        # prompts, context <= 4096): every sequence advances one token per step; up to 16 share a weight pass
+        # prompts, context <= 4096): every sequence advances one token per step; up to 64 share a weight pass
         global MODEL_PRESET
         MODEL_PRESET = "3b"
         if rank == 0:
@@ -567,13 +567,13 @@ def run_ours(args, rank, world, local_rank):
         print(json.dumps({
             "metric": "batched greedy decode tok/s (all sequences), Qwen2.5-3B shape, batch 64, all-q4_0 weights, fp16 KV", "value": round(64 / (ms64 * 1e-3), 1),
             "unit": "tok/s", "n_gpus": world, "steps": K, "warmup": warmup, "ms_per_step": round(ms64, 4), "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "uint4 x int8 -> int32 on tcgen05 (kind::i8); fp64-carried sums stored fp32; fp16 KV", "data": "synthetic",
+            "vs_baseline": None, "dtype": "uint4 x int8 -> int32 on tensor cores; fp64-carried sums stored fp32; fp16 KV", "data": "synthetic",
             "config": {"workload": f"batch(config 4): Qwen2.5-3B shape, batch 1 / 16 / 64 independent sequences, {n_prompt}-token seeded prompts, "
                                    f"positions {n_prompt + warmup}..{n_prompt + warmup + K - 1}; 16 sequences per weight pass (batch 64 = 4 passes per step)",
                        "l2": "1.74 GB of weights per pass, larger than L2"},
             "roofline": {"bound": "hbm", "achieved": round(byt / (ms64 * 1e-3) / 1e9, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(byt / (ms64 * 1e-3) / 1e9 / peak, 4), "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})", "traffic": None,
-                         "kernel": "whole step (gemm_q4_q8_tc_kernel + vf_attention + glue)", "algorithmic_bytes_per_launch": byt,
+                         "kernel": "whole step (gemm_q4_q8_tok_kernel + attn_tok_kernel + glue)", "algorithmic_bytes_per_launch": byt,
                          "note": "algorithmic bytes count the weights once per step; batch 64 streams them four times"},
             "step_ms_by_batch": {str(B): round(v[0], 3) for B, v in res.items()},
             "tok_s_by_batch": {str(B): round(B / (v[0] * 1e-3), 1) for B, v in res.items()},
@@ -651,15 +651,15 @@ def run_ours(args, rank, world, local_rank):
         head = res[(512, 8)]
         byt = cfg.q4_weight_bytes_per_token + kvb * (512 + 8)
         print(json.dumps({
-            "metric": "M-token verify step (tcgen05 GEMM projections + M-query split-KV attention): tokens/s at M=8, context 512",
+            "metric": "M-token verify step (tensor-core projections + M-query split-KV attention): tokens/s at M=8, context 512",
             "value": round(8 / (head * 1e-3), 1), "unit": "tok/s", "n_gpus": world, "steps": max(3, min(args.steps, 20)), "warmup": warmup,
             "ms_per_step": round(head, 4), "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "uint4 x int8 -> int32 on tcgen05 (kind::i8); fp64-carried sums stored fp32; fp16 KV", "data": "synthetic",
+            "dtype": "uint4 x int8 -> int32 on tensor cores; fp64-carried sums stored fp32; fp16 KV", "data": "synthetic",
             "config": {"workload": "verify(config 3): Qwen2.5-1.5B shape, M in 1,2,4,8,16 drafted tokens per weight pass, KV cache N(0,1) fp16 at "
                                    "512 / 8192 / 32768 cached positions", "l2": "868 MB of weights per pass, larger than L2"},
             "roofline": {"bound": "hbm", "achieved": round(byt / (head * 1e-3) / 1e9, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(byt / (head * 1e-3) / 1e9 / peak, 4), "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})",
-                         "traffic": None, "kernel": "whole pass (gemm_q4_q8_tc_kernel + vf_attention + glue)", "algorithmic_bytes_per_launch": byt},
+                         "traffic": None, "kernel": "whole pass (gemm_q4_q8_tok_kernel + attn_tok_kernel + glue)", "algorithmic_bytes_per_launch": byt},
             "pass_ms": {f"ctx{c}_M{M}": round(v, 3) for (c, M), v in res.items()},
             "tok_s": {f"ctx{c}_M{M}": round(M / (v * 1e-3), 1) for (c, M), v in res.items()},
             "logits_identical_for_every_M": same,

@@ -193,9 +193,8 @@ MI_API int mi_gemv_q4_q8_noalloc(mi_ctx* ctx, const mi_weight* w, const int8_t* 
 
 /* Y[m][r] = the GEMV sum of row r against token vector m, for M = 1..16 token vectors in
  * one pass over the weights (speculative verify, chunked prefill, small batches).  The
- * integer block dot products run on the tensor cores (tcgen05.mma.kind::i8, one K=32 MMA
- * per q4_0 block, int32 accumulators in tensor memory), the per-block fp16 scaling on the
- * CUDA cores with the GEMV's own expression, so Y[m] carries exactly the bits
+ * integer block dot products run on the tensor cores (one K=32 int8 MMA per q4_0 block),
+ * the per-block fp16 scaling in double with the GEMV's one rounding per block, so Y[m] carries the bits
  * mi_gemv_q4_q8 gives for xq[m] alone, whatever M is.  xq_dev [M][cols] int8, xd_dev
  * [M][cols/32] fp16 bits, y_dev [M][rows] fp32; w must be a single matrix (count == 1).
  * Replaces gemv_dp4a_batch<T> (src/cuda_infer.cu:183-222, T <= 8) and the mma.sync path
@@ -363,9 +362,9 @@ MI_API int mi_verify_margins(mi_ctx* ctx, mi_model* model, int n, float* margins
 /* A batch object owns n_slots KV-cache slabs of max_seq positions each (fp16, laid out like the
  * model's own cache) for sequences decoded together.  mi_batch_step runs ONE decode step for n
  * of them: sequence i has its current token tokens_host[i] at position positions_host[i] of slab
- * slots_host[i] (distinct slots within a call).  Up to 16 sequences share one pass over the
- * weights as columns of the M-token step (tcgen05 GEMM, one attention CTA set per column over
- * that column's own slab); more sequences run further passes.  Every column is processed exactly
+ * slots_host[i] (distinct slots within a call).  Up to 64 sequences share one pass over the
+ * weights as columns of the M-token step (one attention CTA set per column over that
+ * column's own slab); more sequences run further passes.  Every column is processed exactly
  * as if it were alone: out_tokens_host[i] and logits_dev[i][n_vocab] are the bits a batch-1 decode
  * of that sequence gives.  Prompts enter the same way, one token per step and sequence (or through
  * mi_verify on the model's own cache for a single sequence).  The reference has no independent-

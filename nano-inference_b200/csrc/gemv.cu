@@ -167,7 +167,9 @@ static int launch_one(mi_ctx* ctx, const mi_weight* w, const GemvIO& io, int ksp
         if (st != MI_OK) return st;
         sc.part = ctx->part; sc.counters = ctx->counters;
     }
-    MI_CUDA(ctx, launch_k(true, kern, dim3((unsigned)ctas), dim3(NW * 32), smem, ctx->stream, sh, sc, io));
+    // A single matrix follows the quantizer of its vector and starts beside its tail (151936 x 1536: 28.8 -> 25.5 us per pair).  A stack
+    // is a sweep of its own, mostly behind an event or a copy, where a programmatic launch comes 2 us later than a plain one.
+    MI_CUDA(ctx, launch_k(w->count == 1, kern, dim3((unsigned)ctas), dim3(NW * 32), smem, ctx->stream, sh, sc, io));
     return MI_OK;
 }
 

@@ -180,7 +180,7 @@ struct GemvWarp {
     __device__ __forceinline__ void issue_one(const GemvShape& sh) {
         if (pc.u >= n_units) return;
         const int slot = issued % S;
-        const int bytes = min(kSlotTiles<KB>, sh.nt - pc.t * kSlotTiles<KB>) * tile_bytes(KB);
+        const int bytes = KB == 8 ? TB : min(kSlotTiles<KB>, sh.nt - pc.t * kSlotTiles<KB>) * tile_bytes(KB);
         mbar_expect_tx(&bars[slot], bytes);
         bulk_g2s_hint(ring + (size_t)slot * TB, pc.gbase + (size_t)pc.t * TB, bytes, &bars[slot], policy);
         issued++;
@@ -202,10 +202,13 @@ struct GemvWarp {
             for (int t = cc.t; t < cc.t1; t++) {
                 const int slot = consumed % S;
                 if (!mbar_wait_bounded(&bars[slot], (consumed / S) & 1)) { ok = false; break; }
-                const int n = min(kSlotTiles<KB>, sh.nt - t * kSlotTiles<KB>);
-                #pragma unroll 1
-                for (int s = 0; s < n; s++)
-                    acc = tile_dot_row<KB, DUMP>(ring + (size_t)slot * TB + s * tile_bytes(KB), lane, (t * kSlotTiles<KB> + s) * KB, xq_s, xs_s, acc, isum_row);
+                if constexpr (KB == 8) acc = tile_dot_row<KB, DUMP>(ring + (size_t)slot * TB, lane, t * KB, xq_s, xs_s, acc, isum_row);     // (the loop below costs whole tiles 3 %)
+                else {
+                    const int n = min(kSlotTiles<KB>, sh.nt - t * kSlotTiles<KB>);
+                    #pragma unroll 1
+                    for (int s = 0; s < n; s++)
+                        acc = tile_dot_row<KB, DUMP>(ring + (size_t)slot * TB + s * tile_bytes(KB), lane, (t * kSlotTiles<KB> + s) * KB, xq_s, xs_s, acc, isum_row);
+                }
                 consumed++;
                 __syncwarp();                       // every lane is done with the slot before it is refilled
                 if (lane == 0) issue_one(sh);

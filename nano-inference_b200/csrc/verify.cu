@@ -1,17 +1,16 @@
-// The M-token step: M <= 16 tokens at consecutive positions scored in one pass over the
-// weights (speculative verify, chunked prompt processing), and the stand-alone split-KV
-// attention entry point.
+// The M-token step: several tokens in one pass over the weights - up to 16 drafted tokens with logits (mi_verify), up to 512
+// prompt tokens (mi_prefill), up to 64 sequences of their own (mi_batch_step) - and the stand-alone split-KV attention
+// entry point.
 //
 // Replaces forward_batch (reference src/cuda_infer.cu:990-1029: quant_x_q8_batch,
 // gemv_dp4a_batch<T>, rope / kv_store / attention per token) and the M-token path of the
 // persistent kernel (reference src/mega.cu:246-299 gemv_seq, :414-521 attention).
 //
 // One pass is a sequence of launches per layer
-//     norm+q8 (M tokens) -> tcgen05 GEMM QKV -> RoPE + fp16 KV store -> attention (M queries)
-//     -> GEMM O -> residual + norm+q8 -> GEMM gate/up -> SwiGLU+q8 -> GEMM down
-// and finally norm+q8 -> GEMM lm_head -> argmax per token.  Every token goes through the
-// very expressions of the single-token decode kernel (same quantizer, same double-carried
-// sums, the same attention code with the token's own causal range and chunking), so its
+//     norm+q8 (M tokens) -> QKV product + RoPE + fp16 KV store -> attention (M queries)
+//     -> O product -> residual + norm+q8 -> gate/up product + SwiGLU + q8 -> down product
+// and finally norm+q8 -> lm_head product -> greedy pick per token.  Every token goes through the
+// expressions of the single-token decode kernel (same quantizer, same sums carried in double), so its
 // logits do not depend on how many tokens share the pass.
 #include "model.cuh"
 #include "attn_tok.cuh"
@@ -446,7 +445,7 @@ extern "C" int mi_attn_splitkv(mi_ctx* ctx, const float* q_dev, const uint16_t* 
 
 // ---- batched decode of independent sequences -------------------------------------------------------------
 // One step of up to B sequences per call: the current token of each goes through ONE pass over the weights as a column
-// of the M-token step (sixteen columns per pass; larger batches run several passes), with its own position and its
+// of the M-token step (up to 64 columns per pass; larger batches run several passes), with its own position and its
 // own slab of a KV cache that belongs to the batch object.  Every column is processed exactly as if it were alone, so
 // a sequence's ids and logits are the bits of its batch-1 run, whatever else shares the pass.  The reference serves one
 // sequence at a time (README.md:54); the closest code is gemv_dp4a_batch<T> (src/cuda_infer.cu:183-222).
