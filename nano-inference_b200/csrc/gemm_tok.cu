@@ -26,7 +26,10 @@
 // meeting another warp.  Small ones: kw warps of a CTA share the K tiles of a unit and fold their sums through shared memory.
 // Each warp streams its tiles through a ring of bulk copies that starts before the kernel waits for its predecessor (weights
 // depend on nothing); the activations of the CTA's K range and token tile are staged once, or chunk by chunk where they do
-// not fit.  With 32 rows x 32 tokens per warp an A fragment serves four MMAs and a B fragment two.
+// not fit.  With 32 rows x 32 tokens per warp an A fragment serves four MMAs and a B fragment two.  For many tokens a tcgen05 kernel of
+// four roles (unpackers, MMA issuer, activation copies, scaling warps reading tensor memory) was measured as well: 17920 x 1536 with 333
+// tokens 130 us against 123, 2048 x 11008 with 64 tokens 26.6 against 28; one thread issuing an MMA per 32-element block took 150 cycles
+// for each, and the unpackers' issue slots are missing beside the scaling.
 #include "gemm_tok.cuh"
 #include <algorithm>
 #include <atomic>
@@ -37,7 +40,7 @@ namespace mi {
 constexpr int kRing = 2;                                     // ring slots per warp
 constexpr int kStaticSmem = 64;                              // room for static shared memory
 constexpr int kFoldLd = 34;                                  // doubles per token in the fold buffer: conflict-free for the MMA's layout
-__host__ __device__ constexpr int tok_warps(int NT) { return NT <= 2 ? 12 : 8; }
+__host__ __device__ constexpr int tok_warps(int NT) { return NT <= 3 ? 12 : 8; }
 
 constexpr int kStepBlk = 8;                                  // blocks per ring slot: one tile of eight blocks, or as many smaller ones (they are contiguous)
 constexpr int kStepBytes = kStepBlk * kTileRowBytes;
@@ -352,12 +355,12 @@ SmemNeed smem_need(int NT) {
 // the consumer adds them, GEMM_PART).  Small matrices want every sub-partition of every SM to have a tile, large ones want
 // warps that never meet.  The choice is the minimum of a rough model in clocks, from the measured costs: a tile costs its blocks'
 // issue slots, which the warps of a sub-partition share, the end of a unit its stores or a pass through shared memory.
-int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* out) {
-    const TokTiling tl = tok_tiling(M);
+int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, const TokTiling& tl, GemmPlan* out) {
     const int NT = tl.NT, TT = tl.TT, W = tok_warps(NT), N = NT * 8, U = mode == GEMM_GU ? 2 : 1, ntok = std::min(M, N);
     const SmemNeed need = smem_need(NT);
     const int nt = (w->nb + kStepBlk - 1) / kStepBlk;                                     // steps of eight blocks
-    const double c_tile = kStepBlk * (45.0 + 76.0 * NT + (w->kb < 8 ? 30 : 0)) + 100;
+    const double c_blk[kMaxTokNT + 1] = {0, 121, 200, 290, 400};                          // clocks per block, two or three warps per sub-partition
+    const double c_tile = kStepBlk * (c_blk[NT] + (w->kb < 8 ? 30 : 0)) + 100;
     const double c_tok = mode == GEMM_GU ? 640 : mode == GEMM_QKV ? 300 : 60;             // end of a round, per token and warp
     double best = 1e300;
     const int max_ksg = mode == GEMM_PART ? std::min(nt, 8) : 1;
@@ -385,10 +388,11 @@ int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* ou
             cost = waves * (cost + 600 + (nchunk > 1 ? rounds * nchunk * 1500.0 : 0.0)) + (mode == GEMM_PART ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
             if (cost < best) {
                 best = cost;
-                *out = GemmPlan{NT, TT, ksg, kct, C, kw, fold, (size_t)fixed + (size_t)kct * need.x_step};
+                *out = GemmPlan{NT, TT, ksg, kct, C, kw, fold, (size_t)fixed + (size_t)kct * need.x_step, cost};
             }
         }
     }
+    out->cost += 0.4 * TT * (double)w->groups * w->nb * kTileRowBytes / 3400.0;     // every token tile reads the weights again (3400 bytes per clock of HBM)
     if (best == 1e300) return set_error(ctx, MI_ERR_UNSUPPORTED, "gemm: tile depth %d does not fit the shared memory", w->kb);
     return MI_OK;
 }
@@ -462,7 +466,7 @@ extern "C" int mi_gemm_q4_q8(mi_ctx* ctx, const mi_weight* w, const int8_t* xq_d
     if (w->count != 1) return set_error(ctx, MI_ERR_UNSUPPORTED, "gemm: matrix stacks are not supported");
     if (w->rows == 0) return MI_OK;
     GemmPlan pl;
-    int st = plan_gemm_tok(ctx, w, GEMM_PLAIN, M, &pl);
+    int st = plan_gemm_tok(ctx, w, GEMM_PLAIN, M, tok_tiling(M), &pl);
     if (st != MI_OK) return st;
     GemmParams p{};
     p.M = M; p.xq = xq_dev; p.xd = reinterpret_cast<const __half*>(xd_dev); p.bias = bias_dev; p.y = y_dev;
@@ -470,7 +474,7 @@ extern "C" int mi_gemm_q4_q8(mi_ctx* ctx, const mi_weight* w, const int8_t* xq_d
     if (pl.kct >= steps) return launch_gemm_tok(ctx, w, pl, GEMM_PLAIN, true, p, true);
     // The activations of all of K do not fit a CTA's staging: K ranges over the grid and a small kernel that adds them, instead of
     // staging chunk after chunk in every CTA (1536 x 8960, 16 tokens: 27.7 us that way).
-    if ((st = plan_gemm_tok(ctx, w, GEMM_PART, M, &pl)) != MI_OK) return st;
+    if ((st = plan_gemm_tok(ctx, w, GEMM_PART, M, tok_tiling(M), &pl)) != MI_OK) return st;
     if ((st = ensure_scratch(ctx, (size_t)pl.ksg * M * w->rows, 0)) != MI_OK) return st;
     p.part = ctx->part; p.ldp = (int)w->rows;
     if ((st = launch_gemm_tok(ctx, w, pl, GEMM_PART, true, p, true)) != MI_OK) return st;

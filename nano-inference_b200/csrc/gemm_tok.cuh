@@ -104,13 +104,13 @@ struct GemmParams {
 
 // Token tiles of a pass over M tokens: TT tiles of NT groups of eight; operand buffers hold J = NT * TT groups per block.
 struct TokTiling { int NT, TT; int J() const { return NT * TT; } };
-inline TokTiling tok_tiling(int M) {
-    const int J = (M + 7) / 8, TT = (J + kMaxTokNT - 1) / kMaxTokNT;
+inline TokTiling tok_tiling(int M, int max_nt = kMaxTokNT) {
+    const int J = (M + 7) / 8, TT = (J + max_nt - 1) / max_nt;
     return TokTiling{(J + TT - 1) / TT, TT};
 }
 // How a launch over one matrix and M tokens is cut (see plan_gemm_tok).
-struct GemmPlan { int NT, TT, ksg, kct, C, kw; bool fold; size_t smem; };
-int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, GemmPlan* out);
+struct GemmPlan { int NT, TT, ksg, kct, C, kw; bool fold; size_t smem; double cost; };
+int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, const TokTiling& tiles, GemmPlan* out);
 int launch_gemm_tok(mi_ctx* ctx, const mi_weight* w, const GemmPlan& plan, int mode, bool rowmajor, GemmParams p, bool pdl);
 
 }  // namespace mi
