@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 using namespace mi;
 
@@ -33,11 +34,11 @@ constexpr size_t kMaxPassGraphs = 64;
 // q8_0(rmsnorm(x) * w) (src/cpu_infer.cpp:40-46) in operand order.  One CTA per token, four consecutive elements per
 // thread: every load of a thread is requested before the first is used, a block of 32 is eight threads.  Token m0 + blockIdx.x
 // of X is token blockIdx.x of the output.
-__global__ void __launch_bounds__(1024) vf_norm_quant(const DecodeParams P, const int* __restrict__ tokens, bool embed, int m0, float* X, const double* part,
+template <int R>
+__global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const DecodeParams P, const int* __restrict__ tokens, bool embed, int m0, float* X, const double* part,
                                                        int ranges, long long range_stride, int ldp, const float* __restrict__ w, TokX out) {
     __shared__ double red[32];
     const int E = P.E, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5, mo = blockIdx.x, m = m0 + mo;
-    constexpr int R = 2;                                             // rounds of blockDim.x * 4 elements: E <= 8192
     float4 wv[R];
     #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -75,10 +76,24 @@ __global__ void __launch_bounds__(1024) vf_norm_quant(const DecodeParams P, cons
         if (part) {
             const double* pp = part + (size_t)m * ldp + e;
             double s[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int q = 0; q < ranges; q++) {
-                const double2 a = __ldcg(reinterpret_cast<const double2*>(pp + q * range_stride)), b = __ldcg(reinterpret_cast<const double2*>(pp + q * range_stride + 2));
-                s[0] = __dadd_rn(s[0], a.x); s[1] = __dadd_rn(s[1], a.y); s[2] = __dadd_rn(s[2], b.x); s[3] = __dadd_rn(s[3], b.y);
-            }
+            // (a row of ranges is requested four at a time, and what remains together: a loop over single ones waits for each)
+            auto add = [&](auto count, int q0) {
+                constexpr int U = decltype(count)::value;
+                double2 a[U], b[U];
+                #pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const double2* p2 = reinterpret_cast<const double2*>(pp + (q0 + u) * range_stride);
+                    a[u] = __ldcg(p2); b[u] = __ldcg(p2 + 1);
+                }
+                #pragma unroll
+                for (int u = 0; u < U; u++) { s[0] = __dadd_rn(s[0], a[u].x); s[1] = __dadd_rn(s[1], a[u].y); s[2] = __dadd_rn(s[2], b[u].x); s[3] = __dadd_rn(s[3], b[u].y); }
+            };
+            int q0 = 0;
+            #pragma unroll 1
+            for (; q0 + 4 <= ranges; q0 += 4) add(std::integral_constant<int, 4>{}, q0);
+            if (ranges - q0 == 3) add(std::integral_constant<int, 3>{}, q0);
+            else if (ranges - q0 == 2) add(std::integral_constant<int, 2>{}, q0);
+            else if (ranges - q0 == 1) add(std::integral_constant<int, 1>{}, q0);
             #pragma unroll
             for (int i = 0; i < 4; i++) v[r][i] = __fadd_rn(v[r][i], __double2float_rn(s[i]));
         }
@@ -293,7 +308,7 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     GemmParams g{};
     g.M = M;
     auto norm = [&](bool embed, int m0, int count, int ranges, const float* w, const TokX& out) -> int {
-        MI_CUDA(ctx, launch_k(pdl, vf_norm_quant, dim3(count), dim3(nt_norm), 0, ctx->stream, P, tokens, embed, m0, b.X, (const double*)(ranges ? b.part : nullptr), ranges,
+        MI_CUDA(ctx, launch_k(pdl, E <= 2048 ? vf_norm_quant<1> : vf_norm_quant<2>, dim3(count), dim3(nt_norm), 0, ctx->stream, P, tokens, embed, m0, b.X, (const double*)(ranges ? b.part : nullptr), ranges,
                               (long long)M * b.ldp, b.ldp, w, out));
         return MI_OK;
     };
