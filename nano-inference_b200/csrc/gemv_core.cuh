@@ -19,6 +19,7 @@
 // traffic that scales with the matrix.
 #pragma once
 #include "mi_internal.cuh"
+#include "div_known.cuh"
 
 namespace mi {
 
@@ -117,17 +118,6 @@ __device__ __forceinline__ double tile_dot_row(const uint8_t* tile, int lane, in
         acc = blk_acc(acc, dw[k], s.x, isum, s.y);
     }
     return acc;
-}
-
-// a / b with y = 1 / b rounded to double, both computed once: the correctly rounded quotient by P. Markstein's theorem ("Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990): a quotient within one ulp, corrected with its exact remainder
-// times y, rounds correctly.  a * y may be a little further off than that, hence two corrections.  Five multiply-adds in a row
-// where the general division takes some 360 cycles in the middle of every norm.  a finite and far from the ends of the
-// exponent range (a NaN stays one).
-__device__ __forceinline__ double div_known(double a, double b, double y) {
-    double q = __dmul_rn(a, y);
-    q = __fma_rn(__fma_rn(-q, b, a), y, q);
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
 }
 
 // Stage a q8_0 activation vector already in global memory: int8 values, and per
