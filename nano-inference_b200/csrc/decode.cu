@@ -462,6 +462,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         x.cand = take(kMaxWorldTP * m->grid * 4);
         x.attm = take(m->NH * m->max_chunks);
         x.tokw = take(2);
+        x.attdone = take(2 * m->attn_ctas);
         x.total = off;
     }
     if ((st = dev_alloc(ctx, m, &P.h_in, E)) || (st = dev_alloc(ctx, m, &P.h_mid, E)) || (st = dev_alloc(ctx, m, &P.att, NQ)) ||

@@ -17,7 +17,8 @@
 // atomic).  The tag numbers the (step, phase) that produced the value.  A consumer
 // simply loads the words it needs and looks at their tags; words that are not there
 // yet are polled (bounded by a time budget).  There is no separate flag, hence no
-// release fence before it and no second round trip after it: a phase boundary costs
+// release fence before it and no second round trip after it (what travels beside the words, rows of the KV cache and partial sums of
+// the long-range attention, has fences of its own): a phase boundary costs
 // one store-to-load hop through the L2 instead of arrive + poll + reload, and a CTA
 // waits only for the values it actually consumes.  Buffers are reused every layer;
 // a word can only be overwritten after every reader has passed on, because the
@@ -171,6 +172,7 @@ struct XwLayout {
     int cand;       // [kMaxWorldTP][grid][4]: argmax candidates {best value}, {its row}, {second-best value}, -   (pushed)
     int attm;       // [NH][max_chunks] fp32 bits: maximum of every chunk of the long-range attention
     int tokw;       // [2]: the token picked by the step that just ended, for the attention CTAs (written only under a stop rule)
+    int attdone;    // [2][attn_ctas]: by step parity, "this attention CTA has left the step" (see rows_ordered)
     int total;
 };
 
@@ -889,9 +891,8 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
             }
             cp_async_commit();
         };
-        // (A model of one layer waits for q first: between two steps nothing else orders the last position's rows before this read.)
-        const bool early = P.L > 1;
-        if (early) { copy_rows(ks, KLD, P.kc, 0); copy_rows(vs, VLD, P.vc, 0); }
+        // rows of earlier positions: written before this launch, or by steps that the greedy pick orders before this one (rows_ordered)
+        copy_rows(ks, KLD, P.kc, 0); copy_rows(vs, VLD, P.vc, 0);
         // q of the group, and k / v of the new position (packed order: dim d of a head sits at 2d (d < HD/2) or 2(d-HD/2)+1)
         constexpr int QN = (G * HD + DNT - 1) / DNT;
         unsigned qw[QN + 2], valid = 0;
@@ -907,7 +908,6 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
             }
             return k == QN ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
         }, qw);
-        if (!early) { copy_rows(ks, KLD, P.kc, 0); copy_rows(vs, VLD, P.vc, 0); }
         // the order the MMA reads q in: lane (row, t) takes the 16-byte pieces t, t + 4, .. of a row
         auto qslot = [](int row, int d) { return ((d >> 5) * 8 + (d & 7)) * 32 + row * 4 + ((d >> 3) & 3); };
         #pragma unroll
@@ -1025,9 +1025,11 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                     for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + i, __dadd_rn(o[0][i][e], o[1][i][e]));
             }
             if (tid < G) __stcg(P.attn_part + ((size_t)(h0 + tid) * P.max_chunks + ch) * SW + HD, rl[tid]);
-            fence_acq_rel_gpu();                    // the partial, and the new position's rows, before the word that announces them
             __syncthreads();
-            if (tid < G) pub.local(P.xo.attm + (h0 + tid) * P.max_chunks + ch, __float_as_uint((float)rm[tid]));
+            if (tid < G) {
+                fence_acq_rel_gpu();                // the partial, and the new position's rows, before the word that announces them
+                pub.local(P.xo.attm + (h0 + tid) * P.max_chunks + ch, __float_as_uint((float)rm[tid]));
+            }
         }
         prof_mark(P, 16);
     }
@@ -1041,6 +1043,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
         const unsigned long long* mv = P.xw + P.xo.attm + (size_t)head * P.max_chunks;
         const bool okm = tw_poll(P, pub.tag, valid, [&](int k) { return mv + lane + 32 * k; }, mw);
         fence_acq_rel_gpu();
+        __syncwarp();                               // a lane reads sums whose words other lanes polled
         float m = -INFINITY;
         #pragma unroll
         for (int k = 0; k < kMaxChunkWords; k++) if (valid >> k & 1u) m = fmaxf(m, __uint_as_float(mw[k]));
@@ -1509,6 +1512,32 @@ __device__ __forceinline__ bool lean_regime_ok(int pos, int attn_ctas) {
 #endif
 }
 
+// Where rows of the cache that one CTA writes in a step become readable by every CTA in the next one.  attention_split requests the rows
+// of earlier positions before it has polled anything of its layer, and the tagged words that its CTA has polled since the last
+// step carry no order for them: they came from CTAs that had passed on other words without a fence.  So the greedy pick, which every GEMV CTA
+// publishes to and polls once per step, is an ordering point in the builds that have attention_split: a CTA's candidate is
+// stored behind a fence (and behind a barrier, so the fence speaks for all its threads), and a CTA's threads fence once they
+// have polled all candidates.  The attention CTAs, which take chunks as well but have no part in the pick, say behind a fence that they have left the step
+// (attdone; two sets by step parity, because an attention CTA may leave the next step before a GEMV CTA has looked), and poll the
+// candidates before their next step.  No candidate is overwritten before they have: every CTA below attn_ctas has a chunk in every layer
+// (attn_ctas <= 7 NKV, and there are at least 9 NKV chunks or as many as the grid holds), so the next pick descends from it.
+// Two fences per step where the chain of a step is a hundred and forty hops.
+constexpr bool kRowsCross = MI_LEAN != 1;
+__device__ __forceinline__ int attdone_off(const DecodeParams& P, int step) { return P.xo.attdone + (step & 1) * P.attn_ctas; }
+
+// attention CTAs, before a step that reads rows of the step before it; tag: that step's pick.  Whole CTA, returns a CTA-uniform ok.
+static __device__ __noinline__ bool rows_ordered(const DecodeParams& P, unsigned tag, int step) {
+    const int n_cand = (P.tp.on ? P.tp.world : 1) * ((int)gridDim.x - P.attn_ctas), n = n_cand + P.attn_ctas, done = attdone_off(P, step);
+    bool ok = true;
+    for (int i0 = 0; i0 < n && ok; i0 += DNT) {
+        const int i = i0 + (int)threadIdx.x;
+        unsigned w[1];
+        ok = tw_poll(P, tag, i < n ? 1u : 0u, [&](int) { return P.xw + (i < n_cand ? P.xo.cand + i * 4 : done + i - n_cand); }, w);
+    }
+    fence_acq_rel_gpu();
+    return __syncthreads_and(ok ? 1 : 0) != 0;
+}
+
 template <int HD, int G>
 static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int step0, int step1, int ph0, int ph1, uint8_t* smem, uint8_t* stage, uint64_t* bar) {
     const int nph = 5 * P.L + 1;
@@ -1534,6 +1563,8 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
             ok = __syncthreads_and(got ? 1 : 0) != 0;
             if (!ok || (int)tw[0] == P.stop_token) break;
         }
+        // (only a launch over whole steps has more than one)
+        if (kRowsCross && step > step0 && ph0 == 0 && ph1 == nph && pos + 1 > kShortAttnMax && !(ok = rows_ordered(P, tag0 - 1u, step - 1))) break;
         for (int l = max(0, (ph0 + 3) / 5); 5 * l + 1 < ph1 && l < P.L && ok; l++) {
             const int ph = 5 * l + 1;
             Pub pub;
@@ -1561,6 +1592,10 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
 #endif
             ok = __syncthreads_and(ok ? 1 : 0) != 0;
             prof_mark(P, 3);
+        }
+        if (kRowsCross && ok && ph1 == nph && threadIdx.x == 0) {
+            fence_acq_rel_gpu();
+            tw_st(P.xw + attdone_off(P, step) + blockIdx.x, tag0 + (unsigned)nph - 1u, 1u);
         }
     }
 #if MI_PROF
@@ -1770,6 +1805,7 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                 if (tid == 0) {
                     Cand t; t.best = cv[0]; t.idx = ci[0]; t.second = c2[0];
                     for (int w = 1; w < DNW; w++) { Cand o; o.best = cv[w]; o.idx = ci[w]; o.second = c2[w]; t.merge(o); }
+                    if (kRowsCross) fence_acq_rel_gpu();                // rows of the cache written in this step (rows_ordered)
                     pub.shared(my_cand, __float_as_uint(t.best));
                     pub.shared(my_cand + 1, (unsigned)t.idx);
                     pub.shared(my_cand + 2, __float_as_uint(t.second));
@@ -1780,12 +1816,14 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                 prof_mark(P, 2 * k + 1);
                 cd.best = -INFINITY; cd.idx = 0x7fffffff; cd.second = -INFINITY;
                 bool okc = ok;
+                constexpr int CW = kRowsCross ? 7 : 6;
                 for (int c0 = 0; c0 < n_cand && okc; c0 += 2 * DNT) {
-                    unsigned cw[6], valid = 0;
+                    unsigned cw[CW], valid = 0;
                     if (c0 + tid < n_cand) valid |= 7u;
                     if (c0 + DNT + tid < n_cand) valid |= 56u;
+                    if (kRowsCross && c0 == 0 && tid < P.attn_ctas) valid |= 64u;
                     const unsigned long long* cb = P.xw + P.xo.cand + (size_t)(c0 + tid) * 4;
-                    okc = tw_poll(P, pub.tag, valid, [&](int q) { return cb + (q / 3) * (4 * DNT) + (q % 3); }, cw);
+                    okc = tw_poll(P, pub.tag, valid, [&](int q) { return q == 6 ? P.xw + attdone_off(P, step) + tid : cb + (q / 3) * (4 * DNT) + (q % 3); }, cw);
                     #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         if (okc && (valid >> (3 * h) & 1u)) {
@@ -1794,6 +1832,7 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                         }
                     }
                 }
+                if (kRowsCross) fence_acq_rel_gpu();
                 prof_mark(P, kProfWait);
                 cd.warp_reduce();
                 ok = __syncthreads_and(okc ? 1 : 0) != 0;       // also: cv / ci / c2 are free again
