@@ -663,11 +663,14 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
         if (in_tokens_host[i] < 0 || in_tokens_host[i] >= m->V) return set_error(ctx, MI_ERR_INVALID, "decode: token id %d out of range", in_tokens_host[i]);
     MI_CUDA(ctx, cudaSetDevice(ctx->device));
     int st;
+    // (a capacity counts only while its buffer exists: an allocation that fails leaves the pointer null)
     if (n_forced > m->in_capacity) {
+        m->in_capacity = 0;
         if ((st = dev_alloc(ctx, m, &m->d_in_tokens, (size_t)n_forced * 2))) return st;
         m->in_capacity = n_forced * 2;
     }
     if (n_steps > m->out_capacity) {
+        m->out_capacity = 0; m->last_steps = 0;
         if ((st = dev_alloc(ctx, m, &m->d_out_tokens, (size_t)n_steps * 2)) || (st = dev_alloc(ctx, m, &m->d_margins, (size_t)n_steps * 2))) return st;
         m->out_capacity = n_steps * 2;
     }

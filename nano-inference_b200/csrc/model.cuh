@@ -2,6 +2,7 @@
 #pragma once
 #include "decode_kernel.cuh"
 #include "gemm_tok.cuh"
+#include "buffer_set.cuh"
 
 #include <map>
 #include <set>
@@ -17,7 +18,7 @@ struct PassKey {
 // device buffers of the M-token step (all [tokens][...], token-major)
 struct VerifyBufs {
     int cap = 0, cap_logits = 0;       // tokens the buffers hold
-    std::vector<void*> mem;            // the allocations behind the pointers below
+    BufferSet mem;                     // the allocations behind the pointers below; clears them when it frees
     float* X = nullptr;                // residual stream [M][E]
     double* part = nullptr; int ldp = 0;    // sums of a projection per K range [range][M][ldp]
     float* Y = nullptr;                // fp32 rows of the QKV and gate/up products (more than kMaxFusedTok tokens)

@@ -203,21 +203,29 @@ void drop_graphs(VerifyBufs& b) {
     b.graphs.clear();
 }
 
+void release_bufs(VerifyBufs& b) {
+    b.mem.release([](void* p) { cudaFree(p); });
+    b.cap = b.cap_logits = 0;
+}
+
 // Buffers of a pass over up to M tokens (logits for up to ML of them).  They grow in steps and are kept; graphs that point into
-// replaced ones go with them.
+// replaced ones go with them.  After an allocation that failed there are none, and the next call starts over.
 int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
     VerifyBufs& b = m->vb;
     if (b.cap >= M && b.cap_logits >= ML) return MI_OK;
     MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (!b.h_meta && cudaMallocHost((void**)&b.h_meta, (3 * PMAX + 4) * sizeof(int)) != cudaSuccess) {
+        b.h_meta = nullptr;
+        return set_error(ctx, MI_ERR_NOMEM, "M-token step: pinned allocation failed");
+    }
     drop_graphs(b);
     const int cap = std::max(b.cap, M <= VMAX ? VMAX : M <= BMAX ? BMAX : PMAX), capl = std::max(b.cap_logits, ML <= VMAX ? VMAX : BMAX);
-    for (void* p : b.mem) cudaFree(p);
-    b.mem.clear(); b.cap = b.cap_logits = 0;
+    release_bufs(b);
     auto take = [&](auto** p, size_t n) -> int {
-        cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n, 4) * sizeof(**p));
-        if (e != cudaSuccess) return set_error(ctx, MI_ERR_NOMEM, "M-token step: cudaMalloc(%zu) failed: %s", n * sizeof(**p), cudaGetErrorString(e));
-        b.mem.push_back(*p);
-        MI_CUDA(ctx, cudaMemsetAsync(*p, 0, std::max<size_t>(n, 4) * sizeof(**p), ctx->stream));
+        const size_t bytes = std::max<size_t>(n, 4) * sizeof(**p);
+        if (!b.mem.take(p, bytes, [](void** q, size_t k) { return cudaMalloc(q, k) == cudaSuccess; }))
+            return set_error(ctx, MI_ERR_NOMEM, "M-token step: cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(cudaGetLastError()));
+        MI_CUDA(ctx, cudaMemsetAsync(*p, 0, bytes, ctx->stream));
         return MI_OK;
     };
     auto take_tok = [&](TokX* x, int n, int tokens) -> int {
@@ -233,10 +241,10 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
         (st = take(&b.att, (size_t)cap * NQ)) || (st = take(&b.Y, cap > kMaxFusedTok ? (size_t)cap * std::max(2 * FF, m->qkv_rows) : 0)) || (st = take(&b.logits, (size_t)capl * m->V)) ||
         (st = take(&b.meta, (size_t)3 * cap + 4)) || (st = take(&b.out, (size_t)cap)) || (st = take(&b.margins, (size_t)cap)) ||
         (st = take(&b.attn_part, attn_part_max(ctx, m->NH, m->NKV, m->HD))) ||
-        (st = take(&b.pick, (size_t)capl * kPickSlices * 3)) || (st = take(&b.pick_cnt, (size_t)capl)))
+        (st = take(&b.pick, (size_t)capl * kPickSlices * 3)) || (st = take(&b.pick_cnt, (size_t)capl))) {
+        cudaStreamSynchronize(ctx->stream);                            // (the fills of those that were made)
+        release_bufs(b);
         return st;
-    if (!b.h_meta) {
-        if (cudaMallocHost((void**)&b.h_meta, (3 * PMAX + 4) * sizeof(int)) != cudaSuccess) return set_error(ctx, MI_ERR_NOMEM, "M-token step: pinned allocation failed");
     }
     b.cap = cap; b.cap_logits = capl;
     return MI_OK;
@@ -246,8 +254,7 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
 
 void mi::free_verify_bufs(mi_model* m) {
     drop_graphs(m->vb);
-    for (void* p : m->vb.mem) cudaFree(p);
-    m->vb.mem.clear();
+    release_bufs(m->vb);
     if (m->vb.h_meta) cudaFreeHost(m->vb.h_meta);
 }
 
