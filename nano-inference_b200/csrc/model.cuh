@@ -3,9 +3,8 @@
 #include "decode_kernel.cuh"
 #include "gemm_tok.cuh"
 #include "buffer_set.cuh"
+#include "pass_graphs.cuh"
 
-#include <map>
-#include <set>
 #include <tuple>
 #include <vector>
 
@@ -28,8 +27,7 @@ struct VerifyBufs {
     float* logits = nullptr;           // [M][V]
     int* meta = nullptr; int* h_meta = nullptr;         // tokens | positions | slots, or tokens | first position; its pinned image
     int* out = nullptr;                // [M]
-    std::map<PassKey, void*> graphs;   // cudaGraphExec_t
-    std::set<PassKey> warm;            // kinds of pass that have run plainly once
+    PassGraphs<PassKey> graphs;        // cudaGraphExec_t
     double* attn_part = nullptr;       // chunk sums of the attention (attn_tok.cu)
     float* pick = nullptr; unsigned* pick_cnt = nullptr;         // greedy pick: candidates per slice, arrival counters (self-clearing)
     float* margins = nullptr;          // [M] greedy logit minus the runner-up

@@ -28,7 +28,6 @@ constexpr int VMAX = 16;                    // tokens of one mi_verify call
 constexpr int BMAX = 64;                    // sequences of one batched pass
 constexpr int PMAX = 512;                   // prompt tokens of one pass
 constexpr int kMaxRanges = 8;               // K ranges of a split product (plan_gemm_tok)
-constexpr size_t kMaxPassGraphs = 64;
 
 // x = (embedding row | X) (+ the projection's sum over its K ranges, rounded to fp32 once), committed to X;
 // q8_0(rmsnorm(x) * w) (src/cpu_infer.cpp:40-46) in operand order.  One CTA per token, four consecutive elements per
@@ -198,10 +197,7 @@ __global__ void __launch_bounds__(512) vf_pick(const float* logits, long long st
     }
 }
 
-void drop_graphs(VerifyBufs& b) {
-    for (auto& g : b.graphs) cudaGraphExecDestroy((cudaGraphExec_t)g.second);
-    b.graphs.clear();
-}
+void destroy_graph(void* g) { cudaGraphExecDestroy((cudaGraphExec_t)g); }
 
 void release_bufs(VerifyBufs& b) {
     b.mem.release([](void* p) { cudaFree(p); });
@@ -218,7 +214,7 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
         b.h_meta = nullptr;
         return set_error(ctx, MI_ERR_NOMEM, "M-token step: pinned allocation failed");
     }
-    drop_graphs(b);
+    b.graphs.drop_graphs(destroy_graph);
     const int cap = std::max(b.cap, M <= VMAX ? VMAX : M <= BMAX ? BMAX : PMAX), capl = std::max(b.cap_logits, ML <= VMAX ? VMAX : BMAX);
     release_bufs(b);
     auto take = [&](auto** p, size_t n) -> int {
@@ -253,7 +249,7 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
 }  // namespace
 
 void mi::free_verify_bufs(mi_model* m) {
-    drop_graphs(m->vb);
+    m->vb.graphs.drop_graphs(destroy_graph);
     release_bufs(m->vb);
     if (m->vb.h_meta) cudaFreeHost(m->vb.h_meta);
 }
@@ -359,10 +355,10 @@ int run_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (!use_graph || a.head != HEAD_ALL || cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return enqueue_pass(ctx, m, a);
     const PassKey key{a.M, regime, a.ragged ? 1 : 0, (const void*)a.kc, (const void*)a.vc, a.max_seq};
-    auto it = b.graphs.find(key);
-    if (it == b.graphs.end()) {
-        if (b.warm.insert(key).second) return enqueue_pass(ctx, m, a);
-        if (b.graphs.size() >= kMaxPassGraphs) drop_graphs(b);
+    bool again;
+    void* graph = b.graphs.use(key, &again, destroy_graph);
+    if (!graph) {
+        if (!again) return enqueue_pass(ctx, m, a);
         cudaStream_t cs = nullptr, user = ctx->stream;
         MI_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
@@ -381,9 +377,10 @@ int run_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         e = cudaGraphInstantiate(&ge, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return set_error(ctx, MI_ERR_CUDA, "verify: graph instantiation failed: %s", cudaGetErrorString(e));
-        it = b.graphs.emplace(key, (void*)ge).first;
+        graph = ge;
+        b.graphs.put(key, graph, destroy_graph);                       // (no pass is in flight here: every call ends with a wait)
     }
-    MI_CUDA(ctx, cudaGraphLaunch((cudaGraphExec_t)it->second, ctx->stream));
+    MI_CUDA(ctx, cudaGraphLaunch((cudaGraphExec_t)graph, ctx->stream));
     return MI_OK;
 }
 
