@@ -352,23 +352,41 @@ __global__ void __launch_bounds__(kAT) attn_tok_merge(const __grid_constant__ At
 
 // ---- host side -----------------------------------------------------------------------------------------------------
 
-// Queries per CTA: four where the ranges are long (their work is FP64 time, and an MMA's rows should be full: 4 x 6 heads are three
-// whole row tiles, one query's 6 heads fill three quarters of one), one where they are short or belong to different sequences
-// (the work is latency, and more CTAs share it).  Chunks: one up to 320 positions where CTAs have one query (a CTA walks them in the
-// time a second launch takes), up to 128 where they have four; beyond, enough that two CTAs per SM have work, and none
-// shorter than 64 positions.
+// Queries per CTA and chunks per range: the cheapest by a rough model in microseconds, from times of whole passes (three head shapes,
+// 1 .. 16 queries behind 0 .. 32700 positions, prompts of 17 .. 512 tokens behind 0 .. 16000, batches of 2 .. 64; attention's share of a layer).
+// A CTA costs its start and end and a time per position, which grows with the row tiles of its MMAs and with the CTAs that share its SM:
+//     one row tile (one query), alone / two on an SM / each of more: 0.032 / 0.052 / 0.026 us per position at head_dim 128
+//     (HD = 64, where three fit an SM: 0.022 / 0.045 / 0.016); three or four row tiles (four queries): 0.051 each (0.032), 0.59 of that alone.
+// (Up to half as many CTAs as SMs are alone; more meet on the SMs that the projection before them leaves first.)  The merge is a launch of about 5.
+// So four queries share a CTA where one per CTA would begin another wave, or where the FP64 pipe is what counts and the row tiles are fuller that way (6 heads:
+// 24 of 24 rows instead of 6 of 8), and a range is cut from about 200 positions on.  Passes of the 1.5B shape, ms: 16 tokens at 8100 2.35 with four queries
+// per CTA, 2.66 with one; 8 at 2000 1.39 and 1.15; prompt of 96 at 4000 6.1 and 9.0, of 333 10.3 and 9.9 at 500; one token at 300 1.02 cut in five,
+// 1.12 in one chunk, at 60 1.00 and 0.90.  The rule finds the best of the four choices to 0.2 % on average and 5 % at most over
+// those measurements; the thresholds before it (four queries from M x range = 16384 on, one chunk up to 320) lost 3.6 % on average and up to 54 %.
+static double attn_cost_us(int sms, int HD, int G, int qb, int ctas, int nch, int range, int shorter) {
+    const int rt = attn_row_tiles(G, qb), k = ctas <= sms / 2 ? 1 : std::max(2, (ctas + sms - 1) / sms);
+    const double two = rt == 1 ? 0.038 + 0.00011 * HD : rt * (0.012 + 0.000305 * HD), alone = rt == 1 ? 0.012 + 0.000156 * HD : 0.59 * two,
+                 many = rt == 1 ? 0.005 + 0.000164 * HD : 0.5 * two, start = qb == 1 ? 2.0 : 5.5;
+    const double positions = (range - 0.5 * shorter * (1.0 - 1.0 / k)) / nch;             // earlier queries of a prompt see fewer, by up to `shorter`
+    return start * std::max(1.0, 0.5 * k) + positions * (k == 1 ? alone : k == 2 ? two : k * many) + (nch > 1 ? 4.5 + 0.02 * nch : 0.0);
+}
+// No chunk is shorter than 64 positions, and no more than two CTAs per SM are made by cutting.
 AttnPlan plan_attn_tok(const mi_ctx* ctx, int NH, int NKV, int HD, int M, int lp_max, bool ragged) {
-    AttnPlan a;
-    a.qb = !ragged && M > 1 && (long long)M * lp_max >= 16384 ? kMaxQB : 1;
-    const int units = NKV * ((M + a.qb - 1) / a.qb);
-    const int share = a.qb > 1 ? (2 * ctx->sm_count + units - 1) / units : 2 * ctx->sm_count / units;
-    a.nch = lp_max <= (a.qb > 1 ? 128 : 320) ? 1 : std::max(1, std::min((lp_max + 63) / 64, share));
+    AttnPlan a{1, 1, 0};
+    double best = 1e300;
+    for (int qb = 1; qb <= (ragged || M == 1 ? 1 : kMaxQB); qb += kMaxQB - 1) {
+        const int units = NKV * ((M + qb - 1) / qb), most = std::max(1, std::min((lp_max + 63) / 64, 2 * ctx->sm_count / units));
+        for (int nch = 1; nch <= most; nch += std::max(1, most - 1)) {                    // one, and as many as may be
+            const double us = attn_cost_us(ctx->sm_count, HD, NH / NKV, qb, units * nch, nch, lp_max, ragged ? 0 : M);
+            if (us < best) { best = us; a.qb = qb; a.nch = nch; }
+        }
+    }
     a.part_doubles = a.nch > 1 ? (size_t)M * NH * a.nch * (HD + 2) : 0;
     return a;
 }
 
-// with more than one chunk, units x chunks is below two CTAs per SM and another unit each; a unit is at most kMaxQB queries of one group
-size_t attn_part_max(const mi_ctx* ctx, int NH, int NKV, int HD) { return (size_t)kMaxQB * (NH / NKV) * 4 * ctx->sm_count * (HD + 2); }
+// with more than one chunk there are at most two CTAs per SM, of at most kMaxQB queries of one group each
+size_t attn_part_max(const mi_ctx* ctx, int NH, int NKV, int HD) { return (size_t)kMaxQB * (NH / NKV) * 2 * ctx->sm_count * (HD + 2); }
 
 namespace {
 template <int HD, int G, int QB>

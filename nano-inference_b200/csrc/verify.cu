@@ -267,12 +267,13 @@ struct Pass {
 };
 enum { HEAD_ALL, HEAD_LAST, HEAD_NONE };
 
-// Positions that a launch sequence is planned for: captured passes of up to 320 cached positions share one plan, beyond that those
-// of a power of two (the plan only cuts the ranges, it is right for any position).
+// Positions that a launch sequence is planned for: captured passes of up to 160 cached positions (one chunk: see plan_attn_tok) share one
+// plan, beyond that those up to 512, 768, 1024, 1536, .. (the plan only cuts the ranges, it is right for any position).
 int attn_bucket(int lp_max) {
-    int b = 320;
-    if (lp_max > b) for (b = 512; b < lp_max;) b *= 2;
-    return b;
+    if (lp_max <= 160) return 160;
+    int b = 512;
+    while (b < lp_max) b *= 2;
+    return b > 512 && lp_max <= b / 4 * 3 ? b / 4 * 3 : b;
 }
 
 // Every launch may overlap its predecessor's tail (each kernel waits before it touches what the predecessor wrote);
@@ -286,7 +287,7 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     P.prof = nullptr;
     TokX xf = b.xf, attf = b.attf, actf = b.actf;
     const std::vector<LayerPtrs>& lp = m->layer_ptrs;
-    const AttnPlan pa = plan_attn_tok(ctx, m->NH, m->NKV, m->HD, M, attn_bucket(a.lp_max), a.ragged);
+    const AttnPlan pa = plan_attn_tok(ctx, m->NH, m->NKV, m->HD, M, a.head == HEAD_ALL ? attn_bucket(a.lp_max) : a.lp_max, a.ragged);      // (the others are not captured)
     static const bool pdl = [] { const char* e = getenv("MINFER_VERIFY_PDL"); return !(e && atoi(e) == 0); }();
     const bool fused = M <= kMaxFusedTok;
     // The token tile of the whole pass (the products share the operand order): wide ones issue less per value and read the weights
