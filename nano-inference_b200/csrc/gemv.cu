@@ -173,11 +173,32 @@ static int launch_one(mi_ctx* ctx, const mi_weight* w, const GemvIO& io, int ksp
     return MI_OK;
 }
 
+// Whether the streaming kernel takes a stack, without a K split; otherwise the folded one does.  The streaming kernel's warps take whole row groups, so it
+// goes by rounds of SMs x 8 groups, and one that begins costs half its time even for a single group; the folded one's time follows the
+// bytes, at about 5 TB/s with eight warps per CTA (up to 2048 columns), at 4 with the 16 or 24 that a deeper matrix needs: few of those fit
+// an SM.  Measured (us, folded / streaming; distinct matrices beyond the L2):
+//     rows            14000        20000        37800        44000        61000        66000        75000
+//     1536 columns   3.6 / 6.1    5.7 / 6.9    8.8 / 7.7   9.9 / 11.9  12.8 / 12.7  13.8 / 12.7  15.1 / 13.1
+//     2048           4.3 / 7.7    6.5 / 8.3   10.2 / 9.5  11.1 / 14.4  14.7 / 15.7  15.4 / 15.8  17.2 / 16.2
+//     3072           8.5 / 9.9   12.6 / 11.2  22.1 / 13.3 24.5 / 20.1  33.8 / 21.9  35.3 / 21.7  39.7 / 22.8
+//     4864          11.3 / 13.7  15.9 / 14.2  27.0 / 18.1 31.2 / 28.9  42.7 / 32.1  45.0 / 31.7  50.6 / 33.2
+//     8960          17.9 / 23.3  26.8 / 24.2  43.4 / 30.8 50.6 / 51.3  65.2 / 52.9  70.1 / 53.2  79.4 / 57.5
+//     11008         20.0 / 28.3  28.8 / 28.8  46.9 / 37.1 55.3 / 62.1  72.0 / 64.2  76.7 / 64.8  86.8 / 70.7
+static bool stream_whole(const mi_ctx* ctx, const mi_weight* w) {
+    const long long units = (long long)w->count * w->groups, sms = ctx->sm_count, round = sms * 8;
+    const int steps = (w->nb + 7) / 8;
+    if (units >= 2 * round) return true;
+    if (steps <= 8) return units >= 14 * sms;
+    return units >= 4 * sms && !(steps >= 24 && units > round && units < round + round / 3);
+}
+
 template <int KB, bool DUMP>
 static int launch_kb(mi_ctx* ctx, const mi_weight* w, const GemvIO& io, int ksplit, int variant) {
     if (DUMP) return launch_one<KB, 8, 2, true>(ctx, w, io, 1);
-    // fewer than two row groups per warp of the streaming kernel's grid: there it would have to split K over the grid
-    if (variant == 0 && ksplit <= 0 && w->count * w->groups < 2LL * ctx->sm_count * 8) return launch_fold<KB>(ctx, w, io);
+    if (variant == 0 && ksplit <= 0) {
+        if (!stream_whole(ctx, w)) return launch_fold<KB>(ctx, w, io);
+        ksplit = 1;
+    }
     switch (variant) {
         case 0: return launch_one<KB, 8, 3, false>(ctx, w, io, ksplit);
         case 1: return launch_one<KB, 8, 4, false>(ctx, w, io, ksplit);
