@@ -267,10 +267,11 @@ struct Pass {
 };
 enum { HEAD_ALL, HEAD_LAST, HEAD_NONE };
 
-// Positions that a launch sequence is planned for: captured passes of up to 160 cached positions (one chunk: see plan_attn_tok) share one
-// plan, beyond that those up to 512, 768, 1024, 1536, .. (the plan only cuts the ranges, it is right for any position).
+// Positions that a launch sequence is planned for: captured passes of up to 160 cached positions share one plan, for 128 (one chunk: see
+// plan_attn_tok; 48 sequences of the 1.5B shape at 40 positions 2.32 ms with the plan for 160, which cuts them, 2.23 so), beyond that those up to
+// 512, 768, 1024, 1536, .. (the plan only cuts the ranges, it is right for any position).
 int attn_bucket(int lp_max) {
-    if (lp_max <= 160) return 160;
+    if (lp_max <= 160) return 128;
     int b = 512;
     while (b < lp_max) b *= 2;
     return b > 512 && lp_max <= b / 4 * 3 ? b / 4 * 3 : b;
