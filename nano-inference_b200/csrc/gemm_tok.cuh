@@ -111,6 +111,8 @@ inline TokTiling tok_tiling(int M, int max_nt = kMaxTokNT) {
 // How a launch over one matrix and M tokens is cut (see plan_gemm_tok).
 struct GemmPlan { int NT, TT, ksg, kct, C, kw; bool fold; size_t smem; double cost; };
 int plan_gemm_tok(mi_ctx* ctx, const mi_weight* w, int mode, int M, const TokTiling& tiles, GemmPlan* out);
+// The products of a pass of M tokens over L layers, QKV, O, gate/up, down (mats: those of one layer) and the lm_head over the last n_head of them (0: none)
+int plan_pass_products(mi_ctx* ctx, const mi_weight* const mats[5], int L, int M, int n_head, TokTiling* tiles, GemmPlan plans[5]);
 int launch_gemm_tok(mi_ctx* ctx, const mi_weight* w, const GemmPlan& plan, int mode, bool rowmajor, GemmParams p, bool pdl);
 
 }  // namespace mi

@@ -291,23 +291,13 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     const AttnPlan pa = plan_attn_tok(ctx, m->NH, m->NKV, m->HD, M, a.head == HEAD_ALL ? attn_bucket(a.lp_max) : a.lp_max, a.ragged);      // (the others are not captured)
     static const bool pdl = [] { const char* e = getenv("MINFER_VERIFY_PDL"); return !(e && atoi(e) == 0); }();
     const bool fused = M <= kMaxFusedTok;
-    // The token tile of the whole pass (the products share the operand order): wide ones issue less per value and read the weights
-    // less often, narrow ones leave more warps per sub-partition and divide the work more evenly (333 tokens of the 1.5B shape
-    // 8.72 -> 8.21 ms with 24 per tile, 64 sequences of the 3B shape 4.86 -> 4.66 ms with 16).  The cheapest by the products' cost model.
     const int ML = a.head == HEAD_LAST ? 1 : M;
-    GemmPlan pq, po, pg, pd, pl;
-    TokTiling tiles = tok_tiling(M);
-    double best = 1e300;
+    const mi_weight* const mats[5] = {&m->views[0], &m->views[1], &m->views[2], &m->views[3], &m->views[4 * L]};
+    GemmPlan plans[5];
+    TokTiling tiles;
     int st;
-    for (int max_nt = kMaxTokNT; max_nt >= 2 && (max_nt == kMaxTokNT || M > kMaxFusedTok); max_nt--) {
-        const TokTiling tl = tok_tiling(M, max_nt);
-        GemmPlan p[5];
-        if ((st = plan_gemm_tok(ctx, &m->views[0], fused ? GEMM_QKV : GEMM_PLAIN, M, tl, &p[0])) || (st = plan_gemm_tok(ctx, &m->views[1], GEMM_PART, M, tl, &p[1])) ||
-            (st = plan_gemm_tok(ctx, &m->views[2], fused ? GEMM_GU : GEMM_PLAIN, M, tl, &p[2])) || (st = plan_gemm_tok(ctx, &m->views[3], GEMM_PART, M, tl, &p[3])) ||
-            (st = plan_gemm_tok(ctx, &m->views[4 * L], GEMM_PLAIN, ML, ML == M ? tl : tok_tiling(ML), &p[4]))) return st;
-        const double cost = L * (p[0].cost + p[1].cost + p[2].cost + p[3].cost) + (a.head == HEAD_NONE ? 0.0 : p[4].cost);
-        if (cost < best) { best = cost; tiles = tl; pq = p[0]; po = p[1]; pg = p[2]; pd = p[3]; pl = p[4]; }
-    }
+    if ((st = plan_pass_products(ctx, mats, L, M, a.head == HEAD_NONE ? 0 : ML, &tiles, plans))) return st;
+    const GemmPlan &pq = plans[0], &po = plans[1], &pg = plans[2], &pd = plans[3], &pl = plans[4];
     xf.J = attf.J = actf.J = tiles.J();
     const int nt_norm = std::min(1024, (E / 4 + 31) / 32 * 32);
     GemmParams g{};
