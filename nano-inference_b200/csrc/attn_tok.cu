@@ -55,11 +55,13 @@ __device__ __forceinline__ double half_hi(unsigned w) { return (double)__half2fl
 __device__ __forceinline__ void attn_emit(const AttnParams& p, int token, int e, float4 v) {
     *reinterpret_cast<float4*>(p.out + (size_t)token * p.NH * p.HD + e) = v;
     if (!p.x.q) return;                            // uniform
-    float a = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+    // the maximum over the bits, as in the single-token kernel: a NaN counts as the largest
+    unsigned am = max(max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.y))), max(__float_as_uint(fabsf(v.z)), __float_as_uint(fabsf(v.w))));
     const unsigned mask = 0xffu << (threadIdx.x & 24);               // a block's eight threads, all here or none
-    a = fmaxf(a, __shfl_xor_sync(mask, a, 1));
-    a = fmaxf(a, __shfl_xor_sync(mask, a, 2));
-    a = fmaxf(a, __shfl_xor_sync(mask, a, 4));
+    am = max(am, __shfl_xor_sync(mask, am, 1));
+    am = max(am, __shfl_xor_sync(mask, am, 2));
+    am = max(am, __shfl_xor_sync(mask, am, 4));
+    const float a = __uint_as_float(am);
     const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
     const unsigned q = ((unsigned)__float2int_rn(__fmul_rn(v.x, inv)) & 0xffu) | (((unsigned)__float2int_rn(__fmul_rn(v.y, inv)) & 0xffu) << 8) |
                        (((unsigned)__float2int_rn(__fmul_rn(v.z, inv)) & 0xffu) << 16) | ((unsigned)__float2int_rn(__fmul_rn(v.w, inv)) << 24);

@@ -62,7 +62,7 @@ __device__ __forceinline__ void mma_s8(int (&d)[4], unsigned a0, unsigned a1, un
 
 // One tile (32 rows, KB blocks) against NT * 8 tokens.  Lane (g = lane / 4, t = lane % 4) holds rows g + 8 i (i = 0..3) and tokens
 // 2t, 2t + 1 of every token group: acc[j][2 i + c] is row g + 8 i, token 8 j + 2 t + c.
-// poison: 0 + 0 * scale over all scales seen: NaN once a weight scale was not finite (its bits would pass for a number above).
+// poison: 0 + 0 * scale over all scales seen: NaN once a weight scale was not finite (its bits pass for a number here; see row_sum).
 // pair: upper halves 0x43300000.
 template <int KB, int NT>
 __device__ __forceinline__ void tile_mma(const uint8_t* tile, const uint2* bs, const double* dxs, int lane, double (&acc)[NT][8], __half2 (&poison)[4], double (&pair)[4]) {
@@ -110,6 +110,35 @@ __device__ __forceinline__ void tile_mma(const uint8_t* tile, const uint2* bs, c
                 }
         }
     }
+}
+
+// One row's sum over a warp's steps (every kw-th from t0 on, below t1) for token n, formed as the GEMV forms it.  For rows with a weight scale that is not
+// finite: infinities and NaN come out as they do there.  Straight from global memory; such rows do not occur in a working model.
+template <int KB, bool ROWMAJOR>
+__device__ __forceinline__ double row_sum(const GemmParams& p, int grp, int row, int n, int t0, int t1, int kw) {
+    double acc = 0.0;
+    #pragma unroll 1
+    for (int t = t0; t < t1; t += kw) {
+        #pragma unroll 1
+        for (int b = t * kStepBlk; b < min((t + 1) * kStepBlk, p.nb); b++) {
+            const uint8_t* tile = p.base + ((size_t)grp * p.nb + b / KB * KB) * kTileRowBytes;
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(tile) + b % KB * 32 + row);
+            const float dw = __half2float(__ldg(reinterpret_cast<const __half*>(tile + KB * 512) + row * KB + b % KB));
+            int4 xa, xc;
+            float dx;
+            if constexpr (ROWMAJOR) {
+                const int4* x = reinterpret_cast<const int4*>(p.xq + ((size_t)n * p.nb + b) * 32);
+                xa = __ldcg(x); xc = __ldcg(x + 1);
+                dx = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(p.xd) + (size_t)n * p.nb + b)));
+            } else {
+                auto word = [&](int e) { return (int)__ldcg(p.x.q + tok_word(p.x.J, b, n, e)); };
+                xa = make_int4(word(0), word(4), word(8), word(12)); xc = make_int4(word(16), word(20), word(24), word(28));
+                dx = (float)__dmul_rn(__ldcg(p.x.d + tok_scale(p.x.J, b, n)), 0x1p-1004);
+            }
+            acc = blk_acc(acc, dw, dx, dot_q4_block(w, xa, xc), __int2float_rn(8 * sum_x_block(xa, xc)));
+        }
+    }
+    return acc;
 }
 
 template <int KB, int NT, int MODE, bool ROWMAJOR, bool FOLD>
@@ -259,12 +288,21 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
                 }
             }
         }
+        unsigned bad = 0;                                                                // bit i: row g + 8 i has such a scale among this warp's tiles
         #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const double po = (double)__half2float(__hadd(__low2half(poison[i]), __high2half(poison[i])));
-            #pragma unroll
-            for (int j = 0; j < NT; j++) { acc[j][2 * i] = __dadd_rn(acc[j][2 * i], po); acc[j][2 * i + 1] = __dadd_rn(acc[j][2 * i + 1], po); }
-        }
+        for (int i = 0; i < 4; i++) bad |= (unsigned)__hisnan(__hadd(__low2half(poison[i]), __high2half(poison[i]))) << i;
+        // those rows' sums again, over the ones the lane has just stored: store(row of the group, token of the tile, sum)
+        auto again = [&](auto store) {
+            #pragma unroll 1
+            for (; bad; bad &= bad - 1) {
+                const int row = g + 8 * (__ffs(bad) - 1);
+                #pragma unroll 1
+                for (int q = 0; q < 2 * NT; q++) {
+                    const int n = 8 * (q >> 1) + 2 * t4 + (q & 1);
+                    if (n < ntok) store(row, n, row_sum<KB, ROWMAJOR>(p, grp0, row, tt * N + n, k0 + part, k1, kw));
+                }
+            }
+        };
         if constexpr (!FOLD) {
             if (!mine) continue;
             // straight from the MMA's layout: lane (g, t4) has rows g + 8 i and tokens 8 j + 2 t4 + cc
@@ -282,6 +320,12 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
                         else p.y[(size_t)(tt * N + n) * p.rows + row] = __double2float_rn(acc[j][2 * i + cc]) + bv;
                     }
             }
+            if (bad) again([&](int r32, int n, double v) {
+                const int row = grp0 * 32 + r32;
+                if (row >= p.rows) return;
+                if constexpr (MODE == GEMM_PART) __stcg(p.part + ((size_t)sp * p.M + tt * N + n) * p.ldp + row, v);
+                else p.y[(size_t)(tt * N + n) * p.rows + row] = __double2float_rn(v) + (p.bias ? __ldg(p.bias + row) : 0.f);
+            });
         } else {
             double* fold = reinterpret_cast<double*>(scratch);                           // [warp][token][kFoldLd]
             if (r > 0) __syncthreads();                                                  // the previous round's sums have been read
@@ -291,6 +335,7 @@ __global__ void __launch_bounds__(tok_warps(NT) * 32, 1) gemm_q4_q8_tok_kernel(c
                 for (int j = 0; j < NT; j++)
                     #pragma unroll
                     for (int i = 0; i < 8; i++) fw[(8 * j + 2 * t4 + (i & 1)) * kFoldLd + g + 8 * (i >> 1)] = acc[j][i];
+                if (bad) again([&](int row, int n, double v) { fw[n * kFoldLd + row] = v; });
             }
             __syncthreads();
             // one warp per (row group [pair], token): lane = row
