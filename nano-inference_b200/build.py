@@ -90,10 +90,14 @@ def build_host(force=False, verbose=False):
         _run([GXX, "-O2", "-std=c++17", "-pthread", "-o", synth, HOST / "gguf_synth.cpp"], verbose)
     out.append(synth)
     fast = LIB.parent / "minfer_fastcall.so"
-    if force or _newer(fast, [HOST / "fastcall.cpp", LIB, ROOT / "include" / "minfer_b200.h"]):
-        _run([GXX, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-I", ROOT / "include", "-o", fast,
+    python_h = Path(sysconfig.get_paths()["include"]) / "Python.h"
+    if not python_h.exists():                # an interpreter without headers: the binding calls through ctypes
+        print(f"{python_h} not found: {fast.name} is not built")
+    elif force or _newer(fast, [HOST / "fastcall.cpp", LIB, ROOT / "include" / "minfer_b200.h"]):
+        _run([GXX, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", python_h.parent, "-I", ROOT / "include", "-o", fast,
               HOST / "fastcall.cpp", "-L", LIB.parent, "-lminfer_b200", "-Wl,-rpath,$ORIGIN"], verbose)
-    out.append(fast)
+    if fast.exists():
+        out.append(fast)
     for name in ("cuda_infer", "mega"):
         src = HOST / f"{name}.cpp"
         if not src.exists():

@@ -2,7 +2,10 @@
 // call on converting six arguments, as long as a small product takes on the GPU.  A tensor argument is anything with data_ptr()
 // (torch), a .ctypes.data (numpy), an integer address or None.  Only argument passing lives here; status codes are
 // returned as they are and turned into exceptions by the binding.
+// Only the limited API of Python 3.10 is used, so one build serves every interpreter from there on; where it cannot be loaded, or was not built, the
+// binding makes the same calls through ctypes.
 #define PY_SSIZE_T_CLEAN
+#define Py_LIMITED_API 0x030A0000
 #include <Python.h>
 
 #include "minfer_b200.h"
@@ -15,7 +18,7 @@ PyObject *s_data_ptr, *s_ctypes, *s_data, *s_shape;
 bool address(PyObject* o, void** out) {
     if (o == Py_None) { *out = nullptr; return true; }
     if (PyLong_Check(o)) { *out = PyLong_AsVoidPtr(o); return !PyErr_Occurred(); }
-    PyObject* v = PyObject_CallMethodNoArgs(o, s_data_ptr);
+    PyObject* v = PyObject_CallMethodObjArgs(o, s_data_ptr, static_cast<PyObject*>(nullptr));
     if (!v && PyErr_ExceptionMatches(PyExc_AttributeError)) {
         PyErr_Clear();
         PyObject* c = PyObject_GetAttr(o, s_ctypes);
