@@ -12,6 +12,7 @@
 // extra tokens with one constant slope; here the two step kinds are different code paths, so the loop prices them by what
 // it has measured itself: the device time of its own single-token steps and of its own M-token passes.
 #include "model.cuh"
+#include "step_prices.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -47,7 +48,7 @@ extern "C" int mi_generate_spec(mi_ctx* ctx, mi_model* m, const int32_t* prompt_
     if (!m || !prompt_host || !out_tokens_host || n_prompt < 1 || n_gen < 0) return set_error(ctx, MI_ERR_INVALID, "generate_spec: bad argument");
     if (m->tp_world != 1) return set_error(ctx, MI_ERR_UNSUPPORTED, "generate_spec: the M-token step runs on an unsharded model");
     if (n_prompt + n_gen > m->max_seq) return set_error(ctx, MI_ERR_LIMIT, "generate_spec: %d prompt + %d generated tokens exceed the KV cache of %d", n_prompt, n_gen, m->max_seq);
-    constexpr int kMaxPass = 16;                                     // tokens per M-token pass
+    constexpr int kMaxPass = StepPrices::kMaxPass;                   // tokens per M-token pass
     ngmax = std::max(1, std::min(ngmax, 8));
     const bool forced = draftk < 0;                                   // draft whenever a draft exists, whatever it costs
     draftk = std::max(0, std::min(forced ? -draftk : draftk, kMaxPass - 1));
@@ -73,33 +74,9 @@ extern "C" int mi_generate_spec(mi_ctx* ctx, mi_model* m, const int32_t* prompt_
     }
     int32_t cur = seq.back();
     int pos = n_prompt, n_emit = 0;
-    // What a step costs, as measured by this loop (device milliseconds, running averages): a single-token step, and an
-    // M-token pass for every M used so far; an M not yet seen is priced from the nearest seen one along the measured shape
-    // of the pass time (about 0.49 + 0.032 M of the 16-token pass).
-    float t_dec = 0.f, t_ver[kMaxPass + 1] = {0.f};
-    auto learn = [](float& avg, float ms) { if (ms > 0.f) avg = avg > 0.f ? 0.8f * avg + 0.2f * ms : ms; };
-    for (int M = 1; M <= kMaxPass; M++) t_ver[M] = prompt_ms[M];     // the prompt's own passes are the first measurements
-    auto pass_ms = [&](int M) {
-        if (t_ver[M] > 0.f) return t_ver[M];
-        for (int d = 1; d <= kMaxPass; d++)
-            for (int q : {M - d, M + d})
-                if (q >= 1 && q <= kMaxPass && t_ver[q] > 0.f) return t_ver[q] * (0.49f + 0.032f * M) / (0.49f + 0.032f * q);
-        return 0.f;
-    };
-    // acceptance probability of one drafted token (running estimate), and the draft length that pays best for it
-    float alpha = 0.6f; long probe = 0;
-    auto best_len = [&](int kmax) {
-        if (t_dec <= 0.f) return 0;                                   // nothing to compare with yet: take a plain step and measure it
-        int kb = 0; float vb = 1.f / t_dec, pw = alpha;
-        for (int K = 1; K <= kmax; K++) {
-            pw *= alpha;                                              // alpha^(K+1)
-            const float tv = pass_ms(K + 1);
-            if (tv <= 0.f) continue;
-            const float expect = alpha < 0.999f ? (1.f - pw) / (1.f - alpha) : (float)(K + 1);
-            if (expect / tv > vb) { vb = expect / tv; kb = K; }
-        }
-        return kb;
-    };
+    StepPrices prices;
+    for (int M = 1; M <= kMaxPass; M++) prices.learn_pass(M, prompt_ms[M]);     // the prompt's own passes are the first measurements
+    float alpha = 0.6f; long probe = 0;                               // acceptance probability of one drafted token (running estimate)
     int32_t draft[kMaxPass], hb[kMaxPass], r[kMaxPass];
     const int stop = m->stop_token;                                   // generation ends with this token (src/cuda_infer.cu:1254,1272-1275)
     auto stopped = [&]() { return stop >= 0 && n_emit > 0 && out_tokens_host[n_emit - 1] == stop; };
@@ -108,16 +85,16 @@ extern "C" int mi_generate_spec(mi_ctx* ctx, mi_model* m, const int32_t* prompt_
         K = std::min(K, m->max_seq - 1 - pos);                         // KV headroom
         K = std::min(K, n_gen - n_emit - 1);                          // nothing is gained by drafting past the end
         if (K > 0 && !forced) {
-            const int want = best_len(K);
+            const int want = prices.best_draft(alpha, K, pos);        // the draft length that pays best
             // while drafting does not pay, every 32nd step still tests one drafted token, so that the estimate can recover
             // (src/cuda_infer.cu:1233-1243); a test that succeeds is followed by the next one at once
-            if (want == 0 && t_dec > 0.f && (probe++ % 32) == 0) K = 1;
+            if (want == 0 && prices.knows_step() && (probe++ % 32) == 0) K = 1;
             else K = want;
         }
         if (K <= 0) {
             int32_t nxt; float ms = 0.f;
             if ((st = mi_decode(ctx, m, &cur, 1, 1, pos, &nxt, nullptr, MI_DECODE_PERSISTENT, &ms))) return st;
-            learn(t_dec, ms);
+            prices.learn_step(ms);
             if (margins_host) { margins_host[n_emit] = cur_margin; if ((st = mi_decode_margins(ctx, m, 1, &cur_margin))) return st; }
             out_tokens_host[n_emit++] = cur;
             cur = nxt; pos++; seq.push_back(cur);
@@ -129,7 +106,7 @@ extern "C" int mi_generate_spec(mi_ctx* ctx, mi_model* m, const int32_t* prompt_
         for (int k = 0; k < K; k++) hb[1 + k] = draft[k];
         float vms = 0.f;
         if ((st = mi_verify(ctx, m, hb, T, pos, r, nullptr, &vms))) return st;          // r[j] = the model's token after hb[j]
-        learn(t_ver[T], vms);
+        prices.learn_pass(T, vms);
         int a = 0;
         while (a < K && draft[a] == r[a]) a++;
         if (margins_host) {
