@@ -339,18 +339,23 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
 // The pass as a CUDA graph: the launch sequence is fixed by the number of tokens, the range of positions that its attention
 // grid covers and the cache; tokens and positions live in device memory.  The first pass of a kind runs plainly, the second
 // is captured - on a stream of its own, the caller's may be the legacy default stream - and replayed from then on.
-// MINFER_VERIFY_GRAPH=0 runs everything plainly.
-int run_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
+// MINFER_VERIFY_GRAPH=0 runs everything plainly.  `start`: recorded when the pass is about to run, behind any capturing (which the host does for
+// milliseconds while the stream waits; the time of a pass is what it costs from then on), or null.
+int run_pass(mi_ctx* ctx, mi_model* m, const Pass& a, cudaEvent_t start) {
     VerifyBufs& b = m->vb;
+    auto plainly = [&]() -> int {
+        if (start) MI_CUDA(ctx, cudaEventRecord(start, ctx->stream));
+        return enqueue_pass(ctx, m, a);
+    };
     static const bool use_graph = [] { const char* e = getenv("MINFER_VERIFY_GRAPH"); return !(e && atoi(e) == 0); }();
     const int regime = attn_bucket(a.lp_max);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!use_graph || a.head != HEAD_ALL || cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return enqueue_pass(ctx, m, a);
+    if (!use_graph || a.head != HEAD_ALL || cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return plainly();
     const PassKey key{a.M, regime, a.ragged ? 1 : 0, (const void*)a.kc, (const void*)a.vc, a.max_seq};
     bool again;
     void* graph = b.graphs.use(key, &again, destroy_graph);
     if (!graph) {
-        if (!again) return enqueue_pass(ctx, m, a);
+        if (!again) return plainly();
         cudaStream_t cs = nullptr, user = ctx->stream;
         MI_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
@@ -372,6 +377,7 @@ int run_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         graph = ge;
         b.graphs.put(key, graph, destroy_graph);                       // (no pass is in flight here: every call ends with a wait)
     }
+    if (start) MI_CUDA(ctx, cudaEventRecord(start, ctx->stream));
     MI_CUDA(ctx, cudaGraphLaunch((cudaGraphExec_t)graph, ctx->stream));
     return MI_OK;
 }
@@ -396,8 +402,7 @@ extern "C" int mi_verify(mi_ctx* ctx, mi_model* m, const int32_t* tokens_host, i
     memcpy(b.h_meta, tokens_host, (size_t)M * 4);                     // pinned: free again once the call has synchronized below
     b.h_meta[M] = pos0;
     MI_CUDA(ctx, cudaMemcpyAsync(b.meta, b.h_meta, (size_t)(M + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    MI_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
-    if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + M, HEAD_ALL}))) return st;
+    if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + M, HEAD_ALL}, m->ev0))) return st;
     MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
     if (logits_dev) MI_CUDA(ctx, cudaMemcpyAsync(logits_dev, b.logits, (size_t)M * m->V * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     if (out_tokens_host) MI_CUDA(ctx, cudaMemcpyAsync(b.h_meta, b.out, (size_t)M * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -431,7 +436,7 @@ extern "C" int mi_prefill(mi_ctx* ctx, mi_model* m, const int32_t* tokens_host, 
         b.h_meta[M] = pos0 + i0;
         MI_CUDA(ctx, cudaMemcpyAsync(b.meta, b.h_meta, (size_t)(M + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
         MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
-        if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + i0 + M, k == passes - 1 ? HEAD_LAST : HEAD_NONE}))) return st;
+        if ((st = run_pass(ctx, m, Pass{M, false, m->P.kc, m->P.vc, m->max_seq, 0, pos0 + i0 + M, k == passes - 1 ? HEAD_LAST : HEAD_NONE}, nullptr))) return st;
     }
     MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
     if (next_token_host) MI_CUDA(ctx, cudaMemcpyAsync(b.h_meta, b.out, 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -523,7 +528,6 @@ extern "C" int mi_batch_step(mi_ctx* ctx, mi_batch* b, int n, const int32_t* tok
     if ((st = ensure_bufs(ctx, m, std::min(n, BMAX), std::min(n, BMAX)))) return st;
     VerifyBufs& vb = m->vb;
     if ((st = mi::reset_after_error(ctx, m))) return st;
-    MI_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
     for (int i0 = 0; i0 < n; i0 += BMAX) {
         const int M = std::min(BMAX, n - i0);
         memcpy(vb.h_meta, tokens_host + i0, (size_t)M * 4);
@@ -531,7 +535,7 @@ extern "C" int mi_batch_step(mi_ctx* ctx, mi_batch* b, int n, const int32_t* tok
         memcpy(vb.h_meta + 2 * M, slots_host + i0, (size_t)M * 4);
         const int lp_max = *std::max_element(positions_host + i0, positions_host + i0 + M) + 1;
         MI_CUDA(ctx, cudaMemcpyAsync(vb.meta, vb.h_meta, (size_t)3 * M * 4, cudaMemcpyHostToDevice, ctx->stream));
-        if ((st = run_pass(ctx, m, Pass{M, true, b->kc, b->vc, b->max_seq, b->slab_stride, lp_max, HEAD_ALL}))) return st;
+        if ((st = run_pass(ctx, m, Pass{M, true, b->kc, b->vc, b->max_seq, b->slab_stride, lp_max, HEAD_ALL}, i0 == 0 ? m->ev0 : nullptr))) return st;
         if (logits_dev) MI_CUDA(ctx, cudaMemcpyAsync(logits_dev + (size_t)i0 * m->V, vb.logits, (size_t)M * m->V * 4, cudaMemcpyDeviceToDevice, ctx->stream));
         if (i0 + BMAX >= n) MI_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
         if (out_tokens_host) MI_CUDA(ctx, cudaMemcpyAsync(vb.h_meta, vb.out, (size_t)M * 4, cudaMemcpyDeviceToHost, ctx->stream));
