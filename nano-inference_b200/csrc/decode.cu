@@ -18,6 +18,9 @@ using namespace mi;
 namespace mi {
 const void* decode_kernel_prof(int HD, int G); const void* decode_kernel_tp(int HD, int G); const void* decode_kernel_lean(int HD, int G);
 const void* decode_kernel_prof_lean(int HD, int G);
+const void* decode_kernel_prof_lean_long(int HD, int G);
+const void* decode_kernel_prof_lean_small(int HD, int G);
+const void* decode_kernel_prof_lean_small_long(int HD, int G);
 const void* decode_kernel_tp_lean(int HD, int G);
 const void* decode_kernel_tp_prof_lean(int HD, int G);
 const void* decode_kernel_lean_long(int HD, int G);
@@ -125,8 +128,9 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
         if (lean && shape == 1 && P.prof) pick = decode_kernel_tp_prof_lean(m->HD, m->G);
         if (lean && shape == 1 && !pick) pick = decode_kernel_tp_lean(m->HD, m->G);
         if (!pick) pick = decode_kernel_tp(m->HD, m->G);
-    } else if (P.prof) {                            // the instrumented builds (decode_prof.cu, decode_prof_lean.cu)
-        if (lean && shape == 1) pick = decode_kernel_prof_lean(m->HD, m->G);
+    } else if (P.prof) {                            // the instrumented builds (decode_prof*.cu): one for every build that runs without them
+        if (lean) pick = shape == 1 ? decode_kernel_prof_lean(m->HD, m->G) : decode_kernel_prof_lean_small(m->HD, m->G);
+        else if (far) pick = shape == 1 ? decode_kernel_prof_lean_long(m->HD, m->G) : decode_kernel_prof_lean_small_long(m->HD, m->G);
         if (!pick) pick = decode_kernel_prof(m->HD, m->G);
     } else {
         if (lean) pick = shape == 1 ? decode_kernel_lean(m->HD, m->G) : decode_kernel_lean_small(m->HD, m->G);

@@ -100,7 +100,13 @@
 #ifndef MI_SMALL
 #define MI_SMALL 0
 #endif
-#if MI_SMALL && MI_LEAN == 2
+#if MI_PROF && MI_SMALL && MI_LEAN == 2
+#define MI_KVARIANT profsmalllong
+#elif MI_PROF && MI_SMALL && MI_LEAN
+#define MI_KVARIANT profsmall
+#elif MI_PROF && !MI_TP && MI_LEAN == 2
+#define MI_KVARIANT proflong
+#elif MI_SMALL && MI_LEAN == 2
 #define MI_KVARIANT leansmalllong
 #elif MI_SMALL && MI_LEAN
 #define MI_KVARIANT leansmall
