@@ -110,7 +110,7 @@ __global__ void rope_cs_kernel(const float* __restrict__ freq, float* __restrict
 // beyond) although the position is device-resident; 0: decided from pos0 and the steps.  (A build
 // launched outside its range ends with MI_ERR_LIMIT on every CTA, it computes nothing wrong.)  only_prepare: pick the
 // kernel and raise its shared-memory limit, launch nothing (what must not happen inside a stream capture).
-int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, int step1, int ph0, int ph1, bool coop, int range_hint = 0,
+int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, int step1, int ph0, int ph1, int range_hint = 0,
                     bool only_prepare = false) {
     void (*kern)(DecodeParams, int, int, int, int) = nullptr;
     // every step of this launch ends within the range the dedicated attention CTAs handle, on a shape the short-context
@@ -156,7 +156,6 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
     }
     // Always a cooperative launch: CTAs wait for one another's tagged words inside every phase range (the K-split fold
     // of the down projection, the greedy pick over all CTAs' candidates), so all of them must be resident together.
-    (void)coop;
     if (only_prepare) return MI_OK;
     void* args[] = {(void*)&P, &step0, &step1, &ph0, &ph1};
     MI_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(m->grid), dim3(DNT), args, m->smem, ctx->stream));
@@ -625,7 +624,7 @@ static int step_graph(mi_ctx* ctx, mi_model* m, int range, cudaGraphExec_t* out)
     DecodeParams P = m->P;
     P.in_tokens = nullptr; P.n_forced = 0; P.out_tokens = m->d_step_out; P.out_margins = m->d_step_margin; P.pos0 = 0; P.pos_dev = m->d_pos;
     P.logits = nullptr; P.logits_stride = m->V; P.wait_ns = ctx->wait_ns; P.stop_token = -1;
-    if ((st = dispatch_launch(ctx, m, P, 0, 1, 0, 1, false, range, true))) return st;      // kernel picked, shared-memory limit raised: not inside the capture
+    if ((st = dispatch_launch(ctx, m, P, 0, 1, 0, 1, range, true))) return st;      // kernel picked, shared-memory limit raised: not inside the capture
     // captured on a stream of its own: the context's stream may be the legacy default stream, which cannot capture
     MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     cudaStream_t cs = nullptr, user = ctx->stream;
@@ -635,7 +634,7 @@ static int step_graph(mi_ctx* ctx, mi_model* m, int range, cudaGraphExec_t* out)
     ctx->stream = cs;
     seq_pre_kernel<<<1, 1, 0, cs>>>(static_cast<const SeqCtl*>(m->d_seq_ctl), m->P.cur_token);
     st = MI_OK;
-    for (int ph = 0; ph < nph && st == MI_OK; ph++) st = dispatch_launch(ctx, m, P, 0, 1, ph, ph + 1, false, range);
+    for (int ph = 0; ph < nph && st == MI_OK; ph++) st = dispatch_launch(ctx, m, P, 0, 1, ph, ph + 1, range);
     seq_post_kernel<<<1, 1, 0, cs>>>(static_cast<SeqCtl*>(m->d_seq_ctl), m->d_step_out, m->d_step_margin, m->d_pos);
     ctx->stream = user;
     cudaGraph_t g = nullptr;
@@ -722,7 +721,7 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
             DecodeParams Ps = P;
             if (Ps.logits) Ps.logits += (long long)cuts[i] * Ps.logits_stride;   // the kernel indexes logits and ring entries from its first step
             Ps.ring.base += cuts[i];
-            if ((st = dispatch_launch(ctx, m, Ps, cuts[i], cuts[i + 1], 0, nph, true))) return st;
+            if ((st = dispatch_launch(ctx, m, Ps, cuts[i], cuts[i + 1], 0, nph))) return st;
         }
     } else if (mode == MI_DECODE_PER_PHASE && !logits_dev && stop < 0 && !ring && ph0 == 0 && ph1 == nph && m->tp_world == 1 && P.drop_phase < 0 && !P.prof &&
                !getenv("MINFER_SEQ_NO_GRAPH")) {
@@ -746,7 +745,7 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
             DecodeParams Ps = P;
             if (Ps.logits) Ps.logits += (long long)s * Ps.logits_stride;    // the kernel indexes logits from its first step
             for (int ph = ph0; ph < ph1; ph++)
-                if ((st = dispatch_launch(ctx, m, Ps, s, s + 1, ph, ph + 1, false))) return st;
+                if ((st = dispatch_launch(ctx, m, Ps, s, s + 1, ph, ph + 1))) return st;
             if (stop >= 0 && s + 1 >= n_forced && s + 1 < n_steps) {
                 // under the stop rule this engine looks at every token before it launches the next step, as the reference's
                 // kernel-sequence driver does (src/cuda_infer.cu:1186-1193)
@@ -931,11 +930,11 @@ static int launch_phases(mi_ctx* ctx, mi_model* m, int pos, int phase_begin, int
             else if (k == 4) mi_model_tp_region(m, MI_TP_PART_DOWN, l, &p, &nb);
             if (p) MI_CUDA(ctx, cudaMemsetAsync(p, 0, (size_t)nb, ctx->stream));
         }
-        if (!fused && (st = dispatch_launch(ctx, m, P, 0, 1, ph, ph + 1, false))) return st;
+        if (!fused && (st = dispatch_launch(ctx, m, P, 0, 1, ph, ph + 1))) return st;
     }
     if (fused && phase_end > phase_begin) {
         // one cooperative launch for the range, the weight ring running ahead across its phases
-        if ((st = dispatch_launch(ctx, m, P, 0, 1, phase_begin, phase_end, true))) return st;
+        if ((st = dispatch_launch(ctx, m, P, 0, 1, phase_begin, phase_end))) return st;
     }
     return MI_OK;
 }

@@ -63,21 +63,12 @@
 // observed, not proved.  Each token is processed exactly as if it were alone.
 #pragma once
 #include "gemv_core.cuh"
-#ifndef MI_ATT_FN
-#define MI_ATT_FN static __device__ __noinline__
-#endif
 // functions that sit out of line to keep the loop body small; the short-context build inlines them instead, because every
 // call site inside the step loop, executed or not, makes the compiler keep the loop's values where a call preserves them
 #if defined(MI_LEAN) && MI_LEAN
 #define MI_COLD_FN static __device__ __forceinline__
 #else
 #define MI_COLD_FN static __device__ __noinline__
-#endif
-#ifndef MI_PIECE
-#define MI_PIECE __forceinline__
-#endif
-#ifndef MI_ATTN_HPC_EVEN
-#define MI_ATTN_HPC_EVEN(G) 2
 #endif
 
 // The kernel exists in several builds.  The default one carries no profiling code and no peer stores.  A translation unit
@@ -238,8 +229,8 @@ struct DecodeParams {
 };
 
 // number of KV chunks for a causal range of Lp positions (host and device agree)
-__host__ __device__ inline int attn_chunks(int Lp, int max_chunks, int chunk = kAttnChunk) {
-    int n = (Lp + chunk - 1) / chunk;
+__host__ __device__ inline int attn_chunks(int Lp, int max_chunks) {
+    int n = (Lp + kAttnChunk - 1) / kAttnChunk;
     return n < 1 ? 1 : (n > max_chunks ? max_chunks : n);
 }
 __host__ __device__ inline int q8_words(int n) { return n / 4 + (n / 32 + 1) / 2 * 2; }     // tagged words of a q8_0 vector of n values
@@ -549,7 +540,7 @@ __device__ __forceinline__ double tree_sum8(double a, double b, double c, double
 // Every warp passes the same number of __syncthreads, also after a wait gave up.
 // bias: added to complete sums by epi; requested before the tiles are worked on (it comes from the L2).
 template <class Epi>
-__device__ MI_PIECE bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, int j, int lane,
+__device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, int j, int lane,
                                             const int8_t* xq_s, const float2* xs_s, const Pub& pub, const float* __restrict__ bias, Epi epi) {
     const Job jb = ws.jobs[j];                          // registers: the fields are used many times
     bool ok = true;
@@ -602,7 +593,7 @@ __device__ MI_PIECE bool run_cta_job(WarpStream& ws, const DecodeParams& P, cons
 
 // lm_head: a unit (row group) belongs to one warp; epi(g, lane, v).
 template <class Epi>
-__device__ MI_PIECE bool run_warp_job(WarpStream& ws, int j, int lane, const int8_t* xq_s, const float2* xs_s, Epi epi) {
+__device__ __forceinline__ bool run_warp_job(WarpStream& ws, int j, int lane, const int8_t* xq_s, const float2* xs_s, Epi epi) {
     const Job jb = ws.jobs[j];
     bool ok = true;
     for (int u = ws.first_warp_unit(jb); u < jb.n_units && ok; u += ws.W) {
@@ -773,7 +764,7 @@ __device__ __forceinline__ bool stage_norm_q8u(MI_NORM_ARGS) {
 // scale, float(8 * sum of the block's values)}.  Thread t takes the 16-byte word pairs t, t + 256, ...; all of a
 // thread's loads are in flight together.
 template <int NP>
-__device__ MI_PIECE bool stage_poll_q8_t(const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, float2* xs_s) {
+__device__ __forceinline__ bool stage_poll_q8_t(const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, float2* xs_s) {
     const int tid = threadIdx.x, nq2 = n / 8, tot2 = nq2 + (n / 32 + 1) / 2, nbk = n / 32;     // pairs of value words, all pairs, blocks
     unsigned long long w[NP][2];
     #pragma unroll
@@ -1112,8 +1103,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
 //           32-dim block to q8_0 and publishes it.
 // Same interface as attention_split.
 template <int HD, int GQ>
-MI_ATT_FN bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* stage,
-                                                unsigned tag_in, const Pub pub) {
+static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l, int pos, uint8_t* stage, unsigned tag_in, const Pub pub) {
     constexpr int DPW = HD / 32;
     constexpr int LPP = 8, DPL = HD / LPP, QSTR = DPL + 2;                 // lanes per position in pass 1, dims per lane, padded stride
     constexpr int KV4 = DPL * 2 / 16 > 0 ? DPL * 2 / 16 : 1;              // 16-byte loads per lane and position
@@ -1292,7 +1282,7 @@ __host__ __device__ inline size_t attn_dedicated_smem(int HD, int HPC) {
 }
 // query heads per attention CTA: two where the group size is even (1.5B: six CTAs of two heads; three heads per CTA
 // measured 4.5 us per layer on the critical path), one where it is odd or at most two
-__host__ __device__ constexpr int attn_heads_per_cta(int G) { return (G % 2 == 0 && G > 2) ? MI_ATTN_HPC_EVEN(G) : 1; }
+__host__ __device__ constexpr int attn_heads_per_cta(int G) { return G % 2 == 0 && G > 2 ? 2 : 1; }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
