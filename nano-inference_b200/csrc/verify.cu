@@ -462,7 +462,10 @@ extern "C" int mi_attn_splitkv(mi_ctx* ctx, const float* q_dev, const uint16_t* 
     if (M < 1 || M > VMAX) return set_error(ctx, MI_ERR_LIMIT, "attention: M=%d queries per call; this entry point takes 1..%d", M, VMAX);
     if (n_head <= 0 || n_head_kv <= 0 || n_head % n_head_kv || pos0 < 0) return set_error(ctx, MI_ERR_INVALID, "attention: bad head counts or position");
     MI_CUDA(ctx, cudaSetDevice(ctx->device));
-    const AttnPlan plan = plan_attn_tok(ctx, n_head, n_head_kv, head_dim, M, pos0 + M, false);
+    AttnPlan plan = plan_attn_tok(ctx, n_head, n_head_kv, head_dim, M, pos0 + M, false);
+    // inside a stream capture nothing may be allocated: without the scratch the range stays in one piece
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (plan.part_doubles > ctx->part_count && cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive) { plan.nch = 1; plan.part_doubles = 0; }
     int st = ensure_scratch(ctx, plan.part_doubles, 0);
     if (st != MI_OK) return st;
     const AttnParams p{q_dev, reinterpret_cast<const __half*>(kcache_dev), reinterpret_cast<const __half*>(vcache_dev), M, n_head, n_head_kv, head_dim, n_head_kv * head_dim,

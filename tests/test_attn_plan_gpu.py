@@ -51,3 +51,29 @@ def test_passes_behind_a_context(ctx, pkg, tmp_path, shape, pos, n):
     for name in ("kcache", "vcache"):
         assert torch.equal(a.state_tensor(name), b.state_tensor(name)), name
     a.free(); b.free()
+
+
+def test_captured_without_scratch(pkg):
+    """A first call inside a stream capture, at a length that is cut elsewhere, allocates nothing."""
+    import torch
+    n_head, n_kv, hd, n = 12, 2, 128, 300
+    K, V = (torch.randn((n, n_kv * hd), device="cuda").half() for _ in range(2))
+    q = torch.randn((1, n_head * hd), device="cuda")
+    out, ref = torch.zeros_like(q), torch.zeros_like(q)
+    c = pkg.Context(0)
+    c.use_torch_stream()
+    c.attn_splitkv(q, K.view(torch.int16), V.view(torch.int16), n_head, n_kv, hd, 20, 1, out)         # the kernel is there, no scratch is
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        c.use_torch_stream()
+        c.attn_splitkv(q, K.view(torch.int16), V.view(torch.int16), n_head, n_kv, hd, n - 1, 1, out)
+    out.zero_()
+    g.replay()
+    c.use_torch_stream()
+    c.attn_splitkv(q, K.view(torch.int16), V.view(torch.int16), n_head, n_kv, hd, n - 1, 1, ref)
+    c.sync()
+    assert rel_err(out[0].cpu().numpy(), attention_f64(q[0].cpu().numpy(), K.cpu().numpy(), V.cpu().numpy(), n_head, n_kv, hd, n - 1)) < 1e-5
+    assert torch.equal(out, ref)
+    del g
+    c.close()
