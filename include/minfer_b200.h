@@ -330,8 +330,9 @@ MI_API int mi_verify(mi_ctx* ctx, mi_model* model, const int32_t* tokens_host, i
 /* Prompt processing: n tokens (any number that fits the cache) at positions pos0 .. pos0+n-1, many per pass over the weights;
  * the same keys, values and prediction, bit for bit, as n single-token steps.  next_token_host (optional) = greedy token after the
  * last one, which also becomes the model's current token; its margin is the first one mi_verify_margins returns.
- * Logits of the other tokens are not computed.  Synchronous.  Unsharded models only.  Replaces the chunked prompt
- * processing of src/cuda_infer.cu:1130-1144. */
+ * Logits of the other tokens are not computed.  Synchronous.  Unsharded models only.  What it computes is the chunked prompt
+ * processing of src/cuda_infer.cu:1130-1144; mi_generate_spec and the two driver programs keep that loop's form, up to 16
+ * tokens per mi_verify pass (TCHUNK), and do not call this. */
 MI_API int mi_prefill(mi_ctx* ctx, mi_model* model, const int32_t* tokens_host, int n, int pos0, int32_t* next_token_host,
                       float* elapsed_ms);
 

@@ -1273,7 +1273,8 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
 // no global load at all.  (2) One fp16 -> double conversion of a K or V element serves all HPC heads.
 // The new position's K and V come with q as tagged words; they go into the shared-memory rows directly and to the global
 // cache after the output has been published (fenced before this CTA's next output, which is what later readers wait for).
-// Per head the arithmetic is attention_short's, operation for operation: same bits.
+// The two passes and the softmax are attention_short's; a dot product is added in another order (eight partial sums over an eighth of the dimensions
+// each, in a tree), in double and rounded to fp32 once: the same bits in every test, observed and not proved.
 constexpr int kAttnRows = kShortAttnMax;
 template <int HD> __host__ __device__ constexpr int attn_row_bytes() { return 2 * HD + 16; }
 __host__ __device__ inline size_t attn_dedicated_smem(int HD, int HPC) {

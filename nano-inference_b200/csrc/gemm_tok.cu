@@ -5,10 +5,12 @@
 // src/mega.cu:197-244).
 //
 // What bounds it.  Every q4_0 block has a scale of its own, so an integer sum lives for K = 32 only: per (row, block,
-// token) one int32 has to be scaled by dw*dx and added in double.  Measured on this part, a DFMA takes 2.25 issue cycles of an
-// SM sub-partition during which nothing else issues, and two of them per value are the floor (4.5 of the 10.6 cycles a
-// value costs here at 32 tokens, 12.8 at 16); an mma.m16n8k32.s8 takes 12 for its four values per lane, the rest
-// are the shared-memory loads and the unpacking.  So the design minimizes what is issued per value:
+// token) one int32 has to be scaled by dw*dx and added in double.  Measured alone, a DFMA keeps an SM sub-partition for 2.25 cycles and an
+// mma.m16n8k32.s8 for 12 (four values per lane): 4.5 + 3 cycles a value, the floor of this scheme.  The rest are moves, shared-memory loads and
+// unpacking.  The gate/up product of 333 tokens (17920 x 1536, tiles of 24, three warps per sub-partition) takes 13.6 cycles a value: issue active 54 %
+// of the cycles, FP64 pipe 32 %, int8 MMA 15 %, so no unit by itself is full, but issued instructions and the cycles above together are 94 % of the
+// time of the SMs that have work; 128 tokens (tiles of 32, two warps, the second round nine tenths full): 15 cycles, 46 / 28 / 13 %, 80 %.  Passes of 16
+// tokens are as much waiting as issue (30 cycles a value at the 1.5B shape's gate/up; first tiles and staging).  So the design minimizes what is issued per value:
 //   * mma.sync and not tcgen05: its operands and sums are registers.  A nibble tile becomes an A fragment with three logic
 //     operations per two registers straight from a 4-byte shared-memory load, and a sum goes from the MMA into the FMA.
 //     A tcgen05.kind::i8 kernel with the same scaling was built and measured beside it: its MMAs cost no issue slots, but
@@ -17,7 +19,7 @@
 //   * t = fma(dw, 2^52 + 2^31 + s, -dw (2^52 + 2^31)) = dw * s exactly, then acc = fma(dx, t, acc), the GEMV's one rounding.
 //     The MMA starts from C = 2^31, so its result read as unsigned is s + 2^31 and with 0x43300000 above it is that
 //     double.  Four register pairs keep the upper half for the whole kernel; a sum costs one move into a lower half.
-//     (Left to itself the compiler moves both halves: 16 instead of 10.6 cycles per value at 32 tokens.)
+//     (Left to itself the compiler moves both halves, half as many cycles again.)
 //   * dw's fp16 bits are shifted into a double's exponent field (see TokX for the powers of two);
 //   * the nibble offset costs nothing: (nibble << 4) ^ 0x80 is the signed byte 16 (n - 8).
 //

@@ -1,4 +1,4 @@
-"""GPU parity of the multi-token q4_0 x q8_0 GEMM (tcgen05 int8 MMA) through the C ABI.
+"""GPU parity of the multi-token q4_0 x q8_0 product (int8 MMA) through the C ABI.
 
 Bars: every token's row of Y equals, bit for bit, what the GEMV entry point returns for
 that token alone - for every M (the reference checks the same property with a logit hash

@@ -1,4 +1,4 @@
-"""GPU parity of the M-token step (mi_verify: tcgen05 GEMM projections + M-query attention)
+"""GPU parity of the M-token step (mi_verify: int8-MMA projections + M-query attention)
 and of the stand-alone split-KV attention entry point (mi_attn_splitkv).
 
 Bars: a token's logits are bit-identical for every M (1..16) and bit-identical to the
