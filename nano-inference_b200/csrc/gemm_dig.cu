@@ -1,0 +1,608 @@
+// q4_0 x q8_0 product of many tokens (prompts, batches of sequences) on tcgen05: the sums of the product over blocks (gemm_tok.cu) and of the GEMV, the same
+// bits, without scaling anything per block.
+//
+// What bounds the other product is one FP64 multiplication per (row, block, token) and the instructions around it.  Here the scales move into the operands: every scale
+// is an fp16 number, so within a row (token, K range) all of them are integers times one power of two, an element is an integer of 18 to 24 bits, and that is cut into
+// base-256 digits: three (four) of the weight's against three (four) planes of the token's.  The MMAs (kind::i8, exact int32 sums) run over all of K; partial
+// products of equal weight 256^s share a sum, so 9 int8 products cost three MMAs of N = 3 tokens and five columns of tensor memory a token.  At the end of a unit the sums are
+// put together as one 64-bit integer and rounded once.  9 products at the int8 rate are 0.035 clocks of an SM per (row, block, token), the two FP64 operations 0.031; but
+// the tensor core needs no issue slots beside it.  The digits hold any row whose scales lie at most 16 binades apart and any token with at most 13 (8 and 5 with three
+// digits); other rows and tokens, and scales that are not finite, are summed block by block behind the main loop.
+//
+// Dataflow of a CTA (one per SM, a unit is 128 rows x T <= 64 tokens x one K range):
+//   copies     : one warp streams the q4_0 tiles (bulk copies, ahead of the wait for the predecessor), one the activation planes, four blocks at a time;
+//   16 warps   : nibbles and scale of a block -> three digits of 32 weights per thread (= row), in registers, then with tcgen05.st into a stage of tensor
+//                memory: A operands come from there, so shared memory serves the activations only.  Each of four groups has a stage of two blocks under way, so
+//                that the way from a freed stage to a full one is a store and two barriers;
+//   one warp   : issues the MMAs; the whole warp runs the loop, one lane issues (see there);
+//   the 16 warps again at the end of a unit, when the first stages of the next one are in place.
+// Measured (event time, launches back to back): gate/up of 333 tokens (17920 x 1536) 78 us against 123 for the product over blocks, down (1536 x 8960) 36 / 64, batch of 64
+// on 22016 x 2048 37 / 49, 2048 x 11008 19 / 29, 151936 x 2048 142 / 250; 32 tokens on 22016 x 2048 31 / 31.  A stage of two blocks takes 620 clocks at 64 tokens, its MMAs 576;
+// the rest is the start (7000 clocks until the first MMA) and the end of a unit (6000).  Tried: weights expanded weight by weight or in byte lanes with seven sums per
+// token (the expansion or the tensor memory is full first), stages of one and four blocks, eight expanding warps, results through arrays in
+// registers (spills): 95 to 210 us for the gate/up.
+#include "gemm_dig.cuh"
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+
+namespace mi {
+namespace {
+
+constexpr int kStepBlk = 8, kStepBytes = kStepBlk * kTileRowBytes;          // blocks per weight copy
+constexpr int kRawSlots = 4, kXSlots = 3, kXStage = 4;                       // rings: weight steps; activations, of four blocks
+constexpr int kStage = 2, kRing = 8;                                        // blocks per stage of weight digits; ring of barriers for the stages
+constexpr int kMaxN = kDigPlanes * kDigMaxT;                                // columns of an MMA
+constexpr int kXBytes = kXStage * kMaxN * 32;
+constexpr int kGroups = 4, kExpWarps = 4 * kGroups, kWarps = kExpWarps + 3, kThreads = kWarps * 32;      // groups of four warps, a quarter of the 128 rows each
+constexpr int kRowNone = 255;
+constexpr long long kBias3 = 0x808080ll, kBias4 = 0x80808080ll;          // of three and four weight digits: DigX::bias times this is in the sums
+
+struct DigParams {
+    const uint8_t* base; const uint8_t* row_exp; int groups, nb, nst, rows;     // tiled weights; nst: steps of eight blocks
+    int ksg, M, bad_rows;
+    DigX x; TokX q8;
+    const float* bias; float* y; double* part; int ldp;
+    int* err;
+};
+
+struct Smem {
+    static constexpr int raw = 0, x = raw + kRawSlots * 4 * kStepBytes, bars = x + kXSlots * kXBytes;
+    static constexpr int n_bars = 2 * kRawSlots + 2 * kXSlots + 2 * kRing + 3;
+    static constexpr int bytes = bars + n_bars * 8 + 16;
+};
+
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
+__device__ __forceinline__ void tc_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t a, const unsigned (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_zero32(uint32_t a) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};"
+                 ::"r"(a), "r"(0) : "memory");
+}
+__device__ __forceinline__ void group_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kExpWarps * 32) : "memory"); }     // all warps that read and clear sums
+__device__ __forceinline__ void tmem_ld4(uint32_t a, int (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
+}
+
+// Bounded wait of a whole warp that also ends when another role has given up.
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    unsigned long long t0 = 0;
+    #pragma unroll 1
+    for (unsigned i = 1;; i++) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if ((i & 255) == 0) {
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+            if (i == 256) t0 = gtime_ns();
+            else if (__any_sync(0xffffffffu, gtime_ns() - t0 > kWaitBudgetNs)) { *abort_flag = 1; return false; }
+        }
+    }
+}
+
+// The digits of a block's 32 weights (nibble n - 8) * m in element order, base 256, each 128 too large and so unsigned (what that adds to the sums is
+// subtracted at the end, DigX::bias).  m = a0 + 256 a1, three digits (|m| < 2^20): two weights per multiplication in lanes of 16 bits, n a0 + c0 and
+// n a1 + c1 + the carry of the former, where c0 + 256 c1 = 0x808080 - 8 m.  Four digits: weight by weight.
+template <int NW>
+__device__ __forceinline__ void expand_block(const uint4& w, int m, unsigned (&d)[NW][8]) {
+    const unsigned ww[4] = {w.x, w.y, w.z, w.w};
+    if constexpr (NW == 3) {
+        const unsigned c = 0x808080u - 8u * (unsigned)m, c0 = (c & 255u) * 0x10001u, c1 = (c >> 8) * 0x10001u;
+        const unsigned a0 = (unsigned)m & 255u, a1 = (unsigned)(m >> 8);
+        #pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const unsigned n = (i < 4 ? ww[i] : ww[i - 4] >> 4) & 0x0F0F0F0Fu;
+            const unsigned ne = n & 0x00FF00FFu, no = __byte_perm(n, 0, 0x4341);
+            const unsigned pe = ne * a0 + c0, po = no * a0 + c0;
+            const unsigned se = ne * a1 + c1 + __byte_perm(pe, 0, 0x4341), so = no * a1 + c1 + __byte_perm(po, 0, 0x4341);
+            d[0][i] = __byte_perm(pe, po, 0x6240); d[1][i] = __byte_perm(se, so, 0x6240); d[2][i] = __byte_perm(se, so, 0x7351);
+        }
+    } else {
+        const unsigned c = 0x80808080u - 8u * (unsigned)m;
+        #pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const unsigned n = (i < 4 ? ww[i] : ww[i - 4] >> 4) & 0x0F0F0F0Fu;
+            unsigned v[4];
+            #pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = __byte_perm(n, 0, 0x4440 + j) * (unsigned)m + c;
+            const unsigned a = __byte_perm(v[0], v[1], 0x5140), b = __byte_perm(v[2], v[3], 0x5140), e = __byte_perm(v[0], v[1], 0x7362), f = __byte_perm(v[2], v[3], 0x7362);
+            d[0][i] = __byte_perm(a, b, 0x5410); d[1][i] = __byte_perm(a, b, 0x7632); d[2][i] = __byte_perm(e, f, 0x5410); d[3][i] = __byte_perm(e, f, 0x7632);
+        }
+    }
+}
+
+__device__ __forceinline__ int scale_exponent(unsigned h) { return max((int)(h >> 10 & 31u), 1); }     // of the unit of the fp16's mantissa, in steps from 2^-25
+__device__ __forceinline__ int scale_mantissa(unsigned h) { return (int)(h & 1023u) + ((h & 0x7C00u) ? 1024 : 0); }
+
+// acc + v * f in 64 bits
+__device__ __forceinline__ long long mad_wide(int v, int f, long long acc) {
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(v), "r"(f), "l"(acc));
+    return r;
+}
+
+// One row's sum over blocks b0 .. b1 for token n, formed as the GEMV forms it: for rows and tokens whose scales the digits cannot hold.
+template <int KB>
+static __device__ __noinline__ double row_sum_dig(const DigParams& p, int row, int n, int b0, int b1) {
+    double acc = 0.0;
+    const int grp = row >> 5, r = row & 31;
+    #pragma unroll 1
+    for (int b = b0; b < b1; b++) {
+        const uint8_t* tile = p.base + ((size_t)grp * p.nb + b / KB * KB) * kTileRowBytes;
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(tile) + b % KB * 32 + r);
+        const float dw = __half2float(__ldg(reinterpret_cast<const __half*>(tile + KB * 512) + r * KB + b % KB));
+        auto word = [&](int e) { return (int)__ldcg(p.q8.q + tok_word(p.q8.J, b, n, e)); };
+        const int4 xa = make_int4(word(0), word(4), word(8), word(12)), xc = make_int4(word(16), word(20), word(24), word(28));
+        const float dx = (float)__dmul_rn(__ldcg(p.q8.d + tok_scale(p.q8.J, b, n)), 0x1p-1004);
+        acc = blk_acc(acc, dw, dx, dot_q4_block(w, xa, xc), __int2float_rn(8 * sum_x_block(xa, xc)));
+    }
+    return acc;
+}
+
+template <int KB, int NW, bool PART>
+__global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_constant__ DigParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* raw = smem + Smem::raw;
+    uint8_t* xs = smem + Smem::x;
+    uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + Smem::bars);
+    uint64_t* raw_empty = raw_full + kRawSlots;
+    uint64_t* x_full = raw_empty + kRawSlots;
+    uint64_t* x_empty = x_full + kXSlots;
+    uint64_t* full = x_empty + kXSlots;
+    uint64_t* empty = full + kRing;
+    uint64_t* d_full = empty + kRing;
+    uint64_t* d_empty = d_full + 1;
+    uint64_t* drained = d_empty + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+    __shared__ int s_abort, s_planes, s_none;
+    volatile int* abort_flag = &s_abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int wRaw = kExpWarps, wX = wRaw + 1, wMma = wX + 1;
+
+    if (tid == 0) {
+        for (int i = 0; i < kRawSlots; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], kExpWarps); }
+        for (int i = 0; i < kRing; i++) { mbar_init(&full[i], 4); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < kXSlots; i++) { mbar_init(&x_full[i], 1); mbar_init(&x_empty[i], 1); }
+        mbar_init(d_full, 1); mbar_init(d_empty, kExpWarps); mbar_init(drained, 1);
+        mbar_fence_init();
+        s_abort = 0; s_planes = 3; s_none = 0;
+    }
+    if (warp == wMma) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __reduce_max_sync(0xffffffffu, *tmem_slot);           // (a reduction's result is in a uniform register, where the MMAs want it)
+
+    // unit -> (K range, row tile, token tile), in this order: what a CTA starts with does not depend on the tokens
+    struct Unit { int rt, ts, sp, k0, k1; };
+    const int row_tiles = (p.groups + 3) / 4;
+    auto unit = [&](int u) {
+        Unit r;
+        r.sp = u % p.ksg; const int v = u / p.ksg;
+        r.rt = v % row_tiles; r.ts = v / row_tiles;
+        r.k0 = r.sp * p.nst / p.ksg; r.k1 = (r.sp + 1) * p.nst / p.ksg;
+        return r;
+    };
+
+    // the weights depend on nothing: their ring fills before the wait for the predecessor
+    int raw_issued = 0, ru = blockIdx.x, rt_step = -1;
+    auto raw_issue = [&](const Unit& U, int t) {                       // whole warp wRaw
+        const int s = raw_issued % kRawSlots, bytes = min(kStepBlk, p.nb - t * kStepBlk) * kTileRowBytes;
+        if (lane == 0) mbar_expect_tx(&raw_full[s], 4 * bytes);
+        __syncwarp();
+        if (lane < 4) {
+            const int g = min(U.rt * 4 + lane, p.groups - 1);           // a missing row group re-reads the last one; its rows are never stored
+            bulk_g2s(raw + ((size_t)s * 4 + lane) * kStepBytes, p.base + ((size_t)g * p.nb + t * kStepBlk) * kTileRowBytes, bytes, &raw_full[s]);
+        }
+        raw_issued++;
+    };
+    if (warp == wRaw) {
+        const Unit U = unit(ru);
+        for (rt_step = U.k0; rt_step < U.k1 && raw_issued < kRawSlots; rt_step++) raw_issue(U, rt_step);
+        if (rt_step >= U.k1) { ru += gridDim.x; rt_step = -1; }
+    }
+    if (warp < kExpWarps) {                                            // all sums start at zero
+        #pragma unroll
+        for (int c = 0; c < 512 / kGroups; c += 32) tmem_zero32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * (512 / kGroups) + c);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+    }
+    pdl_launch_dependents();
+    pdl_wait_prior();
+    // planes in use among all tokens (one wide token costs every MMA of the launch a third more)
+    for (int i = tid; i < p.M * p.ksg; i += kThreads) {
+        const int v = __ldcg(p.x.info + i) >> 8;
+        if (v == 4) s_planes = 4;
+        else if (v == kDigNone) s_none = 1;
+    }
+    __syncthreads();
+    tc_fence_after();
+    const int planes = (int)__reduce_max_sync(0xffffffffu, (unsigned)s_planes);
+    const int T = p.x.T, units = p.ksg * row_tiles * p.x.TT, N = planes == 4 ? 4 * T : dig_rows(T);
+    // tensor memory: sums of weight 256^s in columns s * T .. (the MMAs of a token tile of an odd number of eights reach eight columns further), stages of weight
+    // digits at the end
+    const int ns = NW + planes - 1, fit = (512 - (NW - 1) * T - N) / (kStage * NW * 8), slots = fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
+    const uint32_t a_base = tmem + 512 - slots * (kStage * NW * 8);
+
+    if (warp < kExpWarps) {
+        // ---------------- weights: nibbles and scales -> digits in registers, then in tensor memory (each of four groups of four warps takes every fourth
+        // stage); and the sums of a unit -> results, while the next unit is under way
+        const int q = warp & 3, wg = warp >> 2;
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16), a_row = a_base + ((uint32_t)(q * 32) << 16);
+        auto clear_sums = [&]() {                                      // 32 columns per store
+            for (int c = wg * 32; c < ns * T; c += kGroups * 32) tmem_zero32(trow + min(c, ns * T - 32));
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(d_empty);
+        };
+        int n_done = 0;
+        auto finish = [&](int u) -> bool {
+            constexpr int G = kDigMaxT / kGroups;                      // tokens of a group of warps
+            const Unit U = unit(u);
+            const int ew = __ldg(p.row_exp + min(U.rt * 128 + q * 32 + lane, p.groups * 32 - 1));
+            const int n0 = U.ts * T + wg * G, tg = min(min(T - wg * G, G), p.M - n0), row = U.rt * 128 + q * 32 + lane;       // tokens n0 .. n0 + tg
+            const int info = lane < tg ? __ldcg(p.x.info + (size_t)U.sp * p.M + n0 + lane) : 0;
+            const long long bias = lane < tg ? __ldcg(p.x.bias + (size_t)U.sp * p.M + n0 + lane) * (NW == 4 ? kBias4 : kBias3) : 0;
+            const float bv = !PART && p.bias && row < p.rows ? __ldg(p.bias + row) : 0.f;
+            if (!wait_or_abort(d_full, n_done & 1, abort_flag)) return false;
+            n_done++;
+            tc_fence_after();
+            #pragma unroll 1
+            for (int g = 0; g < tg; g += 4) {                          // (rolled: four tokens at a time fit the registers and the instruction cache)
+                const uint32_t a = trow + wg * G + g;
+                int d[NW + 2][4];
+                unsigned high[4] = {0, 0, 0, 0};
+                if (planes == 4) {
+                    tmem_ld4(a + (NW + 2) * T, d[0]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    #pragma unroll
+                    for (int i = 0; i < 4; i++) high[i] = (unsigned)d[0][i] << (8 * NW - 16);
+                }
+                #pragma unroll
+                for (int i = 0; i < NW + 2; i++) tmem_ld4(a + i * T, d[i]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                #pragma unroll
+                for (int i = 0; i < 4; i++) {                          // the sum itself is below 2^63, whatever its parts are
+                    high[i] += (unsigned)d[4][i];
+                    if constexpr (NW == 4) high[i] += (unsigned)d[5][i] << 8;
+                    long long v = (long long)((unsigned long long)high[i] << 32) - __shfl_sync(0xffffffffu, bias, g + i);
+                    v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
+                    const int ex = __shfl_sync(0xffffffffu, info, g + i) & 255;
+                    const double r = __dmul_rn(__ll2double_rn(v), __hiloint2double((1023 - 50 + ew + ex) << 20, 0));
+                    if (g + i < tg && row < p.rows) {
+                        if constexpr (PART) __stcg(p.part + ((size_t)U.sp * p.M + n0 + g + i) * p.ldp + row, r);
+                        else p.y[(size_t)(n0 + g + i) * p.rows + row] = __double2float_rn(r) + bv;
+                    }
+                }
+            }
+            tc_fence_before();
+            group_barrier();                                           // (columns are cleared by other warps than read them)
+            tc_fence_after();
+            clear_sums();
+            return true;
+        };
+        if (lane == 0) mbar_arrive(d_empty);
+        int s = 0, sc0 = 0, pending = -1;                              // sc0: stages of all units before
+        uint32_t raw_phase = 0;
+        bool ok = true;
+        #pragma unroll 1
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            const Unit U = unit(u);
+            const int ew = __ldg(p.row_exp + min(U.rt * 128 + q * 32 + lane, p.groups * 32 - 1));
+            int sc = sc0 + ((wg - sc0) & (kGroups - 1)), step0 = sc0;
+            #pragma unroll 1
+            for (int t = U.k0; t < U.k1; t++) {
+                const int nblk = min(kStepBlk, p.nb - t * kStepBlk), end = step0 + (nblk + 1) / kStage;
+                if (!(ok = wait_or_abort(&raw_full[s], raw_phase, abort_flag))) break;
+                const uint8_t* grp = raw + ((size_t)s * 4 + q) * kStepBytes;
+                #pragma unroll 1
+                for (; sc < end; sc += kGroups) {
+                    // the first stages of a unit fit beside the last ones of the unit before, whose sums are read then: the MMAs that would make room for more wait for it
+                    if (pending >= 0 && sc - sc0 >= slots) { if (!(ok = finish(pending))) break; pending = -1; }
+                    unsigned d[kStage][NW][8];
+                    #pragma unroll
+                    for (int b = 0; b < kStage; b++) {
+                        const int k = min((sc - step0) * kStage + b, nblk - 1);
+                        const uint8_t* tile = grp + k / KB * (KB * kTileRowBytes);
+                        const uint4 w = *reinterpret_cast<const uint4*>(tile + (k % KB * 32 + lane) * 16);
+                        const unsigned h = *reinterpret_cast<const unsigned short*>(tile + KB * 512 + (lane * KB + k % KB) * 2);
+                        const int m = scale_mantissa(h) << ((scale_exponent(h) - ew) & 31);
+                        expand_block<NW>(w, h & 0x8000u ? -m : m, d[b]);
+                    }
+                    // (a ring of eight barriers, whatever the number of slots: a group never falls two phases behind)
+                    if (sc >= slots && !(ok = wait_or_abort(&empty[(sc - slots) % kRing], ((sc - slots) / kRing) & 1, abort_flag))) break;
+                    tc_fence_after();
+                    #pragma unroll
+                    for (int b = 0; b < kStage; b++)
+                        #pragma unroll
+                        for (int j = 0; j < NW; j++) tmem_st8(a_row + ((sc & (slots - 1)) * kStage + b) * (NW * 8) + 8 * j, d[b][j]);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[sc % kRing]);
+                }
+                if (!ok) break;
+                step0 = end;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[s]);
+                if (++s == kRawSlots) { s = 0; raw_phase ^= 1; }
+            }
+            sc0 = step0;
+            if (ok && pending >= 0) ok = finish(pending);
+            pending = u;
+        }
+        if (ok && pending >= 0) finish(pending);
+    } else if (warp == wRaw) {
+        bool ok = true;
+        for (; ru < units && ok; ru += gridDim.x, rt_step = -1) {
+            const Unit U = unit(ru);
+            for (int t = rt_step < 0 ? U.k0 : rt_step; t < U.k1; t++) {
+                if (raw_issued >= kRawSlots && !wait_or_abort(&raw_empty[raw_issued % kRawSlots], (raw_issued / kRawSlots & 1) ^ 1, abort_flag)) { ok = false; break; }
+                raw_issue(U, t);
+            }
+        }
+    } else if (warp == wX) {
+        // ---------------- activations, four blocks at a time: one copy where three planes are in use, else the fourth one from its own place
+        int issued = 0, slot = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            const Unit U = unit(u);
+            const int b1 = min(U.k1 * kStepBlk, p.nb);
+            for (int b = U.k0 * kStepBlk; b < b1; b += kXStage, issued++) {
+                const int nblk = min(kXStage, b1 - b);
+                if (!wait_or_abort(&x_empty[slot], phase ^ 1, abort_flag)) { ok = false; break; }
+                uint8_t* dst = xs + (size_t)slot * kXBytes;
+                if (lane == 0) mbar_expect_tx(&x_full[slot], nblk * N * 32);
+                __syncwarp();
+                if (planes == 3) {
+                    if (lane == 0) bulk_g2s(dst, p.x.q + dig_offset(p.x, p.nb, U.ts, b, 0, 0, 0), nblk * N * 32, &x_full[slot]);
+                } else if (lane < 4 * nblk) {
+                    const int k = lane >> 2, half = lane >> 1 & 1, j = (lane & 1) * 3;
+                    bulk_g2s(dst + ((k * 2 + half) * N + j * T) * 16, p.x.q + dig_offset(p.x, p.nb, U.ts, b + k, half, j, 0), (j ? 1 : 3) * T * 16, &x_full[slot]);
+                }
+                __syncwarp();
+                if (++slot == kXSlots) { slot = 0; phase ^= 1; }
+            }
+        }
+        if (!ok && lane == 0)                                          // copies in flight target this CTA
+            for (int k = max(0, issued - kXSlots); k < issued; k++) (void)mbar_wait_bounded(&x_full[k % kXSlots], (k / kXSlots) & 1);
+    } else {
+        // ---------------- MMAs: a digit of the weights against all planes of the tokens, into the sums from the digit's own weight up.
+        // The whole warp runs the loop and one lane issues: operands of uniform code are in uniform registers already.  (A loop of one lane took
+        // 100 cycles per MMA to move them there; the MMA itself takes N / 2.)
+        const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        uint32_t elected;
+        asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+        auto mma = [&](uint32_t a, uint32_t x) {                       // one block
+            const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | ((uint64_t)N << 16) | ((uint64_t)8 << 32) | (1ull << 46);
+            #pragma unroll
+            for (int i = 0; i < NW; i++)
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+                    ::"r"(tmem + (uint32_t)(i * T)), "r"(a + 8 * i), "l"(db), "r"(idesc) : "memory");
+        };
+        int n_done = 0, sc = 0, xslot = 0;
+        uint32_t x_phase = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x, n_done++) {
+            const Unit U = unit(u);
+            const int b1 = min(U.k1 * kStepBlk, p.nb);
+            if (!wait_or_abort(d_empty, n_done & 1, abort_flag)) { ok = false; break; }
+            #pragma unroll 1
+            for (int b = U.k0 * kStepBlk; b < b1; b += kXStage) {
+                if (!wait_or_abort(&x_full[xslot], x_phase, abort_flag)) { ok = false; break; }
+                #pragma unroll
+                for (int g = 0; g < kXStage / kStage; g++) {
+                    const int left = b1 - b - g * kStage;
+                    if (left <= 0) break;
+                    if (!wait_or_abort(&full[sc % kRing], (sc / kRing) & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t a = a_base + (sc & (slots - 1)) * (kStage * NW * 8), x = smem_u32(xs) + xslot * kXBytes + g * kStage * N * 32;
+                    if (left >= kStage) {
+                        if (elected) { mma(a, x); mma(a + NW * 8, x + N * 32); tc_commit(&empty[sc % kRing]); }
+                    } else {
+                        if (elected) { mma(a, x); tc_commit(&empty[sc % kRing]); }
+                    }
+                    __syncwarp();
+                    sc++;
+                }
+                if (!ok) break;
+                if (elected) tc_commit(&x_empty[xslot]);
+                __syncwarp();
+                if (++xslot == kXSlots) { xslot = 0; x_phase ^= 1; }
+            }
+            if (ok && elected) tc_commit(d_full);
+            __syncwarp();
+        }
+        if (elected) tc_commit(drained);                               // tensor memory is given back below
+        __syncwarp();
+        (void)mbar_wait_bounded(drained, 0);
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        if (tid == 0) atomicMax(p.err, MI_ERR_TIMEOUT);
+        if (warp == wRaw && lane == 0)
+            for (int k = max(0, raw_issued - kRawSlots); k < raw_issued; k++) (void)mbar_wait_bounded(&raw_full[k % kRawSlots], (k / kRawSlots) & 1);
+    }
+    if (warp == wMma) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+    // What the digits cannot hold, again and over the sums stored above.  (Behind the loops: a call inside them, taken or not, keeps their values
+    // out of half the registers.)
+    if (!p.bad_rows && !s_none) return;
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const Unit U = unit(u);
+        const int b0 = U.k0 * kStepBlk, b1 = min(U.k1 * kStepBlk, p.nb);
+        for (int i = tid; i < 128 * T; i += kThreads) {
+            const int row = U.rt * 128 + (i & 127), n = U.ts * T + (i >> 7);
+            if (row >= p.rows || n >= p.M) continue;
+            if (__ldg(p.row_exp + row) != kRowNone && (__ldcg(p.x.info + (size_t)U.sp * p.M + n) >> 8) != kDigNone) continue;
+            const double v = row_sum_dig<KB>(p, row, n, b0, b1);
+            if constexpr (PART) __stcg(p.part + ((size_t)U.sp * p.M + n) * p.ldp + row, v);
+            else p.y[(size_t)n * p.rows + row] = __double2float_rn(v) + (p.bias ? __ldg(p.bias + row) : 0.f);
+        }
+    }
+}
+
+// One CTA per (token, K range)
+__global__ void __launch_bounds__(256) tok_digits_kernel(TokX x, int nb, int nst, DigX out, int M) {
+    __shared__ int s_lo, s_hi;
+    __shared__ long long s_sum[8];
+    const int n = blockIdx.x, sp = blockIdx.y, ksg = gridDim.y, tid = threadIdx.x;
+    const int b0 = (int)((long long)sp * nst / ksg) * kStepBlk, b1 = min((int)((long long)(sp + 1) * nst / ksg) * kStepBlk, nb);
+    if (tid == 0) { s_lo = 31; s_hi = 0; }
+    __syncthreads();
+    pdl_launch_dependents(); pdl_wait_prior();
+    auto bits = [&](int b) { return (unsigned)__half_as_ushort(__float2half_rn((float)__dmul_rn(__ldcg(x.d + tok_scale(x.J, b, n)), 0x1p-1004))); };
+    int lo = 31, hi = 0;
+    for (int b = b0 + tid; b < b1; b += 256) {
+        const unsigned h = bits(b);
+        if (h & 0x7FFFu) { lo = min(lo, scale_exponent(h)); hi = max(hi, scale_exponent(h)); }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo); hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((tid & 31) == 0) { atomicMin(&s_lo, lo); atomicMax(&s_hi, hi); }
+    __syncthreads();
+    lo = min(s_lo, max(s_hi, 1)); hi = s_hi;
+    const int need = hi == 31 || hi - lo > 13 ? kDigNone : hi - lo > 5 ? 4 : 3;
+    if (tid == 0) out.info[(size_t)sp * M + n] = lo | need << 8;
+    const int tt = n / out.T, t = n - tt * out.T;
+    long long sum = 0;
+    for (int i = 2 * b0 + tid; i < 2 * b1; i += 256) {
+        const int b = i >> 1, half = i & 1;
+        const unsigned h = bits(b);
+        const int m = need == kDigNone ? 0 : scale_mantissa(h) << ((scale_exponent(h) - lo) & 31);
+        unsigned d[4][4];
+        #pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const unsigned q = __ldcg(x.q + tok_word(x.J, b, n, 16 * half + 4 * k));
+            unsigned v[4];
+            #pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = (unsigned)((int)(int8_t)(q >> (8 * j)) * m) + 0x80808080u;
+            sum += (long long)__dp4a((int)q, 0x01010101, 0) * m;
+            const unsigned a = __byte_perm(v[0], v[1], 0x5140), c = __byte_perm(v[2], v[3], 0x5140);
+            const unsigned e = __byte_perm(v[0], v[1], 0x7362), f = __byte_perm(v[2], v[3], 0x7362);
+            d[0][k] = __byte_perm(a, c, 0x5410) ^ 0x80808080u; d[1][k] = __byte_perm(a, c, 0x7632) ^ 0x80808080u;
+            d[2][k] = __byte_perm(e, f, 0x5410) ^ 0x80808080u; d[3][k] = __byte_perm(e, f, 0x7632) ^ 0x80808080u;
+        }
+        #pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, j, t)) = make_uint4(d[j][0], d[j][1], d[j][2], d[j][3]);
+        if (3 * out.T + t < dig_rows(out.T)) *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, 0, 3 * out.T + t)) = make_uint4(0, 0, 0, 0);     // rows of padding
+    }
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((tid & 31) == 0) s_sum[tid >> 5] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < 8; w++) sum += s_sum[w];
+        out.bias[(size_t)sp * M + n] = sum;
+    }
+}
+
+// One warp per row
+template <int KB>
+__global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base, int groups, int nb, uint8_t* row_exp, int* wide) {
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= groups * 32) return;
+    int lo = 31, hi = 0;
+    for (int b = lane; b < nb; b += 32) {
+        const uint8_t* tile = base + ((size_t)(row >> 5) * nb + b / KB * KB) * kTileRowBytes;
+        const unsigned h = __ldg(reinterpret_cast<const unsigned short*>(tile + KB * 512) + (row & 31) * KB + b % KB);
+        if (h & 0x7FFFu) { lo = min(lo, scale_exponent(h)); hi = max(hi, scale_exponent(h)); }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo); hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane) return;
+    lo = min(lo, max(hi, 1));
+    row_exp[row] = hi == 31 || hi - lo > 16 ? kRowNone : lo;
+    if (row_exp[row] == kRowNone) atomicOr(wide, 2);
+    else if (hi - lo > 8) atomicOr(wide, 1);
+}
+
+template <int KB, int NW, bool PART>
+int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
+    const int units = (p.groups + 3) / 4 * p.x.TT * p.ksg;             // at least
+    auto kern = gemm_dig_kernel<KB, NW, PART>;
+    static std::mutex mu;
+    static std::atomic<unsigned> raised{0};                   // bit per device
+    if (!(raised.load(std::memory_order_acquire) >> (ctx->device & 31) & 1u)) {
+        std::lock_guard<std::mutex> hold(mu);
+        MI_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::bytes));
+        raised.fetch_or(1u << (ctx->device & 31), std::memory_order_release);
+    }
+    MI_CUDA(ctx, launch_k(pdl, kern, dim3((unsigned)std::min(units, ctx->sm_count)), dim3(kThreads), Smem::bytes, ctx->stream, p));
+    return MI_OK;
+}
+template <int KB>
+int launch_kb(mi_ctx* ctx, const DigParams& p, bool wide, bool part, bool pdl) {
+    if (wide) return part ? launch_dig<KB, 4, true>(ctx, p, pdl) : launch_dig<KB, 4, false>(ctx, p, pdl);
+    return part ? launch_dig<KB, 3, true>(ctx, p, pdl) : launch_dig<KB, 3, false>(ctx, p, pdl);
+}
+
+}  // namespace
+
+// Token tiles and K ranges of a product over digits, the fewest clocks by a model from measured launches: 7000 until the first MMA, 290 per block or what its MMAs take,
+// 4000 and 80 per token for the end of a unit; 4000 for the launch that makes the digits.
+bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* out) {
+    const int nst = (w->nb + kStepBlk - 1) / kStepBlk, rt = (w->groups + 3) / 4;
+    const int TT = (M + kDigMaxT - 1) / kDigMaxT, T = ((M + TT - 1) / TT + 7) / 8 * 8;
+    const int nw = w->wide & 1 ? 4 : 3;
+    const double blk = std::max(nw * dig_rows(T) / 2 + 30.0, nw == 3 ? 290.0 : 450.0);
+    double best = 1e300;
+    if (!w->row_exp) return false;
+    for (int ksg = 1; ksg <= (part ? std::min(nst, 8) : 1); ksg++) {
+        const int steps = (nst + ksg - 1) / ksg;
+        if (steps * kStepBlk * 32 > 16384) continue;                   // a sum of digit products stays below 2^31 (four pairs of 255 * 128 per element)
+        const long long units = (long long)rt * TT * ksg, rounds = (units + ctx->sm_count - 1) / ctx->sm_count;
+        const double cost = 11000 + rounds * (std::min(steps * kStepBlk, w->nb) * blk + 4000 + 80.0 * T) + (part ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
+        if (cost < best) { best = cost; *out = DigPlan{T, TT, ksg, cost}; }
+    }
+    return best < 1e300;
+}
+
+int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode, const DigX& x, GemmParams g, bool pdl) {
+    DigParams p{};
+    p.base = w->dev; p.row_exp = w->row_exp; p.groups = w->groups; p.nb = w->nb; p.nst = (w->nb + kStepBlk - 1) / kStepBlk; p.rows = (int)w->rows;
+    p.ksg = pl.ksg; p.M = g.M;
+    p.x = x; p.q8 = g.x; p.bias = g.bias; p.y = g.y; p.part = g.part; p.ldp = g.ldp; p.err = ctx->d_err; p.bad_rows = w->wide & 2;
+    const bool part = mode == GEMM_PART;
+    switch (w->kb) {
+        case 8: return launch_kb<8>(ctx, p, w->wide & 1, part, pdl);
+        case 4: return launch_kb<4>(ctx, p, w->wide & 1, part, pdl);
+        case 2: return launch_kb<2>(ctx, p, w->wide & 1, part, pdl);
+        default: return launch_kb<1>(ctx, p, w->wide & 1, part, pdl);
+    }
+}
+
+int launch_tok_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const TokX& x, const DigX& out, int M, bool pdl) {
+    MI_CUDA(ctx, launch_k(pdl, tok_digits_kernel, dim3(M, pl.ksg), dim3(256), 0, ctx->stream, x, w->nb, (w->nb + kStepBlk - 1) / kStepBlk, out, M));
+    return MI_OK;
+}
+
+int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* wide) {
+    const dim3 grid((unsigned)(w->groups * 4));
+    if (w->groups == 0) return MI_OK;
+    switch (w->kb) {
+        case 8: row_exponents_kernel<8><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
+        case 4: row_exponents_kernel<4><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
+        case 2: row_exponents_kernel<2><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
+        default: row_exponents_kernel<1><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
+    }
+    MI_CUDA(ctx, cudaGetLastError());
+    return MI_OK;
+}
+
+}  // namespace mi

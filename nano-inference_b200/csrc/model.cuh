@@ -1,7 +1,7 @@
 // The loaded model as the decode and the M-token step see it.
 #pragma once
 #include "decode_kernel.cuh"
-#include "gemm_tok.cuh"
+#include "gemm_dig.cuh"
 #include "buffer_set.cuh"
 #include "pass_graphs.cuh"
 
@@ -23,6 +23,7 @@ struct VerifyBufs {
     float* Y = nullptr;                // fp32 rows of the QKV and gate/up products (more than kMaxFusedTok tokens)
     float* q = nullptr;                // [M][NQ] after bias and RoPE, natural order
     TokX xf{}, attf{}, actf{};         // q8_0 of the normed input, the attention output and SwiGLU, in operand order
+    uint8_t* dig = nullptr; int* dig_info = nullptr; long long* dig_bias = nullptr;     // digits of one product's activations (more than kMaxFusedTok tokens)
     float* att = nullptr;              // [M][NQ]
     float* logits = nullptr;           // [M][V]
     int* meta = nullptr; int* h_meta = nullptr;         // tokens | positions | slots, or tokens | first position; its pinned image
@@ -68,6 +69,7 @@ struct mi_model {
     int* d_pos = nullptr;                 // [2]: device-resident position for position-free launch sequences; the tag epoch
     std::vector<mi_weight> views;         // [4L+1] whole matrices in job order (QKV, O, gate/up, down per layer; lm_head), for the M-token step
     std::vector<mi::LayerPtrs> layer_ptrs;    // host copy of the per-layer norm / bias pointers
+    int products = 0;                     // mi_model_debug_products
     mi::VerifyBufs vb;                    // buffers of the M-token step, allocated on first use
 };
 

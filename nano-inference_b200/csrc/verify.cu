@@ -235,7 +235,8 @@ int ensure_bufs(mi_ctx* ctx, mi_model* m, int M, int ML) {
     if ((st = take(&b.X, (size_t)cap * E)) || (st = take(&b.part, (size_t)kMaxRanges * cap * b.ldp)) || (st = take(&b.q, (size_t)cap * NQ)) ||
         (st = take_tok(&b.xf, E, cap)) || (st = take_tok(&b.attf, NQ, cap)) || (st = take_tok(&b.actf, FF, cap)) ||
         (st = take(&b.att, (size_t)cap * NQ)) || (st = take(&b.Y, cap > kMaxFusedTok ? (size_t)cap * std::max(2 * FF, m->qkv_rows) : 0)) || (st = take(&b.logits, (size_t)capl * m->V)) ||
-        (st = take(&b.meta, (size_t)3 * cap + 4)) || (st = take(&b.out, (size_t)cap)) || (st = take(&b.margins, (size_t)cap)) ||
+        (st = take(&b.dig, cap > kMaxFusedTok ? dig_bytes(std::max(std::max(E, NQ), FF) / 32, cap) : 0)) || (st = take(&b.dig_info, (size_t)kMaxRanges * cap)) ||
+        (st = take(&b.dig_bias, (size_t)kMaxRanges * cap)) || (st = take(&b.meta, (size_t)3 * cap + 4)) || (st = take(&b.out, (size_t)cap)) || (st = take(&b.margins, (size_t)cap)) ||
         (st = take(&b.attn_part, attn_part_max(ctx, m->NH, m->NKV, m->HD))) ||
         (st = take(&b.pick, (size_t)capl * kPickSlices * 3)) || (st = take(&b.pick_cnt, (size_t)capl))) {
         cudaStreamSynchronize(ctx->stream);                            // (the fills of those that were made)
@@ -297,8 +298,23 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     TokTiling tiles;
     int st;
     if ((st = plan_pass_products(ctx, mats, L, M, a.head == HEAD_NONE ? 0 : ML, &tiles, plans))) return st;
-    const GemmPlan &pq = plans[0], &po = plans[1], &pg = plans[2], &pd = plans[3], &pl = plans[4];
+    const GemmPlan &po = plans[1], &pd = plans[3];
     xf.J = attf.J = actf.J = tiles.J();
+    // a product goes over digits where that is faster by the cost models, the digits' own launch included
+    DigPlan dp[5];
+    bool dig[5];
+    for (int i = 0; i < 5; i++) {
+        const int Mi = i == 4 ? ML : M;
+        dig[i] = Mi > kMaxFusedTok && m->products >= 0 && plan_gemm_dig(ctx, mats[i], i == 1 || i == 3, Mi, &dp[i]) && (m->products > 0 || dp[i].cost < plans[i].cost);
+    }
+    // one product: digits of its activations and the product over them, or the product over blocks
+    auto product = [&](int i, const mi_weight* w, int mode, const GemmParams& gp) -> int {
+        if (!dig[i]) return launch_gemm_tok(ctx, w, plans[i], mode, false, gp, pdl);
+        const DigX x{b.dig, b.dig_info, b.dig_bias, dp[i].T, dp[i].TT};
+        const int s = launch_tok_digits(ctx, w, dp[i], gp.x, x, gp.M, pdl);
+        return s ? s : launch_gemm_dig(ctx, w, dp[i], mode, x, gp, pdl);
+    };
+    const int o_ranges = dig[1] ? dp[1].ksg : po.ksg, d_ranges = dig[3] ? dp[3].ksg : pd.ksg;
     const int nt_norm = std::min(1024, (E / 4 + 31) / 32 * 32);
     GemmParams g{};
     g.M = M;
@@ -309,28 +325,28 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     };
     for (int l = 0; l < L; l++) {
         const mi_weight *wqkv = &m->views[4 * l], *wo = &m->views[4 * l + 1], *wgu = &m->views[4 * l + 2], *wdn = &m->views[4 * l + 3];
-        if ((st = norm(l == 0, 0, M, l == 0 ? 0 : pd.ksg, lp[l].attn_norm, xf))) return st;
+        if ((st = norm(l == 0, 0, M, l == 0 ? 0 : d_ranges, lp[l].attn_norm, xf))) return st;
         GemmParams gq = g;
         gq.x = xf; gq.bias = lp[l].bqkv; gq.y = b.Y;
         gq.rope = RopeParams{b.q, NQ, m->HD, P.kc, P.vc, m->KVD, a.slab_stride, l, a.max_seq, P.rope_cs, P.rope_freq, P.rope_rows, pos0, pos_arr, slot_arr};
-        if ((st = launch_gemm_tok(ctx, wqkv, pq, fused ? GEMM_QKV : GEMM_PLAIN, false, gq, pdl))) return st;
+        if ((st = product(0, wqkv, fused ? GEMM_QKV : GEMM_PLAIN, gq))) return st;
         if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_rope, dim3(((int)wqkv->rows / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, gq.rope, (const float*)b.Y, (int)wqkv->rows));
         const AttnParams at{b.q, P.kc, P.vc, M, m->NH, m->NKV, m->HD, m->KVD, l, a.max_seq, pos0, 0, pos_arr, slot_arr, a.slab_stride, b.att, attf, b.attn_part, 1, 1, 1};
         if ((st = launch_attn_tok(ctx, at, pa, pdl))) return st;
         GemmParams go = g; go.x = attf; go.part = b.part; go.ldp = b.ldp;
-        if ((st = launch_gemm_tok(ctx, wo, po, GEMM_PART, false, go, pdl))) return st;
-        if ((st = norm(false, 0, M, po.ksg, lp[l].ffn_norm, xf))) return st;
+        if ((st = product(1, wo, GEMM_PART, go))) return st;
+        if ((st = norm(false, 0, M, o_ranges, lp[l].ffn_norm, xf))) return st;
         GemmParams gg = g; gg.x = xf; gg.act = actf; gg.y = b.Y;
-        if ((st = launch_gemm_tok(ctx, wgu, pg, fused ? GEMM_GU : GEMM_PLAIN, false, gg, pdl))) return st;
+        if ((st = product(2, wgu, fused ? GEMM_GU : GEMM_PLAIN, gg))) return st;
         if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_swiglu, dim3((m->FF / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, (const float*)b.Y, m->FF, actf));
         GemmParams gd = g; gd.x = actf; gd.part = b.part; gd.ldp = b.ldp;
-        if ((st = launch_gemm_tok(ctx, wdn, pd, GEMM_PART, false, gd, pdl))) return st;
+        if ((st = product(3, wdn, GEMM_PART, gd))) return st;
     }
     if (a.head == HEAD_NONE) return MI_OK;
     TokX lf = b.xf; lf.J = ML == M ? tiles.J() : tok_tiling(ML).J();
-    if ((st = norm(false, M - ML, ML, pd.ksg, m->P.out_norm, lf))) return st;
+    if ((st = norm(false, M - ML, ML, d_ranges, m->P.out_norm, lf))) return st;
     GemmParams gl = g; gl.M = ML; gl.x = lf; gl.y = b.logits;
-    if ((st = launch_gemm_tok(ctx, &m->views[4 * L], pl, GEMM_PLAIN, false, gl, pdl))) return st;
+    if ((st = product(4, &m->views[4 * L], GEMM_PLAIN, gl))) return st;
     MI_CUDA(ctx, launch_k(pdl, vf_pick, dim3(kPickSlices, ML), dim3(512), 0, ctx->stream, (const float*)b.logits, (long long)V, V, b.out, b.margins, b.pick, b.pick_cnt,
                           m->P.cur_token));
     return MI_OK;
@@ -443,6 +459,15 @@ extern "C" int mi_prefill(mi_ctx* ctx, mi_model* m, const int32_t* tokens_host, 
     if ((st = mi_ctx_sync(ctx))) return st;
     if (next_token_host) *next_token_host = b.h_meta[0];
     if (elapsed_ms) MI_CUDA(ctx, cudaEventElapsedTime(elapsed_ms, m->ev0, m->ev1));
+    return MI_OK;
+}
+
+extern "C" int mi_model_debug_products(mi_ctx* ctx, mi_model* m, int which) {
+    if (!ctx) return MI_ERR_INVALID;
+    if (!m || which < -1 || which > 1) return set_error(ctx, MI_ERR_INVALID, "debug_products: %d", which);
+    MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    m->products = which;
+    m->vb.graphs.drop_graphs(destroy_graph);
     return MI_OK;
 }
 
