@@ -49,7 +49,8 @@ struct DigParams {
 struct Smem {
     static constexpr int raw = 0, x = raw + kRawSlots * 4 * kStepBytes, bars = x + kXSlots * kXBytes;
     static constexpr int n_bars = 2 * kRawSlots + 2 * kXSlots + 2 * kRing + 3;
-    static constexpr int bytes = bars + n_bars * 8 + 16;
+    static constexpr int table = bars + (n_bars * 8 + 31) / 16 * 16;         // 16 bytes per warp and token of its group
+    static constexpr int bytes = table + kExpWarps * (kDigMaxT / kGroups) * 16;
 };
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -115,9 +116,6 @@ __device__ __forceinline__ void expand_block(const uint4& w, int m, unsigned (&d
         }
     }
 }
-
-__device__ __forceinline__ int scale_exponent(unsigned h) { return max((int)(h >> 10 & 31u), 1); }     // of the unit of the fp16's mantissa, in steps from 2^-25
-__device__ __forceinline__ int scale_mantissa(unsigned h) { return (int)(h & 1023u) + ((h & 0x7C00u) ? 1024 : 0); }
 
 // acc + v * f in 64 bits
 __device__ __forceinline__ long long mad_wide(int v, int f, long long acc) {
@@ -209,6 +207,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         for (rt_step = U.k0; rt_step < U.k1 && raw_issued < kRawSlots; rt_step++) raw_issue(U, rt_step);
         if (rt_step >= U.k1) { ru += gridDim.x; rt_step = -1; }
     }
+    auto row_exp_of = [&](const Unit& U) { return (int)__ldg(p.row_exp + min(U.rt * 128 + (warp & 3) * 32 + lane, p.groups * 32 - 1)); };
+    const int first_exp = row_exp_of(unit(blockIdx.x));
     if (warp < kExpWarps) {                                            // all sums start at zero
         #pragma unroll
         for (int c = 0; c < 512 / kGroups; c += 32) tmem_zero32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * (512 / kGroups) + c);
@@ -244,18 +244,34 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty);
         };
+        constexpr int G = kDigMaxT / kGroups;                          // tokens of a group of warps
+        longlong2* table = reinterpret_cast<longlong2*>(smem + Smem::table) + warp * G;          // per token: what its 128s add to a sum, its exponent
         int n_done = 0;
-        auto finish = [&](int u) -> bool {
-            constexpr int G = kDigMaxT / kGroups;                      // tokens of a group of warps
+        // what the end of a unit needs besides its sums, requested when the unit begins
+        struct Ends { int u, ew, info; long long bias; float bv; };
+        auto ends_of = [&](int u, int ew) {
             const Unit U = unit(u);
-            const int ew = __ldg(p.row_exp + min(U.rt * 128 + q * 32 + lane, p.groups * 32 - 1));
+            const int row = U.rt * 128 + q * 32 + lane, n = U.ts * T + wg * G + lane;
+            const bool has = lane < min(T - wg * G, G) && n < p.M;
+            Ends e;
+            e.u = u;
+            e.ew = ew;
+            e.info = has ? __ldcg(p.x.info + (size_t)U.sp * p.M + n) & 255 : 0;
+            e.bias = has ? __ldcg(p.x.bias + (size_t)U.sp * p.M + n) : 0;
+            e.bv = !PART && p.bias && row < p.rows ? __ldg(p.bias + row) : 0.f;
+            return e;
+        };
+        auto finish = [&](const Ends& e) -> bool {
+            const Unit U = unit(e.u);
             const int n0 = U.ts * T + wg * G, tg = min(min(T - wg * G, G), p.M - n0), row = U.rt * 128 + q * 32 + lane;       // tokens n0 .. n0 + tg
-            const int info = lane < tg ? __ldcg(p.x.info + (size_t)U.sp * p.M + n0 + lane) : 0;
-            const long long bias = lane < tg ? __ldcg(p.x.bias + (size_t)U.sp * p.M + n0 + lane) * (NW == 4 ? kBias4 : kBias3) : 0;
-            const float bv = !PART && p.bias && row < p.rows ? __ldg(p.bias + row) : 0.f;
+            if (lane < G) table[lane] = make_longlong2(e.bias * (NW == 4 ? kBias4 : kBias3), (long long)(1023 - 50 + e.info) << 52);
+            __syncwarp();
             if (!wait_or_abort(d_full, n_done & 1, abort_flag)) return false;
             n_done++;
             tc_fence_after();
+            const long long row_scale = (long long)e.ew << 52;
+            float* y = p.y + (size_t)n0 * p.rows + row;
+            double* part = p.part + ((size_t)U.sp * p.M + n0) * p.ldp + row;
             #pragma unroll 1
             for (int g = 0; g < tg; g += 4) {                          // (rolled: four tokens at a time fit the registers and the instruction cache)
                 const uint32_t a = trow + wg * G + g;
@@ -274,14 +290,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 for (int i = 0; i < 4; i++) {                          // the sum itself is below 2^63, whatever its parts are
                     high[i] += (unsigned)d[4][i];
                     if constexpr (NW == 4) high[i] += (unsigned)d[5][i] << 8;
-                    long long v = (long long)((unsigned long long)high[i] << 32) - __shfl_sync(0xffffffffu, bias, g + i);
+                    const longlong2 tok = table[g + i];
+                    long long v = (long long)((unsigned long long)high[i] << 32) - tok.x;
                     v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
-                    const int ex = __shfl_sync(0xffffffffu, info, g + i) & 255;
-                    const double r = __dmul_rn(__ll2double_rn(v), __hiloint2double((1023 - 50 + ew + ex) << 20, 0));
+                    const double r = __dmul_rn(__ll2double_rn(v), __longlong_as_double(tok.y + row_scale));
                     if (g + i < tg && row < p.rows) {
-                        if constexpr (PART) __stcg(p.part + ((size_t)U.sp * p.M + n0 + g + i) * p.ldp + row, r);
-                        else p.y[(size_t)(n0 + g + i) * p.rows + row] = __double2float_rn(r) + bv;
+                        if constexpr (PART) __stcg(part, r);
+                        else *y = __double2float_rn(r) + e.bv;
                     }
+                    if constexpr (PART) part += p.ldp; else y += p.rows;
                 }
             }
             tc_fence_before();
@@ -291,13 +308,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
             return true;
         };
         if (lane == 0) mbar_arrive(d_empty);
-        int s = 0, sc0 = 0, pending = -1;                              // sc0: stages of all units before
+        int s = 0, sc0 = 0;                                            // sc0: stages of all units before
+        Ends now{}, before{};
+        bool pending = false;
         uint32_t raw_phase = 0;
         bool ok = true;
         #pragma unroll 1
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             const Unit U = unit(u);
-            const int ew = __ldg(p.row_exp + min(U.rt * 128 + q * 32 + lane, p.groups * 32 - 1));
+            now = ends_of(u, u == (int)blockIdx.x ? first_exp : row_exp_of(U));
             int sc = sc0 + ((wg - sc0) & (kGroups - 1)), step0 = sc0;
             #pragma unroll 1
             for (int t = U.k0; t < U.k1; t++) {
@@ -307,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 #pragma unroll 1
                 for (; sc < end; sc += kGroups) {
                     // the first stages of a unit fit beside the last ones of the unit before, whose sums are read then: the MMAs that would make room for more wait for it
-                    if (pending >= 0 && sc - sc0 >= slots) { if (!(ok = finish(pending))) break; pending = -1; }
+                    if (pending && sc - sc0 >= slots) { if (!(ok = finish(before))) break; pending = false; }
                     unsigned d[kStage][NW][8];
                     #pragma unroll
                     for (int b = 0; b < kStage; b++) {
@@ -315,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                         const uint8_t* tile = grp + k / KB * (KB * kTileRowBytes);
                         const uint4 w = *reinterpret_cast<const uint4*>(tile + (k % KB * 32 + lane) * 16);
                         const unsigned h = *reinterpret_cast<const unsigned short*>(tile + KB * 512 + (lane * KB + k % KB) * 2);
-                        const int m = scale_mantissa(h) << ((scale_exponent(h) - ew) & 31);
+                        const int m = scale_mantissa(h) << ((scale_exponent(h) - now.ew) & 31);
                         expand_block<NW>(w, h & 0x8000u ? -m : m, d[b]);
                     }
                     // (a ring of eight barriers, whatever the number of slots: a group never falls two phases behind)
@@ -337,10 +356,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 if (++s == kRawSlots) { s = 0; raw_phase ^= 1; }
             }
             sc0 = step0;
-            if (ok && pending >= 0) ok = finish(pending);
-            pending = u;
+            if (ok && pending) ok = finish(before);
+            before = now; pending = true;
         }
-        if (ok && pending >= 0) finish(pending);
+        if (ok && pending) finish(before);
     } else if (warp == wRaw) {
         bool ok = true;
         for (; ru < units && ok; ru += gridDim.x, rt_step = -1) {
@@ -460,56 +479,88 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
 
 // One CTA per (token, K range)
 __global__ void __launch_bounds__(256) tok_digits_kernel(TokX x, int nb, int nst, DigX out, int M) {
-    __shared__ int s_lo, s_hi;
-    __shared__ long long s_sum[8];
+    __shared__ DigReduce red;
     const int n = blockIdx.x, sp = blockIdx.y, ksg = gridDim.y, tid = threadIdx.x;
-    const int b0 = (int)((long long)sp * nst / ksg) * kStepBlk, b1 = min((int)((long long)(sp + 1) * nst / ksg) * kStepBlk, nb);
-    if (tid == 0) { s_lo = 31; s_hi = 0; }
-    __syncthreads();
+    const int b0 = sp * nst / ksg * kStepBlk, b1 = min((sp + 1) * nst / ksg * kStepBlk, nb);
     pdl_launch_dependents(); pdl_wait_prior();
     auto bits = [&](int b) { return (unsigned)__half_as_ushort(__float2half_rn((float)__dmul_rn(__ldcg(x.d + tok_scale(x.J, b, n)), 0x1p-1004))); };
-    int lo = 31, hi = 0;
-    for (int b = b0 + tid; b < b1; b += 256) {
-        const unsigned h = bits(b);
-        if (h & 0x7FFFu) { lo = min(lo, scale_exponent(h)); hi = max(hi, scale_exponent(h)); }
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo); hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((tid & 31) == 0) { atomicMin(&s_lo, lo); atomicMax(&s_hi, hi); }
-    __syncthreads();
-    lo = min(s_lo, max(s_hi, 1)); hi = s_hi;
-    const int need = hi == 31 || hi - lo > 13 ? kDigNone : hi - lo > 5 ? 4 : 3;
-    if (tid == 0) out.info[(size_t)sp * M + n] = lo | need << 8;
-    const int tt = n / out.T, t = n - tt * out.T;
-    long long sum = 0;
+    DigRange mine;
     for (int i = 2 * b0 + tid; i < 2 * b1; i += 256) {
-        const int b = i >> 1, half = i & 1;
-        const unsigned h = bits(b);
-        const int m = need == kDigNone ? 0 : scale_mantissa(h) << ((scale_exponent(h) - lo) & 31);
+        const unsigned h = bits(i >> 1);
+        int sum = 0;
+        #pragma unroll
+        for (int k = 0; k < 4; k++) sum = __dp4a((int)__ldcg(x.q + tok_word(x.J, i >> 1, n, 16 * (i & 1) + 4 * k)), 0x01010101, sum);
+        mine.add(h, sum);
+    }
+    const DigRange all = mine.over_cta(red);
+    const int need = all.planes();
+    if (tid == 0) { out.info[(size_t)sp * M + n] = all.unit() | need << 8; out.bias[(size_t)sp * M + n] = all.total(); }
+    const int tt = n / out.T, t = n - tt * out.T;
+    for (int i = 2 * b0 + tid; i < 2 * b1; i += 256) {
+        const int b = i >> 1, half = i & 1, m = all.factor(bits(b));
         unsigned d[4][4];
         #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const unsigned q = __ldcg(x.q + tok_word(x.J, b, n, 16 * half + 4 * k));
             unsigned v[4];
+            dig_word(__ldcg(x.q + tok_word(x.J, b, n, 16 * half + 4 * k)), m, v);
             #pragma unroll
-            for (int j = 0; j < 4; j++) v[j] = (unsigned)((int)(int8_t)(q >> (8 * j)) * m) + 0x80808080u;
-            sum += (long long)__dp4a((int)q, 0x01010101, 0) * m;
-            const unsigned a = __byte_perm(v[0], v[1], 0x5140), c = __byte_perm(v[2], v[3], 0x5140);
-            const unsigned e = __byte_perm(v[0], v[1], 0x7362), f = __byte_perm(v[2], v[3], 0x7362);
-            d[0][k] = __byte_perm(a, c, 0x5410) ^ 0x80808080u; d[1][k] = __byte_perm(a, c, 0x7632) ^ 0x80808080u;
-            d[2][k] = __byte_perm(e, f, 0x5410) ^ 0x80808080u; d[3][k] = __byte_perm(e, f, 0x7632) ^ 0x80808080u;
+            for (int j = 0; j < 4; j++) d[j][k] = v[j];
         }
         #pragma unroll
         for (int j = 0; j < 4; j++)
             *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, j, t)) = make_uint4(d[j][0], d[j][1], d[j][2], d[j][3]);
         if (3 * out.T + t < dig_rows(out.T)) *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, 0, 3 * out.T + t)) = make_uint4(0, 0, 0, 0);     // rows of padding
     }
-    #pragma unroll
-    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((tid & 31) == 0) s_sum[tid >> 5] = sum;
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < 8; w++) sum += s_sum[w];
-        out.bias[(size_t)sp * M + n] = sum;
+}
+
+// SwiGLU, q8_0 and digits of one token over one K range.  A warp takes every sixteenth block (an element per lane); the blocks wait in shared memory for
+// the range's exponent.
+constexpr int kSwiWarps = 16;
+__global__ void __launch_bounds__(kSwiWarps * 32) swiglu_digits_kernel(const float* y, TokX act, int nb, int nst, DigX out, int M) {
+    __shared__ DigReduce red;
+    extern __shared__ __align__(16) uint8_t smem[];                    // [block] 32 int8, then the scales
+    const int n = blockIdx.x, sp = blockIdx.y, ksg = gridDim.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b0 = sp * nst / ksg * kStepBlk, b1 = min((sp + 1) * nst / ksg * kStepBlk, nb);
+    unsigned* q = reinterpret_cast<unsigned*>(smem);
+    unsigned short* sc = reinterpret_cast<unsigned short*>(smem + (size_t)(b1 - b0) * 32);
+    pdl_launch_dependents(); pdl_wait_prior();
+    const float* row = y + (size_t)n * 64 * nb + lane;
+    DigRange mine;
+    float g = 0.f, u = 0.f;
+    if (b0 + warp < b1) { g = __ldcg(row + (size_t)(b0 + warp) * 64); u = __ldcg(row + (size_t)(b0 + warp) * 64 + 32); }
+    for (int b = b0 + warp; b < b1; b += kSwiWarps) {
+        const float a = swiglu(g, u);
+        if (b + kSwiWarps < b1) { g = __ldcg(row + (size_t)(b + kSwiWarps) * 64); u = __ldcg(row + (size_t)(b + kSwiWarps) * 64 + 32); }
+        const float am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(a))));
+        const float inv = am > 0.f ? __fdiv_rn(127.f, am) : 0.f;
+        const int v = (int)(int8_t)__float2int_rn(__fmul_rn(a, inv));
+        const __half d = __float2half_rn(__fdiv_rn(am, 127.f));
+        unsigned w = (unsigned)v & 0xffu;
+        w |= __shfl_down_sync(0xffffffffu, w, 1) << 8;
+        w |= __shfl_down_sync(0xffffffffu, w, 2) << 16;
+        if ((lane & 3) == 0) { q[(b - b0) * 8 + (lane >> 2)] = w; act.q[tok_word(act.J, b, n, lane)] = w; }
+        const int sum = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0) { sc[b - b0] = __half_as_ushort(d); act.d[tok_scale(act.J, b, n)] = tok_scale_value(d); mine.add(__half_as_ushort(d), sum); }
+    }
+    const DigRange all = mine.over_cta(red);
+    if (tid == 0) { out.info[(size_t)sp * M + n] = all.unit() | all.planes() << 8; out.bias[(size_t)sp * M + n] = all.total(); }
+    const int tt = n / out.T, t = n - tt * out.T;
+    for (int i = tid; i < 2 * (b1 - b0); i += kSwiWarps * 32) {
+        const int b = i >> 1, half = i & 1, m = all.factor(sc[b]);
+        const uint4 w = reinterpret_cast<const uint4*>(q)[i];
+        const unsigned ww[4] = {w.x, w.y, w.z, w.w};
+        unsigned d[4][4];
+        #pragma unroll
+        for (int k = 0; k < 4; k++) {
+            unsigned v[4];
+            dig_word(ww[k], m, v);
+            #pragma unroll
+            for (int j = 0; j < 4; j++) d[j][k] = v[j];
+        }
+        #pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b0 + b, half, j, t)) = make_uint4(d[j][0], d[j][1], d[j][2], d[j][3]);
+        if (3 * out.T + t < dig_rows(out.T)) *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b0 + b, half, 0, 3 * out.T + t)) = make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -555,7 +606,7 @@ int launch_kb(mi_ctx* ctx, const DigParams& p, bool wide, bool part, bool pdl) {
 }  // namespace
 
 // Token tiles and K ranges of a product over digits, the fewest clocks by a model from measured launches: 7000 until the first MMA, 290 per block or what its MMAs take,
-// 4000 and 80 per token for the end of a unit; 4000 for the launch that makes the digits.
+// 4000 and 80 per token for the end of a unit.
 bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* out) {
     const int nst = (w->nb + kStepBlk - 1) / kStepBlk, rt = (w->groups + 3) / 4;
     const int TT = (M + kDigMaxT - 1) / kDigMaxT, T = ((M + TT - 1) / TT + 7) / 8 * 8;
@@ -567,7 +618,7 @@ bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* o
         const int steps = (nst + ksg - 1) / ksg;
         if (steps * kStepBlk * 32 > 16384) continue;                   // a sum of digit products stays below 2^31 (four pairs of 255 * 128 per element)
         const long long units = (long long)rt * TT * ksg, rounds = (units + ctx->sm_count - 1) / ctx->sm_count;
-        const double cost = 11000 + rounds * (std::min(steps * kStepBlk, w->nb) * blk + 4000 + 80.0 * T) + (part ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
+        const double cost = 7000 + rounds * (std::min(steps * kStepBlk, w->nb) * blk + 4000 + 80.0 * T) + (part ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
         if (cost < best) { best = cost; *out = DigPlan{T, TT, ksg, cost}; }
     }
     return best < 1e300;
@@ -589,6 +640,12 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
 
 int launch_tok_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const TokX& x, const DigX& out, int M, bool pdl) {
     MI_CUDA(ctx, launch_k(pdl, tok_digits_kernel, dim3(M, pl.ksg), dim3(256), 0, ctx->stream, x, w->nb, (w->nb + kStepBlk - 1) / kStepBlk, out, M));
+    return MI_OK;
+}
+
+int launch_swiglu_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const float* y, const TokX& act, const DigX& out, int M, bool pdl) {
+    const int nst = (w->nb + kStepBlk - 1) / kStepBlk, blocks = (nst + pl.ksg - 1) / pl.ksg * kStepBlk;        // of a range, at most
+    MI_CUDA(ctx, launch_k(pdl, swiglu_digits_kernel, dim3(M, pl.ksg), dim3(kSwiWarps * 32), (size_t)blocks * 34, ctx->stream, y, act, w->nb, nst, out, M));
     return MI_OK;
 }
 

@@ -35,8 +35,9 @@ constexpr int kMaxRanges = 8;               // K ranges of a split product (plan
 // of X is token blockIdx.x of the output.
 template <int R>
 __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const DecodeParams P, const int* __restrict__ tokens, bool embed, int m0, float* X, const double* part,
-                                                       int ranges, long long range_stride, int ldp, const float* __restrict__ w, TokX out) {
+                                                       int ranges, long long range_stride, int ldp, const float* __restrict__ w, TokX out, DigX dig) {
     __shared__ double red[32];
+    __shared__ DigReduce dred;
     const int E = P.E, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5, mo = blockIdx.x, m = m0 + mo;
     float4 wv[R];
     #pragma unroll
@@ -109,9 +110,12 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const Decod
     for (int o = 16; o; o >>= 1) tot = __dadd_rn(tot, __shfl_xor_sync(0xffffffffu, tot, o));
     const float mean = __double2float_rn(div_known(tot, (double)E, P.inv_e));
     const float scale = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(mean, P.eps)));
+    unsigned q[R], h[R];
+    DigRange mine;
     #pragma unroll
     for (int r = 0; r < R; r++) {
         const int e = (tid + r * blockDim.x) * 4;
+        q[r] = h[r] = 0;
         if (((tid & ~31) + r * (int)blockDim.x) * 4 >= E) break;      // warp-uniform: the folds below are warp-wide
         const float ww[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
         float a = 0.f;
@@ -121,13 +125,30 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const Decod
         a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 2));
         a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 4));
         const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
-        unsigned q = 0;
         #pragma unroll
-        for (int i = 0; i < 4; i++) q |= ((unsigned)__float2int_rn(__fmul_rn(v[r][i], inv)) & 0xffu) << (8 * i);
+        for (int i = 0; i < 4; i++) q[r] |= ((unsigned)__float2int_rn(__fmul_rn(v[r][i], inv)) & 0xffu) << (8 * i);
         if (e < E) {
-            out.q[tok_word(out.J, e >> 5, mo, e & 31)] = q;
-            if ((tid & 7) == 0) out.d[tok_scale(out.J, e >> 5, mo)] = tok_scale_value(__float2half_rn(__fdiv_rn(a, 127.f)));
+            const __half d = __float2half_rn(__fdiv_rn(a, 127.f));
+            out.q[tok_word(out.J, e >> 5, mo, e & 31)] = q[r];
+            if ((tid & 7) == 0) out.d[tok_scale(out.J, e >> 5, mo)] = tok_scale_value(d);
+            h[r] = __half_as_ushort(d);
+            mine.add(h[r], __dp4a((int)q[r], 0x01010101, 0));
         }
+    }
+    if (!dig.q) return;
+    // the digits of a product that takes all of K at once
+    const DigRange all = mine.over_cta(dred);
+    if (tid == 0) { dig.info[mo] = all.unit() | all.planes() << 8; dig.bias[mo] = all.total(); }
+    const int tt = mo / dig.T, t = mo - tt * dig.T;
+    #pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int e = (tid + r * blockDim.x) * 4;
+        if (e >= E) break;
+        unsigned d[4];
+        dig_word(q[r], all.factor(h[r]), d);
+        #pragma unroll
+        for (int j = 0; j < 4; j++) *reinterpret_cast<unsigned*>(dig.q + dig_offset(dig, E / 32, tt, e >> 5, e >> 4 & 1, j, t) + (e & 15)) = d[j];
+        if (3 * dig.T + t < dig_rows(dig.T)) *reinterpret_cast<unsigned*>(dig.q + dig_offset(dig, E / 32, tt, e >> 5, e >> 4 & 1, 0, 3 * dig.T + t) + (e & 15)) = 0;      // rows of padding
     }
 }
 
@@ -300,32 +321,32 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     if ((st = plan_pass_products(ctx, mats, L, M, a.head == HEAD_NONE ? 0 : ML, &tiles, plans))) return st;
     const GemmPlan &po = plans[1], &pd = plans[3];
     xf.J = attf.J = actf.J = tiles.J();
-    // a product goes over digits where that is faster by the cost models, the digits' own launch included
+    // a product goes over digits where that is faster by the cost models (for the attention's output their own launch included: 4000 clocks)
     DigPlan dp[5];
     bool dig[5];
     for (int i = 0; i < 5; i++) {
         const int Mi = i == 4 ? ML : M;
-        dig[i] = Mi > kMaxFusedTok && m->products >= 0 && plan_gemm_dig(ctx, mats[i], i == 1 || i == 3, Mi, &dp[i]) && (m->products > 0 || dp[i].cost < plans[i].cost);
+        dig[i] = Mi > kMaxFusedTok && m->products >= 0 && plan_gemm_dig(ctx, mats[i], i == 1 || i == 3, Mi, &dp[i]) && (m->products > 0 || dp[i].cost + (i == 1 ? 4000 : 0) < plans[i].cost);
     }
-    // one product: digits of its activations and the product over them, or the product over blocks
+    auto digits_for = [&](int i) { return dig[i] ? DigX{b.dig, b.dig_info, b.dig_bias, dp[i].T, dp[i].TT} : DigX{nullptr, nullptr, nullptr, 1, 1}; };
+    // The product over digits has them from the kernel that makes its activations, but for the attention's output.
     auto product = [&](int i, const mi_weight* w, int mode, const GemmParams& gp) -> int {
         if (!dig[i]) return launch_gemm_tok(ctx, w, plans[i], mode, false, gp, pdl);
-        const DigX x{b.dig, b.dig_info, b.dig_bias, dp[i].T, dp[i].TT};
-        const int s = launch_tok_digits(ctx, w, dp[i], gp.x, x, gp.M, pdl);
-        return s ? s : launch_gemm_dig(ctx, w, dp[i], mode, x, gp, pdl);
+        if (i == 1) { const int s = launch_tok_digits(ctx, w, dp[i], gp.x, digits_for(i), gp.M, pdl); if (s) return s; }
+        return launch_gemm_dig(ctx, w, dp[i], mode, digits_for(i), gp, pdl);
     };
     const int o_ranges = dig[1] ? dp[1].ksg : po.ksg, d_ranges = dig[3] ? dp[3].ksg : pd.ksg;
     const int nt_norm = std::min(1024, (E / 4 + 31) / 32 * 32);
     GemmParams g{};
     g.M = M;
-    auto norm = [&](bool embed, int m0, int count, int ranges, const float* w, const TokX& out) -> int {
+    auto norm = [&](bool embed, int m0, int count, int ranges, const float* w, const TokX& out, const DigX& x) -> int {
         MI_CUDA(ctx, launch_k(pdl, E <= 2048 ? vf_norm_quant<1> : vf_norm_quant<2>, dim3(count), dim3(nt_norm), 0, ctx->stream, P, tokens, embed, m0, b.X, (const double*)(ranges ? b.part : nullptr), ranges,
-                              (long long)M * b.ldp, b.ldp, w, out));
+                              (long long)M * b.ldp, b.ldp, w, out, x));
         return MI_OK;
     };
     for (int l = 0; l < L; l++) {
         const mi_weight *wqkv = &m->views[4 * l], *wo = &m->views[4 * l + 1], *wgu = &m->views[4 * l + 2], *wdn = &m->views[4 * l + 3];
-        if ((st = norm(l == 0, 0, M, l == 0 ? 0 : d_ranges, lp[l].attn_norm, xf))) return st;
+        if ((st = norm(l == 0, 0, M, l == 0 ? 0 : d_ranges, lp[l].attn_norm, xf, digits_for(0)))) return st;
         GemmParams gq = g;
         gq.x = xf; gq.bias = lp[l].bqkv; gq.y = b.Y;
         gq.rope = RopeParams{b.q, NQ, m->HD, P.kc, P.vc, m->KVD, a.slab_stride, l, a.max_seq, P.rope_cs, P.rope_freq, P.rope_rows, pos0, pos_arr, slot_arr};
@@ -335,16 +356,17 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         if ((st = launch_attn_tok(ctx, at, pa, pdl))) return st;
         GemmParams go = g; go.x = attf; go.part = b.part; go.ldp = b.ldp;
         if ((st = product(1, wo, GEMM_PART, go))) return st;
-        if ((st = norm(false, 0, M, o_ranges, lp[l].ffn_norm, xf))) return st;
+        if ((st = norm(false, 0, M, o_ranges, lp[l].ffn_norm, xf, digits_for(2)))) return st;
         GemmParams gg = g; gg.x = xf; gg.act = actf; gg.y = b.Y;
         if ((st = product(2, wgu, fused ? GEMM_GU : GEMM_PLAIN, gg))) return st;
-        if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_swiglu, dim3((m->FF / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, (const float*)b.Y, m->FF, actf));
+        if (dig[3]) { if ((st = launch_swiglu_digits(ctx, wdn, dp[3], b.Y, actf, digits_for(3), M, pdl))) return st; }
+        else if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_swiglu, dim3((m->FF / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, (const float*)b.Y, m->FF, actf));
         GemmParams gd = g; gd.x = actf; gd.part = b.part; gd.ldp = b.ldp;
         if ((st = product(3, wdn, GEMM_PART, gd))) return st;
     }
     if (a.head == HEAD_NONE) return MI_OK;
     TokX lf = b.xf; lf.J = ML == M ? tiles.J() : tok_tiling(ML).J();
-    if ((st = norm(false, M - ML, ML, d_ranges, m->P.out_norm, lf))) return st;
+    if ((st = norm(false, M - ML, ML, d_ranges, m->P.out_norm, lf, digits_for(4)))) return st;
     GemmParams gl = g; gl.M = ML; gl.x = lf; gl.y = b.logits;
     if ((st = product(4, &m->views[4 * L], GEMM_PLAIN, gl))) return st;
     MI_CUDA(ctx, launch_k(pdl, vf_pick, dim3(kPickSlices, ML), dim3(512), 0, ctx->stream, (const float*)b.logits, (long long)V, V, b.out, b.margins, b.pick, b.pick_cnt,
