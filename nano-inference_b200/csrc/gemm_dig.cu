@@ -67,7 +67,18 @@ __device__ __forceinline__ void tmem_zero32(uint32_t a) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};"
                  ::"r"(a), "r"(0) : "memory");
 }
-__device__ __forceinline__ void group_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kExpWarps * 32) : "memory"); }     // all warps that read and clear sums
+// The values exist here (the compiler would compute them behind the wait that follows).
+template <int NW>
+__device__ __forceinline__ void keep(unsigned (&d)[2][NW][8]) {
+    #pragma unroll
+    for (int b = 0; b < 2; b++)
+        #pragma unroll
+        for (int j = 0; j < NW; j++)
+            asm volatile("" : "+r"(d[b][j][0]), "+r"(d[b][j][1]), "+r"(d[b][j][2]), "+r"(d[b][j][3]), "+r"(d[b][j][4]), "+r"(d[b][j][5]), "+r"(d[b][j][6]), "+r"(d[b][j][7]));
+}
+__device__ __forceinline__ void tmem_zero4(uint32_t a) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%1,%1};" ::"r"(a), "r"(0) : "memory");
+}
 __device__ __forceinline__ void tmem_ld4(uint32_t a, int (&v)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
 }
@@ -229,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
     const int T = p.x.T, units = p.ksg * row_tiles * p.x.TT, N = planes == 4 ? 4 * T : dig_rows(T);
     // tensor memory: sums of weight 256^s in columns s * T .. (the MMAs of a token tile of an odd number of eights reach eight columns further), stages of weight
     // digits at the end
-    const int ns = NW + planes - 1, fit = (512 - (NW - 1) * T - N) / (kStage * NW * 8), slots = fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
+    const int fit = (512 - (NW - 1) * T - N) / (kStage * NW * 8), slots = fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
     const uint32_t a_base = tmem + 512 - slots * (kStage * NW * 8);
 
     if (warp < kExpWarps) {
@@ -237,13 +248,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         // stage); and the sums of a unit -> results, while the next unit is under way
         const int q = warp & 3, wg = warp >> 2;
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16), a_row = a_base + ((uint32_t)(q * 32) << 16);
-        auto clear_sums = [&]() {                                      // 32 columns per store
-            for (int c = wg * 32; c < ns * T; c += kGroups * 32) tmem_zero32(trow + min(c, ns * T - 32));
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(d_empty);
-        };
         constexpr int G = kDigMaxT / kGroups;                          // tokens of a group of warps
         longlong2* table = reinterpret_cast<longlong2*>(smem + Smem::table) + warp * G;          // per token: what its 128s add to a sum, its exponent
         int n_done = 0;
@@ -256,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
             Ends e;
             e.u = u;
             e.ew = ew;
-            e.info = has ? __ldcg(p.x.info + (size_t)U.sp * p.M + n) & 255 : 0;
+            e.info = has ? __ldcg(p.x.info + (size_t)U.sp * p.M + n) : 0;
             e.bias = has ? __ldcg(p.x.bias + (size_t)U.sp * p.M + n) : 0;
             e.bv = !PART && p.bias && row < p.rows ? __ldg(p.bias + row) : 0.f;
             return e;
@@ -264,16 +268,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         auto finish = [&](const Ends& e) -> bool {
             const Unit U = unit(e.u);
             const int n0 = U.ts * T + wg * G, tg = min(min(T - wg * G, G), p.M - n0), row = U.rt * 128 + q * 32 + lane;       // tokens n0 .. n0 + tg
-            if (lane < G) table[lane] = make_longlong2(e.bias * (NW == 4 ? kBias4 : kBias3), (long long)(1023 - 50 + e.info) << 52);
+            if (lane < G) table[lane] = make_longlong2(e.bias * (NW == 4 ? kBias4 : kBias3), PART ? (1023 - 50 + (e.info & 255)) << 20 : (127 - 50 + (e.info & 255)) << 23);
             __syncwarp();
             if (!wait_or_abort(d_full, n_done & 1, abort_flag)) return false;
             n_done++;
             tc_fence_after();
-            const long long row_scale = (long long)e.ew << 52;
             float* y = p.y + (size_t)n0 * p.rows + row;
             double* part = p.part + ((size_t)U.sp * p.M + n0) * p.ldp + row;
             #pragma unroll 1
-            for (int g = 0; g < tg; g += 4) {                          // (rolled: four tokens at a time fit the registers and the instruction cache)
+            for (int g = 0; g < min(T - wg * G, G); g += 4) {                          // (rolled: four tokens at a time fit the registers and the instruction cache)
                 const uint32_t a = trow + wg * G + g;
                 int d[NW + 2][4];
                 unsigned high[4] = {0, 0, 0, 0};
@@ -287,36 +290,41 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 for (int i = 0; i < NW + 2; i++) tmem_ld4(a + i * T, d[i]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 #pragma unroll
+                for (int i = 0; i < NW + 2; i++) tmem_zero4(a + i * T);      // for the next unit
+                if (planes == 4) tmem_zero4(a + (NW + 2) * T);
+                #pragma unroll
                 for (int i = 0; i < 4; i++) {                          // the sum itself is below 2^63, whatever its parts are
                     high[i] += (unsigned)d[4][i];
                     if constexpr (NW == 4) high[i] += (unsigned)d[5][i] << 8;
                     const longlong2 tok = table[g + i];
                     long long v = (long long)((unsigned long long)high[i] << 32) - tok.x;
                     v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
-                    const double r = __dmul_rn(__ll2double_rn(v), __longlong_as_double(tok.y + row_scale));
                     if (g + i < tg && row < p.rows) {
-                        if constexpr (PART) __stcg(part, r);
-                        else *y = __double2float_rn(r) + e.bv;
+                        if constexpr (PART) __stcg(part, __dmul_rn(__ll2double_rn(v), __hiloint2double((int)tok.y + (e.ew << 20), 0)));
+                        // (times a power of two that leaves the result a normal number: the one rounding is the conversion's)
+                        else *y = __fmul_rn(__ll2float_rn(v), __int_as_float((int)tok.y + (e.ew << 23))) + e.bv;
                     }
                     if constexpr (PART) part += p.ldp; else y += p.rows;
                 }
             }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
-            group_barrier();                                           // (columns are cleared by other warps than read them)
-            tc_fence_after();
-            clear_sums();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(d_empty);
             return true;
         };
         if (lane == 0) mbar_arrive(d_empty);
         int s = 0, sc0 = 0;                                            // sc0: stages of all units before
         Ends now{}, before{};
+        int next_exp = first_exp;
         bool pending = false;
         uint32_t raw_phase = 0;
         bool ok = true;
         #pragma unroll 1
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             const Unit U = unit(u);
-            now = ends_of(u, u == (int)blockIdx.x ? first_exp : row_exp_of(U));
+            now = ends_of(u, next_exp);
+            if (u + (int)gridDim.x < units) next_exp = row_exp_of(unit(u + gridDim.x));        // (its latency is not for the next unit's first block)
             int sc = sc0 + ((wg - sc0) & (kGroups - 1)), step0 = sc0;
             #pragma unroll 1
             for (int t = U.k0; t < U.k1; t++) {
@@ -325,8 +333,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 const uint8_t* grp = raw + ((size_t)s * 4 + q) * kStepBytes;
                 #pragma unroll 1
                 for (; sc < end; sc += kGroups) {
-                    // the first stages of a unit fit beside the last ones of the unit before, whose sums are read then: the MMAs that would make room for more wait for it
-                    if (pending && sc - sc0 >= slots) { if (!(ok = finish(before))) break; pending = false; }
+                    // the first stage of a unit goes beside the last ones of the unit before, whose sums are read then (later stages would wait for its last MMAs)
+                    if (pending && sc > sc0) { if (!(ok = finish(before))) break; pending = false; }
                     unsigned d[kStage][NW][8];
                     #pragma unroll
                     for (int b = 0; b < kStage; b++) {
@@ -337,6 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                         const int m = scale_mantissa(h) << ((scale_exponent(h) - now.ew) & 31);
                         expand_block<NW>(w, h & 0x8000u ? -m : m, d[b]);
                     }
+                    keep(d);
                     // (a ring of eight barriers, whatever the number of slots: a group never falls two phases behind)
                     if (sc >= slots && !(ok = wait_or_abort(&empty[(sc - slots) % kRing], ((sc - slots) / kRing) & 1, abort_flag))) break;
                     tc_fence_after();
@@ -402,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         uint32_t elected;
         asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
-        auto mma = [&](uint32_t a, uint32_t x) {                       // one block
+        auto mma = [&](uint32_t a, uint32_t x) {
             const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | ((uint64_t)N << 16) | ((uint64_t)8 << 32) | (1ull << 46);
             #pragma unroll
             for (int i = 0; i < NW; i++)
@@ -411,35 +420,56 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                     "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
                     ::"r"(tmem + (uint32_t)(i * T)), "r"(a + 8 * i), "l"(db), "r"(idesc) : "memory");
         };
+        // the same; returns whether two barriers' phases are over, asked before the MMAs are issued and answered behind them (a wait for a barrier that is through
+        // already keeps the warp for 110 clocks)
+        auto mma_and_test = [&](uint32_t a, uint32_t x, uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1) -> uint32_t {
+            const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | ((uint64_t)N << 16) | ((uint64_t)8 << 32) | (1ull << 46);
+            uint32_t r;
+            if constexpr (NW == 3)
+                asm volatile(
+                    "{\n\t.reg .pred p, t, u;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+                    "mbarrier.test_wait.parity.shared::cta.b64 t, [%9], %10;\n\t"
+                    "mbarrier.test_wait.parity.shared::cta.b64 u, [%11], %12;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::i8 [%1], [%4], %7, %8, p;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::i8 [%2], [%5], %7, %8, p;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::i8 [%3], [%6], %7, %8, p;\n\t"
+                    "and.pred t, t, u;\n\tselp.u32 %0, 1, 0, t;\n\t}"
+                    : "=r"(r) : "r"(tmem), "r"(tmem + (uint32_t)T), "r"(tmem + (uint32_t)(2 * T)), "r"(a), "r"(a + 8), "r"(a + 16), "l"(db), "r"(idesc),
+                      "r"(bar0), "r"(par0), "r"(bar1), "r"(par1) : "memory");
+            else { mma(a, x); r = 0; }
+            return r;
+        };
         int n_done = 0, sc = 0, xslot = 0;
         uint32_t x_phase = 0;
         bool ok = true;
+        uint32_t ready = 0;                                            // the next stage's operands were seen
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x, n_done++) {
             const Unit U = unit(u);
             const int b1 = min(U.k1 * kStepBlk, p.nb);
             if (!wait_or_abort(d_empty, n_done & 1, abort_flag)) { ok = false; break; }
             #pragma unroll 1
-            for (int b = U.k0 * kStepBlk; b < b1; b += kXStage) {
-                if (!wait_or_abort(&x_full[xslot], x_phase, abort_flag)) { ok = false; break; }
-                #pragma unroll
-                for (int g = 0; g < kXStage / kStage; g++) {
-                    const int left = b1 - b - g * kStage;
-                    if (left <= 0) break;
-                    if (!wait_or_abort(&full[sc % kRing], (sc / kRing) & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a = a_base + (sc & (slots - 1)) * (kStage * NW * 8), x = smem_u32(xs) + xslot * kXBytes + g * kStage * N * 32;
-                    if (left >= kStage) {
-                        if (elected) { mma(a, x); mma(a + NW * 8, x + N * 32); tc_commit(&empty[sc % kRing]); }
-                    } else {
-                        if (elected) { mma(a, x); tc_commit(&empty[sc % kRing]); }
+            for (int b = U.k0 * kStepBlk, g = 0; b < b1; b += kStage, g ^= 1) {
+                if (!__any_sync(0xffffffffu, ready != 0) &&
+                    ((g == 0 && !wait_or_abort(&x_full[xslot], x_phase, abort_flag)) || !wait_or_abort(&full[sc % kRing], (sc / kRing) & 1, abort_flag))) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t a = a_base + (sc & (slots - 1)) * (kStage * NW * 8), x = smem_u32(xs) + xslot * kXBytes + g * kStage * N * 32;
+                const bool last = b + kStage >= b1, turn = g == 1 || last;                    // turn: the next stage begins another copy of activations
+                const int ns = sc + 1, nx = turn ? (xslot + 1 == kXSlots ? 0 : xslot + 1) : xslot;
+                const uint32_t np = turn && nx == 0 ? x_phase ^ 1 : x_phase;
+                ready = 0;
+                if (b + kStage <= b1) {
+                    if (elected) {
+                        mma(a, x);
+                        ready = mma_and_test(a + NW * 8, x + N * 32, smem_u32(&full[ns % kRing]), (ns / kRing) & 1, smem_u32(turn ? &x_full[nx] : &full[ns % kRing]), turn ? np : (ns / kRing) & 1);
+                        tc_commit(&empty[sc % kRing]);
+                        if (turn) tc_commit(&x_empty[xslot]);
                     }
-                    __syncwarp();
-                    sc++;
+                } else {
+                    if (elected) { mma(a, x); tc_commit(&empty[sc % kRing]); tc_commit(&x_empty[xslot]); }
                 }
-                if (!ok) break;
-                if (elected) tc_commit(&x_empty[xslot]);
                 __syncwarp();
-                if (++xslot == kXSlots) { xslot = 0; x_phase ^= 1; }
+                sc = ns; xslot = nx; x_phase = np;
+                if (last) break;
             }
             if (ok && elected) tc_commit(d_full);
             __syncwarp();
