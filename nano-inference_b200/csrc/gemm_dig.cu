@@ -50,7 +50,7 @@ struct Smem {
     static constexpr int raw = 0, x = raw + kRawSlots * 4 * kStepBytes, bars = x + kXSlots * kXBytes;
     static constexpr int n_bars = 2 * kRawSlots + 2 * kXSlots + 2 * kRing + 3;
     static constexpr int table = bars + (n_bars * 8 + 31) / 16 * 16;         // 16 bytes per warp and token of its group
-    static constexpr int bytes = table + kExpWarps * (kDigMaxT / kGroups) * 16;
+    static constexpr int bytes = table + kExpWarps * (kDigMaxT / kGroups) * 16 + 256;
 };
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -155,7 +155,8 @@ static __device__ __noinline__ double row_sum_dig(const DigParams& p, int row, i
 
 template <int KB, int NW, bool PART>
 __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_constant__ DigParams p) {
-    extern __shared__ __align__(128) uint8_t smem[];
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + (0u - smem_u32(smem_raw) & 255u);          // the swizzle goes by address bits
     uint8_t* raw = smem + Smem::raw;
     uint8_t* xs = smem + Smem::x;
     uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + Smem::bars);
@@ -394,9 +395,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 __syncwarp();
                 if (planes == 3) {
                     if (lane == 0) bulk_g2s(dst, p.x.q + dig_offset(p.x, p.nb, U.ts, b, 0, 0, 0), nblk * N * 32, &x_full[slot]);
-                } else if (lane < 4 * nblk) {
-                    const int k = lane >> 2, half = lane >> 1 & 1, j = (lane & 1) * 3;
-                    bulk_g2s(dst + ((k * 2 + half) * N + j * T) * 16, p.x.q + dig_offset(p.x, p.nb, U.ts, b + k, half, j, 0), (j ? 1 : 3) * T * 16, &x_full[slot]);
+                } else if (lane < 2 * nblk) {
+                    const int k = lane >> 1, j = (lane & 1) * 3;
+                    bulk_g2s(dst + (k * N + j * T) * 32, p.x.q + dig_offset(p.x, p.nb, U.ts, b + k, 0, j, 0), (j ? 1 : 3) * T * 32, &x_full[slot]);
                 }
                 __syncwarp();
                 if (++slot == kXSlots) { slot = 0; phase ^= 1; }
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         uint32_t elected;
         asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
         auto mma = [&](uint32_t a, uint32_t x) {
-            const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | ((uint64_t)N << 16) | ((uint64_t)8 << 32) | (1ull << 46);
+            const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)16 << 32) | (1ull << 46) | (6ull << 61);       // eight rows of 32 bytes, 32-byte swizzle
             #pragma unroll
             for (int i = 0; i < NW; i++)
                 asm volatile(
@@ -423,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         // the same; returns whether two barriers' phases are over, asked before the MMAs are issued and answered behind them (a wait for a barrier that is through
         // already keeps the warp for 110 clocks)
         auto mma_and_test = [&](uint32_t a, uint32_t x, uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1) -> uint32_t {
-            const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | ((uint64_t)N << 16) | ((uint64_t)8 << 32) | (1ull << 46);
+            const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)16 << 32) | (1ull << 46) | (6ull << 61);       // eight rows of 32 bytes, 32-byte swizzle
             uint32_t r;
             if constexpr (NW == 3)
                 asm volatile(
@@ -507,6 +508,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
     }
 }
 
+// the digits of 16 elements, all planes
+__device__ __forceinline__ void dig_store(const DigX& out, int nb, int tt, int b, int half, int t, const unsigned (&q)[4], int m) {
+    unsigned d[4][4];
+    #pragma unroll
+    for (int k = 0; k < 4; k++) {
+        unsigned v[4];
+        dig_word(q[k], m, v);
+        #pragma unroll
+        for (int j = 0; j < 4; j++) d[j][k] = v[j];
+    }
+    #pragma unroll
+    for (int j = 0; j < 4; j++)
+        *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, j, t)) = make_uint4(d[j][0], d[j][1], d[j][2], d[j][3]);
+    if (3 * out.T + t < dig_rows(out.T))                              // rows of padding
+        *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, 0, 3 * out.T + t)) = make_uint4(0, 0, 0, 0);
+}
+
 // One CTA per (token, K range)
 __global__ void __launch_bounds__(256) tok_digits_kernel(TokX x, int nb, int nst, DigX out, int M) {
     __shared__ DigReduce red;
@@ -526,20 +544,12 @@ __global__ void __launch_bounds__(256) tok_digits_kernel(TokX x, int nb, int nst
     const int need = all.planes();
     if (tid == 0) { out.info[(size_t)sp * M + n] = all.unit() | need << 8; out.bias[(size_t)sp * M + n] = all.total(); }
     const int tt = n / out.T, t = n - tt * out.T;
-    for (int i = 2 * b0 + tid; i < 2 * b1; i += 256) {
+    for (int i = 2 * b0 + tid; i < 2 * b1; i += 256) {               // two threads have a block's halves, a sector together
         const int b = i >> 1, half = i & 1, m = all.factor(bits(b));
-        unsigned d[4][4];
+        unsigned q[4];
         #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            unsigned v[4];
-            dig_word(__ldcg(x.q + tok_word(x.J, b, n, 16 * half + 4 * k)), m, v);
-            #pragma unroll
-            for (int j = 0; j < 4; j++) d[j][k] = v[j];
-        }
-        #pragma unroll
-        for (int j = 0; j < 4; j++)
-            *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, j, t)) = make_uint4(d[j][0], d[j][1], d[j][2], d[j][3]);
-        if (3 * out.T + t < dig_rows(out.T)) *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b, half, 0, 3 * out.T + t)) = make_uint4(0, 0, 0, 0);     // rows of padding
+        for (int k = 0; k < 4; k++) q[k] = __ldcg(x.q + tok_word(x.J, b, n, 16 * half + 4 * k));
+        dig_store(out, nb, tt, b, half, t, q, m);
     }
 }
 
@@ -579,18 +589,7 @@ __global__ void __launch_bounds__(kSwiWarps * 32) swiglu_digits_kernel(const flo
         const int b = i >> 1, half = i & 1, m = all.factor(sc[b]);
         const uint4 w = reinterpret_cast<const uint4*>(q)[i];
         const unsigned ww[4] = {w.x, w.y, w.z, w.w};
-        unsigned d[4][4];
-        #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            unsigned v[4];
-            dig_word(ww[k], m, v);
-            #pragma unroll
-            for (int j = 0; j < 4; j++) d[j][k] = v[j];
-        }
-        #pragma unroll
-        for (int j = 0; j < 4; j++)
-            *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b0 + b, half, j, t)) = make_uint4(d[j][0], d[j][1], d[j][2], d[j][3]);
-        if (3 * out.T + t < dig_rows(out.T)) *reinterpret_cast<uint4*>(out.q + dig_offset(out, nb, tt, b0 + b, half, 0, 3 * out.T + t)) = make_uint4(0, 0, 0, 0);
+        dig_store(out, nb, tt, b0 + b, half, t, ww, m);
     }
 }
 

@@ -6,16 +6,18 @@ namespace mi {
 
 // Activations as digits.  A token's element is xq * dx with dx an fp16 scale: an integer X = xq * (dx / 2^ex) times 2^ex, with ex the
 // smallest exponent among the blocks of one K range, cut into four balanced base-256 digits (planes).
-//     q    : [token tile of T][block of 32][half of 16 elements][row = plane * T + token, planes 0 .. 2, padded to a multiple of 16 rows] 16 bytes: the MMA's operand;
-//            behind all of it plane 3 as [token tile][block][half][token]
+//     q    : [token tile of T][block of 32][row = plane * T + token, planes 0 .. 2, padded to a multiple of 16 rows] 32 bytes: the MMA's operand with the
+//            32-byte swizzle (the halves of rows 4 .. 7 of eight change places); behind all of it plane 3 as [token tile][block][token].  A token's block is a
+//            whole sector: without the swizzle it is two halves of sectors, which it took SwiGLU 31 us to write for 333 tokens of the 1.5B shape.
 //     info : [K range][token] ex | planes in use << 8 (3 or 4; kDigNone: the digits cannot hold it, see row_sum_dig)
 //     bias : [K range][token] sum of X
 struct DigX { uint8_t* q; int* info; long long* bias; int T, TT; };
 constexpr int kDigPlanes = 4, kDigNone = 255, kDigMaxT = 64;                          // tokens of a tile
 __host__ __device__ inline int dig_rows(int T) { return (3 * T + 15) / 16 * 16; }
+// where 16 elements (half 0 or 1 of a block) of a token of a tile are
 __host__ __device__ inline size_t dig_offset(const DigX& x, int nb, int tt, int b, int half, int plane, int t) {
-    const size_t at = ((size_t)tt * nb + b) * 2 + half;
-    return plane < 3 ? (at * dig_rows(x.T) + plane * x.T + t) * 16 : ((size_t)x.TT * nb * 2 * dig_rows(x.T) + at * x.T + t) * 16;
+    const size_t at = (size_t)tt * nb + b, row = plane < 3 ? at * dig_rows(x.T) + plane * x.T + t : (size_t)x.TT * nb * dig_rows(x.T) + at * x.T + t;
+    return row * 32 + (half ^ (t >> 2 & 1)) * 16;
 }
 inline size_t dig_bytes(int nb, int tokens) { return (size_t)nb * 2 * 16 * (4 * (tokens + kDigMaxT) + 8 * (tokens / kDigMaxT + 1)); }   // room for any tiling of so many tokens
 #ifdef __CUDACC__
