@@ -32,12 +32,12 @@ constexpr int kMaxRanges = 8;               // K ranges of a split product (plan
 // x = (embedding row | X) (+ the projection's sum over its K ranges, rounded to fp32 once), committed to X;
 // q8_0(rmsnorm(x) * w) (src/cpu_infer.cpp:40-46) in operand order.  One CTA per token, four consecutive elements per
 // thread: every load of a thread is requested before the first is used, a block of 32 is eight threads.  Token m0 + blockIdx.x
-// of X is token blockIdx.x of the output.
-template <int R>
+// of X is token blockIdx.x of the output.  DIG: the digits of a product that takes all of K at once as well; a form of its own, because passes of few
+// tokens pay for that code without running it (5 tokens of the 1.5B shape at 2000 positions 1161 us per pass with it, 1132 before it; 16 sequences of the 3B shape 2094 / 2074).
+template <int R, bool DIG>
 __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const DecodeParams P, const int* __restrict__ tokens, bool embed, int m0, float* X, const double* part,
                                                        int ranges, long long range_stride, int ldp, const float* __restrict__ w, TokX out, DigX dig) {
     __shared__ double red[32];
-    __shared__ DigReduce dred;
     const int E = P.E, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5, mo = blockIdx.x, m = m0 + mo;
     float4 wv[R];
     #pragma unroll
@@ -110,12 +110,12 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const Decod
     for (int o = 16; o; o >>= 1) tot = __dadd_rn(tot, __shfl_xor_sync(0xffffffffu, tot, o));
     const float mean = __double2float_rn(div_known(tot, (double)E, P.inv_e));
     const float scale = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(mean, P.eps)));
-    unsigned q[R], h[R];
-    DigRange mine;
+    [[maybe_unused]] unsigned q[R], h[R];
+    [[maybe_unused]] DigRange mine;
     #pragma unroll
     for (int r = 0; r < R; r++) {
         const int e = (tid + r * blockDim.x) * 4;
-        q[r] = h[r] = 0;
+        if constexpr (DIG) q[r] = h[r] = 0;
         if (((tid & ~31) + r * (int)blockDim.x) * 4 >= E) break;      // warp-uniform: the folds below are warp-wide
         const float ww[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
         float a = 0.f;
@@ -125,18 +125,22 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const Decod
         a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 2));
         a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 4));
         const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
+        unsigned qw = 0;
         #pragma unroll
-        for (int i = 0; i < 4; i++) q[r] |= ((unsigned)__float2int_rn(__fmul_rn(v[r][i], inv)) & 0xffu) << (8 * i);
+        for (int i = 0; i < 4; i++) qw |= ((unsigned)__float2int_rn(__fmul_rn(v[r][i], inv)) & 0xffu) << (8 * i);
         if (e < E) {
-            const __half d = __float2half_rn(__fdiv_rn(a, 127.f));
-            out.q[tok_word(out.J, e >> 5, mo, e & 31)] = q[r];
-            if ((tid & 7) == 0) out.d[tok_scale(out.J, e >> 5, mo)] = tok_scale_value(d);
-            h[r] = __half_as_ushort(d);
-            mine.add(h[r], __dp4a((int)q[r], 0x01010101, 0));
+            out.q[tok_word(out.J, e >> 5, mo, e & 31)] = qw;
+            if constexpr (DIG) {
+                const __half d = __float2half_rn(__fdiv_rn(a, 127.f));
+                if ((tid & 7) == 0) out.d[tok_scale(out.J, e >> 5, mo)] = tok_scale_value(d);
+                q[r] = qw; h[r] = __half_as_ushort(d);
+                mine.add(h[r], __dp4a((int)qw, 0x01010101, 0));
+            } else if ((tid & 7) == 0) out.d[tok_scale(out.J, e >> 5, mo)] = tok_scale_value(__float2half_rn(__fdiv_rn(a, 127.f)));
         }
     }
-    if (!dig.q) return;
-    // the digits of a product that takes all of K at once
+    if constexpr (!DIG) return;
+    else {
+    __shared__ DigReduce dred;
     const DigRange all = mine.over_cta(dred);
     if (tid == 0) { dig.info[mo] = all.unit() | all.planes() << 8; dig.bias[mo] = all.total(); }
     const int tt = mo / dig.T, t = mo - tt * dig.T;
@@ -149,6 +153,7 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 1024) vf_norm_quant(const Decod
         #pragma unroll
         for (int j = 0; j < 4; j++) *reinterpret_cast<unsigned*>(dig.q + dig_offset(dig, E / 32, tt, e >> 5, e >> 4 & 1, j, t) + (e & 15)) = d[j];
         if (3 * dig.T + t < dig_rows(dig.T)) *reinterpret_cast<unsigned*>(dig.q + dig_offset(dig, E / 32, tt, e >> 5, e >> 4 & 1, 0, 3 * dig.T + t) + (e & 15)) = 0;      // rows of padding
+    }
     }
 }
 
@@ -340,7 +345,8 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     GemmParams g{};
     g.M = M;
     auto norm = [&](bool embed, int m0, int count, int ranges, const float* w, const TokX& out, const DigX& x) -> int {
-        MI_CUDA(ctx, launch_k(pdl, E <= 2048 ? vf_norm_quant<1> : vf_norm_quant<2>, dim3(count), dim3(nt_norm), 0, ctx->stream, P, tokens, embed, m0, b.X, (const double*)(ranges ? b.part : nullptr), ranges,
+        const auto kern = E <= 2048 ? (x.q ? vf_norm_quant<1, true> : vf_norm_quant<1, false>) : (x.q ? vf_norm_quant<2, true> : vf_norm_quant<2, false>);
+        MI_CUDA(ctx, launch_k(pdl, kern, dim3(count), dim3(nt_norm), 0, ctx->stream, P, tokens, embed, m0, b.X, (const double*)(ranges ? b.part : nullptr), ranges,
                               (long long)M * b.ldp, b.ldp, w, out, x));
         return MI_OK;
     };
