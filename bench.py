@@ -573,8 +573,8 @@ def run_ours(args, rank, world, local_rank):
                        "l2": "1.74 GB of weights per pass, larger than L2"},
             "roofline": {"bound": "hbm", "achieved": round(byt / (ms64 * 1e-3) / 1e9, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(byt / (ms64 * 1e-3) / 1e9 / peak, 4), "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})", "traffic": None,
-                         "kernel": "whole step (gemm_q4_q8_tok_kernel + attn_tok_kernel + glue)", "algorithmic_bytes_per_launch": byt,
-                         "note": "algorithmic bytes count the weights once per step; a pass over 64 sequences reads them once per token tile (16 to 32 tokens), partly from the L2"},
+                         "kernel": "whole step (gemm_q4_q8_tok_kernel or, above 16 sequences, gemm_dig_kernel + attn_tok_kernel + glue)", "algorithmic_bytes_per_launch": byt,
+                         "note": "algorithmic bytes count the weights once per step; a pass over 64 sequences reads them once per token tile (16 to 64 tokens), partly from the L2"},
             "step_ms_by_batch": {str(B): round(v[0], 3) for B, v in res.items()},
             "tok_s_by_batch": {str(B): round(B / (v[0] * 1e-3), 1) for B, v in res.items()},
             "gpu_launches": K * ((7 * cfg.n_layer + 3) * 2 + 9 * cfg.n_layer + 3),       # one pass per step; RoPE and SwiGLU are kernels of their own at 64

@@ -16,11 +16,11 @@
 //                that the way from a freed stage to a full one is a store and two barriers;
 //   one warp   : issues the MMAs; the whole warp runs the loop, one lane issues (see there);
 //   the 16 warps again at the end of a unit, when the first stages of the next one are in place.
-// Measured (event time, launches back to back): gate/up of 333 tokens (17920 x 1536) 78 us against 123 for the product over blocks, down (1536 x 8960) 36 / 64, batch of 64
-// on 22016 x 2048 37 / 49, 2048 x 11008 19 / 29, 151936 x 2048 142 / 250; 32 tokens on 22016 x 2048 31 / 31.  A stage of two blocks takes 620 clocks at 64 tokens, its MMAs 576;
+// Measured (event time, launches back to back): gate/up of 333 tokens (17920 x 1536) 74 us against 123 for the product over blocks, down (1536 x 8960) 36 / 64, batch of 64
+// on 22016 x 2048 35 / 49, 2048 x 11008 19 / 29, 151936 x 2048 133 / 250; it loses at 32 tokens on 22016 x 2048 (32 / 31), at 16 (31 / 19) and at 2560 x 2048 x 64 (20 / 15).  A stage of two blocks takes 620 clocks at 64 tokens, its MMAs 576;
 // the rest is the start (7000 clocks until the first MMA) and the end of a unit (6000).  Tried: weights expanded weight by weight or in byte lanes with seven sums per
 // token (the expansion or the tensor memory is full first), stages of one and four blocks, eight expanding warps, results through arrays in
-// registers (spills): 95 to 210 us for the gate/up.
+// registers (spills): 95 to 210 us for the gate/up.  Carry additions moved to the multiplier's pipe: no change, both sides in turn on one GPU.
 #include "gemm_dig.cuh"
 #include <algorithm>
 #include <atomic>

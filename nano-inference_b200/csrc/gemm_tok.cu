@@ -28,7 +28,7 @@
 // meeting another warp.  Small ones: kw warps of a CTA share the K tiles of a unit and fold their sums through shared memory.
 // Each warp streams its tiles through a ring of bulk copies that starts before the kernel waits for its predecessor (weights
 // depend on nothing); the activations of the CTA's K range and token tile are staged once, or chunk by chunk where they do
-// not fit.  With 32 rows x 32 tokens per warp an A fragment serves four MMAs and a B fragment two.  For many tokens a tcgen05 kernel of
+// not fit.  Products of more tokens go to gemm_dig.cu where the pass's cost model says so.  With 32 rows x 32 tokens per warp an A fragment serves four MMAs and a B fragment two.  For many tokens a tcgen05 kernel with this scaling per block, of
 // four roles (unpackers, MMA issuer, activation copies, scaling warps reading tensor memory) was measured as well: 17920 x 1536 with 333
 // tokens 130 us against 123, 2048 x 11008 with 64 tokens 26.6 against 28; one thread issuing an MMA per 32-element block took 150 cycles
 // for each, and the unpackers' issue slots are missing beside the scaling.
