@@ -385,17 +385,17 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     {   // what the M-token step's product wants to know of the weight scales (gemm_dig.cuh)
         size_t rows = 0;
         for (const mi_weight& v : m->views) rows += (size_t)v.groups * 32;
-        uint8_t* d_exp; int* d_wide;
-        if ((st = dev_alloc(ctx, m, &d_exp, rows)) || (st = dev_alloc(ctx, m, &d_wide, m->views.size()))) return st;
+        uint8_t* d_exp; int* d_bad;
+        if ((st = dev_alloc(ctx, m, &d_exp, rows)) || (st = dev_alloc(ctx, m, &d_bad, m->views.size()))) return st;
         for (size_t i = 0; i < m->views.size(); i++) {
             m->views[i].row_exp = d_exp;
-            if ((st = launch_row_exponents(ctx, &m->views[i], d_exp, d_wide + i))) return st;
+            if ((st = launch_row_exponents(ctx, &m->views[i], d_exp, d_bad + i))) return st;
             d_exp += (size_t)m->views[i].groups * 32;
         }
-        std::vector<int> wide(m->views.size());
-        MI_CUDA(ctx, cudaMemcpyAsync(wide.data(), d_wide, wide.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        std::vector<int> bad(m->views.size());
+        MI_CUDA(ctx, cudaMemcpyAsync(bad.data(), d_bad, bad.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        for (size_t i = 0; i < m->views.size(); i++) m->views[i].wide = wide[i];
+        for (size_t i = 0; i < m->views.size(); i++) m->views[i].bad_rows = bad[i];
     }
 
     // ---- per-warp tile lists: the order in which each warp of the grid consumes tiles during one step

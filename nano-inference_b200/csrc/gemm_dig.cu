@@ -3,11 +3,13 @@
 //
 // What bounds the other product is one FP64 multiplication per (row, block, token) and the instructions around it.  Here the scales move into the operands: every scale
 // is an fp16 number, so within a row (token, K range) all of them are integers times one power of two, an element is an integer of 18 to 24 bits, and that is cut into
-// base-256 digits: three (four) of the weight's against three (four) planes of the token's.  The MMAs (kind::i8, exact int32 sums) run over all of K; partial
+// base-256 digits: three of the weight's against three (four) planes of the token's.  The MMAs (kind::i8, exact int32 sums) run over all of K; partial
 // products of equal weight 256^s share a sum, so 9 int8 products cost three MMAs of N = 3 tokens and five columns of tensor memory a token.  At the end of a unit the sums are
-// put together as one 64-bit integer and rounded once.  9 products at the int8 rate are 0.035 clocks of an SM per (row, block, token), the two FP64 operations 0.031; but
-// the tensor core needs no issue slots beside it.  The digits hold any row whose scales lie at most 16 binades apart and any token with at most 13 (8 and 5 with three
-// digits); other rows and tokens, and scales that are not finite, are summed block by block behind the main loop.
+// put together as one integer and rounded once.  9 products at the int8 rate are 0.035 clocks of an SM per (row, block, token), the two FP64 operations 0.031; but
+// the tensor core needs no issue slots beside it.  The digits hold any row whose scales lie at most 8 binades apart and any token with at most 13 (5 with three
+// planes); other rows and tokens, and scales that are not finite, are summed block by block behind the main loop.  How large the integer gets: a weight is below
+// 8 * 2^11 * 2^8 units, an activation 2^7 * 2^11 * 2^5 with three planes and 2^13 in place of 2^5 with four, so K = 2^14 elements sum to less than 2^59 and 2^67: one
+// 64-bit number holds the former, two of them the latter.
 //
 // Dataflow of a CTA (one per SM, a unit is 128 rows x T <= 64 tokens x one K range):
 //   copies     : one warp streams the q4_0 tiles (bulk copies, ahead of the wait for the predecessor), one the activation planes, four blocks at a time;
@@ -36,7 +38,8 @@ constexpr int kMaxN = kDigPlanes * kDigMaxT;                                // c
 constexpr int kXBytes = kXStage * kMaxN * 32;
 constexpr int kGroups = 4, kExpWarps = 4 * kGroups, kWarps = kExpWarps + 3, kThreads = kWarps * 32;      // groups of four warps, a quarter of the 128 rows each
 constexpr int kRowNone = 255;
-constexpr long long kBias3 = 0x808080ll, kBias4 = 0x80808080ll;          // of three and four weight digits: DigX::bias times this is in the sums
+constexpr int kNW = 3, kMaxSpread = 8;                                   // digits of a weight; binades between a row's scales that they hold
+constexpr long long kBias = 0x808080ll;                                  // DigX::bias times this is in the sums (expand_block)
 
 struct DigParams {
     const uint8_t* base; const uint8_t* row_exp; int groups, nb, nst, rows;     // tiled weights; nst: steps of eight blocks
@@ -68,17 +71,18 @@ __device__ __forceinline__ void tmem_zero32(uint32_t a) {
                  ::"r"(a), "r"(0) : "memory");
 }
 // The values exist here (the compiler would compute them behind the wait that follows).
-template <int NW>
-__device__ __forceinline__ void keep(unsigned (&d)[2][NW][8]) {
+__device__ __forceinline__ void keep(unsigned (&d)[2][kNW][8]) {
     #pragma unroll
     for (int b = 0; b < 2; b++)
         #pragma unroll
-        for (int j = 0; j < NW; j++)
+        for (int j = 0; j < kNW; j++)
             asm volatile("" : "+r"(d[b][j][0]), "+r"(d[b][j][1]), "+r"(d[b][j][2]), "+r"(d[b][j][3]), "+r"(d[b][j][4]), "+r"(d[b][j][5]), "+r"(d[b][j][6]), "+r"(d[b][j][7]));
 }
 __device__ __forceinline__ void tmem_zero4(uint32_t a) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%1,%1};" ::"r"(a), "r"(0) : "memory");
 }
+__device__ __forceinline__ void tmem_zero1(uint32_t a) { asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(a), "r"(0) : "memory"); }
+__device__ __forceinline__ void tmem_ld1(uint32_t a, int& v) { asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(a)); }
 __device__ __forceinline__ void tmem_ld4(uint32_t a, int (&v)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
 }
@@ -98,33 +102,19 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 }
 
 // The digits of a block's 32 weights (nibble n - 8) * m in element order, base 256, each 128 too large and so unsigned (what that adds to the sums is
-// subtracted at the end, DigX::bias).  m = a0 + 256 a1, three digits (|m| < 2^20): two weights per multiplication in lanes of 16 bits, n a0 + c0 and
-// n a1 + c1 + the carry of the former, where c0 + 256 c1 = 0x808080 - 8 m.  Four digits: weight by weight.
-template <int NW>
-__device__ __forceinline__ void expand_block(const uint4& w, int m, unsigned (&d)[NW][8]) {
+// subtracted at the end, DigX::bias).  m = a0 + 256 a1 (|m| < 2^19): two weights per multiplication in lanes of 16 bits, n a0 + c0 and
+// n a1 + c1 + the carry of the former, where c0 + 256 c1 = 0x808080 - 8 m.
+__device__ __forceinline__ void expand_block(const uint4& w, int m, unsigned (&d)[kNW][8]) {
     const unsigned ww[4] = {w.x, w.y, w.z, w.w};
-    if constexpr (NW == 3) {
-        const unsigned c = 0x808080u - 8u * (unsigned)m, c0 = (c & 255u) * 0x10001u, c1 = (c >> 8) * 0x10001u;
-        const unsigned a0 = (unsigned)m & 255u, a1 = (unsigned)(m >> 8);
-        #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const unsigned n = (i < 4 ? ww[i] : ww[i - 4] >> 4) & 0x0F0F0F0Fu;
-            const unsigned ne = n & 0x00FF00FFu, no = __byte_perm(n, 0, 0x4341);
-            const unsigned pe = ne * a0 + c0, po = no * a0 + c0;
-            const unsigned se = ne * a1 + c1 + __byte_perm(pe, 0, 0x4341), so = no * a1 + c1 + __byte_perm(po, 0, 0x4341);
-            d[0][i] = __byte_perm(pe, po, 0x6240); d[1][i] = __byte_perm(se, so, 0x6240); d[2][i] = __byte_perm(se, so, 0x7351);
-        }
-    } else {
-        const unsigned c = 0x80808080u - 8u * (unsigned)m;
-        #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const unsigned n = (i < 4 ? ww[i] : ww[i - 4] >> 4) & 0x0F0F0F0Fu;
-            unsigned v[4];
-            #pragma unroll
-            for (int j = 0; j < 4; j++) v[j] = __byte_perm(n, 0, 0x4440 + j) * (unsigned)m + c;
-            const unsigned a = __byte_perm(v[0], v[1], 0x5140), b = __byte_perm(v[2], v[3], 0x5140), e = __byte_perm(v[0], v[1], 0x7362), f = __byte_perm(v[2], v[3], 0x7362);
-            d[0][i] = __byte_perm(a, b, 0x5410); d[1][i] = __byte_perm(a, b, 0x7632); d[2][i] = __byte_perm(e, f, 0x5410); d[3][i] = __byte_perm(e, f, 0x7632);
-        }
+    const unsigned c = (unsigned)kBias - 8u * (unsigned)m, c0 = (c & 255u) * 0x10001u, c1 = (c >> 8) * 0x10001u;
+    const unsigned a0 = (unsigned)m & 255u, a1 = (unsigned)(m >> 8);
+    #pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const unsigned n = (i < 4 ? ww[i] : ww[i - 4] >> 4) & 0x0F0F0F0Fu;
+        const unsigned ne = n & 0x00FF00FFu, no = __byte_perm(n, 0, 0x4341);
+        const unsigned pe = ne * a0 + c0, po = no * a0 + c0;
+        const unsigned se = ne * a1 + c1 + __byte_perm(pe, 0, 0x4341), so = no * a1 + c1 + __byte_perm(po, 0, 0x4341);
+        d[0][i] = __byte_perm(pe, po, 0x6240); d[1][i] = __byte_perm(se, so, 0x6240); d[2][i] = __byte_perm(se, so, 0x7351);
     }
 }
 
@@ -153,7 +143,7 @@ static __device__ __noinline__ double row_sum_dig(const DigParams& p, int row, i
     return acc;
 }
 
-template <int KB, int NW, bool PART>
+template <int KB, bool PART>
 __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_constant__ DigParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (0u - smem_u32(smem_raw) & 255u);          // the swizzle goes by address bits
@@ -241,8 +231,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
     const int T = p.x.T, units = p.ksg * row_tiles * p.x.TT, N = planes == 4 ? 4 * T : dig_rows(T);
     // tensor memory: sums of weight 256^s in columns s * T .. (the MMAs of a token tile of an odd number of eights reach eight columns further), stages of weight
     // digits at the end
-    const int fit = (512 - (NW - 1) * T - N) / (kStage * NW * 8), slots = fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
-    const uint32_t a_base = tmem + 512 - slots * (kStage * NW * 8);
+    const int fit = (512 - (kNW - 1) * T - N) / (kStage * kNW * 8), slots = fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
+    const uint32_t a_base = tmem + 512 - slots * (kStage * kNW * 8);
 
     if (warp < kExpWarps) {
         // ---------------- weights: nibbles and scales -> digits in registers, then in tensor memory (each of four groups of four warps takes every fourth
@@ -269,41 +259,59 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         auto finish = [&](const Ends& e) -> bool {
             const Unit U = unit(e.u);
             const int n0 = U.ts * T + wg * G, tg = min(min(T - wg * G, G), p.M - n0), row = U.rt * 128 + q * 32 + lane;       // tokens n0 .. n0 + tg
-            if (lane < G) table[lane] = make_longlong2(e.bias * (NW == 4 ? kBias4 : kBias3), PART ? (1023 - 50 + (e.info & 255)) << 20 : (127 - 50 + (e.info & 255)) << 23);
+            if (lane < G) {                                            // (with four planes sums are a high and a low part, units of 2^32 and of 1)
+                const int ex = e.info & 255;
+                if (planes == 3) table[lane] = make_longlong2(e.bias * kBias, PART ? (1023 - 50 + ex) << 20 : (127 - 50 + ex) << 23);
+                else table[lane] = make_longlong2((long long)(unsigned)e.bias * kBias, (e.bias >> 32) * kBias << 8 | ex);
+            }
             __syncwarp();
             if (!wait_or_abort(d_full, n_done & 1, abort_flag)) return false;
             n_done++;
             tc_fence_after();
             float* y = p.y + (size_t)n0 * p.rows + row;
             double* part = p.part + ((size_t)U.sp * p.M + n0) * p.ldp + row;
-            #pragma unroll 1
-            for (int g = 0; g < min(T - wg * G, G); g += 4) {                          // (rolled: four tokens at a time fit the registers and the instruction cache)
-                const uint32_t a = trow + wg * G + g;
-                int d[NW + 2][4];
-                unsigned high[4] = {0, 0, 0, 0};
-                if (planes == 4) {
-                    tmem_ld4(a + (NW + 2) * T, d[0]);
+            const int mine = min(T - wg * G, G);
+            if (planes == 3) {
+                #pragma unroll 1
+                for (int g = 0; g < mine; g += 4) {                    // (rolled: four tokens at a time fit the registers and the instruction cache)
+                    const uint32_t a = trow + wg * G + g;
+                    int d[kNW + 2][4];
+                    #pragma unroll
+                    for (int i = 0; i < kNW + 2; i++) tmem_ld4(a + i * T, d[i]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     #pragma unroll
-                    for (int i = 0; i < 4; i++) high[i] = (unsigned)d[0][i] << (8 * NW - 16);
+                    for (int i = 0; i < kNW + 2; i++) tmem_zero4(a + i * T);       // for the next unit
+                    #pragma unroll
+                    for (int i = 0; i < 4; i++) {                      // the sum is below 2^59, whatever its parts are
+                        const longlong2 tok = table[g + i];
+                        long long v = (long long)((unsigned long long)(unsigned)d[4][i] << 32) - tok.x;
+                        v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
+                        if (g + i < tg && row < p.rows) {
+                            if constexpr (PART) __stcg(part, __dmul_rn(__ll2double_rn(v), __hiloint2double((int)tok.y + (e.ew << 20), 0)));
+                            // (times a power of two that leaves the result a normal number: the one rounding is the conversion's)
+                            else *y = __fmul_rn(__ll2float_rn(v), __int_as_float((int)tok.y + (e.ew << 23))) + e.bv;
+                        }
+                        if constexpr (PART) part += p.ldp; else y += p.rows;
+                    }
                 }
-                #pragma unroll
-                for (int i = 0; i < NW + 2; i++) tmem_ld4(a + i * T, d[i]);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                #pragma unroll
-                for (int i = 0; i < NW + 2; i++) tmem_zero4(a + i * T);      // for the next unit
-                if (planes == 4) tmem_zero4(a + (NW + 2) * T);
-                #pragma unroll
-                for (int i = 0; i < 4; i++) {                          // the sum itself is below 2^63, whatever its parts are
-                    high[i] += (unsigned)d[4][i];
-                    if constexpr (NW == 4) high[i] += (unsigned)d[5][i] << 8;
-                    const longlong2 tok = table[g + i];
-                    long long v = (long long)((unsigned long long)high[i] << 32) - tok.x;
-                    v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
-                    if (g + i < tg && row < p.rows) {
-                        if constexpr (PART) __stcg(part, __dmul_rn(__ll2double_rn(v), __hiloint2double((int)tok.y + (e.ew << 20), 0)));
-                        // (times a power of two that leaves the result a normal number: the one rounding is the conversion's)
-                        else *y = __fmul_rn(__ll2float_rn(v), __int_as_float((int)tok.y + (e.ew << 23))) + e.bv;
+            } else {
+                #pragma unroll 1
+                for (int t = 0; t < mine; t++) {                       // sums below 2^67 in two parts; token by token, so that its code takes no registers from the rest
+                    int d[kNW + 3];
+                    #pragma unroll
+                    for (int i = 0; i < kNW + 3; i++) tmem_ld1(trow + wg * G + t + i * T, d[i]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    #pragma unroll
+                    for (int i = 0; i < kNW + 3; i++) tmem_zero1(trow + wg * G + t + i * T);
+                    const longlong2 tok = table[t];
+                    long long lo = mad_wide(d[0], 1, -tok.x), hi = mad_wide(d[5], 1 << 8, (long long)d[4]) - (tok.y >> 8);
+                    lo = mad_wide(d[1], 1 << 8, lo); lo = mad_wide(d[2], 1 << 16, lo); lo = mad_wide(d[3], 1 << 24, lo);
+                    hi += lo >> 32;                                    // below 2^36, and the rest of lo is 0 .. 2^32 - 1: the double rounds once
+                    const double v = __fma_rn((double)hi, 0x1p32, (double)(unsigned)lo);
+                    const int ex = ((int)tok.y & 255) + e.ew - 50;
+                    if (t < tg && row < p.rows) {
+                        if constexpr (PART) __stcg(part, __dmul_rn(v, __hiloint2double((1023 + ex) << 20, 0)));
+                        else *y = __fmul_rn(__double2float_rn(v), __int_as_float((127 + ex) << 23)) + e.bv;
                     }
                     if constexpr (PART) part += p.ldp; else y += p.rows;
                 }
@@ -336,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 for (; sc < end; sc += kGroups) {
                     // the first stage of a unit goes beside the last ones of the unit before, whose sums are read then (later stages would wait for its last MMAs)
                     if (pending && sc > sc0) { if (!(ok = finish(before))) break; pending = false; }
-                    unsigned d[kStage][NW][8];
+                    unsigned d[kStage][kNW][8];
                     #pragma unroll
                     for (int b = 0; b < kStage; b++) {
                         const int k = min((sc - step0) * kStage + b, nblk - 1);
@@ -344,7 +352,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                         const uint4 w = *reinterpret_cast<const uint4*>(tile + (k % KB * 32 + lane) * 16);
                         const unsigned h = *reinterpret_cast<const unsigned short*>(tile + KB * 512 + (lane * KB + k % KB) * 2);
                         const int m = scale_mantissa(h) << ((scale_exponent(h) - now.ew) & 31);
-                        expand_block<NW>(w, h & 0x8000u ? -m : m, d[b]);
+                        expand_block(w, h & 0x8000u ? -m : m, d[b]);
                     }
                     keep(d);
                     // (a ring of eight barriers, whatever the number of slots: a group never falls two phases behind)
@@ -353,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                     #pragma unroll
                     for (int b = 0; b < kStage; b++)
                         #pragma unroll
-                        for (int j = 0; j < NW; j++) tmem_st8(a_row + ((sc & (slots - 1)) * kStage + b) * (NW * 8) + 8 * j, d[b][j]);
+                        for (int j = 0; j < kNW; j++) tmem_st8(a_row + ((sc & (slots - 1)) * kStage + b) * (kNW * 8) + 8 * j, d[b][j]);
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();
@@ -415,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         auto mma = [&](uint32_t a, uint32_t x) {
             const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)16 << 32) | (1ull << 46) | (6ull << 61);       // eight rows of 32 bytes, 32-byte swizzle
             #pragma unroll
-            for (int i = 0; i < NW; i++)
+            for (int i = 0; i < kNW; i++)
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 1, 0;\n\t"
                     "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
@@ -426,18 +434,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         auto mma_and_test = [&](uint32_t a, uint32_t x, uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1) -> uint32_t {
             const uint64_t db = (uint64_t)((x & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)16 << 32) | (1ull << 46) | (6ull << 61);       // eight rows of 32 bytes, 32-byte swizzle
             uint32_t r;
-            if constexpr (NW == 3)
-                asm volatile(
-                    "{\n\t.reg .pred p, t, u;\n\tsetp.ne.b32 p, 1, 0;\n\t"
-                    "mbarrier.test_wait.parity.shared::cta.b64 t, [%9], %10;\n\t"
-                    "mbarrier.test_wait.parity.shared::cta.b64 u, [%11], %12;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%1], [%4], %7, %8, p;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%2], [%5], %7, %8, p;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%3], [%6], %7, %8, p;\n\t"
-                    "and.pred t, t, u;\n\tselp.u32 %0, 1, 0, t;\n\t}"
-                    : "=r"(r) : "r"(tmem), "r"(tmem + (uint32_t)T), "r"(tmem + (uint32_t)(2 * T)), "r"(a), "r"(a + 8), "r"(a + 16), "l"(db), "r"(idesc),
-                      "r"(bar0), "r"(par0), "r"(bar1), "r"(par1) : "memory");
-            else { mma(a, x); r = 0; }
+            asm volatile(
+                "{\n\t.reg .pred p, t, u;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+                "mbarrier.test_wait.parity.shared::cta.b64 t, [%9], %10;\n\t"
+                "mbarrier.test_wait.parity.shared::cta.b64 u, [%11], %12;\n\t"
+                "tcgen05.mma.cta_group::1.kind::i8 [%1], [%4], %7, %8, p;\n\t"
+                "tcgen05.mma.cta_group::1.kind::i8 [%2], [%5], %7, %8, p;\n\t"
+                "tcgen05.mma.cta_group::1.kind::i8 [%3], [%6], %7, %8, p;\n\t"
+                "and.pred t, t, u;\n\tselp.u32 %0, 1, 0, t;\n\t}"
+                : "=r"(r) : "r"(tmem), "r"(tmem + (uint32_t)T), "r"(tmem + (uint32_t)(2 * T)), "r"(a), "r"(a + 8), "r"(a + 16), "l"(db), "r"(idesc),
+                  "r"(bar0), "r"(par0), "r"(bar1), "r"(par1) : "memory");
             return r;
         };
         int n_done = 0, sc = 0, xslot = 0;
@@ -453,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 if (!__any_sync(0xffffffffu, ready != 0) &&
                     ((g == 0 && !wait_or_abort(&x_full[xslot], x_phase, abort_flag)) || !wait_or_abort(&full[sc % kRing], (sc / kRing) & 1, abort_flag))) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t a = a_base + (sc & (slots - 1)) * (kStage * NW * 8), x = smem_u32(xs) + xslot * kXBytes + g * kStage * N * 32;
+                const uint32_t a = a_base + (sc & (slots - 1)) * (kStage * kNW * 8), x = smem_u32(xs) + xslot * kXBytes + g * kStage * N * 32;
                 const bool last = b + kStage >= b1, turn = g == 1 || last;                    // turn: the next stage begins another copy of activations
                 const int ns = sc + 1, nx = turn ? (xslot + 1 == kXSlots ? 0 : xslot + 1) : xslot;
                 const uint32_t np = turn && nx == 0 ? x_phase ^ 1 : x_phase;
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                 if (b + kStage <= b1) {
                     if (elected) {
                         mma(a, x);
-                        ready = mma_and_test(a + NW * 8, x + N * 32, smem_u32(&full[ns % kRing]), (ns / kRing) & 1, smem_u32(turn ? &x_full[nx] : &full[ns % kRing]), turn ? np : (ns / kRing) & 1);
+                        ready = mma_and_test(a + kNW * 8, x + N * 32, smem_u32(&full[ns % kRing]), (ns / kRing) & 1, smem_u32(turn ? &x_full[nx] : &full[ns % kRing]), turn ? np : (ns / kRing) & 1);
                         tc_commit(&empty[sc % kRing]);
                         if (turn) tc_commit(&x_empty[xslot]);
                     }
@@ -595,7 +601,7 @@ __global__ void __launch_bounds__(kSwiWarps * 32) swiglu_digits_kernel(const flo
 
 // One warp per row
 template <int KB>
-__global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base, int groups, int nb, uint8_t* row_exp, int* wide) {
+__global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base, int groups, int nb, uint8_t* row_exp, int* bad_rows) {
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= groups * 32) return;
     int lo = 31, hi = 0;
@@ -607,15 +613,14 @@ __global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base,
     lo = __reduce_min_sync(0xffffffffu, lo); hi = __reduce_max_sync(0xffffffffu, hi);
     if (lane) return;
     lo = min(lo, max(hi, 1));
-    row_exp[row] = hi == 31 || hi - lo > 16 ? kRowNone : lo;
-    if (row_exp[row] == kRowNone) atomicOr(wide, 2);
-    else if (hi - lo > 8) atomicOr(wide, 1);
+    row_exp[row] = hi == 31 || hi - lo > kMaxSpread ? kRowNone : lo;
+    if (row_exp[row] == kRowNone) atomicAdd(bad_rows, 1);
 }
 
-template <int KB, int NW, bool PART>
+template <int KB, bool PART>
 int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
     const int units = (p.groups + 3) / 4 * p.x.TT * p.ksg;             // at least
-    auto kern = gemm_dig_kernel<KB, NW, PART>;
+    auto kern = gemm_dig_kernel<KB, PART>;
     static std::mutex mu;
     static std::atomic<unsigned> raised{0};                   // bit per device
     if (!(raised.load(std::memory_order_acquire) >> (ctx->device & 31) & 1u)) {
@@ -626,12 +631,6 @@ int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
     MI_CUDA(ctx, launch_k(pdl, kern, dim3((unsigned)std::min(units, ctx->sm_count)), dim3(kThreads), Smem::bytes, ctx->stream, p));
     return MI_OK;
 }
-template <int KB>
-int launch_kb(mi_ctx* ctx, const DigParams& p, bool wide, bool part, bool pdl) {
-    if (wide) return part ? launch_dig<KB, 4, true>(ctx, p, pdl) : launch_dig<KB, 4, false>(ctx, p, pdl);
-    return part ? launch_dig<KB, 3, true>(ctx, p, pdl) : launch_dig<KB, 3, false>(ctx, p, pdl);
-}
-
 }  // namespace
 
 // Token tiles and K ranges of a product over digits, the fewest clocks by a model from measured launches: 7000 until the first MMA, 290 per block or what its MMAs take,
@@ -639,13 +638,12 @@ int launch_kb(mi_ctx* ctx, const DigParams& p, bool wide, bool part, bool pdl) {
 bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* out) {
     const int nst = (w->nb + kStepBlk - 1) / kStepBlk, rt = (w->groups + 3) / 4;
     const int TT = (M + kDigMaxT - 1) / kDigMaxT, T = ((M + TT - 1) / TT + 7) / 8 * 8;
-    const int nw = w->wide & 1 ? 4 : 3;
-    const double blk = std::max(nw * dig_rows(T) / 2 + 30.0, nw == 3 ? 290.0 : 450.0);
+    const double blk = std::max(kNW * dig_rows(T) / 2 + 30.0, 290.0);
     double best = 1e300;
     if (!w->row_exp) return false;
     for (int ksg = 1; ksg <= (part ? std::min(nst, 8) : 1); ksg++) {
         const int steps = (nst + ksg - 1) / ksg;
-        if (steps * kStepBlk * 32 > 16384) continue;                   // a sum of digit products stays below 2^31 (four pairs of 255 * 128 per element)
+        if (steps * kStepBlk * 32 > 16384) continue;                   // a sum of digit products stays below 2^31 (three pairs of 255 * 128 per element)
         const long long units = (long long)rt * TT * ksg, rounds = (units + ctx->sm_count - 1) / ctx->sm_count;
         const double cost = 7000 + rounds * (std::min(steps * kStepBlk, w->nb) * blk + 4000 + 80.0 * T) + (part ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
         if (cost < best) { best = cost; *out = DigPlan{T, TT, ksg, cost}; }
@@ -657,13 +655,13 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
     DigParams p{};
     p.base = w->dev; p.row_exp = w->row_exp; p.groups = w->groups; p.nb = w->nb; p.nst = (w->nb + kStepBlk - 1) / kStepBlk; p.rows = (int)w->rows;
     p.ksg = pl.ksg; p.M = g.M;
-    p.x = x; p.q8 = g.x; p.bias = g.bias; p.y = g.y; p.part = g.part; p.ldp = g.ldp; p.err = ctx->d_err; p.bad_rows = w->wide & 2;
+    p.x = x; p.q8 = g.x; p.bias = g.bias; p.y = g.y; p.part = g.part; p.ldp = g.ldp; p.err = ctx->d_err; p.bad_rows = w->bad_rows;
     const bool part = mode == GEMM_PART;
     switch (w->kb) {
-        case 8: return launch_kb<8>(ctx, p, w->wide & 1, part, pdl);
-        case 4: return launch_kb<4>(ctx, p, w->wide & 1, part, pdl);
-        case 2: return launch_kb<2>(ctx, p, w->wide & 1, part, pdl);
-        default: return launch_kb<1>(ctx, p, w->wide & 1, part, pdl);
+        case 8: return part ? launch_dig<8, true>(ctx, p, pdl) : launch_dig<8, false>(ctx, p, pdl);
+        case 4: return part ? launch_dig<4, true>(ctx, p, pdl) : launch_dig<4, false>(ctx, p, pdl);
+        case 2: return part ? launch_dig<2, true>(ctx, p, pdl) : launch_dig<2, false>(ctx, p, pdl);
+        default: return part ? launch_dig<1, true>(ctx, p, pdl) : launch_dig<1, false>(ctx, p, pdl);
     }
 }
 
@@ -678,14 +676,14 @@ int launch_swiglu_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, con
     return MI_OK;
 }
 
-int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* wide) {
+int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* bad_rows) {
     const dim3 grid((unsigned)(w->groups * 4));
     if (w->groups == 0) return MI_OK;
     switch (w->kb) {
-        case 8: row_exponents_kernel<8><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
-        case 4: row_exponents_kernel<4><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
-        case 2: row_exponents_kernel<2><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
-        default: row_exponents_kernel<1><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, wide); break;
+        case 8: row_exponents_kernel<8><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
+        case 4: row_exponents_kernel<4><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
+        case 2: row_exponents_kernel<2><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
+        default: row_exponents_kernel<1><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
     }
     MI_CUDA(ctx, cudaGetLastError());
     return MI_OK;

@@ -75,7 +75,7 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
 int launch_tok_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const TokX& x, const DigX& out, int M, bool pdl);
 // The same behind SwiGLU: rows of y come as (gate, up) groups of 32, w is the matrix that takes its result; act: the result as q8_0
 int launch_swiglu_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const float* y, const TokX& act, const DigX& out, int M, bool pdl);
-// Exponents of a matrix's rows, for the product's weight digits: row_exp[groups * 32]; *wide: mi_weight::wide.
-int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* wide);
+// Exponents of a matrix's rows, for the product's weight digits: row_exp[groups * 32]; *bad_rows (zero before): mi_weight::bad_rows.
+int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* bad_rows);
 
 }  // namespace mi

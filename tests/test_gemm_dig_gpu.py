@@ -25,6 +25,25 @@ def lower(d, binades):
     return np.where(e > binades, d - (binades << 10), d & 0x8000).astype(np.uint16)
 
 
+def rewrite(path, **tensors):
+    """tensors: name with _ for . -> edit(fp16 scale bits [rows, blocks], nibbles [rows, blocks, 16]) of a q4_0 matrix, or edit(values) of an fp32 vector"""
+    r = gu.GgufReader(path)
+    with open(path, "r+b") as f:
+        for name, edit in tensors.items():
+            name = name.replace("__", ".")
+            typ, rows, cols = r.shape(name)
+            raw = r.tensor_bytes(name)
+            if typ == 0:
+                edit(raw.view(np.float32))
+            else:
+                q = raw.reshape(rows, cols // 32, 18)
+                d, n = np.ascontiguousarray(q[:, :, :2]).view(np.uint16)[:, :, 0], q[:, :, 2:]
+                edit(d, n)
+                q[:, :, :2] = d[:, :, None].view(np.uint8)
+            f.seek(r.tensors[name][2])
+            f.write(raw.tobytes())
+
+
 def same(ctx, pkg, path, n, V):
     """Prompt pass of n tokens, then a batch of min(n, 64) sequences: caches and logits of both products"""
     import torch
@@ -87,3 +106,85 @@ def test_scales_far_apart(ctx, pkg, tmp_path, weights, acts):
 def test_digit_product_on_model_shapes(ctx, pkg, tmp_path, preset, n):
     path = gu.make_synthetic(tmp_path / "m.gguf", preset, seed=2, extra=["--layers", 1, "--vocab", 1500])
     same(ctx, pkg, path, n, 1500)
+
+
+# The widest rows against the widest tokens that the digits hold: all blocks at the top of the range but one at its bottom, sums of one sign (every weight -8 or 7, every
+# activation the block's largest) and random ones.  The integer sum of such a row passes 2^63.  Both products round a sum that wide to 53 bits on the way,
+# the block product at every addition, this one once; what is compared is the fp32 value.
+def top_but_one(d, low, spread):
+    """exponent fields low + spread, one block of a row low; signs and mantissas as they are"""
+    d[:] = (d & 0x83FF) | ((low + spread) << 10)
+    d[:, 5] = (d[:, 5] & 0x83FF) | (low << 10)
+
+
+@pytest.mark.parametrize("spread", [8, 16])
+@pytest.mark.parametrize("signs", ["one", "random"])
+@pytest.mark.parametrize("embd", [1536, 2048, 8192])
+@pytest.mark.parametrize("n", [40, 64])
+def test_sums_beyond_64_bits(ctx, pkg, tmp_path, spread, signs, embd, n):
+    """lm_head on the embedding itself (the layer adds nothing)"""
+    path = gu.make_synthetic(tmp_path / "m.gguf", "tiny", seed=3, std=0.5, extra=["--layers", 1, "--embd", embd, "--heads", embd // 128, "--kv-heads", 8 if embd > 2048 else 2, "--ff", 256, "--vocab", 600, "--untied"])
+
+    def nothing(d, q):
+        d[:] = 0
+
+    def head(d, q):
+        d[:] = d & 0xFF00 | 0xFF if signs == "random" else 0x03FF
+        top_but_one(d, 1, spread)
+        if signs == "one":
+            q[::2], q[1::2] = 0x00, 0xFF                                  # -8 throughout, 7 throughout
+
+    def embedding(d, q):
+        d &= 0x7FFF
+        if signs == "one":
+            d[:], q[:] = 0x3800, 0xFF
+
+    def norm(w):
+        w[:] = 127 * 1.999 if signs == "one" else 30.0                    # block scales of about 2^0 and 2^-13
+        w[32 * 9:32 * 10] *= 2.0 ** -13
+
+    rewrite(path, blk__0__attn_output__weight=nothing, blk__0__ffn_down__weight=nothing, output__weight=head, token_embd__weight=embedding, output_norm__weight=norm)
+    same(ctx, pkg, path, n, 600)
+
+
+@pytest.mark.parametrize("spread", [8, 16])
+@pytest.mark.parametrize("signs", ["one", "random"])
+@pytest.mark.parametrize("ff", [1536, 8960, 16384])
+@pytest.mark.parametrize("n", [40, 64, 120])
+def test_sums_beyond_64_bits_over_ranges(ctx, pkg, tmp_path, spread, signs, ff, n):
+    """down projection: one gate for all, so that SwiGLU's result is that gate times the up rows"""
+    path = gu.make_synthetic(tmp_path / "m.gguf", "tiny", seed=4, std=0.5, extra=["--layers", 1, "--embd", 512, "--heads", 8, "--kv-heads", 4, "--ff", ff, "--vocab", 600])
+
+    def nothing(d, q):
+        d[:] = 0
+
+    def gate(d, q):
+        d[:], q[:] = 0x2800, 0xFF                                         # 512 * 7 / 32 = 112 for an input of ones
+
+    def up(d, q):
+        if signs == "one":
+            q[:] = 0xFF
+            d[:] = 0x1400                                                 # 2^-10
+        else:
+            d[:] = d & 0x8000 | 0x2C00                                    # 2^-4
+        low = np.arange(ff) // 32 % 8 == 3                                # every eighth block 13 binades below: one in each K range at least
+        d[low] = d[low] & 0x8000 | (2 if signs == "one" else 128)
+
+    def down(d, q):
+        d[:] = d & 0xFF00 | 0xFF if signs == "random" else 0x03FF
+        top_but_one(d, 1, spread)
+        for b in range(5, ff // 32, 48):
+            d[:, b] = d[:, 5]
+        if signs == "one":
+            q[::2], q[1::2] = 0x00, 0xFF
+
+    def embedding(d, q):
+        if signs == "one":
+            d[:], q[:] = 0x3800, 0xFF
+
+    def ones(w):
+        w[:] = 1.0
+
+    rewrite(path, blk__0__attn_output__weight=nothing, blk__0__ffn_gate__weight=gate, blk__0__ffn_up__weight=up, blk__0__ffn_down__weight=down, blk__0__ffn_norm__weight=ones,
+            **({"token_embd__weight": embedding, "output__weight": embedding} if signs == "one" else {}))
+    same(ctx, pkg, path, n, 600)
