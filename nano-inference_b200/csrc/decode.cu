@@ -395,7 +395,15 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         std::vector<int> bad(m->views.size());
         MI_CUDA(ctx, cudaMemcpyAsync(bad.data(), d_bad, bad.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        for (size_t i = 0; i < m->views.size(); i++) m->views[i].bad_rows = bad[i];
+        for (size_t i = 0; i < m->views.size(); i++) {
+            mi_weight& v = m->views[i];
+            v.bad_rows = bad[i];
+            if (!bad[i]) continue;
+            int* list;
+            if ((st = dev_alloc(ctx, m, &list, (size_t)bad[i] + 1)) || (st = launch_list_rows(ctx, &v, list, list + bad[i]))) return st;
+            v.bad_list = list;
+        }
+        MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
 
     // ---- per-warp tile lists: the order in which each warp of the grid consumes tiles during one step

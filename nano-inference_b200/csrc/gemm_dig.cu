@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 namespace mi {
 namespace {
@@ -38,12 +39,13 @@ constexpr int kMaxN = kDigPlanes * kDigMaxT;                                // c
 constexpr int kXBytes = kXStage * kMaxN * 32;
 constexpr int kGroups = 4, kExpWarps = 4 * kGroups, kWarps = kExpWarps + 3, kThreads = kWarps * 32;      // groups of four warps, a quarter of the 128 rows each
 constexpr int kRowNone = 255;
+constexpr int kMaxInfo = 4096;                                          // tokens times K ranges of a launch
 constexpr int kNW = 3, kMaxSpread = 8;                                   // digits of a weight; binades between a row's scales that they hold
 constexpr long long kBias = 0x808080ll;                                  // DigX::bias times this is in the sums (expand_block)
 
 struct DigParams {
     const uint8_t* base; const uint8_t* row_exp; int groups, nb, nst, rows;     // tiled weights; nst: steps of eight blocks
-    int ksg, M, bad_rows;
+    int ksg, M; const int* bad_list; int bad_rows;                              // rows without an exponent
     DigX x; TokX q8;
     const float* bias; float* y; double* part; int ldp;
     int* err;
@@ -125,22 +127,113 @@ __device__ __forceinline__ long long mad_wide(int v, int f, long long acc) {
     return r;
 }
 
-// One row's sum over blocks b0 .. b1 for token n, formed as the GEMV forms it: for rows and tokens whose scales the digits cannot hold.
-template <int KB>
-static __device__ __noinline__ double row_sum_dig(const DigParams& p, int row, int n, int b0, int b1) {
-    double acc = 0.0;
-    const int grp = row >> 5, r = row & 31;
-    #pragma unroll 1
-    for (int b = b0; b < b1; b++) {
-        const uint8_t* tile = p.base + ((size_t)grp * p.nb + b / KB * KB) * kTileRowBytes;
-        const uint4 w = __ldg(reinterpret_cast<const uint4*>(tile) + b % KB * 32 + r);
-        const float dw = __half2float(__ldg(reinterpret_cast<const __half*>(tile + KB * 512) + r * KB + b % KB));
-        auto word = [&](int e) { return (int)__ldcg(p.q8.q + tok_word(p.q8.J, b, n, e)); };
-        const int4 xa = make_int4(word(0), word(4), word(8), word(12)), xc = make_int4(word(16), word(20), word(24), word(28));
-        const float dx = (float)__dmul_rn(__ldcg(p.q8.d + tok_scale(p.q8.J, b, n)), 0x1p-1004);
-        acc = blk_acc(acc, dw, dx, dot_q4_block(w, xa, xc), __int2float_rn(8 * sum_x_block(xa, xc)));
+// C consecutive blocks of a row and a token, and their part of the sum: the GEMV's terms
+template <int C> struct BlkIn { uint4 w[C], xa[C], xb[C]; double x[C]; uint2 h; };
+template <int C>
+__device__ __forceinline__ double add_blocks(const BlkIn<C>& v, double acc) {
+    #pragma unroll
+    for (int i = 0; i < C; i++) {
+        const unsigned w[4] = {v.w[i].x, v.w[i].y, v.w[i].z, v.w[i].w}, lo[4] = {v.xa[i].x, v.xa[i].z, v.xb[i].x, v.xb[i].z}, hi[4] = {v.xa[i].y, v.xa[i].w, v.xb[i].y, v.xb[i].w};
+        int c = 0;                                                     // (n ^ 8) << 4 as int8 is 16 (n - 8): with TokX's 2^1004 the powers of two cancel
+        #pragma unroll
+        for (int k = 0; k < 4; k++) c = __dp4a((int)((w[k] & 0xF0F0F0F0u) ^ 0x80808080u), (int)hi[k], __dp4a((int)((w[k] << 4 & 0xF0F0F0F0u) ^ 0x80808080u), (int)lo[k], c));
+        const double scale = __dmul_rn((double)__half2float(__ushort_as_half((unsigned short)((i < 2 ? v.h.x : v.h.y) >> 16 * (i & 1)))), __dmul_rn(v.x[i], 0x1p-1008));
+        acc = __fma_rn(scale, (double)c, acc);
     }
     return acc;
+}
+
+// What the digits cannot hold (the main loop stores nothing there), block by block as the GEMV forms it: rows without an exponent with all tokens, all rows with tokens
+// without planes.  A warp takes one K range of 32 tokens of such a row or of 32 rows of such a token; the whole grid shares these jobs, whose rows and tokens they are, and
+// several warps of a CTA share a job's blocks while there are fewer than warps.  What bounds it is a chain of requests to L2 where there is little to do, then issue.
+// Measured (launches back to back, us; without any / with one token / three / a tenth of the tokens / 1 % of the rows / 10 %, and the product over blocks): 17920x1536 with 333
+// tokens 71.6 / 75.8 / 80.2 / 128.7 / 82.8 / 172.9, 121.3; 1536x8960 with 333 33.1 / 37.4 / 38.8 / 73.8 / 38.9 / 97.1, 62.8; 22016x2048 with 64 31.6 / 38.6 / - / 52.2 / 36.3 / 63.9, 46.6;
+// 2048x11008 with 64 15.6 / 20.1 / - / 31.9 / 19.8 / -, 26.1.  All tokens out of range: 597 and 301 us of the first two.  (One thread per row and token before: 118 and 78 with
+// one token, 1038 and 485 with 1 % of the rows.)  Tried: 16 rows x 8 tokens per warp on mma.sync (7 of 8 columns idle for one token: 85 and 53), units
+// summed by the CTA that has them (97 with 1 % of the rows: rows are not spread evenly).
+template <int KB, bool PART>
+static __device__ __forceinline__ void sum_over_blocks(const DigParams& p, uint8_t* smem, bool any_tokens) {
+    constexpr int C = KB < 4 ? KB : 4, S = KB / C;                     // blocks requested together, of a tile's KB
+    constexpr int kWords = kMaxInfo / (32 * kExpWarps);
+    double* fold = reinterpret_cast<double*>(smem);                    // [warp][lane]
+    unsigned short* toks = reinterpret_cast<unsigned short*>(smem + kExpWarps * 32 * 8);      // tokens without planes: K range * M + token
+    __shared__ int s_count[kExpWarps];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int n_toks = 0;
+    if (any_tokens) {
+        const int total = p.M * p.ksg, words = (total + 32 * kExpWarps - 1) / (32 * kExpWarps);        // 32 entries each, a run of them per warp: the same list in every CTA
+        unsigned none[kWords];
+        int mine = 0;
+        if (warp < kExpWarps) {
+            bool b[kWords];
+            #pragma unroll
+            for (int i = 0; i < kWords; i++) { const int at = (warp * words + i) * 32 + lane; b[i] = i < words && at < total && __ldcg(p.x.info + at) >> 8 == kDigNone; }
+            #pragma unroll
+            for (int i = 0; i < kWords; i++) { none[i] = __ballot_sync(0xffffffffu, b[i]); mine += __popc(none[i]); }
+            if (lane == 0) s_count[warp] = mine;
+        }
+        __syncthreads();
+        int at = 0;
+        for (int k = 0; k < kExpWarps; k++) { if (k < warp) at += s_count[k]; n_toks += s_count[k]; }
+        if (warp < kExpWarps)
+            #pragma unroll
+            for (int i = 0; i < kWords; i++) {
+                if (none[i] >> lane & 1) toks[at + __popc(none[i] & ((1u << lane) - 1))] = (warp * words + i) * 32 + lane;
+                at += __popc(none[i]);
+            }
+        __syncthreads();
+    }
+    const int tg = (p.M + 31) / 32, rg = (p.rows + 31) / 32, by_row = p.bad_rows * p.ksg * tg, jobs = by_row + n_toks * rg;
+    int shift = 0;                                                     // 2^shift warps per job
+    while (shift < 4 && jobs << (shift + 1) <= (int)gridDim.x * kExpWarps) shift++;
+    #pragma unroll 1
+    for (int j0 = blockIdx.x * (kExpWarps >> shift); j0 < jobs; j0 += gridDim.x * (kExpWarps >> shift)) {
+        const int j = j0 + (warp >> shift), part = warp & ((1 << shift) - 1);
+        const bool mine = warp < kExpWarps && j < jobs;
+        int row = 0, n = 0, sp = 0;                                    // this lane's
+        if (mine && j < by_row) { const int q = j / tg; n = (j - q * tg) * 32 + lane; row = __ldg(p.bad_list + q / p.ksg); sp = q % p.ksg; }
+        else if (mine) { const int q = (j - by_row) / rg, e = toks[q]; row = (j - by_row - q * rg) * 32 + lane; sp = e / p.M; n = e - sp * p.M; }
+        const bool has = mine && row < p.rows && n < p.M;
+        double acc = 0.0;
+        if (mine) {
+            const int r = min(row, p.rows - 1), c = min(n, p.M - 1), b0 = sp * p.nst / p.ksg * kStepBlk, tiles = (min((sp + 1) * p.nst / p.ksg * kStepBlk, p.nb) - b0) / KB;
+            const int t0 = b0 / KB + (tiles * part >> shift), t1 = b0 / KB + (tiles * (part + 1) >> shift);
+            const uint8_t* w = p.base + ((size_t)(r >> 5) * p.nb + t0 * KB) * kTileRowBytes, * h = w + KB * 512 + (r & 31) * KB * 2;
+            w += (r & 31) * 16;
+            const unsigned* x = p.q8.q + tok_word(p.q8.J, t0 * KB, c, 0);                      // a block of a token is eight words: elements 0, 16, 4, 20, ..
+            const double* d = p.q8.d + tok_scale(p.q8.J, t0 * KB, c);
+            const size_t x_step = (size_t)p.q8.J * 64, d_step = (size_t)p.q8.J * 8;
+            #pragma unroll 1
+            for (int t = t0; t < t1; t++) {
+                #pragma unroll
+                for (int s = 0; s < S; s++) {
+                    BlkIn<C> v;
+                    #pragma unroll
+                    for (int i = 0; i < C; i++) {
+                        v.w[i] = __ldg(reinterpret_cast<const uint4*>(w + (s * C + i) * 512));
+                        v.xa[i] = __ldcg(reinterpret_cast<const uint4*>(x)); v.xb[i] = __ldcg(reinterpret_cast<const uint4*>(x) + 1);
+                        v.x[i] = __ldcg(d);
+                        x += x_step; d += d_step;
+                    }
+                    if constexpr (C == 4) v.h = __ldg(reinterpret_cast<const uint2*>(h) + s);
+                    else if constexpr (C == 2) v.h.x = __ldg(reinterpret_cast<const unsigned*>(h));
+                    else v.h.x = __ldg(reinterpret_cast<const unsigned short*>(h));
+                    acc = add_blocks(v, acc);
+                }
+                w += KB * kTileRowBytes; h += KB * kTileRowBytes;
+            }
+        }
+        if (shift) {                                                   // (all jobs are under way then)
+            if (mine) fold[warp * 32 + lane] = acc;
+            __syncthreads();
+            if (part) continue;
+            #pragma unroll 1
+            for (int k = 1; k < 1 << shift; k++) if (mine) acc = __dadd_rn(acc, fold[(warp + k) * 32 + lane]);
+        }
+        if (!has) continue;
+        if constexpr (PART) __stcg(p.part + ((size_t)sp * p.M + n) * p.ldp + row, acc);
+        else p.y[(size_t)n * p.rows + row] = __double2float_rn(acc) + (p.bias ? __ldg(p.bias + row) : 0.f);
+    }
 }
 
 template <int KB, bool PART>
@@ -258,7 +351,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         };
         auto finish = [&](const Ends& e) -> bool {
             const Unit U = unit(e.u);
-            const int n0 = U.ts * T + wg * G, tg = min(min(T - wg * G, G), p.M - n0), row = U.rt * 128 + q * 32 + lane;       // tokens n0 .. n0 + tg
+            const int n0 = U.ts * T + wg * G, row = U.rt * 128 + q * 32 + lane;
+            const unsigned good = __ballot_sync(0xffffffffu, lane < min(min(T - wg * G, G), p.M - n0) && e.info >> 8 != kDigNone);        // tokens that are there and have digits
+            const bool has_row = row < p.rows && e.ew != kRowNone;     // (the others: sum_over_blocks)
             if (lane < G) {                                            // (with four planes sums are a high and a low part, units of 2^32 and of 1)
                 const int ex = e.info & 255;
                 if (planes == 3) table[lane] = make_longlong2(e.bias * kBias, PART ? (1023 - 50 + ex) << 20 : (127 - 50 + ex) << 23);
@@ -286,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                         const longlong2 tok = table[g + i];
                         long long v = (long long)((unsigned long long)(unsigned)d[4][i] << 32) - tok.x;
                         v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
-                        if (g + i < tg && row < p.rows) {
+                        if (has_row && good >> (g + i) & 1) {
                             if constexpr (PART) __stcg(part, __dmul_rn(__ll2double_rn(v), __hiloint2double((int)tok.y + (e.ew << 20), 0)));
                             // (times a power of two that leaves the result a normal number: the one rounding is the conversion's)
                             else *y = __fmul_rn(__ll2float_rn(v), __int_as_float((int)tok.y + (e.ew << 23))) + e.bv;
@@ -309,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                     hi += lo >> 32;                                    // below 2^36, and the rest of lo is 0 .. 2^32 - 1: the double rounds once
                     const double v = __fma_rn((double)hi, 0x1p32, (double)(unsigned)lo);
                     const int ex = ((int)tok.y & 255) + e.ew - 50;
-                    if (t < tg && row < p.rows) {
+                    if (has_row && good >> t & 1) {
                         if constexpr (PART) __stcg(part, __dmul_rn(v, __hiloint2double((1023 + ex) << 20, 0)));
                         else *y = __fmul_rn(__double2float_rn(v), __int_as_float((127 + ex) << 23)) + e.bv;
                     }
@@ -497,21 +592,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
-    // What the digits cannot hold, again and over the sums stored above.  (Behind the loops: a call inside them, taken or not, keeps their values
-    // out of half the registers.)
-    if (!p.bad_rows && !s_none) return;
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-        const Unit U = unit(u);
-        const int b0 = U.k0 * kStepBlk, b1 = min(U.k1 * kStepBlk, p.nb);
-        for (int i = tid; i < 128 * T; i += kThreads) {
-            const int row = U.rt * 128 + (i & 127), n = U.ts * T + (i >> 7);
-            if (row >= p.rows || n >= p.M) continue;
-            if (__ldg(p.row_exp + row) != kRowNone && (__ldcg(p.x.info + (size_t)U.sp * p.M + n) >> 8) != kDigNone) continue;
-            const double v = row_sum_dig<KB>(p, row, n, b0, b1);
-            if constexpr (PART) __stcg(p.part + ((size_t)U.sp * p.M + n) * p.ldp + row, v);
-            else p.y[(size_t)n * p.rows + row] = __double2float_rn(v) + (p.bias ? __ldg(p.bias + row) : 0.f);
-        }
-    }
+    // (behind the loops: a call inside them, taken or not, keeps their values out of half the registers)
+    if ((p.bad_rows || s_none) && !*abort_flag) sum_over_blocks<KB, PART>(p, smem, s_none);
 }
 
 // the digits of 16 elements, all planes
@@ -617,6 +699,11 @@ __global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base,
     if (row_exp[row] == kRowNone) atomicAdd(bad_rows, 1);
 }
 
+__global__ void __launch_bounds__(256) list_rows_kernel(const uint8_t* row_exp, int rows, int* list, int* count) {
+    const int row = blockIdx.x * 256 + threadIdx.x;
+    if (row < rows && row_exp[row] == kRowNone) list[atomicAdd(count, 1)] = row;
+}
+
 template <int KB, bool PART>
 int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
     const int units = (p.groups + 3) / 4 * p.x.TT * p.ksg;             // at least
@@ -634,7 +721,15 @@ int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
 }  // namespace
 
 // Token tiles and K ranges of a product over digits, the fewest clocks by a model from measured launches: 7000 until the first MMA, 290 per block or what its MMAs take,
-// 4000 and 80 per token for the end of a unit.
+// 4000 and 80 per token for the end of a unit; for rows without an exponent what sum_over_blocks takes, 480 per block and round of its jobs (it decides whether a
+// matrix with many such rows goes over digits at all; tokens without planes are known on the GPU only).
+static double rows_cost(long long jobs, int nblk, long long ctas) {
+    if (!jobs) return 0.0;
+    int shift = 0;
+    while (shift < 4 && jobs << (shift + 1) <= ctas * kExpWarps) shift++;
+    const long long at_once = ctas * (kExpWarps >> shift);
+    return 2000 + (double)((jobs + at_once - 1) / at_once) * ((nblk >> shift) + 1) * 480;
+}
 bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* out) {
     const int nst = (w->nb + kStepBlk - 1) / kStepBlk, rt = (w->groups + 3) / 4;
     const int TT = (M + kDigMaxT - 1) / kDigMaxT, T = ((M + TT - 1) / TT + 7) / 8 * 8;
@@ -645,7 +740,8 @@ bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* o
         const int steps = (nst + ksg - 1) / ksg;
         if (steps * kStepBlk * 32 > 16384) continue;                   // a sum of digit products stays below 2^31 (three pairs of 255 * 128 per element)
         const long long units = (long long)rt * TT * ksg, rounds = (units + ctx->sm_count - 1) / ctx->sm_count;
-        const double cost = 7000 + rounds * (std::min(steps * kStepBlk, w->nb) * blk + 4000 + 80.0 * T) + (part ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
+        const int nblk = std::min(steps * kStepBlk, w->nb);
+        const double cost = 7000 + rounds * (nblk * blk + 4000 + 80.0 * T) + rows_cost((long long)w->bad_rows * ksg * ((M + 31) / 32), nblk, std::min<long long>(units, ctx->sm_count)) + (part ? ksg * (double)M * w->rows * 16 / (ctx->sm_count * 40.0) : 0.0);
         if (cost < best) { best = cost; *out = DigPlan{T, TT, ksg, cost}; }
     }
     return best < 1e300;
@@ -655,8 +751,9 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
     DigParams p{};
     p.base = w->dev; p.row_exp = w->row_exp; p.groups = w->groups; p.nb = w->nb; p.nst = (w->nb + kStepBlk - 1) / kStepBlk; p.rows = (int)w->rows;
     p.ksg = pl.ksg; p.M = g.M;
-    p.x = x; p.q8 = g.x; p.bias = g.bias; p.y = g.y; p.part = g.part; p.ldp = g.ldp; p.err = ctx->d_err; p.bad_rows = w->bad_rows;
+    p.x = x; p.q8 = g.x; p.bias = g.bias; p.y = g.y; p.part = g.part; p.ldp = g.ldp; p.err = ctx->d_err; p.bad_list = w->bad_list; p.bad_rows = w->bad_rows;
     const bool part = mode == GEMM_PART;
+    if (p.M * p.ksg > kMaxInfo) return set_error(ctx, MI_ERR_LIMIT, "gemm: %d tokens in one launch", p.M);
     switch (w->kb) {
         case 8: return part ? launch_dig<8, true>(ctx, p, pdl) : launch_dig<8, false>(ctx, p, pdl);
         case 4: return part ? launch_dig<4, true>(ctx, p, pdl) : launch_dig<4, false>(ctx, p, pdl);
@@ -685,6 +782,12 @@ int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int*
         case 2: row_exponents_kernel<2><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
         default: row_exponents_kernel<1><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
     }
+    MI_CUDA(ctx, cudaGetLastError());
+    return MI_OK;
+}
+
+int launch_list_rows(mi_ctx* ctx, const mi_weight* w, int* list, int* count) {
+    if (w->rows > 0) list_rows_kernel<<<(unsigned)((w->rows + 255) / 256), 256, 0, ctx->stream>>>(w->row_exp, (int)w->rows, list, count);
     MI_CUDA(ctx, cudaGetLastError());
     return MI_OK;
 }

@@ -9,7 +9,7 @@ namespace mi {
 //     q    : [token tile of T][block of 32][row = plane * T + token, planes 0 .. 2, padded to a multiple of 16 rows] 32 bytes: the MMA's operand with the
 //            32-byte swizzle (the halves of rows 4 .. 7 of eight change places); behind all of it plane 3 as [token tile][block][token].  A token's block is a
 //            whole sector: without the swizzle it is two halves of sectors, which it took SwiGLU 31 us to write for 333 tokens of the 1.5B shape.
-//     info : [K range][token] ex | planes in use << 8 (3 or 4; kDigNone: the digits cannot hold it, see row_sum_dig)
+//     info : [K range][token] ex | planes in use << 8 (3 or 4; kDigNone: the digits cannot hold it, see sum_over_blocks)
 //     bias : [K range][token] sum of X
 struct DigX { uint8_t* q; int* info; long long* bias; int T, TT; };
 constexpr int kDigPlanes = 4, kDigNone = 255, kDigMaxT = 64;                          // tokens of a tile
@@ -75,7 +75,9 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
 int launch_tok_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const TokX& x, const DigX& out, int M, bool pdl);
 // The same behind SwiGLU: rows of y come as (gate, up) groups of 32, w is the matrix that takes its result; act: the result as q8_0
 int launch_swiglu_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const float* y, const TokX& act, const DigX& out, int M, bool pdl);
-// Exponents of a matrix's rows, for the product's weight digits: row_exp[groups * 32]; *bad_rows (zero before): mi_weight::bad_rows.
+// Exponents of a matrix's rows, for the product's weight digits: row_exp[groups * 32]; *bad_rows (zero before): how many have none.
 int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* bad_rows);
+// The rows that have none, in any order; *count: zero before
+int launch_list_rows(mi_ctx* ctx, const mi_weight* w, int* list, int* count);
 
 }  // namespace mi

@@ -328,13 +328,17 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     if ((st = plan_pass_products(ctx, mats, L, M, a.head == HEAD_NONE ? 0 : ML, &tiles, plans))) return st;
     const GemmPlan &po = plans[1], &pd = plans[3];
     xf.J = attf.J = actf.J = tiles.J();
-    // a product goes over digits where that is faster by the cost models (for the attention's output their own launch included: 4000 clocks)
+    // a product goes over digits where that is faster by the cost models (for the attention's output their own launch included: 4000 clocks), which depends on the
+    // layer's rows too: the plans of the layer under way
     DigPlan dp[5];
     bool dig[5];
-    for (int i = 0; i < 5; i++) {
+    int planned[5] = {-1, -1, -1, -1, -1};                             // rows out of the digits' range that dp and dig are for
+    auto plan = [&](int i, const mi_weight* w) {
+        if (planned[i] == w->bad_rows) return;
         const int Mi = i == 4 ? ML : M;
-        dig[i] = Mi > kMaxFusedTok && m->products >= 0 && plan_gemm_dig(ctx, mats[i], i == 1 || i == 3, Mi, &dp[i]) && (m->products > 0 || dp[i].cost + (i == 1 ? 4000 : 0) < plans[i].cost);
-    }
+        dig[i] = Mi > kMaxFusedTok && m->products >= 0 && plan_gemm_dig(ctx, w, i == 1 || i == 3, Mi, &dp[i]) && (m->products > 0 || dp[i].cost + (i == 1 ? 4000 : 0) < plans[i].cost);
+        planned[i] = w->bad_rows;
+    };
     auto digits_for = [&](int i) { return dig[i] ? DigX{b.dig, b.dig_info, b.dig_bias, dp[i].T, dp[i].TT} : DigX{nullptr, nullptr, nullptr, 1, 1}; };
     // The product over digits has them from the kernel that makes its activations, but for the attention's output.
     auto product = [&](int i, const mi_weight* w, int mode, const GemmParams& gp) -> int {
@@ -342,7 +346,7 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         if (i == 1) { const int s = launch_tok_digits(ctx, w, dp[i], gp.x, digits_for(i), gp.M, pdl); if (s) return s; }
         return launch_gemm_dig(ctx, w, dp[i], mode, digits_for(i), gp, pdl);
     };
-    const int o_ranges = dig[1] ? dp[1].ksg : po.ksg, d_ranges = dig[3] ? dp[3].ksg : pd.ksg;
+    int d_ranges = 0;                                                  // K ranges of the down projection before
     const int nt_norm = std::min(1024, (E / 4 + 31) / 32 * 32);
     GemmParams g{};
     g.M = M;
@@ -354,7 +358,8 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     };
     for (int l = 0; l < L; l++) {
         const mi_weight *wqkv = &m->views[4 * l], *wo = &m->views[4 * l + 1], *wgu = &m->views[4 * l + 2], *wdn = &m->views[4 * l + 3];
-        if ((st = norm(l == 0, 0, M, l == 0 ? 0 : d_ranges, lp[l].attn_norm, xf, digits_for(0)))) return st;
+        plan(0, wqkv); plan(1, wo); plan(2, wgu); plan(3, wdn);
+        if ((st = norm(l == 0, 0, M, d_ranges, lp[l].attn_norm, xf, digits_for(0)))) return st;
         GemmParams gq = g;
         gq.x = xf; gq.bias = lp[l].bqkv; gq.y = b.Y;
         gq.rope = RopeParams{b.q, NQ, m->HD, P.kc, P.vc, m->KVD, a.slab_stride, l, a.max_seq, P.rope_cs, P.rope_freq, P.rope_rows, pos0, pos_arr, slot_arr};
@@ -364,15 +369,17 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
         if ((st = launch_attn_tok(ctx, at, pa, pdl))) return st;
         GemmParams go = g; go.x = attf; go.part = b.part; go.ldp = b.ldp;
         if ((st = product(1, wo, GEMM_PART, go))) return st;
-        if ((st = norm(false, 0, M, o_ranges, lp[l].ffn_norm, xf, digits_for(2)))) return st;
+        if ((st = norm(false, 0, M, dig[1] ? dp[1].ksg : po.ksg, lp[l].ffn_norm, xf, digits_for(2)))) return st;
         GemmParams gg = g; gg.x = xf; gg.act = actf; gg.y = b.Y;
         if ((st = product(2, wgu, fused ? GEMM_GU : GEMM_PLAIN, gg))) return st;
         if (dig[3]) { if ((st = launch_swiglu_digits(ctx, wdn, dp[3], b.Y, actf, digits_for(3), M, pdl))) return st; }
         else if (!fused) MI_CUDA(ctx, launch_k(pdl, vf_swiglu, dim3((m->FF / 32 + 7) / 8, M), dim3(256), 0, ctx->stream, (const float*)b.Y, m->FF, actf));
         GemmParams gd = g; gd.x = actf; gd.part = b.part; gd.ldp = b.ldp;
         if ((st = product(3, wdn, GEMM_PART, gd))) return st;
+        d_ranges = dig[3] ? dp[3].ksg : pd.ksg;
     }
     if (a.head == HEAD_NONE) return MI_OK;
+    plan(4, &m->views[4 * L]);
     TokX lf = b.xf; lf.J = ML == M ? tiles.J() : tok_tiling(ML).J();
     if ((st = norm(false, M - ML, ML, d_ranges, m->P.out_norm, lf, digits_for(4)))) return st;
     GemmParams gl = g; gl.M = ML; gl.x = lf; gl.y = b.logits;

@@ -188,3 +188,70 @@ def test_sums_beyond_64_bits_over_ranges(ctx, pkg, tmp_path, spread, signs, ff, 
     rewrite(path, blk__0__attn_output__weight=nothing, blk__0__ffn_gate__weight=gate, blk__0__ffn_up__weight=up, blk__0__ffn_down__weight=down, blk__0__ffn_norm__weight=ones,
             **({"token_embd__weight": embedding, "output__weight": embedding} if signs == "one" else {}))
     same(ctx, pkg, path, n, 600)
+
+
+# Some rows and some tokens out of the digits' range, the rest within: one of each, a half, several rounds of the warps that sum them, all; every tile depth
+@pytest.mark.parametrize("embd,ff", [(192, 352), (320, 1376), (384, 256), (512, 1024)])
+@pytest.mark.parametrize("n,rows,tokens", [(20, 1, 0), (40, 0, 1), (64, 1, 1), (64, 9, 0), (64, 70, 3), (64, 0, 7), (65, 17, 20), (130, 400, 33), (24, 2, 24)])
+def test_rows_and_tokens_out_of_range(ctx, pkg, tmp_path, embd, ff, n, rows, tokens):
+    V = 600
+    path = gu.make_synthetic(tmp_path / "m.gguf", "tiny", seed=embd + n, std=2.0, extra=["--layers", 2, "--embd", embd, "--heads", embd // 32, "--kv-heads", embd // 64, "--ff", ff, "--vocab", V, "--untied"])
+    rng = np.random.default_rng(n + rows)
+
+    def wide(d, q):
+        r = rng.permutation(len(d))[:rows]
+        d[r, -1] = lower(d[r, -1], 12)
+
+    def embedding(d, q):                                              # the tokens that `same` draws last
+        ids = np.random.default_rng(n).integers(0, V, n)[n - tokens:] if tokens else []
+        for t in ids:
+            d[t] += 4 << 10
+            d[t, 1] = d[t, 1] & 0x8000 | 1 << 10
+
+    def norm(w):
+        w[:] = 200.0                                                  # the largest blocks' scales are above one, so that 2^-14 of them is not subnormal
+
+    rewrite(path, token_embd__weight=embedding, blk__0__attn_norm__weight=norm, blk__0__ffn_norm__weight=norm, output_norm__weight=norm,
+            **{t: wide for t in ("blk__0__attn_q__weight", "blk__0__attn_output__weight", "blk__1__ffn_up__weight", "blk__0__ffn_down__weight", "output__weight")})
+    same(ctx, pkg, path, n, V)
+
+
+# What is out of range must not cost more than the product over blocks: one token of a pass whose normed inputs are, and 1 % of every matrix's rows
+@pytest.mark.parametrize("preset,n", [("1.5b", 333), ("3b", 64)])
+@pytest.mark.parametrize("what", ["token", "rows"])
+def test_time_of_passes_out_of_range(ctx, pkg, tmp_path, preset, n, what):
+    std = 0.02 if what == "token" else 64.0
+    path = gu.make_synthetic(tmp_path / "m.gguf", preset, seed=6, std=std, extra=["--layers", 3, "--vocab", 1500, "--untied"])
+
+    def nothing(d, q):
+        d[:] = 0
+
+    def embedding(d, q):
+        d[7] += 4 << 10
+        d[7, 1] = d[7, 1] & 0x8000 | 1 << 10
+
+    def wide(d, q):
+        d[::100, 1] = lower(d[::100, 1], 18)
+
+    def norm(w):
+        w[:] = 4.0 / std
+
+    rewrite(path, **{f"blk__{l}__{t}__weight": norm for l in range(3) for t in ("attn_norm", "ffn_norm")})
+    if what == "token":                                               # (layers that add nothing: the norms see the embedding)
+        rewrite(path, token_embd__weight=embedding, **{f"blk__{l}__{t}__weight": nothing for l in range(3) for t in ("attn_output", "ffn_down")})
+    else:
+        rewrite(path, **{f"blk__{l}__{t}__weight": wide for l in range(3) for t in ("attn_q", "attn_output", "ffn_gate", "ffn_up", "ffn_down")})
+    m = pkg.Model(ctx, path, 400)
+    seq = [7 if i == 10 else 8 + i for i in range(n)]
+    ms = {}
+    for which in (-1, 0):
+        m.debug_products(which)
+        if n > 64:
+            ms[which] = min(m.prefill(seq, 0)[1] for _ in range(12))
+        else:
+            b = pkg.Batch(m, n, 8)
+            ms[which] = min(b.step(seq, list(range(n)), [3] * n)[1] for _ in range(12))
+            b.free()
+    m.free()
+    print(ms)
+    assert ms[0] < 1.03 * ms[-1], ms
