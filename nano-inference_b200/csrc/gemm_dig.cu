@@ -747,6 +747,15 @@ bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* o
     return best < 1e300;
 }
 
+// Where the line lies: both products' cost models, corrected by passes of 17 to 512 tokens of the 0.5B, 1.5B and 3B shapes, each timed with one product at a time over
+// digits.  The block product takes a tenth more than its model says; digits of the attention's output (a launch of their own) and of SwiGLU's cost 28 clocks a token
+// (333 tokens: 5 us), the lm_head over digits 15 us more than its model says.  Of 3 x 31 passes the rule loses 0.1 us a layer against the better choice
+// of each product, 4.7 of 149 at most (the 3B shape's QKV at 72 tokens).
+bool choose_gemm_dig(mi_ctx* ctx, const mi_weight* w, int i, int M, const GemmPlan& blocks, DigPlan* out) {
+    const bool part = i == 1 || i == 3;
+    return M > kMaxFusedTok && plan_gemm_dig(ctx, w, part, M, out) && out->cost + (part ? 28.0 * M : i == 4 ? 28500.0 : 0.0) < 1.1 * blocks.cost;
+}
+
 int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode, const DigX& x, GemmParams g, bool pdl) {
     DigParams p{};
     p.base = w->dev; p.row_exp = w->row_exp; p.groups = w->groups; p.nb = w->nb; p.nst = (w->nb + kStepBlk - 1) / kStepBlk; p.rows = (int)w->rows;

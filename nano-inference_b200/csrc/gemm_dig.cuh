@@ -70,6 +70,8 @@ struct DigRange {
 // How a product of M tokens is cut: token tiles, K ranges.
 struct DigPlan { int T, TT, ksg; double cost; };
 bool plan_gemm_dig(mi_ctx* ctx, const mi_weight* w, bool part, int M, DigPlan* out);
+// Whether product i of a pass (0 QKV, 1 O, 2 gate/up, 3 down, 4 lm_head) over M tokens goes over digits, and how: `blocks` is the plan it has otherwise.
+bool choose_gemm_dig(mi_ctx* ctx, const mi_weight* w, int i, int M, const GemmPlan& blocks, DigPlan* out);
 // y = fp32(sum) + bias (GEMM_PLAIN), or double sums per K range (GEMM_PART); x: the digits, p.x: the same activations as q8_0
 int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode, const DigX& x, GemmParams p, bool pdl);
 int launch_tok_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const TokX& x, const DigX& out, int M, bool pdl);

@@ -328,15 +328,14 @@ int enqueue_pass(mi_ctx* ctx, mi_model* m, const Pass& a) {
     if ((st = plan_pass_products(ctx, mats, L, M, a.head == HEAD_NONE ? 0 : ML, &tiles, plans))) return st;
     const GemmPlan &po = plans[1], &pd = plans[3];
     xf.J = attf.J = actf.J = tiles.J();
-    // a product goes over digits where that is faster by the cost models (for the attention's output their own launch included: 4000 clocks), which depends on the
-    // layer's rows too: the plans of the layer under way
+    // the plans of the layer under way: which product goes over digits depends on the layer's rows too
     DigPlan dp[5];
     bool dig[5];
     int planned[5] = {-1, -1, -1, -1, -1};                             // rows out of the digits' range that dp and dig are for
     auto plan = [&](int i, const mi_weight* w) {
         if (planned[i] == w->bad_rows) return;
         const int Mi = i == 4 ? ML : M;
-        dig[i] = Mi > kMaxFusedTok && m->products >= 0 && plan_gemm_dig(ctx, w, i == 1 || i == 3, Mi, &dp[i]) && (m->products > 0 || dp[i].cost + (i == 1 ? 4000 : 0) < plans[i].cost);
+        dig[i] = m->products == 0 ? choose_gemm_dig(ctx, w, i, Mi, plans[i], &dp[i]) : m->products > 0 && Mi > kMaxFusedTok && plan_gemm_dig(ctx, w, i == 1 || i == 3, Mi, &dp[i]);
         planned[i] = w->bad_rows;
     };
     auto digits_for = [&](int i) { return dig[i] ? DigX{b.dig, b.dig_info, b.dig_bias, dp[i].T, dp[i].TT} : DigX{nullptr, nullptr, nullptr, 1, 1}; };
