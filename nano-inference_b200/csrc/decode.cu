@@ -386,21 +386,21 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         size_t rows = 0;
         for (const mi_weight& v : m->views) rows += (size_t)v.groups * 32;
         uint8_t* d_exp; int* d_bad;
-        if ((st = dev_alloc(ctx, m, &d_exp, rows)) || (st = dev_alloc(ctx, m, &d_bad, m->views.size()))) return st;
+        if ((st = dev_alloc(ctx, m, &d_exp, rows)) || (st = dev_alloc(ctx, m, &d_bad, 2 * m->views.size()))) return st;
         for (size_t i = 0; i < m->views.size(); i++) {
             m->views[i].row_exp = d_exp;
-            if ((st = launch_row_exponents(ctx, &m->views[i], d_exp, d_bad + i))) return st;
+            if ((st = launch_row_exponents(ctx, &m->views[i], d_exp, d_bad + 2 * i))) return st;
             d_exp += (size_t)m->views[i].groups * 32;
         }
-        std::vector<int> bad(m->views.size());
+        std::vector<int> bad(2 * m->views.size());
         MI_CUDA(ctx, cudaMemcpyAsync(bad.data(), d_bad, bad.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         for (size_t i = 0; i < m->views.size(); i++) {
             mi_weight& v = m->views[i];
-            v.bad_rows = bad[i];
-            if (!bad[i]) continue;
+            v.bad_rows = bad[2 * i]; v.row_spread = bad[2 * i + 1];
+            if (!v.bad_rows) continue;
             int* list;
-            if ((st = dev_alloc(ctx, m, &list, (size_t)bad[i] + 1)) || (st = launch_list_rows(ctx, &v, list, list + bad[i]))) return st;
+            if ((st = dev_alloc(ctx, m, &list, (size_t)v.bad_rows + 1)) || (st = launch_list_rows(ctx, &v, list, list + v.bad_rows))) return st;
             v.bad_list = list;
         }
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -8,8 +8,9 @@
 // put together as one integer and rounded once.  9 products at the int8 rate are 0.035 clocks of an SM per (row, block, token), the two FP64 operations 0.031; but
 // the tensor core needs no issue slots beside it.  The digits hold any row whose scales lie at most 8 binades apart and any token with at most 13 (5 with three
 // planes); other rows and tokens, and scales that are not finite, are summed block by block behind the main loop.  How large the integer gets: a weight is below
-// 8 * 2^11 * 2^8 units, an activation 2^7 * 2^11 * 2^5 with three planes and 2^13 in place of 2^5 with four, so K = 2^14 elements sum to less than 2^59 and 2^67: one
-// 64-bit number holds the former, two of them the latter.
+// 2^(14 + s) units, s the binades between its row's scales (at most 8), an activation below 2^(18 + 5) with three planes and 2^(18 + 13) with four, so K = 2^k elements sum to
+// less than 2^(37 + s + k) and 2^(45 + s + k).  The former is below 2^59 for all K; where the latter is above 2^63 (s > 7 for K = 2048), sums of launches with four planes are two
+// numbers.
 //
 // Dataflow of a CTA (one per SM, a unit is 128 rows x T <= 64 tokens x one K range):
 //   copies     : one warp streams the q4_0 tiles (bulk copies, ahead of the wait for the predecessor), one the activation planes, four blocks at a time;
@@ -18,11 +19,13 @@
 //                that the way from a freed stage to a full one is a store and two barriers;
 //   one warp   : issues the MMAs; the whole warp runs the loop, one lane issues (see there);
 //   the 16 warps again at the end of a unit, when the first stages of the next one are in place.
-// Measured (event time, launches back to back): gate/up of 333 tokens (17920 x 1536) 74 us against 123 for the product over blocks, down (1536 x 8960) 36 / 64, batch of 64
-// on 22016 x 2048 35 / 49, 2048 x 11008 19 / 29, 151936 x 2048 133 / 250; it loses at 32 tokens on 22016 x 2048 (32 / 31), at 16 (31 / 19) and at 2560 x 2048 x 64 (20 / 15).  A stage of two blocks takes 620 clocks at 64 tokens, its MMAs 576;
+// Measured (event time, launches back to back, each ahead of its predecessor's end): gate/up of 333 tokens (17920 x 1536) 71 us against 121 for the product over blocks, 82 with
+// four planes, down (1536 x 8960) 32 / 63, batch of 64 on 22016 x 2048 31 / 46, 2048 x 11008 16 / 26, 151936 x 2048 128 / 246; it is even at 32 tokens on 22016 x 2048 (29 / 29),
+// loses at 16 (28 / 19) and at 2560 x 2048 x 64 (17 / 12).  A stage of two blocks takes 620 clocks at 64 tokens, its MMAs 576;
 // the rest is the start (7000 clocks until the first MMA) and the end of a unit (6000).  Tried: weights expanded weight by weight or in byte lanes with seven sums per
 // token (the expansion or the tensor memory is full first), stages of one and four blocks, eight expanding warps, results through arrays in
-// registers (spills): 95 to 210 us for the gate/up.  Carry additions moved to the multiplier's pipe: no change, both sides in turn on one GPU.
+// registers (spills): 95 to 210 us for the gate/up.  Carry additions moved to the multiplier's pipe: no change, both sides in turn on one GPU.  A fourth weight digit for
+// rows of 9 to 16 binades (95 us for the gate/up, however many): half of the instantiations for rows that cost less block by block up to 2 % of them, and go over blocks from 4 % on.
 #include "gemm_dig.cuh"
 #include <algorithm>
 #include <atomic>
@@ -236,7 +239,8 @@ static __device__ __forceinline__ void sum_over_blocks(const DigParams& p, uint8
     }
 }
 
-template <int KB, bool PART>
+// TWO: sums of four planes in two parts (a form of its own: they take a tenth longer, 333 tokens on 17920 x 1536 91 us instead of 83)
+template <int KB, bool PART, bool TWO>
 __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_constant__ DigParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (0u - smem_u32(smem_raw) & 255u);          // the swizzle goes by address bits
@@ -321,6 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
     __syncthreads();
     tc_fence_after();
     const int planes = (int)__reduce_max_sync(0xffffffffu, (unsigned)s_planes);
+    const bool two_parts = TWO && planes == 4;
     const int T = p.x.T, units = p.ksg * row_tiles * p.x.TT, N = planes == 4 ? 4 * T : dig_rows(T);
     // tensor memory: sums of weight 256^s in columns s * T .. (the MMAs of a token tile of an odd number of eights reach eight columns further), stages of weight
     // digits at the end
@@ -352,11 +357,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
         auto finish = [&](const Ends& e) -> bool {
             const Unit U = unit(e.u);
             const int n0 = U.ts * T + wg * G, row = U.rt * 128 + q * 32 + lane;
-            const unsigned good = __ballot_sync(0xffffffffu, lane < min(min(T - wg * G, G), p.M - n0) && e.info >> 8 != kDigNone);        // tokens that are there and have digits
-            const bool has_row = row < p.rows && e.ew != kRowNone;     // (the others: sum_over_blocks)
-            if (lane < G) {                                            // (with four planes sums are a high and a low part, units of 2^32 and of 1)
+            // tokens that are there and have digits, for a row that has (the others: sum_over_blocks)
+            unsigned good = __ballot_sync(0xffffffffu, lane < min(min(T - wg * G, G), p.M - n0) && e.info >> 8 != kDigNone);
+            if (row >= p.rows || e.ew == kRowNone) good = 0;
+            if (lane < G) {                                            // (two parts: units of 2^32 and of 1)
                 const int ex = e.info & 255;
-                if (planes == 3) table[lane] = make_longlong2(e.bias * kBias, PART ? (1023 - 50 + ex) << 20 : (127 - 50 + ex) << 23);
+                if (!two_parts) table[lane] = make_longlong2((long long)((unsigned long long)e.bias * (unsigned long long)kBias), PART ? (1023 - 50 + ex) << 20 : (127 - 50 + ex) << 23);
                 else table[lane] = make_longlong2((long long)(unsigned)e.bias * kBias, (e.bias >> 32) * kBias << 8 | ex);
             }
             __syncwarp();
@@ -366,22 +372,30 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
             float* y = p.y + (size_t)n0 * p.rows + row;
             double* part = p.part + ((size_t)U.sp * p.M + n0) * p.ldp + row;
             const int mine = min(T - wg * G, G);
-            if (planes == 3) {
+            if (!two_parts) {
                 #pragma unroll 1
                 for (int g = 0; g < mine; g += 4) {                    // (rolled: four tokens at a time fit the registers and the instruction cache)
                     const uint32_t a = trow + wg * G + g;
                     int d[kNW + 2][4];
+                    unsigned high[4] = {0, 0, 0, 0};
+                    if (planes == 4) {
+                        tmem_ld4(a + (kNW + 2) * T, d[0]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        #pragma unroll
+                        for (int i = 0; i < 4; i++) high[i] = (unsigned)d[0][i] << 8;
+                    }
                     #pragma unroll
                     for (int i = 0; i < kNW + 2; i++) tmem_ld4(a + i * T, d[i]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     #pragma unroll
                     for (int i = 0; i < kNW + 2; i++) tmem_zero4(a + i * T);       // for the next unit
+                    if (planes == 4) tmem_zero4(a + (kNW + 2) * T);
                     #pragma unroll
-                    for (int i = 0; i < 4; i++) {                      // the sum is below 2^59, whatever its parts are
+                    for (int i = 0; i < 4; i++) {                      // the sum is below 2^63, whatever its parts are
                         const longlong2 tok = table[g + i];
-                        long long v = (long long)((unsigned long long)(unsigned)d[4][i] << 32) - tok.x;
+                        long long v = (long long)((unsigned long long)(high[i] + (unsigned)d[4][i]) << 32) - tok.x;
                         v = mad_wide(d[0][i], 1, v); v = mad_wide(d[1][i], 1 << 8, v); v = mad_wide(d[2][i], 1 << 16, v); v = mad_wide(d[3][i], 1 << 24, v);
-                        if (has_row && good >> (g + i) & 1) {
+                        if (good >> (g + i) & 1) {
                             if constexpr (PART) __stcg(part, __dmul_rn(__ll2double_rn(v), __hiloint2double((int)tok.y + (e.ew << 20), 0)));
                             // (times a power of two that leaves the result a normal number: the one rounding is the conversion's)
                             else *y = __fmul_rn(__ll2float_rn(v), __int_as_float((int)tok.y + (e.ew << 23))) + e.bv;
@@ -404,7 +418,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_dig_kernel(const __grid_cons
                     hi += lo >> 32;                                    // below 2^36, and the rest of lo is 0 .. 2^32 - 1: the double rounds once
                     const double v = __fma_rn((double)hi, 0x1p32, (double)(unsigned)lo);
                     const int ex = ((int)tok.y & 255) + e.ew - 50;
-                    if (has_row && good >> t & 1) {
+                    if (good >> t & 1) {
                         if constexpr (PART) __stcg(part, __dmul_rn(v, __hiloint2double((1023 + ex) << 20, 0)));
                         else *y = __fmul_rn(__double2float_rn(v), __int_as_float((127 + ex) << 23)) + e.bv;
                     }
@@ -683,7 +697,7 @@ __global__ void __launch_bounds__(kSwiWarps * 32) swiglu_digits_kernel(const flo
 
 // One warp per row
 template <int KB>
-__global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base, int groups, int nb, uint8_t* row_exp, int* bad_rows) {
+__global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base, int groups, int nb, uint8_t* row_exp, int* found) {
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= groups * 32) return;
     int lo = 31, hi = 0;
@@ -696,7 +710,8 @@ __global__ void __launch_bounds__(256) row_exponents_kernel(const uint8_t* base,
     if (lane) return;
     lo = min(lo, max(hi, 1));
     row_exp[row] = hi == 31 || hi - lo > kMaxSpread ? kRowNone : lo;
-    if (row_exp[row] == kRowNone) atomicAdd(bad_rows, 1);
+    if (row_exp[row] == kRowNone) atomicAdd(found, 1);
+    else if (hi - lo > found[1]) atomicMax(found + 1, hi - lo);
 }
 
 __global__ void __launch_bounds__(256) list_rows_kernel(const uint8_t* row_exp, int rows, int* list, int* count) {
@@ -704,10 +719,10 @@ __global__ void __launch_bounds__(256) list_rows_kernel(const uint8_t* row_exp, 
     if (row < rows && row_exp[row] == kRowNone) list[atomicAdd(count, 1)] = row;
 }
 
-template <int KB, bool PART>
+template <int KB, bool PART, bool TWO>
 int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
     const int units = (p.groups + 3) / 4 * p.x.TT * p.ksg;             // at least
-    auto kern = gemm_dig_kernel<KB, PART>;
+    auto kern = gemm_dig_kernel<KB, PART, TWO>;
     static std::mutex mu;
     static std::atomic<unsigned> raised{0};                   // bit per device
     if (!(raised.load(std::memory_order_acquire) >> (ctx->device & 31) & 1u)) {
@@ -718,6 +733,12 @@ int launch_dig(mi_ctx* ctx, const DigParams& p, bool pdl) {
     MI_CUDA(ctx, launch_k(pdl, kern, dim3((unsigned)std::min(units, ctx->sm_count)), dim3(kThreads), Smem::bytes, ctx->stream, p));
     return MI_OK;
 }
+template <int KB>
+int launch_kb(mi_ctx* ctx, const DigParams& p, bool part, bool two, bool pdl) {
+    if (two) return part ? launch_dig<KB, true, true>(ctx, p, pdl) : launch_dig<KB, false, true>(ctx, p, pdl);
+    return part ? launch_dig<KB, true, false>(ctx, p, pdl) : launch_dig<KB, false, false>(ctx, p, pdl);
+}
+
 }  // namespace
 
 // Token tiles and K ranges of a product over digits, the fewest clocks by a model from measured launches: 7000 until the first MMA, 290 per block or what its MMAs take,
@@ -760,14 +781,17 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
     DigParams p{};
     p.base = w->dev; p.row_exp = w->row_exp; p.groups = w->groups; p.nb = w->nb; p.nst = (w->nb + kStepBlk - 1) / kStepBlk; p.rows = (int)w->rows;
     p.ksg = pl.ksg; p.M = g.M;
+    int bits = 45 + w->row_spread;                                     // of a sum of one element, four planes
+    for (int k = std::min((p.nst + pl.ksg - 1) / pl.ksg * kStepBlk, w->nb) * 32; k > 1; k = (k + 1) / 2) bits++;
+    const bool two = bits > 63;
     p.x = x; p.q8 = g.x; p.bias = g.bias; p.y = g.y; p.part = g.part; p.ldp = g.ldp; p.err = ctx->d_err; p.bad_list = w->bad_list; p.bad_rows = w->bad_rows;
     const bool part = mode == GEMM_PART;
     if (p.M * p.ksg > kMaxInfo) return set_error(ctx, MI_ERR_LIMIT, "gemm: %d tokens in one launch", p.M);
     switch (w->kb) {
-        case 8: return part ? launch_dig<8, true>(ctx, p, pdl) : launch_dig<8, false>(ctx, p, pdl);
-        case 4: return part ? launch_dig<4, true>(ctx, p, pdl) : launch_dig<4, false>(ctx, p, pdl);
-        case 2: return part ? launch_dig<2, true>(ctx, p, pdl) : launch_dig<2, false>(ctx, p, pdl);
-        default: return part ? launch_dig<1, true>(ctx, p, pdl) : launch_dig<1, false>(ctx, p, pdl);
+        case 8: return launch_kb<8>(ctx, p, part, two, pdl);
+        case 4: return launch_kb<4>(ctx, p, part, two, pdl);
+        case 2: return launch_kb<2>(ctx, p, part, two, pdl);
+        default: return launch_kb<1>(ctx, p, part, two, pdl);
     }
 }
 
@@ -782,14 +806,14 @@ int launch_swiglu_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, con
     return MI_OK;
 }
 
-int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* bad_rows) {
+int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* found) {
     const dim3 grid((unsigned)(w->groups * 4));
     if (w->groups == 0) return MI_OK;
     switch (w->kb) {
-        case 8: row_exponents_kernel<8><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
-        case 4: row_exponents_kernel<4><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
-        case 2: row_exponents_kernel<2><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
-        default: row_exponents_kernel<1><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, bad_rows); break;
+        case 8: row_exponents_kernel<8><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, found); break;
+        case 4: row_exponents_kernel<4><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, found); break;
+        case 2: row_exponents_kernel<2><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, found); break;
+        default: row_exponents_kernel<1><<<grid, 256, 0, ctx->stream>>>(w->dev, w->groups, w->nb, row_exp, found); break;
     }
     MI_CUDA(ctx, cudaGetLastError());
     return MI_OK;

@@ -77,8 +77,8 @@ int launch_gemm_dig(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, int mode
 int launch_tok_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const TokX& x, const DigX& out, int M, bool pdl);
 // The same behind SwiGLU: rows of y come as (gate, up) groups of 32, w is the matrix that takes its result; act: the result as q8_0
 int launch_swiglu_digits(mi_ctx* ctx, const mi_weight* w, const DigPlan& pl, const float* y, const TokX& act, const DigX& out, int M, bool pdl);
-// Exponents of a matrix's rows, for the product's weight digits: row_exp[groups * 32]; *bad_rows (zero before): how many have none.
-int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* bad_rows);
+// Exponents of a matrix's rows, for the product's weight digits: row_exp[groups * 32]; found (zeros before): how many have none, the most binades between the scales of another.
+int launch_row_exponents(mi_ctx* ctx, const mi_weight* w, uint8_t* row_exp, int* found);
 // The rows that have none, in any order; *count: zero before
 int launch_list_rows(mi_ctx* ctx, const mi_weight* w, int* list, int* count);
 

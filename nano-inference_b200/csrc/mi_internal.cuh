@@ -43,7 +43,7 @@ struct mi_weight {
     int nb = 0, kb = 0, nt = 0, groups = 0;
     size_t mat_stride = 0, bytes = 0;
     uint8_t* dev = nullptr;
-    const uint8_t* row_exp = nullptr; const int* bad_list = nullptr; int bad_rows = 0;      // of a model's matrices: exponents of the rows, and which have none (gemm_dig.cuh)
+    const uint8_t* row_exp = nullptr; const int* bad_list = nullptr; int bad_rows = 0, row_spread = 0;      // of a model's matrices: exponents of the rows, which have none; launch_row_exponents
 };
 
 namespace mi {

@@ -12,8 +12,8 @@
 // and finally norm+q8 -> lm_head product -> greedy pick per token.  Every token goes through the
 // expressions of the single-token decode kernel (same quantizer, same sums carried in double), so its
 // logits do not depend on how many tokens share the pass.
-// Above 16 tokens RoPE and SwiGLU are kernels of their own, and each product goes over digits (gemm_dig.cu) where its cost is below the block
-// product's (333 tokens of the 1.5B shape 8040 -> 5718 us, 64 sequences of the 3B shape 4657 -> 3674); the kernel before it then writes the digits.
+// Above 16 tokens RoPE and SwiGLU are kernels of their own, and each product goes over digits (gemm_dig.cu) where that is faster (choose_gemm_dig;
+// 333 tokens of the 1.5B shape 8040 -> 5718 us, 64 sequences of the 3B shape 4657 -> 3674); the kernel before it then writes the digits.
 #include "model.cuh"
 #include "attn_tok.cuh"
 

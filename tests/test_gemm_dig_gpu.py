@@ -109,18 +109,18 @@ def test_digit_product_on_model_shapes(ctx, pkg, tmp_path, preset, n):
 
 
 # The widest rows against the widest tokens that the digits hold: all blocks at the top of the range but one at its bottom, sums of one sign (every weight -8 or 7, every
-# activation the block's largest) and random ones.  The integer sum of such a row passes 2^63.  Both products round a sum that wide to 53 bits on the way,
-# the block product at every addition, this one once; what is compared is the fp32 value.
+# activation the block's largest) and random ones.  The integer sum of such a row passes 2^63 (8 binades; with 7 at up to 2048 elements and 5 at 8192 it stays just
+# below).  Both products round a sum that wide to 53 bits on the way, the block product at every addition, this one once; what is compared is the fp32 value.
 def top_but_one(d, low, spread):
     """exponent fields low + spread, one block of a row low; signs and mantissas as they are"""
     d[:] = (d & 0x83FF) | ((low + spread) << 10)
     d[:, 5] = (d[:, 5] & 0x83FF) | (low << 10)
 
 
-@pytest.mark.parametrize("spread", [8, 16])
+@pytest.mark.parametrize("spread", [5, 7, 8, 16])
 @pytest.mark.parametrize("signs", ["one", "random"])
 @pytest.mark.parametrize("embd", [1536, 2048, 8192])
-@pytest.mark.parametrize("n", [40, 64])
+@pytest.mark.parametrize("n", [24, 40, 56, 64])
 def test_sums_beyond_64_bits(ctx, pkg, tmp_path, spread, signs, embd, n):
     """lm_head on the embedding itself (the layer adds nothing)"""
     path = gu.make_synthetic(tmp_path / "m.gguf", "tiny", seed=3, std=0.5, extra=["--layers", 1, "--embd", embd, "--heads", embd // 128, "--kv-heads", 8 if embd > 2048 else 2, "--ff", 256, "--vocab", 600, "--untied"])
@@ -149,11 +149,10 @@ def test_sums_beyond_64_bits(ctx, pkg, tmp_path, spread, signs, embd, n):
 
 @pytest.mark.parametrize("spread", [8, 16])
 @pytest.mark.parametrize("signs", ["one", "random"])
-@pytest.mark.parametrize("ff", [1536, 8960, 16384])
-@pytest.mark.parametrize("n", [40, 64, 120])
-def test_sums_beyond_64_bits_over_ranges(ctx, pkg, tmp_path, spread, signs, ff, n):
+@pytest.mark.parametrize("embd,ff,n", [(512, ff, n) for ff in (1536, 8960, 16384) for n in (24, 40, 64, 120)] + [(2048, 16384, 512)])       # (the last: all of K in one range)
+def test_sums_beyond_64_bits_over_ranges(ctx, pkg, tmp_path, spread, signs, embd, ff, n):
     """down projection: one gate for all, so that SwiGLU's result is that gate times the up rows"""
-    path = gu.make_synthetic(tmp_path / "m.gguf", "tiny", seed=4, std=0.5, extra=["--layers", 1, "--embd", 512, "--heads", 8, "--kv-heads", 4, "--ff", ff, "--vocab", 600])
+    path = gu.make_synthetic(tmp_path / "m.gguf", "tiny", seed=4, std=0.5, extra=["--layers", 1, "--embd", embd, "--heads", embd // 64, "--kv-heads", embd // 128, "--ff", ff, "--vocab", 600])
 
     def nothing(d, q):
         d[:] = 0
