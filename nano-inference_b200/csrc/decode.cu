@@ -115,7 +115,7 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
     void (*kern)(DecodeParams, int, int, int, int) = nullptr;
     // every step of this launch ends within the range the dedicated attention CTAs handle, on a shape the short-context
     // build takes: that build has no other attention variant in it (decode_lean.cu)
-    const int shape = getenv("MINFER_NO_LEAN") ? 0 : lean_shape(m->E, m->FF, m->NH * m->HD);
+    const int shape = getenv("MINFER_NO_LEAN") || !m->one_batch ? 0 : lean_shape(m->E, m->FF, m->NH * m->HD);
     const bool shape_ok = shape != 0;
     const bool by_pos = !P.pos_dev && range_hint == 0;
     const bool lean = m->attn_ctas > 0 && shape_ok && (range_hint == 1 || (by_pos && (long long)P.pos0 + step1 <= kShortAttnMax));
@@ -158,7 +158,7 @@ int dispatch_launch(mi_ctx* ctx, mi_model* m, const DecodeParams& P, int step0, 
     // of the down projection, the greedy pick over all CTAs' candidates), so all of them must be resident together.
     if (only_prepare) return MI_OK;
     void* args[] = {(void*)&P, &step0, &step1, &ph0, &ph1};
-    MI_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(m->grid), dim3(DNT), args, m->smem, ctx->stream));
+    MI_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(m->grid), dim3(DNT_ALL), args, m->smem, ctx->stream));
     return MI_OK;
 }
 
@@ -219,7 +219,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         return set_error(ctx, MI_ERR_FORMAT, "model: missing qwen2.* metadata or tokenizer.ggml.tokens");
     if (m->E % m->NH || m->NH % m->NKV) return set_error(ctx, MI_ERR_FORMAT, "model: head counts do not divide");
     m->HD = m->E / m->NH; m->KVD = m->NKV * m->HD; m->G = m->NH / m->NKV;
-    if (m->E % 32 || m->FF % 32 || m->HD % 32 || m->HD > 128 || m->G > DNW || m->L > 64 || m->E > 8192 || m->FF > 32768)
+    if (m->E % 32 || m->FF % 32 || m->HD % 32 || m->HD > 128 || m->G > 8 || m->L > 64 || m->E > 8192 || m->FF > 32768)
         return set_error(ctx, MI_ERR_UNSUPPORTED, "model: shape outside this path (E, FF, head_dim multiples of 32; <= 8 query heads per kv head)");
     m->max_seq = max_seq;
     m->grid = ctx->sm_count;
@@ -309,7 +309,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     int rot = 0, wrot = 0;
     auto add_job = [&](const uint8_t* base, int groups, int cols, int nacc, int kind, int layer) {
         Job jb{}; jb.nb = cols / 32; jb.kb = choose_kb(jb.nb); jb.nt = jb.nb / jb.kb;
-        jb.nacc = nacc; jb.kind = kind; jb.layer = layer;
+        jb.nacc = nacc; jb.kind = kind;
         // tensor parallelism: this GPU owns a contiguous range of the job's unit groups (rows); every GPU holds the
         // whole matrix but streams only its rows.  The K-split is planned from the largest share so that all GPUs
         // lay the partial sums out identically.
@@ -325,11 +325,12 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         if (force) jb.ks = std::max(1, std::min(std::min(atoi(force), jb.nt), kMaxKSplit));
         if (jb.ks >= GG) jb.ks = std::max(1, GG - 1);       // the CTAs of a row group's splits must be distinct
         jb.n_units = jb.groups * jb.ks;
-        jb.ks_inv = (unsigned)(((1ull << 32) + (unsigned)jb.ks - 1) / (unsigned)jb.ks);    // ks == 1: 2^32 wraps to 0, and that path does not divide
         if (kind == JOB_LM) { jb.rot = 0; jb.wrot = 0; }
         else {
-            // successive jobs start where the previous one stopped, over CTAs and over the warps of a CTA
-            jb.rot = rot; jb.wrot = wrot;
+            // the jobs of a layer start where the previous one stopped, over CTAs and over the warps of a CTA; every layer is dealt like the first, so that
+            // the kernel needs one description per kind
+            if (layer > 0) { jb.rot = m->jobs[kind].rot; jb.wrot = m->jobs[kind].wrot; }
+            else { jb.rot = rot; jb.wrot = wrot; }
             rot = (int)(((long long)rot + jb.n_units) % GG);
             wrot = (wrot + nacc * ((jb.nt + jb.ks - 1) / jb.ks)) & (DNW - 1);
         }
@@ -406,58 +407,87 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
 
-    // ---- per-warp tile lists: the order in which each warp of the grid consumes tiles during one step
+    // ---- per-warp tile lists: the order in which each warp of the grid consumes tiles during one step; and what each CTA does in a layer (DecodeParams::work)
     {
         const int nj = (int)m->jobs.size(), G = GG;
         std::vector<std::vector<unsigned long long>> lists((size_t)G * DNW);
         std::vector<unsigned> start((size_t)G * DNW * (nj + 1), 0);
+        std::vector<std::vector<unsigned>> work((size_t)G, std::vector<unsigned>(4, 0u));
         for (int j = 0; j < nj; j++) {
             const Job& jb = m->jobs[j];
             const size_t tb = (size_t)jb.kb * kTileRowBytes;
             const unsigned long long code = jb.kb == 8 ? 3 : jb.kb == 4 ? 2 : jb.kb == 2 ? 1 : 0;
             for (int slot = 0; slot < G * DNW; slot++) start[(size_t)slot * (nj + 1) + j] = (unsigned)lists[slot].size();
             if (jb.kind == JOB_LM) {
-                for (int u = 0; u < jb.n_units; u++) {                  // warp unit u -> slot sid = (u + rot) % W, sid = warp*G + cta
-                    const int sid = (int)(((long long)u + jb.rot) % W), cta = sid % G, warp = sid / G;
+                for (int u = 0; u < jb.n_units; u++) {                  // unit u -> warp slot u % W, slot = warp * G + cta
+                    const int sid = u % W, cta = sid % G, warp = sid / G;
                     auto& L = lists[(size_t)cta * DNW + warp];
                     for (int t = 0; t < jb.nt; t++) L.push_back((unsigned long long)(uintptr_t)(jb.base + ((size_t)u * jb.nt + t) * tb) | code);
                 }
-            } else {
-                for (int cta = 0; cta < G; cta++) {
-                    const int r = jb.rot % G, u0 = cta >= r ? cta - r : cta + G - r;
-                    int uidx = 0;
-                    for (int u = u0; u < jb.n_units; u += G, uidx++) {
-                        const int g = u / jb.ks, sp = u % jb.ks, t0 = sp * jb.nt / jb.ks, ntu = (sp + 1) * jb.nt / jb.ks - t0, n = jb.nacc * ntu;
-                        const int wr = (jb.wrot + uidx * 3) & (DNW - 1);
-                        for (int warp = 0; warp < DNW; warp++)
-                            for (int i = (warp - wr) & (DNW - 1); i < n; i += DNW) {
-                                const int a = i / ntu, t = t0 + i % ntu;
-                                lists[(size_t)cta * DNW + warp].push_back(
-                                    (unsigned long long)(uintptr_t)(jb.base + ((size_t)(g * jb.nacc + a) * jb.nt + t) * tb) | code);
+                continue;
+            }
+            for (int cta = 0; cta < G; cta++) {
+                const int r = jb.rot % G, u0 = cta >= r ? cta - r : cta + G - r;
+                std::vector<unsigned>& w = work[cta];
+                size_t link = (size_t)jb.kind;                          // where the offset of the next batch goes
+                for (int u = u0; u < jb.n_units; u += kBatchUnits * G) {
+                    const size_t at = w.size();
+                    if (u != u0) m->one_batch = false;
+                    if (j < 4) {
+                        w[link] |= link < 4 ? (unsigned)at : (unsigned)at << 8;
+                        link = at;
+                        w.resize(at + kBatchWords, 0u);
+                    }
+                    std::vector<unsigned> items[DNW];
+                    int i = jb.wrot, units = 0;
+                    for (int v = u; v < jb.n_units && units < kBatchUnits; v += G, units++) {
+                        const int g = v / jb.ks, sp = v % jb.ks, t0 = sp * jb.nt / jb.ks, t1 = (sp + 1) * jb.nt / jb.ks, ntu = t1 - t0;
+                        if (j < 4) {
+                            w[at + kBatchGroup + units] = (unsigned)(g + jb.g_off);
+                            w[at + kBatchUnit + units] = (unsigned)sp | (unsigned)std::min(ntu, DNW) << 8 | (unsigned)(i & (DNW - 1)) << 16 | (unsigned)((i + ntu) & (DNW - 1)) << 20;
+                        }
+                        for (int a = 0; a < jb.nacc; a++)
+                            for (int t = t0; t < t1; t++, i++) {
+                                lists[(size_t)cta * DNW + (i & (DNW - 1))].push_back((unsigned long long)(uintptr_t)(jb.base + ((size_t)(g * jb.nacc + a) * jb.nt + t) * tb) | code);
+                                items[i & (DNW - 1)].push_back((unsigned)(t * jb.kb) | (unsigned)(2 * units + a) << 16 | (t + DNW >= t1 ? 1u << 20 : 0u));
                             }
+                    }
+                    if (j >= 4) continue;
+                    w[at] |= (unsigned)units;
+                    for (int q = 0; q < DNW; q++) {
+                        w[at + kBatchList + q] = (unsigned)w.size() | (unsigned)items[q].size() << 16;
+                        w.insert(w.end(), items[q].begin(), items[q].end());
                     }
                 }
             }
         }
-        size_t stride = 1;
+        size_t stride = 1, words = 0;
         for (int slot = 0; slot < G * DNW; slot++) {
             start[(size_t)slot * (nj + 1) + nj] = (unsigned)lists[slot].size();
             stride = std::max(stride, lists[slot].size());
         }
+        for (const auto& w : work) words = std::max(words, w.size());
+        if (words > 65535) return set_error(ctx, MI_ERR_UNSUPPORTED, "model: %zu words of work per CTA on a grid of %d", words, m->grid);
         std::vector<unsigned long long> tab((size_t)G * DNW * stride, 0ull);
         for (int slot = 0; slot < G * DNW; slot++) std::copy(lists[slot].begin(), lists[slot].end(), tab.begin() + (size_t)slot * stride);
-        unsigned long long* d_tab; unsigned* d_start;
-        if ((st = dev_alloc(ctx, m, &d_tab, tab.size())) || (st = dev_alloc(ctx, m, &d_start, start.size()))) return st;
+        std::vector<unsigned> wtab((size_t)G * words, 0u);
+        for (int cta = 0; cta < G; cta++) std::copy(work[cta].begin(), work[cta].end(), wtab.begin() + (size_t)cta * words);
+        unsigned long long* d_tab; unsigned* d_start; unsigned* d_work;
+        if ((st = dev_alloc(ctx, m, &d_tab, tab.size())) || (st = dev_alloc(ctx, m, &d_start, start.size())) || (st = dev_alloc(ctx, m, &d_work, wtab.size()))) return st;
         MI_CUDA(ctx, cudaMemcpy(d_tab, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice));
         MI_CUDA(ctx, cudaMemcpy(d_start, start.data(), start.size() * 4, cudaMemcpyHostToDevice));
+        MI_CUDA(ctx, cudaMemcpy(d_work, wtab.data(), wtab.size() * 4, cudaMemcpyHostToDevice));
         P.tile_tab = d_tab; P.tile_start = d_start; P.tile_stride = (int)stride;
+        P.work = d_work; P.work_stride = (int)words; P.work_smem = words <= (size_t)kWorkSmem;
+        for (int k = 0; k < 4; k++) P.kb[k] = m->jobs[k].kb;
+        const Job& lm = m->jobs.back();
+        P.kb[JOB_LM] = lm.kb; P.ks_down = m->jobs[JOB_DOWN].ks; P.lm_units = lm.n_units; P.lm_nt = lm.nt; P.lm_off = lm.g_off;
     }
 
-    LayerPtrs* d_lp; Job* d_jobs;
-    if ((st = dev_alloc(ctx, m, &d_lp, lp.size())) || (st = dev_alloc(ctx, m, &d_jobs, m->jobs.size()))) return st;
+    LayerPtrs* d_lp;
+    if ((st = dev_alloc(ctx, m, &d_lp, lp.size()))) return st;
     MI_CUDA(ctx, cudaMemcpy(d_lp, lp.data(), lp.size() * sizeof(LayerPtrs), cudaMemcpyHostToDevice));
-    MI_CUDA(ctx, cudaMemcpy(d_jobs, m->jobs.data(), m->jobs.size() * sizeof(Job), cudaMemcpyHostToDevice));
-    P.layers = d_lp; P.jobs = d_jobs;
+    P.layers = d_lp;
     m->layer_ptrs = lp;
 
     // rope frequencies exactly as the reference computes them on the host: powf(base, -2i/hd) (src/cpu_infer.cpp:54)
@@ -488,10 +518,11 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         x.attm = take(m->NH * m->max_chunks);
         x.tokw = take(2);
         x.attdone = take(2 * m->attn_ctas);
-        x.total = off;
+        x.total = (off + 15) / 16 * 16;                                // copies begin on lines of their own
+        P.copies = tp_world == 1 ? kXCopies : 1;
     }
     if ((st = dev_alloc(ctx, m, &P.h_in, E)) || (st = dev_alloc(ctx, m, &P.h_mid, E)) || (st = dev_alloc(ctx, m, &P.att, NQ)) ||
-        (st = dev_alloc(ctx, m, &P.xw, (size_t)P.xo.total)) ||
+        (st = dev_alloc(ctx, m, &P.xw, (size_t)kXCopies * P.xo.total)) ||
         (st = dev_alloc(ctx, m, &P.kc, (size_t)L * max_seq * KVD)) || (st = dev_alloc(ctx, m, &P.vc, (size_t)L * max_seq * KVD)) ||
         (st = dev_alloc(ctx, m, &P.attn_part, (size_t)m->NH * m->max_chunks * (HD + 2))) ||
         (st = dev_alloc(ctx, m, &P.prof, kProfSlots)) || (st = dev_alloc(ctx, m, &m->best_buf, 2)) ||
@@ -514,8 +545,8 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     P.inv_e = 1.0 / (double)E;
     // positions per step of the long-range attention: as many as fit, a multiple of 16 so that score rows stay apart in the banks
     P.split_sub = kSplitSubMax;
-    while (P.split_sub > kSplitSubMin && decode_smem_bytes((int)m->jobs.size(), E, FF, HD, P.split_sub) + 1024 > (size_t)ctx->smem_optin) P.split_sub -= 16;
-    m->smem = decode_smem_bytes((int)m->jobs.size(), E, FF, HD, P.split_sub);
+    while (P.split_sub > kSplitSubMin && decode_smem_bytes(E, FF, HD, P.split_sub) + 1024 > (size_t)ctx->smem_optin) P.split_sub -= 16;
+    m->smem = decode_smem_bytes(E, FF, HD, P.split_sub);
     if (m->attn_ctas > 0) {
         const int hpc = attn_heads_per_cta(m->G);
         m->smem = std::max(m->smem, attn_dedicated_smem(HD, hpc));       // the attention CTAs lay the same allocation out their own way
@@ -734,7 +765,7 @@ static int decode_impl(mi_ctx* ctx, mi_model* m, const int32_t* in_tokens_host, 
         // launch's positions), a launch that straddles a boundary would fall back to the general build.  Under the stop
         // rule the host cannot know whether an earlier launch ended the run, so the run stays one launch.
         int cuts[3] = {0, 0, n_steps}, nc = 1;
-        if (stop < 0 && !P.tp.on && lean_shape(m->E, m->FF, m->NH * m->HD) != 0) {
+        if (stop < 0 && !P.tp.on && m->one_batch && lean_shape(m->E, m->FF, m->NH * m->HD) != 0) {
             const long long s = (long long)kShortAttnMax - pos0;       // first step whose position count exceeds the edge
             if (s > 0 && s < n_steps) cuts[nc++] = (int)s;
         }

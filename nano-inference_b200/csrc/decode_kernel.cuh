@@ -121,32 +121,42 @@
 
 namespace mi {
 
-constexpr int DNW = 8;            // warps per CTA
-constexpr int DNT = DNW * 32;
+constexpr int DNW = 8;            // warps per CTA that compute
+constexpr int DNT = DNW * 32;     // their threads
+constexpr int DNT_ALL = DNT + 32; // and one warp that requests the weights
 constexpr int DS = 3;             // ring slots per warp
 constexpr int DSLOT = 4608;       // bytes per slot: the largest tile (8 blocks)
 constexpr int kAttnChunk = 32;    // smallest KV range worth its own CTA
 constexpr int kShortAttnMax = 256;      // up to this many cached positions one CTA handles the whole range of a query head (attention_short)
 constexpr int kMaxKSplit = 4;     // cross-CTA K-splits of the down projection
 constexpr int kMaxWorldTP = 8;
+#ifndef MI_XCOPIES
+#define MI_XCOPIES 4
+#endif
+constexpr int kXCopies = MI_XCOPIES;       // copies of the exchange block (see Pub)
 
 // profile slots: 2*k = staging of phase kind k, 2*k+1 = its main work; 12 = time spent waiting for tagged words, 13 = step prologue
 enum { kProfWait = 12, kProfStep = 13, kProfSlots = 32 };
 
 enum JobKind { JOB_QKV = 0, JOB_O = 1, JOB_GU = 2, JOB_DOWN = 3, JOB_LM = 4 };
 
-struct Job {
+struct Job {               // (host) a tiled matrix and how it is dealt over the grid
     const uint8_t* base;   // tiled weights
     int groups;            // unit groups; one unit group = nacc consecutive 32-row groups
     int nt, ks, nb, kb, nacc, kind;
     int n_units;           // groups * ks
-    int rot;               // CTA (per-layer jobs) or warp slot (lm_head) that gets unit 0
-    int wrot;              // warp that gets tile 0 of a CTA unit
-    unsigned ks_inv;       // ceil(2^32 / ks): x / ks == __umulhi(x, ks_inv) for the unit and tile counts that occur (set by the host)
-    int layer;
+    int rot;               // CTA (per-layer jobs) that gets unit 0
+    int wrot;              // warp that gets tile 0 of a batch
     int g_off;             // first unit group this GPU owns (tensor parallelism; base points at it, groups counts the owned ones)
-    int pad_;
 };
+
+// What a CTA does in the per-layer jobs, listed by the host (all layers are dealt alike): 32-bit words, [kind] = offset of the job's first batch, or 0.
+// A batch is up to kBatchUnits units; its tiles, numbered unit by unit, accumulator by accumulator (gate, up), along K, go round-robin over the eight warps:
+//   [0] number of units | offset of the next batch << 8, or 0      [1 + b] row group of unit b
+//   [4 + b] K-split of unit b | number of warps with tiles of a sum << 8 | first of them << 16 (gate), << 20 (up)
+//   [7 + w] offset of warp w's list | number of its tiles << 16;  list entry: first block | sum (2 b + accumulator) << 16 | last of the sum << 20
+constexpr int kBatchUnits = 3;                        // (the 3B shape's gate/up: two or three units per CTA)
+enum { kBatchGroup = 1, kBatchUnit = kBatchGroup + kBatchUnits, kBatchList = kBatchUnit + kBatchUnits, kBatchWords = kBatchList + 8 };
 
 struct LayerPtrs { const float* attn_norm; const float* ffn_norm; const float* bqkv; };
 
@@ -181,10 +191,11 @@ struct DecodeParams {
     int L, E, FF, NH, NKV, HD, KVD, V;
     float eps;
     double inv_e;                    // 1 / E
-    const Job* jobs;                 // [4L+1] in phase order
-    const unsigned long long* tile_tab;   // per warp slot: source address | kb code of every tile of one step, in consumption order
+    const unsigned* work; int work_stride, work_smem;      // per GEMV CTA: its list (see above); whether it goes to shared memory
+    int kb[5], ks_down, lm_units, lm_nt, lm_off;           // tile depths by JobKind, K-splits of the down projection; lm_head: row groups and tiles of one, first row group
+    const unsigned long long* tile_tab;   // per warp: source address | kb code of every tile of one step, in consumption order
     const unsigned* tile_start;      // [grid*DNW][4L+2]: index of each job's first tile in the warp's list (last = count)
-    int tile_stride;                 // entries reserved per warp slot in tile_tab
+    int tile_stride;                 // entries reserved per warp in tile_tab
     const LayerPtrs* layers;         // [L]
     const float* out_norm;
     const float* rope_freq;          // [HD/2]: base^(-2i/HD), computed on the host with powf
@@ -198,6 +209,7 @@ struct DecodeParams {
     float* h_mid;                    // after the attention block
     // the exchange block: every vector one CTA hands to another, as tagged words
     unsigned long long* xw; XwLayout xo;
+    int copies;                      // how many copies of the block consumers read (1: tensor parallelism, whose exchanges write the first one only)
     // Tag of (step s of the launch, phase p) = epoch + s * (5L+1) + p + 1.  The epoch lives in device memory and the kernel
     // advances it itself: a launch whose phase range ends a step leaves it past every tag the launch used (a launch that
     // gave up on a wait: further still).  Replayed launch sequences and calls after a failure therefore never meet a stale
@@ -239,10 +251,11 @@ __host__ __device__ inline int q8_words(int n) { return n / 4 + (n / 32 + 1) / 2
 inline namespace MI_KVARIANT {
 
 struct DecodeSmem {
-    uint8_t* ring; uint64_t* bars; Job* jobs; LayerPtrs* lp; float* cs; double* red; double* fold; float* h; uint8_t* stage;
+    uint8_t* ring; uint64_t* bars; const unsigned* work; LayerPtrs* lp; float* cs; double* red; double* fold; float* h; uint8_t* stage;
 };
 
-constexpr int kFoldBytes = 2 * DNW * 2 * 32 * 8;      // two buffers of [warp][acc][lane] doubles
+constexpr int kFoldBytes = kBatchUnits * 2 * DNW * 32 * 8;      // [unit of the batch][acc][warp][lane] doubles
+constexpr int kWorkSmem = 512;                        // words of a CTA's list that fit the shared memory
 
 // attention_split: positions per step (as many as the shared memory allows: a chunk that fits one step has all its rows requested
 // before q is waited for; 8192 positions in two steps of 64 instead of one of 112: 3.9 instead of 2 us for the scores), words of
@@ -270,8 +283,8 @@ __host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD, int 
     const size_t b = split > shrt ? split : shrt;
     return ((a > b ? a : b) + 127) / 128 * 128;
 }
-__host__ __device__ inline size_t decode_smem_bytes(int njobs, int E, int FF, int HD, int sub) {
-    return (size_t)DNW * DS * DSLOT + 256 + ((size_t)njobs * sizeof(Job) + 127) / 128 * 128 + 64 * sizeof(LayerPtrs) + 1024 + 256 + kFoldBytes +
+__host__ __device__ inline size_t decode_smem_bytes(int E, int FF, int HD, int sub) {
+    return (size_t)DNW * DS * DSLOT + 512 + kWorkSmem * 4 + 64 * sizeof(LayerPtrs) + 1024 + 256 + kFoldBytes +
            ((size_t)E * 4 + 127) / 128 * 128 + decode_stage_bytes(E, FF, HD, sub);
 }
 
@@ -309,6 +322,14 @@ struct Cand {
     }
 };
 
+// Barriers of the warps that compute (the one that requests weights has no part in them)
+__device__ __forceinline__ void cta__syncthreads() { asm volatile("bar.sync 1, %0;" ::"n"(DNT) : "memory"); }
+__device__ __forceinline__ int cta__syncthreads_and(int p) {
+    int r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(p), "n"(DNT) : "memory");
+    return r;
+}
+
 // ---- tagged words ---------------------------------------------------------------------
 // One 64-bit access carries value and tag together, so there is nothing to order between them.
 // The accesses are volatile: they are performed at the L2 (the point where all SMs of this GPU,
@@ -326,36 +347,45 @@ __device__ __forceinline__ void tw_st(unsigned long long* p, unsigned tag, unsig
 }
 __device__ __forceinline__ bool tw_is(unsigned long long w, unsigned tag) { return (unsigned)(w >> 32) == tag; }
 
-// Where a phase publishes: locally, and (tensor-parallel build, shared vectors) into every other GPU's block.
+// Where a phase publishes.  What (nearly) every CTA reads goes into kXCopies copies of the exchange block, and CTA i reads copy i % P.copies: a vector is a hundred lines of the
+// L2 or less, each read by 142 CTAs, and the slices that hold several of them were what the words waited for.  Words with few readers are in the first copy only.  In the
+// tensor-parallel build shared vectors also go into every other GPU's block.
 struct Pub {
-    unsigned long long* xw; unsigned tag; bool mute;
+    unsigned long long* xw; unsigned tag; bool mute; int stride;
 #if MI_TP
     const TpPeerParams* tp;
 #endif
     __device__ __forceinline__ void local(int off, unsigned payload) const { if (!mute) tw_st(xw + off, tag, payload); }
-    __device__ __forceinline__ void shared(int off, unsigned payload) const {
+    __device__ __forceinline__ void all(int off, unsigned payload) const {
         if (mute) return;
-        tw_st(xw + off, tag, payload);
+        #pragma unroll
+        for (int r = 0; r < (MI_TP ? 1 : kXCopies); r++) tw_st(xw + off + r * stride, tag, payload);
+    }
+    __device__ __forceinline__ void shared(int off, unsigned payload) const {
+        all(off, payload);
 #if MI_TP
+        if (mute) return;
         if (tp->on) {
             for (int p = 0; p < tp->world; p++) if (p != tp->rank) tw_st(tp->xw_peer[p] + off, tag, payload);
         }
 #endif
     }
 };
+__device__ __forceinline__ const unsigned long long* xw_read(const DecodeParams& P) { return P.xw + (blockIdx.x & (unsigned)(P.copies - 1)) * (size_t)P.xo.total; }
 
 // Poll one word until it carries `tag`.  Gives up (false) when the time budget has run out or another CTA has reported
 // an error; the caller then leaves the kernel through its error path.
 MI_COLD_FN bool tw_spin(const unsigned long long* p, unsigned tag, unsigned long long budget_ns, const int* err) {
     unsigned long long t0 = 0;
-    for (unsigned it = 1;; it++) {
-        if (tw_is(tw_ld(p), tag)) return true;
+    #pragma unroll 1
+    for (unsigned it = 1; !tw_is(tw_ld(p), tag); it++) {
         if ((it & 31u) == 0) {
             const unsigned long long now = gtime_ns();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > budget_ns || *reinterpret_cast<const volatile int*>(err) != 0) return false;
+            if (now - t0 > budget_ns || *reinterpret_cast<const volatile int*>(err) != 0) return false;
         }
     }
+    return true;
 }
 
 // One warp waits together: the lowest lane that misses a word polls that word, the other lanes sit at the vote, so a
@@ -398,126 +428,198 @@ __device__ __forceinline__ bool tw_poll(const DecodeParams& P, unsigned tag, uns
     return true;
 }
 
-// ---- the per-warp weight stream -----------------------------------------------
-// Tiles of a unit are numbered i = a*ntu + (t - t0) (a = accumulator, ntu = tiles of
-// the unit's K range).  In a CTA unit warp w owns the tiles with (i + wrot(u)) % 8 == w;
-// in a warp unit (lm_head) the owning warp takes all of them.
-struct UnitShape { int g, sp, t0, ntu, n, wrot; };
-
-__device__ __forceinline__ UnitShape unit_shape(const Job& jb, int u, int uidx) {
-    UnitShape s;
-    if (jb.ks == 1) { s.g = u; s.sp = 0; s.t0 = 0; s.ntu = jb.nt; }
-    else {
-        // divisions by the K-split count through the host's reciprocal: exact for operands below 2^20 with ks <= kMaxKSplit
-        s.g = (int)__umulhi((unsigned)u, jb.ks_inv); s.sp = u - s.g * jb.ks;
-        s.t0 = (int)__umulhi((unsigned)(s.sp * jb.nt), jb.ks_inv);
-        s.ntu = (int)__umulhi((unsigned)((s.sp + 1) * jb.nt), jb.ks_inv) - s.t0;
+// N 16-byte pairs of words, pair k at `base + off[k]` (where bit k of `valid` is set), their payloads in a and b.  As tw_poll, in few instructions: a lane that misses
+// anything fetches all of its pairs again.
+// Among the last NPAD pairs, word `pad` is one that nobody writes.
+template <int N, int NPAD = 0>
+__device__ __forceinline__ bool tw_poll_pairs(const DecodeParams& P, unsigned tag, unsigned valid, const unsigned long long* base, const int (&off)[N], unsigned (&a)[N], unsigned (&b)[N],
+                                              int pad = -1) {
+    const unsigned long long none = (unsigned long long)tag << 32;
+    unsigned round = 0;
+    #pragma unroll 1
+    for (;;) {
+        unsigned long long wa[N], wb[N];
+        #pragma unroll
+        for (int k = 0; k < N; k++) {
+            wa[k] = wb[k] = none;
+            if (valid >> k & 1u) tw_ld2(base + off[k], wa[k], wb[k]);
+        }
+        int miss = -1;
+        #pragma unroll
+        for (int k = 0; k < N; k++) {
+            if (!tw_is(wa[k], tag)) miss = off[k];
+            if (!tw_is(wb[k], tag) && !(k >= N - NPAD && off[k] + 1 == pad)) miss = off[k] + 1;
+            a[k] = (unsigned)wa[k]; b[k] = (unsigned)wb[k];
+        }
+        const int st = tw_wait_warp(miss >= 0 ? base + miss : nullptr, tag, P.wait_ns, P.err, round++);
+        if (st <= 0) return st == 0;
     }
-    s.n = jb.nacc * s.ntu;
-    s.wrot = (jb.wrot + uidx * 3) & (DNW - 1);      // uidx: how many units this CTA had before u in the job
-    return s;
 }
 
-// Producer side of a warp's ring.  The order in which a warp consumes tiles is a pure
-// function of shapes and indices, so the host lists it once per model: entry k of a warp's
-// list is the global address of its k-th tile of a step (16-byte aligned; the low two bits
-// carry log2 of the tile depth).  The producer walks that list, wrapping at the end of the
-// launch's job range, with the next entry already loaded so that issuing a copy costs a
-// handful of instructions and no division.
+// ---- the per-warp weight stream -----------------------------------------------
+// The order in which a warp consumes tiles is a pure function of shapes and indices, so the host lists it once per model: entry k of a warp's
+// list is the global address of its k-th tile of a step (16-byte aligned; the low two bits carry log2 of the tile depth).  A ninth warp walks
+// the lists, a lane per ring, wrapping at the end of the launch's job range, and requests a tile whenever a slot is free.  (A copy takes the warp that issues it
+// some 400 clocks; issued by the computing warps, between tiles or behind a phase, that was a tenth of a token and left copies to be made in bursts, so that
+// the tiles of the next phase were missing.)
 struct WarpStream {
-    uint8_t* ring; uint64_t* bars; const Job* jobs;
-    const unsigned long long* tab;   // this warp's list
-    unsigned e0, e1, c;              // entry range of the launch's jobs within a step; cursor
-    long long left;                  // tiles still to issue in this launch
-    unsigned long long next;         // entry at the cursor (valid while left > 0)
-    int issued, consumed;
-    int W, sid, warp;                // warp slots in the grid, this warp's slot, warp in CTA
-    int gcta, ggrid;                 // this CTA's index among the CTAs that carry GEMV units (negative: attention only), their number
-    uint64_t policy;                 // L2 evict-first for the weight stream
+    const uint8_t* ring; uint64_t* full; uint64_t* empty;
+    unsigned out, phase;             // slot of the next tile, parity of its barrier
+    int warp;                        // warp in CTA
+    int gcta, ggrid;                 // this CTA's index among the CTAs that carry GEMV units, their number
 
-    __device__ __forceinline__ void init(const DecodeSmem& sm, const DecodeParams& P, int warp_, int step0, int step1, int j0, int j1) {
-        warp = warp_; policy = l2_policy_evict_first();
-        ring = sm.ring + (size_t)warp * DS * DSLOT; bars = sm.bars + warp * DS; jobs = sm.jobs;
+    __device__ __forceinline__ void init(const DecodeSmem& sm, const DecodeParams& P, int warp_) {
+        warp = warp_;
+        ring = sm.ring + (size_t)warp * DS * DSLOT; full = sm.bars + warp * DS; empty = full + DNW * DS;
         gcta = (int)blockIdx.x - P.attn_ctas; ggrid = (int)gridDim.x - P.attn_ctas;
-        W = ggrid * DNW; sid = warp * ggrid + gcta;      // consecutive warp units land on different SMs
-        if (gcta < 0) { e0 = e1 = c = 0; issued = consumed = 0; left = 0; next = 0ull; tab = nullptr; return; }
-        const int slot = gcta * DNW + warp, nj = 4 * P.L + 2;
-        tab = P.tile_tab + (size_t)slot * P.tile_stride;
-        e0 = __ldg(P.tile_start + (size_t)slot * nj + j0);
-        e1 = __ldg(P.tile_start + (size_t)slot * nj + j1);
-        c = e0; issued = consumed = 0;
-        left = j0 < j1 ? (long long)(step1 - step0) * (e1 - e0) : 0;
-        next = left > 0 ? __ldg(tab + c) : 0ull;
+        out = phase = 0;
     }
-    __device__ __forceinline__ void issue_one() {       // lane 0 only
-        if (left <= 0) return;
-        const unsigned long long e = next;
-        const int tb = kTileRowBytes << (int)(e & 3ull), slot = issued % DS;
-        mbar_expect_tx(&bars[slot], tb);
-        bulk_g2s_hint(ring + (size_t)slot * DSLOT, reinterpret_cast<const void*>(e & ~15ull), tb, &bars[slot], policy);
-        issued++;
-        if (++c == e1) c = e0;
-        if (--left > 0) next = __ldg(tab + c);
+    // waits for the next tile; release() when every lane is through with it
+    __device__ __forceinline__ bool acquire() const {
+        unsigned long long t0 = 0;
+        #pragma unroll 1
+        for (unsigned i = 1; !mbar_try_wait(&full[out], phase); i++) {
+            if ((i & 255u) == 0) {
+                const unsigned long long now = gtime_ns();
+                if (t0 == 0) t0 = now;
+                if (now - t0 > kWaitBudgetNs) return false;
+            }
+        }
+        return true;
     }
-    __device__ __forceinline__ void drain() {
-        for (int k = consumed; k < issued; k++) (void)mbar_wait_bounded(&bars[k % DS], (k / DS) & 1);
-    }
-    __device__ __forceinline__ int first_cta_unit(const Job& jb) const {
-        const int G = ggrid, r = jb.rot, b = gcta;         // the host keeps rot below the number of GEMV CTAs
-        return b >= r ? b - r : b + G - r;
-    }
-    __device__ __forceinline__ int first_warp_unit(const Job& jb) const {
-        const int r = jb.rot % W; return sid >= r ? sid - r : sid + W - r;
+    __device__ __forceinline__ const uint8_t* tile() const { return ring + (size_t)out * DSLOT; }
+    __device__ __forceinline__ void release(int lane) {
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[out])) : "memory");
+        if (++out == DS) { out = 0; phase ^= 1u; }
     }
 };
+// The ninth warp: lane r < 8 keeps ring r full until the launch's tiles have been requested, or the computing warps have left (quit).  Then it sees its copies land: they
+// target this CTA's shared memory.
+__device__ __forceinline__ void stream_weights(const DecodeSmem& sm, const DecodeParams& P, int lane, int steps, int j0, int j1, const volatile int* quit) {
+    const int r = lane & (DNW - 1), slot = ((int)blockIdx.x - P.attn_ctas) * DNW + r, nj = 4 * P.L + 2;
+    uint8_t* ring = sm.ring + (size_t)r * DS * DSLOT;
+    uint64_t* full = sm.bars + r * DS; uint64_t* empty = full + DNW * DS;
+    const unsigned long long* tab = P.tile_tab + (size_t)slot * P.tile_stride;
+    const unsigned e0 = __ldg(P.tile_start + (size_t)slot * nj + j0), e1 = __ldg(P.tile_start + (size_t)slot * nj + j1);
+    long long left = lane < DNW && j0 < j1 ? (long long)steps * (e1 - e0) : 0;
+    unsigned c = e0, in = 0, lap = 0;
+    int issued = 0;
+    const uint64_t policy = l2_policy_evict_first();          // a weight byte is read once per token
+    unsigned long long next = left > 0 ? __ldg(tab + c) : 0ull;
+    while (__any_sync(0xffffffffu, left > 0) && !__any_sync(0xffffffffu, *quit != 0)) {
+        const bool go = left > 0 && (lap == 0 || mbar_try_wait(&empty[in], (lap - 1) & 1));        // (the first lap finds the slots empty)
+        if (go) {
+            const int tb = kTileRowBytes << (int)(next & 3ull);
+            mbar_expect_tx(&full[in], tb);
+            bulk_g2s_hint(ring + (size_t)in * DSLOT, reinterpret_cast<const void*>(next & ~15ull), tb, &full[in], policy);
+            issued++; left--;
+            if (++in == DS) { in = 0; lap++; }
+            if (++c == e1) c = e0;
+            if (left > 0) next = __ldg(tab + c);
+        }
+        if (!__any_sync(0xffffffffu, go)) __nanosleep(64);
+    }
+    if (lane < DNW)
+        for (int k = max(0, issued - DS); k < issued; k++) (void)mbar_wait_bounded(&full[k % DS], (k / DS) & 1);
+}
 
 // The per-token loop body must stay small: it is executed phase after phase by every SM, and measured, the kernel ran
 // 15 % faster once the four GEMV phases shared one copy of their code.  So the double-precision exponential has one
 // out-of-line copy, and the variants a given model never takes (other tile depths, other norm widths) sit out of line
 // instead of between the hot instructions.
 MI_COLD_FN double exp_shared(double x) { return exp(x); }
-static __device__ __noinline__ double tile_dot_row_rare(int kb, const uint8_t* tile, int lane, int t, const int8_t* xq_s, const float2* xs_s, double acc) {
-    switch (kb) {
-        case 4: return tile_dot_row<4, false>(tile, lane, t * 4, xq_s, xs_s, acc, nullptr);
-        case 2: return tile_dot_row<2, false>(tile, lane, t * 2, xq_s, xs_s, acc, nullptr);
-        default: return tile_dot_row<1, false>(tile, lane, t, xq_s, xs_s, acc, nullptr);
-    }
+// A tile's contribution to the lane's row: the GEMV's terms (blk_acc) from fewer operations.  What bounds it is the integer pipe (an SM makes 64 dp4a a clock, two
+// clocks for a warp on its sub-partition, and logic operations with an immediate twice that: 27 clocks of it per block), and, for the few tiles of a small phase, latency.  So the high
+// nibbles stay where they are, as bytes 16 n, and the dot product is 16 (low - 8 sum x) + high; its 16 is in xs_s, a sixteenth of each block's scale (a power of two: all
+// products stay exact) beside -8 times the sum of the block's activations.  The dot product starts at 2^31, so that below the exponent bits of 2^52 it is a double without a
+// conversion (of which an SM makes 16 a clock).  Tried: the blocks on int8 MMAs, one column of the
+// activations per block (the same throughput, twice the latency); nibbles made signed bytes with an exclusive or (three-operand logic: 38 clocks); sixteen warps with half a
+// tile each (680 us per token of the 1.5B shape: the pipe is as full with eight, and barriers and polls cost more).
+__device__ __forceinline__ int dp4a_us(unsigned w, int x, int c) { int r; asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(x), "r"(c)); return r; }
+struct BlockScale { float d16; int m8s; };                    // a sixteenth of the scale, -8 times the sum of the values
+__device__ __forceinline__ BlockScale block_scale(float d, int sum) { BlockScale b; b.d16 = __fmul_rn(d, 0.0625f); b.m8s = -8 * sum; return b; }
+template <int KB> struct TileRegs { uint4 w[KB]; unsigned d[(KB + 1) / 2]; };          // a lane's row of KB blocks
+template <int KB>
+__device__ __forceinline__ void tile_load(const uint8_t* tile, int lane, TileRegs<KB>& r) {
+    const uint8_t* sp = tile + KB * 512 + lane * (KB * 2);
+    if constexpr (KB == 8) { const uint4 v = *reinterpret_cast<const uint4*>(sp); r.d[0] = v.x; r.d[1] = v.y; r.d[2] = v.z; r.d[3] = v.w; }
+    else if constexpr (KB == 4) { const uint2 v = *reinterpret_cast<const uint2*>(sp); r.d[0] = v.x; r.d[1] = v.y; }
+    else if constexpr (KB == 2) r.d[0] = *reinterpret_cast<const unsigned*>(sp);
+    else r.d[0] = *reinterpret_cast<const unsigned short*>(sp);
+    #pragma unroll
+    for (int k = 0; k < KB; k++) r.w[k] = reinterpret_cast<const uint4*>(tile)[k * 32 + lane];
 }
-
-// consume the next tile of this warp's stream into acc (block index b0 = t * kb)
-__device__ __forceinline__ double tile_consume(WarpStream& ws, int lane, int kb, int t, const int8_t* xq_s, const float2* xs_s,
-                                               double acc, bool& ok, const DecodeParams* PP = nullptr) {
-    if (!ok) return acc;
-    const int slot = ws.consumed % DS;
-    if (PP) prof_mark(*PP, 18);
-    if (!mbar_wait_bounded(&ws.bars[slot], (ws.consumed / DS) & 1)) { ok = false; return acc; }
-    if (PP) prof_mark(*PP, 20);
-    const uint8_t* tile = ws.ring + (size_t)slot * DSLOT;
-#if MI_LEAN
-    // lean_shape(): tiles are 8 blocks deep, or (small build) 8 or 4
-    if (MI_SMALL && kb == 4) acc = tile_dot_row<4, false>(tile, lane, t * 4, xq_s, xs_s, acc, nullptr);
-    else acc = tile_dot_row<8, false>(tile, lane, t * 8, xq_s, xs_s, acc, nullptr);
-#else
-    if (kb == 8) acc = tile_dot_row<8, false>(tile, lane, t * 8, xq_s, xs_s, acc, nullptr);
-    else acc = tile_dot_row_rare(kb, tile, lane, t, xq_s, xs_s, acc);
-#endif
-    ws.consumed++;
-    __syncwarp();
-    if (PP) prof_mark(*PP, 21);
-    if (lane == 0) ws.issue_one();
-    __syncwarp();
-    if (PP) prof_mark(*PP, 22);
+template <int KB>
+__device__ __forceinline__ double tile_dot(const TileRegs<KB>& r, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) {
+    #pragma unroll
+    for (int k = 0; k < KB; k++) {
+        const uint4 w = r.w[k];
+        const int4 xa = *reinterpret_cast<const int4*>(xq_s + (b0 + k) * 32), xc = *reinterpret_cast<const int4*>(xq_s + (b0 + k) * 32 + 16);
+        const BlockScale x = xs_s[b0 + k];
+        constexpr unsigned L = 0x0F0F0F0Fu, H = 0xF0F0F0F0u;
+        int c = dp4a_us(w.x & L, xa.x, x.m8s), d = dp4a_us(w.x & H, xc.x, (int)0x80000000);
+        c = dp4a_us(w.y & L, xa.y, c); d = dp4a_us(w.y & H, xc.y, d);
+        c = dp4a_us(w.z & L, xa.z, c); d = dp4a_us(w.z & H, xc.z, d);
+        c = dp4a_us(w.w & L, xa.w, c); d = dp4a_us(w.w & H, xc.w, d);
+        acc = __fma_rn((double)__fmul_rn(__half2float(__ushort_as_half((unsigned short)(r.d[k / 2] >> 16 * (k & 1)))), x.d16),
+                       __dsub_rn(__hiloint2double(0x43300000, c * 16 + d), 4503601774854144.0), acc);      // 2^52 + 2^31
+    }
     return acc;
 }
+template <int KB>
+static __device__ __noinline__ double tile_dot_rare(const uint8_t* tile, int lane, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) {
+    TileRegs<KB> r;
+    tile_load<KB>(tile, lane, r);
+    return tile_dot<KB>(r, b0, xq_s, xs_s, acc);
+}
+// A tile in registers, and its product: the two are apart because the first tile of a phase is read before its input is there.  lean_shape(): tiles
+// are 8 blocks deep, or (small build) 8 or 4; the general build reads its tiles where it needs them.
+struct WarpTile {
+#if MI_LEAN
+    TileRegs<8> t;
+    __device__ __forceinline__ void load(WarpStream& ws, int lane, int kb) {
+        if (MI_SMALL && kb == 4) {
+            TileRegs<4> r;
+            tile_load<4>(ws.tile(), lane, r);
+            #pragma unroll
+            for (int k = 0; k < 4; k++) { t.w[k] = r.w[k]; t.d[k / 2] = r.d[k / 2]; }
+        } else tile_load<8>(ws.tile(), lane, t);
+        ws.release(lane);
+    }
+    __device__ __forceinline__ double dot(WarpStream&, int, int kb, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) const {
+        if (MI_SMALL && kb == 4) {
+            TileRegs<4> r;
+            #pragma unroll
+            for (int k = 0; k < 4; k++) { r.w[k] = t.w[k]; r.d[k / 2] = t.d[k / 2]; }
+            return tile_dot<4>(r, b0, xq_s, xs_s, acc);
+        }
+        return tile_dot<8>(t, b0, xq_s, xs_s, acc);
+    }
+#else
+    const uint8_t* at;
+    __device__ __forceinline__ void load(const WarpStream& ws, int, int) { at = ws.tile(); }
+    __device__ __forceinline__ double dot(WarpStream& ws, int lane, int kb, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) const {
+        if (kb == 8) {
+            TileRegs<8> r;
+            tile_load<8>(at, lane, r);
+            acc = tile_dot<8>(r, b0, xq_s, xs_s, acc);
+        } else acc = kb == 4 ? tile_dot_rare<4>(at, lane, b0, xq_s, xs_s, acc) : kb == 2 ? tile_dot_rare<2>(at, lane, b0, xq_s, xs_s, acc) : tile_dot_rare<1>(at, lane, b0, xq_s, xs_s, acc);
+        ws.release(lane);
+        return acc;
+    }
+#endif
+};
 
 // q8_0 of one 32-element block held one element per lane; returns the int8 value, and through
 // d_out / s_out (all lanes) the fp16 scale and the integer sum of the block's values.
 __device__ __forceinline__ int quant_block_warp2(float v, __half& d_out, int& s_out) {
     const float a = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v))));
-    const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
-    const int q = __float2int_rn(__fmul_rn(v, inv));
+    const bool odd = threadIdx.x & 1;                       // (one division for 127 / a and a / 127)
+    const float r = __fdiv_rn(odd ? a : 127.f, odd ? 127.f : a), iv = __shfl_sync(0xffffffffu, r, 0);
+    const int q = __float2int_rn(__fmul_rn(v, a > 0.f ? iv : 0.f));
     s_out = __reduce_add_sync(0xffffffffu, q);
-    d_out = __float2half_rn(__fdiv_rn(a, 127.f));
+    d_out = __float2half_rn(__shfl_sync(0xffffffffu, r, 1));
     return q;
 }
 // Publish one q8_0 block (lane = element) as tagged words: lanes 0, 4, 8, .. store four int8 values each, lane 0
@@ -528,81 +630,127 @@ __device__ __forceinline__ void publish_q8_block(const Pub& pub, int qoff, int s
     v |= __shfl_down_sync(0xffffffffu, v, 1) << 8;
     v |= __shfl_down_sync(0xffffffffu, v, 2) << 16;
     const unsigned sw = (unsigned)__half_as_ushort(d) | ((unsigned)s << 16);
-    if ((lane & 3) == 0) { if (SHARED) pub.shared(qoff + b * 8 + (lane >> 2), v); else pub.local(qoff + b * 8 + (lane >> 2), v); }
-    if (lane == 0) { if (SHARED) pub.shared(soff + b, sw); else pub.local(soff + b, sw); }
+    if ((lane & 3) == 0) { if (SHARED) pub.shared(qoff + b * 8 + (lane >> 2), v); else pub.all(qoff + b * 8 + (lane >> 2), v); }
+    if (lane == 0) { if (SHARED) pub.shared(soff + b, sw); else pub.all(soff + b, sw); }
+}
+
+// A per-layer job, before its input is there: the CTA's first batch, and this warp's first tile (range builds: in registers), so that behind the last word
+// that arrives there are only the activations to be read.
+struct JobStart { unsigned at; bool ok; float bias; WarpTile t; };
+// bias: added to complete sums by the epilogue, which needs the one of its unit
+__device__ __forceinline__ float batch_bias(const unsigned* work, unsigned at, int warp, int lane, const float* __restrict__ bias) {
+    return bias && warp < (int)(work[at] & 255u) ? __ldg(bias + work[at + kBatchGroup + warp] * 32 + lane) : 0.f;
+}
+__device__ __forceinline__ JobStart begin_cta_job(WarpStream& ws, const unsigned* work, int kind, int kb, int lane, const float* __restrict__ bias) {
+    JobStart st;
+    st.at = work[kind]; st.ok = true; st.bias = 0.f;
+    if (st.at) {
+        st.bias = batch_bias(work, st.at, ws.warp, lane, bias);
+        if (work[st.at + kBatchList + ws.warp] >> 16) { st.ok = ws.acquire(); st.t.load(ws, lane, kb); }
+    }
+    return st;
 }
 
 __device__ __forceinline__ double tree_sum8(double a, double b, double c, double d, double e, double f, double g, double h) {
     return __dadd_rn(__dadd_rn(__dadd_rn(a, b), __dadd_rn(c, d)), __dadd_rn(__dadd_rn(e, f), __dadd_rn(g, h)));
 }
-// Per-layer job: this CTA's units, tiles split over its warps, partial sums folded in
-// shared memory in warp order by warp 0, which then calls epi(g, lane, v0, v1) with the
-// complete sums rounded to fp32.  A job that is K-split across CTAs (ks > 1; down projection)
+// The job's batches: the warps' shares of every sum meet in shared memory, and warp b adds those of unit b and calls epi(g, lane, v0, v1, bias) with
+// the complete sums rounded to fp32.  A job that is K-split across CTAs (ks > 1; down projection)
 // adds one hop: the CTAs of splits 1.. publish their double partial sums as tagged word pairs,
 // the CTA of split 0 waits for them, adds them to its own in split order and calls epi.
-// Every warp passes the same number of __syncthreads, also after a wait gave up.
-// bias: added to complete sums by epi; requested before the tiles are worked on (it comes from the L2).
+// Every warp passes the same number of barriers, also after a wait gave up.
 template <class Epi>
-__device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, int j, int lane,
-                                            const int8_t* xq_s, const float2* xs_s, const Pub& pub, const float* __restrict__ bias, Epi epi) {
-    const Job jb = ws.jobs[j];                          // registers: the fields are used many times
-    bool ok = true;
-    int uidx = 0;
-    for (int u = ws.first_cta_unit(jb); u < jb.n_units; u += ws.ggrid, uidx++) {
-        const UnitShape s = unit_shape(jb, u, uidx);
-        const float bv = bias && ws.warp == 0 ? __ldg(bias + (s.g + jb.g_off) * 32 + lane) : 0.f;
-        double a0 = 0.0, a1 = 0.0;
-        for (int i = (ws.warp - s.wrot) & (DNW - 1); i < s.n; i += DNW) {
-            const bool first = i < s.ntu;                       // which of the unit's two accumulators (gate / up) the tile feeds
-            const double r = tile_consume(ws, lane, jb.kb, s.t0 + (first ? i : i - s.ntu), xq_s, xs_s, first ? a0 : a1, ok, &P);
-            if (first) a0 = r; else a1 = r;
-        }
-        prof_mark(P, 18);
-        double* fb = sm.fold + (size_t)(uidx & 1) * DNW * 2 * 32;
-        fb[(ws.warp * 2) * 32 + lane] = a0;
-        fb[(ws.warp * 2 + 1) * 32 + lane] = a1;
-        __syncthreads();
-        if (ws.warp == 0) {
-            // (a tree: the seven additions one after the other were 130 cycles of every phase)
-            double v0 = tree_sum8(fb[lane], fb[64 + lane], fb[128 + lane], fb[192 + lane], fb[256 + lane], fb[320 + lane], fb[384 + lane], fb[448 + lane]);
-            const double v1 = jb.nacc > 1 ? tree_sum8(fb[32 + lane], fb[96 + lane], fb[160 + lane], fb[224 + lane], fb[288 + lane], fb[352 + lane], fb[416 + lane], fb[480 + lane]) : 0.0;
-            const int gg = s.g + jb.g_off;
-            if (jb.ks > 1) {
-                const int slot = P.xo.dpart + ((gg * (kMaxKSplit - 1)) * 32 + lane) * 2;
-                if (s.sp != 0) {
-                    const unsigned long long bits = (unsigned long long)__double_as_longlong(v0);
-                    pub.local(slot + (s.sp - 1) * 64, (unsigned)bits);
-                    pub.local(slot + (s.sp - 1) * 64 + 1, (unsigned)(bits >> 32));
-                } else {
-                    unsigned pw[2 * (kMaxKSplit - 1)];
-                    const unsigned long long* base = P.xw + slot;
-                    const bool got = tw_poll(P, pub.tag, (1u << (2 * (jb.ks - 1))) - 1u, [&](int k) { return base + (k >> 1) * 64 + (k & 1); }, pw);   // all lanes, always
-                    ok = __all_sync(0xffffffffu, (ok && got) ? 1 : 0) != 0;
-                    if (ok) {
-                        #pragma unroll
-                        for (int q = 0; q < kMaxKSplit - 1; q++)
-                            if (q < jb.ks - 1) v0 = __dadd_rn(v0, __longlong_as_double((long long)(((unsigned long long)pw[2 * q + 1] << 32) | pw[2 * q])));
-                        epi(gg, lane, __double2float_rn(v0), 0.f, bv);
-                    }
-                }
-            } else {
-                epi(gg, lane, __double2float_rn(v0), __double2float_rn(v1), bv);
+__device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, const JobStart& st, int kb, int ks, bool two, int lane,
+                                            const int8_t* xq_s, const BlockScale* xs_s, const float* __restrict__ bias, const Pub& pub, Epi epi) {
+    bool ok = st.ok;
+    unsigned at = st.at;
+    if (!at) return ok;
+    const unsigned* work = sm.work;
+    WarpTile t = st.t;
+    float bv = st.bias;
+    for (;;) {
+        const unsigned list = work[at + kBatchList + ws.warp], head = work[at];
+        const unsigned* item = work + (list & 0xffffu);
+        int n = (int)(list >> 16);
+        if (n) {
+            double acc = 0.0;
+            for (;;) {
+                const unsigned it = *item++;
+                acc = t.dot(ws, lane, kb, (int)(it & 0xffffu), xq_s, xs_s, acc);
+                if (it >> 20 & 1u) { sm.fold[((it >> 16 & 7u) * DNW + ws.warp) * 32 + lane] = acc; acc = 0.0; }
+                if (--n == 0) break;
+                if (ok) ok = ws.acquire();
+                t.load(ws, lane, kb);
             }
         }
+        prof_mark(P, 18);
+        cta__syncthreads();
+        if (ws.warp < (int)(head & 255u)) {
+            const unsigned gg = work[at + kBatchGroup + ws.warp], u = work[at + kBatchUnit + ws.warp];
+            const double* f0 = sm.fold + ws.warp * (2 * DNW * 32) + lane;
+            double v0 = 0.0, v1 = 0.0;
+            #pragma unroll 1
+            for (int a = two ? 1 : 0; a >= 0; a--) {                    // up, then gate
+                const double* f = f0 + a * (DNW * 32);
+                const unsigned p0 = a ? u >> 20 : u >> 16;
+                const int n8 = (int)(u >> 8 & 15u);
+                double v[DNW];
+                #pragma unroll
+                for (int q = 0; q < DNW; q++) { const double x = f[((p0 + q) & (DNW - 1)) * 32]; v[q] = q < n8 ? x : 0.0; }
+                v1 = v0;
+                v0 = tree_sum8(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+            }
+            bool whole = true;
+            if (ks > 1) {
+                const int sp = (int)(u & 255u), to = P.xo.dpart + (((int)gg * (kMaxKSplit - 1)) * 32 + lane) * 2;
+                whole = sp == 0;
+                if (!whole) {
+                    const unsigned long long bits = (unsigned long long)__double_as_longlong(v0);
+                    pub.local(to + (sp - 1) * 64, (unsigned)bits);
+                    pub.local(to + (sp - 1) * 64 + 1, (unsigned)(bits >> 32));
+                } else {
+                    #pragma unroll 1
+                    for (int q = 0; q < ks - 1; q++) {
+                        const int off[1] = {to + q * 64};
+                        unsigned lo[1], hi[1];
+                        const bool got = tw_poll_pairs<1>(P, pub.tag, 1u, P.xw, off, lo, hi);      // all lanes, always
+                        ok = __all_sync(0xffffffffu, (ok && got) ? 1 : 0) != 0;
+                        v0 = __dadd_rn(v0, __hiloint2double((int)hi[0], (int)lo[0]));
+                    }
+                    whole = ok;
+                }
+            }
+            if (whole) epi((int)gg, lane, __double2float_rn(v0), __double2float_rn(v1), bv);
+        }
         prof_mark(P, 19);
+#if MI_LEAN
+        return ok;                                                      // (a range build runs only where one batch is all there is)
+#endif
+        at = head >> 8;
+        if (!at) return ok;
+        bv = batch_bias(work, at, ws.warp, lane, bias);
+        if (work[at + kBatchList + ws.warp] >> 16) {
+            if (ok) ok = ws.acquire();
+            t.load(ws, lane, kb);
+        }
+        cta__syncthreads();                                                // the sums have been read
     }
-    return ok;
 }
 
 // lm_head: a unit (row group) belongs to one warp; epi(g, lane, v).
 template <class Epi>
-__device__ __forceinline__ bool run_warp_job(WarpStream& ws, int j, int lane, const int8_t* xq_s, const float2* xs_s, Epi epi) {
-    const Job jb = ws.jobs[j];
+__device__ __forceinline__ bool run_warp_job(WarpStream& ws, int /* in phase order */, const DecodeParams& P, int lane, const int8_t* xq_s, const BlockScale* xs_s, Epi epi) {
+    const int nt = P.lm_nt, kb = P.kb[JOB_LM], n_units = P.lm_units, off = P.lm_off;
     bool ok = true;
-    for (int u = ws.first_warp_unit(jb); u < jb.n_units && ok; u += ws.W) {
+    WarpTile h;
+    for (int u = ws.warp * ws.ggrid + ws.gcta; u < n_units && ok; u += ws.ggrid * DNW) {       // (consecutive units land on different SMs)
         double acc = 0.0;
-        for (int t = 0; t < jb.nt; t++) acc = tile_consume(ws, lane, jb.kb, t, xq_s, xs_s, acc, ok);
-        if (ok) epi(u + jb.g_off, lane, __double2float_rn(acc));
+        for (int t = 0; t < nt && ok; t++) {
+            if (!(ok = ws.acquire())) break;
+            h.load(ws, lane, kb);
+            acc = h.dot(ws, lane, kb, t * kb, xq_s, xs_s, acc);
+        }
+        if (ok) epi(u + off, lane, __double2float_rn(acc));
     }
     return ok;
 }
@@ -622,213 +770,196 @@ __device__ __forceinline__ float warp_max_float(float a) {
 //       + the projection output published as tagged fp32 words at addw   [if addw]
 //   h = x;  the first GEMV CTA also commits x to global memory;
 //   xq_s / xs_s = q8_0( x * (1/sqrt(float(ss/n) + eps)) * w )   (src/cpu_infer.cpp:40-46).
-// Two thread mappings.  Gathering (tagged words in, residual add, sum of squares): warp w owns the 32-element blocks
-// w, w+8, ...; lane = element, so every warp-wide load of tagged words is one contiguous 256-byte run and all of a
-// thread's words are requested before anything waits on them.  Quantizing (after the sum of squares is known): EPL
-// consecutive elements per thread, 32/EPL threads per q8_0 block, read back from shared memory; the block maximum and the
-// block sum fold over 32/EPL lanes with log2(32/EPL) shuffles.  (One element per thread and warp-wide REDUX reductions,
-// twelve per warp at the 1.5B shape, measured 1500 cycles for the quantizer alone: the reduction unit, not the
-// arithmetic, set the time.)  Sum of squares in double (every x*x is exact there).
+// What bounds it is a chain of latencies behind the last word that arrives, so a thread keeps its elements in registers from the words to the int8
+// values and nothing on the way branches (a branch, taken or not, is some 16 clocks, an integer operation 2 per warp).  Warp w owns the runs of 64
+// elements w, w+8, ...; a lane has two consecutive ones of each, so a warp's load of tagged words is one contiguous 512-byte run of
+// 16-byte pairs, and a q8_0 block is half a warp.  Sum of squares in double (every x*x is exact there); the lanes' sums are added by two FP64 MMAs
+// against ones (the first adds four lanes each and leaves two of eight sums per lane, the second adds the four pairs), where five rounds of 64-bit shuffles took three
+// times as long.
 // h_s must hold the residual stream already (residual_init below puts the embedding row, or the copy committed to global
 // memory, there with this same thread mapping, so no barrier is needed in between).
-template <int NB, int EPL>
-__device__ __forceinline__ bool stage_norm_q8_t(const DecodeParams& P, float* h_s,
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+__device__ __forceinline__ double warp_sum(double v) {
+    double c[2] = {0.0, 0.0}, d[2] = {0.0, 0.0};
+    dmma884(c, 1.0, v);
+    dmma884(d, 1.0, __dadd_rn(c[0], c[1]));
+    return d[0];
+}
+// ok: whether this warp's part of the phase before was complete.
+template <int NC>
+__device__ __forceinline__ bool stage_norm_q8_t(bool ok, const DecodeParams& P, float* h_s,
                                                 const unsigned long long* addw, unsigned tag, float* commit, const float* __restrict__ w,
-                                                int E, float eps, double* red, int8_t* xq_s, float2* xs_s) {
-    constexpr int LPB = 32 / EPL;                        // lanes per block while quantizing
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nb = E / 32;
-    // the norm weights of the quantizing pass: requested now, used after the barrier
-    const int qt_b = tid / LPB, qt_e0 = tid * EPL;
-    const bool qlive = qt_b < nb;
-    float wv[EPL];
-    #pragma unroll
-    for (int i = 0; i < EPL; i++) wv[i] = __ldg(w + (qlive ? qt_e0 : 0) + i);
-    float x[NB];
+                                                int E, float eps, double* red, int8_t* xq_s, BlockScale* xs_s) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float2 x[NC], wv[NC];
+    int e[NC];
     unsigned valid = 0;
     #pragma unroll
-    for (int k = 0; k < NB; k++) {
-        const int b = min(warp + k * DNW, nb - 1), e = b * 32 + lane;      // clamped: every address is valid
-        if (warp + k * DNW < nb) valid |= 1u << k;
-        x[k] = h_s[e];
+    for (int k = 0; k < NC; k++) {
+        const int at = (warp + k * DNW) * 64 + 2 * lane;
+        valid |= at < E ? 1u << k : 0u;
+        e[k] = at < E ? at : 0;                              // every address is valid; a lane past the vector stores nothing
+        wv[k] = __ldg(reinterpret_cast<const float2*>(w + e[k]));
+        x[k] = *reinterpret_cast<const float2*>(h_s + e[k]);
     }
-    bool ok = true;
     if (addw) {
-        unsigned aw[NB];
+        unsigned a[NC], b[NC];
         prof_mark(P, 27);
-        ok = tw_poll(P, tag, valid, [&](int k) { return addw + (size_t)(warp + k * DNW) * 32 + lane; }, aw);
+        ok = tw_poll_pairs<NC>(P, tag, (1u << NC) - 1u, addw, e, a, b) && ok;
         prof_mark(P, kProfWait);
         #pragma unroll
-        for (int k = 0; k < NB; k++) if (valid >> k & 1u) x[k] = __fadd_rn(x[k], __uint_as_float(aw[k]));
+        for (int k = 0; k < NC; k++) { x[k].x = __fadd_rn(x[k].x, __uint_as_float(a[k])); x[k].y = __fadd_rn(x[k].y, __uint_as_float(b[k])); }
         prof_mark(P, 28);
     }
     double s2[2] = {0.0, 0.0};                           // two chains
     #pragma unroll
-    for (int k = 0; k < NB; k++) {
-        if (valid >> k & 1u) {
-            const int e = (warp + k * DNW) * 32 + lane;
-            h_s[e] = x[k];
-            if (commit && (int)blockIdx.x == P.attn_ctas) __stcg(commit + e, x[k]);
-            const double xd = x[k]; s2[k & 1] = __fma_rn(xd, xd, s2[k & 1]);
-        }
+    for (int k = 0; k < NC; k++) {
+        const bool live = valid >> k & 1u;
+        const double x0 = live ? x[k].x : 0.f, x1 = live ? x[k].y : 0.f;
+        s2[0] = __fma_rn(x0, x0, s2[0]); s2[1] = __fma_rn(x1, x1, s2[1]);
     }
-    double ss = __dadd_rn(s2[0], s2[1]);
-    #pragma unroll
-    for (int o = 16; o; o >>= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+    const double ss = warp_sum(__dadd_rn(s2[0], s2[1]));
     if (lane == 0) red[warp] = ss;
+    #pragma unroll
+    for (int k = 0; k < NC; k++) if (valid >> k & 1u) *reinterpret_cast<float2*>(h_s + e[k]) = x[k];
+    if (commit && (int)blockIdx.x == P.attn_ctas) {
+        #pragma unroll
+        for (int k = 0; k < NC; k++) if (valid >> k & 1u) __stcg(reinterpret_cast<float2*>(commit + e[k]), x[k]);
+    }
     prof_mark(P, 23);
-    if (!__syncthreads_and(ok ? 1 : 0)) return false;
+    if (!cta__syncthreads_and(ok ? 1 : 0)) return false;
     prof_mark(P, 24);
-    const float mean = __double2float_rn(div_known(tree_sum8(red[0], red[1], red[2], red[3], red[4], red[5], red[6], red[7]), (double)E, P.inv_e));
+    const double2* r2 = reinterpret_cast<const double2*>(red);
+    const double2 ra = r2[0], rb = r2[1], rc = r2[2], rd = r2[3];
+    const float mean = __double2float_rn(div_known(tree_sum8(ra.x, ra.y, rb.x, rb.y, rc.x, rc.y, rd.x, rd.y), (double)E, P.inv_e));
     const float scale = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(mean, eps)));
-    // quantize: this thread's EPL elements of block qt_b (vectors beyond 256 * EPL elements: further rounds)
-    for (int t = tid; (t & ~31) / LPB < nb; t += DNT) {              // warp-uniform trip count: the folds below are warp-wide
-        const int b = t / LPB;
-        const bool live = b < nb;
-        const int e0 = live ? t * EPL : 0;                            // a lane past the vector computes on block 0 and stores nothing
-        float v[EPL], a = 0.f;
+    float m[NC];
+    #pragma unroll
+    for (int k = 0; k < NC; k++) {
+        x[k].x = __fmul_rn(__fmul_rn(x[k].x, scale), wv[k].x); x[k].y = __fmul_rn(__fmul_rn(x[k].y, scale), wv[k].y);
+        m[k] = fmaxf(fmaxf(0.f, fabsf(x[k].x)), fabsf(x[k].y));        // (a NaN does not count)
+    }
+    #pragma unroll
+    for (int o = 1; o < 16; o <<= 1)
         #pragma unroll
-        for (int i = 0; i < EPL; i++) {
-            const float wi = t == tid ? wv[i] : __ldg(w + e0 + i);
-            v[i] = __fmul_rn(__fmul_rn(h_s[e0 + i], scale), wi); a = fmaxf(a, fabsf(v[i]));
+        for (int k = 0; k < NC; k++) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+    // one division for up to eight runs: lane 2 k of a half warp has 127 / (its half's maximum of run k), lane 2 k + 1 that maximum / 127
+    // (a division has a branch: two for each run were half of this pass)
+    #pragma unroll
+    for (int k0 = 0; k0 < NC; k0 += 8) {
+        const int mk = k0 + ((lane & 15) >> 1);
+        float a = m[k0];
+        #pragma unroll
+        for (int k = k0 + 1; k < k0 + 8 && k < NC; k++) if (mk == k) a = m[k];
+        const bool odd = lane & 1;
+        const float d = __fdiv_rn(odd ? a : 127.f, odd ? 127.f : a);
+        const int mine = (warp + mk * DNW) * 64 + 2 * (lane & 16);          // first element of the lane's block
+        int sum[8];
+        #pragma unroll
+        for (int k = k0; k < k0 + 8 && k < NC; k++) {
+            const float iv = __shfl_sync(0xffffffffu, d, (lane & 16) + 2 * (k - k0)), inv = m[k] > 0.f ? iv : 0.f;
+            const int q0 = __float2int_rn(__fmul_rn(x[k].x, inv)), q1 = __float2int_rn(__fmul_rn(x[k].y, inv));
+            if (valid >> k & 1u) *reinterpret_cast<unsigned short*>(xq_s + e[k]) = (unsigned short)__byte_perm((unsigned)q0, (unsigned)q1, 0x0040);
+            sum[k - k0] = q0 + q1;
         }
         #pragma unroll
-        for (int o = 1; o < LPB; o <<= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-        const float inv = a > 0.f ? __fdiv_rn(127.f, a) : 0.f;
-        int q[EPL], sq = 0;
+        for (int o = 1; o < 16; o <<= 1)
+            #pragma unroll
+            for (int k = k0; k < k0 + 8 && k < NC; k++) sum[k - k0] += __shfl_xor_sync(0xffffffffu, sum[k - k0], o);
+        int sm = sum[0];
         #pragma unroll
-        for (int i = 0; i < EPL; i++) { q[i] = __float2int_rn(__fmul_rn(v[i], inv)); sq += q[i]; }
-        #pragma unroll
-        for (int o = 1; o < LPB; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (live) {
-            if constexpr (EPL >= 4) {
-                #pragma unroll
-                for (int i = 0; i < EPL; i += 4)
-                    *reinterpret_cast<unsigned*>(xq_s + e0 + i) = (unsigned)(q[i] & 0xff) | ((unsigned)(q[i + 1] & 0xff) << 8) |
-                                                                  ((unsigned)(q[i + 2] & 0xff) << 16) | ((unsigned)(q[i + 3] & 0xff) << 24);
-            } else {
-                #pragma unroll
-                for (int i = 0; i < EPL; i++) xq_s[e0 + i] = (int8_t)q[i];
-            }
-            if ((t % LPB) == 0) xs_s[b] = make_float2(__half2float(__float2half_rn(__fdiv_rn(a, 127.f))), __int2float_rn(8 * sq));
-        }
+        for (int k = k0 + 1; k < k0 + 8 && k < NC; k++) if (mk == k) sm = sum[k - k0];
+        if (odd && mk < NC && mine < E) xs_s[mine >> 5] = block_scale(__half2float(__float2half_rn(d)), sm);
     }
     prof_mark(P, 25);
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 26);
     return true;
 }
+
+// The compiler knows nothing of k from here on: it would otherwise make a copy of what follows for each value that k has had.
+__device__ __forceinline__ void same_code(int& k) { asm volatile("" : "+r"(k)); }
 
 // The residual stream into this CTA's shared memory, where a step or a launch begins: the embedding row of `token`
 // (value (nibble - 8) * d, src/gguf.h:94-102; or a Q8_0 row as stored, int8 * d, src/gguf.h:112-118 and src/mega.cu:639-642),
 // or the copy the first GEMV CTA committed to global memory (a launch that starts in mid-step).  Thread mapping of the norm
 // prologue's gathering pass: each thread later reads only what it wrote here.
 __device__ __forceinline__ void residual_init(const DecodeParams& P, float* h_s, const float* gsrc, int token, int E) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nb = E / 32;
-    for (int b = warp; b < nb; b += DNW) {
-        const int e = b * 32 + lane;
-        float x;
-        if (gsrc) x = __ldcg(gsrc + e);
+    const int tid = threadIdx.x, nb = E / 32;
+    #pragma unroll 1
+    for (int e = 2 * tid; e < E; e += 2 * DNT) {
+        const int b = e >> 5, i = e & 31;                  // elements i and i + 1 of block b
+        float2 x;
+        if (gsrc) x = __ldcg(reinterpret_cast<const float2*>(gsrc + e));
         else if (P.emb_q8) {
             const uint8_t* bp = P.emb_q8 + ((size_t)token * nb + b) * 34;
-            x = __fmul_rn(__int2float_rn((int)(int8_t)__ldg(bp + 2 + lane)), __half2float(__ldg(reinterpret_cast<const __half*>(bp))));
+            const float d = __half2float(__ldg(reinterpret_cast<const __half*>(bp)));
+            const unsigned q = __ldg(reinterpret_cast<const unsigned short*>(bp + 2 + i));
+            x = make_float2(__fmul_rn(__int2float_rn((int)(int8_t)(q & 0xff)), d), __fmul_rn(__int2float_rn((int)(int8_t)(q >> 8)), d));
         } else {
             const int g = token >> 5, r = token & 31, kb = P.emb_kb, t = b / kb, kk = b % kb;
             const uint8_t* tile = P.emb_base + ((size_t)g * P.emb_nt + t) * (kb * kTileRowBytes);
-            const uint8_t byte = __ldg(tile + ((size_t)kk * 32 + r) * 16 + (lane & 15));
+            const unsigned q = (unsigned)__ldg(reinterpret_cast<const unsigned short*>(tile + ((size_t)kk * 32 + r) * 16 + (i & 15))) >> (i < 16 ? 0 : 4);
             const float d = __half2float(__ldg(reinterpret_cast<const __half*>(tile + (size_t)kb * 512 + ((size_t)r * kb + kk) * 2)));
-            x = __fmul_rn(__int2float_rn((lane < 16 ? (byte & 0x0F) : (byte >> 4)) - 8), d);
+            x = make_float2(__fmul_rn(__int2float_rn((int)(q & 15) - 8), d), __fmul_rn(__int2float_rn((int)(q >> 8 & 15) - 8), d));
         }
-        h_s[e] = x;
+        *reinterpret_cast<float2*>(h_s + e) = x;
     }
 }
 
-#define MI_NORM_ARGS const DecodeParams& P, float* h_s, const unsigned long long* addw, unsigned tag, \
-                     float* commit, const float* __restrict__ w, int E, float eps, double* red, int8_t* xq_s, float2* xs_s
-#define MI_NORM_PASS P, h_s, addw, tag, commit, w, E, eps, red, xq_s, xs_s
-// blocks per warp while gathering (NB) and elements per thread while quantizing (EPL: the largest of 8, 4, 2, 1 with
-// which 256 threads cover the vector, 8 in several rounds beyond 2048 elements)
+#define MI_NORM_ARGS bool ok, const DecodeParams& P, float* h_s, const unsigned long long* addw, unsigned tag, \
+                     float* commit, const float* __restrict__ w, int E, float eps, double* red, int8_t* xq_s, BlockScale* xs_s
+#define MI_NORM_PASS ok, P, h_s, addw, tag, commit, w, E, eps, red, xq_s, xs_s
+// runs of 64 elements per warp (NC): as many as the widest vector of a call needs
 static __device__ __noinline__ bool stage_norm_q8_rare(MI_NORM_ARGS) {
-    if (E <= 256) return stage_norm_q8_t<1, 1>(MI_NORM_PASS);
-    if (E <= 512) return stage_norm_q8_t<2, 2>(MI_NORM_PASS);
-    if (E <= 1024) return stage_norm_q8_t<4, 4>(MI_NORM_PASS);
-    if (E <= 4096) return stage_norm_q8_t<16, 8>(MI_NORM_PASS);
-    return stage_norm_q8_t<32, 8>(MI_NORM_PASS);
+    if (E <= 512) return stage_norm_q8_t<1>(MI_NORM_PASS);
+    if (E <= 1024) return stage_norm_q8_t<2>(MI_NORM_PASS);
+    if (E <= 4096) return stage_norm_q8_t<8>(MI_NORM_PASS);
+    return stage_norm_q8_t<16>(MI_NORM_PASS);
 }
+// NC_MAX: the most that a model of this head shape has in a range build
+template <int NC_MAX>
 __device__ __forceinline__ bool stage_norm_q8u(MI_NORM_ARGS) {
 #if MI_LEAN
-    return stage_norm_q8_t<MI_SMALL ? 4 : 8, MI_SMALL ? 4 : 8>(MI_NORM_PASS);           // lean_shape(): 1024 < E <= 2048, or (small build) 512 < E <= 1024
+    return stage_norm_q8_t<NC_MAX>(MI_NORM_PASS);           // lean_shape(): 1024 < E <= 2048, or (small build) 512 < E <= 1024
 #else
-    if (E > 1024 && E <= 2048) return stage_norm_q8_t<8, 8>(MI_NORM_PASS);
+    if (E > 1024 && E <= 2048) return stage_norm_q8_t<4>(MI_NORM_PASS);
     return stage_norm_q8_rare(MI_NORM_PASS);
 #endif
 }
+// E is a multiple of HD * G: the largest one within the range build's widths, in runs of 64 over the warps
+__host__ __device__ constexpr int norm_chunks(int HD, int G) { return ((MI_SMALL ? 1024 : 2048) / (HD * G) * (HD * G) + 64 * DNW - 1) / (64 * DNW); }
 
-// A q8_0 vector published as tagged words by other CTAs -> shared memory: int8 values, and per block {fp32 of the fp16
-// scale, float(8 * sum of the block's values)}.  Thread t takes the 16-byte word pairs t, t + 256, ...; all of a
+// A q8_0 vector published as tagged words by other CTAs -> shared memory: int8 values, and per block what
+// tile_dot wants of its scale and sum.  Thread t takes the 16-byte word pairs t, t + 256, ... of the values (NV at most) and of the scales (NS); all of a
 // thread's loads are in flight together.
-template <int NP>
-__device__ __forceinline__ bool stage_poll_q8_t(const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, float2* xs_s) {
-    const int tid = threadIdx.x, nq2 = n / 8, tot2 = nq2 + (n / 32 + 1) / 2, nbk = n / 32;     // pairs of value words, all pairs, blocks
-    unsigned long long w[NP][2];
+template <int NV, int NS>
+__device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
+    const int tid = threadIdx.x, nq2 = n / 8, nbk = n / 32;
+    int off[NV + NS];
+    unsigned valid = 0, a[NV + NS], b[NV + NS];
     #pragma unroll
-    for (int k = 0; k < NP; k++) {
-        const int pr = tid + k * DNT;
-        if (pr < tot2) tw_ld2(vw + 2 * pr, w[k][0], w[k][1]);
-        else w[k][0] = w[k][1] = (unsigned long long)tag << 32;
-        if (pr == tot2 - 1 && (nbk & 1)) w[k][1] = (unsigned long long)tag << 32;      // odd block count: the pad word is never written
+    for (int k = 0; k < NV + NS; k++) {
+        const int pr = tid + (k < NV ? k : k - NV) * DNT;
+        off[k] = k < NV ? 2 * pr : 2 * nq2 + 2 * pr;
+        valid |= (k < NV ? pr < nq2 : 2 * pr < nbk) ? 1u << k : 0u;
     }
-    bool ok = true;
-    for (unsigned round = 0;; round++) {
-        const unsigned long long* miss = nullptr;
-        #pragma unroll
-        for (int k = NP - 1; k >= 0; k--) {
-            if (!tw_is(w[k][1], tag)) miss = vw + 2 * (tid + k * DNT) + 1;
-            if (!tw_is(w[k][0], tag)) miss = vw + 2 * (tid + k * DNT);
-        }
-        const int st = tw_wait_warp(miss, tag, P.wait_ns, P.err, round);
-        if (st == 0) break;
-        if (st < 0) { ok = false; break; }
-        #pragma unroll
-        for (int k = 0; k < NP; k++) {
-            if (!tw_is(w[k][0], tag) || !tw_is(w[k][1], tag)) {
-                const int pr = tid + k * DNT;
-                tw_ld2(vw + 2 * pr, w[k][0], w[k][1]);
-                if (pr == tot2 - 1 && (nbk & 1)) w[k][1] = (unsigned long long)tag << 32;
-            }
-        }
-    }
+    ok = tw_poll_pairs<NV + NS, NS>(P, tag, valid, vw, off, a, b, nbk & 1 ? 2 * nq2 + nbk : -1) && ok;
     #pragma unroll
-    for (int k = 0; k < NP; k++) {
-        const int pr = tid + k * DNT;
-        if (pr < nq2) {
-            reinterpret_cast<uint2*>(xq_s)[pr] = make_uint2((unsigned)w[k][0], (unsigned)w[k][1]);
-        } else if (pr < tot2) {
-            #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int b = 2 * (pr - nq2) + h;
-                if (b < nbk) {
-                    const unsigned sw = (unsigned)w[k][h];
-                    xs_s[b] = make_float2(__half2float(__ushort_as_half((unsigned short)(sw & 0xffffu))), __int2float_rn(8 * (int)(short)(sw >> 16)));
-                }
-            }
-        }
+    for (int k = 0; k < NV; k++) if (valid >> k & 1u) reinterpret_cast<uint2*>(xq_s)[tid + k * DNT] = make_uint2(a[k], b[k]);
+    #pragma unroll
+    for (int k = NV; k < NV + NS; k++) {
+        auto scale = [](unsigned sw) { return block_scale(__half2float(__ushort_as_half((unsigned short)(sw & 0xffffu))), (int)(short)(sw >> 16)); };
+        const int blk = off[k] - 2 * nq2;
+        if (valid >> k & 1u) { xs_s[blk] = scale(a[k]); if (blk + 1 < nbk) xs_s[blk + 1] = scale(b[k]); }
     }
-    return __syncthreads_and(ok ? 1 : 0) != 0;
+    return cta__syncthreads_and(ok ? 1 : 0) != 0;
 }
-static __device__ __noinline__ bool stage_poll_q8_rare(const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, float2* xs_s) {
-    const int np = (q8_words(n) / 2 + DNT - 1) / DNT;
-    if (np <= 8) return stage_poll_q8_t<8>(P, vw, n, tag, xq_s, xs_s);
-    return stage_poll_q8_t<18>(P, vw, n, tag, xq_s, xs_s);
-}
-__device__ __forceinline__ bool stage_poll_q8(const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, float2* xs_s) {
-    const int np = (q8_words(n) / 2 + DNT - 1) / DNT;
-    if (np <= 1) return stage_poll_q8_t<1>(P, vw, n, tag, xq_s, xs_s);
-    if (np <= 5) return stage_poll_q8_t<5>(P, vw, n, tag, xq_s, xs_s);
-#if MI_LEAN
-    return stage_poll_q8_t<8>(P, vw, n, tag, xq_s, xs_s);                               // lean_shape(): at most 8 word pairs per thread
-#else
-    return stage_poll_q8_rare(P, vw, n, tag, xq_s, xs_s);
-#endif
+// as many pairs as the longest vector wants; one form per build, so that all phases run the same instructions (lean_shape(): at most 8 pairs of values per thread)
+__device__ __forceinline__ bool stage_poll_q8(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
+    return stage_poll_q8_t<MI_LEAN ? 8 : 16, MI_LEAN ? 1 : 2>(ok, P, vw, n, tag, xq_s, xs_s);
 }
 
 // Shapes the context-range builds take: they hold one variant of each prologue and of the tile loop and no call to the others.
@@ -854,9 +985,6 @@ inline int lean_shape(int E, int FF, int NQ) {
 //     arrive read 460 KB alone.
 // Scores: double dot products rounded to fp32 once, scaled in fp32; weights, denominator and sums in double, running maximum across
 // steps, common maximum across chunks.  Returns false if a wait gave up (CTA-uniform).
-__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
-}
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -899,7 +1027,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
         #pragma unroll
         for (int k = 0; k < QN; k++) if (tid + k * DNT < G * HD) valid |= 1u << k;
         if (has_new && tid < HD) valid |= 3u << QN;
-        const unsigned long long* qv = P.xw + P.xo.qkv;
+        const unsigned long long* qv = xw_read(P) + P.xo.qkv;
         const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;
         const bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
             if (k < QN) {
@@ -934,7 +1062,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                 reinterpret_cast<__half*>(ks + (pos - b0) * KLD)[tid] = knew;
                 reinterpret_cast<__half*>(vs + (pos - b0) * VLD)[tid] = vnew;
             }
-            if (s == 0) { if (!__syncthreads_and(okq ? 1 : 0)) { ok = false; break; } } else __syncthreads();
+            if (s == 0) { if (!cta__syncthreads_and(okq ? 1 : 0)) { ok = false; break; } } else cta__syncthreads();
             // scores: warp = every 8th group of 8 positions
             #pragma unroll 1
             for (int t = warp; t * 8 < np; t += DNW) {
@@ -956,7 +1084,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                     if (pp < SUB) sc[g * SCL + pp] = pp < np ? __fmul_rn(__double2float_rn(__dadd_rn(c[0][e], c[1][e])), inv) : -INFINITY;
                 }
             }
-            __syncthreads();
+            cta__syncthreads();
             prof_mark(P, 27);
             if (s + 1 < nsub) copy_rows(ks, KLD, P.kc, s + 1); else cp_async_commit();
             // weights: one warp per head
@@ -983,7 +1111,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                 }
             }
             cp_async_wait<1>();                     // the V rows
-            __syncthreads();
+            cta__syncthreads();
             prof_mark(P, 29);
             // values: warp = HD/8 dims, all positions
             if (warp < VW) {
@@ -1011,7 +1139,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                     }
                 }
             }
-            __syncthreads();                        // scores, weights and V rows may be written again
+            cta__syncthreads();                        // scores, weights and V rows may be written again
             if (s + 1 < nsub) copy_rows(vs, VLD, P.vc, s + 1);
         }
         if (!ok) cp_async_wait<0>();                // copies in flight target the staging area
@@ -1025,7 +1153,7 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
                     for (int e = 0; e < 2; e++) __stcg(gp + warp * (8 * NTW) + (2 * t4 + e) * NTW + i, __dadd_rn(o[0][i][e], o[1][i][e]));
             }
             if (tid < G) __stcg(P.attn_part + ((size_t)(h0 + tid) * P.max_chunks + ch) * SW + HD, rl[tid]);
-            __syncthreads();
+            cta__syncthreads();
             if (tid < G) {
                 fence_acq_rel_gpu();                // the partial, and the new position's rows, before the word that announces them
                 pub.local(P.xo.attm + (h0 + tid) * P.max_chunks + ch, __float_as_uint((float)rm[tid]));
@@ -1073,10 +1201,10 @@ __device__ __forceinline__ bool attention_split(const DecodeParams& P, int l, in
         }
         #pragma unroll
         for (int q = 16; q; q >>= 1) lb = __dadd_rn(lb, __shfl_xor_sync(0xffffffffu, lb, q));
-        __syncthreads();                            // the buffer below is free (a second block of this CTA)
+        cta__syncthreads();                            // the buffer below is free (a second block of this CTA)
         red[warp * 33 + lane] = ob;
         if (lane == 0) red[warp * 33 + 32] = lb;
-        ok = __syncthreads_and(okm ? 1 : 0) != 0;
+        ok = cta__syncthreads_and(okm ? 1 : 0) != 0;
         if (warp == 0 && ok) {
             double den = red[32];
             ob = red[lane];
@@ -1121,7 +1249,7 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
     const int nq = P.NH * HD;
     unsigned qw[3], valid = 0;
     if (tid < HD) valid = 7u;
-    const unsigned long long* qv = P.xw + P.xo.qkv;
+    const unsigned long long* qv = xw_read(P) + P.xo.qkv;
     const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;    // packed slot of dim `tid`
     const bool okq = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
         return k == 0 ? qv + (size_t)head * HD + dk : k == 1 ? qv + nq + (size_t)kvh * HD + dk : qv + nq + P.KVD + (size_t)kvh * HD + tid;
@@ -1132,7 +1260,7 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
         P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[1]));
         P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = __float2half_rn(__uint_as_float(qw[2]));
     }
-    if (!__syncthreads_and(okq ? 1 : 0)) return false;
+    if (!cta__syncthreads_and(okq ? 1 : 0)) return false;
     prof_mark(P, 14);
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
     const int a0 = (int)((long long)Lp * warp / DNW), a1 = (int)((long long)Lp * (warp + 1) / DNW);      // at most 32 positions
@@ -1204,7 +1332,7 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
     };
     if (np > 0) load_v(0);
     prof_mark(P, 28);
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 15);
     // maximum over the whole range (every warp scans all scores), then one weight per thread
     float mx = -INFINITY;
@@ -1213,7 +1341,7 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
     mx = warp_max_float(mx);
     if (tid < Lp) wt[tid] = exp_shared((double)sc[tid] - (double)mx);
     prof_mark(P, 29);
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 30);
     // pass 2
     double o[DPW], ls = 0.0;
@@ -1250,7 +1378,7 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
     prof_mark(P, 31);
     // the new position's K / V rows (plain stores above) are performed before anything this CTA publishes
     if (tid < HD) __threadfence();
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 16);
     if (warp < DPW) {
         const int d = warp * 32 + lane;
@@ -1300,7 +1428,7 @@ __device__ __forceinline__ void attn_prefetch_issue(const DecodeParams& P, uint8
     pf.layer = layer; pf.pos = pos; pf.pending = pos > 0;
     if (pos <= 0) return;
     if (tid == 0) { fence_proxy_async(); mbar_expect_tx(pf.bar, 2u * (unsigned)pos * (2u * HD)); }
-    __syncthreads();
+    cta__syncthreads();
     uint8_t* Kb = smem; uint8_t* Vb = smem + (size_t)kAttnRows * RSB;
     for (int p = tid; p < pos; p += DNT) {
         const size_t row = ((size_t)layer * P.max_seq + p) * P.KVD + (size_t)kvh * HD;
@@ -1334,7 +1462,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
     #pragma unroll
     for (int k = 0; k < QN; k++) if (tid + k * DNT < HPC * HD) valid |= 1u << k;
     if (tid < HD) valid |= 3u << QN;
-    const unsigned long long* qv = P.xw + P.xo.qkv;
+    const unsigned long long* qv = xw_read(P) + P.xo.qkv;
     const int dk = tid < HD / 2 ? 2 * tid : 2 * (tid - HD / 2) + 1;
     bool ok = tw_poll(P, tag_in, valid, [&](int k) -> const unsigned long long* {
         if (k < QN) {
@@ -1355,7 +1483,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
     }
     prof_mark(P, 14);
     if (ok && pf.pending) { ok = mbar_wait_bounded(pf.bar, pf.parity); pf.parity ^= 1u; pf.pending = false; }
-    if (!__syncthreads_and(ok ? 1 : 0)) { pf.ok = false; return pf; }
+    if (!cta__syncthreads_and(ok ? 1 : 0)) { pf.ok = false; return pf; }
     prof_mark(P, 27);
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
     const int a0 = (int)((long long)Lp * warp / DNW), a1 = (int)((long long)Lp * (warp + 1) / DNW), np = a1 - a0;
@@ -1394,7 +1522,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
             for (int j = 0; j < HPC; j++) pd[(warp * HPC + j) * kAttnRows + p0 + lane] = __dadd_rn(acc[j][0], acc[j][1]);
         }
     }
-    __syncthreads();
+    cta__syncthreads();
     if (tid < Lp) {
         #pragma unroll
         for (int j = 0; j < HPC; j++) {
@@ -1403,7 +1531,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
             sc[j * kAttnRows + tid] = __fmul_rn(__double2float_rn(tree_sum8(p[0], p[S], p[2 * S], p[3 * S], p[4 * S], p[5 * S], p[6 * S], p[7 * S])), inv);
         }
     }
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 15);
     // per head: maximum over the whole range, then one weight per (head, position)
     float mx[HPC];
@@ -1422,7 +1550,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
         wt[j * kAttnRows + p] = exp_shared((double)sc[j * kAttnRows + p] - (double)mj);
     }
     prof_mark(P, 29);
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 30);
     // pass 2: lane = the dim pairs {2 lane, 2 lane + 1} + 64 jj (head_dim 32: lane = dim)
     constexpr int VP = DPW >= 2 ? DPW / 2 : 1;
@@ -1466,7 +1594,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
         if (lane == 0) lw[warp * HPC + j] = ls[j];
     }
     prof_mark(P, 31);
-    __syncthreads();
+    cta__syncthreads();
     prof_mark(P, 16);
     // finish: one 32-dim block of one head per warp and round
     for (int b = warp; b < HPC * DPW; b += DNW) {
@@ -1490,7 +1618,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
         __threadfence();
         fence_proxy_async();
     }
-    __syncthreads();                                  // the buffer is free, the stores are fenced
+    cta__syncthreads();                                  // the buffer is free, the stores are fenced
     if (next_layer >= 0 && next_pos + 1 <= kShortAttnMax) attn_prefetch_issue<HD>(P, smem, pf, next_layer, next_pos, kvh);
     else { pf.layer = -1; pf.pending = false; }
     pf.ok = true;
@@ -1532,10 +1660,10 @@ static __device__ __noinline__ bool rows_ordered(const DecodeParams& P, unsigned
     for (int i0 = 0; i0 < n && ok; i0 += DNT) {
         const int i = i0 + (int)threadIdx.x;
         unsigned w[1];
-        ok = tw_poll(P, tag, i < n ? 1u : 0u, [&](int) { return P.xw + (i < n_cand ? P.xo.cand + i * 4 : done + i - n_cand); }, w);
+        ok = tw_poll(P, tag, i < n ? 1u : 0u, [&](int) { return i < n_cand ? xw_read(P) + P.xo.cand + i * 4 : P.xw + done + i - n_cand; }, w);
     }
     fence_acq_rel_gpu();
-    return __syncthreads_and(ok ? 1 : 0) != 0;
+    return cta__syncthreads_and(ok ? 1 : 0) != 0;
 }
 
 template <int HD, int G>
@@ -1560,7 +1688,7 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
             // the stop rule: learn the token the previous step picked (its lm_head phase carries tag tag0 - 1)
             unsigned tw[1];
             const bool got = tw_poll(P, tag0 - 1u, 1u, [&](int) { return P.xw + P.xo.tokw; }, tw);
-            ok = __syncthreads_and(got ? 1 : 0) != 0;
+            ok = cta__syncthreads_and(got ? 1 : 0) != 0;
             if (!ok || (int)tw[0] == P.stop_token) break;
         }
         // (only a launch over whole steps has more than one)
@@ -1568,7 +1696,7 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
         for (int l = max(0, (ph0 + 3) / 5); 5 * l + 1 < ph1 && l < P.L && ok; l++) {
             const int ph = 5 * l + 1;
             Pub pub;
-            pub.xw = P.xw; pub.tag = tag0 + (unsigned)ph; pub.mute = ph == P.drop_phase;
+            pub.xw = P.xw; pub.tag = tag0 + (unsigned)ph; pub.mute = ph == P.drop_phase; pub.stride = P.xo.total;
 #if MI_TP
             pub.tp = &P.tp;
 #endif
@@ -1590,7 +1718,7 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
 #elif MI_LEAN == 2
             ok = attention_split<HD, G>(P, l, pos, stage, pub.tag - 1u, pub);
 #endif
-            ok = __syncthreads_and(ok ? 1 : 0) != 0;
+            ok = cta__syncthreads_and(ok ? 1 : 0) != 0;
             prof_mark(P, 3);
         }
         if (kRowsCross && ok && ph1 == nph && threadIdx.x == 0) {
@@ -1601,7 +1729,7 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
 #if MI_PROF
     if (P.prof && (int)blockIdx.x == P.prof_cta) {
         if (threadIdx.x == 0) { s_prof[8] = (unsigned long long)(clock64() - prof_c0); s_prof[9] = gtime_ns() - prof_t0; }
-        __syncthreads();
+        cta__syncthreads();
         if (threadIdx.x < kProfSlots) P.prof[threadIdx.x] += s_prof[threadIdx.x];
     }
 #endif
@@ -1611,7 +1739,7 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
 
 // ---- the kernel ---------------------------------------------------------------------
 template <int HD, int G>
-__global__ void __launch_bounds__(DNT, 1)
+__global__ void __launch_bounds__(DNT_ALL, 1)
 decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int ph0, int ph1) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1619,8 +1747,8 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
     DecodeSmem sm;
     sm.ring = smem;
     sm.bars = reinterpret_cast<uint64_t*>(smem + (size_t)DNW * DS * DSLOT);
-    sm.jobs = reinterpret_cast<Job*>(smem + (size_t)DNW * DS * DSLOT + 256);
-    uint8_t* after_jobs = reinterpret_cast<uint8_t*>(sm.jobs) + ((size_t)njobs * sizeof(Job) + 127) / 128 * 128;
+    unsigned* work_s = reinterpret_cast<unsigned*>(smem + (size_t)DNW * DS * DSLOT + 512);
+    uint8_t* after_jobs = reinterpret_cast<uint8_t*>(work_s + kWorkSmem);
     sm.lp = reinterpret_cast<LayerPtrs*>(after_jobs);              // [<= 64]
     after_jobs += 64 * sizeof(LayerPtrs);
     sm.cs = reinterpret_cast<float*>(after_jobs);                 // [HD]: cos then sin
@@ -1630,27 +1758,32 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
     sm.stage = after_jobs + 1024 + 256 + kFoldBytes + ((size_t)P.E * 4 + 127) / 128 * 128;
     __shared__ int s_tok;
     __shared__ uint64_t s_attn_bar;
+    __shared__ int s_quit;                             // the computing warps have left
 #if MI_PROF
     if (tid < kProfSlots) s_prof[tid] = 0;
 #endif
 
-    for (int i = tid; i < njobs * (int)(sizeof(Job) / 4); i += DNT)
-        reinterpret_cast<int*>(sm.jobs)[i] = __ldg(reinterpret_cast<const int*>(P.jobs) + i);
-    for (int i = tid; i < P.L * (int)(sizeof(LayerPtrs) / 4); i += DNT)
+    for (int i = tid; i < P.L * (int)(sizeof(LayerPtrs) / 4); i += DNT_ALL)
         reinterpret_cast<int*>(sm.lp)[i] = __ldg(reinterpret_cast<const int*>(P.layers) + i);
     const bool attn_only = (int)blockIdx.x < P.attn_ctas;        // this CTA does nothing but attention; it lays the shared memory out its own way
-    if (lane == 0) {
+    if (!attn_only) {
+        const unsigned* work = P.work + (size_t)((int)blockIdx.x - P.attn_ctas) * P.work_stride;
+        sm.work = P.work_smem ? work_s : work;
+        if (P.work_smem) for (int i = tid; i < P.work_stride; i += DNT_ALL) work_s[i] = __ldg(work + i);
+    }
+    if (tid == 0) s_quit = 0;
+    if (lane == 0 && warp < DNW) {
         if (!attn_only) {
             #pragma unroll
-            for (int s = 0; s < DS; s++) mbar_init(&sm.bars[warp * DS + s], 1);
+            for (int s = 0; s < 2 * DS; s++) mbar_init(&sm.bars[(s < DS ? 0 : DNW * DS - DS) + warp * DS + s], 1);
         }
         if (warp == 0) mbar_init(&s_attn_bar, 1);
         mbar_fence_init();
     }
-    __syncthreads();
+    __syncthreads();                                  // (all nine warps; the last time)
 
     if (attn_only) {                                  // CTAs [0, attn_ctas): attention and nothing else
-        attn_cta_main<HD, G>(P, step0, step1, ph0, ph1, smem, sm.stage, &s_attn_bar);
+        if (warp < DNW) attn_cta_main<HD, G>(P, step0, step1, ph0, ph1, smem, sm.stage, &s_attn_bar);
         return;
     }
 
@@ -1660,20 +1793,19 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
         const int l = ph / 5, k = ph % 5;
         return 4 * l + (k == 0 ? 0 : k <= 2 ? 1 : k == 3 ? 2 : 3);
     };
-    WarpStream ws;
-    ws.init(sm, P, warp, step0, step1, job_of_phase(ph0), job_of_phase(ph1));
-    if (lane == 0) {
-        #pragma unroll
-        for (int s = 0; s < DS; s++) ws.issue_one();
+    if (warp == DNW) {                                // weights depend on nothing: their stream runs ahead of all waits
+        stream_weights(sm, P, lane, step1 - step0, job_of_phase(ph0), job_of_phase(ph1), &s_quit);
+        return;
     }
+    WarpStream ws;
+    ws.init(sm, P, warp);
     pdl_launch_dependents();
     pdl_wait_prior();
 
     const int maxin = P.E > P.FF ? P.E : P.FF;
     int8_t* xq_s = reinterpret_cast<int8_t*>(sm.stage);
-    float2* xs_s = reinterpret_cast<float2*>(sm.stage + maxin);
-    bool ok = true, h_valid = false;                   // h_valid: this CTA's shared-memory copy of the residual stream is current
-    bool stopped = false;                              // the run ended early on the stop token: tiles of later steps are in flight
+    BlockScale* xs_s = reinterpret_cast<BlockScale*>(sm.stage + maxin);
+    bool ok = true, done = true, h_valid = false;                   // h_valid: this CTA's shared-memory copy of the residual stream is current
     int err_code = MI_ERR_TIMEOUT;
     const unsigned epoch = __ldcg(P.epoch_dev);
     const int pos_base = P.pos_dev ? __ldcg(P.pos_dev) : P.pos0;
@@ -1692,20 +1824,27 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
     if (tid == 0) s_prof_t = prof_t0;
 #endif
     if (step0 < step1) rope_table(pos_base + step0);
-    __syncthreads();
+    cta__syncthreads();
     for (int step = step0; step < step1 && ok; step++) {
         const int pos = pos_base + step;
         if (pos < 0 || pos >= P.max_seq || !lean_regime_ok(pos, P.attn_ctas)) { ok = false; err_code = MI_ERR_LIMIT; break; }   // the same on every CTA: nobody waits for anybody
         const unsigned tag0 = epoch + (unsigned)(step - step0) * (unsigned)nph + 1u;        // tag of (step, phase 0)
-        if (step > step0 && ph1 != nph) { rope_table(pos); __syncthreads(); }     // (otherwise the previous step's lm_head phase has made the table)
+        if (step > step0 && ph1 != nph) { rope_table(pos); cta__syncthreads(); }     // (otherwise the previous step's lm_head phase has made the table)
         prof_mark(P, kProfStep);
         for (int ph = ph0; ph < ph1 && ok; ph++) {
-            const int l = ph / 5, k = ph == nph - 1 ? 5 : ph % 5;
+            const int l = ph / 5;
+            int k = ph == nph - 1 ? 5 : ph % 5;
             Pub pub;
-            pub.xw = P.xw; pub.tag = tag0 + (unsigned)ph; pub.mute = ph == P.drop_phase;
+            pub.xw = P.xw; pub.tag = tag0 + (unsigned)ph; pub.mute = ph == P.drop_phase; pub.stride = P.xo.total;
 #if MI_TP
             pub.tp = &P.tp;
 #endif
+            const int kind = k == 0 ? JOB_QKV : k == 2 ? JOB_O : k == 3 ? JOB_GU : JOB_DOWN, kb = P.kb[kind];
+            const float* bias = k == 0 ? sm.lp[l].bqkv : nullptr;
+            JobStart js;
+            js.at = 0;
+            if (k != 1 && k != 5) js = begin_cta_job(ws, sm.work, kind, kb, lane, bias);
+            same_code(k);
             // One call site each for the norm prologue, the q8 prologue and the CTA job: the four per-layer GEMV
             // phases run the same instructions (they stay in the instruction cache from phase to phase) and differ
             // only in pointers and in the few lines of their epilogue.
@@ -1720,28 +1859,27 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                     residual_init(P, sm.h, nullptr, tok, P.E);
                     commit = P.h_in; nw = sm.lp[0].attn_norm;
                 } else if (k == 0) {
-                    gsrc = h_valid ? nullptr : P.h_mid; addw = P.xw + P.xo.down; commit = P.h_in; nw = sm.lp[l].attn_norm;
+                    gsrc = h_valid ? nullptr : P.h_mid; addw = xw_read(P) + P.xo.down; commit = P.h_in; nw = sm.lp[l].attn_norm;
                 } else if (k == 3) {
-                    gsrc = h_valid ? nullptr : P.h_in; addw = P.xw + P.xo.o; commit = P.h_mid; nw = sm.lp[l].ffn_norm;
+                    gsrc = h_valid ? nullptr : P.h_in; addw = xw_read(P) + P.xo.o; commit = P.h_mid; nw = sm.lp[l].ffn_norm;
                 } else {
-                    gsrc = h_valid ? nullptr : P.h_mid; addw = P.xw + P.xo.down; nw = P.out_norm;
+                    gsrc = h_valid ? nullptr : P.h_mid; addw = xw_read(P) + P.xo.down; nw = P.out_norm;
                 }
                 if (gsrc) residual_init(P, sm.h, gsrc, 0, P.E);                 // a launch that starts in mid-step
                 // the committed copy serves launches that start in mid-step (and state read-back); a launch over whole steps has no reader for it
                 if (MI_LEAN && ph0 == 0 && ph1 == nph) commit = nullptr;
-                ok = stage_norm_q8u(P, sm.h, addw, pub.tag - 1u, commit, nw, P.E, P.eps, sm.red, xq_s, xs_s);
+                ok = stage_norm_q8u<norm_chunks(HD, G)>(done, P, sm.h, addw, pub.tag - 1u, commit, nw, P.E, P.eps, sm.red, xq_s, xs_s);
                 h_valid = true;
                 prof_mark(P, 2 * k);
             } else if (k == 2 || k == 4) {
-                const Job& jb = sm.jobs[4 * l + (k == 2 ? 1 : 3)];
-                if (ws.first_cta_unit(jb) < jb.n_units) {        // only CTAs that have a unit of the job consume its input
+                if (js.at) {                                      // only CTAs that have a unit of the job consume its input
                     prof_mark(P, 2 * k);
-                    if (k == 2) ok = stage_poll_q8(P, P.xw + P.xo.att, P.NH * HD, pub.tag - 1u, xq_s, xs_s);
-                    else ok = stage_poll_q8(P, P.xw + P.xo.act, P.FF, pub.tag - 1u, xq_s, xs_s);
+                    ok = stage_poll_q8(done, P, xw_read(P) + (k == 2 ? P.xo.att : P.xo.act), k == 2 ? P.NH * HD : P.FF, pub.tag - 1u, xq_s, xs_s);
                     prof_mark(P, kProfWait);
                 }
             }
             if (!ok) break;
+            same_code(k);
             if (k == 1) {
                 if (pos + 1 <= kShortAttnMax && P.attn_ctas > 0) {
                     // the attention CTAs' business
@@ -1753,10 +1891,8 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                 else ok = attention_split<HD, G>(P, l, pos, sm.stage, pub.tag - 1u, pub);
 #endif
             } else if (k != 5) {
-                const int jn = 4 * l + (k == 0 ? 0 : k == 2 ? 1 : k == 3 ? 2 : 3);
-                const float* bias = sm.lp[l].bqkv;
                 const int nq = P.NH * HD;
-                ok = run_cta_job(ws, P, sm, jn, lane, xq_s, xs_s, pub, k == 0 ? bias : nullptr, [&](int g, int ln, float v0, float v1, float bv) {
+                done = run_cta_job(ws, P, sm, js, kb, k == 4 ? P.ks_down : 1, k == 3, lane, xq_s, xs_s, bias, pub, [&](int g, int ln, float v0, float v1, float bv) {
                     if (k == 0) {                                            // + bias, RoPE, packed q / k / v
                         const int p = g * 32 + ln;
                         const float v = __fadd_rn(v0, bv);
@@ -1768,7 +1904,7 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                             if ((within & 1) == 0) out = __double2float_rn(__dsub_rn(__dmul_rn((double)v, c), __dmul_rn((double)partner, s)));
                             else out = __double2float_rn(__dadd_rn(__dmul_rn((double)partner, s), __dmul_rn((double)v, c)));
                         }
-                        if (p < nq + 2 * P.KVD) pub.local(P.xo.qkv + p, __float_as_uint(out));
+                        if (p < nq + 2 * P.KVD) pub.all(P.xo.qkv + p, __float_as_uint(out));
                     } else if (k == 3) {                                     // SwiGLU of (gate, up), one q8_0 block per warp
                         const double gd = (double)v0;
                         const float a = __double2float_rn(__dmul_rn(__ddiv_rn(gd, __dadd_rn(1.0, exp_shared(-gd))), (double)v1));
@@ -1776,18 +1912,18 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                         const int qv = quant_block_warp2(a, dq, sq);         // FF is a multiple of 32: group g is block g
                         publish_q8_block<true>(pub, P.xo.act, P.xo.act + P.FF / 4, g, ln, qv, dq, sq);
                     } else if (k == 2) {
-                        pub.local(P.xo.o + g * 32 + ln, __float_as_uint(v0));
+                        pub.all(P.xo.o + g * 32 + ln, __float_as_uint(v0));
                     } else {
                         pub.shared(P.xo.down + g * 32 + ln, __float_as_uint(v0));
                     }
-                });
+                }) && done;
             } else {
                 // ---- lm_head on the staged final norm, greedy argmax (lowest index wins ties)
                 // Each candidate is {best value, its row, second-best value}: the runner-up gives the logit margin (top-1 minus
                 // top-2) that the reference's engine reports per token (src/mega.cu:523-550, 385-392).
                 Cand cd; cd.best = -INFINITY; cd.idx = 0x7fffffff; cd.second = -INFINITY;
                 float* lg = P.logits ? P.logits + (long long)(step - step0) * P.logits_stride : nullptr;
-                ok = run_warp_job(ws, 4 * P.L, lane, xq_s, xs_s, [&](int g, int ln, float v0) {
+                ok = run_warp_job(ws, 4 * P.L, P, lane, xq_s, xs_s, [&](int g, int ln, float v0) {
                     const int r = g * 32 + ln;
                     if (r < P.V) {
                         if (lg) lg[r] = v0;
@@ -1798,10 +1934,10 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                     }
                 });
                 cd.warp_reduce();
-                __syncthreads();
+                cta__syncthreads();
                 float* cv = reinterpret_cast<float*>(sm.red); int* ci = reinterpret_cast<int*>(sm.red) + 16; float* c2 = reinterpret_cast<float*>(sm.red) + 32;
                 if (lane == 0) { cv[warp] = cd.best; ci[warp] = cd.idx; c2[warp] = cd.second; }
-                __syncthreads();
+                cta__syncthreads();
                 if (tid == 0) {
                     Cand t; t.best = cv[0]; t.idx = ci[0]; t.second = c2[0];
                     for (int w = 1; w < DNW; w++) { Cand o; o.best = cv[w]; o.idx = ci[w]; o.second = c2[w]; t.merge(o); }
@@ -1822,7 +1958,7 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                     if (c0 + tid < n_cand) valid |= 7u;
                     if (c0 + DNT + tid < n_cand) valid |= 56u;
                     if (kRowsCross && c0 == 0 && tid < P.attn_ctas) valid |= 64u;
-                    const unsigned long long* cb = P.xw + P.xo.cand + (size_t)(c0 + tid) * 4;
+                    const unsigned long long* cb = xw_read(P) + P.xo.cand + (size_t)(c0 + tid) * 4;
                     okc = tw_poll(P, pub.tag, valid, [&](int q) { return q == 6 ? P.xw + attdone_off(P, step) + tid : cb + (q / 3) * (4 * DNT) + (q % 3); }, cw);
                     #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -1835,9 +1971,9 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                 if (kRowsCross) fence_acq_rel_gpu();
                 prof_mark(P, kProfWait);
                 cd.warp_reduce();
-                ok = __syncthreads_and(okc ? 1 : 0) != 0;       // also: cv / ci / c2 are free again
+                ok = cta__syncthreads_and(okc ? 1 : 0) != 0;       // also: cv / ci / c2 are free again
                 if (lane == 0) { cv[warp] = cd.best; ci[warp] = cd.idx; c2[warp] = cd.second; }
-                __syncthreads();
+                cta__syncthreads();
                 if (tid == 0) {
                     Cand t; t.best = cv[0]; t.idx = ci[0]; t.second = c2[0];
                     for (int w = 1; w < DNW; w++) { Cand o; o.best = cv[w]; o.idx = ci[w]; o.second = c2[w]; t.merge(o); }
@@ -1861,19 +1997,19 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                     }
                 }
             }
-            ok = __syncthreads_and(ok ? 1 : 0) != 0;          // a wait that gave up in one warp stops the whole CTA
+            // a wait that gave up in one warp stops the whole CTA: behind an attention phase or a pick here, behind a job at the next barrier of a prologue
+            if (k == 5 || (k == 1 && !(pos + 1 <= kShortAttnMax && P.attn_ctas > 0)) || ph + 1 == ph1) { ok = cta__syncthreads_and(ok && done ? 1 : 0) != 0; done = true; }
             prof_mark(P, 2 * k + 1);
         }
         // the stop rule (every CTA has made the same pick): the step that produced the stop token was the last
         if (P.stop_token >= 0 && ok && ph0 == 0 && ph1 == nph && s_tok == P.stop_token && step + 1 >= P.n_forced && step + 1 < step1) {
-            stopped = true;
             break;
         }
     }
 #if MI_PROF
     if (P.prof && (int)blockIdx.x == P.prof_cta) {
         if (tid == 0) { s_prof[8] = (unsigned long long)(clock64() - prof_c0); s_prof[9] = gtime_ns() - prof_t0; }     // SM cycles and nanoseconds of the launch (overwrites two phase slots)
-        __syncthreads();
+        cta__syncthreads();
         if (tid < kProfSlots) P.prof[tid] += s_prof[tid];
     }
 #endif
@@ -1881,12 +2017,8 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
     // up after a full time budget): all CTAs have read the epoch
     if (ws.gcta == 0 && tid == 0 && (ph1 == nph || !ok))
         *P.epoch_dev = epoch + (unsigned)(step1 - step0) * (unsigned)nph + (ok ? 0u : (unsigned)nph);
-    if (!ok) {
-        if (lane == 0) atomicMax(P.err, err_code);
-        ws.drain();
-    } else if (stopped) {
-        ws.drain();
-    }
+    if (!ok && lane == 0) atomicMax(P.err, err_code);
+    if (tid == 0) *const_cast<volatile int*>(&s_quit) = 1;      // (tiles may be on their way: an error, or the stop token)
 }
 
 }  // inline namespace

@@ -40,6 +40,7 @@ struct mi_model {
     int L = 0, E = 0, FF = 0, NH = 0, NKV = 0, HD = 0, KVD = 0, V = 0, G = 0;
     float eps = 1e-6f, rope_base = 1e6f;
     int max_seq = 0, grid = 0, max_chunks = 0, attn_ctas = 0;
+    bool one_batch = true;                 // every CTA has at most one batch of units per job (what the range builds of the decode kernel take)
     int tp_rank = 0, tp_world = 1;
     bool tied = false;
     int requantized = 0;                  // matrices that were stored in another block format and re-quantized at load
