@@ -622,8 +622,8 @@ __device__ __forceinline__ int quant_block_warp2(float v, __half& d_out, int& s_
     d_out = __float2half_rn(__shfl_sync(0xffffffffu, r, 1));
     return q;
 }
-// Publish one q8_0 block (lane = element) as tagged words: lanes 0, 4, 8, .. store four int8 values each, lane 0
-// also the scale word.  qoff / soff: word offsets of the vector's value and scale parts; b: block index.
+// Publish one q8_0 block (lane = element) as tagged words: lanes 0, 4, 8, .. store four int8 values each, lane 1
+// the scale word.  qoff / soff: word offsets of the vector's value and scale parts; b: block index.
 template <bool SHARED>
 __device__ __forceinline__ void publish_q8_block(const Pub& pub, int qoff, int soff, int b, int lane, int q, __half d, int s) {
     unsigned v = (unsigned)q & 0xffu;
@@ -1399,9 +1399,9 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
 // ---- short-range attention on the CTAs set aside for it ------------------------------------------------
 // A CTA of [0, attn_ctas) handles HPC query heads of one kv head and nothing else, which buys two things.  (1) The K and V
 // rows of the cached positions are known long before the layer's q arrives, so the CTA copies them into shared memory
-// ahead of time (one bulk copy per row, rows padded by 16 bytes against bank conflicts; the copy for the next layer is
-// issued as soon as this layer's arithmetic has left the buffer): between q's arrival and the published output there is
-// no global load at all.  (2) One fp16 -> double conversion of a K or V element serves all HPC heads.
+// ahead of time (asynchronous 16-byte copies, rows padded by 16 bytes against bank conflicts; requested as soon as the layer before has left
+// the buffer): between q's arrival and the published output there is
+// no global load at all.  (Bulk copies, a thread for each row, were 28 KB of code.)  (2) One fp16 -> double conversion of a K or V element serves all HPC heads.
 // The new position's K and V come with q as tagged words; they go into the shared-memory rows directly and to the global
 // cache after the output has been published (fenced before this CTA's next output, which is what later readers wait for).
 // The two passes and the softmax are attention_short's; a dot product is added in another order (eight partial sums over an eighth of the dimensions
@@ -1416,30 +1416,9 @@ __host__ __device__ inline size_t attn_dedicated_smem(int HD, int HPC) {
 // measured 4.5 us per layer on the critical path), one where it is odd or at most two
 __host__ __device__ constexpr int attn_heads_per_cta(int G) { return G % 2 == 0 && G > 2 ? 2 : 1; }
 
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
-
-struct AttnPrefetch { uint64_t* bar; unsigned parity; int layer, pos; bool pending; bool ok; };
-
-// Request the K and V rows of positions [0, pos) of `layer` for this CTA's kv head (whole CTA; ends with the copies in flight).
-template <int HD>
-__device__ __forceinline__ void attn_prefetch_issue(const DecodeParams& P, uint8_t* smem, AttnPrefetch& pf, int layer, int pos, int kvh) {
-    constexpr int RSB = attn_row_bytes<HD>();
-    const int tid = threadIdx.x;
-    pf.layer = layer; pf.pos = pos; pf.pending = pos > 0;
-    if (pos <= 0) return;
-    if (tid == 0) { fence_proxy_async(); mbar_expect_tx(pf.bar, 2u * (unsigned)pos * (2u * HD)); }
-    cta__syncthreads();
-    uint8_t* Kb = smem; uint8_t* Vb = smem + (size_t)kAttnRows * RSB;
-    for (int p = tid; p < pos; p += DNT) {
-        const size_t row = ((size_t)layer * P.max_seq + p) * P.KVD + (size_t)kvh * HD;
-        bulk_g2s(Kb + (size_t)p * RSB, P.kc + row, 2 * HD, pf.bar);
-        bulk_g2s(Vb + (size_t)p * RSB, P.vc + row, 2 * HD, pf.bar);
-    }
-}
-
+// Returns a CTA-uniform ok.
 template <int HD, int GQ, int HPC>
-__device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& P, int l, int pos, uint8_t* smem, AttnPrefetch pf,
-                                                                unsigned tag_in, const Pub pub, int next_layer, int next_pos) {
+__device__ __forceinline__ bool attention_dedicated(const DecodeParams& P, int l, int pos, uint8_t* smem, unsigned tag_in, const Pub pub) {
     constexpr int DPW = HD / 32, RSB = attn_row_bytes<HD>();
     constexpr int LPP = 8, DPL = HD / LPP, QSTR = DPL + 2;
     constexpr int QN = (HPC * HD + DNT - 1) / DNT;
@@ -1452,11 +1431,15 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
     double* lw = ow + DNW * HPC * HD;                                           // [DNW][HPC]
     double* pd = lw + DNW * HPC;                                                // [DNW][HPC][rows] partial scores
     float* sc = reinterpret_cast<float*>(pd + DNW * HPC * kAttnRows);           // [HPC][rows]
-    // the rows of this (layer, position) should be on their way already; a launch's first layer requests them here
-    if (!(pf.layer == l && pf.pos == pos)) {
-        if (pf.pending) { (void)mbar_wait_bounded(pf.bar, pf.parity); pf.parity ^= 1u; }
-        attn_prefetch_issue<HD>(P, smem, pf, l, pos, kvh);
+    // the rows of the earlier positions: requested before q is waited for (this CTA has nothing else to do)
+    #pragma unroll 2
+    for (int i = tid; i < pos * (HD / 8); i += DNT) {
+        const int r = i / (HD / 8), c = (i % (HD / 8)) * 16;
+        const size_t row = ((size_t)l * P.max_seq + r) * P.KVD + (size_t)kvh * HD + c / 2;
+        cp_async16(Kb + r * RSB + c, P.kc + row);
+        cp_async16(Vb + r * RSB + c, P.vc + row);
     }
+    cp_async_commit();
     // q of this CTA's heads and k / v of the new position (tagged words, packed order: dim d sits at 2d (d < HD/2) or 2(d-HD/2)+1)
     unsigned qw[QN + 2], valid = 0;
     #pragma unroll
@@ -1482,8 +1465,8 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
         reinterpret_cast<__half*>(Vb + (size_t)pos * RSB)[tid] = vnew;
     }
     prof_mark(P, 14);
-    if (ok && pf.pending) { ok = mbar_wait_bounded(pf.bar, pf.parity); pf.parity ^= 1u; pf.pending = false; }
-    if (!cta__syncthreads_and(ok ? 1 : 0)) { pf.ok = false; return pf; }
+    cp_async_wait<0>();
+    if (!cta__syncthreads_and(ok ? 1 : 0)) return false;
     prof_mark(P, 27);
     const float inv = __fdiv_rn(1.f, __fsqrt_rn((float)HD));
     const int a0 = (int)((long long)Lp * warp / DNW), a1 = (int)((long long)Lp * (warp + 1) / DNW), np = a1 - a0;
@@ -1498,7 +1481,7 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
         for (int j = 0; j < HPC; j++)
             #pragma unroll
             for (int e = 0; e < DW; e++) qr[j][e] = qs[(j * LPP + (warp * DW + e) / DPL) * QSTR + (warp * DW + e) % DPL];
-        #pragma unroll 2
+        #pragma unroll 1
         for (int p0 = 0; p0 < Lp; p0 += 32) {
             const uint8_t* kr = Kb + (size_t)min(p0 + lane, Lp - 1) * RSB + warp * (DW * 2);
             unsigned kw[DW / 2];
@@ -1610,19 +1593,14 @@ __device__ __forceinline__ AttnPrefetch attention_dedicated(const DecodeParams& 
         publish_q8_block<false>(pub, P.xo.att, P.xo.att + P.NH * HD / 4, e >> 5, lane, qv8, dq, sq);
     }
     prof_mark(P, 17);
-    // the new position into the global cache (CTAs that share a kv head store the same bits); performed, for the generic and
-    // the bulk-copy path alike, before this CTA publishes anything else
+    // the new position into the global cache (CTAs that share a kv head store the same bits); performed before this CTA publishes anything else
     if (tid < HD) {
         P.kc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = knew;
         P.vc[((size_t)l * P.max_seq + pos) * P.KVD + (size_t)kvh * HD + tid] = vnew;
         __threadfence();
-        fence_proxy_async();
     }
     cta__syncthreads();                                  // the buffer is free, the stores are fenced
-    if (next_layer >= 0 && next_pos + 1 <= kShortAttnMax) attn_prefetch_issue<HD>(P, smem, pf, next_layer, next_pos, kvh);
-    else { pf.layer = -1; pf.pending = false; }
-    pf.ok = true;
-    return pf;
+    return true;
 }
 
 // The whole life of a CTA that does nothing but attention: every step, every layer, wait for q, attend, publish.  One call
@@ -1667,11 +1645,10 @@ static __device__ __noinline__ bool rows_ordered(const DecodeParams& P, unsigned
 }
 
 template <int HD, int G>
-static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int step0, int step1, int ph0, int ph1, uint8_t* smem, uint8_t* stage, uint64_t* bar) {
+static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int step0, int step1, int ph0, int ph1, uint8_t* smem, uint8_t* stage) {
     const int nph = 5 * P.L + 1;
     pdl_launch_dependents();
     pdl_wait_prior();
-    AttnPrefetch apf; apf.bar = bar; apf.parity = 0; apf.layer = -1; apf.pos = -1; apf.pending = false; apf.ok = true;
     const unsigned epoch = __ldcg(P.epoch_dev);
     const int pos_base = P.pos_dev ? __ldcg(P.pos_dev) : P.pos0;
     bool ok = true;
@@ -1701,20 +1678,10 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
             pub.tp = &P.tp;
 #endif
 #if MI_LEAN <= 1
-            if (pos + 1 <= kShortAttnMax) {
-                // where this CTA's next attention will be: the next layer of this step, or layer 0 of the next step
-                int nl = -1, np_ = pos;
-                if (ph + 5 < ph1 && l + 1 < P.L) nl = l + 1;
-                else if (step + 1 < step1 && ph0 <= 1) { nl = 0; np_ = pos + 1; }
-                apf = attention_dedicated<HD, G, attn_heads_per_cta(G)>(P, l, pos, smem, apf, pub.tag - 1u, pub, nl, np_);
-                ok = apf.ok;
-            }
+            if (pos + 1 <= kShortAttnMax) ok = attention_dedicated<HD, G, attn_heads_per_cta(G)>(P, l, pos, smem, pub.tag - 1u, pub);
 #endif
 #if MI_LEAN == 0
-            else {
-                if (apf.pending) { (void)mbar_wait_bounded(apf.bar, apf.parity); apf.parity ^= 1u; apf.pending = false; apf.layer = -1; }
-                ok = attention_split<HD, G>(P, l, pos, stage, pub.tag - 1u, pub);
-            }
+            else ok = attention_split<HD, G>(P, l, pos, stage, pub.tag - 1u, pub);
 #elif MI_LEAN == 2
             ok = attention_split<HD, G>(P, l, pos, stage, pub.tag - 1u, pub);
 #endif
@@ -1733,7 +1700,6 @@ static __device__ __noinline__ void attn_cta_main(const DecodeParams& P, int ste
         if (threadIdx.x < kProfSlots) P.prof[threadIdx.x] += s_prof[threadIdx.x];
     }
 #endif
-    if (apf.pending) (void)mbar_wait_bounded(apf.bar, apf.parity);      // copies in flight target this CTA's shared memory
     if (!ok && (threadIdx.x & 31) == 0) atomicMax(P.err, err_code);
 }
 
@@ -1757,7 +1723,6 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
     sm.h = reinterpret_cast<float*>(after_jobs + 1024 + 256 + kFoldBytes);
     sm.stage = after_jobs + 1024 + 256 + kFoldBytes + ((size_t)P.E * 4 + 127) / 128 * 128;
     __shared__ int s_tok;
-    __shared__ uint64_t s_attn_bar;
     __shared__ int s_quit;                             // the computing warps have left
 #if MI_PROF
     if (tid < kProfSlots) s_prof[tid] = 0;
@@ -1777,13 +1742,12 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
             #pragma unroll
             for (int s = 0; s < 2 * DS; s++) mbar_init(&sm.bars[(s < DS ? 0 : DNW * DS - DS) + warp * DS + s], 1);
         }
-        if (warp == 0) mbar_init(&s_attn_bar, 1);
         mbar_fence_init();
     }
     __syncthreads();                                  // (all nine warps; the last time)
 
     if (attn_only) {                                  // CTAs [0, attn_ctas): attention and nothing else
-        if (warp < DNW) attn_cta_main<HD, G>(P, step0, step1, ph0, ph1, smem, sm.stage, &s_attn_bar);
+        if (warp < DNW) attn_cta_main<HD, G>(P, step0, step1, ph0, ph1, smem, sm.stage);
         return;
     }
 
