@@ -87,6 +87,29 @@ __device__ __forceinline__ float swiglu(float gate, float up) {
     const double gd = (double)gate;
     return __double2float_rn(__dmul_rn(__ddiv_rn(gd, __dadd_rn(1.0, exp(-gd))), (double)up));
 }
+// SwiGLU and q8_0 of one block by eight lanes of a warp, four consecutive elements each (all lanes of the warp call): the lane's four int8 values, the block's fp16 scale and the
+// sum of its values.  Of what a block takes besides its 32 exponentials and divisions (reductions, one division for 127 / max and max / 127) a warp does four at once.
+struct SwiBlock { unsigned q; __half d; int sum; };
+__device__ __forceinline__ SwiBlock swiglu_block(float4 g, float4 u) {
+    const float a[4] = {swiglu(g.x, u.x), swiglu(g.y, u.y), swiglu(g.z, u.z), swiglu(g.w, u.w)};
+    unsigned am = 0;                                       // over the bits: a NaN counts as the largest
+    #pragma unroll
+    for (int i = 0; i < 4; i++) am = max(am, __float_as_uint(fabsf(a[i])));
+    #pragma unroll
+    for (int o = 1; o < 8; o <<= 1) am = max(am, __shfl_xor_sync(0xffffffffu, am, o));
+    const float m = __uint_as_float(am);
+    const bool odd = threadIdx.x & 1;
+    const float r = __fdiv_rn(odd ? m : 127.f, odd ? 127.f : m), other = __shfl_xor_sync(0xffffffffu, r, 1), inv = m > 0.f ? (odd ? other : r) : 0.f;
+    SwiBlock b;
+    b.d = __float2half_rn(odd ? r : other);
+    b.q = 0;
+    #pragma unroll
+    for (int i = 0; i < 4; i++) b.q |= ((unsigned)__float2int_rn(__fmul_rn(a[i], inv)) & 0xffu) << (8 * i);
+    b.sum = __dp4a((int)b.q, 0x01010101, 0);
+    #pragma unroll
+    for (int o = 1; o < 8; o <<= 1) b.sum += __shfl_xor_sync(0xffffffffu, b.sum, o);
+    return b;
+}
 #endif
 
 struct GemmParams {
