@@ -86,12 +86,12 @@ int alloc_tiled(mi_ctx* ctx, mi_model* m, int64_t rows, int64_t cols, uint8_t** 
 
 // Cross-CTA K-split of a per-layer job.  A job whose result feeds an in-phase epilogue
 // (QKV: bias + RoPE; gate/up: SwiGLU + q8_0) is never split across CTAs: its eight warps
-// already share every unit, and so is the O projection (measured: 6 tiles per row group, one
-// per warp, gains nothing from a split).  The down projection (35 tiles per row group at the
-// 1.5B shape, 48 row groups for 148 CTAs) is split until every CTA has a unit; the CTA of
-// split 0 collects the other splits' partial sums (see run_cta_job).
-int plan_ks(int kind, int groups, int nt, int grid) {
-    if (kind != JOB_DOWN) return 1;
+// already share every unit, and so is the O projection.  The down projection has few row groups
+// of many tiles; where halves of them give every CTA a unit at most they are dealt (Job::half), which needs no
+// exchange (1.5B shape, us per token: two K ranges 573, whole groups 556, halves 549; a split's second hop is longer than two more rounds of tiles).  Else it is
+// split until every CTA has a unit; the CTA of split 0 collects the other splits' partial sums (see run_cta_job).
+int plan_ks(int kind, int groups, int nt, int kb, int grid) {
+    if (kind != JOB_DOWN || (kb >= 4 && 2 * groups <= grid)) return 1;
     int ks = grid / std::max(groups, 1);
     return std::max(1, std::min(std::min(ks, nt), kMaxKSplit));
 }
@@ -306,7 +306,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     std::vector<LayerPtrs> lp(L);
     const int qkv_rows = NQ + 2 * KVD, W = GG * DNW;
     m->qkv_rows = qkv_rows;
-    int rot = 0, wrot = 0;
+    int wrot = 0;
     auto add_job = [&](const uint8_t* base, int groups, int cols, int nacc, int kind, int layer) {
         Job jb{}; jb.nb = cols / 32; jb.kb = choose_kb(jb.nb); jb.nt = jb.nb / jb.kb;
         jb.nacc = nacc; jb.kind = kind;
@@ -320,18 +320,21 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         if (!replicated) mi_tp_partition(groups, tp_rank, tp_world, &g0, &g1);
         jb.g_off = g0; jb.groups = g1 - g0;
         jb.base = base + (size_t)g0 * nacc * jb.nt * tile_bytes(jb.kb);
-        jb.ks = plan_ks(kind, replicated ? groups : (groups + tp_world - 1) / tp_world, jb.nt, GG);
+        jb.ks = plan_ks(kind, replicated ? groups : (groups + tp_world - 1) / tp_world, jb.nt, jb.kb, GG);
         const char* force = kind == JOB_DOWN ? getenv("MINFER_KS_DOWN") : nullptr;   // tuning knob
         if (force) jb.ks = std::max(1, std::min(std::min(atoi(force), jb.nt), kMaxKSplit));
         if (jb.ks >= GG) jb.ks = std::max(1, GG - 1);       // the CTAs of a row group's splits must be distinct
-        jb.n_units = jb.groups * jb.ks;
+        // units of half a row group where that leaves no CTA with two of them; pairs of groups (gate/up) stay whole, as q8_0 blocks of their result
+        jb.half = nacc == 1 && jb.ks == 1 && kind != JOB_LM && jb.kb >= 4 && 2 * jb.groups <= GG;
+        jb.n_units = jb.groups * (jb.half ? 2 : jb.ks);
         if (kind == JOB_LM) { jb.rot = 0; jb.wrot = 0; }
         else {
-            // the jobs of a layer start where the previous one stopped, over CTAs and over the warps of a CTA; every layer is dealt like the first, so that
-            // the kernel needs one description per kind
-            if (layer > 0) { jb.rot = m->jobs[kind].rot; jb.wrot = m->jobs[kind].wrot; }
-            else { jb.rot = rot; jb.wrot = wrot; }
-            rot = (int)(((long long)rot + jb.n_units) % GG);
+            // Every layer is dealt alike, so that the kernel needs one list per CTA.  Where the down projection is split, the CTAs that fold the splits publish last, so they are the first
+            // ones (unit order: split by split), and the job that follows them, QKV, is dealt from the other end; and O with it (each job from where the one before it
+            // stopped: 3B shape 827 us per token instead of 817, 1.5B and 0.5B 1 % less).  Over the warps of a CTA a job starts where the previous one stopped.
+            jb.rot = kind == JOB_QKV || kind == JOB_O ? std::max(0, GG - jb.n_units) : 0;
+            if (layer > 0) jb.wrot = m->jobs[kind].wrot;
+            else jb.wrot = wrot;
             wrot = (wrot + nacc * ((jb.nt + jb.ks - 1) / jb.ks)) & (DNW - 1);
         }
         m->jobs.push_back(jb);
@@ -441,15 +444,17 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
                     std::vector<unsigned> items[DNW];
                     int i = jb.wrot, units = 0;
                     for (int v = u; v < jb.n_units && units < kBatchUnits; v += G, units++) {
-                        const int g = v / jb.ks, sp = v % jb.ks, t0 = sp * jb.nt / jb.ks, t1 = (sp + 1) * jb.nt / jb.ks, ntu = t1 - t0;
+                        // (a unit per CTA at most: split by split; else a row group's splits one after the other, so that no batch waits for a later one)
+                        const bool by_split = jb.n_units <= G;
+                        const int per = jb.half ? 2 : jb.ks, g = by_split ? v % jb.groups : v / per, q = by_split ? v / jb.groups : v % per, sp = jb.half ? 0 : q, t0 = sp * jb.nt / jb.ks, t1 = (sp + 1) * jb.nt / jb.ks, ntu = t1 - t0;
                         if (j < 4) {
-                            w[at + kBatchGroup + units] = (unsigned)(g + jb.g_off);
+                            w[at + kBatchGroup + units] = (unsigned)(jb.kind == JOB_GU ? g + jb.g_off : (g + jb.g_off) * 32 + (jb.half ? 16 * q : 0));
                             w[at + kBatchUnit + units] = (unsigned)sp | (unsigned)std::min(ntu, DNW) << 8 | (unsigned)(i & (DNW - 1)) << 16 | (unsigned)((i + ntu) & (DNW - 1)) << 20;
                         }
                         for (int a = 0; a < jb.nacc; a++)
                             for (int t = t0; t < t1; t++, i++) {
                                 lists[(size_t)cta * DNW + (i & (DNW - 1))].push_back((unsigned long long)(uintptr_t)(jb.base + ((size_t)(g * jb.nacc + a) * jb.nt + t) * tb) | code);
-                                items[i & (DNW - 1)].push_back((unsigned)(t * jb.kb) | (unsigned)(2 * units + a) << 16 | (t + DNW >= t1 ? 1u << 20 : 0u));
+                                items[i & (DNW - 1)].push_back((unsigned)(t * jb.kb) | (unsigned)(2 * units + a) << 16 | (t + DNW >= t1 ? 1u << 20 : 0u) | (jb.half && q ? 1u << 21 : 0u));
                             }
                     }
                     if (j >= 4) continue;
@@ -479,7 +484,8 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         MI_CUDA(ctx, cudaMemcpy(d_work, wtab.data(), wtab.size() * 4, cudaMemcpyHostToDevice));
         P.tile_tab = d_tab; P.tile_start = d_start; P.tile_stride = (int)stride;
         P.work = d_work; P.work_stride = (int)words; P.work_smem = words <= (size_t)kWorkSmem;
-        for (int k = 0; k < 4; k++) P.kb[k] = m->jobs[k].kb;
+        P.half_rows = 0;
+        for (int k = 0; k < 4; k++) { P.kb[k] = m->jobs[k].kb; P.half_rows |= m->jobs[k].half ? 1 << k : 0; }
         const Job& lm = m->jobs.back();
         P.kb[JOB_LM] = lm.kb; P.ks_down = m->jobs[JOB_DOWN].ks; P.lm_units = lm.n_units; P.lm_nt = lm.nt; P.lm_off = lm.g_off;
     }

@@ -144,7 +144,8 @@ struct Job {               // (host) a tiled matrix and how it is dealt over the
     const uint8_t* base;   // tiled weights
     int groups;            // unit groups; one unit group = nacc consecutive 32-row groups
     int nt, ks, nb, kb, nacc, kind;
-    int n_units;           // groups * ks
+    bool half;             // units of half a row group
+    int n_units;           // groups * ks, or groups * 2
     int rot;               // CTA (per-layer jobs) that gets unit 0
     int wrot;              // warp that gets tile 0 of a batch
     int g_off;             // first unit group this GPU owns (tensor parallelism; base points at it, groups counts the owned ones)
@@ -152,9 +153,11 @@ struct Job {               // (host) a tiled matrix and how it is dealt over the
 
 // What a CTA does in the per-layer jobs, listed by the host (all layers are dealt alike): 32-bit words, [kind] = offset of the job's first batch, or 0.
 // A batch is up to kBatchUnits units; its tiles, numbered unit by unit, accumulator by accumulator (gate, up), along K, go round-robin over the eight warps:
-//   [0] number of units | offset of the next batch << 8, or 0      [1 + b] row group of unit b
+//   [0] number of units | offset of the next batch << 8, or 0      [1 + b] unit b: its q8_0 block (gate/up), else its first row
 //   [4 + b] K-split of unit b | number of warps with tiles of a sum << 8 | first of them << 16 (gate), << 20 (up)
-//   [7 + w] offset of warp w's list | number of its tiles << 16;  list entry: first block | sum (2 b + accumulator) << 16 | last of the sum << 20
+//   [7 + w] offset of warp w's list | number of its tiles << 16;  list entry: first block | sum (2 b + accumulator) << 16 | last of the sum << 20 | second half of the rows << 21
+// Where twice the row groups of a job are no more than the CTAs, its units are half row groups (DecodeParams::half_rows): both CTAs of a group read its tiles, the second one from
+// the L2, and a lane has a row of sixteen and half of a tile's blocks.  The down projection of the 1.5B shape is 35 tiles on 96 CTAs instead of 48 so.
 constexpr int kBatchUnits = 3;                        // (the 3B shape's gate/up: two or three units per CTA)
 enum { kBatchGroup = 1, kBatchUnit = kBatchGroup + kBatchUnits, kBatchList = kBatchUnit + kBatchUnits, kBatchWords = kBatchList + 8 };
 
@@ -192,7 +195,8 @@ struct DecodeParams {
     float eps;
     double inv_e;                    // 1 / E
     const unsigned* work; int work_stride, work_smem;      // per GEMV CTA: its list (see above); whether it goes to shared memory
-    int kb[5], ks_down, lm_units, lm_nt, lm_off;           // tile depths by JobKind, K-splits of the down projection; lm_head: row groups and tiles of one, first row group
+    int kb[5], ks_down, half_rows;                         // tile depths by JobKind, K-splits of the down projection, which jobs' units are half row groups (bit per JobKind)
+    int lm_units, lm_nt, lm_off;                           // lm_head: row groups and tiles of one, first row group
     const unsigned long long* tile_tab;   // per warp: source address | kb code of every tile of one step, in consumption order
     const unsigned* tile_start;      // [grid*DNW][4L+2]: index of each job's first tile in the warp's list (last = count)
     int tile_stride;                 // entries reserved per warp in tile_tab
@@ -567,6 +571,16 @@ __device__ __forceinline__ double tile_dot(const TileRegs<KB>& r, int b0, const 
     }
     return acc;
 }
+// The same for sixteen rows of a tile (second: the latter ones): lane 16 j + r has row r and the j-th half of the blocks
+template <int KB>
+__device__ __forceinline__ void tile_load_half(const uint8_t* tile, int lane, bool second, TileRegs<KB / 2>& r) {
+    const int row = (lane & 15) + (second ? 16 : 0), j = lane >> 4;
+    const uint8_t* sp = tile + KB * 512 + row * (KB * 2) + j * KB;
+    if constexpr (KB == 8) { const uint2 v = *reinterpret_cast<const uint2*>(sp); r.d[0] = v.x; r.d[1] = v.y; }
+    else r.d[0] = *reinterpret_cast<const unsigned*>(sp);
+    #pragma unroll
+    for (int k = 0; k < KB / 2; k++) r.w[k] = reinterpret_cast<const uint4*>(tile)[(j * (KB / 2) + k) * 32 + row];
+}
 template <int KB>
 static __device__ __noinline__ double tile_dot_rare(const uint8_t* tile, int lane, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) {
     TileRegs<KB> r;
@@ -578,29 +592,43 @@ static __device__ __noinline__ double tile_dot_rare(const uint8_t* tile, int lan
 struct WarpTile {
 #if MI_LEAN
     TileRegs<8> t;
-    __device__ __forceinline__ void load(WarpStream& ws, int lane, int kb) {
+    template <int N> __device__ __forceinline__ void keep(const TileRegs<N>& r) {
+        #pragma unroll
+        for (int k = 0; k < N; k++) { t.w[k] = r.w[k]; t.d[k / 2] = r.d[k / 2]; }
+    }
+    template <int N> __device__ __forceinline__ TileRegs<N> first() const {
+        TileRegs<N> r;
+        #pragma unroll
+        for (int k = 0; k < N; k++) { r.w[k] = t.w[k]; r.d[k / 2] = t.d[k / 2]; }
+        return r;
+    }
+    // half: the tile belongs to a unit of sixteen rows; second: the latter ones
+    __device__ __forceinline__ void load(WarpStream& ws, int lane, int kb, bool half, bool second) {
         if (MI_SMALL && kb == 4) {
-            TileRegs<4> r;
-            tile_load<4>(ws.tile(), lane, r);
-            #pragma unroll
-            for (int k = 0; k < 4; k++) { t.w[k] = r.w[k]; t.d[k / 2] = r.d[k / 2]; }
-        } else tile_load<8>(ws.tile(), lane, t);
+            if (half) { TileRegs<2> r; tile_load_half<4>(ws.tile(), lane, second, r); keep<2>(r); }
+            else { TileRegs<4> r; tile_load<4>(ws.tile(), lane, r); keep<4>(r); }
+        } else if (half) { TileRegs<4> r; tile_load_half<8>(ws.tile(), lane, second, r); keep<4>(r); }
+        else tile_load<8>(ws.tile(), lane, t);
         ws.release(lane);
     }
-    __device__ __forceinline__ double dot(WarpStream&, int, int kb, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) const {
-        if (MI_SMALL && kb == 4) {
-            TileRegs<4> r;
-            #pragma unroll
-            for (int k = 0; k < 4; k++) { r.w[k] = t.w[k]; r.d[k / 2] = t.d[k / 2]; }
-            return tile_dot<4>(r, b0, xq_s, xs_s, acc);
+    __device__ __forceinline__ double dot(WarpStream&, int lane, int kb, bool half, bool, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) const {
+        if (half) {
+            b0 += (lane >> 4) * (kb >> 1);
+            if (MI_SMALL && kb == 4) return tile_dot<2>(first<2>(), b0, xq_s, xs_s, acc);
+            return tile_dot<4>(first<4>(), b0, xq_s, xs_s, acc);
         }
+        if (MI_SMALL && kb == 4) return tile_dot<4>(first<4>(), b0, xq_s, xs_s, acc);
         return tile_dot<8>(t, b0, xq_s, xs_s, acc);
     }
 #else
     const uint8_t* at;
-    __device__ __forceinline__ void load(const WarpStream& ws, int, int) { at = ws.tile(); }
-    __device__ __forceinline__ double dot(WarpStream& ws, int lane, int kb, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) const {
-        if (kb == 8) {
+    __device__ __forceinline__ void load(const WarpStream& ws, int, int, bool, bool) { at = ws.tile(); }
+    __device__ __forceinline__ double dot(WarpStream& ws, int lane, int kb, bool half, bool second, int b0, const int8_t* xq_s, const BlockScale* xs_s, double acc) const {
+        if (half) {                                        // (tiles of 8 or 4 blocks)
+            b0 += (lane >> 4) * (kb >> 1);
+            if (kb == 8) { TileRegs<4> r; tile_load_half<8>(at, lane, second, r); acc = tile_dot<4>(r, b0, xq_s, xs_s, acc); }
+            else { TileRegs<2> r; tile_load_half<4>(at, lane, second, r); acc = tile_dot<2>(r, b0, xq_s, xs_s, acc); }
+        } else if (kb == 8) {
             TileRegs<8> r;
             tile_load<8>(at, lane, r);
             acc = tile_dot<8>(r, b0, xq_s, xs_s, acc);
@@ -637,16 +665,17 @@ __device__ __forceinline__ void publish_q8_block(const Pub& pub, int qoff, int s
 // A per-layer job, before its input is there: the CTA's first batch, and this warp's first tile (range builds: in registers), so that behind the last word
 // that arrives there are only the activations to be read.
 struct JobStart { unsigned at; bool ok; float bias; WarpTile t; };
-// bias: added to complete sums by the epilogue, which needs the one of its unit
-__device__ __forceinline__ float batch_bias(const unsigned* work, unsigned at, int warp, int lane, const float* __restrict__ bias) {
-    return bias && warp < (int)(work[at] & 255u) ? __ldg(bias + work[at + kBatchGroup + warp] * 32 + lane) : 0.f;
+// bias: added to complete sums by the epilogue, which needs those of its unit's rows
+__device__ __forceinline__ float batch_bias(const unsigned* work, unsigned at, int warp, int lane, bool half, const float* __restrict__ bias) {
+    return bias && warp < (int)(work[at] & 255u) ? __ldg(bias + work[at + kBatchGroup + warp] + (half ? lane & 15 : lane)) : 0.f;
 }
-__device__ __forceinline__ JobStart begin_cta_job(WarpStream& ws, const unsigned* work, int kind, int kb, int lane, const float* __restrict__ bias) {
+__device__ __forceinline__ JobStart begin_cta_job(WarpStream& ws, const unsigned* work, int kind, int kb, bool half, int lane, const float* __restrict__ bias) {
     JobStart st;
     st.at = work[kind]; st.ok = true; st.bias = 0.f;
     if (st.at) {
-        st.bias = batch_bias(work, st.at, ws.warp, lane, bias);
-        if (work[st.at + kBatchList + ws.warp] >> 16) { st.ok = ws.acquire(); st.t.load(ws, lane, kb); }
+        st.bias = batch_bias(work, st.at, ws.warp, lane, half, bias);
+        const unsigned list = work[st.at + kBatchList + ws.warp];
+        if (list >> 16) { st.ok = ws.acquire(); st.t.load(ws, lane, kb, half, work[list & 0xffffu] >> 21 & 1u); }
     }
     return st;
 }
@@ -660,7 +689,7 @@ __device__ __forceinline__ double tree_sum8(double a, double b, double c, double
 // the CTA of split 0 waits for them, adds them to its own in split order and calls epi.
 // Every warp passes the same number of barriers, also after a wait gave up.
 template <class Epi>
-__device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, const JobStart& st, int kb, int ks, bool two, int lane,
+__device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& P, const DecodeSmem& sm, const JobStart& st, int kb, int ks, bool two, bool half, int lane,
                                             const int8_t* xq_s, const BlockScale* xs_s, const float* __restrict__ bias, const Pub& pub, Epi epi) {
     bool ok = st.ok;
     unsigned at = st.at;
@@ -676,11 +705,11 @@ __device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& 
             double acc = 0.0;
             for (;;) {
                 const unsigned it = *item++;
-                acc = t.dot(ws, lane, kb, (int)(it & 0xffffu), xq_s, xs_s, acc);
+                acc = t.dot(ws, lane, kb, half, it >> 21 & 1u, (int)(it & 0xffffu), xq_s, xs_s, acc);
                 if (it >> 20 & 1u) { sm.fold[((it >> 16 & 7u) * DNW + ws.warp) * 32 + lane] = acc; acc = 0.0; }
                 if (--n == 0) break;
                 if (ok) ok = ws.acquire();
-                t.load(ws, lane, kb);
+                t.load(ws, lane, kb, half, *item >> 21 & 1u);
             }
         }
         prof_mark(P, 18);
@@ -700,9 +729,10 @@ __device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& 
                 v1 = v0;
                 v0 = tree_sum8(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
             }
+            if (half) v0 = __dadd_rn(v0, __shfl_xor_sync(0xffffffffu, v0, 16));          // (the two halves of the blocks)
             bool whole = true;
             if (ks > 1) {
-                const int sp = (int)(u & 255u), to = P.xo.dpart + (((int)gg * (kMaxKSplit - 1)) * 32 + lane) * 2;
+                const int sp = (int)(u & 255u), to = P.xo.dpart + ((int)gg * (kMaxKSplit - 1) + lane) * 2;
                 whole = sp == 0;
                 if (!whole) {
                     const unsigned long long bits = (unsigned long long)__double_as_longlong(v0);
@@ -728,10 +758,11 @@ __device__ __forceinline__ bool run_cta_job(WarpStream& ws, const DecodeParams& 
 #endif
         at = head >> 8;
         if (!at) return ok;
-        bv = batch_bias(work, at, ws.warp, lane, bias);
-        if (work[at + kBatchList + ws.warp] >> 16) {
+        bv = batch_bias(work, at, ws.warp, lane, half, bias);
+        const unsigned next = work[at + kBatchList + ws.warp];
+        if (next >> 16) {
             if (ok) ok = ws.acquire();
-            t.load(ws, lane, kb);
+            t.load(ws, lane, kb, half, work[next & 0xffffu] >> 21 & 1u);
         }
         cta__syncthreads();                                                // the sums have been read
     }
@@ -747,8 +778,8 @@ __device__ __forceinline__ bool run_warp_job(WarpStream& ws, int /* in phase ord
         double acc = 0.0;
         for (int t = 0; t < nt && ok; t++) {
             if (!(ok = ws.acquire())) break;
-            h.load(ws, lane, kb);
-            acc = h.dot(ws, lane, kb, t * kb, xq_s, xs_s, acc);
+            h.load(ws, lane, kb, false, false);
+            acc = h.dot(ws, lane, kb, false, false, t * kb, xq_s, xs_s, acc);
         }
         if (ok) epi(u + off, lane, __double2float_rn(acc));
     }
@@ -1804,10 +1835,11 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
             pub.tp = &P.tp;
 #endif
             const int kind = k == 0 ? JOB_QKV : k == 2 ? JOB_O : k == 3 ? JOB_GU : JOB_DOWN, kb = P.kb[kind];
+            const bool half = P.half_rows >> kind & 1;
             const float* bias = k == 0 ? sm.lp[l].bqkv : nullptr;
             JobStart js;
             js.at = 0;
-            if (k != 1 && k != 5) js = begin_cta_job(ws, sm.work, kind, kb, lane, bias);
+            if (k != 1 && k != 5) js = begin_cta_job(ws, sm.work, kind, kb, half, lane, bias);
             same_code(k);
             // One call site each for the norm prologue, the q8 prologue and the CTA job: the four per-layer GEMV
             // phases run the same instructions (they stay in the instruction cache from phase to phase) and differ
@@ -1856,9 +1888,9 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
 #endif
             } else if (k != 5) {
                 const int nq = P.NH * HD;
-                done = run_cta_job(ws, P, sm, js, kb, k == 4 ? P.ks_down : 1, k == 3, lane, xq_s, xs_s, bias, pub, [&](int g, int ln, float v0, float v1, float bv) {
+                done = run_cta_job(ws, P, sm, js, kb, k == 4 ? P.ks_down : 1, k == 3, half, lane, xq_s, xs_s, bias, pub, [&](int g, int ln, float v0, float v1, float bv) {
                     if (k == 0) {                                            // + bias, RoPE, packed q / k / v
-                        const int p = g * 32 + ln;
+                        const int p = g + (half ? ln & 15 : ln);      // g: the unit's first row
                         const float v = __fadd_rn(v0, bv);
                         const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
                         float out = v;
@@ -1868,7 +1900,7 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                             if ((within & 1) == 0) out = __double2float_rn(__dsub_rn(__dmul_rn((double)v, c), __dmul_rn((double)partner, s)));
                             else out = __double2float_rn(__dadd_rn(__dmul_rn((double)partner, s), __dmul_rn((double)v, c)));
                         }
-                        if (p < nq + 2 * P.KVD) pub.all(P.xo.qkv + p, __float_as_uint(out));
+                        if (p < nq + 2 * P.KVD && (!half || ln < 16)) pub.all(P.xo.qkv + p, __float_as_uint(out));
                     } else if (k == 3) {                                     // SwiGLU of (gate, up), one q8_0 block per warp
                         const double gd = (double)v0;
                         const float a = __double2float_rn(__dmul_rn(__ddiv_rn(gd, __dadd_rn(1.0, exp_shared(-gd))), (double)v1));
@@ -1876,9 +1908,9 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
                         const int qv = quant_block_warp2(a, dq, sq);         // FF is a multiple of 32: group g is block g
                         publish_q8_block<true>(pub, P.xo.act, P.xo.act + P.FF / 4, g, ln, qv, dq, sq);
                     } else if (k == 2) {
-                        pub.all(P.xo.o + g * 32 + ln, __float_as_uint(v0));
+                        if (!half || ln < 16) pub.all(P.xo.o + g + ln, __float_as_uint(v0));
                     } else {
-                        pub.shared(P.xo.down + g * 32 + ln, __float_as_uint(v0));
+                        if (!half || ln < 16) pub.shared(P.xo.down + g + ln, __float_as_uint(v0));
                     }
                 }) && done;
             } else {
