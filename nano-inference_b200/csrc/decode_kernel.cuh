@@ -130,10 +130,7 @@ constexpr int kAttnChunk = 32;    // smallest KV range worth its own CTA
 constexpr int kShortAttnMax = 256;      // up to this many cached positions one CTA handles the whole range of a query head (attention_short)
 constexpr int kMaxKSplit = 4;     // cross-CTA K-splits of the down projection
 constexpr int kMaxWorldTP = 8;
-#ifndef MI_XCOPIES
-#define MI_XCOPIES 4
-#endif
-constexpr int kXCopies = MI_XCOPIES;       // copies of the exchange block (see Pub)
+constexpr int kXCopies = 8;       // copies of the exchange block (see Pub)
 
 // profile slots: 2*k = staging of phase kind k, 2*k+1 = its main work; 12 = time spent waiting for tagged words, 13 = step prologue
 enum { kProfWait = 12, kProfStep = 13, kProfSlots = 32 };
@@ -352,7 +349,8 @@ __device__ __forceinline__ void tw_st(unsigned long long* p, unsigned tag, unsig
 __device__ __forceinline__ bool tw_is(unsigned long long w, unsigned tag) { return (unsigned)(w >> 32) == tag; }
 
 // Where a phase publishes.  What (nearly) every CTA reads goes into kXCopies copies of the exchange block, and CTA i reads copy i % P.copies: a vector is a hundred lines of the
-// L2 or less, each read by 142 CTAs, and the slices that hold several of them were what the words waited for.  Words with few readers are in the first copy only.  In the
+// L2 or less, each read by 142 CTAs, and the slices that hold several of them were what the words waited for (four copies instead of eight: 1.5B shape
+// 538 us per token instead of 532, 855 instead of 782 behind 8192 positions, but the 3B shape 798 instead of 821).  Words with few readers are in the first copy only.  In the
 // tensor-parallel build shared vectors also go into every other GPU's block.
 struct Pub {
     unsigned long long* xw; unsigned tag; bool mute; int stride;
@@ -392,17 +390,16 @@ MI_COLD_FN bool tw_spin(const unsigned long long* p, unsigned tag, unsigned long
     return true;
 }
 
-// One warp waits together: the lowest lane that misses a word polls that word, the other lanes sit at the vote, so a
-// waiting warp keeps one load in flight, not thirty-two (148 CTAs polling with every thread load the L2 as hard as the
-// weight stream does).  Once one missing word has arrived the others are about to: from then on every lane fetches its own missing
-// words again without such a wait in between, which is a round trip less behind the last word (1.5B shape 611 -> 598 us per token, 0.5B
-// 428 -> 411); only every 64th round waits (and looks at the time).
+// What a warp does that misses words: every lane fetches its missing words again at once.  Each 64th round the lowest lane that misses one polls that word alone, looks at the time and
+// at the error word, and the other lanes sit at the vote.  (One lane polling from the start, which keeps one load of a warp in flight instead of
+// thirty-two, costs a round trip behind the last word: with the exchange block in eight copies the 1.5B shape took 552 us per token so and takes 532, the 0.5B shape 375 and 364; with a pause
+// of 40 or 150 ns between polls 594 and 604 where 585 was without.)
 // Called by all lanes of a warp with the first missing address of each (null: none).  Returns 0 when
 // no lane misses anything, 1 when the lanes are to fetch their missing words again, -1 when the wait gave up.
 __device__ __forceinline__ int tw_wait_warp(const unsigned long long* miss, unsigned tag, unsigned long long budget_ns, const int* err, unsigned round) {
     const unsigned mm = __ballot_sync(0xffffffffu, miss != nullptr);
     if (!mm) return 0;
-    if (round & 63u) return 1;
+    if ((round & 63u) != 63u) return 1;
     const int leader = __ffs(mm) - 1;
     int r = 1;
     if ((int)(threadIdx.x & 31) == leader) r = tw_spin(miss, tag, budget_ns, err) ? 1 : -1;
