@@ -34,18 +34,18 @@
 // for launches that start in the middle of a step, and for inspection.
 //
 // Work split.  Every GEMV phase is a "job" over a tiled q4_0 matrix.  For the
-// per-layer matrices a unit is (32-row group [gate/up: a pair of groups], K-split)
-// and belongs to a CTA: its eight warps take the unit's tiles round-robin and
-// fold their double partial sums through shared memory.  The down projection has
-// fewer row groups than the grid has CTAs, so its K dimension is additionally split
+// per-layer matrices a unit is a 32-row group (gate/up: a pair of groups), half of one where that leaves no CTA
+// with two, or (group, K-split), and belongs to a CTA: its eight warps take the tiles of all its units round-robin and
+// fold their double partial sums through shared memory.  Where a down projection has
+// fewer row groups than the grid has CTAs and halves would be too many, its K dimension is split
 // across CTAs; splits 1.. hand their double partial sums (two tagged words each) to
 // the CTA of split 0, which adds them in split order and publishes the fp32 row.
 // The lm_head has thousands of row groups: there a unit is a row group and belongs
 // to one warp.
 //
 // Weight streaming.  The whole tile sequence of a warp - across phases, layers
-// and steps - follows from shapes and indices alone, so lane 0 of every warp
-// keeps a private shared-memory ring full with bulk copies that run ahead of
+// and steps - follows from shapes and indices alone, so a ninth warp keeps the eight
+// private shared-memory rings full with bulk copies that run ahead of
 // the phase boundaries: weights are immutable, the HBM stream never waits for a
 // phase, only for ring space.
 //
@@ -407,8 +407,8 @@ __device__ __forceinline__ int tw_wait_warp(const unsigned long long* miss, unsi
 }
 
 // Load the N words addr(k) (k with bit k of `valid` set) and return their payloads once all carry `tag`.  All loads are
-// issued before any is looked at; if some word is not there yet, the warp polls one such word and then every lane fetches
-// its missing words again (they were produced together, most have landed meanwhile).  All 32 lanes of a warp must call.
+// issued before any is looked at; while some word is not there yet, every lane fetches
+// its missing words again (tw_wait_warp).  All 32 lanes of a warp must call.
 template <int N, class AddrFn>
 __device__ __forceinline__ bool tw_poll(const DecodeParams& P, unsigned tag, unsigned valid, AddrFn addr, unsigned (&out)[N]) {
     unsigned long long w[N];
