@@ -308,6 +308,9 @@ MI_API int mi_decode_run(mi_ctx* ctx, mi_model* model, const int32_t* in_tokens_
  * out after the context's wait budget and the call returns MI_ERR_TIMEOUT - nothing hangs or
  * faults.  -1 restores normal operation.  No counterpart in the reference. */
 MI_API int mi_model_debug_drop_phase(mi_model* model, int phase);
+/* Test hook of the instrumented builds (MINFER_PROFILE): CTA `cta` comes `us` microseconds (at most 1000) late to every norm
+ * prologue of the decode kernel; it is also the CTA whose profile is kept.  0: normal operation. */
+MI_API int mi_model_debug_hold(mi_model* model, int cta, int us);
 /* Test hook: which product passes of more than 16 tokens use: 0 the faster one by the cost models (as created), 1 the one over
  * digits wherever it can run, -1 the one over blocks.  Same results either way. */
 MI_API int mi_model_debug_products(mi_ctx* ctx, mi_model* model, int which);

@@ -46,6 +46,7 @@ SIGNATURES = {
     "mi_probe_read_bw": (_i32, [_vp, C.c_size_t, _i32, _i32, C.POINTER(C.c_float)]),
     "mi_probe_hop_ns": (_i32, [_vp, _i32, C.POINTER(C.c_float)]),
     "mi_model_debug_drop_phase": (_i32, [_vp, _i32]),
+    "mi_model_debug_hold": (_i32, [_vp, _i32, _i32]),
     "mi_model_debug_products": (_i32, [_vp, _vp, _i32]),
     "mi_ctx_sm_count": (_i32, [_vp]),
     "mi_device_malloc": (_i32, [_vp, C.c_size_t, C.POINTER(_vp)]),
@@ -517,6 +518,10 @@ class Model:
     def debug_drop_phase(self, phase):
         """Test hook: the producers of `phase` publish nothing (its consumers' waits then run out); -1 = normal."""
         self.ctx.check(self.ctx.lib.mi_model_debug_drop_phase(self.h, int(phase)), "mi_model_debug_drop_phase")
+
+    def debug_hold(self, cta, us):
+        """Test hook of the instrumented builds: `cta` comes `us` microseconds late to every norm prologue of the decode kernel."""
+        self.ctx.check(self.ctx.lib.mi_model_debug_hold(self.h, int(cta), int(us)), "mi_model_debug_hold")
 
     def debug_products(self, which):
         """Test hook: the product of passes of more than 16 tokens: 0 by cost, 1 over digits where it can run, -1 over blocks."""

@@ -84,18 +84,6 @@ int alloc_tiled(mi_ctx* ctx, mi_model* m, int64_t rows, int64_t cols, uint8_t** 
     return dev_alloc(ctx, m, out, groups * nt * tile_bytes(kb), true);
 }
 
-// Cross-CTA K-split of a per-layer job.  A job whose result feeds an in-phase epilogue
-// (QKV: bias + RoPE; gate/up: SwiGLU + q8_0) is never split across CTAs: its eight warps
-// already share every unit, and so is the O projection.  The down projection has few row groups
-// of many tiles; where halves of them give every CTA a unit at most they are dealt (Job::half), which needs no
-// exchange (1.5B shape, us per token: two K ranges 573, whole groups 556, halves 549; a split's second hop is longer than two more rounds of tiles).  Else it is
-// split until every CTA has a unit; the CTA of split 0 collects the other splits' partial sums (see run_cta_job).
-int plan_ks(int kind, int groups, int nt, int kb, int grid) {
-    if (kind != JOB_DOWN || (kb >= 4 && 2 * groups <= grid)) return 1;
-    int ks = grid / std::max(groups, 1);
-    return std::max(1, std::min(std::min(ks, nt), kMaxKSplit));
-}
-
 // cos and sin of the rotary angles of every position: angle = fp32(pos * freq) as src/cpu_infer.cpp:54, then the double
 // cosine / sine rounded to fp32 once (the products of the rotation are formed in double by the QKV epilogue)
 __global__ void rope_cs_kernel(const float* __restrict__ freq, float* __restrict__ cs, int HD, int max_seq) {
@@ -180,9 +168,10 @@ extern "C" int mi_model_free(mi_ctx* ctx, mi_model* m) {
 }
 
 extern "C" void mi_tp_partition(int groups, int rank, int world, int* begin, int* end) {
-    if (world < 1) world = 1;
-    if (begin) *begin = (int)((long long)groups * rank / world);
-    if (end) *end = (int)((long long)groups * (rank + 1) / world);
+    int b, e;
+    tp_share(groups, rank, std::max(world, 1), &b, &e);
+    if (begin) *begin = b;
+    if (end) *end = e;
 }
 
 extern "C" int mi_model_load_gguf(mi_ctx* ctx, const char* path, int max_seq, mi_model** out) {
@@ -308,33 +297,11 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     m->qkv_rows = qkv_rows;
     int wrot = 0;
     auto add_job = [&](const uint8_t* base, int groups, int cols, int nacc, int kind, int layer) {
-        Job jb{}; jb.nb = cols / 32; jb.kb = choose_kb(jb.nb); jb.nt = jb.nb / jb.kb;
-        jb.nacc = nacc; jb.kind = kind;
-        // tensor parallelism: this GPU owns a contiguous range of the job's unit groups (rows); every GPU holds the
-        // whole matrix but streams only its rows.  The K-split is planned from the largest share so that all GPUs
-        // lay the partial sums out identically.
-        // The QKV and O projections (a tenth of a layer's bytes) are the exception: every GPU computes all their rows,
-        // so that attention and the O projection need no exchange at all.
-        const bool replicated = kind == JOB_QKV || kind == JOB_O;
-        int g0 = 0, g1 = groups;
-        if (!replicated) mi_tp_partition(groups, tp_rank, tp_world, &g0, &g1);
-        jb.g_off = g0; jb.groups = g1 - g0;
-        jb.base = base + (size_t)g0 * nacc * jb.nt * tile_bytes(jb.kb);
-        jb.ks = plan_ks(kind, replicated ? groups : (groups + tp_world - 1) / tp_world, jb.nt, jb.kb, GG);
         const char* force = kind == JOB_DOWN ? getenv("MINFER_KS_DOWN") : nullptr;   // tuning knob
-        if (force) jb.ks = std::max(1, std::min(std::min(atoi(force), jb.nt), kMaxKSplit));
-        if (jb.ks >= GG) jb.ks = std::max(1, GG - 1);       // the CTAs of a row group's splits must be distinct
-        // units of half a row group where that leaves no CTA with two of them; pairs of groups (gate/up) stay whole, as q8_0 blocks of their result
-        jb.half = nacc == 1 && jb.ks == 1 && kind != JOB_LM && jb.kb >= 4 && 2 * jb.groups <= GG;
-        jb.n_units = jb.groups * (jb.half ? 2 : jb.ks);
-        if (kind == JOB_LM) { jb.rot = 0; jb.wrot = 0; }
-        else {
-            // Every layer is dealt alike, so that the kernel needs one list per CTA.  Where the down projection is split, the CTAs that fold the splits publish last, so they are the first
-            // ones (unit order: split by split), and the job that follows them, QKV, is dealt from the other end; and O with it (each job from where the one before it
-            // stopped: 3B shape 827 us per token instead of 817, 1.5B and 0.5B 1 % less).  Over the warps of a CTA a job starts where the previous one stopped.
-            jb.rot = kind == JOB_QKV || kind == JOB_O ? std::max(0, GG - jb.n_units) : 0;
-            if (layer > 0) jb.wrot = m->jobs[kind].wrot;
-            else jb.wrot = wrot;
+        Job jb = deal_job(kind, groups, cols / 32, choose_kb(cols / 32), nacc, GG, tp_rank, tp_world, force ? std::max(1, atoi(force)) : 0);
+        jb.base = base + (size_t)jb.g_off * nacc * jb.nt * tile_bytes(jb.kb);
+        if (kind != JOB_LM) {                               // over the warps of a CTA a job starts where the one before it stopped, in all layers alike
+            jb.wrot = layer > 0 ? m->jobs[kind].wrot : wrot;
             wrot = (wrot + nacc * ((jb.nt + jb.ks - 1) / jb.ks)) & (DNW - 1);
         }
         m->jobs.push_back(jb);
@@ -430,7 +397,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
                 continue;
             }
             for (int cta = 0; cta < G; cta++) {
-                const int r = jb.rot % G, u0 = cta >= r ? cta - r : cta + G - r;
+                const int u0 = first_unit(jb, cta, G);
                 std::vector<unsigned>& w = work[cta];
                 size_t link = (size_t)jb.kind;                          // where the offset of the next batch goes
                 for (int u = u0; u < jb.n_units; u += kBatchUnits * G) {
@@ -486,6 +453,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         P.work = d_work; P.work_stride = (int)words; P.work_smem = words <= (size_t)kWorkSmem;
         P.half_rows = 0;
         for (int k = 0; k < 4; k++) { P.kb[k] = m->jobs[k].kb; P.half_rows |= m->jobs[k].half ? 1 << k : 0; }
+        bystanders(m->jobs[JOB_QKV], m->jobs[JOB_GU], G, &P.seen_first, &P.seen_n);
         const Job& lm = m->jobs.back();
         P.kb[JOB_LM] = lm.kb; P.ks_down = m->jobs[JOB_DOWN].ks; P.lm_units = lm.n_units; P.lm_nt = lm.nt; P.lm_off = lm.g_off;
     }
@@ -515,7 +483,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         int off = 0;
         auto take = [&](int words) { const int o = off; off += (words + 1) / 2 * 2; return o; };     // every vector 16-byte aligned
         x.qkv = take((qkv_rows + 31) / 32 * 32);
-        x.att = take(q8_words(NQ));
+        x.att = take(q8_words(NQ) + P.seen_n);
         x.o = take((E + 31) / 32 * 32);
         x.act = take(q8_words(FF));
         x.down = take((E + 31) / 32 * 32);
@@ -543,7 +511,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         MI_CUDA(ctx, cudaMemcpy(m->d_pos, init, sizeof(init), cudaMemcpyHostToDevice));
     }
     P.epoch_dev = reinterpret_cast<unsigned*>(m->d_pos + 1);
-    P.drop_phase = -1; P.attn_ctas = m->attn_ctas; P.prof_cta = m->attn_ctas;
+    P.drop_phase = -1; P.hold_us = 0; P.attn_ctas = m->attn_ctas; P.prof_cta = m->attn_ctas;
     if (const char* pc = getenv("MINFER_PROFILE_CTA")) P.prof_cta = std::max(0, std::min(atoi(pc), m->grid - 1));
     P.max_seq = max_seq; P.max_chunks = m->max_chunks; P.err = ctx->d_err;
     m->prof_buf = P.prof;
@@ -1010,6 +978,12 @@ int mi::reset_after_error(mi_ctx* ctx, mi_model* m) {
 
 // Test hook: the producers of one phase (index 5 * layer + kind, or the lm_head phase 5 * n_layer) publish nothing from
 // now on, so that the waits of its consumers run out; -1 restores normal operation.
+extern "C" int mi_model_debug_hold(mi_model* m, int cta, int us) {
+    if (!m || cta < 0 || cta >= m->grid || us < 0 || us > 1000) return MI_ERR_INVALID;
+    m->P.prof_cta = cta; m->P.hold_us = us;
+    return MI_OK;
+}
+
 extern "C" int mi_model_debug_drop_phase(mi_model* m, int phase) {
     if (!m) return MI_ERR_INVALID;
     m->P.drop_phase = phase;

@@ -21,9 +21,14 @@
 // the long-range attention, has fences of its own): a phase boundary costs
 // one store-to-load hop through the L2 instead of arrive + poll + reload, and a CTA
 // waits only for the values it actually consumes.  Buffers are reused every layer;
-// a word can only be overwritten after every reader has passed on, because the
-// writer's own inputs descend from outputs of those readers (each layer has phases
-// in which every CTA produces something that every CTA consumes).  A reader that
+// a word is overwritten only after every reader has passed on, because the
+// writer's own inputs descend from outputs of those readers.  The readers of q / k / v, of
+// the attention output, of the activations, of chunk maxima and of partial sums publish something of the same phase
+// that the next writer needs.  The words of the O and of the down projection are read by every GEMV CTA: one with
+// a unit of QKV or of gate/up has read both before it publishes that unit's rows, which all later writers of either need (a unit of O alone or of down alone
+// protects one of the two).  A CTA with neither publishes in its place a word of the attention phase, which says
+// that it has read them and which the CTAs of the O projection await with the attention output (bystanders).
+// (A GPU of a tensor-parallel group that has no unit of gate/up, fewer groups of 32 than GPUs, is not held by this.)  A reader that
 // nevertheless fell behind would see a wrong tag and time out - never wrong data.
 // The same words, stored additionally into the other GPUs' copies of the buffers
 // over NVLink (plain 8-byte peer stores), are the whole tensor-parallel exchange.
@@ -63,6 +68,7 @@
 // observed, not proved.  Each token is processed exactly as if it were alone.
 #pragma once
 #include "gemv_core.cuh"
+#include "decode_deal.cuh"
 // functions that sit out of line to keep the loop body small; the short-context build inlines them instead, because every
 // call site inside the step loop, executed or not, makes the compiler keep the loop's values where a call preserves them
 #if defined(MI_LEAN) && MI_LEAN
@@ -121,32 +127,17 @@
 
 namespace mi {
 
-constexpr int DNW = 8;            // warps per CTA that compute
-constexpr int DNT = DNW * 32;     // their threads
+constexpr int DNT = DNW * 32;     // threads of the warps that compute
 constexpr int DNT_ALL = DNT + 32; // and one warp that requests the weights
 constexpr int DS = 3;             // ring slots per warp
 constexpr int DSLOT = 4608;       // bytes per slot: the largest tile (8 blocks)
 constexpr int kAttnChunk = 32;    // smallest KV range worth its own CTA
 constexpr int kShortAttnMax = 256;      // up to this many cached positions one CTA handles the whole range of a query head (attention_short)
-constexpr int kMaxKSplit = 4;     // cross-CTA K-splits of the down projection
 constexpr int kMaxWorldTP = 8;
 constexpr int kXCopies = 8;       // copies of the exchange block (see Pub)
 
 // profile slots: 2*k = staging of phase kind k, 2*k+1 = its main work; 12 = time spent waiting for tagged words, 13 = step prologue
 enum { kProfWait = 12, kProfStep = 13, kProfSlots = 32 };
-
-enum JobKind { JOB_QKV = 0, JOB_O = 1, JOB_GU = 2, JOB_DOWN = 3, JOB_LM = 4 };
-
-struct Job {               // (host) a tiled matrix and how it is dealt over the grid
-    const uint8_t* base;   // tiled weights
-    int groups;            // unit groups; one unit group = nacc consecutive 32-row groups
-    int nt, ks, nb, kb, nacc, kind;
-    bool half;             // units of half a row group
-    int n_units;           // groups * ks, or groups * 2
-    int rot;               // CTA (per-layer jobs) that gets unit 0
-    int wrot;              // warp that gets tile 0 of a batch
-    int g_off;             // first unit group this GPU owns (tensor parallelism; base points at it, groups counts the owned ones)
-};
 
 // What a CTA does in the per-layer jobs, listed by the host (all layers are dealt alike): 32-bit words, [kind] = offset of the job's first batch, or 0.
 // A batch is up to kBatchUnits units; its tiles, numbered unit by unit, accumulator by accumulator (gate, up), along K, go round-robin over the eight warps:
@@ -171,7 +162,7 @@ struct TpPeerParams {
 // [n/4] words of four int8 values followed by [n/32 (+1 if odd)] words of {fp16 scale bits | int16 sum of the block's values << 16}.
 struct XwLayout {
     int qkv;        // [qkv rows, padded to 32]   fp32 bits: q | k | v after bias and RoPE, packed (pair-adjacent) order
-    int att;        // q8_0 of the merged attention output [NH*HD]
+    int att;        // q8_0 of the merged attention output [NH*HD]; behind its scales a word of every CTA without a unit of QKV and gate/up (see bystanders)
     int o;          // [E] fp32 bits: O projection
     int act;        // q8_0 of SwiGLU(gate, up) [FF]                                     (pushed to the other GPUs)
     int down;       // [E] fp32 bits: down projection                                    (pushed)
@@ -192,6 +183,7 @@ struct DecodeParams {
     float eps;
     double inv_e;                    // 1 / E
     const unsigned* work; int work_stride, work_smem;      // per GEMV CTA: its list (see above); whether it goes to shared memory
+    int seen_first, seen_n;                                // GEMV CTAs without a unit of QKV and gate/up (bystanders)
     int kb[5], ks_down, half_rows;                         // tile depths by JobKind, K-splits of the down projection, which jobs' units are half row groups (bit per JobKind)
     int lm_units, lm_nt, lm_off;                           // lm_head: row groups and tiles of one, first row group
     const unsigned long long* tile_tab;   // per warp: source address | kb code of every tile of one step, in consumption order
@@ -218,6 +210,7 @@ struct DecodeParams {
     unsigned* epoch_dev;
     unsigned long long wait_ns;      // time budget of every device-side wait
     int drop_phase;                  // test hook: the producers of this phase publish nothing (-1: none), so that its consumers' waits run out
+    int hold_us;                     // test hook of the instrumented builds: CTA prof_cta comes this much late to every norm prologue
     float* att;                      // merged attention output, fp32, for inspection
     __half* kc; __half* vc; int max_seq;       // [L][max_seq][KVD]
     double* attn_part; int max_chunks, split_sub;       // [NH][max_chunks][HD+2]: weighted sums and denominator of every chunk (attention_split)
@@ -962,32 +955,32 @@ __host__ __device__ constexpr int norm_chunks(int HD, int G) { return ((MI_SMALL
 
 // A q8_0 vector published as tagged words by other CTAs -> shared memory: int8 values, and per block what
 // tile_dot wants of its scale and sum.  Thread t takes the 16-byte word pairs t, t + 256, ... of the values (NV at most) and of the scales (NS); all of a
-// thread's loads are in flight together.
+// thread's loads are in flight together.  more: words behind the scales that have to be there too.
 template <int NV, int NS>
-__device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
-    const int tid = threadIdx.x, nq2 = n / 8, nbk = n / 32;
+__device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int more, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
+    const int tid = threadIdx.x, nq2 = n / 8, nbk = n / 32, nw = nbk + more;
     int off[NV + NS];
     unsigned valid = 0, a[NV + NS], b[NV + NS];
     #pragma unroll
     for (int k = 0; k < NV + NS; k++) {
         const int pr = tid + (k < NV ? k : k - NV) * DNT;
         off[k] = k < NV ? 2 * pr : 2 * nq2 + 2 * pr;
-        valid |= (k < NV ? pr < nq2 : 2 * pr < nbk) ? 1u << k : 0u;
+        valid |= (k < NV ? pr < nq2 : 2 * pr < nw) ? 1u << k : 0u;
     }
-    ok = tw_poll_pairs<NV + NS, NS>(P, tag, valid, vw, off, a, b, nbk & 1 ? 2 * nq2 + nbk : -1) && ok;
+    ok = tw_poll_pairs<NV + NS, NS>(P, tag, valid, vw, off, a, b, nw & 1 ? 2 * nq2 + nw : -1) && ok;
     #pragma unroll
     for (int k = 0; k < NV; k++) if (valid >> k & 1u) reinterpret_cast<uint2*>(xq_s)[tid + k * DNT] = make_uint2(a[k], b[k]);
     #pragma unroll
     for (int k = NV; k < NV + NS; k++) {
         auto scale = [](unsigned sw) { return block_scale(__half2float(__ushort_as_half((unsigned short)(sw & 0xffffu))), (int)(short)(sw >> 16)); };
         const int blk = off[k] - 2 * nq2;
-        if (valid >> k & 1u) { xs_s[blk] = scale(a[k]); if (blk + 1 < nbk) xs_s[blk + 1] = scale(b[k]); }
+        if (blk < nbk) { xs_s[blk] = scale(a[k]); if (blk + 1 < nbk) xs_s[blk + 1] = scale(b[k]); }
     }
     return cta__syncthreads_and(ok ? 1 : 0) != 0;
 }
 // as many pairs as the longest vector wants; one form per build, so that all phases run the same instructions (lean_shape(): at most 8 pairs of values per thread)
-__device__ __forceinline__ bool stage_poll_q8(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
-    return stage_poll_q8_t<MI_LEAN ? 8 : 16, MI_LEAN ? 1 : 2>(ok, P, vw, n, tag, xq_s, xs_s);
+__device__ __forceinline__ bool stage_poll_q8(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int more, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
+    return stage_poll_q8_t<MI_LEAN ? 8 : 16, MI_LEAN ? 1 : 2>(ok, P, vw, n, more, tag, xq_s, xs_s);
 }
 
 // Shapes the context-range builds take: they hold one variant of each prologue and of the tile loop and no call to the others.
@@ -1841,6 +1834,10 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
             // One call site each for the norm prologue, the q8 prologue and the CTA job: the four per-layer GEMV
             // phases run the same instructions (they stay in the instruction cache from phase to phase) and differ
             // only in pointers and in the few lines of their epilogue.
+#if MI_PROF
+            if (P.hold_us && (int)blockIdx.x == P.prof_cta && (k == 0 || k == 3 || k == 5))
+                for (const unsigned long long t0 = gtime_ns(); gtime_ns() - t0 < (unsigned long long)P.hold_us * 1000ull;) {}
+#endif
             if (k == 0 || k == 3 || k == 5) {
                 // QKV : h = (l == 0) ? embedding : h + down projection of layer l-1        (committed as h_in)
                 // GU  : h = h + O projection                                                 (committed as h_mid)
@@ -1867,13 +1864,15 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
             } else if (k == 2 || k == 4) {
                 if (js.at) {                                      // only CTAs that have a unit of the job consume its input
                     prof_mark(P, 2 * k);
-                    ok = stage_poll_q8(done, P, xw_read(P) + (k == 2 ? P.xo.att : P.xo.act), k == 2 ? P.NH * HD : P.FF, pub.tag - 1u, xq_s, xs_s);
+                    ok = stage_poll_q8(done, P, xw_read(P) + (k == 2 ? P.xo.att : P.xo.act), k == 2 ? P.NH * HD : P.FF, k == 2 ? P.seen_n : 0, pub.tag - 1u, xq_s, xs_s);
                     prof_mark(P, kProfWait);
                 }
             }
             if (!ok) break;
             same_code(k);
             if (k == 1) {
+                const int by = ws.gcta - P.seen_first;
+                if ((unsigned)by < (unsigned)P.seen_n && tid == 0) pub.all(P.xo.att + P.NH * HD / 4 + P.NH * HD / 32 + by, 0u);        // (bystanders)
                 if (pos + 1 <= kShortAttnMax && P.attn_ctas > 0) {
                     // the attention CTAs' business
                 }
