@@ -454,6 +454,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         P.half_rows = 0;
         for (int k = 0; k < 4; k++) { P.kb[k] = m->jobs[k].kb; P.half_rows |= m->jobs[k].half ? 1 << k : 0; }
         bystanders(m->jobs[JOB_QKV], m->jobs[JOB_GU], G, &P.seen_first, &P.seen_n);
+        P.att_scales = NQ / 32 + P.seen_n;
         const Job& lm = m->jobs.back();
         P.kb[JOB_LM] = lm.kb; P.ks_down = m->jobs[JOB_DOWN].ks; P.lm_units = lm.n_units; P.lm_nt = lm.nt; P.lm_off = lm.g_off;
     }

@@ -183,7 +183,7 @@ struct DecodeParams {
     float eps;
     double inv_e;                    // 1 / E
     const unsigned* work; int work_stride, work_smem;      // per GEMV CTA: its list (see above); whether it goes to shared memory
-    int seen_first, seen_n;                                // GEMV CTAs without a unit of QKV and gate/up (bystanders)
+    int seen_first, seen_n, att_scales;                    // GEMV CTAs without a unit of QKV and gate/up (bystanders); scales of the attention output and those CTAs' words
     int kb[5], ks_down, half_rows;                         // tile depths by JobKind, K-splits of the down projection, which jobs' units are half row groups (bit per JobKind)
     int lm_units, lm_nt, lm_off;                           // lm_head: row groups and tiles of one, first row group
     const unsigned long long* tile_tab;   // per warp: source address | kb code of every tile of one step, in consumption order
@@ -271,7 +271,7 @@ struct SplitSmem {
 
 __host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD, int sub) {
     const int maxin = E > FF ? E : FF;
-    size_t a = (size_t)maxin + (size_t)(maxin / 32) * 8;               // xq, xs
+    size_t a = (size_t)maxin + (size_t)(maxin / 32) * 8;               // xq, xs (bystanders' words behind the latter: where there are any, maxin is below 32 times the grid and b is more than enough)
     const size_t split = SplitSmem{HD, sub}.bytes();
     const size_t shrt = (size_t)(8 * (HD / 8 + 2) + 256 + DNW * HD + DNW) * 8 + 1024;                // attention_short
     const size_t b = split > shrt ? split : shrt;
@@ -955,10 +955,10 @@ __host__ __device__ constexpr int norm_chunks(int HD, int G) { return ((MI_SMALL
 
 // A q8_0 vector published as tagged words by other CTAs -> shared memory: int8 values, and per block what
 // tile_dot wants of its scale and sum.  Thread t takes the 16-byte word pairs t, t + 256, ... of the values (NV at most) and of the scales (NS); all of a
-// thread's loads are in flight together.  more: words behind the scales that have to be there too.
+// thread's loads are in flight together.  nw: scales, and words behind them that have to be there too (what is stored of those nobody reads).
 template <int NV, int NS>
-__device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int more, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
-    const int tid = threadIdx.x, nq2 = n / 8, nbk = n / 32, nw = nbk + more;
+__device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int nw, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
+    const int tid = threadIdx.x, nq2 = n / 8;
     int off[NV + NS];
     unsigned valid = 0, a[NV + NS], b[NV + NS];
     #pragma unroll
@@ -974,13 +974,13 @@ __device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, 
     for (int k = NV; k < NV + NS; k++) {
         auto scale = [](unsigned sw) { return block_scale(__half2float(__ushort_as_half((unsigned short)(sw & 0xffffu))), (int)(short)(sw >> 16)); };
         const int blk = off[k] - 2 * nq2;
-        if (blk < nbk) { xs_s[blk] = scale(a[k]); if (blk + 1 < nbk) xs_s[blk + 1] = scale(b[k]); }
+        if (valid >> k & 1u) { xs_s[blk] = scale(a[k]); if (blk + 1 < nw) xs_s[blk + 1] = scale(b[k]); }
     }
     return cta__syncthreads_and(ok ? 1 : 0) != 0;
 }
 // as many pairs as the longest vector wants; one form per build, so that all phases run the same instructions (lean_shape(): at most 8 pairs of values per thread)
-__device__ __forceinline__ bool stage_poll_q8(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int more, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
-    return stage_poll_q8_t<MI_LEAN ? 8 : 16, MI_LEAN ? 1 : 2>(ok, P, vw, n, more, tag, xq_s, xs_s);
+__device__ __forceinline__ bool stage_poll_q8(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int nw, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
+    return stage_poll_q8_t<MI_LEAN ? 8 : 16, MI_LEAN ? 1 : 2>(ok, P, vw, n, nw, tag, xq_s, xs_s);
 }
 
 // Shapes the context-range builds take: they hold one variant of each prologue and of the tile loop and no call to the others.
@@ -1864,7 +1864,7 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
             } else if (k == 2 || k == 4) {
                 if (js.at) {                                      // only CTAs that have a unit of the job consume its input
                     prof_mark(P, 2 * k);
-                    ok = stage_poll_q8(done, P, xw_read(P) + (k == 2 ? P.xo.att : P.xo.act), k == 2 ? P.NH * HD : P.FF, k == 2 ? P.seen_n : 0, pub.tag - 1u, xq_s, xs_s);
+                    ok = stage_poll_q8(done, P, xw_read(P) + (k == 2 ? P.xo.att : P.xo.act), k == 2 ? P.NH * HD : P.FF, k == 2 ? P.att_scales : P.FF / 32, pub.tag - 1u, xq_s, xs_s);
                     prof_mark(P, kProfWait);
                 }
             }

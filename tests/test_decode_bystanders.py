@@ -51,7 +51,7 @@ def test_every_cta_that_reads_the_residual_stream_holds_its_writers_back(tmp_pat
     assert some > 20
     # their words, behind the attention output's scales, are awaited by whoever computes the O projection
     kernel = (SRC / "decode_kernel.cuh").read_text()
-    assert "pub.all(P.xo.att + P.NH * HD / 4 + P.NH * HD / 32 + by, 0u)" in kernel and "k == 2 ? P.seen_n : 0, pub.tag - 1u" in kernel
+    assert "pub.all(P.xo.att + P.NH * HD / 4 + P.NH * HD / 32 + by, 0u)" in kernel and "k == 2 ? P.att_scales :" in kernel
 
 
 # 24 of 134 CTAs without a unit of QKV or gate/up (110 of 148 without attention CTAs): one of them comes 200 us late to every read of the residual stream's
