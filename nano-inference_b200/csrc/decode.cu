@@ -377,6 +377,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         MI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
 
+    int units = 3;                                            // of a batch; (room for three in any case: the positions per step of the long-range attention follow from what is left)
     // ---- per-warp tile lists: the order in which each warp of the grid consumes tiles during one step; and what each CTA does in a layer (DecodeParams::work)
     {
         const int nj = (int)m->jobs.size(), G = GG;
@@ -402,30 +403,29 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
                 size_t link = (size_t)jb.kind;                          // where the offset of the next batch goes
                 for (int u = u0; u < jb.n_units; u += kBatchUnits * G) {
                     const size_t at = w.size();
-                    if (u != u0) m->one_batch = false;
                     if (j < 4) {
                         w[link] |= link < 4 ? (unsigned)at : (unsigned)at << 8;
                         link = at;
                         w.resize(at + kBatchWords, 0u);
                     }
                     std::vector<unsigned> items[DNW];
-                    int i = jb.wrot, units = 0;
-                    for (int v = u; v < jb.n_units && units < kBatchUnits; v += G, units++) {
+                    int i = jb.wrot, b = 0;
+                    for (int v = u; v < jb.n_units && b < kBatchUnits; v += G, b++) {
                         // (a unit per CTA at most: split by split; else a row group's splits one after the other, so that no batch waits for a later one)
                         const bool by_split = jb.n_units <= G;
                         const int per = jb.half ? 2 : jb.ks, g = by_split ? v % jb.groups : v / per, q = by_split ? v / jb.groups : v % per, sp = jb.half ? 0 : q, t0 = sp * jb.nt / jb.ks, t1 = (sp + 1) * jb.nt / jb.ks, ntu = t1 - t0;
                         if (j < 4) {
-                            w[at + kBatchGroup + units] = (unsigned)(jb.kind == JOB_GU ? g + jb.g_off : (g + jb.g_off) * 32 + (jb.half ? 16 * q : 0));
-                            w[at + kBatchUnit + units] = (unsigned)sp | (unsigned)std::min(ntu, DNW) << 8 | (unsigned)(i & (DNW - 1)) << 16 | (unsigned)((i + ntu) & (DNW - 1)) << 20;
+                            w[at + kBatchGroup + b] = (unsigned)(jb.kind == JOB_GU ? g + jb.g_off : (g + jb.g_off) * 32 + (jb.half ? 16 * q : 0));
+                            w[at + kBatchUnit + b] = (unsigned)sp | (unsigned)std::min(ntu, DNW) << 8 | (unsigned)(i & (DNW - 1)) << 16 | (unsigned)((i + ntu) & (DNW - 1)) << 20;
                         }
                         for (int a = 0; a < jb.nacc; a++)
                             for (int t = t0; t < t1; t++, i++) {
                                 lists[(size_t)cta * DNW + (i & (DNW - 1))].push_back((unsigned long long)(uintptr_t)(jb.base + ((size_t)(g * jb.nacc + a) * jb.nt + t) * tb) | code);
-                                items[i & (DNW - 1)].push_back((unsigned)(t * jb.kb) | (unsigned)(2 * units + a) << 16 | (t + DNW >= t1 ? 1u << 20 : 0u) | (jb.half && q ? 1u << 21 : 0u));
+                                items[i & (DNW - 1)].push_back((unsigned)(t * jb.kb) | (unsigned)(2 * b + a) << 16 | (t + DNW >= t1 ? 1u << 20 : 0u) | (jb.half && q ? 1u << 21 : 0u));
                             }
                     }
                     if (j >= 4) continue;
-                    w[at] |= (unsigned)units;
+                    w[at] |= (unsigned)b;
                     for (int q = 0; q < DNW; q++) {
                         w[at + kBatchList + q] = (unsigned)w.size() | (unsigned)items[q].size() << 16;
                         w.insert(w.end(), items[q].begin(), items[q].end());
@@ -453,6 +453,7 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
         P.work = d_work; P.work_stride = (int)words; P.work_smem = words <= (size_t)kWorkSmem;
         P.half_rows = 0;
         for (int k = 0; k < 4; k++) { P.kb[k] = m->jobs[k].kb; P.half_rows |= m->jobs[k].half ? 1 << k : 0; }
+        for (int k = 0; k < 4; k++) units = std::max(units, std::min(most_units(m->jobs[k], G), kBatchUnits)), m->one_batch &= most_units(m->jobs[k], G) <= kBatchUnits;
         bystanders(m->jobs[JOB_QKV], m->jobs[JOB_GU], G, &P.seen_first, &P.seen_n);
         P.att_scales = NQ / 32 + P.seen_n;
         const Job& lm = m->jobs.back();
@@ -520,8 +521,9 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
     P.inv_e = 1.0 / (double)E;
     // positions per step of the long-range attention: as many as fit, a multiple of 16 so that score rows stay apart in the banks
     P.split_sub = kSplitSubMax;
-    while (P.split_sub > kSplitSubMin && decode_smem_bytes(E, FF, HD, P.split_sub) + 1024 > (size_t)ctx->smem_optin) P.split_sub -= 16;
-    m->smem = decode_smem_bytes(E, FF, HD, P.split_sub);
+    while (P.split_sub > kSplitSubMin && decode_smem_bytes(E, FF, HD, P.split_sub, units) + 1024 > (size_t)ctx->smem_optin) P.split_sub -= 16;
+    m->smem = decode_smem_bytes(E, FF, HD, P.split_sub, units);
+    P.fold_at = (int)decode_fold_at(E, FF, HD, P.split_sub);
     if (m->attn_ctas > 0) {
         const int hpc = attn_heads_per_cta(m->G);
         m->smem = std::max(m->smem, attn_dedicated_smem(HD, hpc));       // the attention CTAs lay the same allocation out their own way

@@ -6,7 +6,9 @@
 namespace mi {
 
 constexpr int DNW = 8;            // warps per CTA that compute
+constexpr int DNT = DNW * 32;     // their threads
 constexpr int kMaxKSplit = 4;     // cross-CTA K-splits of the down projection
+constexpr int kBatchUnits = 4;    // units of a job that a CTA works on at once: all it has, on the shapes of the range builds (lean_shape)
 
 enum JobKind { JOB_QKV = 0, JOB_O = 1, JOB_GU = 2, JOB_DOWN = 3, JOB_LM = 4 };
 
@@ -70,6 +72,21 @@ inline Job deal_job(int kind, int groups, int nb, int kb, int nacc, int grid, in
 inline int first_unit(const Job& jb, int cta, int grid) {
     const int r = jb.rot % grid;
     return cta >= r ? cta - r : cta + grid - r;
+}
+
+// the most units of the job that a CTA has
+inline int most_units(const Job& jb, int grid) { return (jb.n_units + grid - 1) / grid; }
+
+// Shapes the context-range builds take: they hold one variant of each prologue and of the tile loop and no call to the others, and one batch of units per CTA and job
+// (a full grid deals these shapes at most 455 units to 130 CTAs; with three units per batch a feed-forward width of 14336 had some of four, ran the general
+// build and took 410 us per token for 12 layers where the range build takes 288).  On a smaller grid (MINFER_GRID) more than kBatchUnits units per CTA mean the general build.
+// 1: embedding widths of 1025 to 2048 with tiles of 8 blocks; 2: of 513 to 1024 with tiles of 8 or 4 blocks (the small builds,
+// MI_SMALL: 443 us per token at the 0.5B shape where the general build, whose loop spills, took 539); 0: neither.
+inline int lean_shape(int E, int FF, int NQ) {
+    auto kb = [&](int k) { return (E / 32) % k == 0 && (FF / 32) % k == 0 && (NQ / 32) % k == 0; };
+    auto np = [](int n) { return (n / 8 + (n / 32 + 1) / 2 + DNT - 1) / DNT; };          // pairs of words of a q8_0 vector per thread
+    if (np(FF) > 8 || np(NQ) > 8) return 0;
+    return E > 1024 && E <= 2048 && kb(8) ? 1 : E > 512 && E <= 1024 && kb(4) ? 2 : 0;
 }
 
 // The CTAs with neither a gate/up nor a QKV unit, which the units just dealt leave in one run [*first, *first + *n).  They read the residual stream's words in every layer

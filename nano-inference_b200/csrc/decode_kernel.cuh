@@ -127,7 +127,6 @@
 
 namespace mi {
 
-constexpr int DNT = DNW * 32;     // threads of the warps that compute
 constexpr int DNT_ALL = DNT + 32; // and one warp that requests the weights
 constexpr int DS = 3;             // ring slots per warp
 constexpr int DSLOT = 4608;       // bytes per slot: the largest tile (8 blocks)
@@ -142,11 +141,10 @@ enum { kProfWait = 12, kProfStep = 13, kProfSlots = 32 };
 // What a CTA does in the per-layer jobs, listed by the host (all layers are dealt alike): 32-bit words, [kind] = offset of the job's first batch, or 0.
 // A batch is up to kBatchUnits units; its tiles, numbered unit by unit, accumulator by accumulator (gate, up), along K, go round-robin over the eight warps:
 //   [0] number of units | offset of the next batch << 8, or 0      [1 + b] unit b: its q8_0 block (gate/up), else its first row
-//   [4 + b] K-split of unit b | number of warps with tiles of a sum << 8 | first of them << 16 (gate), << 20 (up)
-//   [7 + w] offset of warp w's list | number of its tiles << 16;  list entry: first block | sum (2 b + accumulator) << 16 | last of the sum << 20 | second half of the rows << 21
+//   [5 + b] K-split of unit b | number of warps with tiles of a sum << 8 | first of them << 16 (gate), << 20 (up)
+//   [9 + w] offset of warp w's list | number of its tiles << 16;  list entry: first block | sum (2 b + accumulator) << 16 | last of the sum << 20 | second half of the rows << 21
 // Where twice the row groups of a job are no more than the CTAs, its units are half row groups (DecodeParams::half_rows): both CTAs of a group read its tiles, the second one from
 // the L2, and a lane has a row of sixteen and half of a tile's blocks.  The down projection of the 1.5B shape is 35 tiles on 96 CTAs instead of 48 so.
-constexpr int kBatchUnits = 3;                        // (the 3B shape's gate/up: two or three units per CTA)
 enum { kBatchGroup = 1, kBatchUnit = kBatchGroup + kBatchUnits, kBatchList = kBatchUnit + kBatchUnits, kBatchWords = kBatchList + 8 };
 
 struct LayerPtrs { const float* attn_norm; const float* ffn_norm; const float* bqkv; };
@@ -183,6 +181,7 @@ struct DecodeParams {
     float eps;
     double inv_e;                    // 1 / E
     const unsigned* work; int work_stride, work_smem;      // per GEMV CTA: its list (see above); whether it goes to shared memory
+    int fold_at;                                           // byte of the shared memory where the sums of a batch meet (decode_fold_at)
     int seen_first, seen_n, att_scales;                    // GEMV CTAs without a unit of QKV and gate/up (bystanders); scales of the attention output and those CTAs' words
     int kb[5], ks_down, half_rows;                         // tile depths by JobKind, K-splits of the down projection, which jobs' units are half row groups (bit per JobKind)
     int lm_units, lm_nt, lm_off;                           // lm_head: row groups and tiles of one, first row group
@@ -248,7 +247,6 @@ struct DecodeSmem {
     uint8_t* ring; uint64_t* bars; const unsigned* work; LayerPtrs* lp; float* cs; double* red; double* fold; float* h; uint8_t* stage;
 };
 
-constexpr int kFoldBytes = kBatchUnits * 2 * DNW * 32 * 8;      // [unit of the batch][acc][warp][lane] doubles
 constexpr int kWorkSmem = 512;                        // words of a CTA's list that fit the shared memory
 
 // attention_split: positions per step (as many as the shared memory allows: a chunk that fits one step has all its rows requested
@@ -277,9 +275,13 @@ __host__ __device__ inline size_t decode_stage_bytes(int E, int FF, int HD, int 
     const size_t b = split > shrt ? split : shrt;
     return ((a > b ? a : b) + 127) / 128 * 128;
 }
-__host__ __device__ inline size_t decode_smem_bytes(int E, int FF, int HD, int sub) {
-    return (size_t)DNW * DS * DSLOT + 512 + kWorkSmem * 4 + 64 * sizeof(LayerPtrs) + 1024 + 256 + kFoldBytes +
+// where the sums of a batch of `units` meet ([unit][acc][warp][lane] doubles), behind everything else
+__host__ __device__ inline size_t decode_fold_at(int E, int FF, int HD, int sub) {
+    return (size_t)DNW * DS * DSLOT + 512 + kWorkSmem * 4 + 64 * sizeof(LayerPtrs) + 1024 + 256 +
            ((size_t)E * 4 + 127) / 128 * 128 + decode_stage_bytes(E, FF, HD, sub);
+}
+__host__ __device__ inline size_t decode_smem_bytes(int E, int FF, int HD, int sub, int units) {
+    return decode_fold_at(E, FF, HD, sub) + (size_t)units * 2 * DNW * 32 * 8;
 }
 
 // close the current profile interval: charge the time since t to slot k (CTA 0, thread 0 only).
@@ -981,16 +983,6 @@ __device__ __forceinline__ bool stage_poll_q8_t(bool ok, const DecodeParams& P, 
 // as many pairs as the longest vector wants; one form per build, so that all phases run the same instructions (lean_shape(): at most 8 pairs of values per thread)
 __device__ __forceinline__ bool stage_poll_q8(bool ok, const DecodeParams& P, const unsigned long long* vw, int n, int nw, unsigned tag, int8_t* xq_s, BlockScale* xs_s) {
     return stage_poll_q8_t<MI_LEAN ? 8 : 16, MI_LEAN ? 1 : 2>(ok, P, vw, n, nw, tag, xq_s, xs_s);
-}
-
-// Shapes the context-range builds take: they hold one variant of each prologue and of the tile loop and no call to the others.
-// 1: embedding widths of 1025 to 2048 with tiles of 8 blocks; 2: of 513 to 1024 with tiles of 8 or 4 blocks (the small builds,
-// MI_SMALL: 443 us per token at the 0.5B shape where the general build, whose loop spills, took 539); 0: neither.
-inline int lean_shape(int E, int FF, int NQ) {
-    auto kb = [&](int k) { return (E / 32) % k == 0 && (FF / 32) % k == 0 && (NQ / 32) % k == 0; };
-    auto np = [](int n) { return (q8_words(n) / 2 + DNT - 1) / DNT; };
-    if (np(FF) > 8 || np(NQ) > 8) return 0;
-    return E > 1024 && E <= 2048 && kb(8) ? 1 : E > 512 && E <= 1024 && kb(4) ? 2 : 0;
 }
 
 // ---- attention over a long causal range --------------------------------------------------
@@ -1740,9 +1732,9 @@ decode_kernel(const __grid_constant__ DecodeParams P, int step0, int step1, int 
     after_jobs += 64 * sizeof(LayerPtrs);
     sm.cs = reinterpret_cast<float*>(after_jobs);                 // [HD]: cos then sin
     sm.red = reinterpret_cast<double*>(after_jobs + 1024);         // 32 doubles
-    sm.fold = reinterpret_cast<double*>(after_jobs + 1024 + 256);
-    sm.h = reinterpret_cast<float*>(after_jobs + 1024 + 256 + kFoldBytes);
-    sm.stage = after_jobs + 1024 + 256 + kFoldBytes + ((size_t)P.E * 4 + 127) / 128 * 128;
+    sm.h = reinterpret_cast<float*>(after_jobs + 1024 + 256);
+    sm.stage = after_jobs + 1024 + 256 + ((size_t)P.E * 4 + 127) / 128 * 128;
+    sm.fold = reinterpret_cast<double*>(smem + P.fold_at);
     __shared__ int s_tok;
     __shared__ int s_quit;                             // the computing warps have left
 #if MI_PROF
