@@ -413,7 +413,8 @@ extern "C" int mi_model_load_gguf_tp(mi_ctx* ctx, const char* path, int max_seq,
                     for (int v = u; v < jb.n_units && b < kBatchUnits; v += G, b++) {
                         // (a unit per CTA at most: split by split; else a row group's splits one after the other, so that no batch waits for a later one)
                         const bool by_split = jb.n_units <= G;
-                        const int per = jb.half ? 2 : jb.ks, g = by_split ? v % jb.groups : v / per, q = by_split ? v / jb.groups : v % per, sp = jb.half ? 0 : q, t0 = sp * jb.nt / jb.ks, t1 = (sp + 1) * jb.nt / jb.ks, ntu = t1 - t0;
+                        const int per = jb.half ? 2 : jb.ks, g = by_split ? v % jb.groups : v / per, q = by_split ? v / jb.groups : v % per;      // row group; which half or split of it
+                        const int sp = jb.half ? 0 : q, t0 = sp * jb.nt / jb.ks, t1 = (sp + 1) * jb.nt / jb.ks, ntu = t1 - t0;
                         if (j < 4) {
                             w[at + kBatchGroup + b] = (unsigned)(jb.kind == JOB_GU ? g + jb.g_off : (g + jb.g_off) * 32 + (jb.half ? 16 * q : 0));
                             w[at + kBatchUnit + b] = (unsigned)sp | (unsigned)std::min(ntu, DNW) << 8 | (unsigned)(i & (DNW - 1)) << 16 | (unsigned)((i + ntu) & (DNW - 1)) << 20;

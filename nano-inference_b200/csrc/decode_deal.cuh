@@ -81,7 +81,7 @@ inline int most_units(const Job& jb, int grid) { return (jb.n_units + grid - 1) 
 // (a full grid deals these shapes at most 455 units to 130 CTAs; with three units per batch a feed-forward width of 14336 had some of four, ran the general
 // build and took 410 us per token for 12 layers where the range build takes 288).  On a smaller grid (MINFER_GRID) more than kBatchUnits units per CTA mean the general build.
 // 1: embedding widths of 1025 to 2048 with tiles of 8 blocks; 2: of 513 to 1024 with tiles of 8 or 4 blocks (the small builds,
-// MI_SMALL: 443 us per token at the 0.5B shape where the general build, whose loop spills, took 539); 0: neither.
+// MI_SMALL: 370 us per token at the 0.5B shape where the general build, whose loop spills, takes 430; 1.5B 520 and 772, 3B 794 and 1089); 0: neither.
 inline int lean_shape(int E, int FF, int NQ) {
     auto kb = [&](int k) { return (E / 32) % k == 0 && (FF / 32) % k == 0 && (NQ / 32) % k == 0; };
     auto np = [](int n) { return (n / 8 + (n / 32 + 1) / 2 + DNT - 1) / DNT; };          // pairs of words of a q8_0 vector per thread

@@ -344,9 +344,13 @@ __device__ __forceinline__ void tw_st(unsigned long long* p, unsigned tag, unsig
 __device__ __forceinline__ bool tw_is(unsigned long long w, unsigned tag) { return (unsigned)(w >> 32) == tag; }
 
 // Where a phase publishes.  What (nearly) every CTA reads goes into kXCopies copies of the exchange block, and CTA i reads copy i % P.copies: a vector is a hundred lines of the
-// L2 or less, each read by 142 CTAs, and the slices that hold several of them were what the words waited for (four copies instead of eight: 1.5B shape
-// 538 us per token instead of 532, 855 instead of 782 behind 8192 positions, but the 3B shape 798 instead of 821).  Words with few readers are in the first copy only.  In the
-// tensor-parallel build shared vectors also go into every other GPU's block.
+// L2 or less, each read by 142 CTAs, and the slices that hold several of them were what the words waited for.  Where a copy's lines lie decides much: a model loaded
+// eight times in one process, us per token, mean (least - most), with 1, 2, 4 and 8 copies:
+//   1.5B shape 582 (570 - 608), 547 (541 - 556), 521 (515 - 535), 521 (516 - 526)        behind 8192 positions 868 (809 - 920), 832 (773 - 870), 780 (753 - 856), 819 (790 - 842)
+//   0.5B shape 371 (347 - 383), 382 (378 - 384), 372 (366 - 376), 369 (366 - 373)        3B shape 827 (797 - 855), 817 (803 - 844), 797 (787 - 802), 801 (793 - 830)
+// Words with few readers are in the first copy only.  The tensor-parallel build, whose shared vectors also go into every other GPU's block, writes and reads the first copy alone
+// (that build without a peer, mean of eight loads: 1.5B shape 536, with the vectors that stay on this GPU in eight copies 577).  A sharded model that the host drives writes
+// all copies and reads the first: one store there would be a test in every publish here (0.6 % of that form's time against 0.9 % of every token).
 struct Pub {
     unsigned long long* xw; unsigned tag; bool mute; int stride;
 #if MI_TP
@@ -387,8 +391,8 @@ MI_COLD_FN bool tw_spin(const unsigned long long* p, unsigned tag, unsigned long
 
 // What a warp does that misses words: every lane fetches its missing words again at once.  Each 64th round the lowest lane that misses one polls that word alone, looks at the time and
 // at the error word, and the other lanes sit at the vote.  (One lane polling from the start, which keeps one load of a warp in flight instead of
-// thirty-two, costs a round trip behind the last word: with the exchange block in eight copies the 1.5B shape took 552 us per token so and takes 532, the 0.5B shape 375 and 364; with a pause
-// of 40 or 150 ns between polls 594 and 604 where 585 was without.)
+// thirty-two, costs a round trip behind the last word: tensor-parallel build without a peer, mean of eight loads, 1.5B shape 561 us per token so and 536, 0.5B 464 and 441, 3B 826 and 800; with a pause
+// of 40 or 150 ns between polls, one load each, 594 and 604 where 585 was without.)
 // Called by all lanes of a warp with the first missing address of each (null: none).  Returns 0 when
 // no lane misses anything, 1 when the lanes are to fetch their missing words again, -1 when the wait gave up.
 __device__ __forceinline__ int tw_wait_warp(const unsigned long long* miss, unsigned tag, unsigned long long budget_ns, const int* err, unsigned round) {
@@ -501,7 +505,7 @@ __device__ __forceinline__ void stream_weights(const DecodeSmem& sm, const Decod
     long long left = lane < DNW && j0 < j1 ? (long long)steps * (e1 - e0) : 0;
     unsigned c = e0, in = 0, lap = 0;
     int issued = 0;
-    const uint64_t policy = l2_policy_evict_first();          // a weight byte is read once per token
+    const uint64_t policy = l2_policy_evict_first();          // a weight byte leaves the HBM once per token: also where two CTAs read a tile (halves) the second finds it in the L2 (1.5B shape: 868.4 MB read, 868.3 of weights)
     unsigned long long next = left > 0 ? __ldg(tab + c) : 0ull;
     while (__any_sync(0xffffffffu, left > 0) && !__any_sync(0xffffffffu, *quit != 0)) {
         const bool go = left > 0 && (lap == 0 || mbar_try_wait(&empty[in], (lap - 1) & 1));        // (the first lap finds the slots empty)
@@ -1414,7 +1418,7 @@ static __device__ __noinline__ bool attention_short(const DecodeParams& P, int l
 // rows of the cached positions are known long before the layer's q arrives, so the CTA copies them into shared memory
 // ahead of time (asynchronous 16-byte copies, rows padded by 16 bytes against bank conflicts; requested as soon as the layer before has left
 // the buffer): between q's arrival and the published output there is
-// no global load at all.  (Bulk copies, a thread for each row, were 28 KB of code.)  (2) One fp16 -> double conversion of a K or V element serves all HPC heads.
+// no global load at all.  (2) One fp16 -> double conversion of a K or V element serves all HPC heads.
 // The new position's K and V come with q as tagged words; they go into the shared-memory rows directly and to the global
 // cache after the output has been published (fenced before this CTA's next output, which is what later readers wait for).
 // The two passes and the softmax are attention_short's; a dot product is added in another order (eight partial sums over an eighth of the dimensions

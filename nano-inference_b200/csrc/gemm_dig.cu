@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(256) tok_digits_kernel(TokX x, int nb, int nst
 }
 
 // SwiGLU, q8_0 and digits of one token over one K range.  What bounds it is the FP64 pipe (about 40 operations per element, an exponential and a division) as long as little is issued beside
-// it: a warp has four blocks at once, four elements per lane (an element per lane and a block per warp at a time, which this replaces, took 28 us for 333 tokens of the
-// 1.5B shape, where 2.98 million elements are 6.5 us of the pipe; now 21).  Sixteen warps: 64 sequences of the 3B shape 3570 us instead of 3526.  The blocks wait in shared memory for the range's exponent.
+// it: a warp has four blocks at once, four elements per lane (333 tokens of the 1.5B shape, where 2.98 million elements are 6.5 us of the pipe: 21 us; with an element
+// per lane and a block per warp at a time 28).  Eight warps: 64 sequences of the 3B shape 3526 us, with sixteen 3570.  The blocks wait in shared memory for the range's exponent.
 constexpr int kSwiWarps = 8;
 __global__ void __launch_bounds__(kSwiWarps * 32) swiglu_digits_kernel(const float* y, TokX act, int nb, int nst, DigX out, int M) {
     __shared__ DigReduce red;

@@ -21,8 +21,7 @@ sys.path.insert(0, str(Path(__file__).resolve().parent.parent))
 import __graft_entry__ as ge    # noqa: E402
 
 SLOTS = {12: "waiting for other CTAs' / GPUs' words", 27: "norm: before the poll", 28: "norm: residual add", 23: "norm: sum of squares",
-         24: "norm: barrier", 25: "norm: quantize", 26: "norm: barrier 2", 18: "tiles: loop and unit bookkeeping", 20: "tiles: ring wait",
-         21: "tiles: arithmetic", 22: "tiles: issuing the next copy", 19: "fold + epilogues", 11: "lm_head rows + pick",
+         24: "norm: barrier", 25: "norm: quantize", 26: "norm: barrier 2", 18: "tiles, with waits for the ring", 19: "fold + epilogues", 11: "lm_head rows + pick",
          0: "QKV stage", 1: "QKV tail", 3: "attention (this CTA)", 4: "O stage", 5: "O tail", 6: "gate/up stage", 7: "gate/up tail", 13: "step prologue"}
 
 
